@@ -172,18 +172,27 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int rows,
 // experts % 32 == 0, experts <= 256, hidden % 64 == 0.
 cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* inv_rms,
                                       const float* norm_weight, const CUtensorMap& tmap_gate,
-                                      int rows, int experts, int hidden, float* logits,
-                                      int32_t* error, cudaStream_t stream);
+                                      int rows, int experts, int hidden, int splits,
+                                      float* logits, int32_t* error, cudaStream_t stream);
 // Pass 1 for bf16 layer inputs: the RMSNorm weight folded into the gate (three bf16 terms of
 // fl32(w[i] * gate[e][i]), `planes` = [3][experts][hidden], built once by launch_fold_gate),
 // the input rows read by TMA through `tmap_x` ([rows][hidden] bf16, box 64 x 128, 128-byte
 // swizzle; `tmap_planes` = [3 * experts][hidden], box 64 x experts), inv_rms applied to the sums.
 cudaError_t launch_fold_gate(const __nv_bfloat16* gate, const float* norm_weight, int experts,
                              int hidden, __nv_bfloat16* planes, cudaStream_t stream);
-// `splits` CTAs share the contraction of one 128-row tile; split s writes its partial sums to
-// logits + s * rows * experts, and launch_router_select_exact adds them up.
-// router_folded_splits picks the split count (1, 2 or 4) for a batch.
-int router_folded_splits(int rows, int hidden, int num_sms);
+// In both forms `splits` CTAs share the contraction of one 128-row tile; split s writes its
+// partial sums to logits + s * rows * experts, and launch_router_select_exact adds them up.
+// router_pass1_splits picks the split count for a batch; splits * rows stays below
+// router_pass1_rows(rows).
+constexpr int kMaxPass1Splits = 32;
+int router_pass1_splits(int rows, int hidden, int num_sms);
+// Rows of partial sums that any batch of up to `max_rows` rows may write.
+inline size_t router_pass1_rows(size_t max_rows, int num_sms) {
+  const size_t split_rows = static_cast<size_t>(num_sms) * 128;  // splits * tiles <= num_sms
+  const size_t small = max_rows * kMaxPass1Splits;
+  const size_t most = small < split_rows ? small : split_rows;
+  return most > max_rows ? most : max_rows;
+}
 cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtensorMap& tmap_planes,
                                         const float* inv_rms, int rows, int experts, int hidden,
                                         int splits, float* logits, int32_t* error,

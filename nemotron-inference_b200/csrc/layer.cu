@@ -874,8 +874,8 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   const size_t token_slots = (T + 127) / 128;
   L->inv_rms.allocate(T * sizeof(float));
   L->normalized.allocate(T * H * sizeof(float));
-  // (a split router pass 1 keeps up to four partial sums per logit for small batches)
-  L->logits.allocate(std::min<size_t>(T, 4736) * 3 * E * sizeof(float) + T * E * sizeof(float));
+  // (a split router pass 1 keeps several partial sums per logit)
+  L->logits.allocate((L->fast_router ? router_pass1_rows(T, device_sm_count()) : T) * E * sizeof(float));
   L->top_index.allocate(T * K * sizeof(int32_t));
   L->top_weight.allocate(T * K * sizeof(float));
   L->y_packed.allocate(token_slots * 128 * H / 2, true);
@@ -1119,21 +1119,20 @@ void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dt
   NMOE_CUDA(cudaMemsetAsync(L->counts.as<int32_t>(), 0, E * sizeof(int32_t), stream));
   const float* offset = L->has_logit_offset ? L->logit_offset.as<float>() : nullptr;
   if (two_pass_router) {
-    int logit_splits = 1;
+    const int logit_splits = router_pass1_splits(tokens, H, L->num_sms);
     if (L->folded_router && in_bf16 && reinterpret_cast<uintptr_t>(input) % 16 == 0) {
       if (L->input_map_base != input || L->input_map_rows != tokens) {
         L->input_map = make_bf16_map(input, tokens, H, 128);
         L->input_map_base = input;
         L->input_map_rows = tokens;
       }
-      logit_splits = router_folded_splits(tokens, H, L->num_sms);
       NMOE_CUDA(launch_router_folded_logits(L->input_map, L->planes_map, L->inv_rms.as<float>(),
                                             tokens, E, H, logit_splits, L->logits.as<float>(),
                                             error, stream));
     } else {
       NMOE_CUDA(launch_router_fast_logits(input, in_bf16, L->inv_rms.as<float>(),
                                           L->norm_weight.as<float>(), L->gate_map, tokens, E, H,
-                                          L->logits.as<float>(), error, stream));
+                                          logit_splits, L->logits.as<float>(), error, stream));
     }
     // A stream forked here runs the shared expert beside the selection, plan and permute
     // kernels; forked before pass 1 its persistent GEMM CTAs would hold the shared memory

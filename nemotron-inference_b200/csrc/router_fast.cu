@@ -22,6 +22,7 @@
 // top-k set is contained in the candidates, so indices AND weights equal the
 // all-FP64 path.  tie_margin is ~20x the largest pass-1 error measured.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(kFastThreads, 1)
 router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ inv_rms,
                           const float* __restrict__ norm_weight,
                           const __grid_constant__ CUtensorMap tmap_gate, int rows, int experts,
-                          int hidden, float* __restrict__ logits, int32_t* error) {
+                          int hidden, int splits, float* __restrict__ logits, int32_t* error) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
                                              ~static_cast<uintptr_t>(1023u));
@@ -92,8 +93,13 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int row0 = blockIdx.x * 128;
-  const int k_blocks = hidden / kFastBlockK;
+  // `splits` CTAs share the contraction of a tile (see router_folded_logits_kernel)
+  const int tile = static_cast<int>(blockIdx.x) / splits;
+  const int split = static_cast<int>(blockIdx.x) - tile * splits;
+  const int row0 = tile * 128;
+  const int all_k_blocks = hidden / kFastBlockK;
+  const int kb_begin = all_k_blocks * split / splits;
+  const int k_blocks = all_k_blocks * (split + 1) / splits - kb_begin;
   const uint32_t tmem_cols = experts <= 32 ? 32 : experts <= 64 ? 64 : experts <= 128 ? 128 : 256;
 
   if (threadIdx.x == 0) {
@@ -126,7 +132,8 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
           break;
         }
         mbar_arrive_expect_tx(&full_bar[stage], b_bytes);
-        tma_load_2d(sB + stage * b_bytes, &tmap_gate, kb * kFastBlockK, 0, &full_bar[stage]);
+        tma_load_2d(sB + stage * b_bytes, &tmap_gate, (kb_begin + kb) * kFastBlockK, 0,
+                    &full_bar[stage]);
         if (++stage == kFastStages) {
           stage = 0;
           phase ^= 1u;
@@ -189,8 +196,8 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int row = min(row0 + row_of[j], rows - 1);
-        load_x8<IN_BF16>(x, static_cast<size_t>(row) * hidden + kb * kFastBlockK + chunk * 8,
-                         dst[j]);
+        load_x8<IN_BF16>(
+            x, static_cast<size_t>(row) * hidden + (kb_begin + kb) * kFastBlockK + chunk * 8, dst[j]);
       }
     };
     fetch(0, xv[0]);
@@ -199,9 +206,9 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
     uint32_t phase = 0;
     bool ok = true;
     for (int kb = 0; kb < k_blocks; ++kb) {
-      const float4 w0 = *reinterpret_cast<const float4*>(norm_weight + kb * kFastBlockK + chunk * 8);
-      const float4 w1 =
-          *reinterpret_cast<const float4*>(norm_weight + kb * kFastBlockK + chunk * 8 + 4);
+      const float* w_at = norm_weight + (kb_begin + kb) * kFastBlockK + chunk * 8;
+      const float4 w0 = *reinterpret_cast<const float4*>(w_at);
+      const float4 w1 = *reinterpret_cast<const float4*>(w_at + 4);
       const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
       uint32_t words[4][3][4];
       auto split = [&](float (&src)[4][8]) {
@@ -269,7 +276,7 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
           float v[16];
           tmem_ld_x16(t_addr + c, v);
           if (row < rows) {
-            float* dst = logits + static_cast<size_t>(row) * experts + c;
+            float* dst = logits + (static_cast<size_t>(split) * rows + row) * experts + c;
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
               *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
@@ -300,7 +307,6 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
 // the size of the FP32 accumulation error already covered by the tie margin.
 // ---------------------------------------------------------------------------
 constexpr int kFoldThreads = 6 * 32;
-constexpr int kFoldMaxSplits = 4;
 constexpr int kFoldABytes = 128 * 128;  // 128 rows x 64 bf16
 
 __global__ void fold_gate_kernel(const __nv_bfloat16* __restrict__ gate,
@@ -460,6 +466,7 @@ router_folded_logits_kernel(const __grid_constant__ CUtensorMap tmap_x,
 // ---------------------------------------------------------------------------
 constexpr int kSelectWarps = 4;
 constexpr int kSelectPerLane = 8;  // experts <= 256
+constexpr int kSelectWholeBlockRows = 1024;
 
 __device__ __forceinline__ float sigmoid_exact(float v) {
   // Sigmoid of expert_layer.cpp:129-136 with exp evaluated in double
@@ -486,11 +493,43 @@ __device__ __forceinline__ void warp_arg_max(uint32_t key, uint32_t index, uint3
   best_index = __reduce_min_sync(0xffffffffu, key == best_key ? index : 0xffffffffu);
 }
 
-// One warp per token.  The FP64 dot products dominate; everything around them is kept
-// to a few warp-wide redux steps per selected expert.
-constexpr int kSelectBatch = 4;
-template <bool IN_BF16>
-__global__ void __launch_bounds__(kSelectWarps * 32, 8)
+// A bf16 value (the upper half of `w`; the lower half is ignored) times 2^-896 as a double, in
+// two integer instructions: the bits of a bf16 moved three places down are those of a double
+// whose exponent field still has the 8-bit bias (subnormals included).  The conversion unit
+// would be what this kernel waits for: it has a quarter of the FP64 unit's rate.
+constexpr double kGateUnscale = 0x1p896;
+__device__ __forceinline__ double gate_scaled(uint32_t w) {
+  return __hiloint2double((static_cast<int>(w) >> 3) & static_cast<int>(0x8fffe000u), 0);
+}
+
+// Sums eight values over the warp: after the call lane L holds the total of value
+// ((L >> 4) & 1) * 4 + ((L >> 3) & 1) * 2 + ((L >> 2) & 1).  Half of the values change hands in
+// each of the first three steps, nine shuffles instead of forty.
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int half = 4; half > 0; half >>= 1) {
+    const int stride = half * 4;
+    const bool upper = (lane & stride) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double send = upper ? v[i] : v[i + half];
+      const double keep = upper ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, stride);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
+// WARPS warps per token: one for large batches (four tokens a block, nothing exchanged), four
+// for small ones, where the chain of loads and FP64 sums of one token is what counts: they
+// share the contraction and repeat the short steps around it.  BATCH candidates are evaluated
+// per pass over the row (at least top_k, so that one pass is the rule).
+// Measured, 128 experts, hidden 2688, bf16 in: 256 tokens 35 -> 17 us, 16384 tokens
+// 143 -> 119 us.
+template <bool IN_BF16, int WARPS, int BATCH>
+__global__ void __launch_bounds__(kSelectWarps * 32)
 router_select_exact_kernel(float* __restrict__ logits, int splits, const void* __restrict__ x,
                            const float* __restrict__ inv_rms,
                            const float* __restrict__ norm_weight,
@@ -500,14 +539,37 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
                            float routed_scaling, float tie_margin,
                            int32_t* __restrict__ top_index, float* __restrict__ top_weight,
                            int32_t* __restrict__ expert_counts) {
+  static_assert(WARPS == 1 || WARPS == kSelectWarps, "one warp, or the block, per token");
   __shared__ int16_t candidate_list[kSelectWarps][256];
+  __shared__ float logit_smem[WARPS > 1 ? 256 : 1];
+  __shared__ double partial_smem[WARPS > 1 ? kSelectWarps : 1][8];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const int row = blockIdx.x * kSelectWarps + warp;
+  const int part = WARPS > 1 ? warp : 0;  // this warp's share of the contraction
+  const int row = WARPS > 1 ? static_cast<int>(blockIdx.x) : blockIdx.x * kSelectWarps + warp;
   if (row >= rows) return;
   const int per_lane = experts / 32;
   float* row_logits = logits + static_cast<size_t>(row) * experts;
 
+  // pass-1 logit of expert e: the partial sums of a split pass 1, in split order
+  const bool changed = logit_offset != nullptr || splits > 1;
+  auto pass1_logit = [&](int e) {
+    float l = row_logits[e];
+    const size_t step = static_cast<size_t>(rows) * experts;
+    const float* next = row_logits + e;
+#pragma unroll 8
+    for (int sp = 1; sp < splits; ++sp) {
+      next += step;
+      l = __fadd_rn(l, *next);
+    }
+    if (logit_offset != nullptr) l = __fadd_rn(l, logit_offset[e]);
+    if (changed) row_logits[e] = l;  // what the trace shows for experts not re-evaluated
+    return l;
+  };
+  if constexpr (WARPS > 1) {
+    for (int e = threadIdx.x; e < experts; e += kSelectWarps * 32) logit_smem[e] = pass1_logit(e);
+    __syncthreads();
+  }
   // pass-1 choice scores (single precision is enough here: the margin covers it);
   // lane L holds experts L, L + 32, ...
   float choice[kSelectPerLane];
@@ -518,15 +580,7 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
     key[j] = 0u;
     if (j < per_lane) {
       const int e = lane + 32 * j;
-      float l = row_logits[e];
-      // partial sums of a split pass 1, in split order
-      for (int sp = 1; sp < splits; ++sp) {
-        l = __fadd_rn(l, row_logits[static_cast<size_t>(sp) * rows * experts + e]);
-      }
-      if (logit_offset != nullptr) l = __fadd_rn(l, logit_offset[e]);
-      if (logit_offset != nullptr || splits > 1) {
-        row_logits[e] = l;  // what the trace shows for experts that are not re-evaluated
-      }
+      const float l = WARPS > 1 ? logit_smem[e] : pass1_logit(e);
       choice[j] = __fdividef(1.0f, 1.0f + __expf(-l)) + bias[e];
       key[j] = ordered_bits(choice[j]);
     }
@@ -578,61 +632,65 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
   }
   __syncwarp();
 
-  // FP64 logits of the candidates, up to kSelectBatch at a time; every lane takes
-  // eight consecutive hidden elements per step.  y is rebuilt from the layer input with
-  // the RMSNorm kernel's own two roundings: (x * inv_rms) * w.
+  // FP64 logits of the candidates, BATCH at a time; every lane takes eight consecutive hidden
+  // elements per step.  y is rebuilt from the layer input with the RMSNorm kernel's own two
+  // roundings: (x * inv_rms) * w.
   const float rinv = inv_rms[row];
   const int chunks = hidden / 8;
-  constexpr int kBatch = kSelectBatch;
-  for (int base = 0; base < total; base += kBatch) {
-    const int batch = min(kBatch, total - base);
-    int e[kBatch];
-    double acc[kBatch];
+  for (int base = 0; base < total; base += BATCH) {
+    const int batch = min(BATCH, total - base);
+    const uint4* gate_row[BATCH];
+    double acc[8];
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      e[i] = candidate_list[warp][min(base + i, total - 1)];
-      acc[i] = 0.0;
+    for (int i = 0; i < 8; ++i) acc[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) {
+      // (past the end of the list the last candidate once more, ignored below)
+      const int e = candidate_list[warp][min(base + i, total - 1)];
+      gate_row[i] = reinterpret_cast<const uint4*>(gate + static_cast<size_t>(e) * hidden);
     }
-    for (int ch = lane; ch < chunks; ch += 32) {
+    for (int ch = lane + 32 * part; ch < chunks; ch += 32 * WARPS) {
+      uint4 g[BATCH];
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) g[i] = gate_row[i][ch];
       float xv[8];
       load_x8<IN_BF16>(x, static_cast<size_t>(row) * hidden + ch * 8, xv);
       const float4 w0 = *reinterpret_cast<const float4*>(norm_weight + ch * 8);
       const float4 w1 = *reinterpret_cast<const float4*>(norm_weight + ch * 8 + 4);
       const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-      double a[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        a[i] = static_cast<double>(__fmul_rn(__fmul_rn(xv[i], rinv), w[i]));
-      }
+      for (int j = 0; j < 4; ++j) {
+        const double a0 =
+            static_cast<double>(__fmul_rn(__fmul_rn(xv[2 * j], rinv), w[2 * j])) * kGateUnscale;
+        const double a1 =
+            static_cast<double>(__fmul_rn(__fmul_rn(xv[2 * j + 1], rinv), w[2 * j + 1])) *
+            kGateUnscale;
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) {
-        if (i < batch) {
-          const uint4 g = *reinterpret_cast<const uint4*>(gate + static_cast<size_t>(e[i]) * hidden +
-                                                          ch * 8);
-          const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[i] = fma(a[2 * j], static_cast<double>(__uint_as_float(gw[j] << 16)), acc[i]);
-            acc[i] = fma(a[2 * j + 1], static_cast<double>(__uint_as_float(gw[j] & 0xffff0000u)),
-                         acc[i]);
-          }
+        for (int i = 0; i < BATCH; ++i) {
+          const uint32_t two = j == 0 ? g[i].x : j == 1 ? g[i].y : j == 2 ? g[i].z : g[i].w;
+          acc[i] = fma(a0, gate_scaled(two << 16), acc[i]);
+          acc[i] = fma(a1, gate_scaled(two), acc[i]);
         }
       }
     }
+    double sum = warp_sum8(acc, lane);
+    const int mine_of_batch = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+    if constexpr (WARPS > 1) {
+      if ((lane & 3) == 0) partial_smem[warp][mine_of_batch] = sum;
+      __syncthreads();
+      sum = 0.0;
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      if (i < batch) {
-        double v = acc[i];
-#pragma unroll
-        for (int stride = 16; stride > 0; stride >>= 1) v += __shfl_xor_sync(0xffffffffu, v, stride);
-        if (lane == 0) {
-          float logit = static_cast<float>(v);
-          if (logit_offset != nullptr) logit = __fadd_rn(logit, logit_offset[e[i]]);
-          row_logits[e[i]] = logit;
-        }
-      }
+      for (int p = 0; p < WARPS; ++p) sum += partial_smem[p][mine_of_batch];
+      __syncthreads();
+    }
+    if ((lane & 3) == 0 && mine_of_batch < batch && part == 0) {
+      const int e = candidate_list[warp][base + mine_of_batch];
+      float logit = static_cast<float>(sum);
+      if (logit_offset != nullptr) logit = __fadd_rn(logit, logit_offset[e]);
+      row_logits[e] = logit;
     }
   }
+  if (part != 0) return;
   __syncwarp();
 
   // exact scores, compacted: lane L takes candidates L, L + 32, ... of the list, so the
@@ -700,7 +758,9 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
     w = __fmul_rn(w, routed_scaling);
     top_index[static_cast<size_t>(row) * top_k + lane] = my_index;
     top_weight[static_cast<size_t>(row) * top_k + lane] = w;
-    if (expert_counts != nullptr) atomicAdd(&expert_counts[my_index], 1);
+    if (expert_counts != nullptr && static_cast<uint32_t>(my_index) < static_cast<uint32_t>(experts)) {
+      atomicAdd(&expert_counts[my_index], 1);
+    }
   }
 }
 
@@ -708,26 +768,27 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
 
 cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* inv_rms,
                                       const float* norm_weight, const CUtensorMap& tmap_gate,
-                                      int rows, int experts, int hidden, float* logits,
-                                      int32_t* error, cudaStream_t stream) {
-  if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0) {
+                                      int rows, int experts, int hidden, int splits,
+                                      float* logits, int32_t* error, cudaStream_t stream) {
+  if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0 ||
+      splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
   }
   const int smem = kFastStages * (kFastABytes + experts * 128) + (2 * kFastStages + 1) * 8 + 16 + 1024;
-  const int grid = (rows + 127) / 128;
+  const int grid = (rows + 127) / 128 * splits;
   cudaError_t err;
   if (x_bf16) {
     err = cudaFuncSetAttribute(router_fast_logits_kernel<true>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return err;
     router_fast_logits_kernel<true><<<grid, kFastThreads, smem, stream>>>(
-        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, logits, error);
+        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
   } else {
     err = cudaFuncSetAttribute(router_fast_logits_kernel<false>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return err;
     router_fast_logits_kernel<false><<<grid, kFastThreads, smem, stream>>>(
-        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, logits, error);
+        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
   }
   return cudaGetLastError();
 }
@@ -739,14 +800,13 @@ cudaError_t launch_fold_gate(const __nv_bfloat16* gate, const float* norm_weight
   return cudaGetLastError();
 }
 
-int router_folded_splits(int rows, int hidden, int num_sms) {
+// As many CTAs per row tile as keep every CTA on an SM of its own, each with two K blocks at
+// least: the chain of K blocks is what a CTA takes its time for (FP32 input, 256 rows: 78 us on
+// two CTAs, 14 us on 42).
+int router_pass1_splits(int rows, int hidden, int num_sms) {
   const int tiles = (rows + 127) / 128;
-  int splits = 1;
-  while (splits < kFoldMaxSplits && tiles * splits * 2 <= num_sms &&
-         hidden / kFastBlockK >= 8 * splits) {
-    splits *= 2;
-  }
-  return splits;
+  const int most = std::max(1, hidden / kFastBlockK / 2);
+  return std::min(std::max(1, num_sms / tiles), std::min(most, kMaxPass1Splits));
 }
 
 cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtensorMap& tmap_planes,
@@ -754,7 +814,7 @@ cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtenso
                                         int splits, float* logits, int32_t* error,
                                         cudaStream_t stream) {
   if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0 ||
-      splits < 1 || splits > kFoldMaxSplits || hidden / kFastBlockK < splits) {
+      splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
   }
   const int stage_bytes = kFoldABytes + 3 * experts * 128;
@@ -780,15 +840,28 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
       top_k > 32 || top_k > experts || hidden % 8 != 0 || splits < 1) {
     return cudaErrorInvalidValue;
   }
-  const int grid = (rows + kSelectWarps - 1) / kSelectWarps;
+  const bool whole_block = rows <= kSelectWholeBlockRows;
+  const int grid = whole_block ? rows : (rows + kSelectWarps - 1) / kSelectWarps;
+  auto run = [&](auto kernel) {
+    kernel<<<grid, kSelectWarps * 32, 0, stream>>>(
+        logits, splits, x, inv_rms, norm_weight, gate, logit_offset, bias, rows, experts, hidden,
+        top_k, norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts);
+  };
+  auto run_batch = [&](auto bf16, auto warps) {
+    if (top_k <= 4) {
+      run(router_select_exact_kernel<decltype(bf16)::value, decltype(warps)::value, 4>);
+    } else if (top_k <= 6) {
+      run(router_select_exact_kernel<decltype(bf16)::value, decltype(warps)::value, 6>);
+    } else {
+      run(router_select_exact_kernel<decltype(bf16)::value, decltype(warps)::value, 8>);
+    }
+  };
+  using One = std::integral_constant<int, 1>;
+  using Block = std::integral_constant<int, kSelectWarps>;
   if (x_bf16) {
-    router_select_exact_kernel<true><<<grid, kSelectWarps * 32, 0, stream>>>(
-        logits, splits, x, inv_rms, norm_weight, gate, logit_offset, bias, rows, experts, hidden, top_k,
-        norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts);
+    if (whole_block) run_batch(std::true_type(), Block()); else run_batch(std::true_type(), One());
   } else {
-    router_select_exact_kernel<false><<<grid, kSelectWarps * 32, 0, stream>>>(
-        logits, splits, x, inv_rms, norm_weight, gate, logit_offset, bias, rows, experts, hidden, top_k,
-        norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts);
+    if (whole_block) run_batch(std::false_type(), Block()); else run_batch(std::false_type(), One());
   }
   return cudaGetLastError();
 }
