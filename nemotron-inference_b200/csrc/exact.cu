@@ -1,0 +1,822 @@
+// Correctly rounded linears on the tensor cores: y = x W^T with the sum the reference
+// accumulates in double (UploadedLinearOp, runtime/src/backend/linear_op.cpp:97-118, and
+// ScaledFp8LinearOp, runtime/src/backend/scaled_fp8_linear.cu:222-283) and rounds to FP32 once.
+//
+// FP64 arithmetic runs at 1/70 of the int8 tensor rate here, and widening FP32 operands for it
+// is slower still (15 conversions per clock and SM), so a matrix of any size is done in integers:
+//   * every row of x and of W is written once as fixed point below its own largest magnitude,
+//     39 bits in five signed base-256 digits ("slices", after Ootomo, Ozaki and Yokota's use of
+//     integer matrix units for FP64 products);
+//   * tcgen05.mma.kind::i8 multiplies the slices and accumulates exactly in 32-bit integers:
+//     digit i of W times digit j of x belongs to level i + j, the 22 products of levels 0..6 are
+//     computed, the rest and the bits below the fixed point are bounded;
+//   * the seven levels are put together in double, r, with a bound B on everything left out.  When
+//     r - B and r + B round to the same FP32 number that number is the result (Ziv's test);
+//     otherwise -- one value in tens of thousands -- the sum is formed in FP64 from the operands.
+//     (Without level 6 one in a thousand stays open, and those take longer than level 6 does.)
+// One token row or a handful is bound by reading W instead: exact_gemv_kernel reads W in the
+// form it came in (FP8, bf16 or FP32) and sums in FP64.
+#include <algorithm>
+
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace nmoe {
+namespace {
+
+constexpr int kSlices = 5;
+constexpr int kLevels = 7;
+constexpr int kFixedBits = 38;       // |x| < 2^e is stored as round(x * 2^(38 - e)); the top digit
+                                     // then stays below 65 with the carries of the others
+constexpr int kNoExponent = 1 << 20; // a row that holds an infinity or NaN
+
+// Weight values as the reference multiplies with them: FP32, widened bf16, or
+// DecodeFp8(byte) * weight_scale.
+template <int KIND>
+__device__ __forceinline__ float weight_value(const void* w, size_t i, float scale) {
+  if constexpr (KIND == kWeightFp8) {
+    return __fmul_rn(decode_e4m3(reinterpret_cast<const uint8_t*>(w)[i]), scale);
+  } else if constexpr (KIND == kWeightBf16) {
+    return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w)[i]);
+  } else {
+    return reinterpret_cast<const float*>(w)[i];
+  }
+}
+
+// The activation the linear multiplies with: the row itself, or for the scaled-FP8 family its
+// round trip through E4M3 (scaled_fp8_linear.cu:94-106).
+__device__ __forceinline__ float input_value(float v, float fp8_scale) {
+  if (fp8_scale == 0.0f) return v;
+  return __fmul_rn(decode_e4m3(encode_e4m3(__fdiv_rn(v, fp8_scale))), fp8_scale);
+}
+
+// Exponent e with |v| < 2^e for every v of magnitude up to `amax`.
+__device__ __forceinline__ int exponent_above(float amax) {
+  if (!(amax < INFINITY)) return kNoExponent;  // infinity or NaN
+  const int biased = static_cast<int>(__float_as_uint(amax) >> 23);
+  return (biased == 0 ? 1 : biased) - 126;
+}
+
+// Five digits of v below 2^e, the most significant first; returns whether they hold v exactly.
+__device__ __forceinline__ bool digits_of(float v, int e, int8_t (&d)[kSlices]) {
+  const uint32_t bits = __float_as_uint(v);
+  const int biased = static_cast<int>((bits >> 23) & 0xffu);
+  const uint32_t mantissa = (bits & 0x7fffffu) | (biased != 0 ? 0x800000u : 0u);
+  // v = mantissa * 2^(max(biased, 1) - 150)
+  const int shift = (biased == 0 ? 1 : biased) - 150 + kFixedBits - e;
+  long long m = 0;
+  bool exact = true;
+  if (shift >= 0) {
+    m = static_cast<long long>(mantissa) << min(shift, 62 - 24);
+  } else if (shift > -25) {
+    m = (static_cast<long long>(mantissa) + (1ll << (-shift - 1))) >> -shift;
+    exact = (mantissa & ((1u << -shift) - 1u)) == 0u;
+  } else {
+    exact = mantissa == 0u;
+  }
+  if (bits >> 31) m = -m;
+#pragma unroll
+  for (int i = kSlices - 1; i >= 0; --i) {
+    d[i] = static_cast<int8_t>(m & 0xff);
+    m = (m - d[i]) >> 8;
+  }
+  return exact;
+}
+
+constexpr int kExactRows = 128;  // weight rows per tile
+constexpr int kExactChunk = 64;  // bytes of K per pipeline stage (64-byte swizzle)
+
+// Where the 8 bytes of row `row`, slice `slice`, columns k .. k + 7 go.  A tile of `tile_rows` rows
+// keeps every 64-byte chunk of K as one contiguous piece, [slice][row][64], already in the shared-
+// memory image of the tensor core's 64-byte swizzle, so that a stage is one bulk copy.
+__device__ __forceinline__ size_t slice_offset(size_t row, int slice, int k, int K,
+                                               int tile_rows) {
+  const size_t tile = row / tile_rows;
+  const int r = static_cast<int>(row - tile * tile_rows);
+  const size_t chunk = tile * (K / kExactChunk) + k / kExactChunk;
+  const int c = k & (kExactChunk - 1);
+  return (chunk * kSlices + slice) * (static_cast<size_t>(tile_rows) * kExactChunk) +
+         r * kExactChunk + ((((c >> 4) ^ (r >> 1)) & 3) << 4) + (c & 15);
+}
+
+constexpr int kSliceThreads = 256;
+
+// One block per row, the row in registers (STEPS times eight consecutive values per thread): its
+// largest magnitude, then the digits.  KIND < 0: FP32 activation rows.
+template <int KIND, int STEPS>
+__global__ void __launch_bounds__(kSliceThreads)
+slice_rows_kernel(const void* __restrict__ in, int K, float scale, int tile_rows,
+                  int8_t* __restrict__ slices, SliceRow* __restrict__ info) {
+  __shared__ float warp_max[kSliceThreads / 32];
+  const size_t row = blockIdx.x;
+  float v[STEPS][8];
+  float amax = 0.0f;
+  bool bad = false;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+    const int k = (s * kSliceThreads + static_cast<int>(threadIdx.x)) * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[s][j] = 0.0f;
+    if (k < K) {
+      if constexpr (KIND < 0) {
+        const float4* from =
+            reinterpret_cast<const float4*>(reinterpret_cast<const float*>(in) + row * K + k);
+        const float4 a = from[0], b = from[1];
+        const float raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[s][j] = input_value(raw[j], scale);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[s][j] = weight_value<KIND < 0 ? 0 : KIND>(in, row * K + k + j, scale);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float magnitude = fabsf(v[s][j]);
+      bad = bad || !(magnitude < INFINITY);
+      amax = fmaxf(amax, magnitude);
+    }
+  }
+  if (bad) amax = INFINITY;
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1) {
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, stride));
+  }
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = amax;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kSliceThreads / 32; ++w) amax = fmaxf(amax, warp_max[w]);
+  const int e = exponent_above(amax);
+  int inexact = 0;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+    const int k = (s * kSliceThreads + static_cast<int>(threadIdx.x)) * 8;
+    if (k >= K) continue;
+    uint32_t words[kSlices][2] = {};
+    if (e != kNoExponent) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        int8_t d[kSlices];
+        if (!digits_of(v[s][j], e, d)) ++inexact;
+#pragma unroll
+        for (int i = 0; i < kSlices; ++i) {
+          words[i][j >> 2] |= static_cast<uint32_t>(static_cast<uint8_t>(d[i])) << (8 * (j & 3));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kSlices; ++i) {
+      *reinterpret_cast<uint2*>(slices + slice_offset(row, i, k, K, tile_rows)) =
+          make_uint2(words[i][0], words[i][1]);
+    }
+  }
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1) {
+    inexact += __shfl_xor_sync(0xffffffffu, inexact, stride);
+  }
+  __shared__ int warp_inexact[kSliceThreads / 32];
+  if ((threadIdx.x & 31) == 0) warp_inexact[threadIdx.x >> 5] = inexact;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int total = 0;
+    for (int w = 0; w < kSliceThreads / 32; ++w) total += warp_inexact[w];
+    info[row] = SliceRow{e, total};
+  }
+}
+
+template <int KIND>
+void launch_slices(const void* in, int rows, int K, float scale, int tile_rows, int8_t* slices,
+                   SliceRow* info, cudaStream_t stream) {
+  auto run = [&](auto kernel) {
+    kernel<<<rows, kSliceThreads, 0, stream>>>(in, K, scale, tile_rows, slices, info);
+  };
+  if (K <= 2 * kSliceThreads * 8) {
+    run(slice_rows_kernel<KIND, 2>);
+  } else if (K <= 4 * kSliceThreads * 8) {
+    run(slice_rows_kernel<KIND, 4>);
+  } else {
+    run(slice_rows_kernel<KIND, 8>);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// the integer product: 128 weight rows x `nt` token rows per CTA
+//
+// A = the weight slices (M = 128), B = the token slices.  For weight digit i the token digits that
+// meet it are the rows of one B tile, and level s of the sum lies at TMEM column s * nt, so one
+// MMA of up to 256 columns multiplies digit i with several token digits and adds each product to
+// the level it belongs to; A is read once for all of them.  A CTA takes one tile, or a share of
+// its K range, and stores the levels put together as doubles.
+// Bound by the int8 MMA rate, which measures half of the FP8 rate here (64 token rows: 3300
+// cycles of MMA per 60 KB stage).  The checkpoint's shared_up (5376 x 4096), 1000 rows: 13,800 ->
+// 580 us with the two kernels around it; 40 rows: 381 -> 60 us.
+// ---------------------------------------------------------------------------
+constexpr int kExactStages = 3;
+constexpr int kExactThreads = 6 * 32;
+constexpr int kExactABytes = kSlices * kExactRows * kExactChunk;
+
+__device__ __forceinline__ void tcgen05_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                               uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// kind::i8 instruction descriptor: S32 accumulate, S8 x S8, K-major, M = 128
+__device__ __forceinline__ uint32_t make_idesc_i8(uint32_t n) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+__global__ void __launch_bounds__(kExactThreads, 1)
+exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict__ x_slices,
+                  int rows, int N, int K, int nt, int row_tiles, int splits,
+                  double* __restrict__ partial, int32_t* error) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
+                                             ~static_cast<uintptr_t>(1023u));
+  const int b_bytes = kSlices * nt * kExactChunk;
+  uint8_t* sA = smem;
+  uint8_t* sB = sA + kExactStages * kExactABytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sB + kExactStages * b_bytes);
+  uint64_t* empty_bar = full_bar + kExactStages;
+  uint64_t* done_bar = empty_bar + kExactStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  // consecutive CTAs share a weight tile
+  int index = static_cast<int>(blockIdx.x);
+  const int split = index % splits;
+  index /= splits;
+  const int row_tile = index % row_tiles;
+  const int n0 = index / row_tiles * kExactRows;
+  const int row0 = row_tile * nt;
+  const int all_chunks = K / kExactChunk;
+  const int chunk0 = all_chunks * split / splits;
+  const int chunks = all_chunks * (split + 1) / splits - chunk0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kExactStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int8_t* w_from =
+          w_slices + (static_cast<size_t>(n0 / kExactRows) * all_chunks + chunk0) * kExactABytes;
+      const int8_t* x_from =
+          x_slices + (static_cast<size_t>(row_tile) * all_chunks + chunk0) * b_bytes;
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int c = 0; c < chunks; ++c) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1u)) {
+          if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
+          break;
+        }
+        mbar_arrive_expect_tx(&full_bar[stage], kExactABytes + b_bytes);
+        bulk_load(sA + stage * kExactABytes, w_from, kExactABytes, &full_bar[stage]);
+        bulk_load(sB + stage * b_bytes, x_from, b_bytes, &full_bar[stage]);
+        w_from += kExactABytes;
+        x_from += b_bytes;
+        if (++stage == kExactStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const int most = 256 / nt;  // token digits of one MMA
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int c = 0; c < chunks; ++c) {
+        if (!mbar_wait(&full_bar[stage], phase)) {
+          if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
+          ok = false;
+          break;
+        }
+        tcgen05_fence_after();
+        const uint32_t a_addr = smem_u32(sA + stage * kExactABytes);
+        const uint32_t b_addr = smem_u32(sB + stage * b_bytes);
+#pragma unroll 1
+        for (int ks = 0; ks < kExactChunk / 32; ++ks) {
+#pragma unroll 1
+          for (int i = 0; i < kSlices; ++i) {
+            const uint64_t a_desc =
+                make_smem_desc(a_addr + i * (kExactRows * kExactChunk) + ks * 32, 0, 512, 4);
+            const int meet = min(kSlices, kLevels - i);  // token digits within the levels
+            for (int j = 0; j < meet;) {
+              int count = min(most, meet - j);
+              uint32_t accumulate = 1u;
+              if ((c | ks) == 0) {
+                // digit 0 of W starts the first kSlices levels, the next digits one more each
+                if (i == 0) {
+                  accumulate = 0u;
+                } else if (i <= kLevels - kSlices) {
+                  accumulate = j + 1 == meet ? 0u : 1u;
+                  count = min(count, accumulate != 0u ? meet - 1 - j : 1);
+                }
+              }
+              tcgen05_mma_i8(tmem_base + (i + j) * nt, a_desc,
+                             make_smem_desc(b_addr + j * nt * kExactChunk + ks * 32, 0, 512, 4),
+                             make_idesc_i8(static_cast<uint32_t>(count * nt)), accumulate);
+              j += count;
+            }
+          }
+        }
+        tcgen05_commit(&empty_bar[stage]);
+        if (++stage == kExactStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      if (ok) tcgen05_commit(done_bar);
+    }
+  } else {
+    // epilogue: warp w owns TMEM lane quarter w % 4; a thread owns a weight row
+    const int quarter = warp & 3;
+    const int n = n0 + quarter * 32 + lane;
+    if (mbar_wait(done_bar, 0)) {
+      tcgen05_fence_after();
+      const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+      double* out = partial + static_cast<size_t>(split) * rows * N;
+      for (int c = 0; c < nt && row0 + c < rows; c += 16) {
+        double sum[16];
+#pragma unroll
+        for (int s = 0; s < kLevels; ++s) {
+          float raw[16];
+          tmem_ld_x16(t_addr + s * nt + c, raw);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const double level = static_cast<double>(__float_as_int(raw[i]));
+            sum[i] = s == 0 ? level : fma(sum[i], 256.0, level);
+          }
+        }
+        if (n < N) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            if (row0 + c + i < rows) out[static_cast<size_t>(row0 + c + i) * N + n] = sum[i];
+          }
+        }
+      }
+    } else if (error != nullptr) {
+      atomicCAS(error, kDevOk, kDevWaitTimeout);
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+__device__ __forceinline__ double two_to(int e) {
+  return e < -1022 ? 0.0 : __hiloint2double((min(e, 1023) + 1023) << 20, 0);
+}
+
+template <int KIND>
+struct WeightVector;  // 16 bytes of W as FP32 values
+template <>
+struct WeightVector<kWeightFp8> {
+  static constexpr int kCount = 16;
+  static __device__ __forceinline__ void unpack(const uint4& raw, float scale, float (&v)[16]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __half2_raw two = __nv_cvt_fp8x2_to_halfraw2(
+          static_cast<__nv_fp8x2_storage_t>(w[i >> 1] >> (16 * (i & 1))), __NV_E4M3);
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+      v[2 * i] = __fmul_rn(f.x, scale);
+      v[2 * i + 1] = __fmul_rn(f.y, scale);
+    }
+  }
+};
+template <>
+struct WeightVector<kWeightBf16> {
+  static constexpr int kCount = 8;
+  static __device__ __forceinline__ void unpack(const uint4& raw, float, float (&v)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+};
+template <>
+struct WeightVector<kWeightF32> {
+  static constexpr int kCount = 4;
+  static __device__ __forceinline__ void unpack(const uint4& raw, float, float (&v)[4]) {
+    v[0] = __uint_as_float(raw.x);
+    v[1] = __uint_as_float(raw.y);
+    v[2] = __uint_as_float(raw.z);
+    v[3] = __uint_as_float(raw.w);
+  }
+};
+
+constexpr int kFinishThreads = 256;
+
+// FP32 results from the doubles of exact_gemm_kernel: one thread per value.
+//
+// B, in units of 2^(ea + ew): K * 2^-52 for the digit products of level 7 and beyond (two pairs of
+// digits up to 128 at level 7, one at level 8: K * 2^-53 * 1.01); 2^-39 for every value of the two
+// rows that its digits do not hold exactly; and |r| * 2^-50 for the roundings of the doubles.
+template <int KIND>
+__global__ void __launch_bounds__(kFinishThreads)
+exact_finish_kernel(const double* __restrict__ partial, int splits, int rows, int N, int K,
+                    const float* __restrict__ in, float fp8_scale,
+                    const SliceRow* __restrict__ in_info, const void* __restrict__ weight,
+                    float weight_scale, const SliceRow* __restrict__ weight_info,
+                    const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
+  constexpr int V = WeightVector<KIND>::kCount;
+  __shared__ int open_count;
+  __shared__ int open_list[kFinishThreads];
+  __shared__ double warp_sum[kFinishThreads / 32];
+  if (threadIdx.x == 0) open_count = 0;
+  __syncthreads();
+  const int t = blockIdx.y;
+  const int n = blockIdx.x * kFinishThreads + threadIdx.x;
+  const size_t i = static_cast<size_t>(t) * N + n;
+  float result = 0.0f;
+  bool decided = true;
+  if (n < N) {
+    const size_t count = static_cast<size_t>(rows) * N;
+    double r = partial[i];
+#pragma unroll 4
+    for (int s = 1; s < splits; ++s) r += partial[i + s * count];
+    const SliceRow a = in_info[t], w = weight_info[n];
+    decided = a.exponent != kNoExponent && w.exponent != kNoExponent;
+    if (decided) {
+      const int e = a.exponent + w.exponent;
+      r *= two_to(e - (12 + 8 * (kLevels - 1)));
+      const double left_out = K + 8192.0 * (a.inexact + w.inexact);
+      const double bound = left_out * two_to(e - 52) + fabs(r) * 0x1p-50;
+      const float low = static_cast<float>(r - bound), high = static_cast<float>(r + bound);
+      decided = low == high;
+      result = static_cast<float>(r);
+    }
+  }
+  if (!decided) open_list[atomicAdd(&open_count, 1)] = n;
+  __syncthreads();
+  // the block forms the FP64 sum of one undecided value at a time, each thread a part of it
+  for (int o = 0; o < open_count; ++o) {
+    const float* x = in + static_cast<size_t>(t) * K;
+    const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
+                                                    static_cast<size_t>(open_list[o]) * K * (16 / V));
+    double sum = 0.0;
+    for (int q = threadIdx.x; q * V < K; q += kFinishThreads) {
+      float v[V];
+      WeightVector<KIND>::unpack(w[q], weight_scale, v);
+#pragma unroll
+      for (int j = 0; j < V; j += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + q * V + j);
+        const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          sum = fma(static_cast<double>(input_value(av[h], fp8_scale)),
+                    static_cast<double>(v[j + h]), sum);
+        }
+      }
+    }
+#pragma unroll
+    for (int stride = 16; stride > 0; stride >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, stride);
+    }
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (n == open_list[o]) {
+      double total = 0.0;
+#pragma unroll
+      for (int w8 = 0; w8 < kFinishThreads / 32; ++w8) total += warp_sum[w8];
+      result = static_cast<float>(total);
+    }
+    __syncthreads();
+  }
+  if (n < N) {
+    if (offset != nullptr) result = __fadd_rn(result, offset[n]);
+    if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
+    out[i] = result;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// a few token rows: W in its own format, FP64 sums
+// ---------------------------------------------------------------------------
+constexpr int kGemvThreads = 256;
+// xs[] of exact_gemv_kernel: 16 values and a gap, so that lanes reading their own 4, 8 or 16
+// consecutive values meet no bank conflict.
+__host__ __device__ constexpr int gemv_slot(int k) { return k + (k >> 4); }
+
+// One warp per weight row at a time; the ROWS token rows wait in shared memory as doubles, so that
+// they are widened once per block.  Bound by reading W at one row: shared_up of the checkpoint
+// layer (22 MB of FP8) 37 -> 15 us.
+template <int KIND, int ROWS>
+__global__ void __launch_bounds__(kGemvThreads)
+exact_gemv_kernel(const float* __restrict__ in, float fp8_scale, int N, int K,
+                  const void* __restrict__ weight, float weight_scale,
+                  const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
+  constexpr int V = WeightVector<KIND>::kCount;
+  constexpr int kWarps = kGemvThreads / 32;
+  extern __shared__ double xs[];
+  const int lane = threadIdx.x & 31;
+  const int padded = gemv_slot(K);
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+#pragma unroll 4
+    for (int k = threadIdx.x; k < K; k += kGemvThreads) {
+      xs[r * padded + gemv_slot(k)] =
+          static_cast<double>(input_value(in[static_cast<size_t>(r) * K + k], fp8_scale));
+    }
+  }
+  __syncthreads();
+  // two weight rows at a time: a token value read from shared memory serves both
+  const int pairs = (N + 1) / 2;
+  for (int p = blockIdx.x * kWarps + (threadIdx.x >> 5); p < pairs; p += gridDim.x * kWarps) {
+    const int n0 = 2 * p, n1 = min(n0 + 1, N - 1);
+    const size_t row_bytes = static_cast<size_t>(K) * (16 / V);
+    const uint4* w0 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
+                                                     n0 * row_bytes);
+    const uint4* w1 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
+                                                     n1 * row_bytes);
+    double acc[ROWS][2];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0.0;
+#pragma unroll 4
+    for (int q = lane; q * V < K; q += 32) {
+      float v0[V], v1[V];
+      WeightVector<KIND>::unpack(w0[q], weight_scale, v0);
+      WeightVector<KIND>::unpack(w1[q], weight_scale, v1);
+      const double* x = xs + gemv_slot(q * V);
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const double d0 = static_cast<double>(v0[j]), d1 = static_cast<double>(v1[j]);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const double a = x[r * padded + j];
+          acc[r][0] = fma(a, d0, acc[r][0]);
+          acc[r][1] = fma(a, d1, acc[r][1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        double v = acc[r][h];
+#pragma unroll
+        for (int stride = 16; stride > 0; stride >>= 1) {
+          v += __shfl_xor_sync(0xffffffffu, v, stride);
+        }
+        const int n = n0 + h;
+        if (lane == 0 && n < N) {
+          float result = static_cast<float>(v);
+          if (offset != nullptr) result = __fadd_rn(result, offset[n]);
+          if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
+          out[static_cast<size_t>(r) * N + n] = result;
+        }
+      }
+    }
+  }
+}
+
+// One block per weight row and ROWS token rows, for the short weights of a router's gate: every
+// thread widens its own part of both.
+template <int KIND, int ROWS>
+__global__ void __launch_bounds__(kGemvThreads)
+exact_gemv_block_kernel(const float* __restrict__ in, float fp8_scale, int rows, int N, int K,
+                        const void* __restrict__ weight, float weight_scale,
+                        const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
+  constexpr int V = WeightVector<KIND>::kCount;
+  __shared__ double warp_sum[ROWS][kGemvThreads / 32];
+  const int n = blockIdx.x;
+  const int row0 = blockIdx.y * ROWS;
+  const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
+                                                  static_cast<size_t>(n) * K * (16 / V));
+  double acc[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) acc[r] = 0.0;
+#pragma unroll 2
+  for (int q = threadIdx.x; q * V < K; q += kGemvThreads) {
+    float v[V];
+    WeightVector<KIND>::unpack(w[q], weight_scale, v);
+    double d[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) d[j] = static_cast<double>(v[j]);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const float* x = in + static_cast<size_t>(min(row0 + r, rows - 1)) * K + q * V;
+#pragma unroll
+      for (int j = 0; j < V; j += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + j);
+        const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          acc[r] = fma(static_cast<double>(input_value(av[h], fp8_scale)), d[j + h], acc[r]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+    for (int stride = 16; stride > 0; stride >>= 1) {
+      acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], stride);
+    }
+    if ((threadIdx.x & 31) == 0) warp_sum[r][threadIdx.x >> 5] = acc[r];
+  }
+  __syncthreads();
+  const int r = threadIdx.x;
+  if (r < ROWS && row0 + r < rows) {
+    double v = 0.0;
+#pragma unroll
+    for (int i = 0; i < kGemvThreads / 32; ++i) v += warp_sum[r][i];
+    float result = static_cast<float>(v);
+    if (offset != nullptr) result = __fadd_rn(result, offset[n]);
+    if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
+    out[static_cast<size_t>(row0 + r) * N + n] = result;
+  }
+}
+
+bool gemv_by_blocks(int N, int num_sms) {
+  return N <= 4 * num_sms;  // sixteen outputs a block would leave most SMs idle
+}
+
+template <int KIND, int ROWS>
+cudaError_t launch_gemv_rows(const float* in, float fp8_scale, int N, int K, const void* weight,
+                             float weight_scale, const float* offset, bool relu2, float* out,
+                             int num_sms, cudaStream_t stream) {
+  const int smem = ROWS * gemv_slot(K) * static_cast<int>(sizeof(double));
+  auto kernel = exact_gemv_kernel<KIND, ROWS>;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return err;
+  // no more blocks than are resident together: each widens the token rows for itself
+  const int resident = std::min(8, std::max(1, 220 * 1024 / (smem + 1024)));
+  const int per_block = 2 * (kGemvThreads / 32);
+  const int grid = std::min((N + per_block - 1) / per_block, num_sms * resident);
+  kernel<<<grid, kGemvThreads, smem, stream>>>(in, fp8_scale, N, K, weight, weight_scale, offset,
+                                               relu2, out);
+  return cudaGetLastError();
+}
+
+template <int KIND>
+cudaError_t launch_gemv_kind(const float* in, float fp8_scale, int rows, int N, int K,
+                             const void* weight, float weight_scale, const float* offset,
+                             bool relu2, float* out, int num_sms, cudaStream_t stream) {
+  if (gemv_by_blocks(N, num_sms)) {
+    auto run = [&](auto kernel, int per_block) {
+      kernel<<<dim3(N, (rows + per_block - 1) / per_block), kGemvThreads, 0, stream>>>(
+          in, fp8_scale, rows, N, K, weight, weight_scale, offset, relu2, out);
+    };
+    if (rows == 1) {
+      run(exact_gemv_block_kernel<KIND, 1>, 1);
+    } else if (rows == 2) {
+      run(exact_gemv_block_kernel<KIND, 2>, 2);
+    } else {
+      run(exact_gemv_block_kernel<KIND, 4>, 4);
+    }
+    return cudaGetLastError();
+  }
+  const int fit = kExactGemvMaxK / K;  // rows whose doubles fit shared memory
+  while (rows > 0) {
+    cudaError_t err;
+    int done;
+    if (rows >= 4 && fit >= 4) {
+      done = 4;
+      err = launch_gemv_rows<KIND, 4>(in, fp8_scale, N, K, weight, weight_scale, offset, relu2, out,
+                                      num_sms, stream);
+    } else if (rows >= 2 && fit >= 2) {
+      done = 2;
+      err = launch_gemv_rows<KIND, 2>(in, fp8_scale, N, K, weight, weight_scale, offset, relu2, out,
+                                      num_sms, stream);
+    } else {
+      done = 1;
+      err = launch_gemv_rows<KIND, 1>(in, fp8_scale, N, K, weight, weight_scale, offset, relu2, out,
+                                      num_sms, stream);
+    }
+    if (err != cudaSuccess) return err;
+    rows -= done;
+    in += static_cast<size_t>(done) * K;
+    out += static_cast<size_t>(done) * N;
+  }
+  return cudaSuccess;
+}
+
+}  // namespace
+
+bool exact_supported(int N, int K) {
+  // K: whole chunks, 32-bit level sums (six pairs of digits up to 128), the rows of a gemv
+  return N > 0 && K > 0 && K % kExactChunk == 0 && K <= kExactGemvMaxK && K <= 16384;
+}
+
+size_t slice_bytes(size_t rows, int K, int tile_rows) {
+  return (rows + tile_rows - 1) / tile_rows * tile_rows * K * kSlices;
+}
+
+int exact_weight_tile_rows() { return kExactRows; }
+
+cudaError_t launch_slice_weights(const void* weight, int kind, float scale, int N, int K,
+                                 int8_t* slices, SliceRow* info, cudaStream_t stream) {
+  if (kind == kWeightFp8) {
+    launch_slices<kWeightFp8>(weight, N, K, scale, kExactRows, slices, info, stream);
+  } else if (kind == kWeightBf16) {
+    launch_slices<kWeightBf16>(weight, N, K, scale, kExactRows, slices, info, stream);
+  } else {
+    launch_slices<kWeightF32>(weight, N, K, scale, kExactRows, slices, info, stream);
+  }
+  return cudaGetLastError();
+}
+
+// Token rows per tile: as many as the seven levels leave room for in TMEM (7 * 64 columns of 512),
+// fewer when there are fewer.
+int exact_tile_rows(int rows) { return rows >= 49 ? 64 : (rows + 15) / 16 * 16; }
+
+// The K range is shared by several CTAs while that still leaves an SM for each.
+int exact_splits(int rows, int N, int K, int num_sms) {
+  const int nt = exact_tile_rows(rows);
+  const int tiles = (N + kExactRows - 1) / kExactRows * ((rows + nt - 1) / nt);
+  return std::max(1, std::min(num_sms / tiles, K / kExactChunk));
+}
+
+cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows, float fp8_scale,
+                                const float* offset, bool relu2, const ExactWorkspace& space,
+                                float* out, int32_t* error, int num_sms, cudaStream_t stream) {
+  if (rows <= 0 || !exact_supported(w.N, w.K)) return cudaErrorInvalidValue;
+  const int nt = exact_tile_rows(rows);
+  launch_slices<-1>(in, rows, w.K, fp8_scale, nt, space.slices, space.info, stream);
+  const int row_tiles = (rows + nt - 1) / nt;
+  const int splits = exact_splits(rows, w.N, w.K, num_sms);
+  const int grid = (w.N + kExactRows - 1) / kExactRows * row_tiles * splits;
+  const int smem = kExactStages * (kExactABytes + kSlices * nt * kExactChunk) +
+                   (2 * kExactStages + 1) * 8 + 16 + 1024;
+  cudaError_t err = cudaFuncSetAttribute(exact_gemm_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return err;
+  exact_gemm_kernel<<<grid, kExactThreads, smem, stream>>>(w.slices, space.slices, rows, w.N, w.K,
+                                                           nt, row_tiles, splits, space.partial,
+                                                           error);
+  err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  const dim3 blocks((w.N + kFinishThreads - 1) / kFinishThreads, rows, 1);
+  auto run = [&](auto kernel) {
+    kernel<<<blocks, kFinishThreads, 0, stream>>>(space.partial, splits, rows, w.N, w.K, in,
+                                                  fp8_scale, space.info, w.weight, w.scale, w.info,
+                                                  offset, relu2, out);
+  };
+  if (w.kind == kWeightFp8) {
+    run(exact_finish_kernel<kWeightFp8>);
+  } else if (w.kind == kWeightBf16) {
+    run(exact_finish_kernel<kWeightBf16>);
+  } else {
+    run(exact_finish_kernel<kWeightF32>);
+  }
+  return cudaGetLastError();
+}
+
+// FP64 over the operands as they are, or integers over their slices?  The first reads W in its own
+// format, which counts for few rows: up to four are no slower on a large W (22 MB of FP8 against
+// 110 MB of slices for the checkpoint's shared_up).  A short W costs no more than widening its
+// values (15 a clock and SM), which up to 36 million products is less than the three launches of
+// the second take (64 rows of a 128 x 2688 gate: 20 us against 31 between events).
+bool exact_prefers_gemv(int rows, int N, int K, int num_sms) {
+  if (rows <= 4) return true;
+  return gemv_by_blocks(N, num_sms) && static_cast<long long>(rows) * N * K <= 36000000ll;
+}
+
+cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,
+                              const float* offset, bool relu2, float* out, int num_sms,
+                              cudaStream_t stream) {
+  if (rows <= 0 || !exact_supported(w.N, w.K)) return cudaErrorInvalidValue;
+  if (w.kind == kWeightFp8) {
+    return launch_gemv_kind<kWeightFp8>(in, fp8_scale, rows, w.N, w.K, w.weight, w.scale, offset,
+                                        relu2, out, num_sms, stream);
+  }
+  if (w.kind == kWeightBf16) {
+    return launch_gemv_kind<kWeightBf16>(in, fp8_scale, rows, w.N, w.K, w.weight, w.scale, offset,
+                                         relu2, out, num_sms, stream);
+  }
+  return launch_gemv_kind<kWeightF32>(in, fp8_scale, rows, w.N, w.K, w.weight, w.scale, offset,
+                                      relu2, out, num_sms, stream);
+}
+
+}  // namespace nmoe

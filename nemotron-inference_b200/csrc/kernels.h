@@ -205,6 +205,48 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        float tie_margin, int32_t* top_index, float* top_weight,
                                        int32_t* expert_counts, cudaStream_t stream);
 
+// --- correctly rounded linears (csrc/exact.cu) ---------------------------------
+// y[rows][N] = x[rows][K] x W[N][K]^T in FP32, each value the FP64 sum rounded once.
+enum WeightKind : int { kWeightF32 = 0, kWeightBf16 = 1, kWeightFp8 = 2 };
+// A row in fixed point: every value is below 2^exponent; `inexact` values have bits below the
+// last digit.
+struct SliceRow {
+  int32_t exponent;
+  int32_t inexact;
+};
+struct ExactWeight {
+  int N = 0, K = 0;
+  int kind = kWeightF32;           // how `weight` is stored; FP8 codes count times `scale`
+  const void* weight = nullptr;    // [N][K], 16-byte aligned
+  float scale = 1.0f;
+  const int8_t* slices = nullptr;  // slice_bytes(N, K, exact_weight_tile_rows()) bytes, 16-byte
+                                   // aligned, zero where no row is
+  const SliceRow* info = nullptr;  // [N]
+};
+constexpr int kExactGemvMaxK = 25 * 1024;  // values of K whose doubles fit shared memory
+bool exact_supported(int N, int K);
+size_t slice_bytes(size_t rows, int K, int tile_rows);
+int exact_weight_tile_rows();
+int exact_tile_rows(int rows);  // token rows per tile for a batch
+int exact_splits(int rows, int N, int K, int num_sms);
+cudaError_t launch_slice_weights(const void* weight, int kind, float scale, int N, int K,
+                                 int8_t* slices, SliceRow* info, cudaStream_t stream);
+struct ExactWorkspace {
+  int8_t* slices;   // slice_bytes(rows, K, exact_tile_rows(rows))
+  SliceRow* info;   // [rows]
+  double* partial;  // exact_splits() * rows * N
+};
+// `fp8_scale` != 0: every value of `in` takes the round trip of the scaled-FP8 family first.
+// `offset` (nullable [N]) is added to the rounded sum, `relu2` then squares what is positive.
+cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows, float fp8_scale,
+                                const float* offset, bool relu2, const ExactWorkspace& space,
+                                float* out, int32_t* error, int num_sms, cudaStream_t stream);
+bool exact_prefers_gemv(int rows, int N, int K, int num_sms);
+// The same for a handful of rows: reads W once per four rows, no slices.
+cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,
+                              const float* offset, bool relu2, float* out, int num_sms,
+                              cudaStream_t stream);
+
 // --- dense and scaled-FP8 linear families, latent-MoE data flow (csrc/dense.cu) -
 // The dense matmul itself is launch_router_logits: out[rows][experts] =
 // a[rows][hidden] x w[experts][hidden]^T, FP64 accumulation, FP32 result.

@@ -532,26 +532,57 @@ void upload_dense_fp32(const nmoe_dense_tensor& t, size_t count, const char* nam
   }
 }
 
-// A dense or scaled-FP8 linear resident in HBM as FP32 [out][in], the form the
-// reference's UploadedLinearOp / ScaledFp8LinearOp multiply with
-// (linear_op.cpp:274-303, scaled_fp8_linear.cu:121-139).
+// A weight of a correctly rounded linear with its slices.
+struct ExactOperand {
+  ExactWeight w;
+  DeviceBuffer slices, info;
+  void bind(const void* weight, int kind, float scale, int n, int k, cudaStream_t stream) {
+    w.N = n;
+    w.K = k;
+    w.kind = kind;
+    w.weight = weight;
+    w.scale = scale;
+    slices.allocate(slice_bytes(n, k, exact_weight_tile_rows()), true);
+    info.allocate(static_cast<size_t>(n) * sizeof(SliceRow));
+    NMOE_CUDA(launch_slice_weights(weight, kind, scale, n, k, slices.as<int8_t>(),
+                                   info.as<SliceRow>(), stream));
+    w.slices = slices.as<int8_t>();
+    w.info = info.as<SliceRow>();
+  }
+};
+
+// A dense or scaled-FP8 linear resident in HBM in the format it came in, with its fixed-point
+// slices; the values that count are FP32 [out][in], what the reference's UploadedLinearOp /
+// ScaledFp8LinearOp multiply with (linear_op.cpp:274-303, scaled_fp8_linear.cu:121-139).
+// Contractions too long for the slices keep the FP32 matrix itself.
 struct DenseLinear {
   bool present = false;
   bool fp8 = false;
+  bool exact = false;
   int out = 0, in = 0;
   float input_scale = 1.0f;
   DeviceBuffer weight;
+  ExactOperand operand;
 
   void upload(const nmoe_linear& linear, size_t out_rows, size_t in_cols, const char* name,
               cudaStream_t stream) {
     const std::string n(name);
     out = static_cast<int>(out_rows);
     in = static_cast<int>(in_cols);
+    exact = exact_supported(out, in);
     const size_t count = out_rows * in_cols;
     if (linear.family == NMOE_LINEAR_DENSE) {
-      nmoe_dense_tensor t = linear.weight;
+      const nmoe_dense_tensor& t = linear.weight;
       NMOE_REQUIRE(t.rows == out_rows && t.cols == in_cols, n + ": shape mismatch");
-      upload_dense_fp32(t, count, name, &weight, stream);
+      if (!exact || t.dtype == NMOE_F32) {
+        upload_dense_fp32(t, count, name, &weight, stream);
+        if (exact) operand.bind(weight.as<void>(), kWeightF32, 1.0f, out, in, stream);
+      } else {
+        NMOE_REQUIRE(t.data != nullptr && t.nbytes == count * 2, n + ": byte count");
+        weight.allocate(count * 2);
+        NMOE_CUDA(cudaMemcpyAsync(weight.as<void>(), t.data, count * 2, cudaMemcpyDefault, stream));
+        operand.bind(weight.as<void>(), kWeightBf16, 1.0f, out, in, stream);
+      }
     } else if (linear.family == NMOE_LINEAR_SCALED_FP8) {
       // DequantizeScaledFp8WeightToHostFp32 (scaled_fp8_linear.cu:121-139)
       NMOE_REQUIRE(linear.weight.data != nullptr && linear.weight.nbytes == count &&
@@ -559,22 +590,70 @@ struct DenseLinear {
                    n + ": FP8 weight bytes");
       NMOE_REQUIRE(linear.weight_scale > 0.0f && linear.weight_scale < 3.0e38f,
                    n + ": weight_scale must be finite and positive");
-      DeviceBuffer staging;
-      staging.allocate(count);
-      NMOE_CUDA(cudaMemcpyAsync(staging.as<void>(), linear.weight.data, count, cudaMemcpyDefault,
-                                stream));
-      weight.allocate(count * sizeof(float));
-      NMOE_CUDA(launch_fp8_weight_dequant(staging.as<uint8_t>(), count, linear.weight_scale,
-                                          weight.as<float>(), stream));
-      NMOE_CUDA(cudaStreamSynchronize(stream));
       fp8 = true;
       input_scale = linear.input_scale;
+      if (exact) {
+        weight.allocate(count);
+        NMOE_CUDA(cudaMemcpyAsync(weight.as<void>(), linear.weight.data, count, cudaMemcpyDefault,
+                                  stream));
+        operand.bind(weight.as<void>(), kWeightFp8, linear.weight_scale, out, in, stream);
+      } else {
+        DeviceBuffer staging;
+        staging.allocate(count);
+        NMOE_CUDA(cudaMemcpyAsync(staging.as<void>(), linear.weight.data, count, cudaMemcpyDefault,
+                                  stream));
+        weight.allocate(count * sizeof(float));
+        NMOE_CUDA(launch_fp8_weight_dequant(staging.as<uint8_t>(), count, linear.weight_scale,
+                                            weight.as<float>(), stream));
+        NMOE_CUDA(cudaStreamSynchronize(stream));
+      }
     } else {
       throw Failure{NMOE_ERR_INVALID_ARGUMENT, n + ": unknown linear family"};
     }
     present = true;
   }
 };
+
+// Workspace of the correctly rounded linears: sliced activation rows (up to `max_rows` at a time;
+// longer batches go through in turn) and the partial sums.
+struct ExactScratch {
+  int max_rows = 0;
+  DeviceBuffer slices, info, partial;
+  // `shapes`: (N, K) of every linear that will run
+  void allocate(size_t tokens, const std::vector<std::pair<int, int>>& shapes, int num_sms) {
+    max_rows = static_cast<int>(std::min<size_t>(tokens, 1024));
+    size_t most_k = 0, most_n = 0;
+    for (const auto& shape : shapes) {
+      most_n = std::max<size_t>(most_n, shape.first);
+      most_k = std::max<size_t>(most_k, shape.second);
+    }
+    if (shapes.empty()) return;
+    // (rows come in tiles of up to 64)
+    slices.allocate(slice_bytes(max_rows, static_cast<int>(most_k), 64));
+    info.allocate(max_rows * sizeof(SliceRow));
+    // a split contraction has at most one tile of 128 x 64 sums per SM
+    partial.allocate(std::max(max_rows * most_n, static_cast<size_t>(num_sms) * 128 * 64) *
+                     sizeof(double));
+  }
+};
+
+void run_exact(const ExactWeight& w, ExactScratch& scratch, const float* in, float fp8_scale,
+               int rows, const float* offset, bool relu2, float* out, int32_t* error, int num_sms,
+               cudaStream_t stream) {
+  if (fp8_scale != 0.0f) fp8_scale = clamp_scale_host(fp8_scale);  // scaled_fp8_linear.cu:27-33
+  if (exact_prefers_gemv(rows, w.N, w.K, num_sms)) {
+    NMOE_CUDA(launch_exact_gemv(w, in, fp8_scale, rows, offset, relu2, out, num_sms, stream));
+    return;
+  }
+  for (int first = 0; first < rows; first += scratch.max_rows) {
+    const int count = std::min(rows - first, scratch.max_rows);
+    const float* from = in + static_cast<size_t>(first) * w.K;
+    const ExactWorkspace space{scratch.slices.as<int8_t>(), scratch.info.as<SliceRow>(),
+                               scratch.partial.as<double>()};
+    NMOE_CUDA(launch_exact_linear(w, from, count, fp8_scale, offset, relu2, space,
+                                  out + static_cast<size_t>(first) * w.N, error, num_sms, stream));
+  }
+}
 
 }  // namespace
 }  // namespace nmoe
@@ -713,6 +792,9 @@ struct nmoe_layer {
   int decode_pairs_limit = 0;
 
   DeviceBuffer norm_weight, gate, bias, logit_offset;
+  ExactOperand gate_exact;  // the router's FP64 logits of small batches
+  bool has_gate_exact = false;
+  ExactScratch exact;
   bool has_logit_offset = false;
   // two-pass router (tensor-core logits + FP64 re-evaluation of near-ties)
   bool fast_router = false;
@@ -894,12 +976,20 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
     L->projected.allocate(T * H * sizeof(float));
     L->shared_rows.allocate(T * H * sizeof(float));
   }
-  if (L->fc1.fp8 || L->shared_up_dense.fp8 || L->shared_down_dense.fp8) {
+  if ((L->fc1.fp8 && !L->fc1.exact) || (L->shared_up_dense.fp8 && !L->shared_up_dense.exact) ||
+      (L->shared_down_dense.fp8 && !L->shared_down_dense.exact)) {
     L->fp8_tmp.allocate(T * static_cast<size_t>(std::max(H, S)) * sizeof(float));
   }
   if (L->shared_up_dense.present || L->shared_down_dense.present || L->unfused) {
     L->shared_raw.allocate(T * S * sizeof(float));
   }
+  std::vector<std::pair<int, int>> linears;
+  if (L->has_gate_exact) linears.emplace_back(E, H);
+  for (const DenseLinear* linear :
+       {&L->fc1, &L->fc2, &L->shared_up_dense, &L->shared_down_dense}) {
+    if (linear->present && linear->exact) linears.emplace_back(linear->out, linear->in);
+  }
+  L->exact.allocate(T, linears, device_sm_count());
   if (L->ep_world == 1) {
     L->parts.allocate(T * (K + 1) * static_cast<size_t>(std::max(H, Lr)) * sizeof(float));
   }
@@ -1053,13 +1143,21 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
     L->shared_down.upload(&w.shared_down, 1, H, S, false, "shared down_proj", stream);
   }
 
+  if (w.gate_weight.dtype == NMOE_BF16) {
+    L->gate_bf16.allocate(static_cast<size_t>(E) * H * 2);
+    NMOE_CUDA(cudaMemcpyAsync(L->gate_bf16.as<void>(), w.gate_weight.data,
+                              static_cast<size_t>(E) * H * 2, cudaMemcpyDefault, stream));
+  }
+  L->has_gate_exact = exact_supported(E, H);
+  if (L->has_gate_exact) {
+    const bool bf16 = w.gate_weight.dtype == NMOE_BF16;
+    L->gate_exact.bind(bf16 ? L->gate_bf16.as<void>() : L->gate.as<void>(),
+                       bf16 ? kWeightBf16 : kWeightF32, 1.0f, E, H, stream);
+  }
   // The tensor-core pass needs the gate exactly in bf16.
   L->fast_router = w.gate_weight.dtype == NMOE_BF16 && c.n_group == 1 && E % 32 == 0 &&
                    E <= 256 && H % 64 == 0 && std::getenv("NMOE_ROUTER_FP64_ONLY") == nullptr;
   if (L->fast_router) {
-    L->gate_bf16.allocate(static_cast<size_t>(E) * H * 2);
-    NMOE_CUDA(cudaMemcpyAsync(L->gate_bf16.as<void>(), w.gate_weight.data,
-                              static_cast<size_t>(E) * H * 2, cudaMemcpyDefault, stream));
     L->gate_map = make_bf16_map(L->gate_bf16.as<void>(), E, H, E);
     L->folded_router = std::getenv("NMOE_ROUTER_SPLIT_INPUT") == nullptr;
     if (L->folded_router) {
@@ -1077,9 +1175,14 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   NMOE_CUDA(cudaDeviceSynchronize());
 }
 
-// y = x W^T of a dense / scaled-FP8 linear, FP64 accumulation.
+// y = x W^T of a dense / scaled-FP8 linear, rounded once from the FP64 sum [, relu^2 of it].
 void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, int rows,
-                float* out_rows, cudaStream_t stream) {
+                float* out_rows, bool relu2, cudaStream_t stream) {
+  if (linear.exact) {
+    run_exact(linear.operand.w, L->exact, in_rows, linear.fp8 ? linear.input_scale : 0.0f, rows,
+              nullptr, relu2, out_rows, L->error.device.as<int32_t>(), L->num_sms, stream);
+    return;
+  }
   const float* source = in_rows;
   if (linear.fp8) {
     NMOE_CUDA(launch_fp8_round_trip(in_rows, static_cast<size_t>(rows) * linear.in,
@@ -1088,6 +1191,9 @@ void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, 
   }
   NMOE_CUDA(launch_router_logits(source, linear.weight.as<float>(), nullptr, rows, linear.out,
                                  linear.in, out_rows, stream));
+  if (relu2) {
+    NMOE_CUDA(launch_relu2(out_rows, static_cast<size_t>(rows) * linear.out, stream));
+  }
 }
 
 // RMSNorm + activation quantiser + router: fills normalized, y_*, logits,
@@ -1148,8 +1254,13 @@ void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dt
         L->router_tie_margin, L->top_index.as<int32_t>(), L->top_weight.as<float>(),
         L->counts.as<int32_t>(), stream));
   } else {
-    NMOE_CUDA(launch_router_logits(L->normalized.as<float>(), L->gate.as<float>(), offset, tokens,
-                                   E, H, L->logits.as<float>(), stream));
+    if (L->has_gate_exact) {
+      run_exact(L->gate_exact.w, L->exact, L->normalized.as<float>(), 0.0f, tokens, offset, false,
+                L->logits.as<float>(), error, L->num_sms, stream);
+    } else {
+      NMOE_CUDA(launch_router_logits(L->normalized.as<float>(), L->gate.as<float>(), offset, tokens,
+                                     E, H, L->logits.as<float>(), stream));
+    }
     L->mark(2, stream);
     NMOE_CUDA(launch_router_topk(L->logits.as<float>(), L->bias.as<float>(), tokens, E, K,
                                  c.n_group, c.topk_group, c.norm_topk_prob != 0,
@@ -1266,8 +1377,8 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
   // shared_up -> FP32 rows -> relu^2 in place (:956-964)
   float* raw = L->shared_raw.as<float>();
   if (L->shared_up_dense.present) {
-    run_linear(L, L->shared_up_dense, L->normalized.as<float>(), tokens, raw, stream);
-    NMOE_CUDA(launch_relu2(raw, static_cast<size_t>(tokens) * S, stream));
+    run_linear(L, L->shared_up_dense, L->normalized.as<float>(), tokens, raw, /*relu2=*/true,
+               stream);
   } else {
     run_down_gemm(L->shared_up,
                   shared_class == kClassPrefill || shared_class == kClassPair ? kClassDecodeWide
@@ -1281,7 +1392,7 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
     // only the latent data flow (FP32 rows of `hidden` per token) reaches this
     NMOE_REQUIRE(dest_mul == 1 && dest_add == 0 && out_kind == kRowF32,
                  "a dense shared_down writes FP32 token rows");
-    run_linear(L, L->shared_down_dense, raw, tokens, static_cast<float*>(out_rows), stream);
+    run_linear(L, L->shared_down_dense, raw, tokens, static_cast<float*>(out_rows), false, stream);
     (void)H;
     return;
   }
@@ -1334,7 +1445,8 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   if (L->latent_mode) {
     // latent = fc1_latent(normalized) (:809-813); every routed expert's up_proj packs
     // the same latent row (:913 -> nvfp4_packing.cpp:90)
-    run_linear(L, L->fc1, L->normalized.as<float>(), tokens, L->latent_rows.as<float>(), stream);
+    run_linear(L, L->fc1, L->normalized.as<float>(), tokens, L->latent_rows.as<float>(), false,
+               stream);
     NMOE_CUDA(launch_norm_quant(L->latent_rows.as<float>(), false, tokens, Lr, nullptr, 0.0f,
                                 nullptr, L->lat_packed.as<uint8_t>(),
                                 L->lat_sf_row_major.as<uint8_t>(), nullptr, 0,
@@ -1354,7 +1466,8 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     // residual (:1064-1069)
     NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
                                stream));
-    run_linear(L, L->fc2, L->routed_latent.as<float>(), tokens, L->projected.as<float>(), stream);
+    run_linear(L, L->fc2, L->routed_latent.as<float>(), tokens, L->projected.as<float>(), false,
+               stream);
     NMOE_CUDA(launch_mixer(input, in_dtype == NMOE_BF16, L->projected.as<float>(),
                            L->shared_rows.as<float>(), tokens, H, output, out_dtype == NMOE_BF16,
                            stream));
