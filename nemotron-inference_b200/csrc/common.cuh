@@ -101,14 +101,23 @@ __device__ __forceinline__ float div_by_reciprocal(float x, float d, float r) {
   return __fmaf_rn(e, r, q);
 }
 
+// Scale of a block before its rounding to E4M3 (nvfp4_packing.cpp:130-139): amax / (6 * ts),
+// given `divisor` = RN(6 * ts) and `reciprocal` = RN(1 / divisor).  Quotients too small for the
+// residual to be exact are below the smallest scale and clamped.
+__device__ __forceinline__ float block_scale(float block_max, float divisor, float reciprocal) {
+  if (!(block_max > 0.0f)) return 1.0f;
+  const bool exact = (__float_as_uint(divisor) & 0x007fffffu) != 0x007fffffu && block_max < 1.0e37f;
+  return clamp_scale(exact ? div_by_reciprocal(block_max, divisor, reciprocal)
+                           : __fdiv_rn(block_max, divisor));
+}
+
 // The fused quantiser of the up-projection epilogue: 16 non-negative values
 // whose maximum is `amax`, per-row tensor scale 1 (nvfp4_packing.cpp:119-153
 // with tensor_scale == 1.0).  Bit-identical to quantize_block16(v, 1.0f, ..).
 __device__ __forceinline__ uint32_t quantize_block16_unit_scale(const float (&v)[16], float amax,
                                                                 uint32_t& lo_word,
                                                                 uint32_t& hi_word) {
-  float bs = 1.0f;
-  if (amax > 0.0f) bs = clamp_scale(__fdiv_rn(amax, kFp4Max));
+  const float bs = block_scale(amax, kFp4Max, 1.0f / kFp4Max);
   const uint32_t scale_byte = encode_e4m3(bs);
   uint32_t w[2] = {0u, 0u};
   if ((__float_as_uint(bs) & 0x007fffffu) != 0x007fffffu) {
@@ -218,6 +227,60 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity) {
   return true;
 }
 
+// The same operations by shared-memory address, for loops whose every instruction counts: a role
+// of one thread runs a K block's bookkeeping as one dependent chain.
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
+  const long long start = clock64();
+  while (!mbar_try_wait_at(bar, parity)) {
+    if (clock64() - start > (1ll << 31)) return false;
+  }
+  return true;
+}
+
+__device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity) {
+  return mbar_try_wait_at(bar, parity) || mbar_wait_slow(bar, parity);
+}
+
+__device__ __forceinline__ void mbar_arrive_expect_tx_at(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+
+__device__ __forceinline__ void tma_load_2d_at(uint32_t smem_dst, const CUtensorMap* map, int x,
+                                               int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void bulk_load_at(uint32_t smem_dst, const void* gmem_src,
+                                             uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+      ::"r"(smem_dst), "l"(gmem_src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void tcgen05_commit_at(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                   bar)
+               : "memory");
+}
+
 // 2-D tiled TMA load (no multicast) into this CTA's shared memory.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y,
                                             uint64_t* bar) {
@@ -285,6 +348,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
          (static_cast<uint64_t>(lbo_bytes >> 4) << 16) |
          (static_cast<uint64_t>(sbo_bytes >> 4) << 32) | (1ull << 46) |
          (static_cast<uint64_t>(swizzle) << 61);
+}
+
+// The same descriptor for another address: `offset` bytes (a multiple of 16) further on.
+__device__ __forceinline__ uint64_t advance_smem_desc(uint64_t desc, uint32_t offset) {
+  const uint32_t low = static_cast<uint32_t>(desc) + (offset >> 4);
+  return (desc & 0xffffffff00000000ull) | low;
 }
 
 // Copy 32 rows x 16 bytes of scale factors from shared memory into 4 TMEM
@@ -437,6 +506,45 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       " [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
       : "memory");
+}
+
+__device__ __forceinline__ void tma_load_2d_pair_at(uint32_t smem_dst, const CUtensorMap* map, int x,
+                                                    int y, uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
+      : "memory");
+}
+
+// Arrive on an mbarrier by its shared::cluster address (this CTA's or the partner's).
+__device__ __forceinline__ void mbar_arrive_cluster_at(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar)
+               : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try_wait_cluster_at(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+static __device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parity) {
+  const long long start = clock64();
+  while (!mbar_try_wait_cluster_at(bar, parity)) {
+    if (clock64() - start > (1ll << 31)) return false;
+  }
+  return true;
+}
+
+__device__ __forceinline__ bool mbar_wait_cluster_at(uint32_t bar, uint32_t parity) {
+  return mbar_try_wait_cluster_at(bar, parity) || mbar_wait_cluster_slow(bar, parity);
 }
 
 // The shared::cluster address of `local` (an address in this CTA's shared memory) in

@@ -1,0 +1,569 @@
+// Expert FFNs of batches that are bound by reading the weights: up and down projections of the
+// routed experts and of the shared expert as the tiles of ONE persistent launch.
+//
+// As four launches (up and down, routed and shared) these sizes paid for every launch's start and
+// for every launch's last wave with idle HBM: 64 tokens took 72 + 75 us of routed GEMMs for 670 MB.
+// Here every CTA walks one list of tiles -- shared up, routed up, shared down, routed down -- and
+// its loads never stop in between: a down tile needs the quantised hidden rows of its row tile
+// only for its A operand, so its weights are on their way before those rows are complete.  A row
+// tile's completed up tiles are counted in global memory; the producer of a down tile waits for the
+// count (bounded, like every wait here).  All up tiles precede all down tiles in the list and every
+// CTA of the grid is resident (one per SM), so the wait ends.
+//
+// Tiles are 128 weight rows (B, BN = 128) of one row tile of up to 128 activation rows (A); the
+// activation box is 8 to 128 rows high, by the rows the tile holds, and the last weight tile of
+// a matrix loads the rows that exist.  At 148 SMs and the measured copy rate a K block's 18 KB of
+// weights take 800 cycles to arrive.  Roles of a single thread cost about as much when they wait
+// twice a K block and build their descriptors from scratch, so the loops here wait once and advance
+// descriptors (64 tokens, routed up and down 131 -> 120 us).
+// Measured, whole pass of the benchmark layer: 64 tokens 196 -> 164 us, 256 tokens 205 -> 178,
+// 1003 tokens 240 -> 229.
+//
+// Warp roles as in grouped_gemm_kernel (csrc/gemm.cu): warps 0 and 12-14 load, warp 1 issues MMAs,
+// warps 2-9 run epilogues, warps 10-11 copy block scales to TMEM; warp 15 hands
+// finished tiles on.
+#include <algorithm>
+
+#include "common.cuh"
+#include "gemm_common.cuh"
+#include "kernels.h"
+
+namespace nmoe {
+namespace {
+
+constexpr int kBN = 128;
+constexpr int kMaxStages = 8;
+constexpr int kScaleWarp = 2 + kEpilogueWarps;
+constexpr int kScaleWarps = 2;
+// One thread needs about 530 cycles for a stage's waits and bookkeeping and 90 for each of its four
+// copies (measured on a ring of bulk copies that does nothing else), more than a K block's 800, so
+// four threads take turns: 64 tokens, routed up and
+// down 137 -> 131 us.
+constexpr int kProducers = 4;
+constexpr int kSignalWarp = 1 + kEpilogueWarps + kScaleWarps + kProducers;
+constexpr int kThreads = (kSignalWarp + 1) * 32;
+constexpr int kBBytes = kBN * 128;
+constexpr int kSfaBytes = 2048;
+constexpr int kSfbBytes = 2048;     // four groups of 32 weight rows x four MMAs x 16 bytes
+constexpr int kSfBufCols = 32;      // TMEM columns of one K block's scales: 16 for A, 16 for B
+constexpr int kSfCol = 2 * kBN;     // behind the two accumulators
+constexpr int kTmemCols = 512;
+constexpr int kBarBytes = ((3 * kMaxStages + 6) * 8 + 16 + 15) / 16 * 16;
+static_assert(kProducers <= 6, "a producer advances less than a ring at a time");
+static_assert(kSfCol + kMaxStages * kSfBufCols <= kTmemCols, "TMEM budget");
+
+// Tiles of up to kFewRows rows hand their accumulator over through shared memory: a thread per row
+// would leave most lanes of the two warps that can read those rows idle and the others with four
+// chunks in turn.
+constexpr int kFewRows = 16;
+constexpr int kFewStride = kBN / 2 + 4;  // floats per row of one warp's half of the columns
+constexpr int kFewRowsBytes = 2 * kFewRows * kFewStride * 4;
+
+// The room for activation rows in a stage is no larger than the launch's tiles (32, 64 or 128 rows).
+constexpr int stage_bytes(int tile_rows) {
+  return tile_rows * 128 + kBBytes + kSfaBytes + kSfbBytes;
+}
+constexpr int stages_for(int tile_rows) { return tile_rows <= 32 ? 8 : tile_rows <= 64 ? 7 : 6; }
+constexpr int smem_bytes(int tile_rows) {
+  return stages_for(tile_rows) * stage_bytes(tile_rows) + kBarBytes + kFewRowsBytes + 1024;
+}
+static_assert(smem_bytes(32) <= 232448 && smem_bytes(64) <= 232448 && smem_bytes(128) <= 232448,
+              "shared memory budget");
+// The MMA always reads 128 A rows: behind a stage of fewer rows it reads what follows (those output
+// rows are never stored), which must lie inside the allocation.
+static_assert(stages_for(32) * kBBytes >= 128 * 128, "A over-read stays inside shared memory");
+
+// Where a tile of the list lies.
+struct Tile {
+  int phase;
+  int row0;    // first row of its 128-row slot
+  int rows;    // valid rows in it
+  int expert;
+  int nt;      // weight tile
+};
+
+struct TileList {
+  int first[kStreamPhases + 1];  // first tile of each phase, then the end
+  __device__ __forceinline__ void load(const StreamArgs& args) {
+    int running = 0;
+#pragma unroll
+    for (int p = 0; p < kStreamPhases; ++p) {
+      first[p] = running;
+      if (p < args.phases) {
+        const GemmArgs& g = args.phase[p].gemm;
+        const int row_tiles =
+            g.row_tiles != nullptr ? *g.num_row_tiles : (g.dense_rows + 127) / 128;
+        running += row_tiles * g.n_tiles;
+      }
+    }
+    first[kStreamPhases] = running;
+  }
+  __device__ __forceinline__ int total() const { return first[kStreamPhases]; }
+  __device__ __forceinline__ Tile locate(const StreamArgs& args, int t) const {
+    Tile tile;
+    tile.phase = 0;
+    int base = 0;
+#pragma unroll
+    for (int p = 1; p < kStreamPhases; ++p) {
+      if (t >= first[p] && p < args.phases) {
+        tile.phase = p;
+        base = first[p];
+      }
+    }
+    const GemmArgs& g = args.phase[tile.phase].gemm;
+    const int index = t - base;
+    const int rt = index / g.n_tiles;
+    tile.nt = index - rt * g.n_tiles;
+    if (g.row_tiles != nullptr) {
+      const RowTile row_tile = g.row_tiles[rt];
+      tile.row0 = row_tile.row0;
+      tile.rows = row_tile.rows;
+      tile.expert = row_tile.expert;
+    } else {
+      tile.row0 = rt * 128;
+      tile.rows = min(128, g.dense_rows - tile.row0);
+      tile.expert = 0;
+    }
+    return tile;
+  }
+};
+
+__device__ __forceinline__ int load_acquire(const int32_t* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void add_release(int32_t* p, int v) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Orders generic accesses (other SMs' stores, once they have been acquired) before those of the async
+// proxy (bulk and tensor copies).
+__device__ __forceinline__ void fence_proxy_async() {
+  asm volatile("fence.proxy.async;" ::: "memory");
+}
+
+// Waits (about a second at most) until *count >= target.
+__device__ __forceinline__ bool wait_count(const int32_t* count, int target) {
+  if (load_acquire(count) >= target) return true;
+  const long long start = clock64();
+  while (load_acquire(count) < target) {
+    if (clock64() - start > (1ll << 31)) return false;
+  }
+  return true;
+}
+
+template <int PART>
+__device__ __forceinline__ void issue_scale_copies(uint32_t sf_tmem, uint64_t sfa_desc,
+                                                   uint64_t sfb_desc) {
+#pragma unroll
+  for (int c = PART; c < 4; c += kScaleWarps) {
+    tcgen05_cp_32x128b_warpx4(sf_tmem + 4 * c, advance_smem_desc(sfa_desc, c * 512));
+    tcgen05_cp_32x128b_warpx4(sf_tmem + 16 + 4 * c, advance_smem_desc(sfb_desc, c * 512));
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+expert_stream_kernel(const __grid_constant__ StreamArgs args) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
+                                             ~static_cast<uintptr_t>(1023u));
+  uint8_t* sA = smem;
+  const int stages = stages_for(args.tile_rows);
+  const int a_room = args.tile_rows * 128;
+  uint8_t* sB = sA + stages * a_room;
+  uint8_t* sSFA = sB + stages * kBBytes;
+  uint8_t* sSFB = sSFA + stages * kSfaBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sSFB + stages * kSfbBytes);
+  uint64_t* empty_bar = full_bar + kMaxStages;
+  uint64_t* tmem_full_bar = empty_bar + kMaxStages;
+  uint64_t* tmem_empty_bar = tmem_full_bar + 2;
+  uint64_t* sf_ready_bar = tmem_empty_bar + 2;
+  uint64_t* stored_bar = sf_ready_bar + kMaxStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stored_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int unit = static_cast<int>(blockIdx.x);
+  const int units = static_cast<int>(gridDim.x);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+      mbar_init(&sf_ready_bar[s], kScaleWarps);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&tmem_full_bar[a], 1);
+      mbar_init(&tmem_empty_bar[a], 1);
+      mbar_init(&stored_bar[a], kEpilogueWarps);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  float* few_rows = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(full_bar) + kBarBytes);
+  const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
+  const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+  const uint32_t sf_ready0 = smem_u32(sf_ready_bar);
+
+  TileList list;
+  list.load(args);
+  const int total_tiles = list.total();
+
+  if (warp == kSignalWarp) {
+    // ---------------------------------------------------------------- signals
+    // Once the epilogue warps have stored a tile: give its accumulator back, and count the tile
+    // for the down projection.  Making the stores visible first takes some 1500 cycles, which here
+    // nobody waits for.
+    if (lane == 0) {
+      int local = 0;
+      for (int t = unit; t < total_tiles; t += units, ++local) {
+        const Tile tile = list.locate(args, t);
+        const StreamPhase& ph = args.phase[tile.phase];
+        const int acc = local & 1;
+        if (!mbar_wait(&stored_bar[acc], (local >> 1) & 1u)) {
+          report_timeout(args.error, abort_flag);
+          break;
+        }
+        mbar_arrive(&tmem_empty_bar[acc]);
+        if (ph.mode == kGemmUp && ph.ready != nullptr) {
+          __threadfence();
+          add_release(ph.ready + (tile.row0 >> 7), 1);
+        }
+      }
+    }
+  } else if (warp == 0 || warp >= kScaleWarp + kScaleWarps) {
+    // ------------------------------------------------------------- producers
+    // Producer p loads the K blocks p, p + kProducers, ... of the CTA's sequence.
+    if (lane == 0) {
+      const int producer = warp == 0 ? 0 : warp - (kScaleWarp + kScaleWarps) + 1;
+      int stage = producer;
+      uint32_t phase = 0;
+      auto advance = [&](int& at, uint32_t& at_phase) {
+        at += kProducers;
+        if (at >= stages) {
+          at -= stages;
+          at_phase ^= 1u;
+        }
+      };
+      int kb = producer;  // K block of the current tile this producer loads next
+      bool ok = true;
+      for (int t = unit; t < total_tiles && ok; t += units) {
+        const Tile tile = list.locate(args, t);
+        const StreamPhase& ph = args.phase[tile.phase];
+        const GemmArgs& g = ph.gemm;
+        const int k_blocks = g.k_blocks;
+        const int box = tile.rows <= 8 ? 0 : 29 - __clz(tile.rows - 1);  // 8 << box >= rows
+        const uint32_t a_bytes = 8u * 128u << box;
+        const int b_row = tile.nt * kBN;
+        const uint32_t b_bytes = static_cast<uint32_t>(min(kBN, g.N - b_row)) * 128u;
+        const uint8_t* sfa_src =
+            g.sfa + static_cast<size_t>(tile.row0 >> 7) * k_blocks * kSfaBytes;
+        const uint8_t* sfb_src =
+            g.sfb + (static_cast<size_t>(tile.expert) * g.n_tiles + tile.nt) * k_blocks * kSfbBytes;
+        const uint8_t* b_src =
+            g.b_full + (static_cast<size_t>(tile.expert) * g.kb_full * g.N + b_row) * 128;
+        auto load_weights = [&](int block, int at, uint32_t at_phase) {
+          if (!mbar_wait_at(empty0 + at * 8, at_phase ^ 1u)) return false;
+          const uint32_t bar = full0 + at * 8;
+          const bool full_block = block < g.kb_full;
+          mbar_arrive_expect_tx_at(bar, a_bytes + (full_block ? b_bytes : kBBytes) + kSfaBytes +
+                                            kSfbBytes);
+          if (full_block) {
+            // one contiguous, pre-swizzled panel slice: a single bulk copy
+            bulk_load_at(b0 + at * kBBytes, b_src + static_cast<size_t>(block) * g.N * 128, b_bytes,
+                         bar);
+          } else {
+            tma_load_2d_at(b0 + at * kBBytes, &ph.b_tail, 0, tile.expert * g.N + b_row, bar);
+          }
+          bulk_load_at(sfb0 + at * kSfbBytes, sfb_src + block * kSfbBytes, kSfbBytes, bar);
+          return true;
+        };
+        auto load_rows = [&](int block, int at) {
+          const uint32_t bar = full0 + at * 8;
+          tma_load_2d_at(a0 + at * a_room, &ph.a[box], block * 128, tile.row0, bar);
+          bulk_load_at(sfa0 + at * kSfaBytes, sfa_src + block * kSfaBytes, kSfaBytes, bar);
+        };
+        if (ph.wait_target > 0 && kb < k_blocks) {
+          const int32_t* count = ph.ready + (tile.row0 >> 7);
+          int at = stage;
+          uint32_t at_phase = phase;
+          ok = load_weights(kb, at, at_phase);
+          advance(at, at_phase);
+          int loaded = kb + kProducers;
+          if (ok && load_acquire(count) < ph.wait_target) {
+            // rows still being written: the weights of the ring's other K blocks go out meanwhile
+            const int ahead = min(stages, k_blocks);
+            for (; loaded < ahead && ok; loaded += kProducers) {
+              ok = load_weights(loaded, at, at_phase);
+              advance(at, at_phase);
+            }
+            ok = ok && wait_count(count, ph.wait_target);
+          }
+          fence_proxy_async();
+          for (; kb < loaded && ok; kb += kProducers) {
+            load_rows(kb, stage);
+            advance(stage, phase);
+          }
+        }
+        for (; kb < k_blocks && ok; kb += kProducers) {
+          ok = load_weights(kb, stage, phase);
+          if (ok) load_rows(kb, stage);
+          advance(stage, phase);
+        }
+        kb -= k_blocks;
+        if (!ok) report_timeout(args.error, abort_flag);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_nvf4(kBN);
+      const uint64_t a_desc0 = make_smem_desc(a0, 0, 1024, 2);
+      const uint64_t b_desc0 = make_smem_desc(b0, 0, 1024, 2);
+      int stage = 0;
+      uint32_t phase = 0;
+      int local = 0;
+      bool ok = true;
+      for (int t = unit; t < total_tiles && ok; t += units, ++local) {
+        const GemmArgs& g = args.phase[list.locate(args, t).phase].gemm;
+        const int k_blocks = g.k_blocks, last_mmas = g.K / 64 - 4 * (k_blocks - 1);
+        const int acc = local & 1;
+        const uint32_t acc_phase = (local >> 1) & 1u;
+        if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
+          report_timeout(args.error, abort_flag);
+          break;
+        }
+        tcgen05_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * kBN;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          // this block's scales are in TMEM, and its operands had landed before they were copied
+          if (!mbar_wait_at(sf_ready0 + stage * 8, phase)) {
+            report_timeout(args.error, abort_flag);
+            ok = false;
+            break;
+          }
+          tcgen05_fence_after();
+          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * a_room);
+          const uint64_t b_desc = advance_smem_desc(b_desc0, stage * kBBytes);
+          const uint32_t sf_tmem = tmem_base + kSfCol + stage * kSfBufCols;
+          if (kb + 1 < k_blocks || last_mmas == 4) {
+#pragma unroll
+            for (int kt = 0; kt < 4; ++kt) {
+              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                               advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
+                               sf_tmem + 16 + 4 * kt, kt != 0 ? 1u : kb != 0 ? 1u : 0u);
+            }
+          } else {
+            for (int kt = 0; kt < last_mmas; ++kt) {
+              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                               advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
+                               sf_tmem + 16 + 4 * kt, (kb | kt) != 0 ? 1u : 0u);
+            }
+          }
+          tcgen05_commit_at(empty0 + stage * 8);
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+        if (ok) tcgen05_commit(&tmem_full_bar[acc]);
+      }
+    }
+  } else if (warp >= kScaleWarp) {  // (the producers behind them are taken)
+    // ------------------------------------------------------- block-scale copiers
+    // Every stage has TMEM columns of its own: once its operands have landed, the MMAs that read
+    // those columns before are known to be done (the producer waited for them).
+    if (lane == 0) {
+      const int part = warp - kScaleWarp;
+      const uint64_t sfa_desc0 = make_smem_desc(sfa0, 0, 128, 0);
+      const uint64_t sfb_desc0 = make_smem_desc(sfb0, 0, 128, 0);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = unit; t < total_tiles && ok; t += units) {
+        const GemmArgs& g = args.phase[list.locate(args, t).phase].gemm;
+        const int k_blocks = g.k_blocks, last_mmas = g.K / 64 - 4 * (k_blocks - 1);
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait_at(full0 + stage * 8, phase)) {
+            report_timeout(args.error, abort_flag);
+            ok = false;
+            break;
+          }
+          tcgen05_fence_after();
+          const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * kSfaBytes);
+          const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * kSfbBytes);
+          const uint32_t sf_tmem = tmem_base + kSfCol + stage * kSfBufCols;
+          if (kb + 1 < k_blocks || last_mmas == 4) {
+            static_assert(kScaleWarps == 2, "one branch per copier");
+            if (part == 0) {
+              issue_scale_copies<0>(sf_tmem, sfa_desc, sfb_desc);
+            } else {
+              issue_scale_copies<1>(sf_tmem, sfa_desc, sfb_desc);
+            }
+          } else {
+            for (int c = part; c < last_mmas; c += kScaleWarps) {
+              tcgen05_cp_32x128b_warpx4(sf_tmem + 4 * c, advance_smem_desc(sfa_desc, c * 512));
+              tcgen05_cp_32x128b_warpx4(sf_tmem + 16 + 4 * c, advance_smem_desc(sfb_desc, c * 512));
+            }
+          }
+          tcgen05_commit_at(sf_ready0 + stage * 8);
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+    }
+  } else {
+    // -------------------------------------------------------------- epilogue
+    const int quarter = warp & 3;           // TMEM lanes a warp may read: 32 * (warp % 4)
+    const int half = (warp - 2) >> 2;       // which half of the tile's columns
+    const int r = quarter * 32 + lane;      // row inside the tile == TMEM lane
+    constexpr int kHalfChunks = kBN / 16 / 2;
+    int local = 0;
+    for (int t = unit; t < total_tiles; t += units, ++local) {
+      const int acc = local & 1;
+      const uint32_t acc_phase = (local >> 1) & 1u;
+      const Tile tile = list.locate(args, t);
+      const StreamPhase& ph = args.phase[tile.phase];
+      const GemmArgs& g = ph.gemm;
+      const bool row_valid = r < tile.rows;
+      const int grow = tile.row0 + r;
+      float scale = g.w_tensor_scale[tile.expert];
+      if (g.a_tensor_scale != nullptr && row_valid) scale *= g.a_tensor_scale[grow];
+      unsigned long long dest = 0;
+      float wt = 1.0f;
+      if (ph.mode == kGemmDown && row_valid) {
+        dest = output_row_address(g, grow);
+        if (g.row_weight != nullptr) wt = g.row_weight[grow];
+      }
+      if (!mbar_wait(&tmem_full_bar[acc], acc_phase)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      const int n0 = tile.nt * kBN;
+      const uint32_t t_addr =
+          tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kBN;
+      if (tile.rows <= kFewRows) {
+        if (quarter == 0) {
+          tcgen05_fence_after();
+          const int columns = min(kBN / 2, g.N - n0 - half * (kBN / 2));  // may be none
+          float* few = few_rows + half * (kFewRows * kFewStride);
+#pragma unroll 1
+          for (int c = 0; c < columns; c += 16) {
+            float v[16];
+            tmem_ld_x16(t_addr + half * (kBN / 2) + c, v);
+            if (row_valid) {
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                *reinterpret_cast<float4*>(few + r * kFewStride + c + i) =
+                    make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+              }
+            }
+          }
+          tcgen05_fence_before();
+          __syncwarp();
+          // one 16-column chunk of one row per lane and round, four chunks to a row
+#pragma unroll 1
+          for (int first = 0; first < tile.rows * 4; first += 32) {
+            const int from = (first + lane) >> 2, chunk = lane & 3;
+            const float row_scale = __shfl_sync(0xffffffffu, scale, from & 31);
+            const float row_wt = __shfl_sync(0xffffffffu, wt, from & 31);
+            const unsigned long long row_dest = __shfl_sync(0xffffffffu, dest, from & 31);
+            const int n = n0 + half * (kBN / 2) + chunk * 16;
+            if (from >= tile.rows || chunk * 16 >= columns) continue;
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+              const float4 four = *reinterpret_cast<const float4*>(
+                  few + from * kFewStride + chunk * 16 + i);
+              v[i] = four.x;
+              v[i + 1] = four.y;
+              v[i + 2] = four.z;
+              v[i + 3] = four.w;
+            }
+            if (ph.mode == kGemmUp) {
+              report_range(g, quantise_chunk(g, v, n, tile.row0 + from, row_scale, true));
+            } else if (row_dest != 0) {
+              store_chunk(g, v, n, row_dest, row_scale, row_wt);
+            }
+          }
+        }
+      } else if (quarter * 32 < tile.rows) {  // (else none of the warp's rows exist)
+        tcgen05_fence_after();
+        if (ph.mode == kGemmUp) {
+          epilogue_quantise<2>(g, t_addr, n0, half * kHalfChunks, (half + 1) * kHalfChunks, grow,
+                               row_valid, scale);
+        } else {
+          epilogue_rows_direct<2>(g, t_addr, n0, half * kHalfChunks, (half + 1) * kHalfChunks, dest,
+                                  scale, wt);
+        }
+        tcgen05_fence_before();
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&stored_bar[acc]);
+    }
+  }
+
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  } else if (warp == 0 && args.ready_count > 0) {
+    // the last CTA leaves the counts at zero for the next launch
+    int ticket = 0;
+    if (lane == 0) {
+      __threadfence();
+      ticket = atomicAdd(args.finished, 1);
+    }
+    ticket = __shfl_sync(0xffffffffu, ticket, 0);
+    if (ticket == units - 1) {
+      for (int i = lane; i < args.ready_count; i += 32) args.ready[i] = 0;
+      if (lane == 0) *args.finished = 0;
+    }
+  }
+}
+
+}  // namespace
+
+GemmVariantInfo stream_variant_info() {
+  return GemmVariantInfo{kBN, 128, 4, kSfbBytes, smem_bytes(128), kBN};
+}
+
+cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, cudaStream_t stream) {
+  if (args.phases < 1 || args.phases > kStreamPhases || num_sms < 1 ||
+      (args.tile_rows != 32 && args.tile_rows != 64 && args.tile_rows != 128)) {
+    return cudaErrorInvalidValue;
+  }
+  cudaError_t err = cudaFuncSetAttribute(expert_stream_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem_bytes(args.tile_rows));
+  if (err != cudaSuccess) return err;
+  // one persistent CTA per SM, fewer when the tiles are known to be fewer
+  int grid = num_sms;
+  int dense_tiles = 0;
+  bool grouped = false;
+  for (int p = 0; p < args.phases; ++p) {
+    const GemmArgs& g = args.phase[p].gemm;
+    grouped = grouped || g.row_tiles != nullptr;
+    dense_tiles += (g.dense_rows + 127) / 128 * g.n_tiles;
+  }
+  if (!grouped) grid = std::max(1, std::min(grid, dense_tiles));
+  expert_stream_kernel<<<grid, kThreads, smem_bytes(args.tile_rows), stream>>>(args);
+  return cudaGetLastError();
+}
+
+}  // namespace nmoe

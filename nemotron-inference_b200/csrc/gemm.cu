@@ -30,20 +30,18 @@
 #include <algorithm>
 #include <cstdlib>
 
-#include <cuda_fp16.h>
-
 #include "common.cuh"
+#include "gemm_common.cuh"
 #include "kernels.h"
 
 namespace nmoe {
 namespace {
 
-constexpr int kEpilogueWarps = 8;
 constexpr int kScaleWarp = 2 + kEpilogueWarps;  // issues the block-scale copies into TMEM
 constexpr int kScaleWarps = 2;  // the copies are split between this many issuing threads
                                 // (four measured no faster than two)
-constexpr int kGemmThreads = (2 + kEpilogueWarps + kScaleWarps) * 32;
-constexpr int kStageStride = 36;  // floats per staged row: 32 + 4 keeps float4 accesses conflict-free
+constexpr int kProducers = 1;
+constexpr int kGemmThreads = (1 + kEpilogueWarps + kScaleWarps + kProducers) * 32;
 
 template <int BN_, int A_ROWS_, int SFB_GS_, int STAGES_, bool ROW_STAGING_ = true>
 struct TileCfg {
@@ -88,31 +86,19 @@ struct TileCfg {
 
 using CfgPrefillUp = TileCfg<208, 128, 8, 4, false>;
 using CfgPrefillDown = TileCfg<192, 128, 8, 4>;
-using CfgDecode = TileCfg<128, 32, 4, 7>;
-using CfgDecodeWide = TileCfg<128, 128, 4, 5>;
-
-__device__ __forceinline__ void report_timeout(int32_t* error, volatile int* abort_flag) {
-  *abort_flag = 1;
-  if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
-}
 
 // All scale copies of one full K block that fall to copier `PART`; compile-time
 // indices only, so that no copy carries a run-time predicate.
-template <class C>
-__device__ __forceinline__ void scale_copy(uint32_t taddr, uint64_t desc) {
-  tcgen05_cp_32x128b_warpx4(taddr, desc);
-}
-
 template <class C, int PART>
-__device__ __forceinline__ void issue_scale_copies(uint32_t sf_tmem, uint32_t sfa_addr,
-                                                   uint32_t sfb_addr) {
+__device__ __forceinline__ void issue_scale_copies(uint32_t sf_tmem, uint64_t sfa_desc,
+                                                   uint64_t sfb_desc) {
 #pragma unroll
   for (int c = PART; c < 4; c += kScaleWarps) {
-    scale_copy<C>(sf_tmem + C::SFA_COL + 4 * c, make_smem_desc(sfa_addr + c * 512, 0, 128, 0));
+    tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFA_COL + 4 * c, advance_smem_desc(sfa_desc, c * 512));
   }
 #pragma unroll
   for (int c = PART; c < C::SFB_GS; c += kScaleWarps) {
-    scale_copy<C>(sf_tmem + C::SFB_COL + 4 * c, make_smem_desc(sfb_addr + c * 512, 0, 128, 0));
+    tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFB_COL + 4 * c, advance_smem_desc(sfb_desc, c * 512));
   }
 }
 
@@ -203,11 +189,18 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
   const int total_tiles = num_row_tiles * args.n_tiles;
   const int k_mmas = args.K / 64;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------- producer
+  if (warp == 0 || warp >= kScaleWarp + kScaleWarps) {
+    // ------------------------------------------------------------- producers
+    // Producer p loads the K blocks p, p + kProducers, ... of the CTA's sequence.
     if (lane == 0) {
-      int stage = 0;
+      const int producer = warp == 0 ? 0 : warp - (kScaleWarp + kScaleWarps) + 1;
+      static_assert(kProducers <= C::STAGES, "a producer advances at most a ring at a time");
+      const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA),
+                     sfb0 = smem_u32(sSFB);
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      int stage = producer % C::STAGES;
       uint32_t phase = 0;
+      int kb = producer;  // K block of the current tile this producer loads next
       bool ok = true;
       for (int t = unit; t < total_tiles && ok; t += units) {
         const int rt = t / args.n_tiles;
@@ -219,165 +212,163 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
         const uint8_t* sfb_src = args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) *
                                                 args.k_blocks * C::SFB_BYTES;
         // weights are stored K-block-major: [expert][k block][row][128 B], then the
-        // partial last K block as [expert][row][tail bytes]; a pair's CTA takes the
-        // half of the tile's rows that belongs to its rank
+        // partial last K block as [expert][row][tail bytes]
         const int b_row = nt * C::BN;
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u)) {
+        const uint8_t* b_src =
+            args.b_full + (static_cast<size_t>(expert) * args.kb_full * args.N + b_row) * 128;
+        for (; kb < args.k_blocks; kb += kProducers) {
+          if (!mbar_wait_at(empty0 + stage * 8, phase ^ 1u)) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&full_bar[stage], C::STAGE_TX);
-          tma_load_2d(sA + stage * C::A_BYTES, &tmap_a, kb * 128, rows.load_row0,
-                      &full_bar[stage]);
+          const uint32_t bar = full0 + stage * 8;
+          mbar_arrive_expect_tx_at(bar, C::STAGE_TX);
+          tma_load_2d_at(a0 + stage * C::A_BYTES, &tmap_a, kb * 128, rows.load_row0, bar);
           if (kb < args.kb_full) {
             // one contiguous, pre-swizzled panel slice: a single bulk copy
-            bulk_load(sB + stage * C::B_BYTES,
-                      args.b_full + (static_cast<size_t>(expert * args.kb_full + kb) * args.N +
-                                     b_row) * 128,
-                      C::B_BYTES, &full_bar[stage]);
+            bulk_load_at(b0 + stage * C::B_BYTES, b_src + static_cast<size_t>(kb) * args.N * 128,
+                         C::B_BYTES, bar);
           } else {
-            tma_load_2d(sB + stage * C::B_BYTES, &tmap_b_tail, 0, expert * args.N + b_row,
-                        &full_bar[stage]);
+            tma_load_2d_at(b0 + stage * C::B_BYTES, &tmap_b_tail, 0, expert * args.N + b_row, bar);
           }
-          bulk_load(sSFA + stage * C::SFA_BYTES, sfa_src + kb * C::SFA_BYTES, C::SFA_BYTES,
-                    &full_bar[stage]);
-          bulk_load(sSFB + stage * C::SFB_BYTES, sfb_src + kb * C::SFB_BYTES, C::SFB_BYTES,
-                    &full_bar[stage]);
-          if (++stage == C::STAGES) {
-            stage = 0;
+          bulk_load_at(sfa0 + stage * C::SFA_BYTES, sfa_src + kb * C::SFA_BYTES, C::SFA_BYTES, bar);
+          bulk_load_at(sfb0 + stage * C::SFB_BYTES, sfb_src + kb * C::SFB_BYTES, C::SFB_BYTES, bar);
+          stage += kProducers;
+          if (stage >= C::STAGES) {
+            stage -= C::STAGES;
             phase ^= 1u;
           }
         }
+        kb -= args.k_blocks;
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_nvf4(C::BN);
+      const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
+      const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
+      const uint32_t empty0 = smem_u32(empty_bar), sf_ready0 = smem_u32(sf_ready_bar);
+      const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
       int stage = 0;
-      uint32_t phase = 0;
       int local = 0;
-      int sf_buf = 0;
-      uint32_t sf_phase = 0;
+      uint32_t sf_buf = 0, sf_phase = 0;
       bool ok = true;
       for (int t = unit; t < total_tiles && ok; t += units, ++local) {
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1u;
-        // both CTAs' epilogues have drained this accumulator
+        // the epilogue has drained this accumulator
         if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
           report_timeout(args.error, abort_flag);
           break;
         }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * C::ACC_STRIDE;
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
-          // the operands have landed (in both CTAs) and the scale copies of this K
-          // block are done
-          // (a pair's full barrier counts the bytes of both CTAs)
-          const bool landed = mbar_wait(&full_bar[stage], phase);
-          if (!landed || !mbar_wait(&sf_ready_bar[sf_buf], sf_phase)) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          // this block's scales are in TMEM, and its operands had landed before they were copied
+          if (!mbar_wait_at(sf_ready0 + sf_buf * 8, sf_phase)) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
           }
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * C::A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * C::B_BYTES);
+          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * C::A_BYTES);
+          const uint64_t b_desc = advance_smem_desc(b_desc0, stage * C::B_BYTES);
           const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
-          const int kt_count = min(4, k_mmas - kb * 4);
-          if (kt_count == 4) {
+          if (kb + 1 < k_blocks || last_mmas == 4) {
 #pragma unroll
             for (int kt = 0; kt < 4; ++kt) {
-              tcgen05_mma_nvf4(d_tmem, make_smem_desc(a_addr + kt * 32, 0, 1024, 2),
-                               make_smem_desc(b_addr + kt * 32, 0, 1024, 2), idesc,
+              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                               advance_smem_desc(b_desc, kt * 32), idesc,
                                sf_tmem + C::SFA_COL + 4 * kt,
-                               sf_tmem + C::SFB_COL + C::SFB_GS * kt, (kb | kt) != 0 ? 1u : 0u);
+                               sf_tmem + C::SFB_COL + C::SFB_GS * kt,
+                               kt != 0 ? 1u : kb != 0 ? 1u : 0u);
             }
           } else {
-            for (int kt = 0; kt < kt_count; ++kt) {
-              tcgen05_mma_nvf4(d_tmem, make_smem_desc(a_addr + kt * 32, 0, 1024, 2),
-                               make_smem_desc(b_addr + kt * 32, 0, 1024, 2), idesc,
+            for (int kt = 0; kt < last_mmas; ++kt) {
+              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                               advance_smem_desc(b_desc, kt * 32), idesc,
                                sf_tmem + C::SFA_COL + 4 * kt,
                                sf_tmem + C::SFB_COL + C::SFB_GS * kt, (kb | kt) != 0 ? 1u : 0u);
             }
           }
-          // frees the stage for the producer(s) and, SF_BUFS K blocks later, this
-          // block's scale columns for the copier
-          tcgen05_commit(&empty_bar[stage]);
+          // frees the stage for the producer and, SF_BUFS K blocks later, this block's scale
+          // columns for the copier
+          tcgen05_commit_at(empty0 + stage * 8);
           if (++sf_buf == C::SF_BUFS) {
             sf_buf = 0;
             sf_phase ^= 1u;
           }
-          if (++stage == C::STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (++stage == C::STAGES) stage = 0;
         }
         if (ok) {
           tcgen05_commit(&tmem_full_bar[acc]);
         }
       }
     }
-  } else if (warp >= kScaleWarp) {
-    if (lane == 0) {
-    // ------------------------------------------------------- block-scale copier
+  } else if (warp >= kScaleWarp) {  // (the producers behind them are taken)
+    // ------------------------------------------------------- block-scale copiers
     // The copies of one K block's scales into TMEM take longer to issue than
-    // its MMAs; a thread of their own lets them run ahead of the MMA thread.
+    // its MMAs; threads of their own let them run ahead of the MMA thread.
+    if (lane == 0) {
       const int part = warp - kScaleWarp;
+      const uint64_t sfa_desc0 = make_smem_desc(smem_u32(sSFA), 0, 128, 0);
+      const uint64_t sfb_desc0 = make_smem_desc(smem_u32(sSFB), 0, 128, 0);
+      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint32_t sf_ready0 = smem_u32(sf_ready_bar);
+      const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
       int stage = 0;
       uint32_t phase = 0;
-      int sf_buf = 0;
+      uint32_t sf_buf = 0;
       // the scale columns written now were last read by the MMAs of the K block
       // SF_BUFS iterations back; those MMAs also release that block's stage
       int old_stage = 0;
       uint32_t old_phase = 0;
-      int iteration = 0;
+      int unread = C::SF_BUFS;  // buffers nothing has read yet
       bool ok = true;
       for (int t = unit; t < total_tiles && ok; t += units) {
-        for (int kb = 0; kb < args.k_blocks; ++kb, ++iteration) {
-          bool ready = true;
-          if (iteration >= C::SF_BUFS) {
-            ready = mbar_wait(&empty_bar[old_stage], old_phase);
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          bool ready = mbar_wait_at(full0 + stage * 8, phase);
+          if (unread > 0) {
+            --unread;
+          } else {
+            ready = ready && mbar_wait_at(empty0 + old_stage * 8, old_phase);
             if (++old_stage == C::STAGES) {
               old_stage = 0;
               old_phase ^= 1u;
             }
           }
-          ready = ready && mbar_wait(&full_bar[stage], phase);
           if (!ready) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
           }
           tcgen05_fence_after();
-          const uint32_t sfa_addr = smem_u32(sSFA + stage * C::SFA_BYTES);
-          const uint32_t sfb_addr = smem_u32(sSFB + stage * C::SFB_BYTES);
+          const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * C::SFA_BYTES);
+          const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * C::SFB_BYTES);
           const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
           // a partial last K block needs the scales of the MMAs it issues only;
           // the full block keeps its copies free of run-time predicates, which
           // slow their issue down considerably
-          const int kt_count = min(4, k_mmas - kb * 4);
-          constexpr int kWeightCopiesPerMma = C::SFB_GS / 4;
-          if (kt_count == 4) {
+          if (kb + 1 < k_blocks || last_mmas == 4) {
             static_assert(kScaleWarps == 2, "one branch per copier");
             if (part == 0) {
-              issue_scale_copies<C, 0>(sf_tmem, sfa_addr, sfb_addr);
+              issue_scale_copies<C, 0>(sf_tmem, sfa_desc, sfb_desc);
             } else {
-              issue_scale_copies<C, 1>(sf_tmem, sfa_addr, sfb_addr);
+              issue_scale_copies<C, 1>(sf_tmem, sfa_desc, sfb_desc);
             }
           } else {
-            for (int c = part; c < kt_count; c += kScaleWarps) {
-              scale_copy<C>(sf_tmem + C::SFA_COL + 4 * c,
-                            make_smem_desc(sfa_addr + c * 512, 0, 128, 0));
+            for (int c = part; c < last_mmas; c += kScaleWarps) {
+              tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFA_COL + 4 * c,
+                                        advance_smem_desc(sfa_desc, c * 512));
             }
-            for (int c = part; c < kt_count * kWeightCopiesPerMma; c += kScaleWarps) {
-              scale_copy<C>(sf_tmem + C::SFB_COL + 4 * c,
-                            make_smem_desc(sfb_addr + c * 512, 0, 128, 0));
+            for (int c = part; c < last_mmas * (C::SFB_GS / 4); c += kScaleWarps) {
+              tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFB_COL + 4 * c,
+                                        advance_smem_desc(sfb_desc, c * 512));
             }
           }
-          tcgen05_commit(&sf_ready_bar[sf_buf]);
+          tcgen05_commit_at(sf_ready0 + sf_buf * 8);
           if (++sf_buf == C::SF_BUFS) sf_buf = 0;
           if (++stage == C::STAGES) {
             stage = 0;
@@ -418,126 +409,12 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
       const int chunk_end = half == 0 ? (kChunks + 1) / 2 : kChunks;
 
       if constexpr (MODE == kGemmUp) {
-        uint8_t* packed_row = args.out_packed + static_cast<size_t>(grow) * (args.N / 2);
-        float row_max = 0.0f;
-        for (int ch = chunk_begin; ch < chunk_end; ++ch) {
-          const int n = n0 + ch * 16;
-          if (n >= args.N) break;
-          float v[16];
-          tmem_ld_x16(t_addr + ch * 16, v);
-          float amax = 0.0f;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float x = fmaxf(__fmul_rn(v[i], scale), 0.0f);  // Relu2: x > 0 ? x*x : 0
-            v[i] = __fmul_rn(x, x);
-            amax = fmaxf(amax, v[i]);
-          }
-          row_max = fmaxf(row_max, amax);
-          uint32_t lo, hi;
-          const uint32_t sf = quantize_block16_unit_scale(v, amax, lo, hi);
-          if (row_valid) {
-            *reinterpret_cast<uint2*>(packed_row + n / 2) = make_uint2(lo, hi);
-            args.out_sf[swizzled_scale_offset(grow, n / 16, args.out_k_blocks * 4)] =
-                static_cast<uint8_t>(sf);
-          }
-        }
-        if (row_valid && row_max > kFp4Max * kFp8Max && args.error != nullptr) {
-          atomicCAS(args.error, kDevOk, kDevActivationRange);
-        }
+        epilogue_quantise<1>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
       } else {
-        // byte address of this row's output row (0 = nothing to store); with
-        // out_segments it lies in the memory of the rank the row returns to
-        unsigned long long dest = 0;
-        float wt = 1.0f;
-        if (row_valid) {
-          const int d = args.dest_row != nullptr ? args.dest_row[grow]
-                                                 : grow * args.dest_mul + args.dest_add;
-          const size_t row_bytes = static_cast<size_t>(args.N) * (args.out_kind == kRowF32 ? 4 : 2);
-          if (d >= 0) {
-            if (args.out_segments != nullptr) {
-              const int slot = d + args.segment_slot0;
-              const int segment = slot / args.segment_rows;
-              dest = args.out_segments[segment] +
-                     static_cast<size_t>(slot - segment * args.segment_rows) * row_bytes;
-            } else {
-              dest = reinterpret_cast<unsigned long long>(args.out_rows) + d * row_bytes;
-            }
-          }
-          if (args.row_weight != nullptr) wt = args.row_weight[grow];
-        }
-        // Each thread owns one output row of the tile, but a store instruction
-        // should write whole lines: stage 32 columns of 32 rows in shared memory,
-        // then let every 8 lanes write 128 contiguous bytes of one row (4 rows
-        // per instruction).
-        float* stage = stage_base + (warp - 2) * (32 * kStageStride);
-        const int sub = lane >> 3;
-        const int c4 = (lane & 7) * 4;
-        for (int ch = chunk_begin; ch < chunk_end; ch += 2) {
-          const int n = n0 + ch * 16;
-          if (n >= args.N) break;
-          const bool wide = ch + 1 < chunk_end && n + 16 < args.N;
-          float va[16], vb[16];
-          tmem_ld_x16(t_addr + ch * 16, va);
-          if (wide) {
-            tmem_ld_x16(t_addr + ch * 16 + 16, vb);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) vb[i] = 0.0f;
-          }
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            va[i] = __fmul_rn(va[i], scale);
-            vb[i] = __fmul_rn(vb[i], scale);
-            if (args.row_weight != nullptr) {
-              va[i] = __fmul_rn(va[i], wt);
-              vb[i] = __fmul_rn(vb[i], wt);
-            }
-            if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
-              const float pa = fmaxf(va[i], 0.0f), pb = fmaxf(vb[i], 0.0f);
-              va[i] = __fmul_rn(pa, pa);
-              vb[i] = __fmul_rn(pb, pb);
-            }
-          }
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            *reinterpret_cast<float4*>(stage + lane * kStageStride + i) =
-                make_float4(va[i], va[i + 1], va[i + 2], va[i + 3]);
-            if (wide) {
-              *reinterpret_cast<float4*>(stage + lane * kStageStride + 16 + i) =
-                  make_float4(vb[i], vb[i + 1], vb[i + 2], vb[i + 3]);
-            }
-          }
-          __syncwarp();
-          const bool col_ok = c4 < (wide ? 32 : 16);
-#pragma unroll 4
-          for (int it = 0; it < 8; ++it) {
-            const int rr = 4 * it + sub;
-            const unsigned long long d = __shfl_sync(0xffffffffu, dest, rr);
-            if (d != 0 && col_ok) {
-              const float4 value = *reinterpret_cast<const float4*>(stage + rr * kStageStride + c4);
-              if (args.out_kind == kRowBf16) {
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(value.x, value.y);
-                const __nv_bfloat162 hi = __floats2bfloat162_rn(value.z, value.w);
-                uint2 bits;
-                bits.x = *reinterpret_cast<const uint32_t*>(&lo);
-                bits.y = *reinterpret_cast<const uint32_t*>(&hi);
-                *reinterpret_cast<uint2*>(d + static_cast<size_t>(n + c4) * 2) = bits;
-              } else if (args.out_kind == kRowF16) {
-                // a value beyond binary16's 65504 becomes an infinity here; the combine
-                // kernel reports it
-                const __half2 lo = __floats2half2_rn(value.x, value.y);
-                const __half2 hi = __floats2half2_rn(value.z, value.w);
-                uint2 bits;
-                bits.x = *reinterpret_cast<const uint32_t*>(&lo);
-                bits.y = *reinterpret_cast<const uint32_t*>(&hi);
-                *reinterpret_cast<uint2*>(d + static_cast<size_t>(n + c4) * 2) = bits;
-              } else {
-                *reinterpret_cast<float4*>(d + static_cast<size_t>(n + c4) * 4) = value;
-              }
-            }
-          }
-        }
+        const unsigned long long dest = row_valid ? output_row_address(args, grow) : 0ull;
+        const float wt = row_valid && args.row_weight != nullptr ? args.row_weight[grow] : 1.0f;
+        epilogue_rows(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt,
+                      stage_base + (warp - 2) * (32 * kStageStride));
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -558,35 +435,36 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
 }
 
 // ---------------------------------------------------------------------------
-// CTA-pair kernel (kVariantPairUp / kVariantPairDown): one 256 x kPairBN tile per cluster
-// of two CTAs (tcgen05.mma.cta_group::2, M = 256).
+// CTA-pair kernel (kVariantPair): one 256 x kPairBN tile per cluster of two CTAs
+// (tcgen05.mma.cta_group::2, M = 256).
 //
-// What bounds the grouped GEMM at prefill sizes is the rate at which an SM can pull its
-// operands from L2 into shared memory (measured: ~50-58 B per cycle per SM with every SM
-// streaming), not the tensor pipe: a 128 x 208 tile stages 49 KB per 256-element K block
-// for 416 cycles of MMA.  A pair stages each weight tile once for 256 rows (half in each
-// CTA), 33 KB per CTA and K block for 352 cycles of MMA.
+// A 128 x 208 tile of one CTA takes 1220 cycles per 256-element K block for 416 cycles of MMA: the
+// twelve tcgen05.cp of its block scales run through the tensor pipe at 47 cycles each beside the
+// MMAs, and every K block brings 49 KB from L2 into an SM that takes about 50 bytes a cycle.  A
+// pair stages each weight tile once for 256 rows (half in each CTA: 35 KB per CTA and K block),
+// and its scales go shared memory -> registers -> TMEM (tcgen05.st), off the tensor pipe, from
+// four warps per CTA, one per TMEM lane quarter, each CTA for its own TMEM.
 //
-// Two more measurements shape the kernel.  A tcgen05.cp of 512 scale bytes costs ~47
-// cycles of the tensor pipe alone and more while MMAs run, and the MMAs that need the
-// scales queue behind it (12 copies per K block outweigh its four MMAs), so the scales go
-// shared memory -> registers -> TMEM (tcgen05.st) from four warps per CTA, one per TMEM
-// lane quarter, each CTA for its own TMEM.  And an mbarrier wait costs the waiting
-// thread 100-250 cycles even when the phase has completed, so every role waits at most
-// twice per K block and the scales rotate through three TMEM buffers.
+// The roles are single threads or warps whose every step is latency: a wait costs 140 cycles when
+// there is nothing to wait for and 250 when there is, so a K block has ONE barrier the MMA thread
+// waits for -- the full barrier of the leader counts the activation and weight bytes of both CTAs
+// and the arrivals of all eight scale warps -- and two producers per CTA take turns.
 //
-// Roles per CTA: warp 0 loads (its own 128 activation rows, its half of the weight tile,
-// the scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues
-// the MMAs for both, warps 2-9 run the epilogue of the CTA's 128 rows, warps 10-13 write
-// scales.  Activation and weight bytes of BOTH CTAs complete on rank 0's full barrier
-// (the loads name it; no multicast); scale bytes complete on a barrier of their own CTA.
+// Roles per CTA: warps 0 and 14 load (the CTA's own 128 activation rows, its half of the weight
+// tile, the scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues the
+// MMAs for both, warps 2-9 run the epilogue of the CTA's 128 rows, warps 10-13 write scales.  No
+// multicast: the loads of the partner name the leader's barrier.
+//
+// Measured, benchmark layer, up / down projection: 16384 tokens 331 / 401 -> @P1@ us, 8192 tokens
+// 188 / 221 -> @P2@.
 // ---------------------------------------------------------------------------
-constexpr int kPairBN = 176;
+constexpr int kPairBN = 208;
 constexpr int kPairBRows = kPairBN / 2;        // weight rows staged per CTA
 constexpr int kPairStages = 6;
-constexpr int kPairSfBufs = 3;
+constexpr int kPairSfBufs = 2;
 constexpr int kPairScaleWarps = 4;             // one per TMEM lane quarter
-constexpr int kPairThreads = (2 + kEpilogueWarps + kPairScaleWarps) * 32;
+constexpr int kPairProducers = 2;
+constexpr int kPairThreads = (1 + kEpilogueWarps + kPairScaleWarps + kPairProducers) * 32;
 constexpr int kPairABytes = 128 * 128;
 constexpr int kPairBBytes = kPairBRows * 128;
 constexpr int kPairSfaBytes = 2048;
@@ -595,7 +473,7 @@ constexpr int kPairSfbBytes = kPairSfbGroups * 512;
 constexpr int kPairStageBytes = kPairABytes + kPairBBytes + kPairSfaBytes + kPairSfbBytes;
 constexpr int kPairSfCol = 2 * kPairBN;        // TMEM: two accumulators, then the scale buffers
 constexpr int kPairSfBufCols = 16 + 4 * kPairSfbGroups;
-constexpr int kPairBarBytes = ((3 * kPairStages + 4 + kPairSfBufs) * 8 + 16 + 15) / 16 * 16;
+constexpr int kPairBarBytes = ((3 * kPairStages + 4) * 8 + 16 + 15) / 16 * 16;
 constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + kPairBarBytes + 1024;
 static_assert(kPairSfCol + kPairSfBufs * kPairSfBufCols <= 512, "TMEM budget");
 static_assert(kPairBRows % 8 == 0, "half a weight tile is whole 8-row swizzle groups");
@@ -604,7 +482,6 @@ static_assert(kPairSmemBytes <= 232448, "shared memory budget");
 
 struct PairShape {  // what tile_rows_of reads
   static constexpr bool PAIR = true;
-  static constexpr int BN = kPairBN;
 };
 
 template <int MODE>
@@ -618,13 +495,13 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   uint8_t* sB = sA + kPairStages * kPairABytes;
   uint8_t* sSFA = sB + kPairStages * kPairBBytes;
   uint8_t* sSFB = sSFA + kPairStages * kPairSfaBytes;
+  // full_bar (the leader's): operand bytes of both CTAs and the scale warps of both
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(sSFB + kPairStages * kPairSfbBytes);
   uint64_t* sf_full_bar = full_bar + kPairStages;   // this CTA's scale bytes landed
   uint64_t* empty_bar = sf_full_bar + kPairStages;  // both CTAs: the MMAs have read the stage
   uint64_t* tmem_full_bar = empty_bar + kPairStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
-  uint64_t* sf_ready_bar = tmem_empty_bar + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sf_ready_bar + kPairSfBufs);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -636,7 +513,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
-      mbar_init(&full_bar[s], 1);
+      mbar_init(&full_bar[s], 1 + 2 * kPairScaleWarps);
       mbar_init(&sf_full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -644,7 +521,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       mbar_init(&tmem_full_bar[a], 1);
       mbar_init(&tmem_empty_bar[a], 2 * kEpilogueWarps);
     }
-    for (int b = 0; b < kPairSfBufs; ++b) mbar_init(&sf_ready_bar[b], 2 * kPairScaleWarps);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tensormap(&maps.a);
@@ -665,70 +541,76 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128;
   const int row_units = (num_row_tiles + 1) / 2;
   const int total_tiles = row_units * args.n_tiles;
-  const int k_mmas = args.K / 64;
+  const int k_blocks = args.k_blocks;
+  const uint32_t full0 = smem_u32(full_bar), sf_full0 = smem_u32(sf_full_bar);
+  const uint32_t empty0 = smem_u32(empty_bar);
+  const uint32_t leader_full0 = cluster_address_of(&full_bar[0], 0);
 
-  if (warp == 0) {
-    // ------------------------------------------------------------- producer
+  if (warp == 0 || warp >= kScaleWarp + kPairScaleWarps) {
+    // ------------------------------------------------------------- producers
+    // Producer p loads the K blocks p, p + kPairProducers, ... of the CTA's sequence.
     if (lane == 0) {
-      int stage = 0;
+      const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+      const uint32_t sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
+      int stage = warp == 0 ? 0 : warp - (kScaleWarp + kPairScaleWarps) + 1;
+      int kb = stage;  // K block of the current tile this producer loads next
       uint32_t phase = 0;
       bool ok = true;
-      const uint32_t leader_full0 = cluster_address_of(&full_bar[0], 0);
       for (int t = unit; t < total_tiles && ok; t += units) {
         const int rt = t / args.n_tiles;
         const int nt = t - rt * args.n_tiles;
         const TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
         const int expert = rows.expert;
         const uint8_t* sfa_src =
-            args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * args.k_blocks * kPairSfaBytes;
-        const uint8_t* sfb_src = args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) *
-                                                args.k_blocks * kPairSfbBytes;
+            args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * k_blocks * kPairSfaBytes;
+        const uint8_t* sfb_src =
+            args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) * k_blocks * kPairSfbBytes;
         const int b_row = nt * kPairBN + static_cast<int>(cta_rank) * kPairBRows;
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u)) {
+        for (; kb < k_blocks; kb += kPairProducers) {
+          if (!mbar_wait_at(empty0 + stage * 8, phase ^ 1u)) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
           }
-          if (args.ablate & 4) {
-            if (leader) mbar_arrive(&full_bar[stage]);
-            mbar_arrive(&sf_full_bar[stage]);
-          } else {
-            // activation and weight bytes of both CTAs are counted on the leader's barrier
-            const uint32_t bar = leader_full0 + static_cast<uint32_t>(stage) * 8u;
-            if (leader) {
-              mbar_arrive_expect_tx(&full_bar[stage], 2 * (kPairABytes + kPairBBytes));
-            }
-            mbar_arrive_expect_tx(&sf_full_bar[stage], kPairSfaBytes + kPairSfbBytes);
-            tma_load_2d_pair(sA + stage * kPairABytes, &maps.a, kb * 128, rows.load_row0, bar);
-            if (kb < args.kb_full) {
-              tma_load_2d_pair(sB + stage * kPairBBytes, &maps.b_full, 0,
-                               (expert * args.kb_full + kb) * args.N + b_row, bar);
-            } else {
-              tma_load_2d_pair(sB + stage * kPairBBytes, &maps.b_tail, 0, expert * args.N + b_row,
-                               bar);
-            }
-            bulk_load(sSFA + stage * kPairSfaBytes, sfa_src + kb * kPairSfaBytes, kPairSfaBytes,
-                      &sf_full_bar[stage]);
-            bulk_load(sSFB + stage * kPairSfbBytes, sfb_src + kb * kPairSfbBytes, kPairSfbBytes,
-                      &sf_full_bar[stage]);
+          const uint32_t bar = leader_full0 + stage * 8, sf_bar = sf_full0 + stage * 8;
+          mbar_arrive_expect_tx_at(sf_bar, kPairSfaBytes + kPairSfbBytes);
+          bulk_load_at(sfa0 + stage * kPairSfaBytes, sfa_src + kb * kPairSfaBytes, kPairSfaBytes,
+                       sf_bar);
+          bulk_load_at(sfb0 + stage * kPairSfbBytes, sfb_src + kb * kPairSfbBytes, kPairSfbBytes,
+                       sf_bar);
+          // activation and weight bytes of both CTAs are counted on the leader's barrier
+          if (leader) {
+            mbar_arrive_expect_tx_at(full0 + stage * 8, 2 * (kPairABytes + kPairBBytes));
           }
-          if (++stage == kPairStages) {
-            stage = 0;
+          tma_load_2d_pair_at(a0 + stage * kPairABytes, &maps.a, kb * 128, rows.load_row0, bar);
+          if (kb < args.kb_full) {
+            // the map's rows are eight weight rows' 128 bytes of a K block
+            tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_full, 0,
+                                ((expert * args.kb_full + kb) * args.N + b_row) >> 3, bar);
+          } else {
+            tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_tail, 0, expert * args.N + b_row,
+                                bar);
+          }
+          stage += kPairProducers;
+          if (stage >= kPairStages) {
+            stage -= kPairStages;
             phase ^= 1u;
           }
         }
+        kb -= k_blocks;
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0 && leader) {
       constexpr uint32_t idesc = make_idesc_nvf4_pair(kPairBN);
+      const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
+      const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
+      const int last_mmas = args.K / 64 - 4 * (k_blocks - 1);
       int stage = 0;
       uint32_t phase = 0;
       int local = 0;
-      int sf_buf = 0;
-      uint32_t sf_phase = 0;
+      uint32_t sf_buf = 0;
       bool ok = true;
       for (int t = unit; t < total_tiles && ok; t += units, ++local) {
         const int acc = local & 1;
@@ -740,42 +622,36 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kPairBN;
-        for (int kb = 0; kb < args.k_blocks; ++kb) {
+        for (int kb = 0; kb < k_blocks; ++kb) {
           // the operands of both CTAs have landed and both have written this block's scales
-          if (!mbar_wait_cluster(&full_bar[stage], phase) ||
-              !mbar_wait_cluster(&sf_ready_bar[sf_buf], sf_phase)) {
+          if (!mbar_wait_cluster_at(full0 + stage * 8, phase)) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
           }
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * kPairABytes);
-          const uint32_t b_addr = smem_u32(sB + stage * kPairBBytes);
+          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * kPairABytes);
+          const uint64_t b_desc = advance_smem_desc(b_desc0, stage * kPairBBytes);
           const uint32_t sf_tmem = tmem_base + kPairSfCol + sf_buf * kPairSfBufCols;
-          const int kt_count = (args.ablate & 8) ? 0 : min(4, k_mmas - kb * 4);
-          if (kt_count == 4) {
+          if (kb + 1 < k_blocks || last_mmas == 4) {
 #pragma unroll
             for (int kt = 0; kt < 4; ++kt) {
-              tcgen05_mma_pair_nvf4(d_tmem, make_smem_desc(a_addr + kt * 32, 0, 1024, 2),
-                                    make_smem_desc(b_addr + kt * 32, 0, 1024, 2), idesc,
-                                    sf_tmem + 4 * kt, sf_tmem + 16 + kPairSfbGroups * kt,
-                                    (kb | kt) != 0 ? 1u : 0u);
+              tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                                    advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
+                                    sf_tmem + 16 + kPairSfbGroups * kt,
+                                    kt != 0 ? 1u : kb != 0 ? 1u : 0u);
             }
           } else {
-            for (int kt = 0; kt < kt_count; ++kt) {
-              tcgen05_mma_pair_nvf4(d_tmem, make_smem_desc(a_addr + kt * 32, 0, 1024, 2),
-                                    make_smem_desc(b_addr + kt * 32, 0, 1024, 2), idesc,
-                                    sf_tmem + 4 * kt, sf_tmem + 16 + kPairSfbGroups * kt,
-                                    (kb | kt) != 0 ? 1u : 0u);
+            for (int kt = 0; kt < last_mmas; ++kt) {
+              tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                                    advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
+                                    sf_tmem + 16 + kPairSfbGroups * kt, (kb | kt) != 0 ? 1u : 0u);
             }
           }
           // frees the stage in both CTAs and, kPairSfBufs K blocks later, this block's
           // scale columns
           tcgen05_commit_pair(&empty_bar[stage], 3);
-          if (++sf_buf == kPairSfBufs) {
-            sf_buf = 0;
-            sf_phase ^= 1u;
-          }
+          if (++sf_buf == kPairSfBufs) sf_buf = 0;
           if (++stage == kPairStages) {
             stage = 0;
             phase ^= 1u;
@@ -784,75 +660,68 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         if (ok) tcgen05_commit_pair(&tmem_full_bar[acc], 3);
       }
     }
-  } else if (warp >= kScaleWarp) {
+  } else if (warp >= kScaleWarp) {  // (the producer behind them is taken)
     // ------------------------------------------------------- block-scale writers
     // Each warp writes the same 32 x 16 B of every 512-byte chunk to its own lane
     // quarter: the layout a tcgen05.cp.32x128b.warpx4 produces.
     const int quarter = warp & 3;
-    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t sf_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kPairSfCol;
     int stage = 0;
     uint32_t phase = 0;
-    int sf_buf = 0;
+    uint32_t sf_buf = 0;
     // the scale columns written now were last read by the MMAs of the K block kPairSfBufs
     // iterations back; those MMAs also release that block's stage
     int old_stage = 0;
     uint32_t old_phase = 0;
-    int iteration = 0;
+    int unread = kPairSfBufs;  // buffers nothing has read yet
     bool ok = true;
     for (int t = unit; t < total_tiles && ok; t += units) {
-      for (int kb = 0; kb < args.k_blocks; ++kb, ++iteration) {
-        bool ready = true;
-        if (iteration >= kPairSfBufs) {
-          ready = mbar_wait(&empty_bar[old_stage], old_phase);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        bool ready = mbar_wait_at(sf_full0 + stage * 8, phase);
+        const uint4* sfa = reinterpret_cast<const uint4*>(sSFA + stage * kPairSfaBytes) + lane;
+        const uint4* sfb = reinterpret_cast<const uint4*>(sSFB + stage * kPairSfbBytes) + lane;
+        uint32_t row_words[16], lo_words[16], hi_words[16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint4 q = sfa[c * 32];
+          row_words[4 * c] = q.x;
+          row_words[4 * c + 1] = q.y;
+          row_words[4 * c + 2] = q.z;
+          row_words[4 * c + 3] = q.w;
+          const uint4 u = sfb[c * 32];
+          lo_words[4 * c] = u.x;
+          lo_words[4 * c + 1] = u.y;
+          lo_words[4 * c + 2] = u.z;
+          lo_words[4 * c + 3] = u.w;
+          const uint4 v = sfb[(c + 4) * 32];
+          hi_words[4 * c] = v.x;
+          hi_words[4 * c + 1] = v.y;
+          hi_words[4 * c + 2] = v.z;
+          hi_words[4 * c + 3] = v.w;
+        }
+        if (unread > 0) {
+          --unread;
+        } else {
+          ready = ready && mbar_wait_at(empty0 + old_stage * 8, old_phase);
           if (++old_stage == kPairStages) {
             old_stage = 0;
             old_phase ^= 1u;
           }
         }
-        ready = ready && mbar_wait(&sf_full_bar[stage], phase);
         if (!ready) {
           if (lane == 0) report_timeout(args.error, abort_flag);
           ok = false;
           break;
         }
-        if (!(args.ablate & 2)) {
-          tcgen05_fence_after();
-          const uint32_t sf_tmem = tmem_base + lane_base + kPairSfCol + sf_buf * kPairSfBufCols;
-          const uint4* sfa = reinterpret_cast<const uint4*>(sSFA + stage * kPairSfaBytes) + lane;
-          const uint4* sfb = reinterpret_cast<const uint4*>(sSFB + stage * kPairSfbBytes) + lane;
-          uint32_t row_words[16], lo_words[16], hi_words[16];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 q = sfa[c * 32];
-            row_words[4 * c] = q.x;
-            row_words[4 * c + 1] = q.y;
-            row_words[4 * c + 2] = q.z;
-            row_words[4 * c + 3] = q.w;
-            const uint4 u = sfb[c * 32];
-            lo_words[4 * c] = u.x;
-            lo_words[4 * c + 1] = u.y;
-            lo_words[4 * c + 2] = u.z;
-            lo_words[4 * c + 3] = u.w;
-            const uint4 v = sfb[(c + 4) * 32];
-            hi_words[4 * c] = v.x;
-            hi_words[4 * c + 1] = v.y;
-            hi_words[4 * c + 2] = v.z;
-            hi_words[4 * c + 3] = v.w;
-          }
-          tmem_st_x16(sf_tmem, row_words);
-          tmem_st_x16(sf_tmem + 16, lo_words);
-          tmem_st_x16(sf_tmem + 32, hi_words);
-          tmem_st_wait();
-          tcgen05_fence_before();
-        }
+        tcgen05_fence_after();
+        const uint32_t sf_tmem = sf_tmem0 + sf_buf * kPairSfBufCols;
+        tmem_st_x16(sf_tmem, row_words);
+        tmem_st_x16(sf_tmem + 16, lo_words);
+        tmem_st_x16(sf_tmem + 32, hi_words);
+        tmem_st_wait();
+        tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          if (leader) {
-            mbar_arrive(&sf_ready_bar[sf_buf]);
-          } else {
-            mbar_arrive_remote(&sf_ready_bar[sf_buf], 0);
-          }
-        }
+        if (lane == 0) mbar_arrive_cluster_at(leader_full0 + stage * 8);
         if (++sf_buf == kPairSfBufs) sf_buf = 0;
         if (++stage == kPairStages) {
           stage = 0;
@@ -865,9 +734,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
     const int quarter = warp & 3;           // TMEM lanes a warp may read: 32 * (warp % 4)
     const int half = (warp - 2) >> 2;       // which part of the tile's 16-column chunks
     const int r = quarter * 32 + lane;      // row inside this CTA's 128 rows == TMEM lane
-    constexpr int kChunks = kPairBN / 16;   // 11: six for the first warp of a quarter, five
+    constexpr int kChunks = kPairBN / 16;   // 13: seven for the first warp of a quarter, six
     const int chunk_begin = half == 0 ? 0 : (kChunks + 1) / 2;
     const int chunk_end = half == 0 ? (kChunks + 1) / 2 : kChunks;
+    const uint32_t leader_empty0 = cluster_address_of(&tmem_empty_bar[0], 0);
     int local = 0;
     for (int t = unit; t < total_tiles; t += units, ++local) {
       const int acc = local & 1;
@@ -875,133 +745,34 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       const int rt = t / args.n_tiles;
       const int nt = t - rt * args.n_tiles;
       const TileRows tile = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
-      const int row0 = tile.row0, rows = tile.rows, expert = tile.expert;
-      const bool row_valid = r < rows;
-      const int grow = row0 + r;
-      float scale = args.w_tensor_scale[expert];
+      const bool row_valid = r < tile.rows;
+      const int grow = tile.row0 + r;
+      float scale = args.w_tensor_scale[tile.expert];
       if (args.a_tensor_scale != nullptr && row_valid) scale *= args.a_tensor_scale[grow];
-      // kGemmDown: byte address of this row's output row (0 = nothing to store); with
-      // out_segments it lies in the memory of the rank the row returns to
       unsigned long long dest = 0;
       float wt = 1.0f;
       if (MODE == kGemmDown && row_valid) {
-        const int d = args.dest_row != nullptr ? args.dest_row[grow]
-                                               : grow * args.dest_mul + args.dest_add;
-        const size_t row_bytes = static_cast<size_t>(args.N) * (args.out_kind == kRowF32 ? 4 : 2);
-        if (d >= 0) {
-          if (args.out_segments != nullptr) {
-            const int slot = d + args.segment_slot0;
-            const int segment = slot / args.segment_rows;
-            dest = args.out_segments[segment] +
-                   static_cast<size_t>(slot - segment * args.segment_rows) * row_bytes;
-          } else {
-            dest = reinterpret_cast<unsigned long long>(args.out_rows) + d * row_bytes;
-          }
-        }
+        dest = output_row_address(args, grow);
         if (args.row_weight != nullptr) wt = args.row_weight[grow];
       }
       if (!mbar_wait(&tmem_full_bar[acc], acc_phase)) {
         report_timeout(args.error, abort_flag);
         break;
       }
-      tcgen05_fence_after();
-      const uint32_t t_addr =
-          tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kPairBN;
-      const int n0 = nt * kPairBN;
-      float row_max = 0.0f;
-      // two batches of up to three chunks: three loads in flight, one wait; the
-      // accumulator goes back to the MMA thread once the second batch is in registers
-      // (columns past N hold accumulator garbage and are never stored)
-#pragma unroll 1
-      for (int batch = chunk_begin; batch < chunk_end; batch += 3) {
-        uint32_t raw[3][16];
-        const bool last = batch + 3 >= chunk_end;
-        if (!(args.ablate & 1)) {
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            if (batch + j < chunk_end) tmem_ld_x16_async(t_addr + (batch + j) * 16, raw[j]);
-          }
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 3; ++j) tmem_ld_fence(raw[j]);
+      if (quarter * 32 < tile.rows) {  // (else none of the warp's rows exist)
+        tcgen05_fence_after();
+        const uint32_t t_addr =
+            tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kPairBN;
+        const int n0 = nt * kPairBN;
+        if constexpr (MODE == kGemmUp) {
+          epilogue_quantise<2>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
+        } else {
+          epilogue_rows_direct<2>(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt);
         }
-        if (last) {
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (leader) {
-              mbar_arrive(&tmem_empty_bar[acc]);
-            } else {
-              mbar_arrive_remote(&tmem_empty_bar[acc], 0);  // the leader waits for both CTAs
-            }
-          }
-        }
-        if (args.ablate & 1) continue;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int n = n0 + (batch + j) * 16;
-          if (batch + j >= chunk_end || n >= args.N) continue;
-          float v[16];
-          if constexpr (MODE == kGemmUp) {
-            float amax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              // Relu2: x > 0 ? x*x : 0
-              const float x = fmaxf(__fmul_rn(__uint_as_float(raw[j][i]), scale), 0.0f);
-              v[i] = __fmul_rn(x, x);
-              amax = fmaxf(amax, v[i]);
-            }
-            row_max = fmaxf(row_max, amax);
-            uint32_t lo, hi;
-            const uint32_t sf = quantize_block16_unit_scale(v, amax, lo, hi);
-            if (row_valid) {
-              uint8_t* packed_row = args.out_packed + static_cast<size_t>(grow) * (args.N / 2);
-              *reinterpret_cast<uint2*>(packed_row + n / 2) = make_uint2(lo, hi);
-              args.out_sf[swizzled_scale_offset(grow, n / 16, args.out_k_blocks * 4)] =
-                  static_cast<uint8_t>(sf);
-            }
-          } else if (dest != 0) {
-            // every thread stores its own row: 16 columns are 32 (16-bit rows) or 64
-            // bytes, whole sectors either way
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              v[i] = __fmul_rn(__uint_as_float(raw[j][i]), scale);
-              if (args.row_weight != nullptr) v[i] = __fmul_rn(v[i], wt);
-              if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
-                const float p = fmaxf(v[i], 0.0f);
-                v[i] = __fmul_rn(p, p);
-              }
-            }
-            if (args.out_kind == kRowF32) {
-              float4* d = reinterpret_cast<float4*>(dest + static_cast<size_t>(n) * 4);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-              }
-            } else {
-              uint32_t w[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                if (args.out_kind == kRowBf16) {
-                  const __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                  w[i] = *reinterpret_cast<const uint32_t*>(&two);
-                } else {
-                  // a value beyond binary16's 65504 becomes an infinity here; the combine
-                  // kernel reports it
-                  const __half2 two = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-                  w[i] = *reinterpret_cast<const uint32_t*>(&two);
-                }
-              }
-              uint4* d = reinterpret_cast<uint4*>(dest + static_cast<size_t>(n) * 2);
-              d[0] = make_uint4(w[0], w[1], w[2], w[3]);
-              d[1] = make_uint4(w[4], w[5], w[6], w[7]);
-            }
-          }
-        }
+        tcgen05_fence_before();
       }
-      if (MODE == kGemmUp && row_valid && row_max > kFp4Max * kFp8Max && args.error != nullptr) {
-        atomicCAS(args.error, kDevOk, kDevActivationRange);
-      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster_at(leader_empty0 + acc * 8);
     }
   }
 
@@ -1151,10 +922,7 @@ GemmVariantInfo gemm_variant_info(GemmVariant v) {
   switch (v) {
     case kVariantPrefillUp: return info_of<CfgPrefillUp>();
     case kVariantPrefillDown: return info_of<CfgPrefillDown>();
-    case kVariantDecode: return info_of<CfgDecode>();
-    case kVariantDecodeWide: return info_of<CfgDecodeWide>();
-    case kVariantPairUp:
-    case kVariantPairDown:
+    case kVariantPair:
       return GemmVariantInfo{kPairBN, 128, kPairSfbGroups, kPairSfbBytes, kPairSmemBytes,
                              kPairBRows};
     default: return GemmVariantInfo{0, 0, 0, 0, 0, 0};
@@ -1166,10 +934,7 @@ cudaError_t launch_grouped_gemm(GemmVariant v, GemmMode mode, const GemmMaps& ma
   switch (v) {
     case kVariantPrefillUp: return launch_cfg<CfgPrefillUp>(mode, maps, args, num_sms, stream);
     case kVariantPrefillDown: return launch_cfg<CfgPrefillDown>(mode, maps, args, num_sms, stream);
-    case kVariantDecode: return launch_cfg<CfgDecode>(mode, maps, args, num_sms, stream);
-    case kVariantDecodeWide: return launch_cfg<CfgDecodeWide>(mode, maps, args, num_sms, stream);
-    case kVariantPairUp:
-    case kVariantPairDown:
+    case kVariantPair:
       if (num_sms < 2) return cudaErrorInvalidValue;
       return mode == kGemmUp ? launch_pair<kGemmUp>(maps, args, num_sms, stream)
                              : launch_pair<kGemmDown>(maps, args, num_sms, stream);

@@ -1,0 +1,237 @@
+// What the expert GEMM kernels share: the row tile a CTA works on, and the two epilogues that take
+// a 128-row accumulator out of TMEM.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace nmoe {
+
+constexpr int kEpilogueWarps = 8;    // two per TMEM lane quarter
+constexpr int kStageStride = 36;     // floats per staged row: 32 + 4 keeps float4 accesses conflict-free
+
+__device__ __forceinline__ void report_timeout(int32_t* error, volatile int* abort_flag) {
+  *abort_flag = 1;
+  if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
+}
+
+// BATCH 16-column chunks of this warp's TMEM lane quarter, all in flight before one wait: a chunk's
+// arithmetic is one long dependent chain, several of them fill each other's gaps.
+template <int BATCH>
+__device__ __forceinline__ void load_chunks(uint32_t t_addr, int count, uint32_t (&raw)[BATCH][16]) {
+#pragma unroll
+  for (int j = 0; j < BATCH; ++j) {
+    if (j < count) tmem_ld_x16_async(t_addr + j * 16, raw[j]);
+  }
+  tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < BATCH; ++j) tmem_ld_fence(raw[j]);
+}
+
+// relu^2 and NVFP4 quantisation of 16 columns from `n` of row `grow`; returns the largest value.
+__device__ __forceinline__ float quantise_chunk(const GemmArgs& args, float (&v)[16], int n, int grow,
+                                                float scale, bool store) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float x = fmaxf(__fmul_rn(v[i], scale), 0.0f);  // Relu2: x > 0 ? x*x : 0
+    v[i] = __fmul_rn(x, x);
+    amax = fmaxf(amax, v[i]);
+  }
+  uint32_t lo, hi;
+  const uint32_t sf = quantize_block16_unit_scale(v, amax, lo, hi);
+  if (!store) return 0.0f;
+  *reinterpret_cast<uint2*>(args.out_packed + static_cast<size_t>(grow) * (args.N / 2) + n / 2) =
+      make_uint2(lo, hi);
+  args.out_sf[swizzled_scale_offset(grow, n / 16, args.out_k_blocks * 4)] = static_cast<uint8_t>(sf);
+  return amax;
+}
+
+__device__ __forceinline__ void report_range(const GemmArgs& args, float largest) {
+  if (largest > kFp4Max * kFp8Max && args.error != nullptr) {
+    atomicCAS(args.error, kDevOk, kDevActivationRange);
+  }
+}
+
+// Scale [x routing weight] [-> relu^2] of 16 columns from `n`, stored in the output row at `dest`.
+__device__ __forceinline__ void store_chunk(const GemmArgs& args, float (&v)[16], int n,
+                                            unsigned long long dest, float scale, float wt) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    v[i] = __fmul_rn(v[i], scale);
+    if (args.row_weight != nullptr) v[i] = __fmul_rn(v[i], wt);
+    if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
+      const float p = fmaxf(v[i], 0.0f);
+      v[i] = __fmul_rn(p, p);
+    }
+  }
+  if (args.out_kind == kRowF32) {
+    float4* d = reinterpret_cast<float4*>(dest + static_cast<size_t>(n) * 4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+    return;
+  }
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (args.out_kind == kRowBf16) {
+      const __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&two);
+    } else {
+      // a value beyond binary16's 65504 becomes an infinity here; the combine kernel reports it
+      const __half2 two = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&two);
+    }
+  }
+  uint4* d = reinterpret_cast<uint4*>(dest + static_cast<size_t>(n) * 2);
+  d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// Up projection: relu^2 and NVFP4 quantisation of columns [n0 + 16 * chunk_begin,
+// n0 + 16 * chunk_end) of the accumulator at `t_addr` (this warp's lane quarter); the thread owns
+// row `grow` of the hidden activations.
+template <int BATCH>
+__device__ __forceinline__ void epilogue_quantise(const GemmArgs& args, uint32_t t_addr, int n0,
+                                                  int chunk_begin, int chunk_end, int grow,
+                                                  bool row_valid, float scale) {
+  float row_max = 0.0f;
+  chunk_end = min(chunk_end, (args.N - n0) / 16);
+  for (int first = chunk_begin; first < chunk_end; first += BATCH) {
+    uint32_t raw[BATCH][16];
+    load_chunks<BATCH>(t_addr + first * 16, chunk_end - first, raw);
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[j][i]);
+      row_max = fmaxf(row_max, quantise_chunk(args, v, n0 + (first + j) * 16, grow, scale,
+                                              row_valid && first + j < chunk_end));
+    }
+  }
+  report_range(args, row_max);
+}
+
+// Byte address of the output row of activation row `grow` (0 = nothing to store); with
+// out_segments it lies in the memory of the rank the row returns to.
+__device__ __forceinline__ unsigned long long output_row_address(const GemmArgs& args, int grow) {
+  const int d = args.dest_row != nullptr ? args.dest_row[grow]
+                                         : grow * args.dest_mul + args.dest_add;
+  if (d < 0) return 0;
+  const size_t row_bytes = static_cast<size_t>(args.N) * (args.out_kind == kRowF32 ? 4 : 2);
+  if (args.out_segments != nullptr) {
+    const int slot = d + args.segment_slot0;
+    const int segment = slot / args.segment_rows;
+    return args.out_segments[segment] +
+           static_cast<size_t>(slot - segment * args.segment_rows) * row_bytes;
+  }
+  return reinterpret_cast<unsigned long long>(args.out_rows) + d * row_bytes;
+}
+
+// Row-storing epilogue without staging: every thread stores its own row, 16 columns (32 or 64
+// bytes, whole sectors) at a time.
+template <int BATCH>
+__device__ __forceinline__ void epilogue_rows_direct(const GemmArgs& args, uint32_t t_addr, int n0,
+                                                     int chunk_begin, int chunk_end,
+                                                     unsigned long long dest, float scale,
+                                                     float wt) {
+  chunk_end = min(chunk_end, (args.N - n0) / 16);
+  for (int first = chunk_begin; first < chunk_end; first += BATCH) {
+    uint32_t raw[BATCH][16];
+    load_chunks<BATCH>(t_addr + first * 16, chunk_end - first, raw);
+    if (dest == 0) continue;
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      if (first + j >= chunk_end) break;
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[j][i]);
+      store_chunk(args, v, n0 + (first + j) * 16, dest, scale, wt);
+    }
+  }
+}
+
+// Row-storing epilogue: scale [x routing weight] [-> relu^2], scattered.  Each thread owns one row
+// of the tile, but a store instruction should write whole lines: 32 columns of 32 rows are staged
+// in shared memory (`stage`: 32 * kStageStride floats of this warp's own), then every 8 lanes
+// write 128 contiguous bytes of one row (4 rows per instruction).
+__device__ __forceinline__ void epilogue_rows(const GemmArgs& args, uint32_t t_addr, int n0,
+                                              int chunk_begin, int chunk_end,
+                                              unsigned long long dest, float scale, float wt,
+                                              float* stage) {
+  const int lane = threadIdx.x & 31;
+  const int sub = lane >> 3;
+  const int c4 = (lane & 7) * 4;
+  for (int ch = chunk_begin; ch < chunk_end; ch += 2) {
+    const int n = n0 + ch * 16;
+    if (n >= args.N) break;
+    const bool wide = ch + 1 < chunk_end && n + 16 < args.N;
+    float va[16], vb[16];
+    tmem_ld_x16(t_addr + ch * 16, va);
+    if (wide) {
+      tmem_ld_x16(t_addr + ch * 16 + 16, vb);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) vb[i] = 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      va[i] = __fmul_rn(va[i], scale);
+      vb[i] = __fmul_rn(vb[i], scale);
+      if (args.row_weight != nullptr) {
+        va[i] = __fmul_rn(va[i], wt);
+        vb[i] = __fmul_rn(vb[i], wt);
+      }
+      if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
+        const float pa = fmaxf(va[i], 0.0f), pb = fmaxf(vb[i], 0.0f);
+        va[i] = __fmul_rn(pa, pa);
+        vb[i] = __fmul_rn(pb, pb);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+      *reinterpret_cast<float4*>(stage + lane * kStageStride + i) =
+          make_float4(va[i], va[i + 1], va[i + 2], va[i + 3]);
+      if (wide) {
+        *reinterpret_cast<float4*>(stage + lane * kStageStride + 16 + i) =
+            make_float4(vb[i], vb[i + 1], vb[i + 2], vb[i + 3]);
+      }
+    }
+    __syncwarp();
+    const bool col_ok = c4 < (wide ? 32 : 16);
+#pragma unroll 4
+    for (int it = 0; it < 8; ++it) {
+      const int rr = 4 * it + sub;
+      const unsigned long long d = __shfl_sync(0xffffffffu, dest, rr);
+      if (d != 0 && col_ok) {
+        const float4 value = *reinterpret_cast<const float4*>(stage + rr * kStageStride + c4);
+        if (args.out_kind == kRowBf16) {
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(value.x, value.y);
+          const __nv_bfloat162 hi = __floats2bfloat162_rn(value.z, value.w);
+          uint2 bits;
+          bits.x = *reinterpret_cast<const uint32_t*>(&lo);
+          bits.y = *reinterpret_cast<const uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(d + static_cast<size_t>(n + c4) * 2) = bits;
+        } else if (args.out_kind == kRowF16) {
+          // a value beyond binary16's 65504 becomes an infinity here; the combine
+          // kernel reports it
+          const __half2 lo = __floats2half2_rn(value.x, value.y);
+          const __half2 hi = __floats2half2_rn(value.z, value.w);
+          uint2 bits;
+          bits.x = *reinterpret_cast<const uint32_t*>(&lo);
+          bits.y = *reinterpret_cast<const uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(d + static_cast<size_t>(n + c4) * 2) = bits;
+        } else {
+          *reinterpret_cast<float4*>(d + static_cast<size_t>(n + c4) * 4) = value;
+        }
+      }
+    }
+  }
+}
+
+}  // namespace nmoe

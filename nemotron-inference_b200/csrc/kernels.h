@@ -69,23 +69,16 @@ struct GemmArgs {
   int32_t segment_rows = 0;
   int32_t segment_slot0 = 0;
   int32_t* error = nullptr;           // device error slot (DeviceError)
-  // Timing experiments on the CTA-pair kernel only (results are WRONG when set):
-  // bit 0 the epilogue drains nothing, bit 1 no scale writes, bit 2 no operand loads,
-  // bit 3 no MMAs.  Every barrier handshake stays in place.
-  int32_t ablate = 0;
 };
 
 // Tile shapes compiled into the library.  The block scales of every MMA must
 // start on a 4-column TMEM boundary, so a weight tile stores its scales in
-// whole groups of 128 rows; BN = 128 makes that exact for the HBM-bound sizes.
+// whole groups of 128 rows.
 enum GemmVariant : int {
   kVariantPrefillUp = 0,    // BN 208, 128-row A box
   kVariantPrefillDown = 1,  // BN 192, 128-row A box
-  kVariantDecode = 2,       // BN 128, 32-row A box, deep pipeline
-  kVariantDecodeWide = 3,   // BN 128, 128-row A box
-  kVariantPairUp = 4,       // 256 x 176 over a CTA pair (cta_group::2), quantising epilogue
-  kVariantPairDown = 5,     // the same tile, row-storing epilogue
-  kVariantCount = 6,
+  kVariantPair = 2,         // 256 x 208 over a CTA pair (cta_group::2), both epilogues
+  kVariantCount = 3,
 };
 
 struct GemmVariantInfo {
@@ -101,14 +94,43 @@ struct GemmVariantInfo {
 // (the partial last K block of the weights) are used by every variant; the CTA-pair
 // variants also load the full weight K blocks through a map (`b_full`: the K-block-major
 // panels as [rows][128 B], no swizzle), so that both CTAs' copies can complete on the
-// leader's barrier.
+// leader's barrier; b_full: rows of eight weight rows' 128 bytes, 1024 bytes each).
 struct GemmMaps {
   CUtensorMap a;
   CUtensorMap b_tail;
   CUtensorMap b_full;
 };
 
+// Up to four GEMMs whose tiles one persistent launch walks in order (csrc/expert_stream.cu): the
+// batch sizes that are bound by reading the weights.
+constexpr int kStreamPhases = 4;
+constexpr int kStreamBoxes = 5;
+struct StreamPhase {
+  CUtensorMap a[kStreamBoxes];  // activation rows, boxes of 8, 16, 32, 64 and 128 rows
+  CUtensorMap b_tail;  // the partial last K block of the weights
+  GemmArgs gemm;
+  int32_t mode = kGemmUp;  // GemmMode
+  // per 128-row slot: finished up tiles are counted here, down tiles wait for `wait_target` of
+  // them (0 = their rows were complete before the launch)
+  int32_t* ready = nullptr;
+  int32_t wait_target = 0;
+};
+struct StreamArgs {
+  StreamPhase phase[kStreamPhases];
+  int32_t phases = 0;
+  int32_t tile_rows = 128;  // most rows a row tile holds: 32, 64 or 128
+  int32_t* error = nullptr;
+  // all `ready` words of the phases, zero between launches, and a CTA ticket behind which the last
+  // CTA zeroes them
+  int32_t* ready = nullptr;
+  int32_t ready_count = 0;
+  int32_t* finished = nullptr;
+};
+inline int stream_tile_rows(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, cudaStream_t stream);
+
 GemmVariantInfo gemm_variant_info(GemmVariant v);
+GemmVariantInfo stream_variant_info();
 cudaError_t launch_grouped_gemm(GemmVariant v, GemmMode mode, const GemmMaps& maps,
                                 const GemmArgs& args, int num_sms, cudaStream_t stream);
 

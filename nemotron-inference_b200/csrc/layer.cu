@@ -131,18 +131,18 @@ CUtensorMap make_bf16_map(const void* base, size_t rows, size_t cols, int box_ro
   return map;
 }
 
-// Bytes that are already in their shared-memory order, viewed as [rows][128 B]: box =
-// 128 bytes x box_rows, no swizzle.  The CTA-pair GEMM loads its weight panels through
-// such a map.
+// Bytes that are already in their shared-memory order, viewed as [rows][1024 B]: box = 1024 bytes x
+// box_rows, no swizzle.  The CTA-pair GEMM loads its weight panels through such a map, eight weight
+// rows of a K block at a time.
 CUtensorMap make_raw_map(const void* base, size_t rows, int box_rows) {
   NMOE_REQUIRE(reinterpret_cast<uintptr_t>(base) % 16 == 0, "tensor map base must be 16-byte aligned");
   CUtensorMap map;
-  const cuuint64_t dims[2] = {128u, rows};
-  const cuuint64_t strides[1] = {128u};
-  const cuuint32_t box[2] = {128u, static_cast<cuuint32_t>(box_rows)};
+  const cuuint64_t dims[2] = {256u, rows};
+  const cuuint64_t strides[1] = {1024u};
+  const cuuint32_t box[2] = {256u, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t elem_strides[2] = {1u, 1u};
   const CUresult rc = encode_tiled_fn()(
-      &map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box,
+      &map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box,
       elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) {
@@ -188,9 +188,10 @@ void validate_matrix(const nmoe_nvfp4_matrix& m, size_t rows, size_t cols, const
 // A stack of same-shaped NVFP4 matrices resident in HBM with the scale layouts
 // and tensor maps of every GEMM tile shape that may consume it.
 // ---------------------------------------------------------------------------
-// kClassPair: 256 x 176 tiles over CTA pairs (cta_group::2), each CTA staging half of the
-// weight tile; measured slower than the single-CTA shapes, selected only by NMOE_GEMM_PAIR.
-enum TileClass : int { kClassPrefill = 0, kClassDecode = 1, kClassDecodeWide = 2, kClassPair = 3 };
+// kClassPair: 256 x 208 tiles over CTA pairs (cta_group::2), each CTA staging half of the
+// weight tile.
+// kClassStream: csrc/expert_stream.cu, the batches bound by reading the weights.
+enum TileClass : int { kClassPrefill = 0, kClassStream = 1, kClassPair = 2 };
 
 struct WeightStack {
   int experts = 0;
@@ -204,18 +205,15 @@ struct WeightStack {
   int kb_full = 0;
   DeviceBuffer tensor_scale;  // [experts]
   DeviceBuffer sf_prefill;    // scale layout for the prefill tile of this projection
-  DeviceBuffer sf_decode;     // scale layout for the BN=128 tiles
+  DeviceBuffer sf_stream;     // scale layout for the BN=128 tiles
   DeviceBuffer sf_pair;       // scale layout for the CTA-pair tile
   GemmVariant prefill_variant = kVariantPrefillUp;
-  GemmVariant decode_variant = kVariantDecode;
-  GemmVariant decode_wide_variant = kVariantDecodeWide;
-  GemmVariant pair_variant = kVariantPairUp;
   // tensor maps exist only for the partial last K block; full K blocks are
   // plain bulk copies of contiguous, pre-swizzled panels
   CUtensorMap tail_prefill;
-  CUtensorMap tail_decode;
+  CUtensorMap tail_stream;
   CUtensorMap tail_pair;
-  CUtensorMap full_pair;  // the K-block-major panels as [rows][128 B], for the CTA-pair variants
+  CUtensorMap full_pair;  // the K-block-major panels as [rows][1024 B], for the CTA-pair variant
 
   void upload(const nmoe_nvfp4_matrix* matrices, int count, int rows, int cols, bool is_up,
               const char* name, cudaStream_t stream) {
@@ -223,20 +221,19 @@ struct WeightStack {
     n = rows;
     k = cols;
     prefill_variant = is_up ? kVariantPrefillUp : kVariantPrefillDown;
-    pair_variant = is_up ? kVariantPairUp : kVariantPairDown;
     const size_t packed_each = static_cast<size_t>(rows) * cols / 2;
     const size_t sf_each = static_cast<size_t>(rows) * (cols / 16);
     tensor_scale.allocate(sizeof(float) * count);
     for (int e = 0; e < count; ++e) validate_matrix(matrices[e], rows, cols, name);
     const GemmVariantInfo pi = gemm_variant_info(prefill_variant);
-    const GemmVariantInfo di = gemm_variant_info(decode_variant);
-    const int pair_rows = gemm_variant_info(pair_variant).b_rows;
+    const GemmVariantInfo di = stream_variant_info();
+    const int pair_rows = gemm_variant_info(kVariantPair).b_rows;
     const size_t sf_prefill_each = weight_scale_layout_bytes(1, rows, cols, pi.bn, pi.sfb_groups);
-    const size_t sf_decode_each = weight_scale_layout_bytes(1, rows, cols, di.bn, di.sfb_groups);
-    const GemmVariantInfo qi = gemm_variant_info(pair_variant);
+    const size_t sf_stream_each = weight_scale_layout_bytes(1, rows, cols, di.bn, di.sfb_groups);
+    const GemmVariantInfo qi = gemm_variant_info(kVariantPair);
     const size_t sf_pair_each = weight_scale_layout_bytes(1, rows, cols, qi.bn, qi.sfb_groups);
     sf_prefill.allocate(sf_prefill_each * count);
-    sf_decode.allocate(sf_decode_each * count);
+    sf_stream.allocate(sf_stream_each * count);
     sf_pair.allocate(sf_pair_each * count);
     kb_full = cols / 256;
     const int tail_bytes = (cols % 256) / 2;
@@ -252,7 +249,7 @@ struct WeightStack {
       packed_tail.allocate(panel_rows * tail_pitch);
       try {
         tail_prefill = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pi.bn);
-        tail_decode = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, di.bn);
+        tail_stream = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, di.bn);
         tail_pair = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pair_rows);
       } catch (const Failure&) {
         narrow_tail = false;
@@ -262,7 +259,7 @@ struct WeightStack {
       tail_pitch = 128;
       packed_tail.allocate(panel_rows * tail_pitch, true);
       tail_prefill = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pi.bn);
-      tail_decode = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, di.bn);
+      tail_stream = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, di.bn);
       tail_pair = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pair_rows);
     }
     if (tail_bytes == 0) {
@@ -293,7 +290,7 @@ struct WeightStack {
                                        pi.sfb_groups, sf_prefill.as<uint8_t>() + sf_prefill_each * e,
                                        stream));
       NMOE_CUDA(relayout_weight_scales(staging_sf.as<uint8_t>(), 1, rows, cols, di.bn,
-                                       di.sfb_groups, sf_decode.as<uint8_t>() + sf_decode_each * e,
+                                       di.sfb_groups, sf_stream.as<uint8_t>() + sf_stream_each * e,
                                        stream));
       NMOE_CUDA(relayout_weight_scales(staging_sf.as<uint8_t>(), 1, rows, cols, qi.bn,
                                        qi.sfb_groups, sf_pair.as<uint8_t>() + sf_pair_each * e,
@@ -301,28 +298,29 @@ struct WeightStack {
     }
     NMOE_CUDA(cudaStreamSynchronize(stream));  // the staging buffers die here
     if (kb_full > 0) {
-      full_pair = make_raw_map(packed.as<uint8_t>(), panel_rows * kb_full + 256, pair_rows);
+      full_pair = make_raw_map(packed.as<uint8_t>(), (panel_rows * kb_full + 256) / 8, pair_rows / 8);
     } else {
-      full_pair = make_raw_map(packed.as<uint8_t>(), 256, pair_rows);  // never read
+      full_pair = make_raw_map(packed.as<uint8_t>(), 256 / 8, pair_rows / 8);  // never read
     }
     if (tail_bytes == 0) {
       // never read (k_blocks == kb_full), but the kernel takes a valid map
       tail_prefill = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, pi.bn);
-      tail_decode = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, di.bn);
+      tail_stream = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, di.bn);
       tail_pair = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, pair_rows);
     }
   }
 
   GemmVariant variant(TileClass c) const {
-    return c == kClassPrefill ? prefill_variant
-           : c == kClassPair  ? pair_variant
-           : c == kClassDecode ? decode_variant : decode_wide_variant;
+    return c == kClassPair ? kVariantPair : prefill_variant;
   }
   const CUtensorMap& tail_map(TileClass c) const {
-    return c == kClassPrefill ? tail_prefill : c == kClassPair ? tail_pair : tail_decode;
+    return c == kClassPrefill ? tail_prefill : c == kClassPair ? tail_pair : tail_stream;
   }
   const uint8_t* sf(TileClass c) const {
-    return (c == kClassPrefill ? sf_prefill : c == kClassPair ? sf_pair : sf_decode).as<uint8_t>();
+    return (c == kClassPrefill ? sf_prefill : c == kClassPair ? sf_pair : sf_stream).as<uint8_t>();
+  }
+  int tile_cols(TileClass c) const {
+    return c == kClassStream ? stream_variant_info().bn : gemm_variant_info(variant(c)).bn;
   }
 };
 
@@ -330,36 +328,26 @@ struct WeightStack {
 struct ActivationOperand {
   const uint8_t* packed = nullptr;
   const uint8_t* sf_tiled = nullptr;
-  CUtensorMap map_box128;
-  CUtensorMap map_box32;
+  CUtensorMap boxes[kStreamBoxes];  // 8, 16, 32, 64 and 128 rows
   void bind(const uint8_t* packed_rows, const uint8_t* sf, size_t rows, int k) {
     packed = packed_rows;
     sf_tiled = sf;
-    map_box128 = make_packed_map(packed_rows, rows, static_cast<size_t>(k) / 2, 128);
-    map_box32 = make_packed_map(packed_rows, rows, static_cast<size_t>(k) / 2, 32);
+    for (int i = 0; i < kStreamBoxes; ++i) {
+      boxes[i] = make_packed_map(packed_rows, rows, static_cast<size_t>(k) / 2, 8 << i);
+    }
   }
-  const CUtensorMap& map(TileClass c) const { return c == kClassDecode ? map_box32 : map_box128; }
 };
-
 
 GemmMaps gemm_maps(const WeightStack& weights, TileClass tile_class, const ActivationOperand& a) {
   GemmMaps maps;
-  maps.a = a.map(tile_class);
+  maps.a = a.boxes[kStreamBoxes - 1];
   maps.b_tail = weights.tail_map(tile_class);
   maps.b_full = weights.full_pair;
   return maps;
 }
 
-// NMOE_GEMM_ABLATE: timing experiments only (GemmArgs::ablate); results are wrong when set.
-int gemm_ablation() {
-  static const int value = [] {
-    const char* env = std::getenv("NMOE_GEMM_ABLATE");
-    return env != nullptr ? std::atoi(env) : 0;
-  }();
-  return value;
-}
-
 struct Schedule {
+  int most_rows = 128;  // no row tile holds more
   const RowTile* row_tiles = nullptr;  // grouped when non-null
   const int32_t* num_row_tiles = nullptr;
   int dense_rows = 0;
@@ -373,81 +361,173 @@ struct RowSegments {
   int slot0 = 0;
 };
 
-// One GEMM with the row-storing epilogue: rows = A x W^T times the tensor scales
+// What every GEMM of a tile class takes from its weights, activations and schedule.
+GemmArgs gemm_args(const WeightStack& weights, TileClass tile_class, const ActivationOperand& a,
+                   const float* a_tensor_scale, const Schedule& schedule, int32_t* error) {
+  GemmArgs g;
+  const int bn = weights.tile_cols(tile_class);
+  g.K = weights.k;
+  g.N = weights.n;
+  g.n_tiles = (weights.n + bn - 1) / bn;
+  g.k_blocks = k_blocks_of(weights.k);
+  g.kb_full = weights.kb_full;
+  g.b_full = weights.packed.as<uint8_t>();
+  g.sfa = a.sf_tiled;
+  g.sfb = weights.sf(tile_class);
+  g.a_tensor_scale = a_tensor_scale;
+  g.w_tensor_scale = weights.tensor_scale.as<float>();
+  g.row_tiles = schedule.row_tiles;
+  g.num_row_tiles = schedule.num_row_tiles;
+  g.dense_rows = schedule.dense_rows;
+  g.error = error;
+  return g;
+}
+
+// The row-storing epilogue's side of a down projection: rows = A x W^T times the tensor scales
 // [x routing weight] [-> relu^2], scattered by dest_row.
+struct RowOutput {
+  void* rows = nullptr;
+  RowKind kind = kRowF32;
+  const int32_t* dest_row = nullptr;
+  int dest_mul = 1;
+  int dest_add = 0;
+  const float* row_weight = nullptr;
+  bool relu2 = false;
+  RowSegments segments;
+};
+
+void set_row_output(GemmArgs* g, const RowOutput& out) {
+  g->out_rows = out.rows;
+  g->out_kind = out.kind;
+  g->dest_row = out.dest_row;
+  g->dest_mul = out.dest_mul;
+  g->dest_add = out.dest_add;
+  g->row_weight = out.row_weight;
+  g->relu2 = out.relu2 ? 1 : 0;
+  g->out_segments = out.segments.bases;
+  g->segment_rows = out.segments.rows;
+  g->segment_slot0 = out.segments.slot0;
+}
+
+// The quantising epilogue's side of an up projection.
+void set_hidden_output(GemmArgs* g, uint8_t* hidden_packed, uint8_t* hidden_sf) {
+  g->out_packed = hidden_packed;
+  g->out_sf = hidden_sf;
+  g->out_k_blocks = k_blocks_of(g->N);
+}
+
+void set_phase(StreamPhase* phase, GemmMode mode, const WeightStack& weights,
+               const ActivationOperand& a, const GemmArgs& g) {
+  for (int i = 0; i < kStreamBoxes; ++i) phase->a[i] = a.boxes[i];
+  phase->b_tail = weights.tail_map(kClassStream);
+  phase->gemm = g;
+  phase->mode = mode;
+}
+
+void run_gemm(GemmMode mode, const WeightStack& weights, TileClass tile_class,
+              const ActivationOperand& a, const GemmArgs& g, int most_rows, int num_sms,
+              cudaStream_t stream) {
+  if (tile_class != kClassStream) {
+    NMOE_CUDA(launch_grouped_gemm(weights.variant(tile_class), mode,
+                                  gemm_maps(weights, tile_class, a), g, num_sms, stream));
+    return;
+  }
+  StreamArgs args;
+  set_phase(&args.phase[0], mode, weights, a, g);
+  args.phases = 1;
+  args.tile_rows = stream_tile_rows(most_rows);
+  args.error = g.error;
+  NMOE_CUDA(launch_expert_stream(args, num_sms, stream));
+}
+
 void run_down_gemm(const WeightStack& weights, TileClass tile_class, const ActivationOperand& a,
-                   const float* a_tensor_scale, const Schedule& schedule, void* out_rows,
-                   const int32_t* dest_row, int dest_mul, int dest_add, const float* row_weight,
-                   bool relu2, int32_t* error, int num_sms, cudaStream_t stream, RowKind out_kind,
-                   RowSegments segments) {
-  GemmArgs d;
-  const GemmVariant variant = weights.variant(tile_class);
-  const int bn = gemm_variant_info(variant).bn;
-  d.K = weights.k;
-  d.N = weights.n;
-  d.n_tiles = (weights.n + bn - 1) / bn;
-  d.k_blocks = k_blocks_of(weights.k);
-  d.kb_full = weights.kb_full;
-  d.b_full = weights.packed.as<uint8_t>();
-  d.sfa = a.sf_tiled;
-  d.sfb = weights.sf(tile_class);
-  d.a_tensor_scale = a_tensor_scale;
-  d.w_tensor_scale = weights.tensor_scale.as<float>();
-  d.row_tiles = schedule.row_tiles;
-  d.num_row_tiles = schedule.num_row_tiles;
-  d.dense_rows = schedule.dense_rows;
-  d.out_rows = out_rows;
-  d.out_kind = out_kind;
-  d.dest_row = dest_row;
-  d.dest_mul = dest_mul;
-  d.dest_add = dest_add;
-  d.row_weight = row_weight;
-  d.relu2 = relu2 ? 1 : 0;
-  d.out_segments = segments.bases;
-  d.segment_rows = segments.rows;
-  d.segment_slot0 = segments.slot0;
-  d.error = error;
-  d.ablate = gemm_ablation();
-  NMOE_CUDA(launch_grouped_gemm(variant, kGemmDown, gemm_maps(weights, tile_class, a), d, num_sms,
-                                stream));
+                   const float* a_tensor_scale, const Schedule& schedule, const RowOutput& out,
+                   int32_t* error, int num_sms, cudaStream_t stream) {
+  GemmArgs d = gemm_args(weights, tile_class, a, a_tensor_scale, schedule, error);
+  set_row_output(&d, out);
+  run_gemm(kGemmDown, weights, tile_class, a, d, schedule.most_rows, num_sms, stream);
+}
+
+// One expert FFN of a launch of csrc/expert_stream.cu: up (relu^2 + quantise, tensor scale 1) ->
+// down.  Without `up` the hidden rows are complete before the launch.
+struct StreamFfn {
+  const WeightStack* up = nullptr;
+  const WeightStack* down = nullptr;
+  const ActivationOperand* a = nullptr;
+  const float* a_tensor_scale = nullptr;
+  Schedule schedule;
+  uint8_t* hidden_packed = nullptr;
+  uint8_t* hidden_sf = nullptr;
+  const ActivationOperand* hidden = nullptr;
+  const float* hidden_tensor_scale = nullptr;
+  RowOutput out;
+  int row_slots = 0;  // most 128-row slots the schedule may use
+};
+
+// Row slots' completion counts of such launches; zero whenever no launch is running.
+struct StreamCounts {
+  DeviceBuffer words;  // one ticket, then the counts
+  int capacity = 0;
+  void allocate(size_t slots) {
+    capacity = static_cast<int>(slots);
+    words.allocate((slots + 1) * sizeof(int32_t), true);
+  }
+};
+
+// The shared expert comes first among the up projections and among the down projections: its down
+// tiles are the longest, and short ones end together.
+void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCounts& counts,
+                int32_t* error, int num_sms, cudaStream_t stream) {
+  StreamArgs args;
+  args.error = error;
+  args.finished = counts.words.as<int32_t>();
+  args.ready = counts.words.as<int32_t>() + 1;
+  auto add = [&](const StreamFfn& ffn, bool up, int32_t* ready) {
+    StreamPhase* phase = &args.phase[args.phases++];
+    const WeightStack& weights = up ? *ffn.up : *ffn.down;
+    const ActivationOperand& a = up ? *ffn.a : *ffn.hidden;
+    GemmArgs g = gemm_args(weights, kClassStream, a, up ? ffn.a_tensor_scale : ffn.hidden_tensor_scale,
+                           ffn.schedule, error);
+    if (up) {
+      set_hidden_output(&g, ffn.hidden_packed, ffn.hidden_sf);
+    } else {
+      set_row_output(&g, ffn.out);
+    }
+    set_phase(phase, up ? kGemmUp : kGemmDown, weights, a, g);
+    if (ffn.up != nullptr) {
+      phase->ready = ready;
+      if (!up) {
+        const int bn = stream_variant_info().bn;
+        phase->wait_target = (ffn.up->n + bn - 1) / bn;
+      }
+    }
+  };
+  int32_t* routed_ready = args.ready;
+  int32_t* shared_ready = args.ready + (routed != nullptr ? routed->row_slots : 0);
+  args.ready_count = (routed != nullptr ? routed->row_slots : 0) +
+                     (shared != nullptr ? shared->row_slots : 0);
+  NMOE_REQUIRE(args.ready_count <= counts.capacity, "row slots of the fused experts");
+  if (shared != nullptr && shared->up != nullptr) add(*shared, true, shared_ready);
+  if (routed != nullptr) add(*routed, true, routed_ready);
+  if (shared != nullptr) add(*shared, false, shared_ready);
+  if (routed != nullptr) add(*routed, false, routed_ready);
+  args.tile_rows = stream_tile_rows(std::max(routed != nullptr ? routed->schedule.most_rows : 0,
+                                             shared != nullptr ? shared->schedule.most_rows : 0));
+  NMOE_CUDA(launch_expert_stream(args, num_sms, stream));
 }
 
 // up GEMM (relu^2 + quantise) followed by down GEMM (scale, weight, scatter).
 void run_expert_gemms(const WeightStack& up, const WeightStack& down, TileClass tile_class,
                       const ActivationOperand& a, const float* a_tensor_scale,
                       const Schedule& schedule, uint8_t* hidden_packed, uint8_t* hidden_sf,
-                      const ActivationOperand& hidden, void* out_rows, const int32_t* dest_row,
-                      int dest_mul, int dest_add, const float* row_weight, int32_t* error,
-                      int num_sms, cudaStream_t stream, cudaEvent_t between = nullptr,
-                      RowKind out_kind = kRowF32, RowSegments segments = RowSegments()) {
-  GemmArgs g;
-  const GemmVariant up_variant = up.variant(tile_class);
-  g.K = up.k;
-  g.N = up.n;
-  g.n_tiles = (up.n + gemm_variant_info(up_variant).bn - 1) / gemm_variant_info(up_variant).bn;
-  g.k_blocks = k_blocks_of(up.k);
-  g.kb_full = up.kb_full;
-  g.b_full = up.packed.as<uint8_t>();
-  g.sfa = a.sf_tiled;
-  g.sfb = up.sf(tile_class);
-  g.a_tensor_scale = a_tensor_scale;
-  g.w_tensor_scale = up.tensor_scale.as<float>();
-  g.row_tiles = schedule.row_tiles;
-  g.num_row_tiles = schedule.num_row_tiles;
-  g.dense_rows = schedule.dense_rows;
-  g.out_packed = hidden_packed;
-  g.out_sf = hidden_sf;
-  g.out_k_blocks = k_blocks_of(up.n);
-  g.error = error;
-  g.ablate = gemm_ablation();
-  NMOE_CUDA(launch_grouped_gemm(up_variant, kGemmUp, gemm_maps(up, tile_class, a), g, num_sms,
-                                stream));
-
+                      const ActivationOperand& hidden, const RowOutput& out, int32_t* error,
+                      int num_sms, cudaStream_t stream, cudaEvent_t between = nullptr) {
+  GemmArgs g = gemm_args(up, tile_class, a, a_tensor_scale, schedule, error);
+  set_hidden_output(&g, hidden_packed, hidden_sf);
+  run_gemm(kGemmUp, up, tile_class, a, g, schedule.most_rows, num_sms, stream);
   if (between != nullptr) cudaEventRecord(between, stream);
-
   // the fused quantiser always uses tensor scale 1
-  run_down_gemm(down, tile_class, hidden, nullptr, schedule, out_rows, dest_row, dest_mul,
-                dest_add, row_weight, false, error, num_sms, stream, out_kind, segments);
+  run_down_gemm(down, tile_class, hidden, nullptr, schedule, out, error, num_sms, stream);
 }
 
 nmoe_status status_from_device(int code) {
@@ -663,6 +743,10 @@ using namespace nmoe;
 // ===========================================================================
 // nmoe_ffn
 // ===========================================================================
+// Rows of one FFN up to which its weights are read once per 128 rows (the tiles of a prefill shape
+// are too few to fill the GPU until there are many row tiles).
+constexpr int kStreamFfnRows = 256;
+
 struct nmoe_ffn {
   int hidden = 0;
   int inter = 0;
@@ -671,6 +755,7 @@ struct nmoe_ffn {
   WeightStack up, down;
   DeviceBuffer a_packed, a_sf, a_ts, h_packed, h_sf;
   ActivationOperand a_op, h_op;
+  StreamCounts stream_counts;
   ErrorSlot error;
   int last_rows = 0;
   std::string last_error;
@@ -715,6 +800,7 @@ nmoe_status nmoe_ffn_create(const nmoe_nvfp4_matrix* up, const nmoe_nvfp4_matrix
     f->h_sf.allocate(tiled_sf_bytes(slots, f->inter), true);
     f->a_op.bind(f->a_packed.as<uint8_t>(), f->a_sf.as<uint8_t>(), slots * 128, f->hidden);
     f->h_op.bind(f->h_packed.as<uint8_t>(), f->h_sf.as<uint8_t>(), slots * 128, f->inter);
+    f->stream_counts.allocate(slots);
     f->error.create();
     NMOE_CUDA(cudaDeviceSynchronize());
   } catch (const Failure& failure) {
@@ -736,19 +822,39 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
   if (rows > ffn->max_rows) return NMOE_ERR_CAPACITY;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   try {
-    TileClass tile_class = rows <= 32 ? kClassDecode : rows <= 256 ? kClassDecodeWide : kClassPrefill;
-    if (gemm_variant >= 1 && gemm_variant <= 4) tile_class = static_cast<TileClass>(gemm_variant - 1);
-    if (tile_class == kClassDecode && rows > 32) return NMOE_ERR_INVALID_ARGUMENT;
+    if (gemm_variant == 2 && rows > 32) return NMOE_ERR_INVALID_ARGUMENT;
+    const TileClass tile_class = gemm_variant == 1   ? kClassPrefill
+                                 : gemm_variant == 4 ? kClassPair
+                                 : gemm_variant != 0 || rows <= kStreamFfnRows ? kClassStream
+                                                                               : kClassPrefill;
     NMOE_CUDA(launch_norm_quant(input, input_dtype == NMOE_BF16, static_cast<int>(rows),
                                 ffn->hidden, nullptr, 0.0f, nullptr, ffn->a_packed.as<uint8_t>(),
                                 nullptr, ffn->a_sf.as<uint8_t>(), k_blocks_of(ffn->hidden),
                                 ffn->a_ts.as<float>(), stream));
     Schedule schedule;
     schedule.dense_rows = static_cast<int>(rows);
-    run_expert_gemms(ffn->up, ffn->down, tile_class, ffn->a_op, ffn->a_ts.as<float>(), schedule,
-                     ffn->h_packed.as<uint8_t>(), ffn->h_sf.as<uint8_t>(), ffn->h_op, output,
-                     nullptr, 1, 0, nullptr, ffn->error.device.as<int32_t>(), ffn->num_sms,
-                     stream);
+    schedule.most_rows = std::min(128, static_cast<int>(rows));
+    RowOutput out;
+    out.rows = output;
+    int32_t* error = ffn->error.device.as<int32_t>();
+    if (tile_class == kClassStream) {
+      StreamFfn both;
+      both.up = &ffn->up;
+      both.down = &ffn->down;
+      both.a = &ffn->a_op;
+      both.a_tensor_scale = ffn->a_ts.as<float>();
+      both.schedule = schedule;
+      both.hidden_packed = ffn->h_packed.as<uint8_t>();
+      both.hidden_sf = ffn->h_sf.as<uint8_t>();
+      both.hidden = &ffn->h_op;
+      both.out = out;
+      both.row_slots = (static_cast<int>(rows) + 127) / 128;
+      run_stream(nullptr, &both, ffn->stream_counts, error, ffn->num_sms, stream);
+    } else {
+      run_expert_gemms(ffn->up, ffn->down, tile_class, ffn->a_op, ffn->a_ts.as<float>(), schedule,
+                       ffn->h_packed.as<uint8_t>(), ffn->h_sf.as<uint8_t>(), ffn->h_op, out, error,
+                       ffn->num_sms, stream);
+    }
     ffn->last_rows = static_cast<int>(rows);
   } catch (const Failure& failure) {
     ffn->last_error = failure.message;
@@ -789,7 +895,6 @@ struct nmoe_layer {
   int local_experts = 0;
   int first_local_expert = 0;
   int max_row_tiles = 0;
-  int decode_pairs_limit = 0;
 
   DeviceBuffer norm_weight, gate, bias, logit_offset;
   ExactOperand gate_exact;  // the router's FP64 logits of small batches
@@ -878,6 +983,7 @@ struct nmoe_layer {
   } window;
 
   ActivationOperand y_op, sh_op, a_op, h_op;
+  StreamCounts stream_counts;
   ErrorSlot error;
   int last_tokens = 0;
   std::string last_error;
@@ -994,20 +1100,17 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
     L->parts.allocate(T * (K + 1) * static_cast<size_t>(std::max(H, Lr)) * sizeof(float));
   }
 
-  // Row tiles: every expert may leave one partly filled slot.  Small batches
-  // use 32-row tiles (decode tile class), large ones 128-row tiles.
+  // Row tiles: every expert may leave one partly filled slot of 128 rows.
   // With expert parallelism the rows come from every rank: the capacity is
   // max_recv_pairs (default: twice the local pairs, i.e. 2x the uniform share).
-  L->decode_pairs_limit = 32 * EL;
   const size_t local_pairs = T * K;
   const size_t pairs = L->ep_world == 1 ? local_pairs
                        : c.max_recv_pairs > 0 ? static_cast<size_t>(c.max_recv_pairs)
                                               : 2 * local_pairs;
   L->max_pairs = static_cast<int64_t>(pairs);
   // (an expert may leave a partly filled slot, and an empty one when pairs consume them)
-  const size_t tiles_prefill = 2 * static_cast<size_t>(EL) + (pairs + 127) / 128;
-  const size_t tiles_decode = EL + (std::min<size_t>(pairs, L->decode_pairs_limit) + 31) / 32;
-  L->max_row_tiles = static_cast<int>(std::max(tiles_prefill, tiles_decode));
+  L->max_row_tiles = static_cast<int>(2 * static_cast<size_t>(EL) + (pairs + 127) / 128);
+  L->stream_counts.allocate(L->max_row_tiles + token_slots);
   const size_t slots = static_cast<size_t>(L->max_row_tiles);
   L->counts.allocate(E * sizeof(int32_t), true);
   L->cursor.allocate(E * sizeof(int32_t), true);
@@ -1285,50 +1388,66 @@ struct FfnBuffers {
 
 void run_ffn(nmoe_layer* L, bool unfused, const WeightStack& up, const WeightStack& down,
              TileClass tile_class, const ActivationOperand& a, const float* a_ts,
-             const Schedule& schedule, const FfnBuffers& buffers, void* out_rows,
-             const int32_t* dest_row, int dest_mul, int dest_add, const float* row_weight,
-             cudaStream_t stream, cudaEvent_t between, RowKind out_kind, RowSegments segments) {
+             const Schedule& schedule, const FfnBuffers& buffers, const RowOutput& out,
+             cudaStream_t stream, cudaEvent_t between) {
   int32_t* error = L->error.device.as<int32_t>();
   if (!unfused) {
     run_expert_gemms(up, down, tile_class, a, a_ts, schedule, buffers.hidden_packed,
-                     buffers.hidden_sf, *buffers.hidden, out_rows, dest_row, dest_mul, dest_add,
-                     row_weight, error, L->num_sms, stream, between, out_kind, segments);
+                     buffers.hidden_sf, *buffers.hidden, out, error, L->num_sms, stream, between);
     return;
   }
-  // the row-storing epilogue exists for the BN = 128 tile shapes
-  const TileClass raw_class =
-      tile_class == kClassPrefill || tile_class == kClassPair ? kClassDecodeWide : tile_class;
-  run_down_gemm(up, raw_class, a, a_ts, schedule, buffers.raw_rows, nullptr, 1, 0, nullptr,
-                /*relu2=*/true, error, L->num_sms, stream, kRowF32, RowSegments());
+  RowOutput raw;
+  raw.rows = buffers.raw_rows;
+  raw.relu2 = true;
+  run_down_gemm(up, kClassStream, a, a_ts, schedule, raw, error, L->num_sms, stream);
   NMOE_CUDA(launch_norm_quant(buffers.raw_rows, false, buffers.raw_row_count, up.n, nullptr, 0.0f,
                               nullptr, buffers.hidden_packed, nullptr, buffers.hidden_sf,
                               k_blocks_of(up.n), buffers.hidden_ts, stream));
   if (between != nullptr) cudaEventRecord(between, stream);
-  run_down_gemm(down, tile_class, *buffers.hidden, buffers.hidden_ts, schedule, out_rows, dest_row,
-                dest_mul, dest_add, row_weight, /*relu2=*/false, error, L->num_sms, stream,
-                out_kind, segments);
+  run_down_gemm(down, tile_class, *buffers.hidden, buffers.hidden_ts, schedule, out, error,
+                L->num_sms, stream);
 }
 
-// Plan + permute + the two grouped GEMMs over `pairs` (row, slot) pairs whose
-// per-local-expert histogram is already in `counts`.
+// Up to this many tokens the shared expert's tiles join the routed experts' launch; with more its
+// GEMMs are long enough to be worth running beside the router (512 tokens 199 against 203 us,
+// 1003 tokens 231 against 229, 2048 tokens 281 against 274).
+constexpr int kSharedInLaunchTokens = 640;
+
+// Routed rows per expert (on average) up to which csrc/expert_stream.cu takes them: 96 rows
+// measured 274 us for the whole pass against 276 with the prefill tiles, 47 rows 229 against 240,
+// 141 rows 451 against 371 (most experts then have a second row tile).  Up tiles of few K blocks
+// are over before the epilogue of a tile of many rows is (latent size 1024, 43 rows: up projection
+// 204 against 166 us), so there the line lies at the epilogue's short form.
+constexpr int kStreamRowsPerExpert = 100;
+constexpr int kStreamRowsShortTiles = 16;
+
+// Which kernel takes `pairs` routed rows.
+TileClass routed_tile_class(const nmoe_layer* L, int pairs) {
+  const int rows = k_blocks_of(L->latent) >= 6 ? kStreamRowsPerExpert : kStreamRowsShortTiles;
+  if (pairs <= L->local_experts * rows) return kClassStream;
+  const bool pair = L->pair_gemms && !L->unfused && (L->num_sms & 1) == 0 &&
+                    pairs / L->local_experts >= L->pair_min_rows;
+  return pair ? kClassPair : kClassPrefill;
+}
+
+// Plan + permute + the grouped GEMMs over `pairs` (row, slot) pairs whose per-local-expert
+// histogram is already in `counts`.  `shared` (stream class only): the shared expert's tiles join
+// the same launch.
 void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& source, int pairs,
                     int dest_stride, void* out_rows, RowKind out_kind,
-                    RowSegments segments = RowSegments()) {
+                    RowSegments segments = RowSegments(), const StreamFfn* shared = nullptr) {
   const int Lr = L->latent;
   int32_t* error = L->error.device.as<int32_t>();
-  const bool decode = static_cast<long long>(pairs) <= L->decode_pairs_limit / 2;
-  const bool pair = !decode && L->pair_gemms && !L->unfused && (L->num_sms & 1) == 0 &&
-                    pairs / L->local_experts >= L->pair_min_rows;
-  const TileClass routed_class = decode ? kClassDecode : pair ? kClassPair : kClassPrefill;
-  const int tile_rows = decode ? 32 : 128;
+  const TileClass routed_class = routed_tile_class(L, pairs);
+  constexpr int tile_rows = 128;
   PlanBuffers plan;
   plan.expert_counts = L->counts.as<int32_t>();
   plan.expert_cursor = L->cursor.as<int32_t>();
   plan.expert_slot0 = L->slot0.as<int32_t>();
   plan.row_tiles = L->row_tiles.as<RowTile>();
   plan.num_row_tiles = L->num_row_tiles.as<int32_t>();
-  NMOE_CUDA(launch_route_plan(plan, L->local_experts, tile_rows, pair ? 2 : 1, L->max_row_tiles,
-                              error, stream));
+  NMOE_CUDA(launch_route_plan(plan, L->local_experts, tile_rows, routed_class == kClassPair ? 2 : 1,
+                              L->max_row_tiles, error, stream));
   L->mark(4, stream);
   NMOE_CUDA(launch_permute(plan, source, pairs, L->local_experts, tile_rows, L->max_row_tiles, Lr,
                            k_blocks_of(Lr),
@@ -1341,68 +1460,137 @@ void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& sou
   Schedule routed;
   routed.row_tiles = L->row_tiles.as<RowTile>();
   routed.num_row_tiles = L->num_row_tiles.as<int32_t>();
+  // (a token selects an expert once)
+  routed.most_rows = L->ep_world == 1 ? std::min(128, pairs / L->cfg.top_k) : 128;
+  RowOutput out;
+  out.rows = out_rows;
+  out.kind = out_kind;
+  out.dest_row = L->a_dest.as<int32_t>();
+  out.row_weight = L->a_weight.as<float>();
+  out.segments = segments;
+  if (routed_class == kClassStream && !L->unfused && !L->stage_timing) {
+    StreamFfn ffn;
+    ffn.up = &L->up;
+    ffn.down = &L->down;
+    ffn.a = &L->a_op;
+    ffn.a_tensor_scale = L->a_ts.as<float>();
+    ffn.schedule = routed;
+    ffn.hidden_packed = L->h_packed.as<uint8_t>();
+    ffn.hidden_sf = L->h_sf.as<uint8_t>();
+    ffn.hidden = &L->h_op;
+    ffn.out = out;
+    ffn.row_slots = L->max_row_tiles;
+    run_stream(&ffn, shared, L->stream_counts, error, L->num_sms, stream);
+    return;
+  }
   FfnBuffers buffers{L->h_packed.as<uint8_t>(), L->h_sf.as<uint8_t>(), L->h_ts.as<float>(),
                      &L->h_op, L->u_raw.as<float>(), L->max_row_tiles * 128};
   run_ffn(L, L->unfused, L->up, L->down, routed_class, L->a_op, L->a_ts.as<float>(), routed,
-          buffers, out_rows, L->a_dest.as<int32_t>(), 1, 0, L->a_weight.as<float>(), stream,
-          L->stage_timing ? L->stage_events[6] : nullptr, out_kind, segments);
+          buffers, out, stream, L->stage_timing ? L->stage_events[6] : nullptr);
   if (L->unfused && L->ep_world == 1 && pairs <= L->unweighted_tokens * L->cfg.top_k) {
     // the down_proj rows before the routing weight (routed_expert_outputs of the trace)
-    run_down_gemm(L->down, routed_class, L->h_op, L->h_ts.as<float>(), routed,
-                  L->unweighted_rows.as<float>(), L->a_dest.as<int32_t>(), 1, 0, nullptr, false,
-                  error, L->num_sms, stream, kRowF32, RowSegments());
+    RowOutput plain;
+    plain.rows = L->unweighted_rows.as<float>();
+    plain.dest_row = L->a_dest.as<int32_t>();
+    run_down_gemm(L->down, routed_class, L->h_op, L->h_ts.as<float>(), routed, plain, error,
+                  L->num_sms, stream);
   }
+}
+
+TileClass shared_tile_class(const nmoe_layer* L, int tokens) {
+  if (tokens <= kStreamFfnRows) return kClassStream;
+  return L->pair_gemms && (L->num_sms & 1) == 0 && tokens >= 1024 ? kClassPair : kClassPrefill;
+}
+
+// The shared expert's hidden rows in FP32: shared_up and relu^2 (:814-818, :956-964), by a dense /
+// scaled-FP8 linear or an NVFP4 GEMM.
+void shared_hidden_rows(nmoe_layer* L, cudaStream_t stream, int tokens) {
+  float* raw = L->shared_raw.as<float>();
+  if (L->shared_up_dense.present) {
+    run_linear(L, L->shared_up_dense, L->normalized.as<float>(), tokens, raw, /*relu2=*/true,
+               stream);
+    return;
+  }
+  Schedule shared;
+  shared.dense_rows = tokens;
+  shared.most_rows = std::min(128, tokens);
+  RowOutput out;
+  out.rows = raw;
+  out.relu2 = true;
+  run_down_gemm(L->shared_up, kClassStream, L->y_op, L->y_ts.as<float>(), shared, out,
+                L->error.device.as<int32_t>(), L->num_sms, stream);
+}
+
+// ... and quantised for an NVFP4 down projection, through the host linear's own packing step
+// (:981-1005).
+void quantise_shared_hidden(nmoe_layer* L, cudaStream_t stream, int tokens) {
+  const int S = L->cfg.shared_expert_intermediate_size;
+  NMOE_CUDA(launch_norm_quant(L->shared_raw.as<float>(), false, tokens, S, nullptr, 0.0f, nullptr,
+                              L->sh_packed.as<uint8_t>(), nullptr, L->sh_sf.as<uint8_t>(),
+                              k_blocks_of(S), L->sh_ts.as<float>(), stream));
 }
 
 // shared expert (:814-818, :956-964, :981-1005) on the token-order rows
 void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_rows, int dest_mul,
                    int dest_add, cudaEvent_t between, RowKind out_kind = kRowF32) {
-  const int H = L->cfg.hidden_size, S = L->cfg.shared_expert_intermediate_size;
-  const bool pair = L->pair_gemms && (L->num_sms & 1) == 0 && tokens >= 1024;
-  const TileClass shared_class = tokens <= 32    ? kClassDecode
-                                 : tokens <= 256 ? kClassDecodeWide
-                                 : pair          ? kClassPair
-                                                 : kClassPrefill;
+  const TileClass shared_class = shared_tile_class(L, tokens);
   Schedule shared;
   shared.dense_rows = tokens;
-  int32_t* error = L->error.device.as<int32_t>();
+  shared.most_rows = std::min(128, tokens);
+  RowOutput out;
+  out.rows = out_rows;
+  out.kind = out_kind;
+  out.dest_mul = dest_mul;
+  out.dest_add = dest_add;
   if (!L->shared_up_dense.present && !L->shared_down_dense.present) {
     FfnBuffers buffers{L->sh_packed.as<uint8_t>(), L->sh_sf.as<uint8_t>(), L->sh_ts.as<float>(),
                        &L->sh_op, L->shared_raw.as<float>(), tokens};
     run_ffn(L, L->unfused, L->shared_up, L->shared_down, shared_class, L->y_op,
-            L->y_ts.as<float>(), shared, buffers, out_rows, nullptr, dest_mul, dest_add, nullptr,
-            stream, between, out_kind, RowSegments());
+            L->y_ts.as<float>(), shared, buffers, out, stream, between);
     return;
   }
-  // shared_up -> FP32 rows -> relu^2 in place (:956-964)
-  float* raw = L->shared_raw.as<float>();
-  if (L->shared_up_dense.present) {
-    run_linear(L, L->shared_up_dense, L->normalized.as<float>(), tokens, raw, /*relu2=*/true,
-               stream);
-  } else {
-    run_down_gemm(L->shared_up,
-                  shared_class == kClassPrefill || shared_class == kClassPair ? kClassDecodeWide
-                                                                              : shared_class,
-                  L->y_op, L->y_ts.as<float>(), shared, raw, nullptr, 1, 0, nullptr, true, error,
-                  L->num_sms, stream, kRowF32, RowSegments());
-  }
+  shared_hidden_rows(L, stream, tokens);
   if (between != nullptr) cudaEventRecord(between, stream);
   if (L->shared_down_dense.present) {
     // dense / scaled-FP8 down projection (:1006-1045) straight from the FP32 rows;
     // only the latent data flow (FP32 rows of `hidden` per token) reaches this
     NMOE_REQUIRE(dest_mul == 1 && dest_add == 0 && out_kind == kRowF32,
                  "a dense shared_down writes FP32 token rows");
-    run_linear(L, L->shared_down_dense, raw, tokens, static_cast<float*>(out_rows), false, stream);
-    (void)H;
+    run_linear(L, L->shared_down_dense, L->shared_raw.as<float>(), tokens,
+               static_cast<float*>(out_rows), false, stream);
     return;
   }
-  // NVFP4 down projection through the host linear's own packing step (:981-1005)
-  NMOE_CUDA(launch_norm_quant(raw, false, tokens, S, nullptr, 0.0f, nullptr,
-                              L->sh_packed.as<uint8_t>(), nullptr, L->sh_sf.as<uint8_t>(),
-                              k_blocks_of(S), L->sh_ts.as<float>(), stream));
-  run_down_gemm(L->shared_down, shared_class, L->sh_op, L->sh_ts.as<float>(), shared, out_rows,
-                nullptr, dest_mul, dest_add, nullptr, false, error, L->num_sms, stream, out_kind,
-                RowSegments());
+  quantise_shared_hidden(L, stream, tokens);
+  run_down_gemm(L->shared_down, shared_class, L->sh_op, L->sh_ts.as<float>(), shared, out,
+                L->error.device.as<int32_t>(), L->num_sms, stream);
+}
+
+// The shared expert as part of the routed experts' launch (csrc/expert_stream.cu); rows of a dense
+// shared_up are made here, before it.
+StreamFfn shared_stream_ffn(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_rows,
+                            int dest_mul, int dest_add, RowKind out_kind) {
+  StreamFfn ffn;
+  ffn.down = &L->shared_down;
+  ffn.schedule.dense_rows = tokens;
+  ffn.schedule.most_rows = std::min(128, tokens);
+  ffn.hidden_packed = L->sh_packed.as<uint8_t>();
+  ffn.hidden_sf = L->sh_sf.as<uint8_t>();
+  ffn.hidden = &L->sh_op;
+  ffn.out.rows = out_rows;
+  ffn.out.kind = out_kind;
+  ffn.out.dest_mul = dest_mul;
+  ffn.out.dest_add = dest_add;
+  ffn.row_slots = (tokens + 127) / 128;
+  if (L->shared_up_dense.present) {
+    shared_hidden_rows(L, stream, tokens);
+    quantise_shared_hidden(L, stream, tokens);
+    ffn.hidden_tensor_scale = L->sh_ts.as<float>();
+  } else {
+    ffn.up = &L->shared_up;
+    ffn.a = &L->y_op;
+    ffn.a_tensor_scale = L->y_ts.as<float>();
+  }
+  return ffn;
 }
 
 PermuteSource local_source(nmoe_layer* L) {
@@ -1434,7 +1622,12 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   // read, and eight times finer than the bf16 the sum is rounded to in the end.
   const RowKind parts_kind = out_dtype == NMOE_BF16 && !L->force_fp32_parts && !L->latent_mode
                                  ? kRowF16 : kRowF32;
-  const bool fork = L->side_stream != nullptr && !L->stage_timing &&
+  // Small batches bound by reading the weights run both kinds of expert in one launch, the others
+  // fork the shared expert onto a stream of its own.
+  const bool one_launch = routed_tile_class(L, tokens * K) == kClassStream && !L->unfused &&
+                          !L->stage_timing && !L->shared_down_dense.present &&
+                          (L->latent_mode || tokens <= kSharedInLaunchTokens);
+  const bool fork = L->side_stream != nullptr && !L->stage_timing && !one_launch &&
                     tokens <= L->fork_max_tokens && !L->latent_mode && !dense_shared;
   const bool two_pass = L->fast_router && tokens >= L->fast_router_min_tokens;
   route_tokens(L, stream, input, in_dtype, tokens, fork ? L->quant_done : nullptr,
@@ -1457,11 +1650,18 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     source.sf = L->lat_sf_row_major.as<uint8_t>();
     source.sf_stride = static_cast<size_t>(Lr) / 16;
     source.tensor_scale = L->lat_ts.as<float>();
-    routed_experts(L, stream, source, tokens * K, K, L->parts.as<void>(), kRowF32);
-    L->mark(7, stream);
-    shared_expert(L, stream, tokens, L->shared_rows.as<void>(), 1, 0,
-                  L->stage_timing ? L->stage_events[8] : nullptr, kRowF32);
-    L->mark(9, stream);
+    if (one_launch) {
+      const StreamFfn shared =
+          shared_stream_ffn(L, stream, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
+      routed_experts(L, stream, source, tokens * K, K, L->parts.as<void>(), kRowF32, RowSegments(),
+                     &shared);
+    } else {
+      routed_experts(L, stream, source, tokens * K, K, L->parts.as<void>(), kRowF32);
+      L->mark(7, stream);
+      shared_expert(L, stream, tokens, L->shared_rows.as<void>(), 1, 0,
+                    L->stage_timing ? L->stage_events[8] : nullptr, kRowF32);
+      L->mark(9, stream);
+    }
     // routed sum in selection order (:951-953), fc2_latent (:1047-1053), mixer and
     // residual (:1064-1069)
     NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
@@ -1479,9 +1679,18 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     shared_expert(L, L->side_stream, tokens, L->parts.as<void>(), K + 1, K, nullptr, parts_kind);
     NMOE_CUDA(cudaEventRecord(L->shared_done, L->side_stream));
   }
-  routed_experts(L, stream, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind);
+  if (one_launch) {
+    const StreamFfn shared =
+        shared_stream_ffn(L, stream, tokens, L->parts.as<void>(), K + 1, K, parts_kind);
+    routed_experts(L, stream, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind,
+                   RowSegments(), &shared);
+  } else {
+    routed_experts(L, stream, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind);
+  }
   L->mark(7, stream);
-  if (fork) {
+  if (one_launch) {
+    // nothing left to wait for
+  } else if (fork) {
     NMOE_CUDA(cudaStreamWaitEvent(stream, L->shared_done, 0));
   } else {
     shared_expert(L, stream, tokens, L->parts.as<void>(), K + 1, K,

@@ -55,16 +55,6 @@ __device__ __forceinline__ float tensor_scale_from_amax(float amax) {
   return amax > kFp4Max * kFp8Max ? clamp_scale(__fdiv_rn(amax, kFp4Max * kFp8Max)) : 1.0f;
 }
 
-// Scale of a block before its rounding to E4M3 (nvfp4_packing.cpp:130-139): amax / (6 * ts),
-// given `reciprocal` = RN(1 / divisor).  Quotients too small for the residual to be exact are
-// below the smallest scale and clamped.
-__device__ __forceinline__ float block_scale(float block_max, float divisor, float reciprocal) {
-  if (!(block_max > 0.0f)) return 1.0f;
-  const bool exact = (__float_as_uint(divisor) & 0x007fffffu) != 0x007fffffu && block_max < 1.0e37f;
-  return clamp_scale(exact ? div_by_reciprocal(block_max, divisor, reciprocal)
-                           : __fdiv_rn(block_max, divisor));
-}
-
 // Codes of half a 16-element block (nvfp4_packing.cpp:140-153): x / divisor, IEEE-rounded, then
 // E2M1.  One reciprocal per block and a residual correction per value give the correctly rounded
 // quotient unless the divisor's significand is all ones (div_by_reciprocal), where the division
