@@ -517,10 +517,12 @@ __device__ __forceinline__ void tma_load_2d_pair_at(uint32_t smem_dst, const CUt
       : "memory");
 }
 
-// Arrive on an mbarrier by its shared::cluster address (this CTA's or the partner's).
+// Arrive on an mbarrier by its shared::cluster address (this CTA's or the partner's).  What it
+// hands on is tensor memory, whose accesses are complete (tcgen05.wait) and fenced
+// (tcgen05_fence_before) by then; releasing generic memory to the cluster as well
+// (.release.cluster) made every arrival wait about 1100 cycles.
 __device__ __forceinline__ void mbar_arrive_cluster_at(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar)
-               : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait_cluster_at(uint32_t bar, uint32_t parity) {

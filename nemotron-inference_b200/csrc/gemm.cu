@@ -616,7 +616,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1u;
         // both CTAs' epilogues have drained this accumulator
-        if (!mbar_wait_cluster(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
+        if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
           report_timeout(args.error, abort_flag);
           break;
         }
@@ -624,7 +624,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         const uint32_t d_tmem = tmem_base + acc * kPairBN;
         for (int kb = 0; kb < k_blocks; ++kb) {
           // the operands of both CTAs have landed and both have written this block's scales
-          if (!mbar_wait_cluster_at(full0 + stage * 8, phase)) {
+          if (!mbar_wait_at(full0 + stage * 8, phase)) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
