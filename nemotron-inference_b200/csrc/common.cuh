@@ -253,6 +253,33 @@ __device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity) {
   return mbar_try_wait_at(bar, parity) || mbar_wait_slow(bar, parity);
 }
 
+// A role that issues tensor-core or copy instructions runs them from ONE lane, but the loop around
+// them should be executed by the whole warp with warp-uniform values: their operands (descriptors,
+// addresses) live in uniform registers, and in code that only one lane reaches the compiler has to
+// move every operand there one by one (a K block of four MMAs and a commit took 690 cycles of
+// issue that way).
+template <typename T>
+__device__ __forceinline__ T warp_uniform(T value) {
+  return __shfl_sync(0xffffffffu, value, 0);
+}
+
+// True in one lane of the (converged) warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(elected));
+  return elected != 0;
+}
+
+// The bounded wait, by all lanes of a warp; the result is the same in all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_try_wait_at(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity));
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx_at(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");

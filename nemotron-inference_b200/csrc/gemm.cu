@@ -153,7 +153,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
   float* stage_base = reinterpret_cast<float*>(
       reinterpret_cast<uint8_t*>(full_bar) + C::BAR_BYTES);  // down epilogue staging
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int unit = static_cast<int>(blockIdx.x);
   const int units = static_cast<int>(gridDim.x);
@@ -182,46 +182,47 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
-  const int num_row_tiles =
-      args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128;
+  const int num_row_tiles = warp_uniform(
+      args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128);
   const int total_tiles = num_row_tiles * args.n_tiles;
   const int k_mmas = args.K / 64;
 
   if (warp == 0 || warp >= kScaleWarp + kScaleWarps) {
     // ------------------------------------------------------------- producers
     // Producer p loads the K blocks p, p + kProducers, ... of the CTA's sequence.
-    if (lane == 0) {
-      const int producer = warp == 0 ? 0 : warp - (kScaleWarp + kScaleWarps) + 1;
-      static_assert(kProducers <= C::STAGES, "a producer advances at most a ring at a time");
-      const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA),
-                     sfb0 = smem_u32(sSFB);
-      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
-      int stage = producer % C::STAGES;
-      uint32_t phase = 0;
-      int kb = producer;  // K block of the current tile this producer loads next
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units) {
-        const int rt = t / args.n_tiles;
-        const int nt = t - rt * args.n_tiles;
-        const TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, 0u);
-        const int expert = rows.expert;
-        const uint8_t* sfa_src =
-            args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * args.k_blocks * C::SFA_BYTES;
-        const uint8_t* sfb_src = args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) *
-                                                args.k_blocks * C::SFB_BYTES;
-        // weights are stored K-block-major: [expert][k block][row][128 B], then the
-        // partial last K block as [expert][row][tail bytes]
-        const int b_row = nt * C::BN;
-        const uint8_t* b_src =
-            args.b_full + (static_cast<size_t>(expert) * args.kb_full * args.N + b_row) * 128;
-        for (; kb < args.k_blocks; kb += kProducers) {
-          if (!mbar_wait_at(empty0 + stage * 8, phase ^ 1u)) {
-            report_timeout(args.error, abort_flag);
-            ok = false;
-            break;
-          }
+    const int producer = warp == 0 ? 0 : warp - (kScaleWarp + kScaleWarps) + 1;
+    static_assert(kProducers <= C::STAGES, "a producer advances at most a ring at a time");
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA),
+                   sfb0 = smem_u32(sSFB);
+    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+    int stage = producer % C::STAGES;
+    uint32_t phase = 0;
+    int kb = producer;  // K block of the current tile this producer loads next
+    bool ok = true;
+    for (int t = unit; t < total_tiles && ok; t += units) {
+      const int rt = t / args.n_tiles;
+      const int nt = t - rt * args.n_tiles;
+      TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, 0u);
+      rows.load_row0 = warp_uniform(rows.load_row0);
+      const int expert = warp_uniform(rows.expert);
+      const uint8_t* sfa_src =
+          args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * args.k_blocks * C::SFA_BYTES;
+      const uint8_t* sfb_src = args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) *
+                                              args.k_blocks * C::SFB_BYTES;
+      // weights are stored K-block-major: [expert][k block][row][128 B], then the
+      // partial last K block as [expert][row][tail bytes]
+      const int b_row = nt * C::BN;
+      const uint8_t* b_src =
+          args.b_full + (static_cast<size_t>(expert) * args.kb_full * args.N + b_row) * 128;
+      for (; kb < args.k_blocks; kb += kProducers) {
+        if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
+          report_timeout(args.error, abort_flag);
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           const uint32_t bar = full0 + stage * 8;
           mbar_arrive_expect_tx_at(bar, C::STAGE_TX);
           tma_load_2d_at(a0 + stage * C::A_BYTES, &tmap_a, kb * 128, rows.load_row0, bar);
@@ -234,146 +235,143 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
           }
           bulk_load_at(sfa0 + stage * C::SFA_BYTES, sfa_src + kb * C::SFA_BYTES, C::SFA_BYTES, bar);
           bulk_load_at(sfb0 + stage * C::SFB_BYTES, sfb_src + kb * C::SFB_BYTES, C::SFB_BYTES, bar);
-          stage += kProducers;
-          if (stage >= C::STAGES) {
-            stage -= C::STAGES;
-            phase ^= 1u;
-          }
         }
-        kb -= args.k_blocks;
+        stage += kProducers;
+        if (stage >= C::STAGES) {
+          stage -= C::STAGES;
+          phase ^= 1u;
+        }
       }
+      kb -= args.k_blocks;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_nvf4(C::BN);
-      const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
-      const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
-      const uint32_t empty0 = smem_u32(empty_bar), sf_ready0 = smem_u32(sf_ready_bar);
-      const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
-      int stage = 0;
-      int local = 0;
-      uint32_t sf_buf = 0, sf_phase = 0;
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units, ++local) {
-        const int acc = local & 1;
-        const uint32_t acc_phase = (local >> 1) & 1u;
-        // the epilogue has drained this accumulator
-        if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
+    constexpr uint32_t idesc = make_idesc_nvf4(C::BN);
+    const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
+    const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
+    const uint32_t empty0 = smem_u32(empty_bar), sf_ready0 = smem_u32(sf_ready_bar);
+    const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
+    int stage = 0;
+    int local = 0;
+    uint32_t sf_buf = 0, sf_phase = 0;
+    bool ok = true;
+    for (int t = unit; t < total_tiles && ok; t += units, ++local) {
+      const int acc = local & 1;
+      const uint32_t acc_phase = (local >> 1) & 1u;
+      // the epilogue has drained this accumulator
+      if (!mbar_wait_warp(smem_u32(&tmem_empty_bar[acc]), acc_phase ^ 1u)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      tcgen05_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * C::ACC_STRIDE;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        // this block's scales are in TMEM, and its operands had landed before they were copied
+        if (!mbar_wait_warp(sf_ready0 + sf_buf * 8, sf_phase)) {
           report_timeout(args.error, abort_flag);
+          ok = false;
           break;
         }
         tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * C::ACC_STRIDE;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          // this block's scales are in TMEM, and its operands had landed before they were copied
-          if (!mbar_wait_at(sf_ready0 + sf_buf * 8, sf_phase)) {
-            report_timeout(args.error, abort_flag);
-            ok = false;
-            break;
-          }
-          tcgen05_fence_after();
-          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * C::A_BYTES);
-          const uint64_t b_desc = advance_smem_desc(b_desc0, stage * C::B_BYTES);
-          const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
-          if (kb + 1 < k_blocks || last_mmas == 4) {
+        const uint64_t a_desc = advance_smem_desc(a_desc0, stage * C::A_BYTES);
+        const uint64_t b_desc = advance_smem_desc(b_desc0, stage * C::B_BYTES);
+        const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
+        const bool issue = elect_one();
+        if (issue && (kb + 1 < k_blocks || last_mmas == 4)) {
 #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) {
-              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                               advance_smem_desc(b_desc, kt * 32), idesc,
-                               sf_tmem + C::SFA_COL + 4 * kt,
-                               sf_tmem + C::SFB_COL + C::SFB_GS * kt,
-                               kt != 0 ? 1u : kb != 0 ? 1u : 0u);
-            }
-          } else {
-            for (int kt = 0; kt < last_mmas; ++kt) {
-              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                               advance_smem_desc(b_desc, kt * 32), idesc,
-                               sf_tmem + C::SFA_COL + 4 * kt,
-                               sf_tmem + C::SFB_COL + C::SFB_GS * kt, (kb | kt) != 0 ? 1u : 0u);
-            }
+          for (int kt = 0; kt < 4; ++kt) {
+            tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                             advance_smem_desc(b_desc, kt * 32), idesc,
+                             sf_tmem + C::SFA_COL + 4 * kt,
+                             sf_tmem + C::SFB_COL + C::SFB_GS * kt,
+                             kt != 0 ? 1u : kb != 0 ? 1u : 0u);
           }
-          // frees the stage for the producer and, SF_BUFS K blocks later, this block's scale
-          // columns for the copier
-          tcgen05_commit_at(empty0 + stage * 8);
-          if (++sf_buf == C::SF_BUFS) {
-            sf_buf = 0;
-            sf_phase ^= 1u;
+        } else if (issue) {
+          for (int kt = 0; kt < last_mmas; ++kt) {
+            tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                             advance_smem_desc(b_desc, kt * 32), idesc,
+                             sf_tmem + C::SFA_COL + 4 * kt,
+                             sf_tmem + C::SFB_COL + C::SFB_GS * kt, (kb | kt) != 0 ? 1u : 0u);
           }
-          if (++stage == C::STAGES) stage = 0;
         }
-        if (ok) {
-          tcgen05_commit(&tmem_full_bar[acc]);
+        // frees the stage for the producer and, SF_BUFS K blocks later, this block's scale
+        // columns for the copier
+        if (issue) tcgen05_commit_at(empty0 + stage * 8);
+        if (++sf_buf == C::SF_BUFS) {
+          sf_buf = 0;
+          sf_phase ^= 1u;
         }
+        if (++stage == C::STAGES) stage = 0;
       }
+      if (ok && elect_one()) tcgen05_commit(&tmem_full_bar[acc]);
     }
   } else if (warp >= kScaleWarp) {  // (the producers behind them are taken)
     // ------------------------------------------------------- block-scale copiers
     // The copies of one K block's scales into TMEM take longer to issue than
     // its MMAs; threads of their own let them run ahead of the MMA thread.
-    if (lane == 0) {
-      const int part = warp - kScaleWarp;
-      const uint64_t sfa_desc0 = make_smem_desc(smem_u32(sSFA), 0, 128, 0);
-      const uint64_t sfb_desc0 = make_smem_desc(smem_u32(sSFB), 0, 128, 0);
-      const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
-      const uint32_t sf_ready0 = smem_u32(sf_ready_bar);
-      const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
-      int stage = 0;
-      uint32_t phase = 0;
-      uint32_t sf_buf = 0;
-      // the scale columns written now were last read by the MMAs of the K block
-      // SF_BUFS iterations back; those MMAs also release that block's stage
-      int old_stage = 0;
-      uint32_t old_phase = 0;
-      int unread = C::SF_BUFS;  // buffers nothing has read yet
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units) {
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          bool ready = mbar_wait_at(full0 + stage * 8, phase);
-          if (unread > 0) {
-            --unread;
+    const int part = warp - kScaleWarp;
+    const uint64_t sfa_desc0 = make_smem_desc(smem_u32(sSFA), 0, 128, 0);
+    const uint64_t sfb_desc0 = make_smem_desc(smem_u32(sSFB), 0, 128, 0);
+    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+    const uint32_t sf_ready0 = smem_u32(sf_ready_bar);
+    const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t sf_buf = 0;
+    // the scale columns written now were last read by the MMAs of the K block
+    // SF_BUFS iterations back; those MMAs also release that block's stage
+    int old_stage = 0;
+    uint32_t old_phase = 0;
+    int unread = C::SF_BUFS;  // buffers nothing has read yet
+    bool ok = true;
+    for (int t = unit; t < total_tiles && ok; t += units) {
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        bool ready = mbar_wait_warp(full0 + stage * 8, phase);
+        if (unread > 0) {
+          --unread;
+        } else {
+          ready = ready && mbar_wait_warp(empty0 + old_stage * 8, old_phase);
+          if (++old_stage == C::STAGES) {
+            old_stage = 0;
+            old_phase ^= 1u;
+          }
+        }
+        if (!ready) {
+          report_timeout(args.error, abort_flag);
+          ok = false;
+          break;
+        }
+        tcgen05_fence_after();
+        const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * C::SFA_BYTES);
+        const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * C::SFB_BYTES);
+        const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
+        // a partial last K block needs the scales of the MMAs it issues only;
+        // the full block keeps its copies free of run-time predicates, which
+        // slow their issue down considerably
+        const bool issue = elect_one();
+        if (!issue) {
+        } else if (kb + 1 < k_blocks || last_mmas == 4) {
+          static_assert(kScaleWarps == 2, "one branch per copier");
+          if (part == 0) {
+            issue_scale_copies<C, 0>(sf_tmem, sfa_desc, sfb_desc);
           } else {
-            ready = ready && mbar_wait_at(empty0 + old_stage * 8, old_phase);
-            if (++old_stage == C::STAGES) {
-              old_stage = 0;
-              old_phase ^= 1u;
-            }
+            issue_scale_copies<C, 1>(sf_tmem, sfa_desc, sfb_desc);
           }
-          if (!ready) {
-            report_timeout(args.error, abort_flag);
-            ok = false;
-            break;
+        } else {
+          for (int c = part; c < last_mmas; c += kScaleWarps) {
+            tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFA_COL + 4 * c,
+                                      advance_smem_desc(sfa_desc, c * 512));
           }
-          tcgen05_fence_after();
-          const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * C::SFA_BYTES);
-          const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * C::SFB_BYTES);
-          const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
-          // a partial last K block needs the scales of the MMAs it issues only;
-          // the full block keeps its copies free of run-time predicates, which
-          // slow their issue down considerably
-          if (kb + 1 < k_blocks || last_mmas == 4) {
-            static_assert(kScaleWarps == 2, "one branch per copier");
-            if (part == 0) {
-              issue_scale_copies<C, 0>(sf_tmem, sfa_desc, sfb_desc);
-            } else {
-              issue_scale_copies<C, 1>(sf_tmem, sfa_desc, sfb_desc);
-            }
-          } else {
-            for (int c = part; c < last_mmas; c += kScaleWarps) {
-              tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFA_COL + 4 * c,
-                                        advance_smem_desc(sfa_desc, c * 512));
-            }
-            for (int c = part; c < last_mmas * (C::SFB_GS / 4); c += kScaleWarps) {
-              tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFB_COL + 4 * c,
-                                        advance_smem_desc(sfb_desc, c * 512));
-            }
+          for (int c = part; c < last_mmas * (C::SFB_GS / 4); c += kScaleWarps) {
+            tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFB_COL + 4 * c,
+                                      advance_smem_desc(sfb_desc, c * 512));
           }
-          tcgen05_commit_at(sf_ready0 + sf_buf * 8);
-          if (++sf_buf == C::SF_BUFS) sf_buf = 0;
-          if (++stage == C::STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        if (issue) tcgen05_commit_at(sf_ready0 + sf_buf * 8);
+        if (++sf_buf == C::SF_BUFS) sf_buf = 0;
+        if (++stage == C::STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
@@ -504,7 +502,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0u;
@@ -535,10 +533,10 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   __syncthreads();
   cluster_sync_all();  // the partner's barriers exist before anything arrives
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
-  const int num_row_tiles =
-      args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128;
+  const int num_row_tiles = warp_uniform(
+      args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128);
   const int row_units = (num_row_tiles + 1) / 2;
   const int total_tiles = row_units * args.n_tiles;
   const int k_blocks = args.k_blocks;
@@ -549,29 +547,30 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   if (warp == 0 || warp >= kScaleWarp + kPairScaleWarps) {
     // ------------------------------------------------------------- producers
     // Producer p loads the K blocks p, p + kPairProducers, ... of the CTA's sequence.
-    if (lane == 0) {
-      const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-      const uint32_t sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
-      int stage = warp == 0 ? 0 : warp - (kScaleWarp + kPairScaleWarps) + 1;
-      int kb = stage;  // K block of the current tile this producer loads next
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units) {
-        const int rt = t / args.n_tiles;
-        const int nt = t - rt * args.n_tiles;
-        const TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
-        const int expert = rows.expert;
-        const uint8_t* sfa_src =
-            args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * k_blocks * kPairSfaBytes;
-        const uint8_t* sfb_src =
-            args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) * k_blocks * kPairSfbBytes;
-        const int b_row = nt * kPairBN + static_cast<int>(cta_rank) * kPairBRows;
-        for (; kb < k_blocks; kb += kPairProducers) {
-          if (!mbar_wait_at(empty0 + stage * 8, phase ^ 1u)) {
-            report_timeout(args.error, abort_flag);
-            ok = false;
-            break;
-          }
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+    const uint32_t sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
+    int stage = warp == 0 ? 0 : warp - (kScaleWarp + kPairScaleWarps) + 1;
+    int kb = stage;  // K block of the current tile this producer loads next
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = unit; t < total_tiles && ok; t += units) {
+      const int rt = t / args.n_tiles;
+      const int nt = t - rt * args.n_tiles;
+      TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
+      rows.load_row0 = warp_uniform(rows.load_row0);
+      const int expert = warp_uniform(rows.expert);
+      const uint8_t* sfa_src =
+          args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * k_blocks * kPairSfaBytes;
+      const uint8_t* sfb_src =
+          args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) * k_blocks * kPairSfbBytes;
+      const int b_row = nt * kPairBN + static_cast<int>(cta_rank) * kPairBRows;
+      for (; kb < k_blocks; kb += kPairProducers) {
+        if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
+          report_timeout(args.error, abort_flag);
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           const uint32_t bar = leader_full0 + stage * 8, sf_bar = sf_full0 + stage * 8;
           mbar_arrive_expect_tx_at(sf_bar, kPairSfaBytes + kPairSfbBytes);
           bulk_load_at(sfa0 + stage * kPairSfaBytes, sfa_src + kb * kPairSfaBytes, kPairSfaBytes,
@@ -591,18 +590,18 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
             tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_tail, 0, expert * args.N + b_row,
                                 bar);
           }
-          stage += kPairProducers;
-          if (stage >= kPairStages) {
-            stage -= kPairStages;
-            phase ^= 1u;
-          }
         }
-        kb -= k_blocks;
+        stage += kPairProducers;
+        if (stage >= kPairStages) {
+          stage -= kPairStages;
+          phase ^= 1u;
+        }
       }
+      kb -= k_blocks;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && leader) {
+    if (leader) {
       constexpr uint32_t idesc = make_idesc_nvf4_pair(kPairBN);
       const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
       const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
@@ -616,7 +615,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1u;
         // both CTAs' epilogues have drained this accumulator
-        if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
+        if (!mbar_wait_warp(smem_u32(&tmem_empty_bar[acc]), acc_phase ^ 1u)) {
           report_timeout(args.error, abort_flag);
           break;
         }
@@ -624,7 +623,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         const uint32_t d_tmem = tmem_base + acc * kPairBN;
         for (int kb = 0; kb < k_blocks; ++kb) {
           // the operands of both CTAs have landed and both have written this block's scales
-          if (!mbar_wait_at(full0 + stage * 8, phase)) {
+          if (!mbar_wait_warp(full0 + stage * 8, phase)) {
             report_timeout(args.error, abort_flag);
             ok = false;
             break;
@@ -633,7 +632,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
           const uint64_t a_desc = advance_smem_desc(a_desc0, stage * kPairABytes);
           const uint64_t b_desc = advance_smem_desc(b_desc0, stage * kPairBBytes);
           const uint32_t sf_tmem = tmem_base + kPairSfCol + sf_buf * kPairSfBufCols;
-          if (kb + 1 < k_blocks || last_mmas == 4) {
+          const bool issue = elect_one();
+          if (issue && (kb + 1 < k_blocks || last_mmas == 4)) {
 #pragma unroll
             for (int kt = 0; kt < 4; ++kt) {
               tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
@@ -641,7 +641,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
                                     sf_tmem + 16 + kPairSfbGroups * kt,
                                     kt != 0 ? 1u : kb != 0 ? 1u : 0u);
             }
-          } else {
+          } else if (issue) {
             for (int kt = 0; kt < last_mmas; ++kt) {
               tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
                                     advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
@@ -650,14 +650,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
           }
           // frees the stage in both CTAs and, kPairSfBufs K blocks later, this block's
           // scale columns
-          tcgen05_commit_pair(&empty_bar[stage], 3);
+          if (issue) tcgen05_commit_pair(&empty_bar[stage], 3);
           if (++sf_buf == kPairSfBufs) sf_buf = 0;
           if (++stage == kPairStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) tcgen05_commit_pair(&tmem_full_bar[acc], 3);
+        if (ok && elect_one()) tcgen05_commit_pair(&tmem_full_bar[acc], 3);
       }
     }
   } else if (warp >= kScaleWarp) {  // (the producer behind them is taken)
@@ -709,7 +709,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
           }
         }
         if (!ready) {
-          if (lane == 0) report_timeout(args.error, abort_flag);
+          report_timeout(args.error, abort_flag);
           ok = false;
           break;
         }
