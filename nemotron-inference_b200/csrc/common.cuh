@@ -58,6 +58,41 @@ __device__ __forceinline__ uint32_t encode_e2m1x2(float even, float odd) {
       __nv_cvt_float2_to_fp4x2(make_float2(even, odd), __NV_E2M1, cudaRoundNearest));
 }
 
+// Eight floats -> four bytes, the even ones in the low nibbles.
+__device__ __forceinline__ uint32_t encode_e2m1x8(float a, float b, float c, float d, float e,
+                                                  float f, float g, float h) {
+  uint32_t word;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(word)
+      : "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h));
+  return word;
+}
+
+// Two FP32 operations in one instruction, each rounded as the scalar one.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+
 // ClampScale, nvfp4_packing.cpp:19-24
 __device__ __forceinline__ float clamp_scale(float v) {
   return (!isfinite(v) || v < kMinScale) ? kMinScale : v;
@@ -111,33 +146,39 @@ __device__ __forceinline__ float block_scale(float block_max, float divisor, flo
                            : __fdiv_rn(block_max, divisor));
 }
 
-// The fused quantiser of the up-projection epilogue: 16 non-negative values
-// whose maximum is `amax`, per-row tensor scale 1 (nvfp4_packing.cpp:119-153
-// with tensor_scale == 1.0).  Bit-identical to quantize_block16(v, 1.0f, ..).
-__device__ __forceinline__ uint32_t quantize_block16_unit_scale(const float (&v)[16], float amax,
+// div_by_reciprocal of two values by the same divisor.
+__device__ __forceinline__ uint64_t div2_by_reciprocal(uint64_t x, uint64_t minus_d, uint64_t r) {
+  const uint64_t q = mul2(x, r);
+  return fma2(fma2(q, minus_d, x), r, q);
+}
+
+// The fused quantiser of the up-projection epilogue: 16 non-negative values in pairs whose maximum
+// is `amax`, per-row tensor scale 1 (nvfp4_packing.cpp:119-153 with tensor_scale == 1.0).
+// Bit-identical to quantize_block16(v, 1.0f, ..).
+__device__ __forceinline__ uint32_t quantize_block16_unit_scale(const uint64_t (&v)[8], float amax,
                                                                 uint32_t& lo_word,
                                                                 uint32_t& hi_word) {
   const float bs = block_scale(amax, kFp4Max, 1.0f / kFp4Max);
-  const uint32_t scale_byte = encode_e4m3(bs);
-  uint32_t w[2] = {0u, 0u};
+  float q[16];
   if ((__float_as_uint(bs) & 0x007fffffu) != 0x007fffffu) {
     const float r = __frcp_rn(bs);
+    const uint64_t minus_bs = pack2(-bs, -bs), r2 = pack2(r, r);
 #pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-      const uint32_t byte = encode_e2m1x2(div_by_reciprocal(v[i], bs, r),
-                                          div_by_reciprocal(v[i + 1], bs, r));
-      w[i / 8] |= (byte & 0xffu) << (8 * ((i / 2) & 3));
+    for (int i = 0; i < 8; ++i) {
+      unpack2(div2_by_reciprocal(v[i], minus_bs, r2), q[2 * i], q[2 * i + 1]);
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-      const uint32_t byte = encode_e2m1x2(__fdiv_rn(v[i], bs), __fdiv_rn(v[i + 1], bs));
-      w[i / 8] |= (byte & 0xffu) << (8 * ((i / 2) & 3));
+    for (int i = 0; i < 8; ++i) {
+      float a, b;
+      unpack2(v[i], a, b);
+      q[2 * i] = __fdiv_rn(a, bs);
+      q[2 * i + 1] = __fdiv_rn(b, bs);
     }
   }
-  lo_word = w[0];
-  hi_word = w[1];
-  return scale_byte;
+  lo_word = encode_e2m1x8(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
+  hi_word = encode_e2m1x8(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
+  return encode_e4m3(bs);
 }
 
 // Offset of the scale of (row, 16-block) inside the 128-row x 4-block tiled

@@ -33,6 +33,7 @@ namespace {
 
 constexpr int kBN = 128;
 constexpr int kMaxStages = 8;
+constexpr int kEpilogueWarps = 8;  // two per TMEM lane quarter
 constexpr int kScaleWarp = 2 + kEpilogueWarps;
 constexpr int kScaleWarps = 2;
 // One thread needs about 530 cycles for a stage's waits and bookkeeping and 90 for each of its four

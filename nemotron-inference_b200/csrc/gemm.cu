@@ -37,6 +37,7 @@
 namespace nmoe {
 namespace {
 
+constexpr int kEpilogueWarps = 8;  // two per TMEM lane quarter (sixteen measured no faster)
 constexpr int kScaleWarp = 2 + kEpilogueWarps;  // issues the block-scale copies into TMEM
 constexpr int kScaleWarps = 2;  // the copies are split between this many issuing threads
                                 // (four measured no faster than two)
@@ -71,7 +72,7 @@ struct TileCfg {
   static constexpr int BAR_BYTES = ((2 * STAGES + 4 + SF_BUFS) * 8 + 16 + 15) / 16 * 16;
   // staging for the row-scattering epilogue of the down projection
   static constexpr bool ROW_STAGING = ROW_STAGING_;
-  static constexpr int EPI_STAGE_BYTES = ROW_STAGING_ ? kEpilogueWarps * 32 * kStageStride * 4 : 0;
+  static constexpr int EPI_STAGE_BYTES = ROW_STAGING_ ? kEpilogueWarps * kStageBytes : 0;
   // The MMA always reads 128 A rows; with a smaller box the tail rows alias the
   // following stages, which is harmless (those output rows are never stored)
   // but must stay inside the allocation: the B region follows the A region.
@@ -150,8 +151,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
   uint64_t* sf_ready_bar = tmem_empty_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sf_ready_bar + C::SF_BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* stage_base = reinterpret_cast<float*>(
-      reinterpret_cast<uint8_t*>(full_bar) + C::BAR_BYTES);  // down epilogue staging
+  uint8_t* stage_base = reinterpret_cast<uint8_t*>(full_bar) + C::BAR_BYTES;  // row staging
 
   const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -378,7 +378,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
   } else {
     // -------------------------------------------------------------- epilogue
     const int quarter = warp & 3;           // TMEM lanes a warp may read: 32 * (warp % 4)
-    const int half = (warp - 2) >> 2;       // which half of the tile's columns
+    const int group = (warp - 2) >> 2;      // which share of the tile's columns
     const int r = quarter * 32 + lane;      // row inside the tile == TMEM lane
     int local = 0;
     for (int t = unit; t < total_tiles; t += units, ++local) {
@@ -401,10 +401,11 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
       const uint32_t t_addr =
           tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * C::ACC_STRIDE;
       const int n0 = nt * C::BN;
-      // the two warps of a lane quarter split the tile's 16-column chunks
+      // the warps of a lane quarter split the tile's 16-column chunks
       constexpr int kChunks = C::BN / 16;
-      const int chunk_begin = half == 0 ? 0 : (kChunks + 1) / 2;
-      const int chunk_end = half == 0 ? (kChunks + 1) / 2 : kChunks;
+      constexpr int kGroups = kEpilogueWarps / 4;
+      const int chunk_begin = kChunks * group / kGroups;
+      const int chunk_end = kChunks * (group + 1) / kGroups;
 
       if constexpr (MODE == kGemmUp) {
         epilogue_quantise<1>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
@@ -412,7 +413,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
         const unsigned long long dest = row_valid ? output_row_address(args, grow) : 0ull;
         const float wt = row_valid && args.row_weight != nullptr ? args.row_weight[grow] : 1.0f;
         epilogue_rows(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt,
-                      stage_base + (warp - 2) * (32 * kStageStride));
+                      stage_base + (warp - 2) * kStageBytes);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -458,7 +459,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
 // ---------------------------------------------------------------------------
 constexpr int kPairBN = 208;
 constexpr int kPairBRows = kPairBN / 2;        // weight rows staged per CTA
-constexpr int kPairStages = 6;
+constexpr int kPairStages = 5;
 constexpr int kPairSfBufs = 2;
 constexpr int kPairScaleWarps = 4;             // one per TMEM lane quarter
 constexpr int kPairProducers = 2;
@@ -472,7 +473,8 @@ constexpr int kPairStageBytes = kPairABytes + kPairBBytes + kPairSfaBytes + kPai
 constexpr int kPairSfCol = 2 * kPairBN;        // TMEM: two accumulators, then the scale buffers
 constexpr int kPairSfBufCols = 16 + 4 * kPairSfbGroups;
 constexpr int kPairBarBytes = ((3 * kPairStages + 4) * 8 + 16 + 15) / 16 * 16;
-constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + kPairBarBytes + 1024;
+constexpr int kPairSmemBytes =
+    kPairStages * kPairStageBytes + kPairBarBytes + kEpilogueWarps * kStageBytes + 1024;
 static_assert(kPairSfCol + kPairSfBufs * kPairSfBufCols <= 512, "TMEM budget");
 static_assert(kPairBRows % 8 == 0, "half a weight tile is whole 8-row swizzle groups");
 static_assert(kPairBBytes % 1024 == 0, "stage regions keep the 1024-byte swizzle alignment");
@@ -732,11 +734,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   } else {
     // -------------------------------------------------------------- epilogue
     const int quarter = warp & 3;           // TMEM lanes a warp may read: 32 * (warp % 4)
-    const int half = (warp - 2) >> 2;       // which part of the tile's 16-column chunks
+    const int group = (warp - 2) >> 2;      // which share of the tile's 16-column chunks
     const int r = quarter * 32 + lane;      // row inside this CTA's 128 rows == TMEM lane
-    constexpr int kChunks = kPairBN / 16;   // 13: seven for the first warp of a quarter, six
-    const int chunk_begin = half == 0 ? 0 : (kChunks + 1) / 2;
-    const int chunk_end = half == 0 ? (kChunks + 1) / 2 : kChunks;
+    constexpr int kChunks = kPairBN / 16;
+    constexpr int kGroups = kEpilogueWarps / 4;
+    const int chunk_begin = kChunks * group / kGroups;
+    const int chunk_end = kChunks * (group + 1) / kGroups;
     const uint32_t leader_empty0 = cluster_address_of(&tmem_empty_bar[0], 0);
     int local = 0;
     for (int t = unit; t < total_tiles; t += units, ++local) {
@@ -765,9 +768,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kPairBN;
         const int n0 = nt * kPairBN;
         if constexpr (MODE == kGemmUp) {
-          epilogue_quantise<2>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
+          epilogue_quantise<1>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
         } else {
-          epilogue_rows_direct<2>(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt);
+          epilogue_rows(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt,
+                        reinterpret_cast<uint8_t*>(full_bar) + kPairBarBytes +
+                            (warp - 2) * kStageBytes);
         }
         tcgen05_fence_before();
       }

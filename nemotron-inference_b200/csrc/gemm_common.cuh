@@ -9,9 +9,6 @@
 
 namespace nmoe {
 
-constexpr int kEpilogueWarps = 8;    // two per TMEM lane quarter
-constexpr int kStageStride = 36;     // floats per staged row: 32 + 4 keeps float4 accesses conflict-free
-
 __device__ __forceinline__ void report_timeout(int32_t* error, volatile int* abort_flag) {
   *abort_flag = 1;
   if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
@@ -33,15 +30,20 @@ __device__ __forceinline__ void load_chunks(uint32_t t_addr, int count, uint32_t
 // relu^2 and NVFP4 quantisation of 16 columns from `n` of row `grow`; returns the largest value.
 __device__ __forceinline__ float quantise_chunk(const GemmArgs& args, float (&v)[16], int n, int grow,
                                                 float scale, bool store) {
+  const uint64_t scale2 = pack2(scale, scale);
+  uint64_t squares[8];
   float amax = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float x = fmaxf(__fmul_rn(v[i], scale), 0.0f);  // Relu2: x > 0 ? x*x : 0
-    v[i] = __fmul_rn(x, x);
-    amax = fmaxf(amax, v[i]);
+  for (int i = 0; i < 8; ++i) {  // Relu2: x > 0 ? x*x : 0
+    float a, b;
+    unpack2(mul2(pack2(v[2 * i], v[2 * i + 1]), scale2), a, b);
+    const uint64_t x = pack2(fmaxf(a, 0.0f), fmaxf(b, 0.0f));
+    squares[i] = mul2(x, x);
+    unpack2(squares[i], a, b);
+    amax = fmaxf(fmaxf(a, b), amax);
   }
   uint32_t lo, hi;
-  const uint32_t sf = quantize_block16_unit_scale(v, amax, lo, hi);
+  const uint32_t sf = quantize_block16_unit_scale(squares, amax, lo, hi);
   if (!store) return 0.0f;
   *reinterpret_cast<uint2*>(args.out_packed + static_cast<size_t>(grow) * (args.N / 2) + n / 2) =
       make_uint2(lo, hi);
@@ -52,6 +54,21 @@ __device__ __forceinline__ float quantise_chunk(const GemmArgs& args, float (&v)
 __device__ __forceinline__ void report_range(const GemmArgs& args, float largest) {
   if (largest > kFp4Max * kFp8Max && args.error != nullptr) {
     atomicCAS(args.error, kDevOk, kDevActivationRange);
+  }
+}
+
+// Sixteen values as bf16 or binary16 (a value beyond 65504 becomes an infinity here; the combine
+// kernel reports it).
+__device__ __forceinline__ void pack_rows16(int kind, const float (&v)[16], uint32_t (&w)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (kind == kRowBf16) {
+      const __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&two);
+    } else {
+      const __half2 two = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&two);
+    }
   }
 }
 
@@ -76,17 +93,7 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& args, float (&v)[16]
     return;
   }
   uint32_t w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (args.out_kind == kRowBf16) {
-      const __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-      w[i] = *reinterpret_cast<const uint32_t*>(&two);
-    } else {
-      // a value beyond binary16's 65504 becomes an infinity here; the combine kernel reports it
-      const __half2 two = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-      w[i] = *reinterpret_cast<const uint32_t*>(&two);
-    }
-  }
+  pack_rows16(args.out_kind, v, w);
   uint4* d = reinterpret_cast<uint4*>(dest + static_cast<size_t>(n) * 2);
   d[0] = make_uint4(w[0], w[1], w[2], w[3]);
   d[1] = make_uint4(w[4], w[5], w[6], w[7]);
@@ -155,80 +162,63 @@ __device__ __forceinline__ void epilogue_rows_direct(const GemmArgs& args, uint3
   }
 }
 
-// Row-storing epilogue: scale [x routing weight] [-> relu^2], scattered.  Each thread owns one row
-// of the tile, but a store instruction should write whole lines: 32 columns of 32 rows are staged
-// in shared memory (`stage`: 32 * kStageStride floats of this warp's own), then every 8 lanes
-// write 128 contiguous bytes of one row (4 rows per instruction).
+// Row-storing epilogue through shared memory: each thread owns one row of the tile, but a store
+// instruction should write few lines.  64 bytes of 32 rows are staged at a time (`stage`:
+// kStageBytes of this warp's own; a row's pitch of five 16-byte units keeps both directions free
+// of bank conflicts), then every four lanes write one row's 64 bytes.
+constexpr int kStagePitch = 80;
+constexpr int kStageBytes = 32 * kStagePitch;
+
 __device__ __forceinline__ void epilogue_rows(const GemmArgs& args, uint32_t t_addr, int n0,
                                               int chunk_begin, int chunk_end,
                                               unsigned long long dest, float scale, float wt,
-                                              float* stage) {
+                                              uint8_t* stage) {
   const int lane = threadIdx.x & 31;
-  const int sub = lane >> 3;
-  const int c4 = (lane & 7) * 4;
-  for (int ch = chunk_begin; ch < chunk_end; ch += 2) {
-    const int n = n0 + ch * 16;
-    if (n >= args.N) break;
-    const bool wide = ch + 1 < chunk_end && n + 16 < args.N;
-    float va[16], vb[16];
-    tmem_ld_x16(t_addr + ch * 16, va);
-    if (wide) {
-      tmem_ld_x16(t_addr + ch * 16 + 16, vb);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) vb[i] = 0.0f;
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      va[i] = __fmul_rn(va[i], scale);
-      vb[i] = __fmul_rn(vb[i], scale);
-      if (args.row_weight != nullptr) {
-        va[i] = __fmul_rn(va[i], wt);
-        vb[i] = __fmul_rn(vb[i], wt);
-      }
-      if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
-        const float pa = fmaxf(va[i], 0.0f), pb = fmaxf(vb[i], 0.0f);
-        va[i] = __fmul_rn(pa, pa);
-        vb[i] = __fmul_rn(pb, pb);
-      }
-    }
+  uint8_t* own = stage + lane * kStagePitch;
+  const uint8_t* part = stage + (lane >> 2) * kStagePitch + (lane & 3) * 16;
+  const bool f32 = args.out_kind == kRowF32;
+  const float factor = args.row_weight != nullptr ? wt : 1.0f;
+  chunk_end = min(chunk_end, (args.N - n0) / 16);
+  const int step = f32 ? 1 : 2;
+  for (int ch = chunk_begin; ch < chunk_end; ch += step) {
+    const bool wide = !f32 && ch + 1 < chunk_end;
+    uint32_t raw[2][16];
+    load_chunks<2>(t_addr + ch * 16, wide ? 2 : 1, raw);
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 16; i += 4) {
-      *reinterpret_cast<float4*>(stage + lane * kStageStride + i) =
-          make_float4(va[i], va[i + 1], va[i + 2], va[i + 3]);
-      if (wide) {
-        *reinterpret_cast<float4*>(stage + lane * kStageStride + 16 + i) =
-            make_float4(vb[i], vb[i + 1], vb[i + 2], vb[i + 3]);
-      }
-    }
-    __syncwarp();
-    const bool col_ok = c4 < (wide ? 32 : 16);
-#pragma unroll 4
-    for (int it = 0; it < 8; ++it) {
-      const int rr = 4 * it + sub;
-      const unsigned long long d = __shfl_sync(0xffffffffu, dest, rr);
-      if (d != 0 && col_ok) {
-        const float4 value = *reinterpret_cast<const float4*>(stage + rr * kStageStride + c4);
-        if (args.out_kind == kRowBf16) {
-          const __nv_bfloat162 lo = __floats2bfloat162_rn(value.x, value.y);
-          const __nv_bfloat162 hi = __floats2bfloat162_rn(value.z, value.w);
-          uint2 bits;
-          bits.x = *reinterpret_cast<const uint32_t*>(&lo);
-          bits.y = *reinterpret_cast<const uint32_t*>(&hi);
-          *reinterpret_cast<uint2*>(d + static_cast<size_t>(n + c4) * 2) = bits;
-        } else if (args.out_kind == kRowF16) {
-          // a value beyond binary16's 65504 becomes an infinity here; the combine
-          // kernel reports it
-          const __half2 lo = __floats2half2_rn(value.x, value.y);
-          const __half2 hi = __floats2half2_rn(value.z, value.w);
-          uint2 bits;
-          bits.x = *reinterpret_cast<const uint32_t*>(&lo);
-          bits.y = *reinterpret_cast<const uint32_t*>(&hi);
-          *reinterpret_cast<uint2*>(d + static_cast<size_t>(n + c4) * 2) = bits;
-        } else {
-          *reinterpret_cast<float4*>(d + static_cast<size_t>(n + c4) * 4) = value;
+    for (int j = 0; j < 2; ++j) {
+      if (j == 1 && !wide) break;
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        // (a factor of one leaves every value as it is)
+        v[i] = __fmul_rn(__fmul_rn(__uint_as_float(raw[j][i]), scale), factor);
+        if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
+          const float p = fmaxf(v[i], 0.0f);
+          v[i] = __fmul_rn(p, p);
         }
+      }
+      if (f32) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          *reinterpret_cast<float4*>(own + i * 4) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+      } else {
+        uint32_t w[8];
+        pack_rows16(args.out_kind, v, w);
+        *reinterpret_cast<uint4*>(own + j * 32) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(own + j * 32 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+    }
+    __syncwarp();
+    const bool mine = f32 || wide || (lane & 3) < 2;
+    const size_t at = static_cast<size_t>(n0 + ch * 16) * (f32 ? 4 : 2) + (lane & 3) * 16;
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const unsigned long long d = __shfl_sync(0xffffffffu, dest, it * 8 + (lane >> 2));
+      if (d != 0 && mine) {
+        *reinterpret_cast<uint4*>(d + at) =
+            *reinterpret_cast<const uint4*>(part + it * 8 * kStagePitch);
       }
     }
   }
