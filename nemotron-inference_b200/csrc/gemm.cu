@@ -187,7 +187,6 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
   const int num_row_tiles = warp_uniform(
       args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128);
   const int total_tiles = num_row_tiles * args.n_tiles;
-  const int k_mmas = args.K / 64;
 
   if (warp == 0 || warp >= kScaleWarp + kScaleWarps) {
     // ------------------------------------------------------------- producers
@@ -437,33 +436,24 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) 
 // CTA-pair kernel (kVariantPair): one 256 x kPairBN tile per cluster of two CTAs
 // (tcgen05.mma.cta_group::2, M = 256).
 //
-// A 128 x 208 tile of one CTA takes 1220 cycles per 256-element K block for 416 cycles of MMA: the
-// twelve tcgen05.cp of its block scales run through the tensor pipe at 47 cycles each beside the
-// MMAs, and every K block brings 49 KB from L2 into an SM that takes about 50 bytes a cycle.  A
-// pair stages each weight tile once for 256 rows (half in each CTA: 35 KB per CTA and K block),
-// and its scales go shared memory -> registers -> TMEM (tcgen05.st), off the tensor pipe, from
-// four warps per CTA, one per TMEM lane quarter, each CTA for its own TMEM.
+// What bounds a K block is shared memory: at 128 bytes a cycle the copies of a 128 x 208 tile of
+// one CTA write 49 KB (380 cycles) and its MMAs read 43 KB (330), for 416 cycles of MMA.  A pair
+// stages each weight tile once for 256 rows (half in each CTA): 35 KB written and 30 KB read per
+// CTA and K block.
 //
-// The roles are single threads or warps whose every step is latency: a wait costs 140 cycles when
-// there is nothing to wait for and 250 when there is, so a K block has ONE barrier the MMA thread
-// waits for -- the full barrier of the leader counts the activation and weight bytes of both CTAs
-// and the arrivals of all eight scale warps -- and two producers per CTA take turns.
+// Roles per CTA: warp 0 loads (the CTA's own 128 activation rows, its half of the weight tile, the
+// scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues the scale
+// copies and the MMAs for both CTAs, warps 2-9 run the epilogue of the CTA's 128 rows.  Copies
+// and MMAs of one thread execute in order, so nothing waits between them; the bytes of both CTAs
+// complete on rank 0's full barrier, so nothing is handed over inside a K block.  No multicast:
+// the loads of the partner name the leader's barrier.
 //
-// Roles per CTA: warps 0 and 14 load (the CTA's own 128 activation rows, its half of the weight
-// tile, the scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues the
-// MMAs for both, warps 2-9 run the epilogue of the CTA's 128 rows, warps 10-13 write scales.  No
-// multicast: the loads of the partner name the leader's barrier.
-//
-// Measured, benchmark layer, up / down projection: 16384 tokens 331 / 401 -> @P1@ us, 8192 tokens
-// 188 / 221 -> @P2@.
+// Measured, benchmark layer, up / down projection: 16384 tokens @P1@, 8192 tokens @P2@.
 // ---------------------------------------------------------------------------
 constexpr int kPairBN = 208;
 constexpr int kPairBRows = kPairBN / 2;        // weight rows staged per CTA
-constexpr int kPairStages = 5;
 constexpr int kPairSfBufs = 2;
-constexpr int kPairScaleWarps = 4;             // one per TMEM lane quarter
-constexpr int kPairProducers = 2;
-constexpr int kPairThreads = (1 + kEpilogueWarps + kPairScaleWarps + kPairProducers) * 32;
+constexpr int kPairThreads = (2 + kEpilogueWarps) * 32;
 constexpr int kPairABytes = 128 * 128;
 constexpr int kPairBBytes = kPairBRows * 128;
 constexpr int kPairSfaBytes = 2048;
@@ -472,13 +462,18 @@ constexpr int kPairSfbBytes = kPairSfbGroups * 512;
 constexpr int kPairStageBytes = kPairABytes + kPairBBytes + kPairSfaBytes + kPairSfbBytes;
 constexpr int kPairSfCol = 2 * kPairBN;        // TMEM: two accumulators, then the scale buffers
 constexpr int kPairSfBufCols = 16 + 4 * kPairSfbGroups;
-constexpr int kPairBarBytes = ((3 * kPairStages + 4) * 8 + 16 + 15) / 16 * 16;
-constexpr int kPairSmemBytes =
-    kPairStages * kPairStageBytes + kPairBarBytes + kEpilogueWarps * kStageBytes + 1024;
+// the row-storing epilogue's staging takes the place of a pipeline stage
+constexpr int pair_stages(int mode) { return mode == kGemmUp ? 6 : 5; }
+constexpr int kPairBarBytes = ((2 * pair_stages(kGemmUp) + 4) * 8 + 16 + 15) / 16 * 16;
+constexpr int pair_smem_bytes(int mode) {
+  return pair_stages(mode) * kPairStageBytes + kPairBarBytes +
+         (mode == kGemmUp ? 0 : kEpilogueWarps * kStageBytes) + 1024;
+}
 static_assert(kPairSfCol + kPairSfBufs * kPairSfBufCols <= 512, "TMEM budget");
 static_assert(kPairBRows % 8 == 0, "half a weight tile is whole 8-row swizzle groups");
 static_assert(kPairBBytes % 1024 == 0, "stage regions keep the 1024-byte swizzle alignment");
-static_assert(kPairSmemBytes <= 232448, "shared memory budget");
+static_assert(pair_smem_bytes(kGemmUp) <= 232448 && pair_smem_bytes(kGemmDown) <= 232448,
+              "shared memory budget");
 
 struct PairShape {  // what tile_rows_of reads
   static constexpr bool PAIR = true;
@@ -491,15 +486,15 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
                                              ~static_cast<uintptr_t>(1023u));
+  constexpr int kStages = pair_stages(MODE);
   uint8_t* sA = smem;
-  uint8_t* sB = sA + kPairStages * kPairABytes;
-  uint8_t* sSFA = sB + kPairStages * kPairBBytes;
-  uint8_t* sSFB = sSFA + kPairStages * kPairSfaBytes;
-  // full_bar (the leader's): operand bytes of both CTAs and the scale warps of both
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sSFB + kPairStages * kPairSfbBytes);
-  uint64_t* sf_full_bar = full_bar + kPairStages;   // this CTA's scale bytes landed
-  uint64_t* empty_bar = sf_full_bar + kPairStages;  // both CTAs: the MMAs have read the stage
-  uint64_t* tmem_full_bar = empty_bar + kPairStages;
+  uint8_t* sB = sA + kStages * kPairABytes;
+  uint8_t* sSFA = sB + kStages * kPairBBytes;
+  uint8_t* sSFB = sSFA + kStages * kPairSfaBytes;
+  // full_bar (the leader's): the bytes of both CTAs
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sSFB + kStages * kPairSfbBytes);
+  uint64_t* empty_bar = full_bar + kStages;  // both CTAs: the MMAs have read the stage
+  uint64_t* tmem_full_bar = empty_bar + kStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -512,9 +507,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   const int units = static_cast<int>(gridDim.x >> 1);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPairStages; ++s) {
-      mbar_init(&full_bar[s], 1 + 2 * kPairScaleWarps);
-      mbar_init(&sf_full_bar[s], 1);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -526,6 +520,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
     prefetch_tensormap(&maps.a);
     prefetch_tensormap(&maps.b_tail);
     prefetch_tensormap(&maps.b_full);
+    prefetch_tensormap(&maps.sfa);
+    prefetch_tensormap(&maps.sfb);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
@@ -542,48 +538,36 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   const int row_units = (num_row_tiles + 1) / 2;
   const int total_tiles = row_units * args.n_tiles;
   const int k_blocks = args.k_blocks;
-  const uint32_t full0 = smem_u32(full_bar), sf_full0 = smem_u32(sf_full_bar);
-  const uint32_t empty0 = smem_u32(empty_bar);
+  const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
   const uint32_t leader_full0 = cluster_address_of(&full_bar[0], 0);
 
-  if (warp == 0 || warp >= kScaleWarp + kPairScaleWarps) {
-    // ------------------------------------------------------------- producers
-    // Producer p loads the K blocks p, p + kPairProducers, ... of the CTA's sequence.
+  if (warp == 0) {
+    // ------------------------------------------------------------- producer
     const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
     const uint32_t sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
-    int stage = warp == 0 ? 0 : warp - (kScaleWarp + kPairScaleWarps) + 1;
-    int kb = stage;  // K block of the current tile this producer loads next
+    int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int t = unit; t < total_tiles && ok; t += units) {
       const int rt = t / args.n_tiles;
       const int nt = t - rt * args.n_tiles;
-      TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
-      rows.load_row0 = warp_uniform(rows.load_row0);
+      const TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
+      const int load_row0 = warp_uniform(rows.load_row0);
       const int expert = warp_uniform(rows.expert);
-      const uint8_t* sfa_src =
-          args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * k_blocks * kPairSfaBytes;
-      const uint8_t* sfb_src =
-          args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) * k_blocks * kPairSfbBytes;
+      // the scale maps' rows are 1024 bytes: two to a K block of activations, four to one of weights
+      const int sfa_row = (load_row0 >> 7) * k_blocks * 2;
+      const int sfb_row = (expert * args.n_tiles + nt) * k_blocks * 4;
       const int b_row = nt * kPairBN + static_cast<int>(cta_rank) * kPairBRows;
-      for (; kb < k_blocks; kb += kPairProducers) {
+      for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
           report_timeout(args.error, abort_flag);
           ok = false;
           break;
         }
         if (elect_one()) {
-          const uint32_t bar = leader_full0 + stage * 8, sf_bar = sf_full0 + stage * 8;
-          mbar_arrive_expect_tx_at(sf_bar, kPairSfaBytes + kPairSfbBytes);
-          bulk_load_at(sfa0 + stage * kPairSfaBytes, sfa_src + kb * kPairSfaBytes, kPairSfaBytes,
-                       sf_bar);
-          bulk_load_at(sfb0 + stage * kPairSfbBytes, sfb_src + kb * kPairSfbBytes, kPairSfbBytes,
-                       sf_bar);
-          // activation and weight bytes of both CTAs are counted on the leader's barrier
-          if (leader) {
-            mbar_arrive_expect_tx_at(full0 + stage * 8, 2 * (kPairABytes + kPairBBytes));
-          }
-          tma_load_2d_pair_at(a0 + stage * kPairABytes, &maps.a, kb * 128, rows.load_row0, bar);
+          const uint32_t bar = leader_full0 + stage * 8;
+          if (leader) mbar_arrive_expect_tx_at(full0 + stage * 8, 2 * kPairStageBytes);
+          tma_load_2d_pair_at(a0 + stage * kPairABytes, &maps.a, kb * 128, load_row0, bar);
           if (kb < args.kb_full) {
             // the map's rows are eight weight rows' 128 bytes of a K block
             tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_full, 0,
@@ -592,21 +576,23 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
             tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_tail, 0, expert * args.N + b_row,
                                 bar);
           }
+          tma_load_2d_pair_at(sfa0 + stage * kPairSfaBytes, &maps.sfa, 0, sfa_row + kb * 2, bar);
+          tma_load_2d_pair_at(sfb0 + stage * kPairSfbBytes, &maps.sfb, 0, sfb_row + kb * 4, bar);
         }
-        stage += kPairProducers;
-        if (stage >= kPairStages) {
-          stage -= kPairStages;
+        if (++stage == kStages) {
+          stage = 0;
           phase ^= 1u;
         }
       }
-      kb -= k_blocks;
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
+    // ------------------------------------------- scale copies and MMAs, for both CTAs
     if (leader) {
       constexpr uint32_t idesc = make_idesc_nvf4_pair(kPairBN);
       const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
       const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
+      const uint64_t sfa_desc0 = make_smem_desc(smem_u32(sSFA), 0, 128, 0);
+      const uint64_t sfb_desc0 = make_smem_desc(smem_u32(sSFB), 0, 128, 0);
       const int last_mmas = args.K / 64 - 4 * (k_blocks - 1);
       int stage = 0;
       uint32_t phase = 0;
@@ -624,7 +610,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kPairBN;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          // the operands of both CTAs have landed and both have written this block's scales
           if (!mbar_wait_warp(full0 + stage * 8, phase)) {
             report_timeout(args.error, abort_flag);
             ok = false;
@@ -633,102 +618,54 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
           tcgen05_fence_after();
           const uint64_t a_desc = advance_smem_desc(a_desc0, stage * kPairABytes);
           const uint64_t b_desc = advance_smem_desc(b_desc0, stage * kPairBBytes);
+          const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * kPairSfaBytes);
+          const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * kPairSfbBytes);
           const uint32_t sf_tmem = tmem_base + kPairSfCol + sf_buf * kPairSfBufCols;
-          const bool issue = elect_one();
-          if (issue && (kb + 1 < k_blocks || last_mmas == 4)) {
+          if (elect_one()) {
+            if (kb + 1 < k_blocks || last_mmas == 4) {
 #pragma unroll
-            for (int kt = 0; kt < 4; ++kt) {
-              tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                                    advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
-                                    sf_tmem + 16 + kPairSfbGroups * kt,
-                                    kt != 0 ? 1u : kb != 0 ? 1u : 0u);
+              for (int c = 0; c < 4; ++c) {
+                tcgen05_cp_pair_32x128b_warpx4(sf_tmem + 4 * c,
+                                               advance_smem_desc(sfa_desc, c * 512));
+              }
+#pragma unroll
+              for (int c = 0; c < kPairSfbGroups; ++c) {
+                tcgen05_cp_pair_32x128b_warpx4(sf_tmem + 16 + 4 * c,
+                                               advance_smem_desc(sfb_desc, c * 512));
+              }
+#pragma unroll
+              for (int kt = 0; kt < 4; ++kt) {
+                tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                                      advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
+                                      sf_tmem + 16 + kPairSfbGroups * kt,
+                                      kt != 0 ? 1u : kb != 0 ? 1u : 0u);
+              }
+            } else {
+              // the scales of a partial last K block: of the MMAs it issues only
+              for (int c = 0; c < last_mmas; ++c) {
+                tcgen05_cp_pair_32x128b_warpx4(sf_tmem + 4 * c,
+                                               advance_smem_desc(sfa_desc, c * 512));
+              }
+              for (int c = 0; c < last_mmas * (kPairSfbGroups / 4); ++c) {
+                tcgen05_cp_pair_32x128b_warpx4(sf_tmem + 16 + 4 * c,
+                                               advance_smem_desc(sfb_desc, c * 512));
+              }
+              for (int kt = 0; kt < last_mmas; ++kt) {
+                tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
+                                      advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
+                                      sf_tmem + 16 + kPairSfbGroups * kt,
+                                      (kb | kt) != 0 ? 1u : 0u);
+              }
             }
-          } else if (issue) {
-            for (int kt = 0; kt < last_mmas; ++kt) {
-              tcgen05_mma_pair_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                                    advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
-                                    sf_tmem + 16 + kPairSfbGroups * kt, (kb | kt) != 0 ? 1u : 0u);
-            }
+            tcgen05_commit_pair(&empty_bar[stage], 3);  // frees the stage in both CTAs
           }
-          // frees the stage in both CTAs and, kPairSfBufs K blocks later, this block's
-          // scale columns
-          if (issue) tcgen05_commit_pair(&empty_bar[stage], 3);
           if (++sf_buf == kPairSfBufs) sf_buf = 0;
-          if (++stage == kPairStages) {
+          if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (ok && elect_one()) tcgen05_commit_pair(&tmem_full_bar[acc], 3);
-      }
-    }
-  } else if (warp >= kScaleWarp) {  // (the producer behind them is taken)
-    // ------------------------------------------------------- block-scale writers
-    // Each warp writes the same 32 x 16 B of every 512-byte chunk to its own lane
-    // quarter: the layout a tcgen05.cp.32x128b.warpx4 produces.
-    const int quarter = warp & 3;
-    const uint32_t sf_tmem0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kPairSfCol;
-    int stage = 0;
-    uint32_t phase = 0;
-    uint32_t sf_buf = 0;
-    // the scale columns written now were last read by the MMAs of the K block kPairSfBufs
-    // iterations back; those MMAs also release that block's stage
-    int old_stage = 0;
-    uint32_t old_phase = 0;
-    int unread = kPairSfBufs;  // buffers nothing has read yet
-    bool ok = true;
-    for (int t = unit; t < total_tiles && ok; t += units) {
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        bool ready = mbar_wait_at(sf_full0 + stage * 8, phase);
-        const uint4* sfa = reinterpret_cast<const uint4*>(sSFA + stage * kPairSfaBytes) + lane;
-        const uint4* sfb = reinterpret_cast<const uint4*>(sSFB + stage * kPairSfbBytes) + lane;
-        uint32_t row_words[16], lo_words[16], hi_words[16];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint4 q = sfa[c * 32];
-          row_words[4 * c] = q.x;
-          row_words[4 * c + 1] = q.y;
-          row_words[4 * c + 2] = q.z;
-          row_words[4 * c + 3] = q.w;
-          const uint4 u = sfb[c * 32];
-          lo_words[4 * c] = u.x;
-          lo_words[4 * c + 1] = u.y;
-          lo_words[4 * c + 2] = u.z;
-          lo_words[4 * c + 3] = u.w;
-          const uint4 v = sfb[(c + 4) * 32];
-          hi_words[4 * c] = v.x;
-          hi_words[4 * c + 1] = v.y;
-          hi_words[4 * c + 2] = v.z;
-          hi_words[4 * c + 3] = v.w;
-        }
-        if (unread > 0) {
-          --unread;
-        } else {
-          ready = ready && mbar_wait_at(empty0 + old_stage * 8, old_phase);
-          if (++old_stage == kPairStages) {
-            old_stage = 0;
-            old_phase ^= 1u;
-          }
-        }
-        if (!ready) {
-          report_timeout(args.error, abort_flag);
-          ok = false;
-          break;
-        }
-        tcgen05_fence_after();
-        const uint32_t sf_tmem = sf_tmem0 + sf_buf * kPairSfBufCols;
-        tmem_st_x16(sf_tmem, row_words);
-        tmem_st_x16(sf_tmem + 16, lo_words);
-        tmem_st_x16(sf_tmem + 32, hi_words);
-        tmem_st_wait();
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_at(leader_full0 + stage * 8);
-        if (++sf_buf == kPairSfBufs) sf_buf = 0;
-        if (++stage == kPairStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
       }
     }
   } else {
@@ -796,12 +733,13 @@ cudaError_t launch_pair(const GemmMaps& maps, const GemmArgs& args, int num_sms,
                         cudaStream_t stream) {
   auto kernel = grouped_gemm_pair_kernel<MODE>;
   cudaError_t err =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           pair_smem_bytes(MODE));
   if (err != cudaSuccess) return err;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(num_sms & ~1), 1, 1);
   config.blockDim = dim3(kPairThreads, 1, 1);
-  config.dynamicSmemBytes = kPairSmemBytes;
+  config.dynamicSmemBytes = pair_smem_bytes(MODE);
   config.stream = stream;
   cudaLaunchAttribute attribute;
   attribute.id = cudaLaunchAttributeClusterDimension;
@@ -928,7 +866,7 @@ GemmVariantInfo gemm_variant_info(GemmVariant v) {
     case kVariantPrefillUp: return info_of<CfgPrefillUp>();
     case kVariantPrefillDown: return info_of<CfgPrefillDown>();
     case kVariantPair:
-      return GemmVariantInfo{kPairBN, 128, kPairSfbGroups, kPairSfbBytes, kPairSmemBytes,
+      return GemmVariantInfo{kPairBN, 128, kPairSfbGroups, kPairSfbBytes, pair_smem_bytes(kGemmUp),
                              kPairBRows};
     default: return GemmVariantInfo{0, 0, 0, 0, 0, 0};
   }

@@ -99,6 +99,7 @@ struct GemmMaps {
   CUtensorMap a;
   CUtensorMap b_tail;
   CUtensorMap b_full;
+  CUtensorMap sfa, sfb;  // both operands' tiled block scales as rows of 1024 bytes
 };
 
 // Up to four GEMMs whose tiles one persistent launch walks in order (csrc/expert_stream.cu): the

@@ -213,6 +213,7 @@ struct WeightStack {
   CUtensorMap tail_prefill;
   CUtensorMap tail_stream;
   CUtensorMap tail_pair;
+  CUtensorMap sf_pair_map;
   CUtensorMap full_pair;  // the K-block-major panels as [rows][1024 B], for the CTA-pair variant
 
   void upload(const nmoe_nvfp4_matrix* matrices, int count, int rows, int cols, bool is_up,
@@ -235,6 +236,8 @@ struct WeightStack {
     sf_prefill.allocate(sf_prefill_each * count);
     sf_stream.allocate(sf_stream_each * count);
     sf_pair.allocate(sf_pair_each * count);
+    sf_pair_map = make_raw_map(sf_pair.as<uint8_t>(), sf_pair_each * count / 1024,
+                               qi.sfb_bytes / 1024);
     kb_full = cols / 256;
     const int tail_bytes = (cols % 256) / 2;
     const size_t panel_rows = static_cast<size_t>(count) * rows;
@@ -329,9 +332,11 @@ struct ActivationOperand {
   const uint8_t* packed = nullptr;
   const uint8_t* sf_tiled = nullptr;
   CUtensorMap boxes[kStreamBoxes];  // 8, 16, 32, 64 and 128 rows
+  CUtensorMap sf_map;               // the tiled scales as rows of 1024 bytes
   void bind(const uint8_t* packed_rows, const uint8_t* sf, size_t rows, int k) {
     packed = packed_rows;
     sf_tiled = sf;
+    sf_map = make_raw_map(sf, tiled_sf_bytes(rows / 128, k) / 1024, 2);
     for (int i = 0; i < kStreamBoxes; ++i) {
       boxes[i] = make_packed_map(packed_rows, rows, static_cast<size_t>(k) / 2, 8 << i);
     }
@@ -343,6 +348,8 @@ GemmMaps gemm_maps(const WeightStack& weights, TileClass tile_class, const Activ
   maps.a = a.boxes[kStreamBoxes - 1];
   maps.b_tail = weights.tail_map(tile_class);
   maps.b_full = weights.full_pair;
+  maps.sfa = a.sf_map;
+  maps.sfb = weights.sf_pair_map;
   return maps;
 }
 
