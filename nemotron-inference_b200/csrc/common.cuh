@@ -321,6 +321,10 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
   return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity));
 }
 
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx_at(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");

@@ -3,25 +3,24 @@
 //
 // As four launches (up and down, routed and shared) these sizes paid for every launch's start and
 // for every launch's last wave with idle HBM: 64 tokens took 72 + 75 us of routed GEMMs for 670 MB.
-// Here every CTA walks one list of tiles -- shared up, routed up, shared down, routed down -- and
-// its loads never stop in between: a down tile needs the quantised hidden rows of its row tile
+// Here the CTAs take tiles from one list -- shared up, routed up, shared down, routed down -- and
+// their loads do not stop in between: a down tile needs the quantised hidden rows of its row tile
 // only for its A operand, so its weights are on their way before those rows are complete.  A row
 // tile's completed up tiles are counted in global memory; the producer of a down tile waits for the
-// count (bounded, like every wait here).  All up tiles precede all down tiles in the list and every
-// CTA of the grid is resident (one per SM), so the wait ends.
+// count (bounded, like every wait here).  Tiles are taken in order with an atomic ticket, so a tile
+// that others wait for is always in the hands of a running CTA, however many CTAs of the grid are
+// resident beside other work.
 //
 // Tiles are 128 weight rows (B, BN = 128) of one row tile of up to 128 activation rows (A); the
 // activation box is 8 to 128 rows high, by the rows the tile holds, and the last weight tile of
 // a matrix loads the rows that exist.  At 148 SMs and the measured copy rate a K block's 18 KB of
-// weights take 800 cycles to arrive.  Roles of a single thread cost about as much when they wait
-// twice a K block and build their descriptors from scratch, so the loops here wait once and advance
-// descriptors (64 tokens, routed up and down 131 -> 120 us).
-// Measured, whole pass of the benchmark layer: 64 tokens 196 -> 164 us, 256 tokens 205 -> 178,
-// 1003 tokens 240 -> 229.
+// weights take 800 cycles to arrive; its eight scale copies and four MMAs, issued in order by one
+// warp, take about 300.
 //
-// Warp roles as in grouped_gemm_kernel (csrc/gemm.cu): warps 0 and 12-14 load, warp 1 issues MMAs,
-// warps 2-9 run epilogues, warps 10-11 copy block scales to TMEM; warp 15 hands
-// finished tiles on.
+// Roles: warp 0 takes tiles and loads, warp 1 issues scale copies and MMAs, warps 2-9 run
+// epilogues, warp 10 hands finished tiles on.
+// Measured, whole pass of the benchmark layer: 64 tokens 196 -> @S1@ us, 256 tokens 205 -> @S2@,
+// 1003 tokens 240 -> @S3@.
 #include <algorithm>
 
 #include "common.cuh"
@@ -34,24 +33,32 @@ namespace {
 constexpr int kBN = 128;
 constexpr int kMaxStages = 8;
 constexpr int kEpilogueWarps = 8;  // two per TMEM lane quarter
-constexpr int kScaleWarp = 2 + kEpilogueWarps;
-constexpr int kScaleWarps = 2;
-// One thread needs about 530 cycles for a stage's waits and bookkeeping and 90 for each of its four
-// copies (measured on a ring of bulk copies that does nothing else), more than a K block's 800, so
-// four threads take turns: 64 tokens, routed up and
-// down 137 -> 131 us.
-constexpr int kProducers = 4;
-constexpr int kSignalWarp = 1 + kEpilogueWarps + kScaleWarps + kProducers;
+constexpr int kSignalWarp = 2 + kEpilogueWarps;
 constexpr int kThreads = (kSignalWarp + 1) * 32;
 constexpr int kBBytes = kBN * 128;
 constexpr int kSfaBytes = 2048;
 constexpr int kSfbBytes = 2048;     // four groups of 32 weight rows x four MMAs x 16 bytes
+constexpr int kSfBufs = 2;
 constexpr int kSfBufCols = 32;      // TMEM columns of one K block's scales: 16 for A, 16 for B
 constexpr int kSfCol = 2 * kBN;     // behind the two accumulators
 constexpr int kTmemCols = 512;
-constexpr int kBarBytes = ((3 * kMaxStages + 6) * 8 + 16 + 15) / 16 * 16;
-static_assert(kProducers <= 6, "a producer advances less than a ring at a time");
-static_assert(kSfCol + kMaxStages * kSfBufCols <= kTmemCols, "TMEM budget");
+static_assert(kSfCol + kSfBufs * kSfBufCols <= kTmemCols, "TMEM budget");
+
+// Where a tile of the list lies.
+struct Tile {
+  int phase;   // -1: no more tiles
+  int row0;    // first row of its 128-row slot
+  int rows;    // valid rows in it
+  int expert;
+  int nt;      // weight tile
+};
+
+// The producer hands tiles to the other roles through a ring in shared memory.
+constexpr int kRing = 4;
+constexpr int kRingReaders = 1 + kEpilogueWarps + 1;
+constexpr int kBarBytes =
+    ((2 * kMaxStages + 6 + 2 * kRing) * 8 + kRing * static_cast<int>(sizeof(Tile)) + 16 + 15) / 16 *
+    16;
 
 // Tiles of up to kFewRows rows hand their accumulator over through shared memory: a thread per row
 // would leave most lanes of the two warps that can read those rows idle and the others with four
@@ -74,15 +81,6 @@ static_assert(smem_bytes(32) <= 232448 && smem_bytes(64) <= 232448 && smem_bytes
 // rows are never stored), which must lie inside the allocation.
 static_assert(stages_for(32) * kBBytes >= 128 * 128, "A over-read stays inside shared memory");
 
-// Where a tile of the list lies.
-struct Tile {
-  int phase;
-  int row0;    // first row of its 128-row slot
-  int rows;    // valid rows in it
-  int expert;
-  int nt;      // weight tile
-};
-
 struct TileList {
   int first[kStreamPhases + 1];  // first tile of each phase, then the end
   __device__ __forceinline__ void load(const StreamArgs& args) {
@@ -93,7 +91,7 @@ struct TileList {
       if (p < args.phases) {
         const GemmArgs& g = args.phase[p].gemm;
         const int row_tiles =
-            g.row_tiles != nullptr ? *g.num_row_tiles : (g.dense_rows + 127) / 128;
+            warp_uniform(g.row_tiles != nullptr ? *g.num_row_tiles : (g.dense_rows + 127) / 128);
         running += row_tiles * g.n_tiles;
       }
     }
@@ -102,7 +100,9 @@ struct TileList {
   __device__ __forceinline__ int total() const { return first[kStreamPhases]; }
   __device__ __forceinline__ Tile locate(const StreamArgs& args, int t) const {
     Tile tile;
-    tile.phase = 0;
+    tile.phase = t < total() ? 0 : -1;
+    tile.row0 = tile.rows = tile.expert = tile.nt = 0;
+    if (tile.phase < 0) return tile;
     int base = 0;
 #pragma unroll
     for (int p = 1; p < kStreamPhases; ++p) {
@@ -117,9 +117,9 @@ struct TileList {
     tile.nt = index - rt * g.n_tiles;
     if (g.row_tiles != nullptr) {
       const RowTile row_tile = g.row_tiles[rt];
-      tile.row0 = row_tile.row0;
-      tile.rows = row_tile.rows;
-      tile.expert = row_tile.expert;
+      tile.row0 = warp_uniform(row_tile.row0);
+      tile.rows = warp_uniform(row_tile.rows);
+      tile.expert = warp_uniform(row_tile.expert);
     } else {
       tile.row0 = rt * 128;
       tile.rows = min(128, g.dense_rows - tile.row0);
@@ -145,23 +145,53 @@ __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async;" ::: "memory");
 }
 
-// Waits (about a second at most) until *count >= target.
+// Waits (about a second at most) until *count >= target; by all lanes of a warp.
 __device__ __forceinline__ bool wait_count(const int32_t* count, int target) {
-  if (load_acquire(count) >= target) return true;
   const long long start = clock64();
-  while (load_acquire(count) < target) {
-    if (clock64() - start > (1ll << 31)) return false;
+  while (!__all_sync(0xffffffffu, load_acquire(count) >= target)) {
+    if (__any_sync(0xffffffffu, clock64() - start > (1ll << 31))) return false;
   }
   return true;
 }
 
-template <int PART>
-__device__ __forceinline__ void issue_scale_copies(uint32_t sf_tmem, uint64_t sfa_desc,
-                                                   uint64_t sfb_desc) {
+// The next tile from the ring, by all lanes of a warp.
+struct RingReader {
+  const volatile Tile* ring;
+  uint32_t full0, empty0;
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ bool next(Tile& tile) {
+    if (!mbar_wait_warp(full0 + slot * 8, phase)) return false;
+    tile.phase = warp_uniform(static_cast<int>(ring[slot].phase));
+    tile.row0 = warp_uniform(static_cast<int>(ring[slot].row0));
+    tile.rows = warp_uniform(static_cast<int>(ring[slot].rows));
+    tile.expert = warp_uniform(static_cast<int>(ring[slot].expert));
+    tile.nt = warp_uniform(static_cast<int>(ring[slot].nt));
+    __syncwarp();
+    if (elect_one()) mbar_arrive_at(empty0 + slot * 8);
+    if (++slot == kRing) {
+      slot = 0;
+      phase ^= 1u;
+    }
+    return true;
+  }
+};
+
+// The scale copies and MMAs of a K block that holds MMAS times 64 elements (copies and MMAs of one
+// thread execute in order).
+template <int MMAS>
+__device__ __forceinline__ void issue_block(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                            uint64_t sfa_desc, uint64_t sfb_desc, uint32_t sf_tmem,
+                                            uint32_t idesc, int kb) {
 #pragma unroll
-  for (int c = PART; c < 4; c += kScaleWarps) {
+  for (int c = 0; c < MMAS; ++c) {
     tcgen05_cp_32x128b_warpx4(sf_tmem + 4 * c, advance_smem_desc(sfa_desc, c * 512));
     tcgen05_cp_32x128b_warpx4(sf_tmem + 16 + 4 * c, advance_smem_desc(sfb_desc, c * 512));
+  }
+#pragma unroll
+  for (int kt = 0; kt < MMAS; ++kt) {
+    tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32), advance_smem_desc(b_desc, kt * 32),
+                     idesc, sf_tmem + 4 * kt, sf_tmem + 16 + 4 * kt, kt != 0 ? 1u : kb != 0 ? 1u : 0u);
   }
 }
 
@@ -180,12 +210,15 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   uint64_t* empty_bar = full_bar + kMaxStages;
   uint64_t* tmem_full_bar = empty_bar + kMaxStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
-  uint64_t* sf_ready_bar = tmem_empty_bar + 2;
-  uint64_t* stored_bar = sf_ready_bar + kMaxStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stored_bar + 2);
+  uint64_t* stored_bar = tmem_empty_bar + 2;
+  uint64_t* ring_full_bar = stored_bar + 2;
+  uint64_t* ring_empty_bar = ring_full_bar + kRing;
+  volatile Tile* ring = reinterpret_cast<volatile Tile*>(ring_empty_bar + kRing);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(
+      reinterpret_cast<uint8_t*>(ring_empty_bar + kRing) + kRing * sizeof(Tile));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int unit = static_cast<int>(blockIdx.x);
   const int units = static_cast<int>(gridDim.x);
@@ -194,12 +227,15 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
-      mbar_init(&sf_ready_bar[s], kScaleWarps);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full_bar[a], 1);
       mbar_init(&tmem_empty_bar[a], 1);
       mbar_init(&stored_bar[a], kEpilogueWarps);
+    }
+    for (int i = 0; i < kRing; ++i) {
+      mbar_init(&ring_full_bar[i], 1);
+      mbar_init(&ring_empty_bar[i], kRingReaders);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -211,72 +247,70 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   float* few_rows = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(full_bar) + kBarBytes);
   const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
   const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
-  const uint32_t sf_ready0 = smem_u32(sf_ready_bar);
+  RingReader reader{ring, smem_u32(ring_full_bar), smem_u32(ring_empty_bar)};
 
-  TileList list;
-  list.load(args);
-  const int total_tiles = list.total();
-
-  if (warp == kSignalWarp) {
-    // ---------------------------------------------------------------- signals
-    // Once the epilogue warps have stored a tile: give its accumulator back, and count the tile
-    // for the down projection.  Making the stores visible first takes some 1500 cycles, which here
-    // nobody waits for.
-    if (lane == 0) {
-      int local = 0;
-      for (int t = unit; t < total_tiles; t += units, ++local) {
-        const Tile tile = list.locate(args, t);
-        const StreamPhase& ph = args.phase[tile.phase];
-        const int acc = local & 1;
-        if (!mbar_wait(&stored_bar[acc], (local >> 1) & 1u)) {
-          report_timeout(args.error, abort_flag);
-          break;
-        }
-        mbar_arrive(&tmem_empty_bar[acc]);
-        if (ph.mode == kGemmUp && ph.ready != nullptr) {
-          __threadfence();
-          add_release(ph.ready + (tile.row0 >> 7), 1);
-        }
+  if (warp == 0) {
+    // --------------------------------------------------------------- producer
+    TileList list;
+    list.load(args);
+    int slot = 0;
+    uint32_t slot_phase = 0;
+    int stage = 0;
+    uint32_t phase = 0;
+    auto advance = [&](int& at, uint32_t& at_phase) {
+      if (++at == stages) {
+        at = 0;
+        at_phase ^= 1u;
       }
-    }
-  } else if (warp == 0 || warp >= kScaleWarp + kScaleWarps) {
-    // ------------------------------------------------------------- producers
-    // Producer p loads the K blocks p, p + kProducers, ... of the CTA's sequence.
-    if (lane == 0) {
-      const int producer = warp == 0 ? 0 : warp - (kScaleWarp + kScaleWarps) + 1;
-      int stage = producer;
-      uint32_t phase = 0;
-      auto advance = [&](int& at, uint32_t& at_phase) {
-        at += kProducers;
-        if (at >= stages) {
-          at -= stages;
-          at_phase ^= 1u;
-        }
-      };
-      int kb = producer;  // K block of the current tile this producer loads next
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units) {
-        const Tile tile = list.locate(args, t);
-        const StreamPhase& ph = args.phase[tile.phase];
-        const GemmArgs& g = ph.gemm;
-        const int k_blocks = g.k_blocks;
-        const int box = tile.rows <= 8 ? 0 : 29 - __clz(tile.rows - 1);  // 8 << box >= rows
-        const uint32_t a_bytes = 8u * 128u << box;
-        const int b_row = tile.nt * kBN;
-        const uint32_t b_bytes = static_cast<uint32_t>(min(kBN, g.N - b_row)) * 128u;
-        const uint8_t* sfa_src =
-            g.sfa + static_cast<size_t>(tile.row0 >> 7) * k_blocks * kSfaBytes;
-        const uint8_t* sfb_src =
-            g.sfb + (static_cast<size_t>(tile.expert) * g.n_tiles + tile.nt) * k_blocks * kSfbBytes;
-        const uint8_t* b_src =
-            g.b_full + (static_cast<size_t>(tile.expert) * g.kb_full * g.N + b_row) * 128;
-        auto load_weights = [&](int block, int at, uint32_t at_phase) {
-          if (!mbar_wait_at(empty0 + at * 8, at_phase ^ 1u)) return false;
+    };
+    // without a ticket word (nothing waits for another tile then) the tiles are dealt out
+    auto take = [&](int dealt) {
+      return args.ticket != nullptr && lane == 0 ? atomicAdd(args.ticket, 1) : dealt;
+    };
+    bool ok = true;
+    int t = warp_uniform(take(unit));
+    while (ok) {
+      const Tile tile = list.locate(args, t);
+      if (!mbar_wait_warp(reader.empty0 + slot * 8, slot_phase ^ 1u)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      if (elect_one()) {
+        ring[slot].phase = tile.phase;
+        ring[slot].row0 = tile.row0;
+        ring[slot].rows = tile.rows;
+        ring[slot].expert = tile.expert;
+        ring[slot].nt = tile.nt;
+        mbar_arrive_at(reader.full0 + slot * 8);
+      }
+      if (++slot == kRing) {
+        slot = 0;
+        slot_phase ^= 1u;
+      }
+      if (tile.phase < 0) break;
+      // The next ticket is on its way while this tile's loads are issued.  (A CTA that waits for
+      // hidden rows holds no up tile then: those come first in the list.)
+      const int next = take(t + units);
+      const StreamPhase& ph = args.phase[tile.phase];
+      const GemmArgs& g = ph.gemm;
+      const int k_blocks = g.k_blocks;
+      const int box = tile.rows <= 8 ? 0 : 29 - __clz(tile.rows - 1);  // 8 << box >= rows
+      const uint32_t a_bytes = 8u * 128u << box;
+      const int b_row = tile.nt * kBN;
+      const uint32_t b_bytes = static_cast<uint32_t>(min(kBN, g.N - b_row)) * 128u;
+      const uint8_t* sfa_src = g.sfa + static_cast<size_t>(tile.row0 >> 7) * k_blocks * kSfaBytes;
+      const uint8_t* sfb_src =
+          g.sfb + (static_cast<size_t>(tile.expert) * g.n_tiles + tile.nt) * k_blocks * kSfbBytes;
+      const uint8_t* b_src =
+          g.b_full + (static_cast<size_t>(tile.expert) * g.kb_full * g.N + b_row) * 128;
+      auto load_weights = [&](int block, int at, uint32_t at_phase) {
+        if (!mbar_wait_warp(empty0 + at * 8, at_phase ^ 1u)) return false;
+        if (elect_one()) {
           const uint32_t bar = full0 + at * 8;
           const bool full_block = block < g.kb_full;
           mbar_arrive_expect_tx_at(bar, a_bytes + (full_block ? b_bytes : kBBytes) + kSfaBytes +
@@ -289,143 +323,132 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
             tma_load_2d_at(b0 + at * kBBytes, &ph.b_tail, 0, tile.expert * g.N + b_row, bar);
           }
           bulk_load_at(sfb0 + at * kSfbBytes, sfb_src + block * kSfbBytes, kSfbBytes, bar);
-          return true;
-        };
-        auto load_rows = [&](int block, int at) {
+        }
+        return true;
+      };
+      auto load_rows = [&](int block, int at) {
+        if (elect_one()) {
           const uint32_t bar = full0 + at * 8;
           tma_load_2d_at(a0 + at * a_room, &ph.a[box], block * 128, tile.row0, bar);
           bulk_load_at(sfa0 + at * kSfaBytes, sfa_src + block * kSfaBytes, kSfaBytes, bar);
-        };
-        if (ph.wait_target > 0 && kb < k_blocks) {
-          const int32_t* count = ph.ready + (tile.row0 >> 7);
-          int at = stage;
-          uint32_t at_phase = phase;
-          ok = load_weights(kb, at, at_phase);
-          advance(at, at_phase);
-          int loaded = kb + kProducers;
-          if (ok && load_acquire(count) < ph.wait_target) {
-            // rows still being written: the weights of the ring's other K blocks go out meanwhile
-            const int ahead = min(stages, k_blocks);
-            for (; loaded < ahead && ok; loaded += kProducers) {
-              ok = load_weights(loaded, at, at_phase);
-              advance(at, at_phase);
-            }
-            ok = ok && wait_count(count, ph.wait_target);
-          }
-          fence_proxy_async();
-          for (; kb < loaded && ok; kb += kProducers) {
-            load_rows(kb, stage);
-            advance(stage, phase);
-          }
         }
-        for (; kb < k_blocks && ok; kb += kProducers) {
-          ok = load_weights(kb, stage, phase);
-          if (ok) load_rows(kb, stage);
+      };
+      int kb = 0;
+      if (ph.wait_target > 0) {
+        const int32_t* count = ph.ready + (tile.row0 >> 7);
+        int at = stage;
+        uint32_t at_phase = phase;
+        ok = load_weights(0, at, at_phase);
+        advance(at, at_phase);
+        int loaded = 1;
+        if (ok && __any_sync(0xffffffffu, load_acquire(count) < ph.wait_target)) {
+          // rows still being written: the weights of the ring's other K blocks go out meanwhile
+          const int ahead = min(stages, k_blocks);
+          for (; loaded < ahead && ok; ++loaded) {
+            ok = load_weights(loaded, at, at_phase);
+            advance(at, at_phase);
+          }
+          ok = ok && wait_count(count, ph.wait_target);
+        }
+        fence_proxy_async();
+        for (; kb < loaded && ok; ++kb) {
+          load_rows(kb, stage);
           advance(stage, phase);
         }
-        kb -= k_blocks;
-        if (!ok) report_timeout(args.error, abort_flag);
       }
+      for (; kb < k_blocks && ok; ++kb) {
+        ok = load_weights(kb, stage, phase);
+        if (ok) load_rows(kb, stage);
+        advance(stage, phase);
+      }
+      if (!ok) report_timeout(args.error, abort_flag);
+      t = warp_uniform(next);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_nvf4(kBN);
-      const uint64_t a_desc0 = make_smem_desc(a0, 0, 1024, 2);
-      const uint64_t b_desc0 = make_smem_desc(b0, 0, 1024, 2);
-      int stage = 0;
-      uint32_t phase = 0;
-      int local = 0;
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units, ++local) {
-        const GemmArgs& g = args.phase[list.locate(args, t).phase].gemm;
-        const int k_blocks = g.k_blocks, last_mmas = g.K / 64 - 4 * (k_blocks - 1);
-        const int acc = local & 1;
-        const uint32_t acc_phase = (local >> 1) & 1u;
-        if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1u)) {
+    // -------------------------------------------------- scale copies and MMAs
+    constexpr uint32_t idesc = make_idesc_nvf4(kBN);
+    const uint64_t a_desc0 = make_smem_desc(a0, 0, 1024, 2);
+    const uint64_t b_desc0 = make_smem_desc(b0, 0, 1024, 2);
+    const uint64_t sfa_desc0 = make_smem_desc(sfa0, 0, 128, 0);
+    const uint64_t sfb_desc0 = make_smem_desc(sfb0, 0, 128, 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t sf_buf = 0;
+    bool ok = true;
+    for (int local = 0; ok; ++local) {
+      Tile tile;
+      const int acc = local & 1;
+      if (!reader.next(tile)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      if (tile.phase < 0) break;
+      if (!mbar_wait_warp(smem_u32(&tmem_empty_bar[acc]), ((local >> 1) & 1u) ^ 1u)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      const GemmArgs& g = args.phase[tile.phase].gemm;
+      const int k_blocks = g.k_blocks, last_mmas = g.K / 64 - 4 * (k_blocks - 1);
+      tcgen05_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * kBN;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_warp(full0 + stage * 8, phase)) {
           report_timeout(args.error, abort_flag);
+          ok = false;
           break;
         }
         tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * kBN;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          // this block's scales are in TMEM, and its operands had landed before they were copied
-          if (!mbar_wait_at(sf_ready0 + stage * 8, phase)) {
-            report_timeout(args.error, abort_flag);
-            ok = false;
-            break;
-          }
-          tcgen05_fence_after();
-          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * a_room);
-          const uint64_t b_desc = advance_smem_desc(b_desc0, stage * kBBytes);
-          const uint32_t sf_tmem = tmem_base + kSfCol + stage * kSfBufCols;
+        const uint64_t a_desc = advance_smem_desc(a_desc0, stage * a_room);
+        const uint64_t b_desc = advance_smem_desc(b_desc0, stage * kBBytes);
+        const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * kSfaBytes);
+        const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * kSfbBytes);
+        const uint32_t sf_tmem = tmem_base + kSfCol + sf_buf * kSfBufCols;
+        if (elect_one()) {
           if (kb + 1 < k_blocks || last_mmas == 4) {
-#pragma unroll
-            for (int kt = 0; kt < 4; ++kt) {
-              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                               advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
-                               sf_tmem + 16 + 4 * kt, kt != 0 ? 1u : kb != 0 ? 1u : 0u);
-            }
+            issue_block<4>(d_tmem, a_desc, b_desc, sfa_desc, sfb_desc, sf_tmem, idesc, kb);
+          } else if (last_mmas == 3) {
+            issue_block<3>(d_tmem, a_desc, b_desc, sfa_desc, sfb_desc, sf_tmem, idesc, kb);
+          } else if (last_mmas == 2) {
+            issue_block<2>(d_tmem, a_desc, b_desc, sfa_desc, sfb_desc, sf_tmem, idesc, kb);
           } else {
-            for (int kt = 0; kt < last_mmas; ++kt) {
-              tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                               advance_smem_desc(b_desc, kt * 32), idesc, sf_tmem + 4 * kt,
-                               sf_tmem + 16 + 4 * kt, (kb | kt) != 0 ? 1u : 0u);
-            }
+            issue_block<1>(d_tmem, a_desc, b_desc, sfa_desc, sfb_desc, sf_tmem, idesc, kb);
           }
           tcgen05_commit_at(empty0 + stage * 8);
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
         }
-        if (ok) tcgen05_commit(&tmem_full_bar[acc]);
+        sf_buf ^= 1u;
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
       }
+      if (ok && elect_one()) tcgen05_commit(&tmem_full_bar[acc]);
     }
-  } else if (warp >= kScaleWarp) {  // (the producers behind them are taken)
-    // ------------------------------------------------------- block-scale copiers
-    // Every stage has TMEM columns of its own: once its operands have landed, the MMAs that read
-    // those columns before are known to be done (the producer waited for them).
-    if (lane == 0) {
-      const int part = warp - kScaleWarp;
-      const uint64_t sfa_desc0 = make_smem_desc(sfa0, 0, 128, 0);
-      const uint64_t sfb_desc0 = make_smem_desc(sfb0, 0, 128, 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units) {
-        const GemmArgs& g = args.phase[list.locate(args, t).phase].gemm;
-        const int k_blocks = g.k_blocks, last_mmas = g.K / 64 - 4 * (k_blocks - 1);
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait_at(full0 + stage * 8, phase)) {
-            report_timeout(args.error, abort_flag);
-            ok = false;
-            break;
-          }
-          tcgen05_fence_after();
-          const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * kSfaBytes);
-          const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * kSfbBytes);
-          const uint32_t sf_tmem = tmem_base + kSfCol + stage * kSfBufCols;
-          if (kb + 1 < k_blocks || last_mmas == 4) {
-            static_assert(kScaleWarps == 2, "one branch per copier");
-            if (part == 0) {
-              issue_scale_copies<0>(sf_tmem, sfa_desc, sfb_desc);
-            } else {
-              issue_scale_copies<1>(sf_tmem, sfa_desc, sfb_desc);
-            }
-          } else {
-            for (int c = part; c < last_mmas; c += kScaleWarps) {
-              tcgen05_cp_32x128b_warpx4(sf_tmem + 4 * c, advance_smem_desc(sfa_desc, c * 512));
-              tcgen05_cp_32x128b_warpx4(sf_tmem + 16 + 4 * c, advance_smem_desc(sfb_desc, c * 512));
-            }
-          }
-          tcgen05_commit_at(sf_ready0 + stage * 8);
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+  } else if (warp == kSignalWarp) {
+    // ---------------------------------------------------------------- signals
+    // Once the epilogue warps have stored a tile: give its accumulator back, and count the tile
+    // for the down projection.  Making the stores visible first takes some 1500 cycles, which here
+    // nobody waits for.
+    for (int local = 0;; ++local) {
+      Tile tile;
+      const int acc = local & 1;
+      if (!reader.next(tile)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      if (tile.phase < 0) break;
+      if (!mbar_wait_warp(smem_u32(&stored_bar[acc]), (local >> 1) & 1u)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      const StreamPhase& ph = args.phase[tile.phase];
+      if (lane == 0) {
+        mbar_arrive(&tmem_empty_bar[acc]);
+        if (ph.mode == kGemmUp && ph.ready != nullptr) {
+          __threadfence();
+          add_release(ph.ready + (tile.row0 >> 7), 1);
         }
       }
+      __syncwarp();
     }
   } else {
     // -------------------------------------------------------------- epilogue
@@ -433,11 +456,15 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
     const int half = (warp - 2) >> 2;       // which half of the tile's columns
     const int r = quarter * 32 + lane;      // row inside the tile == TMEM lane
     constexpr int kHalfChunks = kBN / 16 / 2;
-    int local = 0;
-    for (int t = unit; t < total_tiles; t += units, ++local) {
+    for (int local = 0;; ++local) {
       const int acc = local & 1;
       const uint32_t acc_phase = (local >> 1) & 1u;
-      const Tile tile = list.locate(args, t);
+      Tile tile;
+      if (!reader.next(tile)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      if (tile.phase < 0) break;
       const StreamPhase& ph = args.phase[tile.phase];
       const GemmArgs& g = ph.gemm;
       const bool row_valid = r < tile.rows;
@@ -523,7 +550,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
-  } else if (warp == 0 && args.ready_count > 0) {
+  } else if (warp == 0 && args.ticket != nullptr) {
     // the last CTA leaves the counts at zero for the next launch
     int ticket = 0;
     if (lane == 0) {
@@ -533,7 +560,10 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
     ticket = __shfl_sync(0xffffffffu, ticket, 0);
     if (ticket == units - 1) {
       for (int i = lane; i < args.ready_count; i += 32) args.ready[i] = 0;
-      if (lane == 0) *args.finished = 0;
+      if (lane == 0) {
+        *args.ticket = 0;
+        *args.finished = 0;
+      }
     }
   }
 }

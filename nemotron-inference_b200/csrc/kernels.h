@@ -121,10 +121,12 @@ struct StreamArgs {
   int32_t phases = 0;
   int32_t tile_rows = 128;  // most rows a row tile holds: 32, 64 or 128
   int32_t* error = nullptr;
-  // all `ready` words of the phases, zero between launches, and a CTA ticket behind which the last
-  // CTA zeroes them
+  // all `ready` words of the phases, the ticket the tiles are taken with and the count of CTAs that
+  // are done, all zero between launches (the last CTA zeroes them); ticket == nullptr: tiles are
+  // dealt out, for launches without waits
   int32_t* ready = nullptr;
   int32_t ready_count = 0;
+  int32_t* ticket = nullptr;
   int32_t* finished = nullptr;
 };
 inline int stream_tile_rows(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }

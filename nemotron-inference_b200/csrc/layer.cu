@@ -473,11 +473,11 @@ struct StreamFfn {
 
 // Row slots' completion counts of such launches; zero whenever no launch is running.
 struct StreamCounts {
-  DeviceBuffer words;  // one ticket, then the counts
+  DeviceBuffer words;  // CTAs done, the tile ticket, then the counts
   int capacity = 0;
   void allocate(size_t slots) {
     capacity = static_cast<int>(slots);
-    words.allocate((slots + 1) * sizeof(int32_t), true);
+    words.allocate((slots + 2) * sizeof(int32_t), true);
   }
 };
 
@@ -488,7 +488,8 @@ void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCo
   StreamArgs args;
   args.error = error;
   args.finished = counts.words.as<int32_t>();
-  args.ready = counts.words.as<int32_t>() + 1;
+  args.ticket = counts.words.as<int32_t>() + 1;
+  args.ready = counts.words.as<int32_t>() + 2;
   auto add = [&](const StreamFfn& ffn, bool up, int32_t* ready) {
     StreamPhase* phase = &args.phase[args.phases++];
     const WeightStack& weights = up ? *ffn.up : *ffn.down;
