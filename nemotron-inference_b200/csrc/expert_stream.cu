@@ -17,8 +17,10 @@
 // weights take 800 cycles to arrive; its eight scale copies and four MMAs, issued in order by one
 // warp, take about 300.
 //
-// Roles: warp 0 takes tiles and loads, warp 1 issues scale copies and MMAs, warps 2-9 run
-// epilogues, warp 10 hands finished tiles on.
+// Roles: warp 0 takes tiles and loads weights, warp 11 loads activation rows (and waits for them:
+// finding out and ordering the copies behind it takes over 1000 cycles a tile, which must not hold
+// up the weights), warp 1 issues scale copies and MMAs, warps 2-9 run epilogues, warp 10 hands
+// finished tiles on.
 // Measured, whole pass of the benchmark layer: 64 tokens 196 -> @S1@ us, 256 tokens 205 -> @S2@,
 // 1003 tokens 240 -> @S3@.
 #include <algorithm>
@@ -34,7 +36,8 @@ constexpr int kBN = 128;
 constexpr int kMaxStages = 8;
 constexpr int kEpilogueWarps = 8;  // two per TMEM lane quarter
 constexpr int kSignalWarp = 2 + kEpilogueWarps;
-constexpr int kThreads = (kSignalWarp + 1) * 32;
+constexpr int kRowWarp = kSignalWarp + 1;
+constexpr int kThreads = (kRowWarp + 1) * 32;
 constexpr int kBBytes = kBN * 128;
 constexpr int kSfaBytes = 2048;
 constexpr int kSfbBytes = 2048;     // four groups of 32 weight rows x four MMAs x 16 bytes
@@ -55,7 +58,7 @@ struct Tile {
 
 // The producer hands tiles to the other roles through a ring in shared memory.
 constexpr int kRing = 4;
-constexpr int kRingReaders = 1 + kEpilogueWarps + 1;
+constexpr int kRingReaders = 1 + kEpilogueWarps + 1 + 1;
 constexpr int kBarBytes =
     ((2 * kMaxStages + 6 + 2 * kRing) * 8 + kRing * static_cast<int>(sizeof(Tile)) + 16 + 15) / 16 *
     16;
@@ -144,6 +147,9 @@ __device__ __forceinline__ void add_release(int32_t* p, int v) {
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async;" ::: "memory");
 }
+
+// The smallest activation box (8 << box rows) that holds `rows`.
+__device__ __forceinline__ int box_of(int rows) { return rows <= 8 ? 0 : 29 - __clz(rows - 1); }
 
 // Waits (about a second at most) until *count >= target; by all lanes of a warp.
 __device__ __forceinline__ bool wait_count(const int32_t* count, int target) {
@@ -255,19 +261,13 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   RingReader reader{ring, smem_u32(ring_full_bar), smem_u32(ring_empty_bar)};
 
   if (warp == 0) {
-    // --------------------------------------------------------------- producer
+    // ------------------------------------------------------- tiles and weights
     TileList list;
     list.load(args);
     int slot = 0;
     uint32_t slot_phase = 0;
     int stage = 0;
     uint32_t phase = 0;
-    auto advance = [&](int& at, uint32_t& at_phase) {
-      if (++at == stages) {
-        at = 0;
-        at_phase ^= 1u;
-      }
-    };
     // without a ticket word (nothing waits for another tile then) the tiles are dealt out
     auto take = [&](int dealt) {
       return args.ticket != nullptr && lane == 0 ? atomicAdd(args.ticket, 1) : dealt;
@@ -299,70 +299,75 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       const StreamPhase& ph = args.phase[tile.phase];
       const GemmArgs& g = ph.gemm;
       const int k_blocks = g.k_blocks;
-      const int box = tile.rows <= 8 ? 0 : 29 - __clz(tile.rows - 1);  // 8 << box >= rows
-      const uint32_t a_bytes = 8u * 128u << box;
+      const uint32_t a_bytes = 8u * 128u << box_of(tile.rows);
       const int b_row = tile.nt * kBN;
       const uint32_t b_bytes = static_cast<uint32_t>(min(kBN, g.N - b_row)) * 128u;
-      const uint8_t* sfa_src = g.sfa + static_cast<size_t>(tile.row0 >> 7) * k_blocks * kSfaBytes;
       const uint8_t* sfb_src =
           g.sfb + (static_cast<size_t>(tile.expert) * g.n_tiles + tile.nt) * k_blocks * kSfbBytes;
       const uint8_t* b_src =
           g.b_full + (static_cast<size_t>(tile.expert) * g.kb_full * g.N + b_row) * 128;
-      auto load_weights = [&](int block, int at, uint32_t at_phase) {
-        if (!mbar_wait_warp(empty0 + at * 8, at_phase ^ 1u)) return false;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
+          ok = false;
+          break;
+        }
         if (elect_one()) {
-          const uint32_t bar = full0 + at * 8;
-          const bool full_block = block < g.kb_full;
+          const uint32_t bar = full0 + stage * 8;
+          const bool full_block = kb < g.kb_full;
+          // (the bytes of warp kRowWarp's copies are counted here too)
           mbar_arrive_expect_tx_at(bar, a_bytes + (full_block ? b_bytes : kBBytes) + kSfaBytes +
                                             kSfbBytes);
           if (full_block) {
             // one contiguous, pre-swizzled panel slice: a single bulk copy
-            bulk_load_at(b0 + at * kBBytes, b_src + static_cast<size_t>(block) * g.N * 128, b_bytes,
+            bulk_load_at(b0 + stage * kBBytes, b_src + static_cast<size_t>(kb) * g.N * 128, b_bytes,
                          bar);
           } else {
-            tma_load_2d_at(b0 + at * kBBytes, &ph.b_tail, 0, tile.expert * g.N + b_row, bar);
+            tma_load_2d_at(b0 + stage * kBBytes, &ph.b_tail, 0, tile.expert * g.N + b_row, bar);
           }
-          bulk_load_at(sfb0 + at * kSfbBytes, sfb_src + block * kSfbBytes, kSfbBytes, bar);
+          bulk_load_at(sfb0 + stage * kSfbBytes, sfb_src + kb * kSfbBytes, kSfbBytes, bar);
         }
-        return true;
-      };
-      auto load_rows = [&](int block, int at) {
-        if (elect_one()) {
-          const uint32_t bar = full0 + at * 8;
-          tma_load_2d_at(a0 + at * a_room, &ph.a[box], block * 128, tile.row0, bar);
-          bulk_load_at(sfa0 + at * kSfaBytes, sfa_src + block * kSfaBytes, kSfaBytes, bar);
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
         }
-      };
-      int kb = 0;
-      if (ph.wait_target > 0) {
-        const int32_t* count = ph.ready + (tile.row0 >> 7);
-        int at = stage;
-        uint32_t at_phase = phase;
-        ok = load_weights(0, at, at_phase);
-        advance(at, at_phase);
-        int loaded = 1;
-        if (ok && __any_sync(0xffffffffu, load_acquire(count) < ph.wait_target)) {
-          // rows still being written: the weights of the ring's other K blocks go out meanwhile
-          const int ahead = min(stages, k_blocks);
-          for (; loaded < ahead && ok; ++loaded) {
-            ok = load_weights(loaded, at, at_phase);
-            advance(at, at_phase);
-          }
-          ok = ok && wait_count(count, ph.wait_target);
-        }
-        fence_proxy_async();
-        for (; kb < loaded && ok; ++kb) {
-          load_rows(kb, stage);
-          advance(stage, phase);
-        }
-      }
-      for (; kb < k_blocks && ok; ++kb) {
-        ok = load_weights(kb, stage, phase);
-        if (ok) load_rows(kb, stage);
-        advance(stage, phase);
       }
       if (!ok) report_timeout(args.error, abort_flag);
       t = warp_uniform(next);
+    }
+  } else if (warp == kRowWarp) {
+    // --------------------------------------------------------- activation rows
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    while (ok) {
+      Tile tile;
+      if (!reader.next(tile)) {
+        report_timeout(args.error, abort_flag);
+        break;
+      }
+      if (tile.phase < 0) break;
+      const StreamPhase& ph = args.phase[tile.phase];
+      const GemmArgs& g = ph.gemm;
+      const int k_blocks = g.k_blocks;
+      const int box = box_of(tile.rows);
+      const uint8_t* sfa_src = g.sfa + static_cast<size_t>(tile.row0 >> 7) * k_blocks * kSfaBytes;
+      if (ph.wait_target > 0) {
+        ok = wait_count(ph.ready + (tile.row0 >> 7), ph.wait_target);
+        fence_proxy_async();
+      }
+      for (int kb = 0; kb < k_blocks && ok; ++kb) {
+        ok = mbar_wait_warp(empty0 + stage * 8, phase ^ 1u);
+        if (ok && elect_one()) {
+          const uint32_t bar = full0 + stage * 8;
+          tma_load_2d_at(a0 + stage * a_room, &ph.a[box], kb * 128, tile.row0, bar);
+          bulk_load_at(sfa0 + stage * kSfaBytes, sfa_src + kb * kSfaBytes, kSfaBytes, bar);
+        }
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+      if (!ok) report_timeout(args.error, abort_flag);
     }
   } else if (warp == 1) {
     // -------------------------------------------------- scale copies and MMAs
