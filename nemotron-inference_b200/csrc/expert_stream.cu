@@ -575,9 +575,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
 
 }  // namespace
 
-GemmVariantInfo stream_variant_info() {
-  return GemmVariantInfo{kBN, 128, 4, kSfbBytes, smem_bytes(128), kBN};
-}
+GemmTileInfo stream_tile_info() { return GemmTileInfo{kBN, 4, kSfbBytes, kBN}; }
 
 cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, cudaStream_t stream) {
   if (args.phases < 1 || args.phases > kStreamPhases || num_sms < 1 ||

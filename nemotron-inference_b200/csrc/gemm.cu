@@ -19,14 +19,9 @@
 // 32-lane x 16-byte form; activations use the reference's 128x4 tile order
 // (runtime/src/backend/nvfp4_scale_layout.cpp:14-28) unchanged.
 //
-// Warp roles (384 threads): warp 0 = TMA producer, warp 1 = MMA issuer and TMEM
-// owner, warps 2-9 = epilogue (two warps per TMEM lane quarter, splitting the
-// tile's columns), warps 10-11 = block-scale copiers.  The twelve scale copies
-// of a K block take longer to issue than its four MMAs and a thread's tcgen05
-// operations execute in order, so the copies have threads of their own and run
-// one K block ahead of the MMAs into double-buffered TMEM columns.  Every
-// mbarrier wait is bounded; on a timeout the CTA records kDevWaitTimeout and
-// unwinds.
+// This file holds the kernel of the batches that are bound by arithmetic, csrc/expert_stream.cu
+// that of the batches bound by reading the weights.  Every mbarrier wait is bounded; on a timeout
+// the CTA records kDevWaitTimeout and unwinds.
 #include <algorithm>
 #include <cstdlib>
 
@@ -38,72 +33,8 @@ namespace nmoe {
 namespace {
 
 constexpr int kEpilogueWarps = 8;  // two per TMEM lane quarter (sixteen measured no faster)
-constexpr int kScaleWarp = 2 + kEpilogueWarps;  // issues the block-scale copies into TMEM
-constexpr int kScaleWarps = 2;  // the copies are split between this many issuing threads
-                                // (four measured no faster than two)
-constexpr int kProducers = 1;
-constexpr int kGemmThreads = (1 + kEpilogueWarps + kScaleWarps + kProducers) * 32;
 
-template <int BN_, int A_ROWS_, int SFB_GS_, int STAGES_, bool ROW_STAGING_ = true>
-struct TileCfg {
-  static constexpr int BN = BN_;
-  static constexpr int A_ROWS = A_ROWS_;
-  static constexpr int SFB_GS = SFB_GS_;  // 32-row scale groups stored per K tile (multiple of 4:
-                                          // an MMA's scale address must be 4-column aligned)
-  static constexpr int STAGES = STAGES_;
-  static constexpr bool PAIR = false;  // (tile_rows_of: one row tile per tile unit)
-  static constexpr int B_ROWS = BN_;
-  static constexpr int A_BYTES = A_ROWS * 128;
-  static constexpr int B_BYTES = B_ROWS * 128;
-  static constexpr int SFA_BYTES = 2048;
-  static constexpr int SFB_BYTES = SFB_GS * 512;
-  static constexpr int STAGE_TX = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;
-  static constexpr int ACC_STRIDE = BN;  // TMEM columns per accumulator
-  // block scales are double-buffered in TMEM so that the copies of K block i+1
-  // do not have to wait for the MMAs of K block i to finish reading theirs
-  static constexpr int SF_BUFS = 2;
-  static constexpr int SF_BUF_COLS = 16 + 4 * SFB_GS;
-  static constexpr int SFA_COL = 2 * ACC_STRIDE;
-  static constexpr int SFB_COL = SFA_COL + 16;
-  static constexpr int TMEM_USED = SFA_COL + SF_BUFS * SF_BUF_COLS;
-  static constexpr int TMEM_COLS = TMEM_USED <= 32 ? 32 : TMEM_USED <= 64 ? 64 : TMEM_USED <= 128 ? 128 : TMEM_USED <= 256 ? 256 : 512;
-  // full and empty per stage; accumulator full / empty; scale-ready
-  // (rounded up: the epilogue's staging area behind it is accessed 16 bytes at a time)
-  static constexpr int BAR_BYTES = ((2 * STAGES + 4 + SF_BUFS) * 8 + 16 + 15) / 16 * 16;
-  // staging for the row-scattering epilogue of the down projection
-  static constexpr bool ROW_STAGING = ROW_STAGING_;
-  static constexpr int EPI_STAGE_BYTES = ROW_STAGING_ ? kEpilogueWarps * kStageBytes : 0;
-  // The MMA always reads 128 A rows; with a smaller box the tail rows alias the
-  // following stages, which is harmless (those output rows are never stored)
-  // but must stay inside the allocation: the B region follows the A region.
-  static constexpr int SMEM_BYTES =
-      STAGES * (A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES) + BAR_BYTES + EPI_STAGE_BYTES + 1024;
-  static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "BN");
-  static_assert(SFB_GS % 4 == 0 && SFB_GS * 32 >= BN, "weight scale groups");
-  static_assert(TMEM_USED <= 512, "TMEM budget");
-  static_assert(STAGES * B_BYTES >= 128 * 128, "A over-read must stay inside shared memory");
-  static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-};
-
-using CfgPrefillUp = TileCfg<208, 128, 8, 4, false>;
-using CfgPrefillDown = TileCfg<192, 128, 8, 4>;
-
-// All scale copies of one full K block that fall to copier `PART`; compile-time
-// indices only, so that no copy carries a run-time predicate.
-template <class C, int PART>
-__device__ __forceinline__ void issue_scale_copies(uint32_t sf_tmem, uint64_t sfa_desc,
-                                                   uint64_t sfb_desc) {
-#pragma unroll
-  for (int c = PART; c < 4; c += kScaleWarps) {
-    tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFA_COL + 4 * c, advance_smem_desc(sfa_desc, c * 512));
-  }
-#pragma unroll
-  for (int c = PART; c < C::SFB_GS; c += kScaleWarps) {
-    tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFB_COL + 4 * c, advance_smem_desc(sfb_desc, c * 512));
-  }
-}
-
-// The row tile a CTA works on in tile unit `rt` (a row tile, or a pair of them).
+// The row tile of CTA `cta_rank` in tile unit `rt`, a pair of row tiles.
 struct TileRows {
   int row0;      // first row of the 128-row slot
   int rows;      // valid rows in it
@@ -111,13 +42,12 @@ struct TileRows {
   int expert;
 };
 
-template <class C>
 __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, int num_row_tiles,
                                                  uint32_t cta_rank) {
   TileRows t;
-  const int index = C::PAIR ? 2 * rt + static_cast<int>(cta_rank) : rt;
+  const int index = 2 * rt + static_cast<int>(cta_rank);
   if (args.row_tiles != nullptr) {
-    // the plan gives every expert an even number of tiles when pairs consume them
+    // the plan gives every expert an even number of tiles
     const int safe = min(index, num_row_tiles - 1);
     t.row0 = args.row_tiles[safe].row0;
     t.rows = index < num_row_tiles ? args.row_tiles[safe].rows : 0;
@@ -132,308 +62,8 @@ __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, i
   return t;
 }
 
-template <class C, int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) {
-  const CUtensorMap& tmap_a = maps.a;
-  const CUtensorMap& tmap_b_tail = maps.b_tail;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
-                                             ~static_cast<uintptr_t>(1023u));
-  uint8_t* sA = smem;
-  uint8_t* sB = sA + C::STAGES * C::A_BYTES;
-  uint8_t* sSFA = sB + C::STAGES * C::B_BYTES;
-  uint8_t* sSFB = sSFA + C::STAGES * C::SFA_BYTES;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sSFB + C::STAGES * C::SFB_BYTES);
-  uint64_t* empty_bar = full_bar + C::STAGES;
-  uint64_t* tmem_full_bar = empty_bar + C::STAGES;
-  uint64_t* tmem_empty_bar = tmem_full_bar + 2;
-  uint64_t* sf_ready_bar = tmem_empty_bar + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sf_ready_bar + C::SF_BUFS);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint8_t* stage_base = reinterpret_cast<uint8_t*>(full_bar) + C::BAR_BYTES;  // row staging
-
-  const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
-  const int lane = threadIdx.x & 31;
-  const int unit = static_cast<int>(blockIdx.x);
-  const int units = static_cast<int>(gridDim.x);
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(&tmem_full_bar[a], 1);
-      mbar_init(&tmem_empty_bar[a], kEpilogueWarps);
-    }
-    for (int b = 0; b < C::SF_BUFS; ++b) {
-      mbar_init(&sf_ready_bar[b], kScaleWarps);
-    }
-    *abort_flag = 0;
-    fence_barrier_init();
-    prefetch_tensormap(&tmap_a);
-    prefetch_tensormap(&tmap_b_tail);
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
-    tmem_relinquish();
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = warp_uniform(*tmem_slot);
-
-  const int num_row_tiles = warp_uniform(
-      args.row_tiles != nullptr ? *args.num_row_tiles : (args.dense_rows + 127) / 128);
-  const int total_tiles = num_row_tiles * args.n_tiles;
-
-  if (warp == 0 || warp >= kScaleWarp + kScaleWarps) {
-    // ------------------------------------------------------------- producers
-    // Producer p loads the K blocks p, p + kProducers, ... of the CTA's sequence.
-    const int producer = warp == 0 ? 0 : warp - (kScaleWarp + kScaleWarps) + 1;
-    static_assert(kProducers <= C::STAGES, "a producer advances at most a ring at a time");
-    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA),
-                   sfb0 = smem_u32(sSFB);
-    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
-    int stage = producer % C::STAGES;
-    uint32_t phase = 0;
-    int kb = producer;  // K block of the current tile this producer loads next
-    bool ok = true;
-    for (int t = unit; t < total_tiles && ok; t += units) {
-      const int rt = t / args.n_tiles;
-      const int nt = t - rt * args.n_tiles;
-      TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, 0u);
-      rows.load_row0 = warp_uniform(rows.load_row0);
-      const int expert = warp_uniform(rows.expert);
-      const uint8_t* sfa_src =
-          args.sfa + static_cast<size_t>(rows.load_row0 >> 7) * args.k_blocks * C::SFA_BYTES;
-      const uint8_t* sfb_src = args.sfb + (static_cast<size_t>(expert) * args.n_tiles + nt) *
-                                              args.k_blocks * C::SFB_BYTES;
-      // weights are stored K-block-major: [expert][k block][row][128 B], then the
-      // partial last K block as [expert][row][tail bytes]
-      const int b_row = nt * C::BN;
-      const uint8_t* b_src =
-          args.b_full + (static_cast<size_t>(expert) * args.kb_full * args.N + b_row) * 128;
-      for (; kb < args.k_blocks; kb += kProducers) {
-        if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
-          report_timeout(args.error, abort_flag);
-          ok = false;
-          break;
-        }
-        if (elect_one()) {
-          const uint32_t bar = full0 + stage * 8;
-          mbar_arrive_expect_tx_at(bar, C::STAGE_TX);
-          tma_load_2d_at(a0 + stage * C::A_BYTES, &tmap_a, kb * 128, rows.load_row0, bar);
-          if (kb < args.kb_full) {
-            // one contiguous, pre-swizzled panel slice: a single bulk copy
-            bulk_load_at(b0 + stage * C::B_BYTES, b_src + static_cast<size_t>(kb) * args.N * 128,
-                         C::B_BYTES, bar);
-          } else {
-            tma_load_2d_at(b0 + stage * C::B_BYTES, &tmap_b_tail, 0, expert * args.N + b_row, bar);
-          }
-          bulk_load_at(sfa0 + stage * C::SFA_BYTES, sfa_src + kb * C::SFA_BYTES, C::SFA_BYTES, bar);
-          bulk_load_at(sfb0 + stage * C::SFB_BYTES, sfb_src + kb * C::SFB_BYTES, C::SFB_BYTES, bar);
-        }
-        stage += kProducers;
-        if (stage >= C::STAGES) {
-          stage -= C::STAGES;
-          phase ^= 1u;
-        }
-      }
-      kb -= args.k_blocks;
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = make_idesc_nvf4(C::BN);
-    const uint64_t a_desc0 = make_smem_desc(smem_u32(sA), 0, 1024, 2);
-    const uint64_t b_desc0 = make_smem_desc(smem_u32(sB), 0, 1024, 2);
-    const uint32_t empty0 = smem_u32(empty_bar), sf_ready0 = smem_u32(sf_ready_bar);
-    const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
-    int stage = 0;
-    int local = 0;
-    uint32_t sf_buf = 0, sf_phase = 0;
-    bool ok = true;
-    for (int t = unit; t < total_tiles && ok; t += units, ++local) {
-      const int acc = local & 1;
-      const uint32_t acc_phase = (local >> 1) & 1u;
-      // the epilogue has drained this accumulator
-      if (!mbar_wait_warp(smem_u32(&tmem_empty_bar[acc]), acc_phase ^ 1u)) {
-        report_timeout(args.error, abort_flag);
-        break;
-      }
-      tcgen05_fence_after();
-      const uint32_t d_tmem = tmem_base + acc * C::ACC_STRIDE;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        // this block's scales are in TMEM, and its operands had landed before they were copied
-        if (!mbar_wait_warp(sf_ready0 + sf_buf * 8, sf_phase)) {
-          report_timeout(args.error, abort_flag);
-          ok = false;
-          break;
-        }
-        tcgen05_fence_after();
-        const uint64_t a_desc = advance_smem_desc(a_desc0, stage * C::A_BYTES);
-        const uint64_t b_desc = advance_smem_desc(b_desc0, stage * C::B_BYTES);
-        const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
-        const bool issue = elect_one();
-        if (issue && (kb + 1 < k_blocks || last_mmas == 4)) {
-#pragma unroll
-          for (int kt = 0; kt < 4; ++kt) {
-            tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                             advance_smem_desc(b_desc, kt * 32), idesc,
-                             sf_tmem + C::SFA_COL + 4 * kt,
-                             sf_tmem + C::SFB_COL + C::SFB_GS * kt,
-                             kt != 0 ? 1u : kb != 0 ? 1u : 0u);
-          }
-        } else if (issue) {
-          for (int kt = 0; kt < last_mmas; ++kt) {
-            tcgen05_mma_nvf4(d_tmem, advance_smem_desc(a_desc, kt * 32),
-                             advance_smem_desc(b_desc, kt * 32), idesc,
-                             sf_tmem + C::SFA_COL + 4 * kt,
-                             sf_tmem + C::SFB_COL + C::SFB_GS * kt, (kb | kt) != 0 ? 1u : 0u);
-          }
-        }
-        // frees the stage for the producer and, SF_BUFS K blocks later, this block's scale
-        // columns for the copier
-        if (issue) tcgen05_commit_at(empty0 + stage * 8);
-        if (++sf_buf == C::SF_BUFS) {
-          sf_buf = 0;
-          sf_phase ^= 1u;
-        }
-        if (++stage == C::STAGES) stage = 0;
-      }
-      if (ok && elect_one()) tcgen05_commit(&tmem_full_bar[acc]);
-    }
-  } else if (warp >= kScaleWarp) {  // (the producers behind them are taken)
-    // ------------------------------------------------------- block-scale copiers
-    // The copies of one K block's scales into TMEM take longer to issue than
-    // its MMAs; threads of their own let them run ahead of the MMA thread.
-    const int part = warp - kScaleWarp;
-    const uint64_t sfa_desc0 = make_smem_desc(smem_u32(sSFA), 0, 128, 0);
-    const uint64_t sfb_desc0 = make_smem_desc(smem_u32(sSFB), 0, 128, 0);
-    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
-    const uint32_t sf_ready0 = smem_u32(sf_ready_bar);
-    const int k_blocks = args.k_blocks, last_mmas = args.K / 64 - 4 * (k_blocks - 1);
-    int stage = 0;
-    uint32_t phase = 0;
-    uint32_t sf_buf = 0;
-    // the scale columns written now were last read by the MMAs of the K block
-    // SF_BUFS iterations back; those MMAs also release that block's stage
-    int old_stage = 0;
-    uint32_t old_phase = 0;
-    int unread = C::SF_BUFS;  // buffers nothing has read yet
-    bool ok = true;
-    for (int t = unit; t < total_tiles && ok; t += units) {
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        bool ready = mbar_wait_warp(full0 + stage * 8, phase);
-        if (unread > 0) {
-          --unread;
-        } else {
-          ready = ready && mbar_wait_warp(empty0 + old_stage * 8, old_phase);
-          if (++old_stage == C::STAGES) {
-            old_stage = 0;
-            old_phase ^= 1u;
-          }
-        }
-        if (!ready) {
-          report_timeout(args.error, abort_flag);
-          ok = false;
-          break;
-        }
-        tcgen05_fence_after();
-        const uint64_t sfa_desc = advance_smem_desc(sfa_desc0, stage * C::SFA_BYTES);
-        const uint64_t sfb_desc = advance_smem_desc(sfb_desc0, stage * C::SFB_BYTES);
-        const uint32_t sf_tmem = tmem_base + sf_buf * C::SF_BUF_COLS;
-        // a partial last K block needs the scales of the MMAs it issues only;
-        // the full block keeps its copies free of run-time predicates, which
-        // slow their issue down considerably
-        const bool issue = elect_one();
-        if (!issue) {
-        } else if (kb + 1 < k_blocks || last_mmas == 4) {
-          static_assert(kScaleWarps == 2, "one branch per copier");
-          if (part == 0) {
-            issue_scale_copies<C, 0>(sf_tmem, sfa_desc, sfb_desc);
-          } else {
-            issue_scale_copies<C, 1>(sf_tmem, sfa_desc, sfb_desc);
-          }
-        } else {
-          for (int c = part; c < last_mmas; c += kScaleWarps) {
-            tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFA_COL + 4 * c,
-                                      advance_smem_desc(sfa_desc, c * 512));
-          }
-          for (int c = part; c < last_mmas * (C::SFB_GS / 4); c += kScaleWarps) {
-            tcgen05_cp_32x128b_warpx4(sf_tmem + C::SFB_COL + 4 * c,
-                                      advance_smem_desc(sfb_desc, c * 512));
-          }
-        }
-        if (issue) tcgen05_commit_at(sf_ready0 + sf_buf * 8);
-        if (++sf_buf == C::SF_BUFS) sf_buf = 0;
-        if (++stage == C::STAGES) {
-          stage = 0;
-          phase ^= 1u;
-        }
-      }
-    }
-  } else {
-    // -------------------------------------------------------------- epilogue
-    const int quarter = warp & 3;           // TMEM lanes a warp may read: 32 * (warp % 4)
-    const int group = (warp - 2) >> 2;      // which share of the tile's columns
-    const int r = quarter * 32 + lane;      // row inside the tile == TMEM lane
-    int local = 0;
-    for (int t = unit; t < total_tiles; t += units, ++local) {
-      const int acc = local & 1;
-      const uint32_t acc_phase = (local >> 1) & 1u;
-      const int rt = t / args.n_tiles;
-      const int nt = t - rt * args.n_tiles;
-      const TileRows tile = tile_rows_of<C>(args, rt, num_row_tiles, 0u);
-      const int row0 = tile.row0, rows = tile.rows, expert = tile.expert;
-      const bool row_valid = r < rows;
-      const int grow = row0 + r;
-      float scale = args.w_tensor_scale[expert];
-      if (args.a_tensor_scale != nullptr && row_valid) scale *= args.a_tensor_scale[grow];
-
-      if (!mbar_wait(&tmem_full_bar[acc], acc_phase)) {
-        report_timeout(args.error, abort_flag);
-        break;
-      }
-      tcgen05_fence_after();
-      const uint32_t t_addr =
-          tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * C::ACC_STRIDE;
-      const int n0 = nt * C::BN;
-      // the warps of a lane quarter split the tile's 16-column chunks
-      constexpr int kChunks = C::BN / 16;
-      constexpr int kGroups = kEpilogueWarps / 4;
-      const int chunk_begin = kChunks * group / kGroups;
-      const int chunk_end = kChunks * (group + 1) / kGroups;
-
-      if constexpr (MODE == kGemmUp) {
-        epilogue_quantise<1>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
-      } else {
-        const unsigned long long dest = row_valid ? output_row_address(args, grow) : 0ull;
-        const float wt = row_valid && args.row_weight != nullptr ? args.row_weight[grow] : 1.0f;
-        epilogue_rows(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt,
-                      stage_base + (warp - 2) * kStageBytes);
-      }
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&tmem_empty_bar[acc]);
-      }
-    }
-  }
-
-  tcgen05_fence_before();
-  __syncthreads();
-  // neither CTA of a pair leaves while the other may still read its shared memory
-  // or signal its barriers
-  if (warp == 1) {
-    tcgen05_fence_after();
-    tmem_dealloc(tmem_base, C::TMEM_COLS);
-  }
-}
-
 // ---------------------------------------------------------------------------
-// CTA-pair kernel (kVariantPair): one 256 x kPairBN tile per cluster of two CTAs
+// CTA-pair kernel: one 256 x kPairBN tile per cluster of two CTAs
 // (tcgen05.mma.cta_group::2, M = 256).
 //
 // What bounds a K block is shared memory: at 128 bytes a cycle the copies of a 128 x 208 tile of
@@ -475,14 +105,9 @@ static_assert(kPairBBytes % 1024 == 0, "stage regions keep the 1024-byte swizzle
 static_assert(pair_smem_bytes(kGemmUp) <= 232448 && pair_smem_bytes(kGemmDown) <= 232448,
               "shared memory budget");
 
-struct PairShape {  // what tile_rows_of reads
-  static constexpr bool PAIR = true;
-};
-
 template <int MODE>
 __global__ void __launch_bounds__(kPairThreads, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs args) {
-  using C = PairShape;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
                                              ~static_cast<uintptr_t>(1023u));
@@ -551,7 +176,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
     for (int t = unit; t < total_tiles && ok; t += units) {
       const int rt = t / args.n_tiles;
       const int nt = t - rt * args.n_tiles;
-      const TileRows rows = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
+      const TileRows rows = tile_rows_of(args, rt, num_row_tiles, cta_rank);
       const int load_row0 = warp_uniform(rows.load_row0);
       const int expert = warp_uniform(rows.expert);
       // the scale maps' rows are 1024 bytes: two to a K block of activations, four to one of weights
@@ -684,7 +309,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       const uint32_t acc_phase = (local >> 1) & 1u;
       const int rt = t / args.n_tiles;
       const int nt = t - rt * args.n_tiles;
-      const TileRows tile = tile_rows_of<C>(args, rt, num_row_tiles, cta_rank);
+      const TileRows tile = tile_rows_of(args, rt, num_row_tiles, cta_rank);
       const bool row_valid = r < tile.rows;
       const int grow = tile.row0 + r;
       float scale = args.w_tensor_scale[tile.expert];
@@ -749,41 +374,6 @@ cudaError_t launch_pair(const GemmMaps& maps, const GemmArgs& args, int num_sms,
   config.attrs = &attribute;
   config.numAttrs = 1;
   return cudaLaunchKernelEx(&config, kernel, maps, args);
-}
-
-template <class C, int MODE>
-cudaError_t launch_kernel(const GemmMaps& maps, const GemmArgs& args, int grid,
-                          cudaStream_t stream) {
-  auto kernel = grouped_gemm_kernel<C, MODE>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-  if (err != cudaSuccess) return err;
-  kernel<<<grid, kGemmThreads, C::SMEM_BYTES, stream>>>(maps, args);
-  return cudaGetLastError();
-}
-
-template <class C>
-cudaError_t launch_cfg(GemmMode mode, const GemmMaps& maps, const GemmArgs& args, int num_sms,
-                       cudaStream_t stream) {
-  // one persistent CTA per SM, fewer when there is less work
-  int grid = num_sms;
-  if (args.row_tiles == nullptr) {
-    const int tiles = ((args.dense_rows + 127) / 128) * args.n_tiles;
-    if (tiles < grid) grid = tiles;
-  }
-  if (grid < 1) grid = 1;
-  if (mode == kGemmUp) {
-    return launch_kernel<C, kGemmUp>(maps, args, grid, stream);
-  } else if constexpr (C::ROW_STAGING) {
-    return launch_kernel<C, kGemmDown>(maps, args, grid, stream);
-  } else {
-    return cudaErrorInvalidValue;  // this tile shape has no staging for the down epilogue
-  }
-}
-
-template <class C>
-GemmVariantInfo info_of() {
-  return GemmVariantInfo{C::BN, C::A_ROWS, C::SFB_GS, C::SFB_BYTES, C::SMEM_BYTES, C::B_ROWS};
 }
 
 __global__ void relayout_weight_scales_kernel(const uint8_t* __restrict__ src, int experts, int N,
@@ -861,28 +451,15 @@ cudaError_t relayout_weight_packed(const uint8_t* row_major, int experts, int N,
   return cudaGetLastError();
 }
 
-GemmVariantInfo gemm_variant_info(GemmVariant v) {
-  switch (v) {
-    case kVariantPrefillUp: return info_of<CfgPrefillUp>();
-    case kVariantPrefillDown: return info_of<CfgPrefillDown>();
-    case kVariantPair:
-      return GemmVariantInfo{kPairBN, 128, kPairSfbGroups, kPairSfbBytes, pair_smem_bytes(kGemmUp),
-                             kPairBRows};
-    default: return GemmVariantInfo{0, 0, 0, 0, 0, 0};
-  }
+GemmTileInfo pair_tile_info() {
+  return GemmTileInfo{kPairBN, kPairSfbGroups, kPairSfbBytes, kPairBRows};
 }
 
-cudaError_t launch_grouped_gemm(GemmVariant v, GemmMode mode, const GemmMaps& maps,
-                                const GemmArgs& args, int num_sms, cudaStream_t stream) {
-  switch (v) {
-    case kVariantPrefillUp: return launch_cfg<CfgPrefillUp>(mode, maps, args, num_sms, stream);
-    case kVariantPrefillDown: return launch_cfg<CfgPrefillDown>(mode, maps, args, num_sms, stream);
-    case kVariantPair:
-      if (num_sms < 2) return cudaErrorInvalidValue;
-      return mode == kGemmUp ? launch_pair<kGemmUp>(maps, args, num_sms, stream)
-                             : launch_pair<kGemmDown>(maps, args, num_sms, stream);
-    default: return cudaErrorInvalidValue;
-  }
+cudaError_t launch_pair_gemm(GemmMode mode, const GemmMaps& maps, const GemmArgs& args, int num_sms,
+                             cudaStream_t stream) {
+  if (num_sms < 2) return cudaErrorInvalidValue;
+  return mode == kGemmUp ? launch_pair<kGemmUp>(maps, args, num_sms, stream)
+                         : launch_pair<kGemmDown>(maps, args, num_sms, stream);
 }
 
 size_t weight_scale_layout_bytes(int experts, int N, int K, int bn, int sfb_groups) {

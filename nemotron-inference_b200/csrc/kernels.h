@@ -71,30 +71,18 @@ struct GemmArgs {
   int32_t* error = nullptr;           // device error slot (DeviceError)
 };
 
-// Tile shapes compiled into the library.  The block scales of every MMA must
-// start on a 4-column TMEM boundary, so a weight tile stores its scales in
-// whole groups of 128 rows.
-enum GemmVariant : int {
-  kVariantPrefillUp = 0,    // BN 208, 128-row A box
-  kVariantPrefillDown = 1,  // BN 192, 128-row A box
-  kVariantPair = 2,         // 256 x 208 over a CTA pair (cta_group::2), both epilogues
-  kVariantCount = 3,
+// A kernel's weight tile.  The block scales of every MMA must start on a 4-column TMEM boundary, so
+// a weight tile stores its scales in whole groups of 128 rows.
+struct GemmTileInfo {
+  int bn;          // output features per tile
+  int sfb_groups;  // 32-row groups of weight scales stored per K-tile
+  int sfb_bytes;   // bytes of weight scales per (n_tile, k_block)
+  int b_rows;      // weight rows one CTA stages per K block (half a tile in a pair)
 };
 
-struct GemmVariantInfo {
-  int bn;            // output features per tile
-  int a_rows;        // rows of the activation box / valid rows per row tile
-  int sfb_groups;    // 32-row groups of weight scales stored per K-tile
-  int sfb_bytes;     // bytes of weight scales per (n_tile, k_block)
-  int smem_bytes;    // dynamic shared memory of the kernel
-  int b_rows;        // weight rows one CTA stages per K block (half a tile in a pair)
-};
-
-// Tensor maps of one GEMM launch.  `a` (activation rows, 128-byte swizzle) and `b_tail`
-// (the partial last K block of the weights) are used by every variant; the CTA-pair
-// variants also load the full weight K blocks through a map (`b_full`: the K-block-major
-// panels as [rows][128 B], no swizzle), so that both CTAs' copies can complete on the
-// leader's barrier; b_full: rows of eight weight rows' 128 bytes, 1024 bytes each).
+// Tensor maps of a CTA-pair GEMM launch.  `a`: activation rows, 128-byte swizzle; `b_full`: the full
+// weight K blocks, the K-block-major panels as rows of eight weight rows' 128 bytes, no swizzle;
+// `b_tail`: the partial last K block of the weights.
 struct GemmMaps {
   CUtensorMap a;
   CUtensorMap b_tail;
@@ -132,10 +120,12 @@ struct StreamArgs {
 inline int stream_tile_rows(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
 cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, cudaStream_t stream);
 
-GemmVariantInfo gemm_variant_info(GemmVariant v);
-GemmVariantInfo stream_variant_info();
-cudaError_t launch_grouped_gemm(GemmVariant v, GemmMode mode, const GemmMaps& maps,
-                                const GemmArgs& args, int num_sms, cudaStream_t stream);
+GemmTileInfo stream_tile_info();
+GemmTileInfo pair_tile_info();
+// 256 x 208 tiles over pairs of CTAs (csrc/gemm.cu): the batches bound by arithmetic.  A grouped
+// schedule gives every expert an even number of row tiles.  Needs two SMs.
+cudaError_t launch_pair_gemm(GemmMode mode, const GemmMaps& maps, const GemmArgs& args, int num_sms,
+                             cudaStream_t stream);
 
 // Packed weights [experts][N][K/2] -> K-block-major (device to device): every
 // (expert, 128-byte K block) becomes a contiguous [N][128 B] panel in `full`, so a

@@ -188,10 +188,9 @@ void validate_matrix(const nmoe_nvfp4_matrix& m, size_t rows, size_t cols, const
 // A stack of same-shaped NVFP4 matrices resident in HBM with the scale layouts
 // and tensor maps of every GEMM tile shape that may consume it.
 // ---------------------------------------------------------------------------
-// kClassPair: 256 x 208 tiles over CTA pairs (cta_group::2), each CTA staging half of the
-// weight tile.
+// kClassPair: csrc/gemm.cu, 256 x 208 tiles over CTA pairs, the batches bound by arithmetic.
 // kClassStream: csrc/expert_stream.cu, the batches bound by reading the weights.
-enum TileClass : int { kClassPrefill = 0, kClassStream = 1, kClassPair = 2 };
+enum TileClass : int { kClassPair = 0, kClassStream = 1 };
 
 struct WeightStack {
   int experts = 0;
@@ -204,36 +203,29 @@ struct WeightStack {
   DeviceBuffer packed_tail;   // [experts][n][tail_pitch]
   int kb_full = 0;
   DeviceBuffer tensor_scale;  // [experts]
-  DeviceBuffer sf_prefill;    // scale layout for the prefill tile of this projection
   DeviceBuffer sf_stream;     // scale layout for the BN=128 tiles
   DeviceBuffer sf_pair;       // scale layout for the CTA-pair tile
-  GemmVariant prefill_variant = kVariantPrefillUp;
   // tensor maps exist only for the partial last K block; full K blocks are
   // plain bulk copies of contiguous, pre-swizzled panels
-  CUtensorMap tail_prefill;
   CUtensorMap tail_stream;
   CUtensorMap tail_pair;
   CUtensorMap sf_pair_map;
   CUtensorMap full_pair;  // the K-block-major panels as [rows][1024 B], for the CTA-pair variant
 
-  void upload(const nmoe_nvfp4_matrix* matrices, int count, int rows, int cols, bool is_up,
+  void upload(const nmoe_nvfp4_matrix* matrices, int count, int rows, int cols,
               const char* name, cudaStream_t stream) {
     experts = count;
     n = rows;
     k = cols;
-    prefill_variant = is_up ? kVariantPrefillUp : kVariantPrefillDown;
     const size_t packed_each = static_cast<size_t>(rows) * cols / 2;
     const size_t sf_each = static_cast<size_t>(rows) * (cols / 16);
     tensor_scale.allocate(sizeof(float) * count);
     for (int e = 0; e < count; ++e) validate_matrix(matrices[e], rows, cols, name);
-    const GemmVariantInfo pi = gemm_variant_info(prefill_variant);
-    const GemmVariantInfo di = stream_variant_info();
-    const int pair_rows = gemm_variant_info(kVariantPair).b_rows;
-    const size_t sf_prefill_each = weight_scale_layout_bytes(1, rows, cols, pi.bn, pi.sfb_groups);
+    const GemmTileInfo di = stream_tile_info();
     const size_t sf_stream_each = weight_scale_layout_bytes(1, rows, cols, di.bn, di.sfb_groups);
-    const GemmVariantInfo qi = gemm_variant_info(kVariantPair);
+    const GemmTileInfo qi = pair_tile_info();
+    const int pair_rows = qi.b_rows;
     const size_t sf_pair_each = weight_scale_layout_bytes(1, rows, cols, qi.bn, qi.sfb_groups);
-    sf_prefill.allocate(sf_prefill_each * count);
     sf_stream.allocate(sf_stream_each * count);
     sf_pair.allocate(sf_pair_each * count);
     sf_pair_map = make_raw_map(sf_pair.as<uint8_t>(), sf_pair_each * count / 1024,
@@ -251,7 +243,6 @@ struct WeightStack {
     if (narrow_tail) {
       packed_tail.allocate(panel_rows * tail_pitch);
       try {
-        tail_prefill = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pi.bn);
         tail_stream = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, di.bn);
         tail_pair = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pair_rows);
       } catch (const Failure&) {
@@ -261,7 +252,6 @@ struct WeightStack {
     if (!narrow_tail && tail_bytes > 0) {
       tail_pitch = 128;
       packed_tail.allocate(panel_rows * tail_pitch, true);
-      tail_prefill = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pi.bn);
       tail_stream = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, di.bn);
       tail_pair = make_packed_map(packed_tail.as<uint8_t>(), panel_rows, tail_pitch, pair_rows);
     }
@@ -289,9 +279,6 @@ struct WeightStack {
                                        packed.as<uint8_t>() + panel_each * e,
                                        packed_tail.as<uint8_t>() + (tail_bytes > 0 ? tail_each * e : 0),
                                        stream));
-      NMOE_CUDA(relayout_weight_scales(staging_sf.as<uint8_t>(), 1, rows, cols, pi.bn,
-                                       pi.sfb_groups, sf_prefill.as<uint8_t>() + sf_prefill_each * e,
-                                       stream));
       NMOE_CUDA(relayout_weight_scales(staging_sf.as<uint8_t>(), 1, rows, cols, di.bn,
                                        di.sfb_groups, sf_stream.as<uint8_t>() + sf_stream_each * e,
                                        stream));
@@ -307,23 +294,17 @@ struct WeightStack {
     }
     if (tail_bytes == 0) {
       // never read (k_blocks == kb_full), but the kernel takes a valid map
-      tail_prefill = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, pi.bn);
       tail_stream = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, di.bn);
       tail_pair = make_packed_map(packed.as<uint8_t>(), panel_rows * kb_full, 128, pair_rows);
     }
   }
 
-  GemmVariant variant(TileClass c) const {
-    return c == kClassPair ? kVariantPair : prefill_variant;
-  }
-  const CUtensorMap& tail_map(TileClass c) const {
-    return c == kClassPrefill ? tail_prefill : c == kClassPair ? tail_pair : tail_stream;
-  }
+  const CUtensorMap& tail_map(TileClass c) const { return c == kClassPair ? tail_pair : tail_stream; }
   const uint8_t* sf(TileClass c) const {
-    return (c == kClassPrefill ? sf_prefill : c == kClassPair ? sf_pair : sf_stream).as<uint8_t>();
+    return (c == kClassPair ? sf_pair : sf_stream).as<uint8_t>();
   }
-  int tile_cols(TileClass c) const {
-    return c == kClassStream ? stream_variant_info().bn : gemm_variant_info(variant(c)).bn;
+  static int tile_cols(TileClass c) {
+    return (c == kClassPair ? pair_tile_info() : stream_tile_info()).bn;
   }
 };
 
@@ -343,14 +324,26 @@ struct ActivationOperand {
   }
 };
 
-GemmMaps gemm_maps(const WeightStack& weights, TileClass tile_class, const ActivationOperand& a) {
+GemmMaps gemm_maps(const WeightStack& weights, const ActivationOperand& a) {
   GemmMaps maps;
   maps.a = a.boxes[kStreamBoxes - 1];
-  maps.b_tail = weights.tail_map(tile_class);
+  maps.b_tail = weights.tail_map(kClassPair);
   maps.b_full = weights.full_pair;
   maps.sfa = a.sf_map;
   maps.sfb = weights.sf_pair_map;
   return maps;
+}
+
+// Which kernel multiplies `rows` rows with one matrix of `n` output features.  A K block of a
+// 256 x 208 tile over two SMs takes 1.2 times as long as one of a 128 x 128 tile on one SM (shared
+// expert of 16384 tokens: 89 us in 16 waves against 120 in 26): the fewer waves times that.
+TileClass dense_tile_class(int rows, int n, int num_sms) {
+  if (num_sms < 2) return kClassStream;
+  auto waves = [](int tiles, int units) { return (tiles + units - 1) / units; };
+  const int stream = waves((rows + 127) / 128 * ((n + 127) / 128), num_sms);
+  const int bn = pair_tile_info().bn;
+  const int pair = waves((rows + 255) / 256 * ((n + bn - 1) / bn), num_sms / 2);
+  return 5 * stream <= 6 * pair ? kClassStream : kClassPair;
 }
 
 struct Schedule {
@@ -435,8 +428,7 @@ void run_gemm(GemmMode mode, const WeightStack& weights, TileClass tile_class,
               const ActivationOperand& a, const GemmArgs& g, int most_rows, int num_sms,
               cudaStream_t stream) {
   if (tile_class != kClassStream) {
-    NMOE_CUDA(launch_grouped_gemm(weights.variant(tile_class), mode,
-                                  gemm_maps(weights, tile_class, a), g, num_sms, stream));
+    NMOE_CUDA(launch_pair_gemm(mode, gemm_maps(weights, a), g, num_sms, stream));
     return;
   }
   StreamArgs args;
@@ -505,7 +497,7 @@ void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCo
     if (ffn.up != nullptr) {
       phase->ready = ready;
       if (!up) {
-        const int bn = stream_variant_info().bn;
+        const int bn = stream_tile_info().bn;
         phase->wait_target = (ffn.up->n + bn - 1) / bn;
       }
     }
@@ -751,10 +743,6 @@ using namespace nmoe;
 // ===========================================================================
 // nmoe_ffn
 // ===========================================================================
-// Rows of one FFN up to which its weights are read once per 128 rows (the tiles of a prefill shape
-// are too few to fill the GPU until there are many row tiles).
-constexpr int kStreamFfnRows = 256;
-
 struct nmoe_ffn {
   int hidden = 0;
   int inter = 0;
@@ -798,8 +786,8 @@ nmoe_status nmoe_ffn_create(const nmoe_nvfp4_matrix* up, const nmoe_nvfp4_matrix
     f->max_rows = max_rows;
     f->num_sms = device_sm_count();
     cudaStream_t stream = nullptr;
-    f->up.upload(up, 1, f->inter, f->hidden, true, "up_proj", stream);
-    f->down.upload(down, 1, f->hidden, f->inter, false, "down_proj", stream);
+    f->up.upload(up, 1, f->inter, f->hidden, "up_proj", stream);
+    f->down.upload(down, 1, f->hidden, f->inter, "down_proj", stream);
     const size_t slots = (static_cast<size_t>(max_rows) + 127) / 128;
     f->a_packed.allocate(slots * 128 * f->hidden / 2, true);
     f->a_sf.allocate(tiled_sf_bytes(slots, f->hidden), true);
@@ -831,10 +819,10 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   try {
     if (gemm_variant == 2 && rows > 32) return NMOE_ERR_INVALID_ARGUMENT;
-    const TileClass tile_class = gemm_variant == 1   ? kClassPrefill
-                                 : gemm_variant == 4 ? kClassPair
-                                 : gemm_variant != 0 || rows <= kStreamFfnRows ? kClassStream
-                                                                               : kClassPrefill;
+    const TileClass tile_class =
+        gemm_variant == 1 || gemm_variant == 4 ? kClassPair
+        : gemm_variant != 0                    ? kClassStream
+                            : dense_tile_class(static_cast<int>(rows), ffn->inter, ffn->num_sms);
     NMOE_CUDA(launch_norm_quant(input, input_dtype == NMOE_BF16, static_cast<int>(rows),
                                 ffn->hidden, nullptr, 0.0f, nullptr, ffn->a_packed.as<uint8_t>(),
                                 nullptr, ffn->a_sf.as<uint8_t>(), k_blocks_of(ffn->hidden),
@@ -999,11 +987,6 @@ struct nmoe_layer {
   bool last_unfused = false;
   bool last_normalized = true;
   bool force_fp32_parts = false;  // NMOE_PARTS_FP32=1: FP32 rows whatever the output type
-  // CTA pairs for the prefill GEMMs (NMOE_GEMM_PAIR=1 turns them on), used once an
-  // expert has this many rows on average.  Off by default: with the partner CTA's
-  // "operands landed" relayed through a thread they measured slower than single CTAs.
-  bool pair_gemms = false;
-  int pair_min_rows = 640;
   // how long a kernel waits for a flag another GPU raises before it gives up with
   // kDevWaitTimeout (clock64 ticks; nmoe_layer_set_wait_limit_ms, NMOE_WAIT_LIMIT_MS)
   long long wait_limit_ticks = 1ll << 34;
@@ -1195,9 +1178,7 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   L->cfg = c;
   L->num_sms = device_sm_count();
   L->force_fp32_parts = std::getenv("NMOE_PARTS_FP32") != nullptr;
-  if (const char* env = std::getenv("NMOE_GEMM_PAIR")) L->pair_gemms = std::atoi(env) != 0;
   if (const char* env = std::getenv("NMOE_GRAPH_MAX_TOKENS")) L->graph_max_tokens = std::atoi(env);
-  if (const char* env = std::getenv("NMOE_GEMM_PAIR_MIN_ROWS")) L->pair_min_rows = std::atoi(env);
   if (const char* env = std::getenv("NMOE_WAIT_LIMIT_MS")) {
     const double ms = std::strtod(env, nullptr);
     if (ms > 0.0) L->wait_limit_ticks = ticks_from_ms(ms);
@@ -1237,8 +1218,8 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   }
   // routed experts act on latent rows: up_proj [I][latent], down_proj [latent][I]
   // (shape checks of expert_layer.cpp:646-689)
-  L->up.upload(w.routed_up, EL, I, Lr, true, "routed up_proj", stream);
-  L->down.upload(w.routed_down, EL, Lr, I, false, "routed down_proj", stream);
+  L->up.upload(w.routed_up, EL, I, Lr, "routed up_proj", stream);
+  L->down.upload(w.routed_down, EL, Lr, I, "routed down_proj", stream);
   if (L->latent_mode) {
     L->fc1.upload(w.fc1_latent, Lr, H, "fc1_latent", stream);
     L->fc2.upload(w.fc2_latent, H, Lr, "fc2_latent", stream);
@@ -1246,12 +1227,12 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   if (w.shared_up_linear.family != NMOE_LINEAR_ABSENT) {
     L->shared_up_dense.upload(w.shared_up_linear, S, H, "shared up_proj", stream);
   } else {
-    L->shared_up.upload(&w.shared_up, 1, S, H, true, "shared up_proj", stream);
+    L->shared_up.upload(&w.shared_up, 1, S, H, "shared up_proj", stream);
   }
   if (w.shared_down_linear.family != NMOE_LINEAR_ABSENT) {
     L->shared_down_dense.upload(w.shared_down_linear, H, S, "shared down_proj", stream);
   } else {
-    L->shared_down.upload(&w.shared_down, 1, H, S, false, "shared down_proj", stream);
+    L->shared_down.upload(&w.shared_down, 1, H, S, "shared down_proj", stream);
   }
 
   if (w.gate_weight.dtype == NMOE_BF16) {
@@ -1421,21 +1402,15 @@ void run_ffn(nmoe_layer* L, bool unfused, const WeightStack& up, const WeightSta
 // 1003 tokens 231 against 229, 2048 tokens 281 against 274).
 constexpr int kSharedInLaunchTokens = 640;
 
-// Routed rows per expert (on average) up to which csrc/expert_stream.cu takes them: 96 rows
-// measured 274 us for the whole pass against 276 with the prefill tiles, 47 rows 229 against 240,
-// 141 rows 451 against 371 (most experts then have a second row tile).  Up tiles of few K blocks
-// are over before the epilogue of a tile of many rows is (latent size 1024, 43 rows: up projection
-// 204 against 166 us), so there the line lies at the epilogue's short form.
+// Routed rows per expert (on average) up to which csrc/expert_stream.cu takes them: with more, most
+// experts have a second row tile and their weights would be read twice (whole pass at 96 rows 250 us,
+// at 141 rows 321 with CTA pairs against 370).
 constexpr int kStreamRowsPerExpert = 100;
-constexpr int kStreamRowsShortTiles = 16;
 
 // Which kernel takes `pairs` routed rows.
 TileClass routed_tile_class(const nmoe_layer* L, int pairs) {
-  const int rows = k_blocks_of(L->latent) >= 6 ? kStreamRowsPerExpert : kStreamRowsShortTiles;
-  if (pairs <= L->local_experts * rows) return kClassStream;
-  const bool pair = L->pair_gemms && !L->unfused && (L->num_sms & 1) == 0 &&
-                    pairs / L->local_experts >= L->pair_min_rows;
-  return pair ? kClassPair : kClassPrefill;
+  if (pairs <= L->local_experts * kStreamRowsPerExpert) return kClassStream;
+  return L->num_sms < 2 ? kClassStream : kClassPair;
 }
 
 // Plan + permute + the grouped GEMMs over `pairs` (row, slot) pairs whose per-local-expert
@@ -1506,8 +1481,7 @@ void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& sou
 }
 
 TileClass shared_tile_class(const nmoe_layer* L, int tokens) {
-  if (tokens <= kStreamFfnRows) return kClassStream;
-  return L->pair_gemms && (L->num_sms & 1) == 0 && tokens >= 1024 ? kClassPair : kClassPrefill;
+  return dense_tile_class(tokens, L->cfg.shared_expert_intermediate_size, L->num_sms);
 }
 
 // The shared expert's hidden rows in FP32: shared_up and relu^2 (:814-818, :956-964), by a dense /
