@@ -211,9 +211,9 @@ void launch_slices(const void* in, int rows, int K, float scale, int tile_rows, 
 // MMA of up to 256 columns multiplies digit i with several token digits and adds each product to
 // the level it belongs to; A is read once for all of them.  A CTA takes one tile, or a share of
 // its K range, and stores the levels put together as doubles.
-// Bound by the int8 MMA rate, which measures half of the FP8 rate here (64 token rows: 3300
-// cycles of MMA per 60 KB stage).  The checkpoint's shared_up (5376 x 4096), 1000 rows: 13,800 ->
-// 580 us with the two kernels around it; 40 rows: 381 -> 60 us.
+// Bound by shared memory (64 token rows: 60 KB written and 154 KB read per 64-byte stage, 1680 cycles
+// at 128 a cycle, against 1400 of MMA).  The checkpoint's shared_up (5376 x 4096), 1000 rows: 13,800 ->
+// 370 us with the two kernels around it; 40 rows: 381 -> 44 us.
 // ---------------------------------------------------------------------------
 constexpr int kExactStages = 3;
 constexpr int kExactThreads = 6 * 32;
@@ -234,14 +234,41 @@ __device__ __forceinline__ uint32_t make_idesc_i8(uint32_t n) {
   return (2u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+// The products of one 32-byte step of K: digit I of W times its token digits, from the given shared-
+// memory descriptors.  A level that digit I is the first to reach is an MMA of its own, so that it
+// can start the sum when `first`.
+template <int NT, int I>
+__device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t a_desc, uint64_t b_desc,
+                                            bool first) {
+  constexpr int kMost = 256 / NT;                                      // token digits of one MMA
+  constexpr int kMeet = kSlices < kLevels - I ? kSlices : kLevels - I;  // ... within the levels
+  constexpr bool kStarts = I > 0 && I <= kLevels - kSlices;
+  constexpr int kTogether = kStarts ? kMeet - 1 : kMeet;
+  const uint64_t a = advance_smem_desc(a_desc, I * kExactRows * kExactChunk);
+#pragma unroll
+  for (int j = 0; j < kTogether; j += kMost) {
+    constexpr int kFull = kMost < kTogether ? kMost : kTogether;
+    const int count = kTogether - j < kFull ? kTogether - j : kFull;
+    tcgen05_mma_i8(tmem + (I + j) * NT, a, advance_smem_desc(b_desc, j * NT * kExactChunk),
+                   make_idesc_i8(static_cast<uint32_t>(count * NT)), I == 0 && first ? 0u : 1u);
+  }
+  if constexpr (kStarts) {
+    tcgen05_mma_i8(tmem + (I + kMeet - 1) * NT, a,
+                   advance_smem_desc(b_desc, (kMeet - 1) * NT * kExactChunk),
+                   make_idesc_i8(static_cast<uint32_t>(NT)), first ? 0u : 1u);
+  }
+}
+
+template <int NT>
 __global__ void __launch_bounds__(kExactThreads, 1)
 exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict__ x_slices,
-                  int rows, int N, int K, int nt, int row_tiles, int splits,
+                  int rows, int N, int K, int row_tiles, int splits,
                   double* __restrict__ partial, int32_t* error) {
+  constexpr int nt = NT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
                                              ~static_cast<uintptr_t>(1023u));
-  const int b_bytes = kSlices * nt * kExactChunk;
+  constexpr int b_bytes = kSlices * nt * kExactChunk;
   uint8_t* sA = smem;
   uint8_t* sB = sA + kExactStages * kExactABytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(sB + kExactStages * b_bytes);
@@ -249,7 +276,7 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
   uint64_t* done_bar = empty_bar + kExactStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   // consecutive CTAs share a weight tile
   int index = static_cast<int>(blockIdx.x);
@@ -277,81 +304,70 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+
+  const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+  const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
 
   if (warp == 0) {
-    if (lane == 0) {
-      const int8_t* w_from =
-          w_slices + (static_cast<size_t>(n0 / kExactRows) * all_chunks + chunk0) * kExactABytes;
-      const int8_t* x_from =
-          x_slices + (static_cast<size_t>(row_tile) * all_chunks + chunk0) * b_bytes;
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int c = 0; c < chunks; ++c) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1u)) {
-          if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
-          break;
-        }
-        mbar_arrive_expect_tx(&full_bar[stage], kExactABytes + b_bytes);
-        bulk_load(sA + stage * kExactABytes, w_from, kExactABytes, &full_bar[stage]);
-        bulk_load(sB + stage * b_bytes, x_from, b_bytes, &full_bar[stage]);
-        w_from += kExactABytes;
-        x_from += b_bytes;
-        if (++stage == kExactStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
+    const int8_t* w_from =
+        w_slices + (static_cast<size_t>(n0 / kExactRows) * all_chunks + chunk0) * kExactABytes;
+    const int8_t* x_from =
+        x_slices + (static_cast<size_t>(row_tile) * all_chunks + chunk0) * b_bytes;
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int c = 0; c < chunks; ++c) {
+      if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
+        if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
+        break;
+      }
+      if (elect_one()) {
+        const uint32_t bar = full0 + stage * 8;
+        mbar_arrive_expect_tx_at(bar, kExactABytes + b_bytes);
+        bulk_load_at(a0 + stage * kExactABytes, w_from, kExactABytes, bar);
+        bulk_load_at(b0 + stage * b_bytes, x_from, b_bytes, bar);
+      }
+      w_from += kExactABytes;
+      x_from += b_bytes;
+      if (++stage == kExactStages) {
+        stage = 0;
+        phase ^= 1u;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const int most = 256 / nt;  // token digits of one MMA
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int c = 0; c < chunks; ++c) {
-        if (!mbar_wait(&full_bar[stage], phase)) {
-          if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
-          ok = false;
-          break;
-        }
-        tcgen05_fence_after();
-        const uint32_t a_addr = smem_u32(sA + stage * kExactABytes);
-        const uint32_t b_addr = smem_u32(sB + stage * b_bytes);
-#pragma unroll 1
-        for (int ks = 0; ks < kExactChunk / 32; ++ks) {
-#pragma unroll 1
-          for (int i = 0; i < kSlices; ++i) {
-            const uint64_t a_desc =
-                make_smem_desc(a_addr + i * (kExactRows * kExactChunk) + ks * 32, 0, 512, 4);
-            const int meet = min(kSlices, kLevels - i);  // token digits within the levels
-            for (int j = 0; j < meet;) {
-              int count = min(most, meet - j);
-              uint32_t accumulate = 1u;
-              if ((c | ks) == 0) {
-                // digit 0 of W starts the first kSlices levels, the next digits one more each
-                if (i == 0) {
-                  accumulate = 0u;
-                } else if (i <= kLevels - kSlices) {
-                  accumulate = j + 1 == meet ? 0u : 1u;
-                  count = min(count, accumulate != 0u ? meet - 1 - j : 1);
-                }
-              }
-              tcgen05_mma_i8(tmem_base + (i + j) * nt, a_desc,
-                             make_smem_desc(b_addr + j * nt * kExactChunk + ks * 32, 0, 512, 4),
-                             make_idesc_i8(static_cast<uint32_t>(count * nt)), accumulate);
-              j += count;
-            }
-          }
-        }
-        tcgen05_commit(&empty_bar[stage]);
-        if (++stage == kExactStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
+    const uint64_t a_desc0 = make_smem_desc(a0, 0, 512, 4);
+    const uint64_t b_desc0 = make_smem_desc(b0, 0, 512, 4);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int c = 0; c < chunks; ++c) {
+      if (!mbar_wait_warp(full0 + stage * 8, phase)) {
+        if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
+        ok = false;
+        break;
       }
-      if (ok) tcgen05_commit(done_bar);
+      tcgen05_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < kExactChunk / 32; ++ks) {
+          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * kExactABytes + ks * 32);
+          const uint64_t b_desc = advance_smem_desc(b_desc0, stage * b_bytes + ks * 32);
+          const bool first = ks == 0 && c == 0;
+          static_assert(kSlices == 5, "one call per digit");
+          issue_digit<NT, 0>(tmem_base, a_desc, b_desc, first);
+          issue_digit<NT, 1>(tmem_base, a_desc, b_desc, first);
+          issue_digit<NT, 2>(tmem_base, a_desc, b_desc, first);
+          issue_digit<NT, 3>(tmem_base, a_desc, b_desc, first);
+          issue_digit<NT, 4>(tmem_base, a_desc, b_desc, first);
+        }
+        tcgen05_commit_at(empty0 + stage * 8);
+      }
+      if (++stage == kExactStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
     }
+    if (ok && elect_one()) tcgen05_commit(done_bar);
   } else {
     // epilogue: warp w owns TMEM lane quarter w % 4; a thread owns a weight row
     const int quarter = warp & 3;
@@ -769,13 +785,18 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
   const int grid = (w.N + kExactRows - 1) / kExactRows * row_tiles * splits;
   const int smem = kExactStages * (kExactABytes + kSlices * nt * kExactChunk) +
                    (2 * kExactStages + 1) * 8 + 16 + 1024;
-  cudaError_t err = cudaFuncSetAttribute(exact_gemm_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (err != cudaSuccess) return err;
-  exact_gemm_kernel<<<grid, kExactThreads, smem, stream>>>(w.slices, space.slices, rows, w.N, w.K,
-                                                           nt, row_tiles, splits, space.partial,
-                                                           error);
-  err = cudaGetLastError();
+  auto multiply = [&](auto kernel) {
+    const cudaError_t attribute =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (attribute != cudaSuccess) return attribute;
+    kernel<<<grid, kExactThreads, smem, stream>>>(w.slices, space.slices, rows, w.N, w.K, row_tiles,
+                                                  splits, space.partial, error);
+    return cudaGetLastError();
+  };
+  const cudaError_t err = nt == 16   ? multiply(exact_gemm_kernel<16>)
+                          : nt == 32 ? multiply(exact_gemm_kernel<32>)
+                          : nt == 48 ? multiply(exact_gemm_kernel<48>)
+                                     : multiply(exact_gemm_kernel<64>);
   if (err != cudaSuccess) return err;
   const dim3 blocks((w.N + kFinishThreads - 1) / kFinishThreads, rows, 1);
   auto run = [&](auto kernel) {
