@@ -147,12 +147,14 @@ size_t weight_scale_layout_bytes(int experts, int N, int K, int bn, int sfb_grou
 //   normalized (optional) fp32 [rows][cols]
 //   packed [rows][cols/2]; sf_row_major (optional) [rows][cols/16];
 //   sf_tiled (optional) tiled layout with k_blocks*4 K-tiles per 128-row slot;
-//   tensor_scale (optional) [rows]; inv_rms (optional) [rows]: 1/sqrt(mean(x^2)+eps)
+//   tensor_scale (optional) [rows]; inv_rms (optional) [rows]: 1/sqrt(mean(x^2)+eps);
+//   `zero` (optional): `zero_count` words set to zero on the way (the histogram of what follows)
 cudaError_t launch_norm_quant(const void* in, bool in_bf16, int rows, int cols,
                               const float* norm_weight, float eps, float* normalized,
                               uint8_t* packed, uint8_t* sf_row_major, uint8_t* sf_tiled,
                               int k_blocks, float* tensor_scale, cudaStream_t stream,
-                              float* inv_rms = nullptr);
+                              float* inv_rms = nullptr, int32_t* zero = nullptr,
+                              int zero_count = 0);
 // Whole-matrix dynamic quantisation with ONE tensor scale (the reference
 // packer's semantics for rows > 1).  `amax_scratch` is one float of device
 // memory; it is overwritten.
@@ -176,6 +178,7 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int rows,
                                int top_k, int n_group, int topk_group, bool norm_topk_prob,
                                float routed_scaling, int32_t* top_index, float* top_weight,
                                int32_t* expert_counts /* nullable, += histogram */,
+                               int32_t* position /* nullable [rows][top_k]: the count before */,
                                cudaStream_t stream);
 
 // Two-pass router for large batches.  Pass 1: logits on the tensor cores (FP32
@@ -218,7 +221,8 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        const float* bias, int rows, int experts, int hidden,
                                        int top_k, bool norm_topk_prob, float routed_scaling,
                                        float tie_margin, int32_t* top_index, float* top_weight,
-                                       int32_t* expert_counts, cudaStream_t stream);
+                                       int32_t* expert_counts, int32_t* position,
+                                       cudaStream_t stream);
 
 // --- correctly rounded linears (csrc/exact.cu) ---------------------------------
 // y[rows][N] = x[rows][K] x W[N][K]^T in FP32, each value the FP64 sum rounded once.
@@ -285,16 +289,10 @@ cudaError_t launch_gather_rows(const float* rows, const int32_t* row_of, int cou
 // --- plan / permute / combine -------------------------------------------------
 struct PlanBuffers {
   int32_t* expert_counts;   // [experts]  (input, filled by the router)
-  int32_t* expert_cursor;   // [experts]  (scratch, zeroed by the plan kernel)
-  int32_t* expert_slot0;    // [experts]  first row slot of each expert
+  int32_t* expert_cursor;   // [experts]  zeroed by the caller where pairs bring no position
   RowTile* row_tiles;       // [max_row_tiles]
   int32_t* num_row_tiles;   // [1]
 };
-// `tile_multiple`: every expert gets a multiple of this many row tiles (2 when CTA
-// pairs consume them: the second tile of an odd expert is left empty).
-cudaError_t launch_route_plan(const PlanBuffers& plan, int experts, int tile_rows,
-                              int tile_multiple, int max_row_tiles, int32_t* error,
-                              cudaStream_t stream);
 // Where permute reads a (row, slot) pair from.  Quantised rows are indexed by
 // source row = pair / pairs_per_row, routing weight and expert id by pair; all
 // strides are in bytes.  Local routing: pairs_per_row = top_k over the token
@@ -311,20 +309,23 @@ struct PermuteSource {
   const int32_t* expert;  // index into the LOCAL expert stack
   size_t expert_stride;
   int pairs_per_row;
+  const int32_t* position = nullptr;  // per pair, its place among its expert's; nullptr: any place
   // fixed-capacity receive buffers: pair i is valid iff (i % capacity) <
   // valid_counts[i / capacity]; nullptr = every pair is valid
   const int32_t* valid_counts = nullptr;
   int capacity = 0;
 };
-// Copies each pair's quantised activation row into its expert's row slots and
-// records where it went; sorted_dest[row] = source_row * dest_stride + slot.
-cudaError_t launch_permute(const PlanBuffers& plan, const PermuteSource& src, int pairs,
-                           int experts /* size of the local expert stack */, int tile_rows,
-                           int max_row_tiles, int cols, int k_blocks,
-                           uint8_t* sorted_packed, uint8_t* sorted_sf_tiled,
-                           float* sorted_tensor_scale, float* sorted_weight,
-                           int32_t* sorted_dest, int32_t* pair_row /* nullable */,
-                           int dest_stride, cudaStream_t stream);
+// Lays out every expert's row slots (128 rows each; `tile_multiple`: every expert gets a multiple of
+// this many, 2 when CTA pairs consume them), writes the tile list, copies each pair's quantised
+// activation row into its expert's slots and records where it went;
+// sorted_dest[row] = source_row * dest_stride + slot.
+cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src, int pairs,
+                              int experts /* size of the local expert stack */, int tile_multiple,
+                              int max_row_tiles, int cols, int k_blocks, uint8_t* sorted_packed,
+                              uint8_t* sorted_sf_tiled, float* sorted_tensor_scale,
+                              float* sorted_weight, int32_t* sorted_dest,
+                              int32_t* pair_row /* nullable */, int dest_stride, int32_t* error,
+                              cudaStream_t stream);
 // --- expert-parallel dispatch / return (csrc/ep.cu) ---------------------------
 int dispatch_record_bytes(int cols);
 cudaError_t launch_dispatch_plan(const int32_t* expert_counts, int experts, int experts_per_rank,

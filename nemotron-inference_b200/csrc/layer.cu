@@ -942,7 +942,7 @@ struct nmoe_layer {
   DeviceBuffer sh_packed, sh_sf;
   DeviceBuffer parts;
   // plan
-  DeviceBuffer counts, cursor, slot0, row_tiles, num_row_tiles, pair_row;
+  DeviceBuffer counts, cursor, position, row_tiles, num_row_tiles, pair_row;
   // expert-sorted scratch
   DeviceBuffer a_packed, a_sf, a_ts, a_weight, a_dest, h_packed, h_sf;
 
@@ -1105,7 +1105,7 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   const size_t slots = static_cast<size_t>(L->max_row_tiles);
   L->counts.allocate(E * sizeof(int32_t), true);
   L->cursor.allocate(E * sizeof(int32_t), true);
-  L->slot0.allocate(E * sizeof(int32_t), true);
+  L->position.allocate(T * K * sizeof(int32_t), true);
   L->row_tiles.allocate(slots * sizeof(RowTile), true);
   L->num_row_tiles.allocate(sizeof(int32_t), true);
   L->pair_row.allocate(pairs * sizeof(int32_t), true);
@@ -1289,7 +1289,7 @@ void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, 
 }
 
 // RMSNorm + activation quantiser + router: fills normalized, y_*, logits,
-// top_index / top_weight and the per-expert histogram `counts` (global ids).
+// top_index / top_weight, the per-expert histogram `counts` (global ids) and each pair's position in it.
 void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype in_dtype,
                   int tokens, cudaEvent_t after_quantise = nullptr,
                   bool fork_after_logits = false) {
@@ -1307,14 +1307,13 @@ void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dt
                               c.rms_epsilon, want_normalized ? L->normalized.as<float>() : nullptr,
                               L->y_packed.as<uint8_t>(), L->y_sf_row_major.as<uint8_t>(),
                               L->y_sf_tiled.as<uint8_t>(), k_blocks_of(H), L->y_ts.as<float>(),
-                              stream, L->inv_rms.as<float>()));
+                              stream, L->inv_rms.as<float>(), L->counts.as<int32_t>(), E));
   L->last_normalized = want_normalized;
   if (after_quantise != nullptr && !fork_after_logits) {
     NMOE_CUDA(cudaEventRecord(after_quantise, stream));
   }
   L->mark(1, stream);
   // gate projection (:797-799) and top-k (:881)
-  NMOE_CUDA(cudaMemsetAsync(L->counts.as<int32_t>(), 0, E * sizeof(int32_t), stream));
   const float* offset = L->has_logit_offset ? L->logit_offset.as<float>() : nullptr;
   if (two_pass_router) {
     const int logit_splits = router_pass1_splits(tokens, H, L->num_sms);
@@ -1344,7 +1343,7 @@ void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dt
         L->norm_weight.as<float>(), L->gate_bf16.as<__nv_bfloat16>(), offset,
         L->bias.as<float>(), tokens, E, H, K, c.norm_topk_prob != 0, c.routed_scaling_factor,
         L->router_tie_margin, L->top_index.as<int32_t>(), L->top_weight.as<float>(),
-        L->counts.as<int32_t>(), stream));
+        L->counts.as<int32_t>(), L->position.as<int32_t>(), stream));
   } else {
     if (L->has_gate_exact) {
       run_exact(L->gate_exact.w, L->exact, L->normalized.as<float>(), 0.0f, tokens, offset, false,
@@ -1357,7 +1356,8 @@ void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dt
     NMOE_CUDA(launch_router_topk(L->logits.as<float>(), L->bias.as<float>(), tokens, E, K,
                                  c.n_group, c.topk_group, c.norm_topk_prob != 0,
                                  c.routed_scaling_factor, L->top_index.as<int32_t>(),
-                                 L->top_weight.as<float>(), L->counts.as<int32_t>(), stream));
+                                 L->top_weight.as<float>(), L->counts.as<int32_t>(),
+                                 L->position.as<int32_t>(), stream));
   }
   L->mark(3, stream);
 }
@@ -1422,22 +1422,22 @@ void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& sou
   const int Lr = L->latent;
   int32_t* error = L->error.device.as<int32_t>();
   const TileClass routed_class = routed_tile_class(L, pairs);
-  constexpr int tile_rows = 128;
   PlanBuffers plan;
   plan.expert_counts = L->counts.as<int32_t>();
   plan.expert_cursor = L->cursor.as<int32_t>();
-  plan.expert_slot0 = L->slot0.as<int32_t>();
   plan.row_tiles = L->row_tiles.as<RowTile>();
   plan.num_row_tiles = L->num_row_tiles.as<int32_t>();
-  NMOE_CUDA(launch_route_plan(plan, L->local_experts, tile_rows, routed_class == kClassPair ? 2 : 1,
-                              L->max_row_tiles, error, stream));
+  if (source.position == nullptr) {
+    NMOE_CUDA(cudaMemsetAsync(plan.expert_cursor, 0, L->local_experts * sizeof(int32_t), stream));
+  }
   L->mark(4, stream);
-  NMOE_CUDA(launch_permute(plan, source, pairs, L->local_experts, tile_rows, L->max_row_tiles, Lr,
-                           k_blocks_of(Lr),
-                           L->a_packed.as<uint8_t>(), L->a_sf.as<uint8_t>(), L->a_ts.as<float>(),
-                           L->a_weight.as<float>(), L->a_dest.as<int32_t>(),
-                           L->ep_world == 1 ? L->pair_row.as<int32_t>() : nullptr, dest_stride,
-                           stream));
+  NMOE_CUDA(launch_place_rows(plan, source, pairs, L->local_experts,
+                              routed_class == kClassPair ? 2 : 1, L->max_row_tiles, Lr,
+                              k_blocks_of(Lr), L->a_packed.as<uint8_t>(), L->a_sf.as<uint8_t>(),
+                              L->a_ts.as<float>(), L->a_weight.as<float>(),
+                              L->a_dest.as<int32_t>(),
+                              L->ep_world == 1 ? L->pair_row.as<int32_t>() : nullptr, dest_stride,
+                              error, stream));
   L->mark(5, stream);
   // routed experts (:896-954)
   Schedule routed;
@@ -1589,6 +1589,7 @@ PermuteSource local_source(nmoe_layer* L) {
   source.expert = L->top_index.as<int32_t>();
   source.expert_stride = sizeof(int32_t);
   source.pairs_per_row = L->cfg.top_k;
+  source.position = L->position.as<int32_t>();
   return source;
 }
 
@@ -2517,7 +2518,7 @@ nmoe_status nmoe_router_topk(void* stream, const float* logits, const float* bia
   }
   return launch_router_topk(logits, bias, static_cast<int>(rows), experts, top_k, n_group,
                             topk_group, norm_topk_prob != 0, routed_scaling, top_index,
-                            top_weight, nullptr,
+                            top_weight, nullptr, nullptr,
                             static_cast<cudaStream_t>(stream)) == cudaSuccess
              ? NMOE_OK
              : NMOE_ERR_INVALID_ARGUMENT;

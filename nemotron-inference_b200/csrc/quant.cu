@@ -79,6 +79,11 @@ __device__ __forceinline__ uint32_t quantize_half_block(const float (&v)[8], flo
   return word;
 }
 
+__device__ __forceinline__ void zero_words(int32_t* words, int count) {
+  if (blockIdx.x != 0) return;
+  for (int i = threadIdx.x; i < count; i += blockDim.x) words[i] = 0;
+}
+
 // Rows of any length, and one tensor scale for a whole matrix (PER_ROW_SCALE false).
 template <bool BF16, bool PER_ROW_SCALE>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
@@ -87,7 +92,8 @@ norm_quant_kernel(const void* __restrict__ in, int rows, int cols,
                   float* __restrict__ normalized, uint8_t* __restrict__ packed,
                   uint8_t* __restrict__ sf_row_major, uint8_t* __restrict__ sf_tiled, int k_tiles,
                   float* __restrict__ tensor_scale, const float* __restrict__ global_amax,
-                  float* __restrict__ inv_rms_out) {
+                  float* __restrict__ inv_rms_out, int32_t* __restrict__ zero, int zero_count) {
+  zero_words(zero, zero_count);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * kWarpsPerBlock + warp;
@@ -218,7 +224,9 @@ norm_quant_row_kernel(const void* __restrict__ in, int rows, int cols,
                       float* __restrict__ normalized, uint8_t* __restrict__ packed,
                       uint8_t* __restrict__ sf_row_major, uint8_t* __restrict__ sf_tiled,
                       int k_tiles, float* __restrict__ tensor_scale,
-                      float* __restrict__ inv_rms_out, int row_warp_shift, bool word_scales) {
+                      float* __restrict__ inv_rms_out, int row_warp_shift, bool word_scales,
+                      int32_t* __restrict__ zero, int zero_count) {
+  zero_words(zero, zero_count);
   const int lane = threadIdx.x & 31;
   const int warp_global = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int row = SHARED ? warp_global >> row_warp_shift : warp_global;
@@ -432,7 +440,7 @@ template <bool BF16, int ITERS>
 void launch_row_kernel(int rows, cudaStream_t stream, const void* in, int cols,
                        const float* norm_weight, float eps, float* normalized, uint8_t* packed,
                        uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles, float* tensor_scale,
-                       float* inv_rms) {
+                       float* inv_rms, int32_t* zero, int zero_count) {
   // A row costs one warp about 2 us of latency, half of it in the quantiser: with few rows
   // eight warps share that half (each still reads the whole row, from L1), with more rows
   // than the GPU has warp slots one warp does it all.
@@ -445,7 +453,7 @@ void launch_row_kernel(int rows, cudaStream_t stream, const void* in, int cols,
   auto run = [&](auto kernel) {
     kernel<<<grid, kWarpsPerBlock * 32, 0, stream>>>(
         in, rows, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
-        tensor_scale, inv_rms, shift, word_scales);
+        tensor_scale, inv_rms, shift, word_scales, zero, zero_count);
   };
   if (shift > 0) {
     run(norm_quant_row_kernel<BF16, ITERS, true>);
@@ -458,10 +466,10 @@ template <bool BF16>
 void launch_norm_quant_t(int rows, cudaStream_t stream, const void* in, int cols,
                          const float* norm_weight, float eps, float* normalized, uint8_t* packed,
                          uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles,
-                         float* tensor_scale, float* inv_rms) {
+                         float* tensor_scale, float* inv_rms, int32_t* zero, int zero_count) {
   auto run = [&](auto launcher) {
     launcher(rows, stream, in, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled,
-             k_tiles, tensor_scale, inv_rms);
+             k_tiles, tensor_scale, inv_rms, zero, zero_count);
   };
   // the row lives in registers (8 floats per lane and iteration); longer rows are read three times
   if (cols <= 4 * 256) {
@@ -476,7 +484,7 @@ void launch_norm_quant_t(int rows, cudaStream_t stream, const void* in, int cols
     const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
     norm_quant_kernel<BF16, true><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
         in, rows, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
-        tensor_scale, nullptr, inv_rms);
+        tensor_scale, nullptr, inv_rms, zero, zero_count);
   }
 }
 
@@ -486,14 +494,16 @@ cudaError_t launch_norm_quant(const void* in, bool in_bf16, int rows, int cols,
                               const float* norm_weight, float eps, float* normalized,
                               uint8_t* packed, uint8_t* sf_row_major, uint8_t* sf_tiled,
                               int k_blocks, float* tensor_scale, cudaStream_t stream,
-                              float* inv_rms) {
+                              float* inv_rms, int32_t* zero, int zero_count) {
   if (rows <= 0 || cols <= 0 || cols % 16 != 0) return cudaErrorInvalidValue;
   if (in_bf16) {
     launch_norm_quant_t<true>(rows, stream, in, cols, norm_weight, eps, normalized, packed,
-                              sf_row_major, sf_tiled, k_blocks * 4, tensor_scale, inv_rms);
+                              sf_row_major, sf_tiled, k_blocks * 4, tensor_scale, inv_rms, zero,
+                              zero_count);
   } else {
     launch_norm_quant_t<false>(rows, stream, in, cols, norm_weight, eps, normalized, packed,
-                               sf_row_major, sf_tiled, k_blocks * 4, tensor_scale, inv_rms);
+                               sf_row_major, sf_tiled, k_blocks * 4, tensor_scale, inv_rms, zero,
+                              zero_count);
   }
   return cudaGetLastError();
 }
@@ -509,7 +519,7 @@ cudaError_t launch_quant_matrix(const float* in, int rows, int cols, uint8_t* pa
   const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
   norm_quant_kernel<false, false><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
       in, rows, cols, nullptr, 0.0f, nullptr, packed, sf_row_major, nullptr, 0, tensor_scale,
-      amax_scratch, nullptr);
+      amax_scratch, nullptr, nullptr, 0);
   return cudaGetLastError();
 }
 

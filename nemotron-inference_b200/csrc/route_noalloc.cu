@@ -103,5 +103,5 @@ extern "C" nmoe_status nmoe_route_tokens_noalloc(
   if (status != NMOE_OK) return status;
   return status_of(nmoe::launch_router_topk(logits, bias, r, experts, top_k, n_group, topk_group,
                                             norm_topk_prob != 0, routed_scaling, top_index,
-                                            top_weight, nullptr, stream));
+                                            top_weight, nullptr, nullptr, stream));
 }

@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(kTopkThreads)
 router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int experts,
                    int top_k, int n_group, int topk_group, bool norm_topk_prob,
                    float routed_scaling, int32_t* __restrict__ top_index,
-                   float* __restrict__ top_weight, int32_t* __restrict__ expert_counts) {
+                   float* __restrict__ top_weight, int32_t* __restrict__ expert_counts,
+                   int32_t* __restrict__ position) {
   __shared__ float score_smem[PER_LANE * 32];
   __shared__ float choice_smem[PER_LANE * 32];
   const int lane = threadIdx.x & 31;
@@ -224,7 +225,10 @@ router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ b
     w = __fmul_rn(w, routed_scaling);
     top_index[static_cast<size_t>(row) * top_k + lane] = my_index;
     top_weight[static_cast<size_t>(row) * top_k + lane] = w;
-    if (expert_counts != nullptr) atomicAdd(&expert_counts[my_index], 1);
+    if (expert_counts != nullptr) {
+      const int place = atomicAdd(&expert_counts[my_index], 1);
+      if (position != nullptr) position[static_cast<size_t>(row) * top_k + lane] = place;
+    }
   }
 }
 
@@ -262,14 +266,14 @@ bool router_topk_arguments_valid(int rows, int experts, int top_k, int n_group, 
 cudaError_t launch_router_topk(const float* logits, const float* bias, int rows, int experts,
                                int top_k, int n_group, int topk_group, bool norm_topk_prob,
                                float routed_scaling, int32_t* top_index, float* top_weight,
-                               int32_t* expert_counts, cudaStream_t stream) {
+                               int32_t* expert_counts, int32_t* position, cudaStream_t stream) {
   if (!router_topk_arguments_valid(rows, experts, top_k, n_group, topk_group)) {
     return cudaErrorInvalidValue;
   }
   auto run = [&](auto kernel) {
     kernel<<<rows, kTopkThreads, 0, stream>>>(logits, bias, experts, top_k, n_group, topk_group,
                                               norm_topk_prob, routed_scaling, top_index, top_weight,
-                                              expert_counts);
+                                              expert_counts, position);
   };
   if (experts <= 128) {
     run(router_topk_kernel<4>);

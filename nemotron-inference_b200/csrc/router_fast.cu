@@ -538,7 +538,7 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
                            int rows, int experts, int hidden, int top_k, bool norm_topk_prob,
                            float routed_scaling, float tie_margin,
                            int32_t* __restrict__ top_index, float* __restrict__ top_weight,
-                           int32_t* __restrict__ expert_counts) {
+                           int32_t* __restrict__ expert_counts, int32_t* __restrict__ position) {
   static_assert(WARPS == 1 || WARPS == kSelectWarps, "one warp, or the block, per token");
   __shared__ int16_t candidate_list[kSelectWarps][256];
   __shared__ float logit_smem[WARPS > 1 ? 256 : 1];
@@ -759,7 +759,8 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
     top_index[static_cast<size_t>(row) * top_k + lane] = my_index;
     top_weight[static_cast<size_t>(row) * top_k + lane] = w;
     if (expert_counts != nullptr && static_cast<uint32_t>(my_index) < static_cast<uint32_t>(experts)) {
-      atomicAdd(&expert_counts[my_index], 1);
+      const int place = atomicAdd(&expert_counts[my_index], 1);
+      if (position != nullptr) position[static_cast<size_t>(row) * top_k + lane] = place;
     }
   }
 }
@@ -835,7 +836,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        const float* bias, int rows, int experts, int hidden,
                                        int top_k, bool norm_topk_prob, float routed_scaling,
                                        float tie_margin, int32_t* top_index, float* top_weight,
-                                       int32_t* expert_counts, cudaStream_t stream) {
+                                       int32_t* expert_counts, int32_t* position, cudaStream_t stream) {
   if (rows <= 0 || experts % 32 != 0 || experts > 32 * kSelectPerLane || top_k <= 0 ||
       top_k > 32 || top_k > experts || hidden % 8 != 0 || splits < 1) {
     return cudaErrorInvalidValue;
@@ -845,7 +846,8 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
   auto run = [&](auto kernel) {
     kernel<<<grid, kSelectWarps * 32, 0, stream>>>(
         logits, splits, x, inv_rms, norm_weight, gate, logit_offset, bias, rows, experts, hidden,
-        top_k, norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts);
+        top_k, norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts,
+        position);
   };
   auto run_batch = [&](auto bf16, auto warps) {
     if (top_k <= 4) {
