@@ -152,6 +152,27 @@ __device__ __forceinline__ uint64_t div2_by_reciprocal(uint64_t x, uint64_t minu
   return fma2(fma2(q, minus_d, x), r, q);
 }
 
+// Programmatic dependent launch.  The successor on the stream may become resident once every CTA has
+// called release_successor(), so a kernel that allocates TMEM calls it after that (a successor that
+// took the columns first would wait for this kernel, and this kernel for the columns).  Every thread
+// calls wait_for_predecessor() before it touches what other kernels write or read: it returns when
+// the predecessor, and with it all that came before, is complete and visible.  Pointers to such data
+// are not `const __restrict__`, so that no load of theirs moves ahead of it.
+__device__ __forceinline__ void release_successor() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_predecessor() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Asks for `bytes` (a multiple of 16, from a 16-byte boundary) to be brought into L2.
+__device__ __forceinline__ void prefetch_l2_bulk(const void* from, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* from) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(from));
+}
+
 // The fused quantiser of the up-projection epilogue: 16 non-negative values in pairs whose maximum
 // is `amax`, per-row tensor scale 1 (nvfp4_packing.cpp:119-153 with tensor_scale == 1.0).
 // Bit-identical to quantize_block16(v, 1.0f, ..).

@@ -53,8 +53,10 @@ __global__ void relu2_kernel(float* __restrict__ values, size_t count) {
 }
 
 // out[t] = ((0 + parts[t][0]) + parts[t][1]) + ... : routed_row of expert_layer.cpp:951-953
-__global__ void sum_parts_kernel(const float* __restrict__ parts, int rows, int cols, int top_k,
+__global__ void sum_parts_kernel(const float* parts, int rows, int cols, int top_k,
                                  float* __restrict__ out) {
+  release_successor();
+  wait_for_predecessor();
   const int quads = cols / 4;
   const size_t total = static_cast<size_t>(rows) * quads;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -75,9 +77,11 @@ __global__ void sum_parts_kernel(const float* __restrict__ parts, int rows, int 
 }
 
 template <bool IN_BF16, bool OUT_BF16>
-__global__ void mixer_kernel(const void* __restrict__ in, const float* __restrict__ projected,
-                             const float* __restrict__ shared, size_t count,
+__global__ void mixer_kernel(const void* __restrict__ in, const float* projected,
+                             const float* shared, size_t count,
                              void* __restrict__ out) {
+  release_successor();
+  wait_for_predecessor();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     float x;
@@ -130,26 +134,26 @@ cudaError_t launch_relu2(float* values, size_t count, cudaStream_t stream) {
 }
 
 cudaError_t launch_sum_parts(const float* parts, int rows, int cols, int top_k, float* out,
-                             cudaStream_t stream) {
+                             LaunchStream stream) {
   if (rows <= 0 || cols % 4 != 0 || top_k < 1) return cudaErrorInvalidValue;
-  sum_parts_kernel<<<blocks_for(static_cast<size_t>(rows) * (cols / 4), 256), 256, 0, stream>>>(
+  launch_kernel(sum_parts_kernel, blocks_for(static_cast<size_t>(rows) * (cols / 4), 256), 256, 0, stream,
       parts, rows, cols, top_k, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_mixer(const void* in, bool in_bf16, const float* projected, const float* shared,
-                         int rows, int hidden, void* out, bool out_bf16, cudaStream_t stream) {
+                         int rows, int hidden, void* out, bool out_bf16, LaunchStream stream) {
   if (rows <= 0 || hidden <= 0) return cudaErrorInvalidValue;
   const size_t count = static_cast<size_t>(rows) * hidden;
   const int blocks = blocks_for(count, 256);
   if (in_bf16 && out_bf16) {
-    mixer_kernel<true, true><<<blocks, 256, 0, stream>>>(in, projected, shared, count, out);
+    launch_kernel(mixer_kernel<true, true>, blocks, 256, 0, stream, in, projected, shared, count, out);
   } else if (in_bf16) {
-    mixer_kernel<true, false><<<blocks, 256, 0, stream>>>(in, projected, shared, count, out);
+    launch_kernel(mixer_kernel<true, false>, blocks, 256, 0, stream, in, projected, shared, count, out);
   } else if (out_bf16) {
-    mixer_kernel<false, true><<<blocks, 256, 0, stream>>>(in, projected, shared, count, out);
+    launch_kernel(mixer_kernel<false, true>, blocks, 256, 0, stream, in, projected, shared, count, out);
   } else {
-    mixer_kernel<false, false><<<blocks, 256, 0, stream>>>(in, projected, shared, count, out);
+    launch_kernel(mixer_kernel<false, false>, blocks, 256, 0, stream, in, projected, shared, count, out);
   }
   return cudaGetLastError();
 }

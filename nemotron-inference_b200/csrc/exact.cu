@@ -549,7 +549,7 @@ __host__ __device__ constexpr int gemv_slot(int k) { return k + (k >> 4); }
 // layer (22 MB of FP8) 37 -> 15 us.
 template <int KIND, int ROWS>
 __global__ void __launch_bounds__(kGemvThreads)
-exact_gemv_kernel(const float* __restrict__ in, float fp8_scale, int N, int K,
+exact_gemv_kernel(const float* in, float fp8_scale, int N, int K,
                   const void* __restrict__ weight, float weight_scale,
                   const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
   constexpr int V = WeightVector<KIND>::kCount;
@@ -557,12 +557,32 @@ exact_gemv_kernel(const float* __restrict__ in, float fp8_scale, int N, int K,
   extern __shared__ double xs[];
   const int lane = threadIdx.x & 31;
   const int padded = gemv_slot(K);
+  release_successor();
+  {
+    // this warp's first two weight rows need not wait for the token rows
+    const size_t row_bytes = static_cast<size_t>(K) * (16 / V);
+    const int p = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (2 * p + 1 < N) {
+      const uint8_t* first = reinterpret_cast<const uint8_t*>(weight) + 2 * p * row_bytes;
+      for (size_t b = lane * 128; b < 2 * row_bytes; b += 32 * 128) prefetch_l2(first + b);
+    }
+  }
+  wait_for_predecessor();
+  // (the loads of four steps are issued before the stores of the first)
+  for (int k0 = threadIdx.x; k0 < ROWS * K; k0 += 4 * kGemvThreads) {
+    float x[4];
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r) {
-#pragma unroll 4
-    for (int k = threadIdx.x; k < K; k += kGemvThreads) {
-      xs[r * padded + gemv_slot(k)] =
-          static_cast<double>(input_value(in[static_cast<size_t>(r) * K + k], fp8_scale));
+    for (int i = 0; i < 4; ++i) {
+      const int k = k0 + i * kGemvThreads;
+      if (k < ROWS * K) x[i] = in[k];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = k0 + i * kGemvThreads;
+      const int r = k / K;
+      if (k < ROWS * K) {
+        xs[r * padded + gemv_slot(k - r * K)] = static_cast<double>(input_value(x[i], fp8_scale));
+      }
     }
   }
   __syncthreads();
@@ -620,7 +640,7 @@ exact_gemv_kernel(const float* __restrict__ in, float fp8_scale, int N, int K,
 // thread widens its own part of both.
 template <int KIND, int ROWS>
 __global__ void __launch_bounds__(kGemvThreads)
-exact_gemv_block_kernel(const float* __restrict__ in, float fp8_scale, int rows, int N, int K,
+exact_gemv_block_kernel(const float* in, float fp8_scale, int rows, int N, int K,
                         const void* __restrict__ weight, float weight_scale,
                         const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
   constexpr int V = WeightVector<KIND>::kCount;
@@ -632,6 +652,14 @@ exact_gemv_block_kernel(const float* __restrict__ in, float fp8_scale, int rows,
   double acc[ROWS];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) acc[r] = 0.0;
+  release_successor();
+  if (row0 == 0) {
+    // the weight row need not wait for the token rows
+    for (int b = threadIdx.x * 128; b < K * (16 / V); b += kGemvThreads * 128) {
+      prefetch_l2(reinterpret_cast<const uint8_t*>(w) + b);
+    }
+  }
+  wait_for_predecessor();
 #pragma unroll 2
   for (int q = threadIdx.x; q * V < K; q += kGemvThreads) {
     float v[V];
@@ -681,7 +709,7 @@ bool gemv_by_blocks(int N, int num_sms) {
 template <int KIND, int ROWS>
 cudaError_t launch_gemv_rows(const float* in, float fp8_scale, int N, int K, const void* weight,
                              float weight_scale, const float* offset, bool relu2, float* out,
-                             int num_sms, cudaStream_t stream) {
+                             int num_sms, LaunchStream stream) {
   const int smem = ROWS * gemv_slot(K) * static_cast<int>(sizeof(double));
   auto kernel = exact_gemv_kernel<KIND, ROWS>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -690,18 +718,20 @@ cudaError_t launch_gemv_rows(const float* in, float fp8_scale, int N, int K, con
   const int resident = std::min(8, std::max(1, 220 * 1024 / (smem + 1024)));
   const int per_block = 2 * (kGemvThreads / 32);
   const int grid = std::min((N + per_block - 1) / per_block, num_sms * resident);
-  kernel<<<grid, kGemvThreads, smem, stream>>>(in, fp8_scale, N, K, weight, weight_scale, offset,
-                                               relu2, out);
+  // not resident early: placed while another kernel's blocks hold part of the shared memory, the
+  // blocks spread unevenly (a latent model's pass over 1 token 127 us, 106 in this way)
+  launch_kernel(kernel, grid, kGemvThreads, smem, stream.stream, in, fp8_scale, N, K, weight,
+                weight_scale, offset, relu2, out);
   return cudaGetLastError();
 }
 
 template <int KIND>
 cudaError_t launch_gemv_kind(const float* in, float fp8_scale, int rows, int N, int K,
                              const void* weight, float weight_scale, const float* offset,
-                             bool relu2, float* out, int num_sms, cudaStream_t stream) {
+                             bool relu2, float* out, int num_sms, LaunchStream stream) {
   if (gemv_by_blocks(N, num_sms)) {
     auto run = [&](auto kernel, int per_block) {
-      kernel<<<dim3(N, (rows + per_block - 1) / per_block), kGemvThreads, 0, stream>>>(
+      launch_kernel(kernel, dim3(N, (rows + per_block - 1) / per_block), kGemvThreads, 0, stream,
           in, fp8_scale, rows, N, K, weight, weight_scale, offset, relu2, out);
     };
     if (rows == 1) {
@@ -826,7 +856,7 @@ bool exact_prefers_gemv(int rows, int N, int K, int num_sms) {
 
 cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,
                               const float* offset, bool relu2, float* out, int num_sms,
-                              cudaStream_t stream) {
+                              LaunchStream stream) {
   if (rows <= 0 || !exact_supported(w.N, w.K)) return cudaErrorInvalidValue;
   if (w.kind == kWeightFp8) {
     return launch_gemv_kind<kWeightFp8>(in, fp8_scale, rows, w.N, w.K, w.weight, w.scale, offset,

@@ -201,6 +201,27 @@ __device__ __forceinline__ void issue_block(uint32_t d_tmem, uint64_t a_desc, ui
   }
 }
 
+// The weights of the shared expert's (dense) phases into L2, tile by tile over all CTAs: HBM is idle
+// while the small kernels before this one route the tokens.
+__device__ __forceinline__ void fetch_dense_weights(const StreamArgs& args, int unit, int units,
+                                                    int lane) {
+  for (int p = 0; p < args.phases; ++p) {
+    const GemmArgs& g = args.phase[p].gemm;
+    if (g.row_tiles != nullptr) continue;
+    for (int nt = unit; nt < g.n_tiles; nt += units) {
+      const int b_row = nt * kBN;
+      const uint32_t b_bytes = static_cast<uint32_t>(min(kBN, g.N - b_row)) * 128u;
+      for (int kb = lane; kb < g.kb_full; kb += 32) {
+        prefetch_l2_bulk(g.b_full + (static_cast<size_t>(kb) * g.N + b_row) * 128, b_bytes);
+      }
+      if (lane == 0) {
+        prefetch_l2_bulk(g.sfb + static_cast<size_t>(nt) * g.k_blocks * kSfbBytes,
+                         static_cast<uint32_t>(g.k_blocks) * kSfbBytes);
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   extern __shared__ uint8_t smem_raw[];
@@ -254,6 +275,9 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  release_successor();
+  if (warp == 0 && args.fetch_dense) fetch_dense_weights(args, unit, units, lane);
+  wait_for_predecessor();
 
   float* few_rows = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(full_bar) + kBarBytes);
   const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), sfa0 = smem_u32(sSFA), sfb0 = smem_u32(sSFB);
@@ -577,7 +601,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
 
 GemmTileInfo stream_tile_info() { return GemmTileInfo{kBN, 4, kSfbBytes, kBN}; }
 
-cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, cudaStream_t stream) {
+cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, LaunchStream stream) {
   if (args.phases < 1 || args.phases > kStreamPhases || num_sms < 1 ||
       (args.tile_rows != 32 && args.tile_rows != 64 && args.tile_rows != 128)) {
     return cudaErrorInvalidValue;
@@ -596,8 +620,7 @@ cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, cudaStream
     dense_tiles += (g.dense_rows + 127) / 128 * g.n_tiles;
   }
   if (!grouped) grid = std::max(1, std::min(grid, dense_tiles));
-  expert_stream_kernel<<<grid, kThreads, smem_bytes(args.tile_rows), stream>>>(args);
-  return cudaGetLastError();
+  return launch_kernel(expert_stream_kernel, grid, kThreads, smem_bytes(args.tile_rows), stream, args);
 }
 
 }  // namespace nmoe

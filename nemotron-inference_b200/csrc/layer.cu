@@ -476,8 +476,9 @@ struct StreamCounts {
 // The shared expert comes first among the up projections and among the down projections: its down
 // tiles are the longest, and short ones end together.
 void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCounts& counts,
-                int32_t* error, int num_sms, cudaStream_t stream) {
+                int32_t* error, int num_sms, LaunchStream stream) {
   StreamArgs args;
+  args.fetch_dense = stream.chained;
   args.error = error;
   args.finished = counts.words.as<int32_t>();
   args.ticket = counts.words.as<int32_t>() + 1;
@@ -719,7 +720,7 @@ struct ExactScratch {
 
 void run_exact(const ExactWeight& w, ExactScratch& scratch, const float* in, float fp8_scale,
                int rows, const float* offset, bool relu2, float* out, int32_t* error, int num_sms,
-               cudaStream_t stream) {
+               LaunchStream stream) {
   if (fp8_scale != 0.0f) fp8_scale = clamp_scale_host(fp8_scale);  // scaled_fp8_linear.cu:27-33
   if (exact_prefers_gemv(rows, w.N, w.K, num_sms)) {
     NMOE_CUDA(launch_exact_gemv(w, in, fp8_scale, rows, offset, relu2, out, num_sms, stream));
@@ -845,7 +846,8 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
       both.hidden = &ffn->h_op;
       both.out = out;
       both.row_slots = (static_cast<int>(rows) + 127) / 128;
-      run_stream(nullptr, &both, ffn->stream_counts, error, ffn->num_sms, stream);
+      run_stream(nullptr, &both, ffn->stream_counts, error, ffn->num_sms,
+                 LaunchStream(stream, true));
     } else {
       run_expert_gemms(ffn->up, ffn->down, tile_class, ffn->a_op, ffn->a_ts.as<float>(), schedule,
                        ffn->h_packed.as<uint8_t>(), ffn->h_sf.as<uint8_t>(), ffn->h_op, out, error,
@@ -1269,7 +1271,7 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
 
 // y = x W^T of a dense / scaled-FP8 linear, rounded once from the FP64 sum [, relu^2 of it].
 void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, int rows,
-                float* out_rows, bool relu2, cudaStream_t stream) {
+                float* out_rows, bool relu2, LaunchStream stream) {
   if (linear.exact) {
     run_exact(linear.operand.w, L->exact, in_rows, linear.fp8 ? linear.input_scale : 0.0f, rows,
               nullptr, relu2, out_rows, L->error.device.as<int32_t>(), L->num_sms, stream);
@@ -1290,7 +1292,7 @@ void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, 
 
 // RMSNorm + activation quantiser + router: fills normalized, y_*, logits,
 // top_index / top_weight, the per-expert histogram `counts` (global ids) and each pair's position in it.
-void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype in_dtype,
+void route_tokens(nmoe_layer* L, LaunchStream stream, const void* input, nmoe_dtype in_dtype,
                   int tokens, cudaEvent_t after_quantise = nullptr,
                   bool fork_after_logits = false) {
   const nmoe_config& c = L->cfg;
@@ -1307,7 +1309,7 @@ void route_tokens(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dt
                               c.rms_epsilon, want_normalized ? L->normalized.as<float>() : nullptr,
                               L->y_packed.as<uint8_t>(), L->y_sf_row_major.as<uint8_t>(),
                               L->y_sf_tiled.as<uint8_t>(), k_blocks_of(H), L->y_ts.as<float>(),
-                              stream, L->inv_rms.as<float>(), L->counts.as<int32_t>(), E));
+                              stream.stream, L->inv_rms.as<float>(), L->counts.as<int32_t>(), E));
   L->last_normalized = want_normalized;
   if (after_quantise != nullptr && !fork_after_logits) {
     NMOE_CUDA(cudaEventRecord(after_quantise, stream));
@@ -1416,7 +1418,7 @@ TileClass routed_tile_class(const nmoe_layer* L, int pairs) {
 // Plan + permute + the grouped GEMMs over `pairs` (row, slot) pairs whose per-local-expert
 // histogram is already in `counts`.  `shared` (stream class only): the shared expert's tiles join
 // the same launch.
-void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& source, int pairs,
+void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& source, int pairs,
                     int dest_stride, void* out_rows, RowKind out_kind,
                     RowSegments segments = RowSegments(), const StreamFfn* shared = nullptr) {
   const int Lr = L->latent;
@@ -1428,6 +1430,7 @@ void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& sou
   plan.row_tiles = L->row_tiles.as<RowTile>();
   plan.num_row_tiles = L->num_row_tiles.as<int32_t>();
   if (source.position == nullptr) {
+    stream.chained = false;
     NMOE_CUDA(cudaMemsetAsync(plan.expert_cursor, 0, L->local_experts * sizeof(int32_t), stream));
   }
   L->mark(4, stream);
@@ -1438,6 +1441,7 @@ void routed_experts(nmoe_layer* L, cudaStream_t stream, const PermuteSource& sou
                               L->a_dest.as<int32_t>(),
                               L->ep_world == 1 ? L->pair_row.as<int32_t>() : nullptr, dest_stride,
                               error, stream));
+  if (!L->stage_timing) stream.chained = true;
   L->mark(5, stream);
   // routed experts (:896-954)
   Schedule routed;
@@ -1486,7 +1490,7 @@ TileClass shared_tile_class(const nmoe_layer* L, int tokens) {
 
 // The shared expert's hidden rows in FP32: shared_up and relu^2 (:814-818, :956-964), by a dense /
 // scaled-FP8 linear or an NVFP4 GEMM.
-void shared_hidden_rows(nmoe_layer* L, cudaStream_t stream, int tokens) {
+void shared_hidden_rows(nmoe_layer* L, LaunchStream stream, int tokens) {
   float* raw = L->shared_raw.as<float>();
   if (L->shared_up_dense.present) {
     run_linear(L, L->shared_up_dense, L->normalized.as<float>(), tokens, raw, /*relu2=*/true,
@@ -1505,7 +1509,7 @@ void shared_hidden_rows(nmoe_layer* L, cudaStream_t stream, int tokens) {
 
 // ... and quantised for an NVFP4 down projection, through the host linear's own packing step
 // (:981-1005).
-void quantise_shared_hidden(nmoe_layer* L, cudaStream_t stream, int tokens) {
+void quantise_shared_hidden(nmoe_layer* L, LaunchStream stream, int tokens) {
   const int S = L->cfg.shared_expert_intermediate_size;
   NMOE_CUDA(launch_norm_quant(L->shared_raw.as<float>(), false, tokens, S, nullptr, 0.0f, nullptr,
                               L->sh_packed.as<uint8_t>(), nullptr, L->sh_sf.as<uint8_t>(),
@@ -1549,7 +1553,7 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
 
 // The shared expert as part of the routed experts' launch (csrc/expert_stream.cu); rows of a dense
 // shared_up are made here, before it.
-StreamFfn shared_stream_ffn(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_rows,
+StreamFfn shared_stream_ffn(nmoe_layer* L, LaunchStream stream, int tokens, void* out_rows,
                             int dest_mul, int dest_add, RowKind out_kind) {
   StreamFfn ffn;
   ffn.down = &L->shared_down;
@@ -1613,7 +1617,11 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   const bool fork = L->side_stream != nullptr && !L->stage_timing && !one_launch &&
                     tokens <= L->fork_max_tokens && !L->latent_mode && !dense_shared;
   const bool two_pass = L->fast_router && tokens >= L->fast_router_min_tokens;
-  route_tokens(L, stream, input, in_dtype, tokens, fork ? L->quant_done : nullptr,
+  // One kernel after the other on one stream, and small enough for the gaps between them to count:
+  // with the two-pass router there was nothing to gain (256 tokens 162 us either way) and at 700
+  // tokens 2 to 4 us to lose.
+  const LaunchStream chain(stream, !fork && !L->stage_timing && !L->unfused && !two_pass);
+  route_tokens(L, chain, input, in_dtype, tokens, fork ? L->quant_done : nullptr,
                fork && two_pass);
   L->last_tokens = tokens;
   L->last_parts_kind = parts_kind;
@@ -1622,11 +1630,11 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     // latent = fc1_latent(normalized) (:809-813); every routed expert's up_proj packs
     // the same latent row (:913 -> nvfp4_packing.cpp:90)
     run_linear(L, L->fc1, L->normalized.as<float>(), tokens, L->latent_rows.as<float>(), false,
-               stream);
+               chain);
     NMOE_CUDA(launch_norm_quant(L->latent_rows.as<float>(), false, tokens, Lr, nullptr, 0.0f,
                                 nullptr, L->lat_packed.as<uint8_t>(),
                                 L->lat_sf_row_major.as<uint8_t>(), nullptr, 0,
-                                L->lat_ts.as<float>(), stream));
+                                L->lat_ts.as<float>(), chain));
     PermuteSource source = local_source(L);
     source.packed = L->lat_packed.as<uint8_t>();
     source.packed_stride = static_cast<size_t>(Lr) / 2;
@@ -1635,11 +1643,11 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     source.tensor_scale = L->lat_ts.as<float>();
     if (one_launch) {
       const StreamFfn shared =
-          shared_stream_ffn(L, stream, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
-      routed_experts(L, stream, source, tokens * K, K, L->parts.as<void>(), kRowF32, RowSegments(),
+          shared_stream_ffn(L, chain, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
+      routed_experts(L, chain, source, tokens * K, K, L->parts.as<void>(), kRowF32, RowSegments(),
                      &shared);
     } else {
-      routed_experts(L, stream, source, tokens * K, K, L->parts.as<void>(), kRowF32);
+      routed_experts(L, chain, source, tokens * K, K, L->parts.as<void>(), kRowF32);
       L->mark(7, stream);
       shared_expert(L, stream, tokens, L->shared_rows.as<void>(), 1, 0,
                     L->stage_timing ? L->stage_events[8] : nullptr, kRowF32);
@@ -1648,12 +1656,12 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     // routed sum in selection order (:951-953), fc2_latent (:1047-1053), mixer and
     // residual (:1064-1069)
     NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
-                               stream));
+                               chain));
     run_linear(L, L->fc2, L->routed_latent.as<float>(), tokens, L->projected.as<float>(), false,
-               stream);
+               chain);
     NMOE_CUDA(launch_mixer(input, in_dtype == NMOE_BF16, L->projected.as<float>(),
                            L->shared_rows.as<float>(), tokens, H, output, out_dtype == NMOE_BF16,
-                           stream));
+                           chain));
     L->mark(10, stream);
     return;
   }
@@ -1664,11 +1672,11 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   }
   if (one_launch) {
     const StreamFfn shared =
-        shared_stream_ffn(L, stream, tokens, L->parts.as<void>(), K + 1, K, parts_kind);
-    routed_experts(L, stream, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind,
+        shared_stream_ffn(L, chain, tokens, L->parts.as<void>(), K + 1, K, parts_kind);
+    routed_experts(L, chain, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind,
                    RowSegments(), &shared);
   } else {
-    routed_experts(L, stream, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind);
+    routed_experts(L, chain, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind);
   }
   L->mark(7, stream);
   if (one_launch) {
@@ -1683,7 +1691,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   L->mark(9, stream);
   NMOE_CUDA(launch_combine(input, in_dtype == NMOE_BF16, L->parts.as<void>(), parts_kind, tokens,
                            H, K, output, out_dtype == NMOE_BF16, L->error.device.as<int32_t>(),
-                           stream));
+                           chain));
   L->mark(10, stream);
 }
 

@@ -119,6 +119,8 @@ place_rows_kernel(PlanBuffers plan, PermuteSource src, int pairs, int share, int
                   int dest_stride, int32_t* error) {
   __shared__ int first_tile[kMaxPlanExperts];
   __shared__ int tiles_of[kMaxPlanExperts];
+  release_successor();
+  wait_for_predecessor();
   const int total = scan_expert_tiles<kPlaceThreads>(plan.expert_counts, experts, tile_multiple,
                                                      first_tile, tiles_of);
   if (blockIdx.x == 0) {
@@ -302,9 +304,11 @@ __device__ __forceinline__ void store_row8(void* base, size_t row, int hidden, i
 // row and the residual (:1064-1069).  Eight elements per thread, 16- or 32-byte
 // accesses; the parts are rows of RowKind PARTS.
 template <bool IN_BF16, bool OUT_BF16, int PARTS>
-__global__ void combine_kernel(const void* __restrict__ in, const void* __restrict__ parts,
+__global__ void combine_kernel(const void* __restrict__ in, const void* parts,
                                int rows, int hidden, int top_k, void* __restrict__ out,
                                int32_t* __restrict__ error) {
+  release_successor();
+  wait_for_predecessor();
   const int octs = hidden / 8;
   const size_t total = static_cast<size_t>(rows) * octs;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -340,15 +344,15 @@ __global__ void combine_kernel(const void* __restrict__ in, const void* __restri
 
 template <bool A, bool B>
 void launch_combine_t(const void* in, const void* parts, RowKind parts_kind, int rows, int hidden,
-                      int top_k, void* out, int32_t* error, int blocks, cudaStream_t stream) {
+                      int top_k, void* out, int32_t* error, int blocks, LaunchStream stream) {
   if (parts_kind == kRowBf16) {
-    combine_kernel<A, B, kRowBf16><<<blocks, 256, 0, stream>>>(in, parts, rows, hidden, top_k, out,
+    launch_kernel(combine_kernel<A, B, kRowBf16>, blocks, 256, 0, stream, in, parts, rows, hidden, top_k, out,
                                                                error);
   } else if (parts_kind == kRowF16) {
-    combine_kernel<A, B, kRowF16><<<blocks, 256, 0, stream>>>(in, parts, rows, hidden, top_k, out,
+    launch_kernel(combine_kernel<A, B, kRowF16>, blocks, 256, 0, stream, in, parts, rows, hidden, top_k, out,
                                                               error);
   } else {
-    combine_kernel<A, B, kRowF32><<<blocks, 256, 0, stream>>>(in, parts, rows, hidden, top_k, out,
+    launch_kernel(combine_kernel<A, B, kRowF32>, blocks, 256, 0, stream, in, parts, rows, hidden, top_k, out,
                                                               error);
   }
 }
@@ -360,7 +364,7 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               int k_blocks, uint8_t* sorted_packed, uint8_t* sorted_sf_tiled,
                               float* sorted_tensor_scale, float* sorted_weight,
                               int32_t* sorted_dest, int32_t* pair_row, int dest_stride,
-                              int32_t* error, cudaStream_t stream) {
+                              int32_t* error, LaunchStream stream) {
   if (pairs <= 0 || src.pairs_per_row <= 0 || src.pairs_per_row > 32 ||
       pairs % src.pairs_per_row != 0 || experts <= 0 || experts > kMaxPlanExperts ||
       tile_multiple < 1) {
@@ -374,7 +378,7 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
   const int blocks = std::min((units + kWarps - 1) / kWarps, 148 * 6);  // each pays for the scan
   const PlacedRows out{sorted_packed, sorted_sf_tiled, sorted_tensor_scale, sorted_weight,
                        sorted_dest, pair_row};
-  place_rows_kernel<<<blocks, kPlaceThreads, 0, stream>>>(plan, src, pairs, share, experts,
+  launch_kernel(place_rows_kernel, blocks, kPlaceThreads, 0, stream, plan, src, pairs, share, experts,
                                                           tile_multiple, max_row_tiles, cols,
                                                           k_blocks * 4, out, dest_stride, error);
   return cudaGetLastError();
@@ -382,7 +386,7 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
 
 cudaError_t launch_combine(const void* in, bool in_bf16, const void* parts, RowKind parts_kind,
                            int rows, int hidden, int top_k, void* out, bool out_bf16,
-                           int32_t* error, cudaStream_t stream) {
+                           int32_t* error, LaunchStream stream) {
   if (rows <= 0 || hidden % 8 != 0 || top_k < 1) return cudaErrorInvalidValue;
   const size_t total = static_cast<size_t>(rows) * (hidden / 8);
   const int blocks = static_cast<int>(std::min<size_t>((total + 255) / 256, 148 * 16));

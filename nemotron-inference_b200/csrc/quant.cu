@@ -87,12 +87,14 @@ __device__ __forceinline__ void zero_words(int32_t* words, int count) {
 // Rows of any length, and one tensor scale for a whole matrix (PER_ROW_SCALE false).
 template <bool BF16, bool PER_ROW_SCALE>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-norm_quant_kernel(const void* __restrict__ in, int rows, int cols,
+norm_quant_kernel(const void* in, int rows, int cols,
                   const float* __restrict__ norm_weight, float eps,
                   float* __restrict__ normalized, uint8_t* __restrict__ packed,
                   uint8_t* __restrict__ sf_row_major, uint8_t* __restrict__ sf_tiled, int k_tiles,
                   float* __restrict__ tensor_scale, const float* __restrict__ global_amax,
                   float* __restrict__ inv_rms_out, int32_t* __restrict__ zero, int zero_count) {
+  release_successor();
+  wait_for_predecessor();
   zero_words(zero, zero_count);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -219,13 +221,15 @@ norm_quant_kernel(const void* __restrict__ in, int rows, int cols,
 // 26.5 -> 23.2, 16384 rows 61 either way.
 template <bool BF16, int ITERS, bool SHARED>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-norm_quant_row_kernel(const void* __restrict__ in, int rows, int cols,
+norm_quant_row_kernel(const void* in, int rows, int cols,
                       const float* __restrict__ norm_weight, float eps,
                       float* __restrict__ normalized, uint8_t* __restrict__ packed,
                       uint8_t* __restrict__ sf_row_major, uint8_t* __restrict__ sf_tiled,
                       int k_tiles, float* __restrict__ tensor_scale,
                       float* __restrict__ inv_rms_out, int row_warp_shift, bool word_scales,
                       int32_t* __restrict__ zero, int zero_count) {
+  release_successor();
+  wait_for_predecessor();
   zero_words(zero, zero_count);
   const int lane = threadIdx.x & 31;
   const int warp_global = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -437,7 +441,7 @@ int grid_for(size_t work, int threads) {
 namespace {
 
 template <bool BF16, int ITERS>
-void launch_row_kernel(int rows, cudaStream_t stream, const void* in, int cols,
+void launch_row_kernel(int rows, LaunchStream stream, const void* in, int cols,
                        const float* norm_weight, float eps, float* normalized, uint8_t* packed,
                        uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles, float* tensor_scale,
                        float* inv_rms, int32_t* zero, int zero_count) {
@@ -451,7 +455,7 @@ void launch_row_kernel(int rows, cudaStream_t stream, const void* in, int cols,
       cols % 64 == 0 && ((reinterpret_cast<uintptr_t>(sf_row_major) |
                           reinterpret_cast<uintptr_t>(sf_tiled)) & 3u) == 0;
   auto run = [&](auto kernel) {
-    kernel<<<grid, kWarpsPerBlock * 32, 0, stream>>>(
+    launch_kernel(kernel, grid, kWarpsPerBlock * 32, 0, stream,
         in, rows, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
         tensor_scale, inv_rms, shift, word_scales, zero, zero_count);
   };
@@ -463,7 +467,7 @@ void launch_row_kernel(int rows, cudaStream_t stream, const void* in, int cols,
 }
 
 template <bool BF16>
-void launch_norm_quant_t(int rows, cudaStream_t stream, const void* in, int cols,
+void launch_norm_quant_t(int rows, LaunchStream stream, const void* in, int cols,
                          const float* norm_weight, float eps, float* normalized, uint8_t* packed,
                          uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles,
                          float* tensor_scale, float* inv_rms, int32_t* zero, int zero_count) {
@@ -482,7 +486,7 @@ void launch_norm_quant_t(int rows, cudaStream_t stream, const void* in, int cols
     run(launch_row_kernel<BF16, 21>);
   } else {
     const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    norm_quant_kernel<BF16, true><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
+    launch_kernel(norm_quant_kernel<BF16, true>, grid, kWarpsPerBlock * 32, 0, stream,
         in, rows, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
         tensor_scale, nullptr, inv_rms, zero, zero_count);
   }
@@ -493,7 +497,7 @@ void launch_norm_quant_t(int rows, cudaStream_t stream, const void* in, int cols
 cudaError_t launch_norm_quant(const void* in, bool in_bf16, int rows, int cols,
                               const float* norm_weight, float eps, float* normalized,
                               uint8_t* packed, uint8_t* sf_row_major, uint8_t* sf_tiled,
-                              int k_blocks, float* tensor_scale, cudaStream_t stream,
+                              int k_blocks, float* tensor_scale, LaunchStream stream,
                               float* inv_rms, int32_t* zero, int zero_count) {
   if (rows <= 0 || cols <= 0 || cols % 16 != 0) return cudaErrorInvalidValue;
   if (in_bf16) {

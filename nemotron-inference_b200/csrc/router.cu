@@ -125,7 +125,7 @@ constexpr int kTopkThreads = 128;
 // (between events): 1 token, 128 experts, top-6 14.9 -> 8.4 us; 512 experts, top-22 33 -> 14.3.
 template <int PER_LANE>
 __global__ void __launch_bounds__(kTopkThreads)
-router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int experts,
+router_topk_kernel(const float* logits, const float* __restrict__ bias, int experts,
                    int top_k, int n_group, int topk_group, bool norm_topk_prob,
                    float routed_scaling, int32_t* __restrict__ top_index,
                    float* __restrict__ top_weight, int32_t* __restrict__ expert_counts,
@@ -134,6 +134,8 @@ router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ b
   __shared__ float choice_smem[PER_LANE * 32];
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x;
+  release_successor();
+  wait_for_predecessor();
   for (int e = threadIdx.x; e < experts; e += kTopkThreads) {
     const float score = sigmoid_ref(logits[static_cast<size_t>(row) * experts + e]);
     score_smem[e] = score;
@@ -266,12 +268,12 @@ bool router_topk_arguments_valid(int rows, int experts, int top_k, int n_group, 
 cudaError_t launch_router_topk(const float* logits, const float* bias, int rows, int experts,
                                int top_k, int n_group, int topk_group, bool norm_topk_prob,
                                float routed_scaling, int32_t* top_index, float* top_weight,
-                               int32_t* expert_counts, int32_t* position, cudaStream_t stream) {
+                               int32_t* expert_counts, int32_t* position, LaunchStream stream) {
   if (!router_topk_arguments_valid(rows, experts, top_k, n_group, topk_group)) {
     return cudaErrorInvalidValue;
   }
   auto run = [&](auto kernel) {
-    kernel<<<rows, kTopkThreads, 0, stream>>>(logits, bias, experts, top_k, n_group, topk_group,
+    launch_kernel(kernel, rows, kTopkThreads, 0, stream, logits, bias, experts, top_k, n_group, topk_group,
                                               norm_topk_prob, routed_scaling, top_index, top_weight,
                                               expert_counts, position);
   };

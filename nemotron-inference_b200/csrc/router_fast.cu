@@ -76,7 +76,7 @@ __device__ __forceinline__ void load_x8(const void* x, size_t index, float (&v)[
 
 template <bool IN_BF16>
 __global__ void __launch_bounds__(kFastThreads, 1)
-router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ inv_rms,
+router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
                           const float* __restrict__ norm_weight,
                           const __grid_constant__ CUtensorMap tmap_gate, int rows, int experts,
                           int hidden, int splits, float* __restrict__ logits, int32_t* error) {
@@ -121,6 +121,8 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* __restrict__ 
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  release_successor();
+  wait_for_predecessor();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -328,7 +330,7 @@ __global__ void fold_gate_kernel(const __nv_bfloat16* __restrict__ gate,
 __global__ void __launch_bounds__(kFoldThreads, 1)
 router_folded_logits_kernel(const __grid_constant__ CUtensorMap tmap_x,
                             const __grid_constant__ CUtensorMap tmap_planes,
-                            const float* __restrict__ inv_rms, int rows, int experts, int hidden,
+                            const float* inv_rms, int rows, int experts, int hidden,
                             int stages, int splits, float* __restrict__ logits, int32_t* error) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
@@ -373,6 +375,8 @@ router_folded_logits_kernel(const __grid_constant__ CUtensorMap tmap_x,
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  release_successor();
+  wait_for_predecessor();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -531,7 +535,7 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 template <bool IN_BF16, int WARPS, int BATCH>
 __global__ void __launch_bounds__(kSelectWarps * 32)
 router_select_exact_kernel(float* __restrict__ logits, int splits, const void* __restrict__ x,
-                           const float* __restrict__ inv_rms,
+                           const float* inv_rms,
                            const float* __restrict__ norm_weight,
                            const __nv_bfloat16* __restrict__ gate,
                            const float* __restrict__ logit_offset, const float* __restrict__ bias,
@@ -543,6 +547,8 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
   __shared__ int16_t candidate_list[kSelectWarps][256];
   __shared__ float logit_smem[WARPS > 1 ? 256 : 1];
   __shared__ double partial_smem[WARPS > 1 ? kSelectWarps : 1][8];
+  release_successor();
+  wait_for_predecessor();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int part = WARPS > 1 ? warp : 0;  // this warp's share of the contraction
@@ -770,7 +776,7 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
 cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* inv_rms,
                                       const float* norm_weight, const CUtensorMap& tmap_gate,
                                       int rows, int experts, int hidden, int splits,
-                                      float* logits, int32_t* error, cudaStream_t stream) {
+                                      float* logits, int32_t* error, LaunchStream stream) {
   if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0 ||
       splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
@@ -782,13 +788,13 @@ cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* i
     err = cudaFuncSetAttribute(router_fast_logits_kernel<true>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return err;
-    router_fast_logits_kernel<true><<<grid, kFastThreads, smem, stream>>>(
+    launch_kernel(router_fast_logits_kernel<true>, grid, kFastThreads, smem, stream,
         x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
   } else {
     err = cudaFuncSetAttribute(router_fast_logits_kernel<false>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return err;
-    router_fast_logits_kernel<false><<<grid, kFastThreads, smem, stream>>>(
+    launch_kernel(router_fast_logits_kernel<false>, grid, kFastThreads, smem, stream,
         x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
   }
   return cudaGetLastError();
@@ -813,7 +819,7 @@ int router_pass1_splits(int rows, int hidden, int num_sms) {
 cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtensorMap& tmap_planes,
                                         const float* inv_rms, int rows, int experts, int hidden,
                                         int splits, float* logits, int32_t* error,
-                                        cudaStream_t stream) {
+                                        LaunchStream stream) {
   if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0 ||
       splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
@@ -825,7 +831,7 @@ cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtenso
   cudaError_t err = cudaFuncSetAttribute(router_folded_logits_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;
-  router_folded_logits_kernel<<<((rows + 127) / 128) * splits, kFoldThreads, smem, stream>>>(
+  launch_kernel(router_folded_logits_kernel, (rows + 127) / 128 * splits, kFoldThreads, smem, stream,
       tmap_x, tmap_planes, inv_rms, rows, experts, hidden, stages, splits, logits, error);
   return cudaGetLastError();
 }
@@ -836,7 +842,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        const float* bias, int rows, int experts, int hidden,
                                        int top_k, bool norm_topk_prob, float routed_scaling,
                                        float tie_margin, int32_t* top_index, float* top_weight,
-                                       int32_t* expert_counts, int32_t* position, cudaStream_t stream) {
+                                       int32_t* expert_counts, int32_t* position, LaunchStream stream) {
   if (rows <= 0 || experts % 32 != 0 || experts > 32 * kSelectPerLane || top_k <= 0 ||
       top_k > 32 || top_k > experts || hidden % 8 != 0 || splits < 1) {
     return cudaErrorInvalidValue;
@@ -844,7 +850,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
   const bool whole_block = rows <= kSelectWholeBlockRows;
   const int grid = whole_block ? rows : (rows + kSelectWarps - 1) / kSelectWarps;
   auto run = [&](auto kernel) {
-    kernel<<<grid, kSelectWarps * 32, 0, stream>>>(
+    launch_kernel(kernel, grid, kSelectWarps * 32, 0, stream,
         logits, splits, x, inv_rms, norm_weight, gate, logit_offset, bias, rows, experts, hidden,
         top_k, norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts,
         position);
