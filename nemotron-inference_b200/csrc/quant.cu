@@ -212,31 +212,24 @@ norm_quant_kernel(const void* in, int rows, int cols,
 
 // norm_quant_kernel for rows of up to ITERS * 256 elements, one tensor scale per row: the row
 // is read once and stays in registers (as FP32) through the three phases -- sum of squares,
-// maximum, codes -- which the general kernel above re-reads it for.  1 << row_warp_shift warps
-// work on a row: each holds all of it and repeats the first two phases (nothing to exchange),
-// the codes are shared out in pairs of 256-element steps.
-//
-// Bound by the latency of one load, one reduction and one step of codes.  Measured (between
-// events, hidden 2688, bf16 in): 1 row 18.5 -> 11.0 us, 1003 rows 17.7 -> 12.9, 4096 rows
-// 26.5 -> 23.2, 16384 rows 61 either way.
-template <bool BF16, int ITERS, bool SHARED>
+// maximum, codes -- which the general kernel above re-reads it for.  For batches whose rows are as
+// many as the warps that fit on the GPU; 4096 rows of 2688 took 26.5 us with the general kernel and
+// take 23.2, 16384 rows 61 either way.
+template <bool BF16, int ITERS>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 norm_quant_row_kernel(const void* in, int rows, int cols,
                       const float* __restrict__ norm_weight, float eps,
                       float* __restrict__ normalized, uint8_t* __restrict__ packed,
                       uint8_t* __restrict__ sf_row_major, uint8_t* __restrict__ sf_tiled,
                       int k_tiles, float* __restrict__ tensor_scale,
-                      float* __restrict__ inv_rms_out, int row_warp_shift, bool word_scales,
+                      float* __restrict__ inv_rms_out, bool word_scales,
                       int32_t* __restrict__ zero, int zero_count) {
   release_successor();
   wait_for_predecessor();
   zero_words(zero, zero_count);
   const int lane = threadIdx.x & 31;
-  const int warp_global = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  const int row = SHARED ? warp_global >> row_warp_shift : warp_global;
+  const int row = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= rows) return;
-  const int share_mask = SHARED ? (1 << row_warp_shift) - 1 : 0;
-  const int share = warp_global & share_mask;
   const size_t row_base = static_cast<size_t>(row) * cols;
   const int chunks = cols / 8;
 
@@ -276,7 +269,7 @@ norm_quant_row_kernel(const void* in, int rows, int cols,
     sum = __shfl_sync(0xffffffffu, sum, 0);
     const float mean = __fdiv_rn(sum, static_cast<float>(cols));
     const float inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
-    if (lane == 0 && share == 0 && inv_rms_out != nullptr) inv_rms_out[row] = inv_rms;
+    if (lane == 0 && inv_rms_out != nullptr) inv_rms_out[row] = inv_rms;
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
       const int ch = it * 32 + lane;
@@ -305,13 +298,13 @@ norm_quant_row_kernel(const void* in, int rows, int cols,
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, stride));
   }
   const float ts = tensor_scale_from_amax(amax);
-  if (lane == 0 && share == 0 && tensor_scale != nullptr) tensor_scale[row] = ts;
+  if (lane == 0 && tensor_scale != nullptr) tensor_scale[row] = ts;
 
   if (normalized != nullptr) {
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
       const int ch = it * 32 + lane;
-      if (((it >> 1) & share_mask) == share && ch < chunks) {
+      if (ch < chunks) {
         float* dst = normalized + row_base + static_cast<size_t>(ch) * 8;
         *reinterpret_cast<float4*>(dst) = make_float4(v[it][0], v[it][1], v[it][2], v[it][3]);
         *reinterpret_cast<float4*>(dst + 4) = make_float4(v[it][4], v[it][5], v[it][6], v[it][7]);
@@ -329,9 +322,6 @@ norm_quant_row_kernel(const void* in, int rows, int cols,
   const bool odd = (lane & 1) != 0;
 #pragma unroll
   for (int it = 0; it < ITERS; it += 2) {
-    if constexpr (SHARED) {
-      if (((it >> 1) & share_mask) != share) continue;
-    }
     const float first_max = fmaxf(half_max[it], __shfl_xor_sync(0xffffffffu, half_max[it], 1));
     const float second_max =
         fmaxf(half_max[it + 1], __shfl_xor_sync(0xffffffffu, half_max[it + 1], 1));
@@ -380,6 +370,152 @@ norm_quant_row_kernel(const void* in, int rows, int cols,
           sf_tiled[swizzled_scale_offset(row, block, k_tiles)] = static_cast<uint8_t>(sf);
         }
       }
+    }
+  }
+}
+
+// The same for few rows, a block per row.  Thread c owns the 8-element chunks c, c + 256, ...: it
+// loads them at once, and hands the values over through shared memory for the sum of squares, in
+// which thread t adds up columns t, t + 256, ... in order.
+//
+// Bound by latency, and by fetching its own instructions: the row kernel unrolls ITERS steps of
+// codes, which made one row of 4096 take @N1@ us alone with cold caches (this one @N2@) and one of
+// 2688 7.1 (@N3@).
+template <bool BF16, int CHUNKS>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+norm_quant_block_kernel(const void* in, int cols, const float* __restrict__ norm_weight, float eps,
+                        float* __restrict__ normalized, uint8_t* __restrict__ packed,
+                        uint8_t* __restrict__ sf_row_major, uint8_t* __restrict__ sf_tiled,
+                        int k_tiles, float* __restrict__ tensor_scale,
+                        float* __restrict__ inv_rms_out, bool word_scales,
+                        int32_t* __restrict__ zero, int zero_count) {
+  constexpr int kThreads = kWarpsPerBlock * 32;
+  __shared__ float4 row_values[CHUNKS * kThreads * 2];
+  __shared__ float partial_sums[kThreads];
+  __shared__ float warp_max[kWarpsPerBlock];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row = blockIdx.x;
+  const int chunks = cols / 8;
+  const size_t row_base = static_cast<size_t>(row) * cols;
+  release_successor();
+  float w[CHUNKS][8];
+  if (norm_weight != nullptr) {
+#pragma unroll
+    for (int j = 0; j < CHUNKS; ++j) {
+      if (j * kThreads + tid < chunks) load8<false>(norm_weight, (j * kThreads + tid) * 8, w[j]);
+    }
+  }
+  wait_for_predecessor();
+  zero_words(zero, zero_count);
+
+  float v[CHUNKS][8];
+#pragma unroll
+  for (int j = 0; j < CHUNKS; ++j) {
+    const int ch = j * kThreads + tid;
+    if (ch < chunks) {
+      load8<BF16>(in, row_base + static_cast<size_t>(ch) * 8, v[j]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[j][i] = 0.0f;
+    }
+  }
+
+  if (norm_weight != nullptr) {
+    // the association of norm_quant_kernel
+#pragma unroll
+    for (int j = 0; j < CHUNKS; ++j) {
+      row_values[(j * kThreads + tid) * 2] = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+      row_values[(j * kThreads + tid) * 2 + 1] = make_float4(v[j][4], v[j][5], v[j][6], v[j][7]);
+    }
+    __syncthreads();
+    const float* values = reinterpret_cast<const float*>(row_values);
+    float partial = 0.0f;
+#pragma unroll 8
+    for (int it = 0; it < CHUNKS * 8; ++it) {
+      const float x = values[it * 256 + tid];
+      partial = __fmaf_rn(x, x, partial);
+    }
+    partial_sums[tid] = partial;
+    __syncthreads();
+    // strides 128, 64 and 32 of the halving tree, by every warp; then inside the warp
+    const float* p = partial_sums + lane;
+    const float a = __fadd_rn(__fadd_rn(p[0], p[128]), __fadd_rn(p[64], p[192]));
+    const float b = __fadd_rn(__fadd_rn(p[32], p[160]), __fadd_rn(p[96], p[224]));
+    float sum = __fadd_rn(a, b);
+#pragma unroll
+    for (int stride = 16; stride > 0; stride >>= 1) {
+      sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, stride));
+    }
+    sum = __shfl_sync(0xffffffffu, sum, 0);
+    const float mean = __fdiv_rn(sum, static_cast<float>(cols));
+    const float inv_rms = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+    if (tid == 0 && inv_rms_out != nullptr) inv_rms_out[row] = inv_rms;
+#pragma unroll
+    for (int j = 0; j < CHUNKS; ++j) {
+      if (j * kThreads + tid < chunks) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[j][i] = __fmul_rn(__fmul_rn(v[j][i], inv_rms), w[j][i]);
+      }
+    }
+  }
+
+  float half_max[CHUNKS];  // of this thread's half blocks
+  float amax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < CHUNKS; ++j) {
+    half_max[j] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) half_max[j] = fmaxf(half_max[j], fabsf(v[j][i]));
+    amax = fmaxf(amax, half_max[j]);
+  }
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1) {
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, stride));
+  }
+  if (lane == 0) warp_max[warp] = amax;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kWarpsPerBlock; ++i) amax = fmaxf(amax, warp_max[i]);
+  const float ts = tensor_scale_from_amax(amax);
+  if (tid == 0 && tensor_scale != nullptr) tensor_scale[row] = ts;
+
+  const int blocks_per_row = cols / 16;
+  const float scale_divisor = __fmul_rn(kFp4Max, ts);
+  const float scale_reciprocal = __frcp_rn(scale_divisor);
+#pragma unroll
+  for (int j = 0; j < CHUNKS; ++j) {
+    const int ch = j * kThreads + tid;
+    if (normalized != nullptr && ch < chunks) {
+      float* dst = normalized + row_base + static_cast<size_t>(ch) * 8;
+      *reinterpret_cast<float4*>(dst) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(v[j][4], v[j][5], v[j][6], v[j][7]);
+    }
+    if (packed == nullptr) continue;
+    // lanes 2i and 2i + 1 hold the two halves of a 16-element block
+    const float block_max = fmaxf(half_max[j], __shfl_xor_sync(0xffffffffu, half_max[j], 1));
+    const float bs = block_scale(block_max, scale_divisor, scale_reciprocal);
+    const float divisor = __fmul_rn(ts, bs);
+    const uint32_t word = quantize_half_block(v[j], divisor, __frcp_rn(divisor));
+    const uint32_t sf = encode_e4m3(bs);
+    // four consecutive blocks (eight lanes) are one aligned word in both layouts
+    uint32_t sf_word = sf | (__shfl_down_sync(0xffffffffu, sf, 2) << 8);
+    sf_word |= __shfl_down_sync(0xffffffffu, sf_word, 4) << 16;
+    if (ch >= chunks) continue;
+    *reinterpret_cast<uint32_t*>(packed + row_base / 2 + static_cast<size_t>(ch) * 4) = word;
+    const int block = ch >> 1;
+    uint8_t* row_major =
+        sf_row_major != nullptr ? sf_row_major + static_cast<size_t>(row) * blocks_per_row + block
+                                : nullptr;
+    uint8_t* tiled =
+        sf_tiled != nullptr ? sf_tiled + swizzled_scale_offset(row, block, k_tiles) : nullptr;
+    if (word_scales) {
+      if ((lane & 7) == 0) {
+        if (row_major != nullptr) *reinterpret_cast<uint32_t*>(row_major) = sf_word;
+        if (tiled != nullptr) *reinterpret_cast<uint32_t*>(tiled) = sf_word;
+      }
+    } else if ((lane & 1) == 0) {
+      if (row_major != nullptr) *row_major = static_cast<uint8_t>(sf);
+      if (tiled != nullptr) *tiled = static_cast<uint8_t>(sf);
     }
   }
 }
@@ -440,55 +576,49 @@ int grid_for(size_t work, int threads) {
 
 namespace {
 
-template <bool BF16, int ITERS>
-void launch_row_kernel(int rows, LaunchStream stream, const void* in, int cols,
-                       const float* norm_weight, float eps, float* normalized, uint8_t* packed,
-                       uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles, float* tensor_scale,
-                       float* inv_rms, int32_t* zero, int zero_count) {
-  // A row costs one warp about 2 us of latency, half of it in the quantiser: with few rows
-  // eight warps share that half (each still reads the whole row, from L1), with more rows
-  // than the GPU has warp slots one warp does it all.
-  int shift = 0;
-  while (shift < 3 && (rows << shift) <= 148 * 4) ++shift;
-  const int grid = ((rows << shift) + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  const bool word_scales =
-      cols % 64 == 0 && ((reinterpret_cast<uintptr_t>(sf_row_major) |
-                          reinterpret_cast<uintptr_t>(sf_tiled)) & 3u) == 0;
-  auto run = [&](auto kernel) {
-    launch_kernel(kernel, grid, kWarpsPerBlock * 32, 0, stream,
-        in, rows, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
-        tensor_scale, inv_rms, shift, word_scales, zero, zero_count);
-  };
-  if (shift > 0) {
-    run(norm_quant_row_kernel<BF16, ITERS, true>);
-  } else {
-    run(norm_quant_row_kernel<BF16, ITERS, false>);
-  }
-}
+// Rows up to which each gets a block: as many as are resident at once.
+constexpr int kBlockRows = 148 * 4;
 
 template <bool BF16>
 void launch_norm_quant_t(int rows, LaunchStream stream, const void* in, int cols,
                          const float* norm_weight, float eps, float* normalized, uint8_t* packed,
                          uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles,
                          float* tensor_scale, float* inv_rms, int32_t* zero, int zero_count) {
-  auto run = [&](auto launcher) {
-    launcher(rows, stream, in, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled,
-             k_tiles, tensor_scale, inv_rms, zero, zero_count);
+  const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  const bool word_scales =
+      cols % 64 == 0 && ((reinterpret_cast<uintptr_t>(sf_row_major) |
+                          reinterpret_cast<uintptr_t>(sf_tiled)) & 3u) == 0;
+  auto run_block = [&](auto kernel) {
+    launch_kernel(kernel, rows, kWarpsPerBlock * 32, 0, stream, in, cols, norm_weight, eps,
+                  normalized, packed, sf_row_major, sf_tiled, k_tiles, tensor_scale, inv_rms,
+                  word_scales, zero, zero_count);
   };
-  // the row lives in registers (8 floats per lane and iteration); longer rows are read three times
-  if (cols <= 4 * 256) {
-    run(launch_row_kernel<BF16, 4>);
+  auto run_row = [&](auto kernel) {
+    launch_kernel(kernel, grid, kWarpsPerBlock * 32, 0, stream, in, rows, cols, norm_weight, eps,
+                  normalized, packed, sf_row_major, sf_tiled, k_tiles, tensor_scale, inv_rms,
+                  word_scales, zero, zero_count);
+  };
+  if (rows <= kBlockRows && cols <= 6144) {
+    if (cols <= 2048) {
+      run_block(norm_quant_block_kernel<BF16, 1>);
+    } else if (cols <= 4096) {
+      run_block(norm_quant_block_kernel<BF16, 2>);
+    } else {
+      run_block(norm_quant_block_kernel<BF16, 3>);
+    }
+  } else if (cols <= 4 * 256) {
+    // the row lives in registers (8 floats per lane and iteration); longer rows are read three times
+    run_row(norm_quant_row_kernel<BF16, 4>);
   } else if (cols <= 11 * 256) {
-    run(launch_row_kernel<BF16, 11>);
+    run_row(norm_quant_row_kernel<BF16, 11>);
   } else if (cols <= 16 * 256) {
-    run(launch_row_kernel<BF16, 16>);
+    run_row(norm_quant_row_kernel<BF16, 16>);
   } else if (cols <= 21 * 256) {
-    run(launch_row_kernel<BF16, 21>);
+    run_row(norm_quant_row_kernel<BF16, 21>);
   } else {
-    const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    launch_kernel(norm_quant_kernel<BF16, true>, grid, kWarpsPerBlock * 32, 0, stream,
-        in, rows, cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
-        tensor_scale, nullptr, inv_rms, zero, zero_count);
+    launch_kernel(norm_quant_kernel<BF16, true>, grid, kWarpsPerBlock * 32, 0, stream, in, rows,
+                  cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,
+                  tensor_scale, nullptr, inv_rms, zero, zero_count);
   }
 }
 
