@@ -53,10 +53,12 @@ __global__ void relu2_kernel(float* __restrict__ values, size_t count) {
 }
 
 // out[t] = ((0 + parts[t][0]) + parts[t][1]) + ... : routed_row of expert_layer.cpp:951-953
+// Bound by its loads: with one in flight per thread 22 parts of one token took 6.2 us.
 __global__ void sum_parts_kernel(const float* parts, int rows, int cols, int top_k,
                                  float* __restrict__ out) {
   release_successor();
   wait_for_predecessor();
+  constexpr int kBatch = 7;  // parts whose loads are in flight together
   const int quads = cols / 4;
   const size_t total = static_cast<size_t>(rows) * quads;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -65,12 +67,23 @@ __global__ void sum_parts_kernel(const float* parts, int rows, int cols, int top
     const int c = static_cast<int>(i - t * quads) * 4;
     const float* base = parts + t * top_k * cols + c;
     float4 acc = *reinterpret_cast<const float4*>(base);
-    for (int k = 1; k < top_k; ++k) {
-      const float4 p = *reinterpret_cast<const float4*>(base + static_cast<size_t>(k) * cols);
-      acc.x = __fadd_rn(acc.x, p.x);
-      acc.y = __fadd_rn(acc.y, p.y);
-      acc.z = __fadd_rn(acc.z, p.z);
-      acc.w = __fadd_rn(acc.w, p.w);
+    for (int k0 = 1; k0 < top_k; k0 += kBatch) {
+      float4 p[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (k0 + k < top_k) {
+          p[k] = *reinterpret_cast<const float4*>(base + static_cast<size_t>(k0 + k) * cols);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (k0 + k < top_k) {
+          acc.x = __fadd_rn(acc.x, p[k].x);
+          acc.y = __fadd_rn(acc.y, p[k].y);
+          acc.z = __fadd_rn(acc.z, p[k].z);
+          acc.w = __fadd_rn(acc.w, p[k].w);
+        }
+      }
     }
     *reinterpret_cast<float4*>(out + t * cols + c) = acc;
   }

@@ -121,17 +121,17 @@ place_rows_kernel(PlanBuffers plan, PermuteSource src, int pairs, int share, int
   __shared__ int tiles_of[kMaxPlanExperts];
   release_successor();
   wait_for_predecessor();
+  const int lane = threadIdx.x & 31;
+  const int units = pairs / src.pairs_per_row * share;
+  const int warps = gridDim.x * (kPlaceThreads / 32);
+  const int row_bytes = cols / 2, blocks = cols / 16;
+  const int first_unit = blockIdx.x * (kPlaceThreads / 32) + (threadIdx.x >> 5);
   const int total = scan_expert_tiles<kPlaceThreads>(plan.expert_counts, experts, tile_multiple,
                                                      first_tile, tiles_of);
   if (blockIdx.x == 0) {
     write_row_tiles<kPlaceThreads>(plan, experts, max_row_tiles, total, first_tile, tiles_of, error);
   }
-  const int lane = threadIdx.x & 31;
-  const int units = pairs / src.pairs_per_row * share;
-  const int warps = gridDim.x * (kPlaceThreads / 32);
-  const int row_bytes = cols / 2, blocks = cols / 16;
-  for (int unit = blockIdx.x * (kPlaceThreads / 32) + (threadIdx.x >> 5); unit < units;
-       unit += warps) {
+  for (int unit = first_unit; unit < units; unit += warps) {
     const int source_row = unit / share, part = unit - source_row * share;
     // Lane l looks up the l-th of this warp's pairs: its row in the sorted buffers, or -1.
     int row = -1;

@@ -99,12 +99,8 @@ router_logits_kernel(const float* __restrict__ y, const float* __restrict__ gate
 // here exp runs in double and is rounded once, which equals the correctly
 // rounded single-precision exponential.
 __device__ __forceinline__ float sigmoid_ref(float v) {
-  if (v >= 0.0f) {
-    const float e = static_cast<float>(exp(-static_cast<double>(v)));
-    return __fdiv_rn(1.0f, __fadd_rn(1.0f, e));
-  }
-  const float e = static_cast<float>(exp(static_cast<double>(v)));
-  return __fdiv_rn(e, __fadd_rn(1.0f, e));
+  const float e = static_cast<float>(exp(-fabs(static_cast<double>(v))));
+  return __fdiv_rn(v >= 0.0f ? 1.0f : e, __fadd_rn(1.0f, e));
 }
 
 // Order-preserving map of a float onto unsigned integers; 0 is left for "taken or absent".
@@ -115,16 +111,15 @@ __device__ __forceinline__ uint32_t choice_key(float v) {
 }
 
 constexpr int kMaxExperts = 512;
-constexpr int kTopkThreads = 128;
 
 // One block per token.  All threads evaluate sigmoids (the exponential in double is the
-// longest single step), one warp selects: expert e lives in lane e % 32, slot e / 32, every
+// longest single step; one for each expert while blocks are few, else 128), one warp selects: expert e lives in lane e % 32, slot e / 32, every
 // lane keeps the best of its remaining slots, and a round is one warp-wide maximum of
 // order-preserving keys, one minimum over the indices that hold it (ties go to the lower
 // expert) and a rescan by the lane that owned it.  Bound by the latency of that chain
-// (between events): 1 token, 128 experts, top-6 14.9 -> 8.4 us; 512 experts, top-22 33 -> 14.3.
+// (between events): 1 token, 128 experts, top-6 14.9 -> 8.2 us; 512 experts, top-22 33 -> 12.2.
 template <int PER_LANE>
-__global__ void __launch_bounds__(kTopkThreads)
+__global__ void __launch_bounds__(PER_LANE * 32 < 128 ? 128 : PER_LANE * 32)
 router_topk_kernel(const float* logits, const float* __restrict__ bias, int experts,
                    int top_k, int n_group, int topk_group, bool norm_topk_prob,
                    float routed_scaling, int32_t* __restrict__ top_index,
@@ -136,7 +131,7 @@ router_topk_kernel(const float* logits, const float* __restrict__ bias, int expe
   const int row = blockIdx.x;
   release_successor();
   wait_for_predecessor();
-  for (int e = threadIdx.x; e < experts; e += kTopkThreads) {
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
     const float score = sigmoid_ref(logits[static_cast<size_t>(row) * experts + e]);
     score_smem[e] = score;
     choice_smem[e] = __fadd_rn(score, bias[e]);
@@ -272,17 +267,18 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int rows,
   if (!router_topk_arguments_valid(rows, experts, top_k, n_group, topk_group)) {
     return cudaErrorInvalidValue;
   }
-  auto run = [&](auto kernel) {
-    launch_kernel(kernel, rows, kTopkThreads, 0, stream, logits, bias, experts, top_k, n_group, topk_group,
+  auto run = [&](auto kernel, int per_expert) {
+    const int threads = rows <= 148 ? per_expert : 128;
+    launch_kernel(kernel, rows, threads, 0, stream, logits, bias, experts, top_k, n_group, topk_group,
                                               norm_topk_prob, routed_scaling, top_index, top_weight,
                                               expert_counts, position);
   };
   if (experts <= 128) {
-    run(router_topk_kernel<4>);
+    run(router_topk_kernel<4>, 4 * 32);
   } else if (experts <= 256) {
-    run(router_topk_kernel<8>);
+    run(router_topk_kernel<8>, 8 * 32);
   } else {
-    run(router_topk_kernel<kMaxExperts / 32>);
+    run(router_topk_kernel<kMaxExperts / 32>, kMaxExperts);
   }
   return cudaGetLastError();
 }
