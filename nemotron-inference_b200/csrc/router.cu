@@ -113,11 +113,11 @@ __device__ __forceinline__ uint32_t choice_key(float v) {
 constexpr int kMaxExperts = 512;
 
 // One block per token.  All threads evaluate sigmoids (the exponential in double is the
-// longest single step; one for each expert while blocks are few, else 128), one warp selects: expert e lives in lane e % 32, slot e / 32, every
-// lane keeps the best of its remaining slots, and a round is one warp-wide maximum of
-// order-preserving keys, one minimum over the indices that hold it (ties go to the lower
-// expert) and a rescan by the lane that owned it.  Bound by the latency of that chain
-// (between events): 1 token, 128 experts, top-6 14.9 -> 8.2 us; 512 experts, top-22 33 -> 12.2.
+// longest single step; one for each expert while blocks are few, else 128), one warp selects:
+// expert e lives in lane e % 32, slot e / 32, every lane keeps the best of its remaining slots,
+// and a round is one warp-wide maximum of order-preserving keys, one minimum over the indices that
+// hold it (ties go to the lower expert) and a rescan by the lane that owned it.  Bound by the
+// latency of that chain (between events): 1 token, 128 experts, top-6 14.9 -> 8.2 us; 512 experts, top-22 33 -> 12.2.
 template <int PER_LANE>
 __global__ void __launch_bounds__(PER_LANE * 32 < 128 ? 128 : PER_LANE * 32)
 router_topk_kernel(const float* logits, const float* __restrict__ bias, int experts,
