@@ -586,10 +586,10 @@ class ExpertFfn:
     def run(self, x: torch.Tensor, variant: int = 0) -> torch.Tensor:
         _require_cuda(x, "x")
         out = torch.empty((x.shape[0], self.hidden), dtype=torch.float32, device=x.device)
-        lib = load_library()
-        _check(lib.nmoe_ffn_run(self._handle, _stream(), x.data_ptr(), _dtype_code(x), x.shape[0],
+        lib, stream = load_library(), _stream()
+        _check(lib.nmoe_ffn_run(self._handle, stream, x.data_ptr(), _dtype_code(x), x.shape[0],
                                 out.data_ptr(), variant), "nmoe_ffn_run")
-        _check(lib.nmoe_ffn_sync_status(self._handle, _stream()), "nmoe_ffn_sync_status")
+        _check(lib.nmoe_ffn_sync_status(self._handle, stream), "nmoe_ffn_sync_status")
         return out
 
     def hidden_codes(self, rows: int):

@@ -541,9 +541,17 @@ nmoe_status status_from_device(int code) {
   }
 }
 
+// Hands the error word to the host and clears it: one launch in the place of a copy and a memset,
+// whose start-up a synchronous call over few rows waits for (64 rows through one expert, measured on
+// the host: 60.6 us with them, 50.7 so).
+__global__ void publish_error_kernel(int32_t* device, volatile int32_t* host) {
+  *host = atomicExch(device, 0);
+  __threadfence_system();
+}
+
 struct ErrorSlot {
   DeviceBuffer device;
-  int32_t* host = nullptr;  // pinned
+  int32_t* host = nullptr;  // pinned, written by publish_error_kernel
   void create() {
     device.allocate(sizeof(int32_t), true);
     NMOE_CUDA(cudaMallocHost(&host, sizeof(int32_t)));
@@ -553,11 +561,10 @@ struct ErrorSlot {
     if (host != nullptr) cudaFreeHost(host);
   }
   nmoe_status sync(cudaStream_t stream) {
-    NMOE_CUDA(cudaMemcpyAsync(host, device.as<int32_t>(), sizeof(int32_t), cudaMemcpyDeviceToHost,
-                              stream));
-    NMOE_CUDA(cudaMemsetAsync(device.as<int32_t>(), 0, sizeof(int32_t), stream));
+    publish_error_kernel<<<1, 1, 0, stream>>>(device.as<int32_t>(), host);
+    NMOE_CUDA(cudaGetLastError());
     NMOE_CUDA(cudaStreamSynchronize(stream));
-    return status_from_device(*host);
+    return status_from_device(*static_cast<volatile int32_t*>(host));
   }
 };
 
