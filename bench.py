@@ -463,9 +463,9 @@ def main():
                        "steps overlap the compute (2 device buffers per direction); working set "
                        "per step (718 MB weights + 88 MB in + 88 MB out) exceeds L2",
                 "one_batch_at_a_time_ms_per_step": serial_ms},
-        "gpu_launches": 10 * args.steps,
+        "gpu_launches": 9 * args.steps,
         "clocks": clocks,
-        "roofline": {"kernel": "grouped_gemm_kernel<BN=208, up: relu^2 + NVFP4 quantise epilogue>",
+        "roofline": {"kernel": "grouped_gemm_pair_kernel<up: 256 x 208 tiles, relu^2 + NVFP4 quantise epilogue>",
                      "bound": "tensor", "achieved": up_tf, "peak": fp4_peak, "unit": "TFLOP/s",
                      "frac": up_tf / fp4_peak, "traffic": up_traffic,
                      "traffic_note": traffic_note,

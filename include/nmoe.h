@@ -400,9 +400,8 @@ NMOE_API nmoe_status nmoe_ffn_create(const nmoe_nvfp4_matrix* up, const nmoe_nvf
                                      int32_t max_rows, nmoe_ffn** out_ffn);
 NMOE_API void nmoe_ffn_destroy(nmoe_ffn* ffn);
 /* input [rows][hidden] device FP32/bf16 -> output [rows][hidden] device FP32.
- * gemm_variant: 0 = choose by size, otherwise 1 + a tile-shape class (for tests):
- * 1 prefill tiles, 2 decode tiles (rows <= 32), 3 wide decode tiles, 4 prefill tiles
- * over CTA pairs. */
+ * gemm_variant: 0 = choose by size, otherwise the kernel (for tests): 1 or 4 the CTA-pair GEMM
+ * of large batches, 2 (rows <= 32) or 3 the streaming kernel of small ones. */
 NMOE_API nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream, const void* input,
                                   nmoe_dtype input_dtype, int64_t rows, float* output,
                                   int32_t gemm_variant);

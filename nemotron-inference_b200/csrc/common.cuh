@@ -265,30 +265,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return true;
 }
 
-// The same bounded wait polling with test_wait, which returns at once instead of
-// suspending the thread for a hardware-chosen time: lower wake-up latency for the waits
-// on a kernel's critical path, at the price of a hot spin.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity) {
-  if (mbar_test_wait(bar, parity)) return true;
-  const long long start = clock64();
-  while (!mbar_test_wait(bar, parity)) {
-    if (clock64() - start > (1ll << 31)) return false;
-  }
-  return true;
-}
-
 // The same operations by shared-memory address, for loops whose every instruction counts: a role
 // of one thread runs a K block's bookkeeping as one dependent chain.
 __device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
@@ -309,10 +285,6 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
     if (clock64() - start > (1ll << 31)) return false;
   }
   return true;
-}
-
-__device__ __forceinline__ bool mbar_wait_at(uint32_t bar, uint32_t parity) {
-  return mbar_try_wait_at(bar, parity) || mbar_wait_slow(bar, parity);
 }
 
 // A role that issues tensor-core or copy instructions runs them from ONE lane, but the loop around
@@ -381,15 +353,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// 1-D bulk copy global -> shared (16-byte aligned addresses and size).
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes,
-                                          uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
 
@@ -509,22 +472,6 @@ __device__ __forceinline__ void tmem_ld_x16_async(uint32_t taddr, uint32_t (&r)[
       : "memory");
 }
 
-// 32 lanes x 16 consecutive 32-bit columns from registers: thread i writes row (lane
-// base + i).  Complete after tmem_st_wait().
-__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-        "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-
-__device__ __forceinline__ void tmem_st_wait() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -535,8 +482,6 @@ __device__ __forceinline__ void tmem_ld_fence(uint32_t (&r)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i]));
 }
-
-__device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 // --- CTA pairs (cta_group::2) -------------------------------------------------
 // Two CTAs of a cluster of size 2 drive one tcgen05.mma with M = 256: each CTA
@@ -555,52 +500,6 @@ __device__ __forceinline__ void cluster_sync_all() {
                "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Arrive on the mbarrier at the same shared-memory offset in CTA `target_rank`
-// of this cluster.
-__device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t target_rank) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-               : "=r"(remote)
-               : "r"(smem_u32(bar)), "r"(target_rank));
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote)
-               : "memory");
-}
-
-// try_wait that acquires at cluster scope: pairs with mbar_arrive_remote.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long start = clock64();
-  while (!mbar_try_wait_cluster(bar, parity)) {
-    if (clock64() - start > (1ll << 31)) return false;
-  }
-  return true;
-}
-
-// 2-D tiled TMA load into this CTA's shared memory whose completion bytes are counted
-// on the mbarrier `leader_bar`, a shared::cluster address that may lie in the partner
-// CTA of the pair (cluster_address_of): both CTAs' loads of a stage complete on the
-// leader's barrier.  No multicast.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int x,
-                                                 int y, uint32_t leader_bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
-      : "memory");
-}
-
 __device__ __forceinline__ void tma_load_2d_pair_at(uint32_t smem_dst, const CUtensorMap* map, int x,
                                                     int y, uint32_t leader_bar) {
   asm volatile(
@@ -616,30 +515,6 @@ __device__ __forceinline__ void tma_load_2d_pair_at(uint32_t smem_dst, const CUt
 // (.release.cluster) made every arrival wait about 1100 cycles.
 __device__ __forceinline__ void mbar_arrive_cluster_at(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait_cluster_at(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-static __device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parity) {
-  const long long start = clock64();
-  while (!mbar_try_wait_cluster_at(bar, parity)) {
-    if (clock64() - start > (1ll << 31)) return false;
-  }
-  return true;
-}
-
-__device__ __forceinline__ bool mbar_wait_cluster_at(uint32_t bar, uint32_t parity) {
-  return mbar_try_wait_cluster_at(bar, parity) || mbar_wait_cluster_slow(bar, parity);
 }
 
 // The shared::cluster address of `local` (an address in this CTA's shared memory) in

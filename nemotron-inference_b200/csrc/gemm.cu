@@ -78,7 +78,8 @@ __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, i
 // complete on rank 0's full barrier, so nothing is handed over inside a K block.  No multicast:
 // the loads of the partner name the leader's barrier.
 //
-// Measured, benchmark layer, up / down projection: 16384 tokens @P1@, 8192 tokens @P2@.
+// Measured, benchmark layer, up / down projection, against 128 x 208 tiles of single CTAs: 16384
+// tokens 334 / 405 -> 258 / 300 us, 8192 tokens 192 / 223 -> 152 / 170.
 // ---------------------------------------------------------------------------
 constexpr int kPairBN = 208;
 constexpr int kPairBRows = kPairBN / 2;        // weight rows staged per CTA
