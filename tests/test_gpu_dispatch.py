@@ -1,0 +1,74 @@
+"""The sizes at which a different kernel, or a different split of one, takes over: results on both
+sides of each line against the CPU oracle, and layers that run beside each other on two streams."""
+import numpy as np
+import pytest
+import torch
+
+import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def small_layer(package, synthetic):
+    cfg = synthetic.baseline_config(max_tokens=2048, experts=32, hidden=512, routed=256, shared=512)
+    data = synthetic.make_layer(cfg, seed=41, device="cuda", norm_weight_uniform=True)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None and layer.valid(), package.ExpertLayerSlice.create_error
+    yield layer, data
+    layer.close()
+
+
+# 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; a warp per pair
+# up to 2368 pairs (394 tokens); CTA pairs from 100 rows per expert (534 tokens); the shared expert in
+# the routed experts' launch up to 640; a block per row in the quantiser up to 1184
+@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 1184, 1185])
+def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
+    layer, data = small_layer
+    x = synthetic.make_tokens(tokens, 512, seed=300 + tokens, device="cuda")
+    out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+    assert layer.run(x, out), layer.last_error
+    rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+    assert rep.ok(), rep.summary()
+
+
+@pytest.mark.parametrize("rows", [3, 1185])
+@pytest.mark.parametrize("cols", [16, 1008, 2048, 2064, 4096, 4112, 5376, 6144, 6160])
+def test_quantiser_row_lengths(package, oracle, rows, cols):
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows + cols)) * 3.0
+    packed, scales, ts, _ = package.quantize_nvfp4(x.cuda(), per_row=True, swizzled=True)
+    w = torch.linspace(0.9, 1.1, cols)
+    y = package.rmsnorm(x.cuda(), w.cuda(), 1e-5)
+    torch.cuda.synchronize()
+    for got, expected in zip((packed, scales, ts), oracle.pack_nvfp4_per_row(x.numpy())):
+        assert np.array_equal(got.cpu().numpy(), expected)
+    assert np.array_equal(y.cpu().numpy(), oracle.rmsnorm(x.numpy(), w.numpy(), 1e-5))
+
+
+def test_two_layers_beside_each_other(package, synthetic):
+    # chained launches and kernels whose tiles wait for one another, on two streams at once
+    cfg = synthetic.baseline_config(max_tokens=512, experts=32, hidden=512, routed=256, shared=512)
+    layers = []
+    for seed in (51, 52):
+        data = synthetic.make_layer(cfg, seed=seed, device="cuda")
+        layers.append(package.ExpertLayerSlice.create(cfg, data.bindings))
+    for tokens in (1, 40, 200, 500):
+        xs = [synthetic.make_tokens(tokens, 512, seed=60 + i, device="cuda") for i in range(2)]
+        alone = []
+        for layer, x in zip(layers, xs):
+            out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+            assert layer.run(x, out), layer.last_error
+            alone.append(out)
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        outs = [torch.empty_like(a) for a in alone]
+        for _ in range(10):
+            for layer, x, out, stream in zip(layers, xs, outs, streams):
+                with torch.cuda.stream(stream):
+                    layer.run_async(x, out)
+        for layer, out, want, stream in zip(layers, outs, alone, streams):
+            with torch.cuda.stream(stream):
+                assert layer.sync_status() == 0
+            assert torch.equal(out, want)
+    for layer in layers:
+        layer.close()
