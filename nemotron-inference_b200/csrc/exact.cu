@@ -702,6 +702,105 @@ exact_gemv_block_kernel(const float* in, float fp8_scale, int rows, int N, int K
   }
 }
 
+// Four values of W, from element i (a multiple of four).
+template <int KIND>
+__device__ __forceinline__ void weight_quad(const void* w, size_t i, float scale, float (&v)[4]) {
+  if constexpr (KIND == kWeightFp8) {
+    const uint32_t raw = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(w) + i);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const __half2_raw two = __nv_cvt_fp8x2_to_halfraw2(
+          static_cast<__nv_fp8x2_storage_t>(raw >> (16 * h)), __NV_E4M3);
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+      v[2 * h] = __fmul_rn(f.x, scale);
+      v[2 * h + 1] = __fmul_rn(f.y, scale);
+    }
+  } else if constexpr (KIND == kWeightBf16) {
+    const uint2 raw =
+        *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(w) + i);
+    v[0] = __uint_as_float(raw.x << 16);
+    v[1] = __uint_as_float(raw.x & 0xffff0000u);
+    v[2] = __uint_as_float(raw.y << 16);
+    v[3] = __uint_as_float(raw.y & 0xffff0000u);
+  } else {
+    const float4 raw = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w) + i);
+    v[0] = raw.x; v[1] = raw.y; v[2] = raw.z; v[3] = raw.w;
+  }
+}
+
+// 8 x 8 outputs per block for a short W and more than a handful of rows: a value of either operand
+// is widened once for eight products, where exact_gemv_block_kernel widens five for four.  The
+// threads share K; each holds all 64 sums in registers.  Bound by the conversions (16 per 64 FMAs,
+// at 15 a clock and SM), the FP64 FMAs (52) and one round of loads per step: 256 threads while every
+// block has an SM, else 128, two blocks to an SM.  Between events, a gate of 128 x 2688: 64 rows
+// 20.2 -> 12.1 us; 128 rows 31 (by slices) -> 14.2 (18.3 with 256 threads), 255 rows 31 -> 24.4.
+constexpr int kTileOutputs = 8;
+template <int KIND, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+exact_tile_kernel(const float* in, float fp8_scale, int rows, int N, int K,
+                  const void* __restrict__ weight, float weight_scale,
+                  const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
+  constexpr int M = kTileOutputs;
+  __shared__ double warp_sum[THREADS / 32][M * M];
+  const int n0 = blockIdx.x * M, row0 = blockIdx.y * M;
+  const int lane = threadIdx.x & 31;
+  release_successor();
+  wait_for_predecessor();
+  double acc[M * M];
+#pragma unroll
+  for (int i = 0; i < M * M; ++i) acc[i] = 0.0;
+#pragma unroll 1
+  for (int k = static_cast<int>(threadIdx.x) * 4; k < K; k += THREADS * 4) {
+    float w[M][4], x[M][4];
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      weight_quad<KIND>(weight, static_cast<size_t>(min(n0 + i, N - 1)) * K + k, weight_scale, w[i]);
+      const float4 a = *reinterpret_cast<const float4*>(
+          in + static_cast<size_t>(min(row0 + i, rows - 1)) * K + k);
+      x[i][0] = a.x; x[i][1] = a.y; x[i][2] = a.z; x[i][3] = a.w;
+    }
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      double d[M];
+#pragma unroll
+      for (int i = 0; i < M; ++i) d[i] = static_cast<double>(w[i][h]);
+#pragma unroll
+      for (int r = 0; r < M; ++r) {
+        const double a = static_cast<double>(input_value(x[r][h], fp8_scale));
+#pragma unroll
+        for (int i = 0; i < M; ++i) acc[r * M + i] = fma(a, d[i], acc[r * M + i]);
+      }
+    }
+  }
+  // Across the lanes: each step adds up one half of the sums a lane still holds and hands the other
+  // half to its partner; two sums per lane are left.
+#pragma unroll
+  for (int step = 0; step < 5; ++step) {
+    const int half = M * M >> (step + 1), mask = 16 >> step;
+    const bool upper = (lane & mask) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double keep = upper ? acc[i + half] : acc[i];
+      const double give = upper ? acc[i] : acc[i + half];
+      acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, mask);
+    }
+  }
+  warp_sum[threadIdx.x >> 5][2 * lane] = acc[0];
+  warp_sum[threadIdx.x >> 5][2 * lane + 1] = acc[1];
+  __syncthreads();
+  const int o = threadIdx.x;
+  const int row = row0 + o / M, n = n0 + o % M;
+  if (o < M * M && row < rows && n < N) {
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) sum += warp_sum[w][o];
+    float result = static_cast<float>(sum);
+    if (offset != nullptr) result = __fadd_rn(result, offset[n]);
+    if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
+    out[static_cast<size_t>(row) * N + n] = result;
+  }
+}
+
 // A block per output where the tiled kernel (sixteen outputs a block) would leave SMs idle; a block
 // widens its token rows for itself, so with more than two of them less so (1 row, N 1024, K 4096 in
 // FP8: 11.7 us tiled, 8.2 by blocks).
@@ -728,6 +827,10 @@ cudaError_t launch_gemv_rows(const float* in, float fp8_scale, int N, int K, con
   return cudaGetLastError();
 }
 
+// Rows up to which a block per output is faster than a block per 8 x 8 outputs (128 x 2688: 7 rows
+// 8.1 us against 12.1 for up to 64 rows, 32 rows 14.2).
+constexpr int kGemvBlockRows = 16;
+
 template <int KIND>
 cudaError_t launch_gemv_kind(const float* in, float fp8_scale, int rows, int N, int K,
                              const void* weight, float weight_scale, const float* offset,
@@ -737,7 +840,14 @@ cudaError_t launch_gemv_kind(const float* in, float fp8_scale, int rows, int N, 
       launch_kernel(kernel, dim3(N, (rows + per_block - 1) / per_block), kGemvThreads, 0, stream,
           in, fp8_scale, rows, N, K, weight, weight_scale, offset, relu2, out);
     };
-    if (rows == 1) {
+    if (rows > kGemvBlockRows) {
+      const dim3 grid((N + kTileOutputs - 1) / kTileOutputs,
+                      (rows + kTileOutputs - 1) / kTileOutputs);
+      const bool alone = static_cast<int>(grid.x * grid.y) <= num_sms;
+      launch_kernel(alone ? exact_tile_kernel<KIND, 256> : exact_tile_kernel<KIND, 128>, grid,
+                    alone ? 256 : 128, 0, stream, in, fp8_scale, rows, N, K, weight, weight_scale,
+                    offset, relu2, out);
+    } else if (rows == 1) {
       run(exact_gemv_block_kernel<KIND, 1>, 1);
     } else if (rows == 2) {
       run(exact_gemv_block_kernel<KIND, 2>, 2);
@@ -849,12 +959,13 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
 
 // FP64 over the operands as they are, or integers over their slices?  The first reads W in its own
 // format, which counts for few rows: up to four are no slower on a large W (22 MB of FP8 against
-// 110 MB of slices for the checkpoint's shared_up).  A short W costs no more than widening its
-// values (15 a clock and SM), which up to 36 million products is less than the three launches of
-// the second take (64 rows of a 128 x 2688 gate: 20 us against 31 between events).
+// 110 MB of slices for the checkpoint's shared_up).  A short W costs no more than widening and
+// multiplying its values, which up to 90 million products is less than the three launches of the
+// second take (255 rows of a 128 x 2688 gate: 24 us against 31 between events, 40 rows of a
+// 512 x 4096 gate 27 either way).
 bool exact_prefers_gemv(int rows, int N, int K, int num_sms) {
   if (rows <= 4) return true;
-  return gemv_by_blocks(rows, N, num_sms) && static_cast<long long>(rows) * N * K <= 36000000ll;
+  return gemv_by_blocks(rows, N, num_sms) && static_cast<long long>(rows) * N * K <= 90000000ll;
 }
 
 cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,
