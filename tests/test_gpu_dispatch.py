@@ -72,3 +72,24 @@ def test_two_layers_beside_each_other(package, synthetic):
             assert torch.equal(out, want)
     for layer in layers:
         layer.close()
+
+
+@pytest.mark.parametrize("family", ["bf16", "fp8", "fp32"])
+def test_integer_linears_at_the_edges_of_their_tiles(package, synthetic, family):
+    # shared_up with 704 outputs (five and a half tiles of weight rows): too many for the FP64 kernels
+    cfg = synthetic.baseline_config(max_tokens=160, experts=64, hidden=320, routed=64, shared=704,
+                                    latent=192)
+    data = synthetic.make_layer(cfg, seed=92, device="cuda", latent_family=family,
+                                shared_up_family=family, shared_down_family=family)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (5, 16, 17, 48, 49, 64, 65, 160):
+        x = synthetic.make_tokens(tokens, 320, seed=tokens, device="cuda").to(torch.float32)
+        x[1] = 0.0
+        x[3, 1:] = 0.0
+        out = torch.empty_like(x)
+        assert layer.run(x, out), layer.last_error
+        rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+        assert rep.ok(), rep.summary()
+        assert rep.latent_max_diff == 0.0 and rep.logits_max_diff == 0.0
+    layer.close()
