@@ -728,7 +728,6 @@ struct ExactScratch {
 void run_exact(const ExactWeight& w, ExactScratch& scratch, const float* in, float fp8_scale,
                int rows, const float* offset, bool relu2, float* out, int32_t* error, int num_sms,
                LaunchStream stream) {
-  if (fp8_scale != 0.0f) fp8_scale = clamp_scale_host(fp8_scale);  // scaled_fp8_linear.cu:27-33
   if (exact_prefers_gemv(rows, w.N, w.K, num_sms)) {
     NMOE_CUDA(launch_exact_gemv(w, in, fp8_scale, rows, offset, relu2, out, num_sms, stream));
     return;
@@ -1280,8 +1279,10 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
 void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, int rows,
                 float* out_rows, bool relu2, LaunchStream stream) {
   if (linear.exact) {
-    run_exact(linear.operand.w, L->exact, in_rows, linear.fp8 ? linear.input_scale : 0.0f, rows,
-              nullptr, relu2, out_rows, L->error.device.as<int32_t>(), L->num_sms, stream);
+    // (clamped first, scaled_fp8_linear.cu:27-33: a scale of zero means no round trip further down)
+    const float fp8_scale = linear.fp8 ? clamp_scale_host(linear.input_scale) : 0.0f;
+    run_exact(linear.operand.w, L->exact, in_rows, fp8_scale, rows, nullptr, relu2, out_rows,
+              L->error.device.as<int32_t>(), L->num_sms, stream);
     return;
   }
   const float* source = in_rows;

@@ -39,3 +39,27 @@ def test_linears_round_the_fp64_sum(latent_layer, synthetic, tokens):
     print(rep.summary())
     assert rep.ok(), rep.summary()
     assert rep.latent_max_diff == 0.0 and rep.logits_max_diff == 0.0
+
+
+def test_an_fp8_input_scale_of_zero_is_the_smallest_scale(package, synthetic):
+    # the reference clamps the scale of the activations' round trip (scaled_fp8_linear.cu:27-33)
+    cfg = synthetic.baseline_config(max_tokens=64, experts=64, hidden=320, routed=64, shared=704,
+                                    latent=192)
+    outs = []
+    for scale in (0.0, 1.0 / 1024.0):
+        data = synthetic.make_layer(cfg, seed=93, device="cuda", latent_family="fp8",
+                                    shared_up_family="fp8", shared_down_family="fp8")
+        for linear in (data.bindings.fc1_latent, data.bindings.shared_up_linear,
+                       data.bindings.shared_down_linear):
+            linear.input_scale = scale
+        layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+        assert layer is not None, package.ExpertLayerSlice.create_error
+        for tokens in (2, 40):  # FP64 and integer kernels
+            x = synthetic.make_tokens(tokens, 320, seed=tokens, device="cuda").to(torch.float32)
+            out = torch.empty_like(x)
+            assert layer.run(x, out), layer.last_error
+            outs.append((out, layer.trace(tokens).latent_output))
+        layer.close()
+    for zero, smallest in zip(outs[:2], outs[2:]):
+        assert torch.equal(zero[1], smallest[1])
+        assert torch.equal(zero[0], smallest[0])
