@@ -814,7 +814,7 @@ cudaError_t launch_gemv_rows(const float* in, float fp8_scale, int N, int K, con
                              int num_sms, LaunchStream stream) {
   const int smem = ROWS * gemv_slot(K) * static_cast<int>(sizeof(double));
   auto kernel = exact_gemv_kernel<KIND, ROWS>;
-  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t err = allow_shared_memory(kernel);
   if (err != cudaSuccess) return err;
   // no more blocks than are resident together: each widens the token rows for itself
   const int resident = std::min(8, std::max(1, 220 * 1024 / (smem + 1024)));
@@ -929,8 +929,7 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
   const int smem = kExactStages * (kExactABytes + kSlices * nt * kExactChunk) +
                    (2 * kExactStages + 1) * 8 + 16 + 1024;
   auto multiply = [&](auto kernel) {
-    const cudaError_t attribute =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t attribute = allow_shared_memory(kernel);
     if (attribute != cudaSuccess) return attribute;
     kernel<<<grid, kExactThreads, smem, stream>>>(w.slices, space.slices, rows, w.N, w.K, row_tiles,
                                                   splits, space.partial, error);

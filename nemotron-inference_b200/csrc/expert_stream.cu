@@ -78,7 +78,8 @@ constexpr int stages_for(int tile_rows) { return tile_rows <= 32 ? 8 : tile_rows
 constexpr int smem_bytes(int tile_rows) {
   return stages_for(tile_rows) * stage_bytes(tile_rows) + kBarBytes + kFewRowsBytes + 1024;
 }
-static_assert(smem_bytes(32) <= 232448 && smem_bytes(64) <= 232448 && smem_bytes(128) <= 232448,
+static_assert(smem_bytes(32) <= kMaxSharedBytes && smem_bytes(64) <= kMaxSharedBytes &&
+                  smem_bytes(128) <= kMaxSharedBytes,
               "shared memory budget");
 // The MMA always reads 128 A rows: behind a stage of fewer rows it reads what follows (those output
 // rows are never stored), which must lie inside the allocation.
@@ -606,9 +607,7 @@ cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, LaunchStre
       (args.tile_rows != 32 && args.tile_rows != 64 && args.tile_rows != 128)) {
     return cudaErrorInvalidValue;
   }
-  cudaError_t err = cudaFuncSetAttribute(expert_stream_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem_bytes(args.tile_rows));
+  cudaError_t err = allow_shared_memory(expert_stream_kernel);
   if (err != cudaSuccess) return err;
   // one persistent CTA per SM, fewer when the tiles are known to be fewer
   int grid = num_sms;

@@ -103,7 +103,8 @@ constexpr int pair_smem_bytes(int mode) {
 static_assert(kPairSfCol + kPairSfBufs * kPairSfBufCols <= 512, "TMEM budget");
 static_assert(kPairBRows % 8 == 0, "half a weight tile is whole 8-row swizzle groups");
 static_assert(kPairBBytes % 1024 == 0, "stage regions keep the 1024-byte swizzle alignment");
-static_assert(pair_smem_bytes(kGemmUp) <= 232448 && pair_smem_bytes(kGemmDown) <= 232448,
+static_assert(pair_smem_bytes(kGemmUp) <= kMaxSharedBytes &&
+                  pair_smem_bytes(kGemmDown) <= kMaxSharedBytes,
               "shared memory budget");
 
 template <int MODE>
@@ -358,9 +359,7 @@ template <int MODE>
 cudaError_t launch_pair(const GemmMaps& maps, const GemmArgs& args, int num_sms,
                         cudaStream_t stream) {
   auto kernel = grouped_gemm_pair_kernel<MODE>;
-  cudaError_t err =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           pair_smem_bytes(MODE));
+  cudaError_t err = allow_shared_memory(kernel);
   if (err != cudaSuccess) return err;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(num_sms & ~1), 1, 1);

@@ -38,6 +38,17 @@ inline cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, int threa
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
+// Lets `kernel` (which has no static shared memory) be launched with all the dynamic shared memory a
+// block can have.  The limit belongs to the kernel and not to the launch, so it never follows the
+// launch's own size: a thread that lowered it between another thread's limit and launch made that
+// launch fail (two threads, row tiles of 32 and 128 rows: 10 of 40000).
+constexpr int kMaxSharedBytes = 227 * 1024;
+template <typename Kernel>
+inline cudaError_t allow_shared_memory(Kernel* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kMaxSharedBytes);
+}
+
 // A row tile is a 128-row aligned slot of the expert-sorted activation buffer
 // holding `rows` (<= 128) valid rows that all belong to `expert`.
 struct RowTile {

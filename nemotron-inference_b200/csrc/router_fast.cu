@@ -785,14 +785,12 @@ cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* i
   const int grid = (rows + 127) / 128 * splits;
   cudaError_t err;
   if (x_bf16) {
-    err = cudaFuncSetAttribute(router_fast_logits_kernel<true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    err = allow_shared_memory(router_fast_logits_kernel<true>);
     if (err != cudaSuccess) return err;
     launch_kernel(router_fast_logits_kernel<true>, grid, kFastThreads, smem, stream,
         x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
   } else {
-    err = cudaFuncSetAttribute(router_fast_logits_kernel<false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    err = allow_shared_memory(router_fast_logits_kernel<false>);
     if (err != cudaSuccess) return err;
     launch_kernel(router_fast_logits_kernel<false>, grid, kFastThreads, smem, stream,
         x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
@@ -828,8 +826,7 @@ cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtenso
   const int stages = std::min(4, (220 * 1024) / stage_bytes);
   if (stages < 2) return cudaErrorInvalidValue;
   const int smem = stages * stage_bytes + (2 * stages + 1) * 8 + 16 + 1024;
-  cudaError_t err = cudaFuncSetAttribute(router_folded_logits_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t err = allow_shared_memory(router_folded_logits_kernel);
   if (err != cudaSuccess) return err;
   launch_kernel(router_folded_logits_kernel, (rows + 127) / 128 * splits, kFoldThreads, smem, stream,
       tmap_x, tmap_planes, inv_rms, rows, experts, hidden, stages, splits, logits, error);

@@ -93,3 +93,37 @@ def test_integer_linears_at_the_edges_of_their_tiles(package, synthetic, family)
         assert rep.ok(), rep.summary()
         assert rep.latent_max_diff == 0.0 and rep.logits_max_diff == 0.0
     layer.close()
+
+
+def test_threads_launch_one_kernel_with_different_shared_memory(package, synthetic):
+    # row tiles of 32 and of 128 rows give the streaming kernel different stages; a thread must not
+    # meet the other's limit between setting its own and launching
+    import ctypes
+    import threading
+    lib, rows = package.load_library(), (8, 128)
+    networks, inputs, outputs, wanted = [], [], [], []
+    for i, count in enumerate(rows):
+        up, down = synthetic.make_ffn_weights(256, 128, seed=70 + i, device="cuda")
+        networks.append(package.ExpertFfn(up, down, max_rows=128))
+        inputs.append(synthetic.make_tokens(count, 256, seed=72, device="cuda"))
+        outputs.append(torch.zeros((count, 256), dtype=torch.float32, device="cuda"))
+        wanted.append(networks[i].run(inputs[i], 3))
+    torch.cuda.synchronize()
+    refused = [None, None]
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        call = (networks[i]._handle, ctypes.c_void_p(stream.cuda_stream), inputs[i].data_ptr(),
+                package.NMOE_BF16, rows[i], outputs[i].data_ptr(), 3)
+        refused[i] = sum(lib.nmoe_ffn_run(*call) != 0 for _ in range(40000))
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert refused == [0, 0]
+    for ffn, out, want in zip(networks, outputs, wanted):
+        assert torch.equal(out, want)
+        ffn.close()
