@@ -611,7 +611,8 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
       }
     }
   }
-  // candidates: everything that could still be in the exact top-k
+  // candidates: everything that could still be in the exact top-k (a score that is no number
+  // could be anywhere, so a row of them is re-evaluated as a whole and keeps them)
   float kth = 0.0f;
   {
     const uint32_t b = (kth_key & 0x80000000u) ? (kth_key & 0x7fffffffu) : ~kth_key;
@@ -621,7 +622,7 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
   uint32_t mine = 0;
 #pragma unroll
   for (int j = 0; j < kSelectPerLane; ++j) {
-    if (j < per_lane && choice[j] >= threshold) mine |= 1u << j;
+    if (j < per_lane && !(choice[j] < threshold)) mine |= 1u << j;
   }
   const int my_count = __popc(mine);
   int prefix = my_count;

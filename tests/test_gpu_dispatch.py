@@ -127,3 +127,24 @@ def test_threads_launch_one_kernel_with_different_shared_memory(package, synthet
     for ffn, out, want in zip(networks, outputs, wanted):
         assert torch.equal(out, want)
         ffn.close()
+
+
+@pytest.mark.parametrize("tokens", [40, 300, 1100])
+def test_a_row_that_is_not_a_number_stays_alone(small_layer, synthetic, tokens):
+    # its scores are no numbers, so nor are its weights and its output (the reference's arithmetic);
+    # no row of an earlier batch takes their place, and the other tokens do not change
+    layer, _ = small_layer
+    x = synthetic.make_tokens(tokens, 512, seed=500 + tokens, device="cuda")
+    clean = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+    assert layer.run(x, clean), layer.last_error
+    bad = x.clone()
+    bad[7, 100] = float("nan")
+    bad[30, 3] = float("inf")
+    out = torch.empty_like(clean)
+    assert layer.run(bad, out), layer.last_error
+    index = layer.trace(tokens).selected_index
+    assert int(index.min()) >= 0 and int(index.max()) < 32
+    assert torch.isnan(out[[7, 30]]).all()
+    others = [t for t in range(tokens) if t not in (7, 30)]
+    assert torch.equal(out[others], clean[others])
+
