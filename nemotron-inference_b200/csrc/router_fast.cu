@@ -31,13 +31,24 @@ namespace nmoe {
 namespace {
 
 // ---------------------------------------------------------------------------
-// pass 1: logits[128 tokens x E] per CTA
+// pass 1: logits[128 tokens x E] per CTA, up to 256 experts
 // ---------------------------------------------------------------------------
-constexpr int kFastStages = 3;
 constexpr int kFastBlockK = 64;                 // bf16 elements per 128-byte row
 constexpr int kFastABytes = 3 * 128 * 128;      // three planes of 128 rows x 128 B
 constexpr int kSplitWarps = 8;                  // warps that build the planes, then store
 constexpr int kFastThreads = (2 + kSplitWarps) * 32;
+
+// Dynamic shared memory: the stages, a full and an empty barrier for each, one more, the TMEM
+// address, and room to align.
+constexpr int pass1_smem_bytes(int stages, int stage_bytes) {
+  return stages * stage_bytes + (2 * stages + 1) * 8 + 16 + 1024;
+}
+// Stages of a launch: up to `most`, as many as fit.
+constexpr int pass1_stages(int most, int stage_bytes) {
+  int stages = most;
+  while (stages > 1 && pass1_smem_bytes(stages, stage_bytes) > kMaxSharedBytes) --stages;
+  return stages;
+}
 
 __device__ __forceinline__ void tcgen05_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                                  uint32_t idesc, uint32_t accumulate) {
@@ -74,7 +85,7 @@ __device__ __forceinline__ void load_x8(const void* x, size_t index, float (&v)[
   }
 }
 
-template <bool IN_BF16>
+template <bool IN_BF16, int STAGES>
 __global__ void __launch_bounds__(kFastThreads, 1)
 router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
                           const float* __restrict__ norm_weight,
@@ -85,10 +96,10 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
                                              ~static_cast<uintptr_t>(1023u));
   const int b_bytes = experts * 128;
   uint8_t* sA = smem;
-  uint8_t* sB = sA + kFastStages * kFastABytes;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sB + kFastStages * b_bytes);
-  uint64_t* empty_bar = full_bar + kFastStages;
-  uint64_t* done_bar = empty_bar + kFastStages;
+  uint8_t* sB = sA + STAGES * kFastABytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sB + STAGES * b_bytes);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* done_bar = empty_bar + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -103,7 +114,7 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
   const uint32_t tmem_cols = experts <= 32 ? 32 : experts <= 64 ? 64 : experts <= 128 ? 128 : 256;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kFastStages; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       // the gate tile arrives by TMA (one arrive + bytes), the planes are written by
       // the split warps (one arrive each)
       mbar_init(&full_bar[s], 1 + kSplitWarps);
@@ -136,7 +147,7 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
         mbar_arrive_expect_tx(&full_bar[stage], b_bytes);
         tma_load_2d(sB + stage * b_bytes, &tmap_gate, (kb_begin + kb) * kFastBlockK, 0,
                     &full_bar[stage]);
-        if (++stage == kFastStages) {
+        if (++stage == STAGES) {
           stage = 0;
           phase ^= 1u;
         }
@@ -168,7 +179,7 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
           }
         }
         tcgen05_commit(&empty_bar[stage]);
-        if (++stage == kFastStages) {
+        if (++stage == STAGES) {
           stage = 0;
           phase ^= 1u;
         }
@@ -262,7 +273,7 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
         __syncwarp();
         if (lane == 0) mbar_arrive(&full_bar[stage]);
       }
-      if (++stage == kFastStages) {
+      if (++stage == STAGES) {
         stage = 0;
         phase ^= 1u;
       }
@@ -782,21 +793,23 @@ cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* i
       splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
   }
-  const int smem = kFastStages * (kFastABytes + experts * 128) + (2 * kFastStages + 1) * 8 + 16 + 1024;
+  // three stages up to 192 experts, two beyond
+  const int stage_bytes = kFastABytes + experts * 128;
+  const int stages = pass1_stages(3, stage_bytes);
   const int grid = (rows + 127) / 128 * splits;
-  cudaError_t err;
+  auto run = [&](auto kernel) {
+    const cudaError_t err = allow_shared_memory(kernel);
+    if (err != cudaSuccess) return err;
+    launch_kernel(kernel, grid, kFastThreads, pass1_smem_bytes(stages, stage_bytes), stream,
+        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
+    return cudaGetLastError();
+  };
   if (x_bf16) {
-    err = allow_shared_memory(router_fast_logits_kernel<true>);
-    if (err != cudaSuccess) return err;
-    launch_kernel(router_fast_logits_kernel<true>, grid, kFastThreads, smem, stream,
-        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
-  } else {
-    err = allow_shared_memory(router_fast_logits_kernel<false>);
-    if (err != cudaSuccess) return err;
-    launch_kernel(router_fast_logits_kernel<false>, grid, kFastThreads, smem, stream,
-        x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
+    return stages == 3 ? run(router_fast_logits_kernel<true, 3>)
+                       : run(router_fast_logits_kernel<true, 2>);
   }
-  return cudaGetLastError();
+  return stages == 3 ? run(router_fast_logits_kernel<false, 3>)
+                     : run(router_fast_logits_kernel<false, 2>);
 }
 
 cudaError_t launch_fold_gate(const __nv_bfloat16* gate, const float* norm_weight, int experts,
@@ -824,9 +837,8 @@ cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtenso
     return cudaErrorInvalidValue;
   }
   const int stage_bytes = kFoldABytes + 3 * experts * 128;
-  const int stages = std::min(4, (220 * 1024) / stage_bytes);
-  if (stages < 2) return cudaErrorInvalidValue;
-  const int smem = stages * stage_bytes + (2 * stages + 1) * 8 + 16 + 1024;
+  const int stages = pass1_stages(4, stage_bytes);  // two at 256 experts
+  const int smem = pass1_smem_bytes(stages, stage_bytes);
   cudaError_t err = allow_shared_memory(router_folded_logits_kernel);
   if (err != cudaSuccess) return err;
   launch_kernel(router_folded_logits_kernel, (rows + 127) / 128 * splits, kFoldThreads, smem, stream,

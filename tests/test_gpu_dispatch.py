@@ -148,3 +148,19 @@ def test_a_row_that_is_not_a_number_stays_alone(small_layer, synthetic, tokens):
     others = [t for t in range(tokens) if t not in (7, 30)]
     assert torch.equal(out[others], clean[others])
 
+
+
+@pytest.mark.parametrize("experts", [192, 224, 256])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_router_of_many_experts(package, synthetic, experts, dtype):
+    # the gate tiles of pass 1 grow with the experts; its stages have to fit shared memory
+    cfg = synthetic.baseline_config(max_tokens=300, experts=experts, hidden=320, routed=64, shared=64)
+    data = synthetic.make_layer(cfg, seed=80, device="cuda", norm_weight_uniform=True)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    x = synthetic.make_tokens(300, 320, seed=81, device="cuda").to(dtype)
+    out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+    assert layer.run(x, out), layer.last_error
+    rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+    layer.close()
+    assert rep.ok(), rep.summary()
