@@ -243,8 +243,9 @@ NMOE_API nmoe_status nmoe_layer_stage_times(nmoe_layer* layer, float* millisecon
  * GEMMs execute.  The GEMMs are persistent kernels with one CTA per SM and
  * nearly all of its shared memory, so a communication kernel launched beside
  * them would not start before they finish.  This call makes the layer launch
- * its GEMMs on (SM count - reserved_sms) SMs; 0 restores the default.  No
- * reference counterpart (the reference runs one GPU per process without
+ * its GEMMs on (SM count - reserved_sms) SMs; 0 restores the default.  Call it
+ * between runs.  With few SMs left it may allocate the router's workspace for
+ * them and synchronise the device once.  No reference counterpart (the reference runs one GPU per process without
  * overlap). */
 NMOE_API nmoe_status nmoe_layer_reserve_sms(nmoe_layer* layer, int32_t reserved_sms);
 

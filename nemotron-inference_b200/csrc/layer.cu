@@ -620,19 +620,22 @@ void upload_dense_fp32(const nmoe_dense_tensor& t, size_t count, const char* nam
   }
 }
 
-// A weight of a correctly rounded linear with its slices.
+// A weight of a correctly rounded linear, with its slices where the integer kernel may run.
 struct ExactOperand {
   ExactWeight w;
   DeviceBuffer slices, info;
-  void bind(const void* weight, int kind, float scale, int n, int k, cudaStream_t stream) {
+  void bind(const void* weight, int kind, float scale, int n, int k) {
     w.N = n;
     w.K = k;
     w.kind = kind;
     w.weight = weight;
     w.scale = scale;
-    slices.allocate(slice_bytes(n, k, exact_weight_tile_rows()), true);
-    info.allocate(static_cast<size_t>(n) * sizeof(SliceRow));
-    NMOE_CUDA(launch_slice_weights(weight, kind, scale, n, k, slices.as<int8_t>(),
+  }
+  void slice(cudaStream_t stream) {
+    if (w.slices != nullptr) return;
+    slices.allocate(slice_bytes(w.N, w.K, exact_weight_tile_rows()), true);
+    info.allocate(static_cast<size_t>(w.N) * sizeof(SliceRow));
+    NMOE_CUDA(launch_slice_weights(w.weight, w.kind, w.scale, w.N, w.K, slices.as<int8_t>(),
                                    info.as<SliceRow>(), stream));
     w.slices = slices.as<int8_t>();
     w.info = info.as<SliceRow>();
@@ -664,12 +667,12 @@ struct DenseLinear {
       NMOE_REQUIRE(t.rows == out_rows && t.cols == in_cols, n + ": shape mismatch");
       if (!exact || t.dtype == NMOE_F32) {
         upload_dense_fp32(t, count, name, &weight, stream);
-        if (exact) operand.bind(weight.as<void>(), kWeightF32, 1.0f, out, in, stream);
+        if (exact) operand.bind(weight.as<void>(), kWeightF32, 1.0f, out, in);
       } else {
         NMOE_REQUIRE(t.data != nullptr && t.nbytes == count * 2, n + ": byte count");
         weight.allocate(count * 2);
         NMOE_CUDA(cudaMemcpyAsync(weight.as<void>(), t.data, count * 2, cudaMemcpyDefault, stream));
-        operand.bind(weight.as<void>(), kWeightBf16, 1.0f, out, in, stream);
+        operand.bind(weight.as<void>(), kWeightBf16, 1.0f, out, in);
       }
     } else if (linear.family == NMOE_LINEAR_SCALED_FP8) {
       // DequantizeScaledFp8WeightToHostFp32 (scaled_fp8_linear.cu:121-139)
@@ -684,7 +687,7 @@ struct DenseLinear {
         weight.allocate(count);
         NMOE_CUDA(cudaMemcpyAsync(weight.as<void>(), linear.weight.data, count, cudaMemcpyDefault,
                                   stream));
-        operand.bind(weight.as<void>(), kWeightFp8, linear.weight_scale, out, in, stream);
+        operand.bind(weight.as<void>(), kWeightFp8, linear.weight_scale, out, in);
       } else {
         DeviceBuffer staging;
         staging.allocate(count);
@@ -698,6 +701,7 @@ struct DenseLinear {
     } else {
       throw Failure{NMOE_ERR_INVALID_ARGUMENT, n + ": unknown linear family"};
     }
+    if (exact) operand.slice(stream);
     present = true;
   }
 };
@@ -732,6 +736,7 @@ void run_exact(const ExactWeight& w, ExactScratch& scratch, const float* in, flo
     NMOE_CUDA(launch_exact_gemv(w, in, fp8_scale, rows, offset, relu2, out, num_sms, stream));
     return;
   }
+  NMOE_REQUIRE(w.slices != nullptr, "an exact linear without its slices");
   for (int first = 0; first < rows; first += scratch.max_rows) {
     const int count = std::min(rows - first, scratch.max_rows);
     const float* from = in + static_cast<size_t>(first) * w.K;
@@ -1050,6 +1055,31 @@ struct nmoe_layer {
 
 namespace {
 
+// Whether some call of up to `T` rows takes the gate through the integer kernel.  In front of the
+// two-pass router only batches too small for it reach the gate: up to 255 rows of 128 x 2688 stay
+// with the FP64 kernels, and such a layer needs 25 MB less.
+bool gate_needs_slices(const nmoe_layer* L, size_t T) {
+  const int most_rows = L->fast_router
+                            ? std::min(static_cast<int>(T), L->fast_router_min_tokens - 1)
+                            : static_cast<int>(T);
+  return L->has_gate_exact &&
+         !exact_prefers_gemv(most_rows, L->cfg.n_routed_experts, L->cfg.hidden_size, L->num_sms);
+}
+
+// Slices of the gate and the workspace of the exact linears, for calls of up to `T` rows.
+void allocate_exact(nmoe_layer* L, size_t T) {
+  std::vector<std::pair<int, int>> linears;
+  if (gate_needs_slices(L, T)) {
+    L->gate_exact.slice(nullptr);
+    linears.emplace_back(L->cfg.n_routed_experts, L->cfg.hidden_size);
+  }
+  for (const DenseLinear* linear :
+       {&L->fc1, &L->fc2, &L->shared_up_dense, &L->shared_down_dense}) {
+    if (linear->present && linear->exact) linears.emplace_back(linear->out, linear->in);
+  }
+  L->exact.allocate(T, linears, device_sm_count());
+}
+
 // Everything whose size follows the token capacity.  Called at creation and by
 // nmoe_layer_reserve_tokens; weights are not touched.
 void allocate_scratch(nmoe_layer* L, size_t T) {
@@ -1088,13 +1118,7 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   if (L->shared_up_dense.present || L->shared_down_dense.present || L->unfused) {
     L->shared_raw.allocate(T * S * sizeof(float));
   }
-  std::vector<std::pair<int, int>> linears;
-  if (L->has_gate_exact) linears.emplace_back(E, H);
-  for (const DenseLinear* linear :
-       {&L->fc1, &L->fc2, &L->shared_up_dense, &L->shared_down_dense}) {
-    if (linear->present && linear->exact) linears.emplace_back(linear->out, linear->in);
-  }
-  L->exact.allocate(T, linears, device_sm_count());
+  allocate_exact(L, T);
   if (L->ep_world == 1) {
     L->parts.allocate(T * (K + 1) * static_cast<size_t>(std::max(H, Lr)) * sizeof(float));
   }
@@ -1252,7 +1276,7 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   if (L->has_gate_exact) {
     const bool bf16 = w.gate_weight.dtype == NMOE_BF16;
     L->gate_exact.bind(bf16 ? L->gate_bf16.as<void>() : L->gate.as<void>(),
-                       bf16 ? kWeightBf16 : kWeightF32, 1.0f, E, H, stream);
+                       bf16 ? kWeightBf16 : kWeightF32, 1.0f, E, H);
   }
   // The tensor-core pass needs the gate exactly in bf16.
   L->fast_router = w.gate_weight.dtype == NMOE_BF16 && c.n_group == 1 && E % 32 == 0 &&
@@ -1836,7 +1860,19 @@ nmoe_status nmoe_layer_reserve_sms(nmoe_layer* layer, int32_t reserved_sms) {
   const int all = device_sm_count();
   if (reserved_sms < 0 || reserved_sms >= all) return NMOE_ERR_INVALID_ARGUMENT;
   layer->drop_recorded();
+  const int before = layer->num_sms;
   layer->num_sms = all - reserved_sms;
+  const size_t tokens = static_cast<size_t>(layer->cfg.max_tokens);
+  if (layer->gate_exact.w.slices != nullptr || !gate_needs_slices(layer, tokens)) return NMOE_OK;
+  try {  // with this few SMs the gate goes through the integer kernel
+    NMOE_CUDA(cudaDeviceSynchronize());
+    allocate_exact(layer, tokens);
+    NMOE_CUDA(cudaDeviceSynchronize());
+  } catch (const Failure& failure) {
+    layer->num_sms = before;
+    layer->last_error = failure.message;
+    return failure.status;
+  }
   return NMOE_OK;
 }
 

@@ -164,3 +164,36 @@ def test_router_of_many_experts(package, synthetic, experts, dtype):
     rep = helpers.compare_layer_with_oracle(layer, data, x, out)
     layer.close()
     assert rep.ok(), rep.summary()
+
+
+def test_gate_slices_exist_where_a_call_needs_them(package, synthetic, monkeypatch):
+    # a gate of 128 x 2688 in front of the two-pass router stays with the FP64 kernels (up to 255
+    # rows): its digits and their workspace (25 MB at 1024 tokens) are for layers without that router
+    cfg = synthetic.baseline_config(max_tokens=1024, hidden=2688, routed=64, shared=64)
+    data = synthetic.make_layer(cfg, seed=82, device="cuda")
+    torch.cuda.synchronize()
+
+    def create():
+        free = torch.cuda.mem_get_info()[0]
+        layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+        assert layer is not None, package.ExpertLayerSlice.create_error
+        return layer, free - torch.cuda.mem_get_info()[0]
+
+    create()[0].close()
+    two_pass, two_pass_bytes = create()
+    monkeypatch.setenv("NMOE_ROUTER_FP64_ONLY", "1")
+    exact_only, exact_only_bytes = create()
+    print(two_pass_bytes, exact_only_bytes)
+    assert two_pass_bytes < exact_only_bytes
+    x = synthetic.make_tokens(200, 2688, seed=83, device="cuda")
+    results = []
+    for layer, reserved in ((exact_only, 0), (two_pass, 0), (two_pass, 130), (two_pass, 0)):
+        layer.reserve_sms(reserved)  # with 18 SMs left the gate's FP64 kernels no longer pay
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        assert layer.run(x, out), layer.last_error
+        results.append((out, layer.trace(200).router_logits))
+    for out, logits in results[1:]:
+        assert torch.equal(logits, results[0][1])
+        assert torch.equal(out, results[0][0])
+    two_pass.close()
+    exact_only.close()
