@@ -36,6 +36,7 @@ struct Failure {
   do {                                                                                     \
     const cudaError_t err__ = (expr);                                                      \
     if (err__ != cudaSuccess) {                                                            \
+      cudaGetLastError(); /* reported here: it must not fail the next launch as well */    \
       throw Failure{NMOE_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(err__)}; \
     }                                                                                      \
   } while (0)

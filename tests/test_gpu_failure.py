@@ -40,3 +40,16 @@ def test_bounded_flag_wait_runs_out_and_the_layer_stays_usable(package, syntheti
     assert layer.run(x, out), layer.last_error
     assert torch.equal(out, before)
     layer.close()
+
+
+def test_a_refused_allocation_does_not_fail_the_next_call(package, synthetic):
+    up, down = synthetic.make_ffn_weights(256, 128, seed=13, device="cuda")
+    ffn = package.ExpertFfn(up, down, max_rows=64)
+    x = synthetic.make_tokens(20, 256, seed=14, device="cuda")
+    want = ffn.run(x)
+    # more scratch than any GPU holds: refused at once
+    cfg = synthetic.baseline_config(max_tokens=2 ** 30, experts=32, hidden=512, routed=64, shared=64)
+    data = synthetic.make_layer(cfg, seed=15, device="cuda")
+    assert package.ExpertLayerSlice.create(cfg, data.bindings) is None
+    assert torch.equal(ffn.run(x), want)
+    ffn.close()
