@@ -1176,6 +1176,30 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   L->last_tokens = 0;
 }
 
+// Other scratch for a layer that has some.  Where there is no memory for it the layer gets back what
+// it had, or, should that fail too, none (every run is then refused): no run finds a freed buffer.
+void reallocate_scratch(nmoe_layer* L, size_t T, bool unfused) {
+  const size_t had = static_cast<size_t>(L->cfg.max_tokens);
+  const bool was_unfused = L->unfused;
+  NMOE_CUDA(cudaDeviceSynchronize());
+  L->cfg.max_tokens = 0;
+  L->last_tokens = 0;
+  L->unfused = unfused;
+  try {
+    allocate_scratch(L, T);
+  } catch (const Failure&) {
+    L->unfused = was_unfused;
+    L->u_raw.reset();
+    try {
+      allocate_scratch(L, had);
+    } catch (const Failure&) {
+      L->cfg.max_tokens = 0;
+    }
+    throw;
+  }
+  NMOE_CUDA(cudaDeviceSynchronize());
+}
+
 void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& w) {
   // config checks of expert_layer.cpp:505-528
   NMOE_REQUIRE(c.hidden_size > 0 && c.moe_latent_size > 0 &&
@@ -2371,9 +2395,7 @@ nmoe_status nmoe_layer_reserve_tokens(nmoe_layer* layer, int32_t max_tokens) {
   if (max_tokens <= layer->cfg.max_tokens) return NMOE_OK;
   if (layer->window.attached) return NMOE_ERR_INVALID_ARGUMENT;  // peers hold the old window
   try {
-    NMOE_CUDA(cudaDeviceSynchronize());
-    allocate_scratch(layer, static_cast<size_t>(max_tokens));
-    NMOE_CUDA(cudaDeviceSynchronize());
+    reallocate_scratch(layer, static_cast<size_t>(max_tokens), layer->unfused);
   } catch (const Failure& failure) {
     layer->last_error = failure.message;
     return failure.status;
@@ -2387,14 +2409,13 @@ nmoe_status nmoe_layer_set_unfused_activation(nmoe_layer* layer, int32_t enable)
   if (want == layer->unfused) return NMOE_OK;
   if (want && layer->ep_world > 1) return NMOE_ERR_UNSUPPORTED;
   try {
-    NMOE_CUDA(cudaDeviceSynchronize());
-    layer->unfused = want;
     if (want && layer->u_raw.bytes() == 0) {
-      allocate_scratch(layer, static_cast<size_t>(layer->cfg.max_tokens));
+      reallocate_scratch(layer, static_cast<size_t>(layer->cfg.max_tokens), true);
+    } else {
       NMOE_CUDA(cudaDeviceSynchronize());
+      layer->unfused = want;
     }
   } catch (const Failure& failure) {
-    layer->unfused = false;
     layer->last_error = failure.message;
     return failure.status;
   }

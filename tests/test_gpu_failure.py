@@ -53,3 +53,22 @@ def test_a_refused_allocation_does_not_fail_the_next_call(package, synthetic):
     assert package.ExpertLayerSlice.create(cfg, data.bindings) is None
     assert torch.equal(ffn.run(x), want)
     ffn.close()
+
+
+def test_a_layer_keeps_its_scratch_when_it_cannot_grow(package, synthetic):
+    cfg = synthetic.baseline_config(max_tokens=64, experts=32, hidden=512, routed=64, shared=64)
+    data = synthetic.make_layer(cfg, seed=16, device="cuda")
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    x = synthetic.make_tokens(64, 512, seed=17, device="cuda")
+    out = torch.empty((64, 512), dtype=torch.float32, device="cuda")
+    assert layer.run(x, out), layer.last_error
+    with pytest.raises(package.NmoeError):
+        layer.reserve_tokens(2 ** 30)
+    again = torch.empty_like(out)
+    assert layer.run(x, again), layer.last_error
+    assert torch.equal(again, out)
+    layer.reserve_tokens(200)
+    layer.set_unfused_activation(True)
+    assert layer.run(x, again), layer.last_error
+    assert torch.equal(again, out)
+    layer.close()
