@@ -1166,6 +1166,8 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
     L->unweighted_tokens = static_cast<int>(std::min<size_t>(T, 64));
     L->unweighted_rows.allocate(static_cast<size_t>(L->unweighted_tokens) * (K + 1) *
                                 std::max(H, Lr) * sizeof(float), true);
+  } else {
+    L->u_raw.reset();  // of another size: the unfused path allocates when it is enabled
   }
 
   L->y_op.bind(L->y_packed.as<uint8_t>(), L->y_sf_tiled.as<uint8_t>(), token_slots * 128, H);
@@ -1189,7 +1191,6 @@ void reallocate_scratch(nmoe_layer* L, size_t T, bool unfused) {
     allocate_scratch(L, T);
   } catch (const Failure&) {
     L->unfused = was_unfused;
-    L->u_raw.reset();
     try {
       allocate_scratch(L, had);
     } catch (const Failure&) {

@@ -72,3 +72,25 @@ def test_a_layer_keeps_its_scratch_when_it_cannot_grow(package, synthetic):
     assert layer.run(x, again), layer.last_error
     assert torch.equal(again, out)
     layer.close()
+
+
+def test_unfused_rows_follow_the_scratch(package, synthetic):
+    # enabled, disabled, grown, enabled: the FP32 rows have to be the larger scratch's
+    cfg = synthetic.baseline_config(max_tokens=16, experts=32, hidden=512, routed=256, shared=256)
+    data = synthetic.make_layer(cfg, seed=18, device="cuda")
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    x = synthetic.make_tokens(700, 512, seed=19, device="cuda")
+    out = torch.empty((700, 512), dtype=torch.float32, device="cuda")
+    layer.set_unfused_activation(True)
+    assert layer.run(x[:16], out[:16]), layer.last_error
+    layer.set_unfused_activation(False)
+    layer.reserve_tokens(700)
+    assert layer.run(x, out), layer.last_error
+    free = torch.cuda.mem_get_info()[0]
+    layer.set_unfused_activation(True)
+    # 4200 pairs in row tiles of 128: at least their FP32 rows
+    assert free - torch.cuda.mem_get_info()[0] >= 4200 * 256 * 4
+    again = torch.empty_like(out)
+    assert layer.run(x, again), layer.last_error
+    assert torch.equal(again, out)
+    layer.close()
