@@ -244,7 +244,6 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   volatile Tile* ring = reinterpret_cast<volatile Tile*>(ring_empty_bar + kRing);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(
       reinterpret_cast<uint8_t*>(ring_empty_bar + kRing) + kRing * sizeof(Tile));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -265,7 +264,6 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       mbar_init(&ring_full_bar[i], 1);
       mbar_init(&ring_empty_bar[i], kRingReaders);
     }
-    *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -302,7 +300,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
     while (ok) {
       const Tile tile = list.locate(args, t);
       if (!mbar_wait_warp(reader.empty0 + slot * 8, slot_phase ^ 1u)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       if (elect_one()) {
@@ -356,7 +354,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
           phase ^= 1u;
         }
       }
-      if (!ok) report_timeout(args.error, abort_flag);
+      if (!ok) report_timeout(args.error);
       t = warp_uniform(next);
     }
   } else if (warp == kRowWarp) {
@@ -367,7 +365,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
     while (ok) {
       Tile tile;
       if (!reader.next(tile)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       if (tile.phase < 0) break;
@@ -392,7 +390,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
           phase ^= 1u;
         }
       }
-      if (!ok) report_timeout(args.error, abort_flag);
+      if (!ok) report_timeout(args.error);
     }
   } else if (warp == 1) {
     // -------------------------------------------------- scale copies and MMAs
@@ -409,12 +407,12 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       Tile tile;
       const int acc = local & 1;
       if (!reader.next(tile)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       if (tile.phase < 0) break;
       if (!mbar_wait_warp(smem_u32(&tmem_empty_bar[acc]), ((local >> 1) & 1u) ^ 1u)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       const GemmArgs& g = args.phase[tile.phase].gemm;
@@ -423,7 +421,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       const uint32_t d_tmem = tmem_base + acc * kBN;
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_warp(full0 + stage * 8, phase)) {
-          report_timeout(args.error, abort_flag);
+          report_timeout(args.error);
           ok = false;
           break;
         }
@@ -462,12 +460,12 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       Tile tile;
       const int acc = local & 1;
       if (!reader.next(tile)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       if (tile.phase < 0) break;
       if (!mbar_wait_warp(smem_u32(&stored_bar[acc]), (local >> 1) & 1u)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       const StreamPhase& ph = args.phase[tile.phase];
@@ -491,7 +489,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       const uint32_t acc_phase = (local >> 1) & 1u;
       Tile tile;
       if (!reader.next(tile)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       if (tile.phase < 0) break;
@@ -508,7 +506,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
         if (g.row_weight != nullptr) wt = g.row_weight[grow];
       }
       if (!mbar_wait(&tmem_full_bar[acc], acc_phase)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       const int n0 = tile.nt * kBN;

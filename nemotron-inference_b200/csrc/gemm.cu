@@ -124,7 +124,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   uint64_t* tmem_full_bar = empty_bar + kStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -142,7 +141,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       mbar_init(&tmem_full_bar[a], 1);
       mbar_init(&tmem_empty_bar[a], 2 * kEpilogueWarps);
     }
-    *abort_flag = 0;
     fence_barrier_init();
     prefetch_tensormap(&maps.a);
     prefetch_tensormap(&maps.b_tail);
@@ -187,7 +185,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       const int b_row = nt * kPairBN + static_cast<int>(cta_rank) * kPairBRows;
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!mbar_wait_warp(empty0 + stage * 8, phase ^ 1u)) {
-          report_timeout(args.error, abort_flag);
+          report_timeout(args.error);
           ok = false;
           break;
         }
@@ -231,14 +229,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         const uint32_t acc_phase = (local >> 1) & 1u;
         // both CTAs' epilogues have drained this accumulator
         if (!mbar_wait_warp(smem_u32(&tmem_empty_bar[acc]), acc_phase ^ 1u)) {
-          report_timeout(args.error, abort_flag);
+          report_timeout(args.error);
           break;
         }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kPairBN;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait_warp(full0 + stage * 8, phase)) {
-            report_timeout(args.error, abort_flag);
+            report_timeout(args.error);
             ok = false;
             break;
           }
@@ -323,7 +321,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         if (args.row_weight != nullptr) wt = args.row_weight[grow];
       }
       if (!mbar_wait(&tmem_full_bar[acc], acc_phase)) {
-        report_timeout(args.error, abort_flag);
+        report_timeout(args.error);
         break;
       }
       if (quarter * 32 < tile.rows) {  // (else none of the warp's rows exist)

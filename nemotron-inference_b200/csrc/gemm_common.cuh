@@ -9,8 +9,7 @@
 
 namespace nmoe {
 
-__device__ __forceinline__ void report_timeout(int32_t* error, volatile int* abort_flag) {
-  *abort_flag = 1;
+__device__ __forceinline__ void report_timeout(int32_t* error) {
   if (error != nullptr) atomicCAS(error, kDevOk, kDevWaitTimeout);
 }
 

@@ -232,7 +232,7 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int rows,
 cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* inv_rms,
                                       const float* norm_weight, const CUtensorMap& tmap_gate,
                                       int rows, int experts, int hidden, int splits,
-                                      float* logits, int32_t* error, LaunchStream stream);
+                                      float* logits, int32_t* error, cudaStream_t stream);
 // Pass 1 for bf16 layer inputs: the RMSNorm weight folded into the gate (three bf16 terms of
 // fl32(w[i] * gate[e][i]), `planes` = [3][experts][hidden], built once by launch_fold_gate),
 // the input rows read by TMA through `tmap_x` ([rows][hidden] bf16, box 64 x 128, 128-byte
@@ -255,7 +255,7 @@ inline size_t router_pass1_rows(size_t max_rows, int num_sms) {
 cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtensorMap& tmap_planes,
                                         const float* inv_rms, int rows, int experts, int hidden,
                                         int splits, float* logits, int32_t* error,
-                                        LaunchStream stream);
+                                        cudaStream_t stream);
 cudaError_t launch_router_select_exact(float* logits, int splits, const void* x, bool x_bf16,
                                        const float* inv_rms, const float* norm_weight,
                                        const __nv_bfloat16* gate, const float* logit_offset,
@@ -263,7 +263,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        int top_k, bool norm_topk_prob, float routed_scaling,
                                        float tie_margin, int32_t* top_index, float* top_weight,
                                        int32_t* expert_counts, int32_t* position,
-                                       LaunchStream stream);
+                                       cudaStream_t stream);
 
 // --- correctly rounded linears (csrc/exact.cu) ---------------------------------
 // y[rows][N] = x[rows][K] x W[N][K]^T in FP32, each value the FP64 sum rounded once.

@@ -22,15 +22,6 @@ namespace {
 constexpr int kWarpsPerBlock = 8;
 
 template <bool BF16>
-__device__ __forceinline__ float load_scalar(const void* base, size_t index) {
-  if constexpr (BF16) {
-    return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(base)[index]);
-  } else {
-    return reinterpret_cast<const float*>(base)[index];
-  }
-}
-
-template <bool BF16>
 __device__ __forceinline__ void load8(const void* base, size_t index, float (&v)[8]) {
   if constexpr (BF16) {
     const uint4 raw = *reinterpret_cast<const uint4*>(

@@ -132,8 +132,6 @@ router_fast_logits_kernel(const void* __restrict__ x, const float* inv_rms,
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  release_successor();
-  wait_for_predecessor();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -386,8 +384,6 @@ router_folded_logits_kernel(const __grid_constant__ CUtensorMap tmap_x,
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  release_successor();
-  wait_for_predecessor();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -558,8 +554,6 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
   __shared__ int16_t candidate_list[kSelectWarps][256];
   __shared__ float logit_smem[WARPS > 1 ? 256 : 1];
   __shared__ double partial_smem[WARPS > 1 ? kSelectWarps : 1][8];
-  release_successor();
-  wait_for_predecessor();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int part = WARPS > 1 ? warp : 0;  // this warp's share of the contraction
@@ -788,7 +782,7 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
 cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* inv_rms,
                                       const float* norm_weight, const CUtensorMap& tmap_gate,
                                       int rows, int experts, int hidden, int splits,
-                                      float* logits, int32_t* error, LaunchStream stream) {
+                                      float* logits, int32_t* error, cudaStream_t stream) {
   if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0 ||
       splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
@@ -800,7 +794,7 @@ cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* i
   auto run = [&](auto kernel) {
     const cudaError_t err = allow_shared_memory(kernel);
     if (err != cudaSuccess) return err;
-    launch_kernel(kernel, grid, kFastThreads, pass1_smem_bytes(stages, stage_bytes), stream,
+    kernel<<<grid, kFastThreads, pass1_smem_bytes(stages, stage_bytes), stream>>>(
         x, inv_rms, norm_weight, tmap_gate, rows, experts, hidden, splits, logits, error);
     return cudaGetLastError();
   };
@@ -831,7 +825,7 @@ int router_pass1_splits(int rows, int hidden, int num_sms) {
 cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtensorMap& tmap_planes,
                                         const float* inv_rms, int rows, int experts, int hidden,
                                         int splits, float* logits, int32_t* error,
-                                        LaunchStream stream) {
+                                        cudaStream_t stream) {
   if (rows <= 0 || experts % 16 != 0 || experts > 256 || hidden % kFastBlockK != 0 ||
       splits < 1 || hidden / kFastBlockK < splits) {
     return cudaErrorInvalidValue;
@@ -841,7 +835,7 @@ cudaError_t launch_router_folded_logits(const CUtensorMap& tmap_x, const CUtenso
   const int smem = pass1_smem_bytes(stages, stage_bytes);
   cudaError_t err = allow_shared_memory(router_folded_logits_kernel);
   if (err != cudaSuccess) return err;
-  launch_kernel(router_folded_logits_kernel, (rows + 127) / 128 * splits, kFoldThreads, smem, stream,
+  router_folded_logits_kernel<<<(rows + 127) / 128 * splits, kFoldThreads, smem, stream>>>(
       tmap_x, tmap_planes, inv_rms, rows, experts, hidden, stages, splits, logits, error);
   return cudaGetLastError();
 }
@@ -852,7 +846,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        const float* bias, int rows, int experts, int hidden,
                                        int top_k, bool norm_topk_prob, float routed_scaling,
                                        float tie_margin, int32_t* top_index, float* top_weight,
-                                       int32_t* expert_counts, int32_t* position, LaunchStream stream) {
+                                       int32_t* expert_counts, int32_t* position, cudaStream_t stream) {
   if (rows <= 0 || experts % 32 != 0 || experts > 32 * kSelectPerLane || top_k <= 0 ||
       top_k > 32 || top_k > experts || hidden % 8 != 0 || splits < 1) {
     return cudaErrorInvalidValue;
@@ -860,7 +854,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
   const bool whole_block = rows <= kSelectWholeBlockRows;
   const int grid = whole_block ? rows : (rows + kSelectWarps - 1) / kSelectWarps;
   auto run = [&](auto kernel) {
-    launch_kernel(kernel, grid, kSelectWarps * 32, 0, stream,
+    kernel<<<grid, kSelectWarps * 32, 0, stream>>>(
         logits, splits, x, inv_rms, norm_weight, gate, logit_offset, bias, rows, experts, hidden,
         top_k, norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts,
         position);
