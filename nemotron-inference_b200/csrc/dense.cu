@@ -22,11 +22,6 @@
 namespace nmoe {
 namespace {
 
-int blocks_for(size_t work, int threads) {
-  const size_t blocks = (work + threads - 1) / threads;
-  return static_cast<int>(blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks));
-}
-
 __global__ void fp8_round_trip_kernel(const float* __restrict__ in, size_t count, float scale,
                                       float* __restrict__ out) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count;
@@ -129,27 +124,27 @@ cudaError_t launch_fp8_round_trip(const float* in, size_t count, float input_sca
   if (count == 0) return cudaErrorInvalidValue;
   // ClampScale (scaled_fp8_linear.cu:27-33)
   const float scale = clamp_scale_host(input_scale);
-  fp8_round_trip_kernel<<<blocks_for(count, 256), 256, 0, stream>>>(in, count, scale, out);
+  fp8_round_trip_kernel<<<stride_blocks(count, 256), 256, 0, stream>>>(in, count, scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_fp8_weight_dequant(const uint8_t* bytes, size_t count, float weight_scale,
                                       float* out, cudaStream_t stream) {
   if (count == 0) return cudaErrorInvalidValue;
-  fp8_weight_kernel<<<blocks_for(count, 256), 256, 0, stream>>>(bytes, count, weight_scale, out);
+  fp8_weight_kernel<<<stride_blocks(count, 256), 256, 0, stream>>>(bytes, count, weight_scale, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_relu2(float* values, size_t count, cudaStream_t stream) {
   if (count == 0) return cudaErrorInvalidValue;
-  relu2_kernel<<<blocks_for(count, 256), 256, 0, stream>>>(values, count);
+  relu2_kernel<<<stride_blocks(count, 256), 256, 0, stream>>>(values, count);
   return cudaGetLastError();
 }
 
 cudaError_t launch_sum_parts(const float* parts, int rows, int cols, int top_k, float* out,
                              LaunchStream stream) {
   if (rows <= 0 || cols % 4 != 0 || top_k < 1) return cudaErrorInvalidValue;
-  launch_kernel(sum_parts_kernel, blocks_for(static_cast<size_t>(rows) * (cols / 4), 256), 256, 0, stream,
+  launch_kernel(sum_parts_kernel, stride_blocks(static_cast<size_t>(rows) * (cols / 4), 256), 256, 0, stream,
       parts, rows, cols, top_k, out);
   return cudaGetLastError();
 }
@@ -158,7 +153,7 @@ cudaError_t launch_mixer(const void* in, bool in_bf16, const float* projected, c
                          int rows, int hidden, void* out, bool out_bf16, LaunchStream stream) {
   if (rows <= 0 || hidden <= 0) return cudaErrorInvalidValue;
   const size_t count = static_cast<size_t>(rows) * hidden;
-  const int blocks = blocks_for(count, 256);
+  const int blocks = stride_blocks(count, 256);
   if (in_bf16 && out_bf16) {
     launch_kernel(mixer_kernel<true, true>, blocks, 256, 0, stream, in, projected, shared, count, out);
   } else if (in_bf16) {

@@ -325,7 +325,7 @@ cudaError_t launch_combine_indexed(const void* in, bool in_bf16, const void* ret
                                    int32_t* error, cudaStream_t stream) {
   if (rows <= 0 || hidden % 4 != 0 || top_k < 1) return cudaErrorInvalidValue;
   const size_t total = static_cast<size_t>(rows) * (hidden / 4);
-  const int blocks = static_cast<int>((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+  const int blocks = stride_blocks(total, 256);
   if (in_bf16 && out_bf16) {
     combine_indexed_kernel<true, true><<<blocks, 256, 0, stream>>>(
         in, returned_rows, rows_kind, position, shared_rows, shared_kind, rows, hidden, top_k, out,

@@ -441,7 +441,7 @@ cudaError_t relayout_weight_packed(const uint8_t* row_major, int experts, int N,
                                    cudaStream_t stream) {
   const int row_chunks = K / 32;
   const size_t chunks = static_cast<size_t>(experts) * N * row_chunks;
-  const int blocks = static_cast<int>(std::min<size_t>((chunks + 255) / 256, 148 * 32));
+  const int blocks = stride_blocks(chunks, 256);
   relayout_weight_packed_kernel<<<blocks, 256, 0, stream>>>(
       reinterpret_cast<const uint4*>(row_major), experts, N, row_chunks, K / 256,
       tail_pitch_bytes / 16, reinterpret_cast<uint4*>(full), reinterpret_cast<uint4*>(tail),

@@ -38,6 +38,24 @@ inline cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, int threa
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
+// SMs of the current device.
+inline int device_sms() {
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    cudaGetLastError();  // (the launch will say what is wrong)
+    return 1;
+  }
+  return sms;
+}
+// Blocks of a kernel that walks its elements with a grid-sized stride: enough to fill the GPU several
+// times over, so that blocks need not be whole waves.
+constexpr int kStrideBlocks = 2368;
+inline int stride_blocks(size_t work, int threads) {
+  const size_t blocks = (work + threads - 1) / threads;
+  return static_cast<int>(blocks < 1 ? 1 : blocks > kStrideBlocks ? kStrideBlocks : blocks);
+}
+
 // Lets `kernel` (which has no static shared memory) be launched with all the dynamic shared memory a
 // block can have.  The limit belongs to the kernel and not to the launch, so it never follows the
 // launch's own size: a thread that lowered it between another thread's limit and launch made that
@@ -193,7 +211,7 @@ size_t weight_scale_layout_bytes(int experts, int N, int K, int bn, int sfb_grou
 cudaError_t launch_norm_quant(const void* in, bool in_bf16, int rows, int cols,
                               const float* norm_weight, float eps, float* normalized,
                               uint8_t* packed, uint8_t* sf_row_major, uint8_t* sf_tiled,
-                              int k_blocks, float* tensor_scale, LaunchStream stream,
+                              int k_blocks, float* tensor_scale, int num_sms, LaunchStream stream,
                               float* inv_rms = nullptr, int32_t* zero = nullptr,
                               int zero_count = 0);
 // Whole-matrix dynamic quantisation with ONE tensor scale (the reference
@@ -211,7 +229,8 @@ cudaError_t launch_swizzle_scales(const uint8_t* row_major, int rows, int cols, 
 // --- router ------------------------------------------------------------------
 cudaError_t launch_router_logits(const float* normalized, const float* gate,
                                  const float* logit_offset /* nullable [experts] */, int rows,
-                                 int experts, int hidden, float* logits, cudaStream_t stream);
+                                 int experts, int hidden, float* logits, int num_sms,
+                                 cudaStream_t stream);
 // The argument rules of launch_router_topk, for callers that must know before they
 // enqueue anything.
 bool router_topk_arguments_valid(int rows, int experts, int top_k, int n_group, int topk_group);
@@ -220,7 +239,7 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int rows,
                                float routed_scaling, int32_t* top_index, float* top_weight,
                                int32_t* expert_counts /* nullable, += histogram */,
                                int32_t* position /* nullable [rows][top_k]: the count before */,
-                               LaunchStream stream);
+                               int num_sms, LaunchStream stream);
 
 // Two-pass router for large batches.  Pass 1: logits on the tensor cores (FP32
 // accumulate) from the bf16 gate and the normalised activations, which the kernel
@@ -366,7 +385,7 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               uint8_t* sorted_sf_tiled, float* sorted_tensor_scale,
                               float* sorted_weight, int32_t* sorted_dest,
                               int32_t* pair_row /* nullable */, int dest_stride, int32_t* error,
-                              LaunchStream stream);
+                              int num_sms, LaunchStream stream);
 // --- expert-parallel dispatch / return (csrc/ep.cu) ---------------------------
 int dispatch_record_bytes(int cols);
 cudaError_t launch_dispatch_plan(const int32_t* expert_counts, int experts, int experts_per_rank,

@@ -615,7 +615,7 @@ void upload_dense_fp32(const nmoe_dense_tensor& t, size_t count, const char* nam
     DeviceBuffer staging;
     staging.allocate(count * 2);
     NMOE_CUDA(cudaMemcpyAsync(staging.as<void>(), t.data, count * 2, cudaMemcpyDefault, stream));
-    widen_bf16_kernel<<<148, 256, 0, stream>>>(staging.as<__nv_bfloat16>(), count, out->as<float>());
+    widen_bf16_kernel<<<stride_blocks(count, 256), 256, 0, stream>>>(staging.as<__nv_bfloat16>(), count, out->as<float>());
     NMOE_CUDA(cudaGetLastError());
     NMOE_CUDA(cudaStreamSynchronize(stream));
   }
@@ -839,7 +839,7 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
     NMOE_CUDA(launch_norm_quant(input, input_dtype == NMOE_BF16, static_cast<int>(rows),
                                 ffn->hidden, nullptr, 0.0f, nullptr, ffn->a_packed.as<uint8_t>(),
                                 nullptr, ffn->a_sf.as<uint8_t>(), k_blocks_of(ffn->hidden),
-                                ffn->a_ts.as<float>(), stream));
+                                ffn->a_ts.as<float>(), ffn->num_sms, stream));
     Schedule schedule;
     schedule.dense_rows = static_cast<int>(rows);
     schedule.most_rows = std::min(128, static_cast<int>(rows));
@@ -1342,7 +1342,7 @@ void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, 
     source = L->fp8_tmp.as<float>();
   }
   NMOE_CUDA(launch_router_logits(source, linear.weight.as<float>(), nullptr, rows, linear.out,
-                                 linear.in, out_rows, stream));
+                                 linear.in, out_rows, L->num_sms, stream));
   if (relu2) {
     NMOE_CUDA(launch_relu2(out_rows, static_cast<size_t>(rows) * linear.out, stream));
   }
@@ -1367,7 +1367,7 @@ void route_tokens(nmoe_layer* L, LaunchStream stream, const void* input, nmoe_dt
                               c.rms_epsilon, want_normalized ? L->normalized.as<float>() : nullptr,
                               L->y_packed.as<uint8_t>(), L->y_sf_row_major.as<uint8_t>(),
                               L->y_sf_tiled.as<uint8_t>(), k_blocks_of(H), L->y_ts.as<float>(),
-                              stream.stream, L->inv_rms.as<float>(), L->counts.as<int32_t>(), E));
+                              L->num_sms, stream.stream, L->inv_rms.as<float>(), L->counts.as<int32_t>(), E));
   L->last_normalized = want_normalized;
   if (after_quantise != nullptr && !fork_after_logits) {
     NMOE_CUDA(cudaEventRecord(after_quantise, stream));
@@ -1410,14 +1410,14 @@ void route_tokens(nmoe_layer* L, LaunchStream stream, const void* input, nmoe_dt
                 L->logits.as<float>(), error, L->num_sms, stream);
     } else {
       NMOE_CUDA(launch_router_logits(L->normalized.as<float>(), L->gate.as<float>(), offset, tokens,
-                                     E, H, L->logits.as<float>(), stream));
+                                     E, H, L->logits.as<float>(), L->num_sms, stream));
     }
     L->mark(2, stream);
     NMOE_CUDA(launch_router_topk(L->logits.as<float>(), L->bias.as<float>(), tokens, E, K,
                                  c.n_group, c.topk_group, c.norm_topk_prob != 0,
                                  c.routed_scaling_factor, L->top_index.as<int32_t>(),
                                  L->top_weight.as<float>(), L->counts.as<int32_t>(),
-                                 L->position.as<int32_t>(), stream));
+                                 L->position.as<int32_t>(), L->num_sms, stream));
   }
   L->mark(3, stream);
 }
@@ -1451,7 +1451,7 @@ void run_ffn(nmoe_layer* L, bool unfused, const WeightStack& up, const WeightSta
   run_down_gemm(up, kClassStream, a, a_ts, schedule, raw, error, L->num_sms, stream);
   NMOE_CUDA(launch_norm_quant(buffers.raw_rows, false, buffers.raw_row_count, up.n, nullptr, 0.0f,
                               nullptr, buffers.hidden_packed, nullptr, buffers.hidden_sf,
-                              k_blocks_of(up.n), buffers.hidden_ts, stream));
+                              k_blocks_of(up.n), buffers.hidden_ts, L->num_sms, stream));
   if (between != nullptr) cudaEventRecord(between, stream);
   run_down_gemm(down, tile_class, *buffers.hidden, buffers.hidden_ts, schedule, out, error,
                 L->num_sms, stream);
@@ -1498,7 +1498,7 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
                               L->a_ts.as<float>(), L->a_weight.as<float>(),
                               L->a_dest.as<int32_t>(),
                               L->ep_world == 1 ? L->pair_row.as<int32_t>() : nullptr, dest_stride,
-                              error, stream));
+                              error, L->num_sms, stream));
   if (!L->stage_timing) stream.chained = true;
   L->mark(5, stream);
   // routed experts (:896-954)
@@ -1571,7 +1571,7 @@ void quantise_shared_hidden(nmoe_layer* L, LaunchStream stream, int tokens) {
   const int S = L->cfg.shared_expert_intermediate_size;
   NMOE_CUDA(launch_norm_quant(L->shared_raw.as<float>(), false, tokens, S, nullptr, 0.0f, nullptr,
                               L->sh_packed.as<uint8_t>(), nullptr, L->sh_sf.as<uint8_t>(),
-                              k_blocks_of(S), L->sh_ts.as<float>(), stream));
+                              k_blocks_of(S), L->sh_ts.as<float>(), L->num_sms, stream));
 }
 
 // shared expert (:814-818, :956-964, :981-1005) on the token-order rows
@@ -1692,7 +1692,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     NMOE_CUDA(launch_norm_quant(L->latent_rows.as<float>(), false, tokens, Lr, nullptr, 0.0f,
                                 nullptr, L->lat_packed.as<uint8_t>(),
                                 L->lat_sf_row_major.as<uint8_t>(), nullptr, 0,
-                                L->lat_ts.as<float>(), chain));
+                                L->lat_ts.as<float>(), L->num_sms, chain));
     PermuteSource source = local_source(L);
     source.packed = L->lat_packed.as<uint8_t>();
     source.packed_stride = static_cast<size_t>(Lr) / 2;
@@ -2503,7 +2503,7 @@ nmoe_status nmoe_quantize_nvfp4(void* stream_ptr, const void* input, nmoe_dtype 
     // the tiled layout of this entry point pads blocks to 4, not to a K block
     err = launch_norm_quant(input, dtype == NMOE_BF16, static_cast<int>(rows),
                             static_cast<int>(cols), nullptr, 0.0f, nullptr, packed,
-                            scales_row_major, nullptr, 0, tensor_scale, stream);
+                            scales_row_major, nullptr, 0, tensor_scale, device_sms(), stream);
     if (err == cudaSuccess && scales_swizzled != nullptr) {
       err = launch_swizzle_scales(scales_row_major, static_cast<int>(rows),
                                   static_cast<int>(cols), scales_swizzled, stream);
@@ -2568,7 +2568,8 @@ nmoe_status nmoe_rmsnorm(void* stream_ptr, const void* input, nmoe_dtype dtype, 
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   const cudaError_t err = launch_norm_quant(input, dtype == NMOE_BF16, static_cast<int>(rows),
                                             static_cast<int>(hidden), weight, epsilon, output,
-                                            nullptr, nullptr, nullptr, 0, nullptr, stream);
+                                            nullptr, nullptr, nullptr, 0, nullptr, device_sms(),
+                                            stream);
   return err == cudaSuccess ? NMOE_OK : NMOE_ERR_CUDA;
 }
 
@@ -2578,7 +2579,7 @@ nmoe_status nmoe_router_logits(void* stream, const float* normalized, const floa
     return NMOE_ERR_INVALID_ARGUMENT;
   }
   return launch_router_logits(normalized, gate, nullptr, static_cast<int>(rows), experts, hidden,
-                              logits,
+                              logits, device_sms(),
                               static_cast<cudaStream_t>(stream)) == cudaSuccess
              ? NMOE_OK
              : NMOE_ERR_INVALID_ARGUMENT;
@@ -2593,7 +2594,7 @@ nmoe_status nmoe_router_topk(void* stream, const float* logits, const float* bia
   }
   return launch_router_topk(logits, bias, static_cast<int>(rows), experts, top_k, n_group,
                             topk_group, norm_topk_prob != 0, routed_scaling, top_index,
-                            top_weight, nullptr, nullptr,
+                            top_weight, nullptr, nullptr, device_sms(),
                             static_cast<cudaStream_t>(stream)) == cudaSuccess
              ? NMOE_OK
              : NMOE_ERR_INVALID_ARGUMENT;

@@ -364,7 +364,7 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               int k_blocks, uint8_t* sorted_packed, uint8_t* sorted_sf_tiled,
                               float* sorted_tensor_scale, float* sorted_weight,
                               int32_t* sorted_dest, int32_t* pair_row, int dest_stride,
-                              int32_t* error, LaunchStream stream) {
+                              int32_t* error, int num_sms, LaunchStream stream) {
   if (pairs <= 0 || src.pairs_per_row <= 0 || src.pairs_per_row > 32 ||
       pairs % src.pairs_per_row != 0 || experts <= 0 || experts > kMaxPlanExperts ||
       tile_multiple < 1) {
@@ -373,9 +373,9 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
   constexpr int kWarps = kPlaceThreads / 32;
   // While pairs are few each gets a warp, then a row's pairs share what was read of it: 1536 pairs
   // took 8.8 us against 10.9 between events, 6018 pairs 12.9 against 10.8.
-  const int share = pairs <= 148 * 2 * kWarps ? src.pairs_per_row : 1;
+  const int share = pairs <= num_sms * 2 * kWarps ? src.pairs_per_row : 1;
   const int units = pairs / src.pairs_per_row * share;
-  const int blocks = std::min((units + kWarps - 1) / kWarps, 148 * 6);  // each pays for the scan
+  const int blocks = std::min((units + kWarps - 1) / kWarps, num_sms * 6);  // each pays for the scan
   const PlacedRows out{sorted_packed, sorted_sf_tiled, sorted_tensor_scale, sorted_weight,
                        sorted_dest, pair_row};
   launch_kernel(place_rows_kernel, blocks, kPlaceThreads, 0, stream, plan, src, pairs, share, experts,
@@ -389,7 +389,7 @@ cudaError_t launch_combine(const void* in, bool in_bf16, const void* parts, RowK
                            int32_t* error, LaunchStream stream) {
   if (rows <= 0 || hidden % 8 != 0 || top_k < 1) return cudaErrorInvalidValue;
   const size_t total = static_cast<size_t>(rows) * (hidden / 8);
-  const int blocks = static_cast<int>(std::min<size_t>((total + 255) / 256, 148 * 16));
+  const int blocks = stride_blocks(total, 256);
   if (in_bf16 && out_bf16) {
     launch_combine_t<true, true>(in, parts, parts_kind, rows, hidden, top_k, out, error, blocks, stream);
   } else if (in_bf16) {

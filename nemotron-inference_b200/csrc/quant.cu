@@ -558,11 +558,6 @@ __global__ void swizzle_kernel(const uint8_t* __restrict__ row_major, int rows, 
   }
 }
 
-int grid_for(size_t work, int threads) {
-  const size_t blocks = (work + threads - 1) / threads;
-  return static_cast<int>(blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks));
-}
-
 }  // namespace
 
 namespace {
@@ -570,10 +565,10 @@ namespace {
 // Rows up to which each gets a block: as many as are resident at once (1003 rows of 2688 12.3 us
 // either way, 1000 rows of 4096 28.7 with a warp each and 14.7 with a block; 4096 rows of 2688
 // 20.6 and 28.6).
-constexpr int kBlockRows = 148 * 8;
+constexpr int kBlockRowsPerSm = 8;
 
 template <bool BF16>
-void launch_norm_quant_t(int rows, LaunchStream stream, const void* in, int cols,
+void launch_norm_quant_t(int rows, int num_sms, LaunchStream stream, const void* in, int cols,
                          const float* norm_weight, float eps, float* normalized, uint8_t* packed,
                          uint8_t* sf_row_major, uint8_t* sf_tiled, int k_tiles,
                          float* tensor_scale, float* inv_rms, int32_t* zero, int zero_count) {
@@ -591,7 +586,7 @@ void launch_norm_quant_t(int rows, LaunchStream stream, const void* in, int cols
                   normalized, packed, sf_row_major, sf_tiled, k_tiles, tensor_scale, inv_rms,
                   word_scales, zero, zero_count);
   };
-  if (rows <= kBlockRows && cols <= 6144) {
+  if (rows <= kBlockRowsPerSm * num_sms && cols <= 6144) {
     if (cols <= 2048) {
       run_block(norm_quant_block_kernel<BF16, 1>);
     } else if (cols <= 4096) {
@@ -620,15 +615,15 @@ void launch_norm_quant_t(int rows, LaunchStream stream, const void* in, int cols
 cudaError_t launch_norm_quant(const void* in, bool in_bf16, int rows, int cols,
                               const float* norm_weight, float eps, float* normalized,
                               uint8_t* packed, uint8_t* sf_row_major, uint8_t* sf_tiled,
-                              int k_blocks, float* tensor_scale, LaunchStream stream,
+                              int k_blocks, float* tensor_scale, int num_sms, LaunchStream stream,
                               float* inv_rms, int32_t* zero, int zero_count) {
   if (rows <= 0 || cols <= 0 || cols % 16 != 0) return cudaErrorInvalidValue;
   if (in_bf16) {
-    launch_norm_quant_t<true>(rows, stream, in, cols, norm_weight, eps, normalized, packed,
+    launch_norm_quant_t<true>(rows, num_sms, stream, in, cols, norm_weight, eps, normalized, packed,
                               sf_row_major, sf_tiled, k_blocks * 4, tensor_scale, inv_rms, zero,
                               zero_count);
   } else {
-    launch_norm_quant_t<false>(rows, stream, in, cols, norm_weight, eps, normalized, packed,
+    launch_norm_quant_t<false>(rows, num_sms, stream, in, cols, norm_weight, eps, normalized, packed,
                                sf_row_major, sf_tiled, k_blocks * 4, tensor_scale, inv_rms, zero,
                               zero_count);
   }
@@ -642,7 +637,7 @@ cudaError_t launch_quant_matrix(const float* in, int rows, int cols, uint8_t* pa
   cudaError_t err = cudaMemsetAsync(amax_scratch, 0, sizeof(float), stream);
   if (err != cudaSuccess) return err;
   const size_t count = static_cast<size_t>(rows) * cols;
-  global_amax_kernel<<<grid_for(count, 256), 256, 0, stream>>>(in, count, amax_scratch);
+  global_amax_kernel<<<stride_blocks(count, 256), 256, 0, stream>>>(in, count, amax_scratch);
   const int grid = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
   norm_quant_kernel<false, false><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
       in, rows, cols, nullptr, 0.0f, nullptr, packed, sf_row_major, nullptr, 0, tensor_scale,
@@ -655,7 +650,7 @@ cudaError_t launch_dequant(const uint8_t* packed, const uint8_t* sf_row_major,
                            float* out, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0 || cols % 16 != 0) return cudaErrorInvalidValue;
   const size_t bytes = static_cast<size_t>(rows) * cols / 2;
-  dequant_kernel<<<grid_for(bytes, 256), 256, 0, stream>>>(packed, sf_row_major, tensor_scale,
+  dequant_kernel<<<stride_blocks(bytes, 256), 256, 0, stream>>>(packed, sf_row_major, tensor_scale,
                                                            per_row_scale, rows, cols, out);
   return cudaGetLastError();
 }
@@ -668,7 +663,7 @@ cudaError_t launch_swizzle_scales(const uint8_t* row_major, int rows, int cols, 
   const size_t padded = static_cast<size_t>((rows + 127) / 128) * 128 * k_tiles * 4;
   cudaError_t err = cudaMemsetAsync(tiled, 0, padded, stream);
   if (err != cudaSuccess) return err;
-  swizzle_kernel<<<grid_for(static_cast<size_t>(rows) * blocks, 256), 256, 0, stream>>>(
+  swizzle_kernel<<<stride_blocks(static_cast<size_t>(rows) * blocks, 256), 256, 0, stream>>>(
       row_major, rows, blocks, k_tiles, tiled);
   return cudaGetLastError();
 }

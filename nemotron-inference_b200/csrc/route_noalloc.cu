@@ -84,7 +84,7 @@ extern "C" nmoe_status nmoe_route_tokens_noalloc(
   float* normalized = scratch;
   float* logits = scratch + kMaxNormalizedFloats;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  const int r = static_cast<int>(rows);
+  const int r = static_cast<int>(rows), sms = nmoe::device_sms();
   // Nothing in the scratch has to start at zero: both regions are fully
   // written for `rows` rows before they are read.
   // a launcher that rejects its arguments says cudaErrorInvalidValue; anything else
@@ -96,12 +96,12 @@ extern "C" nmoe_status nmoe_route_tokens_noalloc(
   };
   nmoe_status status = status_of(nmoe::launch_norm_quant(
       input, dtype == NMOE_BF16, r, hidden, norm_weight, epsilon, normalized, nullptr, nullptr,
-      nullptr, 0, nullptr, stream));
+      nullptr, 0, nullptr, sms, stream));
   if (status != NMOE_OK) return status;
   status = status_of(
-      nmoe::launch_router_logits(normalized, gate, nullptr, r, experts, hidden, logits, stream));
+      nmoe::launch_router_logits(normalized, gate, nullptr, r, experts, hidden, logits, sms, stream));
   if (status != NMOE_OK) return status;
   return status_of(nmoe::launch_router_topk(logits, bias, r, experts, top_k, n_group, topk_group,
                                             norm_topk_prob != 0, routed_scaling, top_index,
-                                            top_weight, nullptr, nullptr, stream));
+                                            top_weight, nullptr, nullptr, sms, stream));
 }

@@ -233,13 +233,13 @@ router_topk_kernel(const float* logits, const float* __restrict__ bias, int expe
 
 cudaError_t launch_router_logits(const float* normalized, const float* gate,
                                  const float* logit_offset, int rows, int experts, int hidden,
-                                 float* logits, cudaStream_t stream) {
+                                 float* logits, int num_sms, cudaStream_t stream) {
   if (rows <= 0 || experts <= 0 || hidden <= 0) return cudaErrorInvalidValue;
   if (rows >= 256 && experts % 16 == 0) {
     const int warps = ((rows + 1) / 2) * (experts / 16);
     router_logits_kernel<2, 16><<<(warps + kWarps - 1) / kWarps, kWarps * 32, 0, stream>>>(
         normalized, gate, logit_offset, rows, experts, hidden, logits);
-  } else if (experts % 4 == 0 && rows * (experts / 4) >= 148 * kWarps) {
+  } else if (experts % 4 == 0 && rows * (experts / 4) >= num_sms * kWarps) {
     // four experts per warp once that still gives every SM a block
     const int warps = rows * (experts / 4);
     router_logits_kernel<1, 4><<<(warps + kWarps - 1) / kWarps, kWarps * 32, 0, stream>>>(
@@ -263,12 +263,13 @@ bool router_topk_arguments_valid(int rows, int experts, int top_k, int n_group, 
 cudaError_t launch_router_topk(const float* logits, const float* bias, int rows, int experts,
                                int top_k, int n_group, int topk_group, bool norm_topk_prob,
                                float routed_scaling, int32_t* top_index, float* top_weight,
-                               int32_t* expert_counts, int32_t* position, LaunchStream stream) {
+                               int32_t* expert_counts, int32_t* position, int num_sms,
+                               LaunchStream stream) {
   if (!router_topk_arguments_valid(rows, experts, top_k, n_group, topk_group)) {
     return cudaErrorInvalidValue;
   }
   auto run = [&](auto kernel, int per_expert) {
-    const int threads = rows <= 148 ? per_expert : 128;
+    const int threads = rows <= num_sms ? per_expert : 128;
     launch_kernel(kernel, rows, threads, 0, stream, logits, bias, experts, top_k, n_group, topk_group,
                                               norm_topk_prob, routed_scaling, top_index, top_weight,
                                               expert_counts, position);

@@ -809,7 +809,7 @@ cudaError_t launch_router_fast_logits(const void* x, bool x_bf16, const float* i
 cudaError_t launch_fold_gate(const __nv_bfloat16* gate, const float* norm_weight, int experts,
                              int hidden, __nv_bfloat16* planes, cudaStream_t stream) {
   if (experts <= 0 || hidden <= 0) return cudaErrorInvalidValue;
-  fold_gate_kernel<<<148 * 4, 256, 0, stream>>>(gate, norm_weight, experts, hidden, planes);
+  fold_gate_kernel<<<stride_blocks(static_cast<size_t>(experts) * hidden, 256), 256, 0, stream>>>(gate, norm_weight, experts, hidden, planes);
   return cudaGetLastError();
 }
 
