@@ -7,7 +7,7 @@
 // SwizzleRowMajorNvfp4ScalesForExecution
 // (runtime/src/backend/nvfp4_scale_layout.cpp:68-87) with one pass per row.
 //
-// One warp owns one row.  The sum of squares reproduces the reference kernel's
+// A warp or a block owns a row.  The sum of squares reproduces the reference kernel's
 // association exactly (256 strided FMA partials, halving tree), so that the
 // normalised activations -- and therefore every FP4 code derived from them --
 // are a pure function of the input bits.  inv_rms is 1/sqrt(mean+eps) with two
@@ -203,9 +203,8 @@ norm_quant_kernel(const void* in, int rows, int cols,
 
 // norm_quant_kernel for rows of up to ITERS * 256 elements, one tensor scale per row: the row
 // is read once and stays in registers (as FP32) through the three phases -- sum of squares,
-// maximum, codes -- which the general kernel above re-reads it for.  For batches whose rows are as
-// many as the warps that fit on the GPU; 4096 rows of 2688 took 26.5 us with the general kernel and
-// take 23.2, 16384 rows 61 either way.
+// maximum, codes -- which the general kernel above re-reads it for.  Issue-bound; 4096 rows of 2688
+// 23.5 us with the general kernel, 18.4 so, 16384 rows 63 and 59.
 template <bool BF16, int ITERS>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 norm_quant_row_kernel(const void* in, int rows, int cols,
@@ -562,10 +561,30 @@ __global__ void swizzle_kernel(const uint8_t* __restrict__ row_major, int rows, 
 
 namespace {
 
-// Rows up to which each gets a block: as many as are resident at once (1003 rows of 2688 12.3 us
-// either way, 1000 rows of 4096 28.7 with a warp each and 14.7 with a block; 4096 rows of 2688
-// 20.6 and 28.6).
-constexpr int kBlockRowsPerSm = 8;
+// Which kernel takes a batch, by measurement (between events, bf16 rows with RMSNorm unless it says
+// otherwise, us).
+//
+// Rows of up to kRegisterCols columns: a block each for few rows, the register kernel for more, which
+// is the one that reads a row once and needs no shared memory.  2688 columns: 300 FP32 rows 8.3 by
+// blocks and 11.2 in registers, 600 bf16 rows 10.3 and 10.5, 1184 rows 13.1 and 11.3.  Its steps are
+// unrolled, so a row pays for all of them: it comes in four lengths, each of which is faster than the
+// general kernel or level with it where it is used (16384 rows of 1280 columns: 6 steps 28.7,
+// 11 steps 45, general 32.8; of 2048: 8 steps 49, general 48; of 2688: 11 steps 59, general 63).
+//
+// Longer rows do not fit the registers (16384 rows of 4096: 16 steps 131, blocks 96, general 89; of
+// 5376: 21 steps 179, blocks 137, general 114).  FP32 rows always get blocks (of 4096: 103 against
+// 147; of 5376 without RMSNorm 97 against 134), bf16 rows up to 24 per SM (2048 rows of 4096: 18.4
+// against 20.5, 4096 rows 30.3 against 30.8; 4096 rows of 5376: 40.2 against 38.1).
+constexpr int kRegisterCols = 11 * 256;
+constexpr int kBlockCols = 6144;
+constexpr int kBlockRowsPerSm = 6;
+constexpr int kLongBlockRowsPerSm = 24;
+
+bool block_per_row(bool bf16, int rows, int cols, int num_sms) {
+  if (cols > kBlockCols) return false;
+  if (cols <= kRegisterCols) return rows <= kBlockRowsPerSm * num_sms;
+  return !bf16 || rows <= kLongBlockRowsPerSm * num_sms;
+}
 
 template <bool BF16>
 void launch_norm_quant_t(int rows, int num_sms, LaunchStream stream, const void* in, int cols,
@@ -586,7 +605,7 @@ void launch_norm_quant_t(int rows, int num_sms, LaunchStream stream, const void*
                   normalized, packed, sf_row_major, sf_tiled, k_tiles, tensor_scale, inv_rms,
                   word_scales, zero, zero_count);
   };
-  if (rows <= kBlockRowsPerSm * num_sms && cols <= 6144) {
+  if (block_per_row(BF16, rows, cols, num_sms)) {
     if (cols <= 2048) {
       run_block(norm_quant_block_kernel<BF16, 1>);
     } else if (cols <= 4096) {
@@ -595,14 +614,13 @@ void launch_norm_quant_t(int rows, int num_sms, LaunchStream stream, const void*
       run_block(norm_quant_block_kernel<BF16, 3>);
     }
   } else if (cols <= 4 * 256) {
-    // the row lives in registers (8 floats per lane and iteration); longer rows are read three times
     run_row(norm_quant_row_kernel<BF16, 4>);
-  } else if (cols <= 11 * 256) {
+  } else if (cols <= 6 * 256) {
+    run_row(norm_quant_row_kernel<BF16, 6>);
+  } else if (cols <= 8 * 256) {
+    run_row(norm_quant_row_kernel<BF16, 8>);
+  } else if (cols <= kRegisterCols) {
     run_row(norm_quant_row_kernel<BF16, 11>);
-  } else if (cols <= 16 * 256) {
-    run_row(norm_quant_row_kernel<BF16, 16>);
-  } else if (cols <= 21 * 256) {
-    run_row(norm_quant_row_kernel<BF16, 21>);
   } else {
     launch_kernel(norm_quant_kernel<BF16, true>, grid, kWarpsPerBlock * 32, 0, stream, in, rows,
                   cols, norm_weight, eps, normalized, packed, sf_row_major, sf_tiled, k_tiles,

@@ -21,8 +21,10 @@ def small_layer(package, synthetic):
 
 # 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; a warp per pair
 # up to 2368 pairs (394 tokens); CTA pairs from 100 rows per expert (534 tokens); the shared expert in
-# the routed experts' launch up to 640; a block per row in the quantiser up to 1184
-@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 1184, 1185])
+# the routed experts' launch up to 640; a block per row in the quantiser up to 888, per token in the
+# exact selection up to 1024
+@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 888, 889, 1024, 1025,
+                                    1184, 1185])
 def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
     layer, data = small_layer
     x = synthetic.make_tokens(tokens, 512, seed=300 + tokens, device="cuda")
@@ -43,6 +45,24 @@ def test_quantiser_row_lengths(package, oracle, rows, cols):
     for got, expected in zip((packed, scales, ts), oracle.pack_nvfp4_per_row(x.numpy())):
         assert np.array_equal(got.cpu().numpy(), expected)
     assert np.array_equal(y.cpu().numpy(), oracle.rmsnorm(x.numpy(), w.numpy(), 1e-5))
+
+
+# 148 SMs: a block per row up to 888 rows of 2816 columns at most, register rows of 4, 6, 8 and 11 steps
+# of 256 from there; longer bf16 rows a block each up to 3552, then three reads of the row
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(888, 2816), (889, 1024), (889, 1040), (889, 1536), (889, 1552),
+                                       (889, 2048), (889, 2064), (889, 2816), (889, 2832),
+                                       (3552, 2832), (3553, 2832), (3553, 6144)])
+def test_quantiser_kernel_lines(package, oracle, rows, cols, dtype):
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(rows + cols)).to(dtype)
+    w = torch.linspace(0.9, 1.1, cols)
+    packed, scales, ts, _ = package.quantize_nvfp4(x.cuda(), per_row=True, swizzled=True)
+    y = package.rmsnorm(x.cuda(), w.cuda(), 1e-5)
+    torch.cuda.synchronize()
+    x = x.to(torch.float32).numpy()
+    for got, expected in zip((packed, scales, ts), oracle.pack_nvfp4_per_row(x)):
+        assert np.array_equal(got.cpu().numpy(), expected)
+    assert np.array_equal(y.cpu().numpy(), oracle.rmsnorm(x, w.numpy(), 1e-5))
 
 
 def test_two_layers_beside_each_other(package, synthetic):
