@@ -960,11 +960,15 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
 // format, which counts for few rows: up to four are no slower on a large W (22 MB of FP8 against
 // 110 MB of slices for the checkpoint's shared_up).  A short W costs no more than widening and
 // multiplying its values, which up to 90 million products is less than the three launches of the
-// second take (255 rows of a 128 x 2688 gate: 24 us against 31 between events, 40 rows of a
-// 512 x 4096 gate 27 either way).
+// second take (between events, us, FP64 against integers: 128 x 2688, 261 rows, 90 million 26.7 and
+// 29.7, 348 rows, 120 million 35.5 and 31.8; 512 x 2688, 65 rows 26.6 and 31.2, 87 rows 34.7 and
+// 29.8; 512 x 4096, 38 rows, 80 million 28.8 and 27.9; 64 x 4096, 343 rows 33.0 and 33.8, 457 rows
+// 34.6 and 33.8; 384 x 1024, 228 rows 26.7 and 26.6, 305 rows 33.0 and 27.4).
+constexpr long long kMostFp64Products = 90000000;
 bool exact_prefers_gemv(int rows, int N, int K, int num_sms) {
   if (rows <= 4) return true;
-  return gemv_by_blocks(rows, N, num_sms) && static_cast<long long>(rows) * N * K <= 90000000ll;
+  return gemv_by_blocks(rows, N, num_sms) &&
+         static_cast<long long>(rows) * N * K <= kMostFp64Products;
 }
 
 cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,

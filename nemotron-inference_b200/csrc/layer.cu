@@ -1463,8 +1463,11 @@ void run_ffn(nmoe_layer* L, bool unfused, const WeightStack& up, const WeightSta
 constexpr int kSharedInLaunchTokens = 640;
 
 // Routed rows per expert (on average) up to which csrc/expert_stream.cu takes them: with more, most
-// experts have a second row tile and their weights would be read twice (whole pass at 96 rows 250 us,
-// at 141 rows 321 with CTA pairs against 370).
+// experts have a second row tile and their weights would be read twice.  Where the two meet depends
+// on how even the routing is, which the host does not know: whole pass over bf16 rows, this kernel
+// against CTA pairs, uniform 96 rows 262 us and 288, 120 rows 322 and 328, 144 rows 397 and 356;
+// popular and unpopular experts 56 rows 218 and 230, 80 rows 250 and 248, 120 rows 331 and 309.  At
+// 100 rows neither loses more than 8 % (273 and 297, 297 and 276).
 constexpr int kStreamRowsPerExpert = 100;
 
 // Which kernel takes `pairs` routed rows.

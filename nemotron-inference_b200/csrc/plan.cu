@@ -371,9 +371,13 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
     return cudaErrorInvalidValue;
   }
   constexpr int kWarps = kPlaceThreads / 32;
-  // While pairs are few each gets a warp, then a row's pairs share what was read of it: 1536 pairs
-  // took 8.8 us against 10.9 between events, 6018 pairs 12.9 against 10.8.
-  const int share = pairs <= num_sms * 2 * kWarps ? src.pairs_per_row : 1;
+  // While there is little to write each pair gets a warp, then a row's pairs share what was read of
+  // it.  The two meet at about 6 MB (between events; six pairs a row of 1512 bytes each: 3072 pairs
+  // 9.9 us against 10.3, 4608 10.2 against 10.3, 6144 12.1 against 10.3; 22 pairs of 576 bytes: 5632
+  // pairs 10.2 against 12.3, 9856 12.2 against 12.3, 14080 14.3 against 12.3).
+  constexpr size_t kPairBytesPerSm = 40 * 1024;
+  const size_t bytes = static_cast<size_t>(pairs) * (cols / 2 + cols / 16);
+  const int share = bytes <= kPairBytesPerSm * num_sms ? src.pairs_per_row : 1;
   const int units = pairs / src.pairs_per_row * share;
   const int blocks = std::min((units + kWarps - 1) / kWarps, num_sms * 6);  // each pays for the scan
   const PlacedRows out{sorted_packed, sorted_sf_tiled, sorted_tensor_scale, sorted_weight,

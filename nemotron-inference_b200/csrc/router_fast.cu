@@ -477,7 +477,6 @@ router_folded_logits_kernel(const __grid_constant__ CUtensorMap tmap_x,
 // ---------------------------------------------------------------------------
 constexpr int kSelectWarps = 4;
 constexpr int kSelectPerLane = 8;  // experts <= 256
-constexpr int kSelectWholeBlockRows = 1024;
 
 __device__ __forceinline__ float sigmoid_exact(float v) {
   // Sigmoid of expert_layer.cpp:129-136 with exp evaluated in double
@@ -539,6 +538,11 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 // per pass over the row (at least top_k, so that one pass is the rule).
 // Measured, 128 experts, hidden 2688, bf16 in: 256 tokens 35 -> 17 us, 16384 tokens
 // 143 -> 119 us.
+// Up to kSelectWholeBlockRows tokens the block form is the faster one (us, block against warp; 128
+// experts of 2688, top-6: 768 tokens 19.8 and 30.2, 1280 28.7 and 31.0, 1536 28.4 and 29.3, 2048 34.9
+// and 29.3; 256 experts, top-8: 1280 35.7 and 43.9, 1536 45.6 and 41.9; 128 experts of 4096: 1280
+// 31.0 and 36.6, 2048 38.5 and 35.6).
+constexpr int kSelectWholeBlockRows = 1280;
 template <bool IN_BF16, int WARPS, int BATCH>
 __global__ void __launch_bounds__(kSelectWarps * 32)
 router_select_exact_kernel(float* __restrict__ logits, int splits, const void* __restrict__ x,

@@ -19,12 +19,11 @@ def small_layer(package, synthetic):
     layer.close()
 
 
-# 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; a warp per pair
-# up to 2368 pairs (394 tokens); CTA pairs from 100 rows per expert (534 tokens); the shared expert in
+# 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; CTA pairs from 100 rows per expert (534 tokens); the shared expert in
 # the routed experts' launch up to 640; a block per row in the quantiser up to 888, per token in the
-# exact selection up to 1024
-@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 888, 889, 1024, 1025,
-                                    1184, 1185])
+# exact selection up to 1280
+@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 888, 889, 1184, 1185,
+                                    1280, 1281])
 def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
     layer, data = small_layer
     x = synthetic.make_tokens(tokens, 512, seed=300 + tokens, device="cuda")
@@ -45,6 +44,21 @@ def test_quantiser_row_lengths(package, oracle, rows, cols):
     for got, expected in zip((packed, scales, ts), oracle.pack_nvfp4_per_row(x.numpy())):
         assert np.array_equal(got.cpu().numpy(), expected)
     assert np.array_equal(y.cpu().numpy(), oracle.rmsnorm(x.numpy(), w.numpy(), 1e-5))
+
+
+def test_placing_on_both_sides_of_its_line(package, synthetic):
+    # a warp per pair up to 40 KB of pairs per SM: 5262 pairs of 1152 bytes, 877 tokens
+    cfg = synthetic.baseline_config(max_tokens=1024, experts=32, hidden=2048, routed=64, shared=64)
+    data = synthetic.make_layer(cfg, seed=84, device="cuda", norm_weight_uniform=True)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (877, 878):
+        x = synthetic.make_tokens(tokens, 2048, seed=tokens, device="cuda")
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        assert layer.run(x, out), layer.last_error
+        rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+        assert rep.ok(), rep.summary()
+    layer.close()
 
 
 # 148 SMs: a block per row up to 888 rows of 2816 columns at most, register rows of 4, 6, 8 and 11 steps
