@@ -63,3 +63,75 @@ def test_an_fp8_input_scale_of_zero_is_the_smallest_scale(package, synthetic):
     for zero, smallest in zip(outs[:2], outs[2:]):
         assert torch.equal(zero[1], smallest[1])
         assert torch.equal(zero[0], smallest[0])
+
+
+def _contraction_layer(package, synthetic, hidden, shared, seed, experts=32):
+    cfg = synthetic.baseline_config(max_tokens=128, experts=experts, hidden=hidden, routed=64,
+                                    shared=shared, latent=64)
+    data = synthetic.make_layer(cfg, seed=seed, device="cuda", norm_weight_uniform=True,
+                                latent_family="fp32", shared_up_family="fp8",
+                                shared_down_family="fp32")
+    return cfg, data
+
+
+def test_router_on_both_sides_of_the_product_line(package, synthetic):
+    # 512 x 4096: FP64 up to 90 million products, 42 rows
+    cfg, data = _contraction_layer(package, synthetic, 4096, 64, 94, experts=512)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (42, 43):
+        x = synthetic.make_tokens(tokens, 4096, seed=tokens, device="cuda")
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        assert layer.run(x, out), layer.last_error
+        rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+        assert rep.ok(), rep.summary()
+        assert rep.logits_max_diff == 0.0 and rep.latent_max_diff == 0.0
+    layer.close()
+
+
+def test_linears_of_the_checkpoints_lengths(package, synthetic, oracle):
+    # contractions over 4096 and 5376: the shared expert's FP64 sums, rounded once
+    cfg, data = _contraction_layer(package, synthetic, 4096, 5376, 95)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    ocfg, ow = helpers.oracle_config(cfg), helpers.oracle_weights(data)
+    for tokens in (3, 65):
+        x = synthetic.make_tokens(tokens, 4096, seed=tokens, device="cuda")
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        assert layer.run(x, out), layer.last_error
+        trace = layer.trace(tokens)
+        y = trace.normalized_input.cpu().numpy()
+        up = oracle.router_logits(oracle.fp8_round_trip(y, ow.shared_up_input_scale),
+                                  ow.shared_up_dense)
+        hidden = np.where(up > 0, up * up, np.float32(0.0))
+        want = oracle.router_logits(hidden, ow.shared_down_dense)
+        assert np.array_equal(trace.shared_output.cpu().numpy(), want)
+    layer.close()
+
+
+def test_longest_contraction_with_digits_of_one_sign(package, synthetic):
+    # 16384 equal products per sum, so that the digits' products add up instead of cancelling: the
+    # level sums reach for 32 bits, and the sum is a power of two times one product, exact in FP64.
+    # Rows of alternating sign sum to zero, which the rounding test leaves to the FP64 sum.
+    cfg, data = _contraction_layer(package, synthetic, 192, 16384, 96)
+    up = torch.zeros((16384, 192), device="cuda")
+    up[:, 0] = 1.0
+    column = torch.randn((192, 1), generator=torch.Generator(device="cuda").manual_seed(97),
+                         device="cuda")
+    down = column.expand(192, 16384).contiguous()
+    down[::16, 1::2] *= -1.0
+    data.bindings.shared_up_linear = package.DenseLinear(up)
+    data.bindings.shared_down_linear = package.DenseLinear(down)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (2, 16, 65, 128):
+        x = synthetic.make_tokens(tokens, 192, seed=tokens, device="cuda").to(torch.float32)
+        x[:, 0] = x[:, 0].abs() + 0.5
+        out = torch.empty_like(x)
+        assert layer.run(x, out), layer.last_error
+        trace = layer.trace(tokens)
+        value = trace.normalized_input[:, :1]
+        want = (16384.0 * (value * value).double() * column.double().T).float()
+        want[:, ::16] = 0.0
+        assert torch.equal(trace.shared_output, want)
+    layer.close()
