@@ -1516,7 +1516,7 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
   out.dest_row = L->a_dest.as<int32_t>();
   out.row_weight = L->a_weight.as<float>();
   out.segments = segments;
-  if (routed_class == kClassStream && !L->unfused && !L->stage_timing) {
+  if (routed_class == kClassStream && !L->unfused) {
     StreamFfn ffn;
     ffn.up = &L->up;
     ffn.down = &L->down;
@@ -1529,6 +1529,7 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
     ffn.out = out;
     ffn.row_slots = L->max_row_tiles;
     run_stream(&ffn, shared, L->stream_counts, error, L->num_sms, stream);
+    L->mark(6, stream);  // (one launch: its time is that of the up projections' stage)
     return;
   }
   FfnBuffers buffers{L->h_packed.as<uint8_t>(), L->h_sf.as<uint8_t>(), L->h_ts.as<float>(),
@@ -1673,7 +1674,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   // Small batches bound by reading the weights run both kinds of expert in one launch, the others
   // fork the shared expert onto a stream of its own.
   const bool one_launch = routed_tile_class(L, tokens * K) == kClassStream && !L->unfused &&
-                          !L->stage_timing && !L->shared_down_dense.present &&
+                          !L->shared_down_dense.present &&
                           (L->latent_mode || tokens <= kSharedInLaunchTokens);
   const bool fork = L->side_stream != nullptr && !L->stage_timing && !one_launch &&
                     tokens <= L->fork_max_tokens && !L->latent_mode && !dense_shared;
@@ -1707,6 +1708,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
           shared_stream_ffn(L, chain, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
       routed_experts(L, chain, source, tokens * K, K, L->parts.as<void>(), kRowF32, RowSegments(),
                      &shared);
+      for (int i = 7; i <= 9; ++i) L->mark(i, stream);
     } else {
       routed_experts(L, chain, source, tokens * K, K, L->parts.as<void>(), kRowF32);
       L->mark(7, stream);
@@ -1741,7 +1743,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   }
   L->mark(7, stream);
   if (one_launch) {
-    // nothing left to wait for
+    L->mark(8, stream);  // nothing left to wait for
   } else if (fork) {
     NMOE_CUDA(cudaStreamWaitEvent(stream, L->shared_done, 0));
   } else {

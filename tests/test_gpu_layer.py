@@ -1,5 +1,5 @@
-"""GPU parity of the whole MoE layer against the CPU oracle: configs[1] (decode sizes),
-configs[2] (skewed prefill) and reduced-size variants, through ExpertLayerSlice."""
+"""GPU parity of the whole MoE layer against the CPU oracle: decode sizes, skewed
+prefill and reduced-size variants, through ExpertLayerSlice."""
 import numpy as np
 import pytest
 import torch
@@ -162,7 +162,7 @@ def test_prefill_skewed_config2(package, synthetic):
 
 
 def test_layer_stack_matches_oracle_applied_layer_by_layer(package, synthetic, oracle):
-    # configs[4] in miniature: independently seeded layers, RMSNorm weight ~U(0.9, 1.1),
+    # a stack in miniature: independently seeded layers, RMSNorm weight ~U(0.9, 1.1),
     # the FP32 hidden state handed from layer to layer (the caller loop of
     # runtime/src/api/single_token_forward_model.cpp:588-656).  Every layer is gated on the
     # full parity report with the DEVICE output of the previous layer as its input, so a
@@ -200,3 +200,26 @@ def test_layer_stack_matches_oracle_applied_layer_by_layer(package, synthetic, o
     assert mixed.sync_status() == 0 and torch.equal(got, want)
     for layer in layers:
         layer.close()
+
+
+def test_stage_times_are_of_the_launches_a_pass_makes(package, synthetic):
+    # all expert projections in one launch, whose time is the first stage's
+    cfg = synthetic.baseline_config(max_tokens=1024, experts=32)
+    data = synthetic.make_layer(cfg, seed=31, device="cuda")
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (40, 500):
+        x = synthetic.make_tokens(tokens, cfg.hidden_size, seed=32, device="cuda")
+        want, out = torch.empty_like(x), torch.empty_like(x)
+        assert layer.run(x, want), layer.last_error
+        layer.enable_stage_timing(True)
+        for _ in range(3):
+            layer.run_async(x, out)
+            times = layer.stage_times_ms()
+        layer.enable_stage_timing(False)
+        print(tokens, times)
+        assert torch.equal(out, want)
+        assert all(ms >= 0.0 for ms in times.values())
+        for name in ("routed_down_gemm", "shared_up_gemm", "shared_down_gemm"):
+            assert times[name] < 0.25 * times["routed_up_gemm"]
+    layer.close()
