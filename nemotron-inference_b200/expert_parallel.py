@@ -590,7 +590,7 @@ def bench_main(args, package, synthetic, peaks, flush_buf, dist_module, bench_mo
         try:
             stack_report = stack_workload(args, package, synthetic, flush_buf, dist_module)
         except Exception as error:  # noqa: BLE001 - a side workload must not lose the line
-            stack_report = {"workload": "configs[4]", "unavailable": str(error)[:300]}
+            stack_report = {"workload": "stack of MoE layers", "unavailable": str(error)[:300]}
     sent = capacity * (world - 1)
     if transport == "window":
         exchange = {
@@ -615,7 +615,7 @@ def bench_main(args, package, synthetic, peaks, flush_buf, dist_module, bench_mo
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
         "dtype": "nvfp4 (e2m1 x ue4m3, fp32 accumulate)", "data": "synthetic",
-        "config": {"workload": f"configs[3]: T={tokens_total} tokens, uniform routing, hidden 2688, "
+        "config": {"workload": f"T={tokens_total} tokens, uniform routing, hidden 2688, "
                                f"128 experts x 1856 top-6 ({128 // world} per GPU), shared 3712 "
                                "replicated, bf16 in/out",
                    "global_tokens": tokens_total, "parallelism": f"ep{world}",
@@ -785,7 +785,7 @@ def stack_workload(args, package, synthetic, flush_buf, dist_module, layers: int
         engine.stages.detach_windows()
         engine.stages.layer.close()
     torch.cuda.empty_cache()
-    return {"workload": f"configs[4]: {layers} MoE layers, residual + RMSNorm per layer, "
+    return {"workload": f"stack of {layers} MoE layers, residual + RMSNorm per layer, "
                         f"expert-parallel over {world} GPUs",
             "decode_batch": decode, "prefill_chunk": prefill,
             "segment_capacity": capacity,

@@ -90,7 +90,7 @@ def _normal(shape, std, generator, device):
 
 def zipf_logit_offset(experts: int, seed: int, head: float = 0.2, tail: float = 2.5,
                       s: float = 1.1) -> torch.Tensor:
-    """Per-expert gate-logit offset that skews the expert load (configs[2]).  A seeded
+    """Per-expert gate-logit offset that skews the expert load.  A seeded
     random ranking gives each expert a Zipf(s) popularity p ~ rank^-s; the offset is
     log p centred on its mean, with the popular side scaled by `head` and the unpopular
     side by `tail`.  With ~N(0,1) logits and top-6 of 128 the defaults give a hottest
@@ -200,7 +200,7 @@ def make_tokens(tokens: int, hidden: int, seed: int, device="cpu") -> torch.Tens
 
 
 def make_ffn_weights(hidden: int, intermediate: int, seed: int, device="cpu"):
-    """one routed expert, W_up [I, H] and W_down [H, I] ~N(0, 0.02)."""
+    """One routed expert, W_up [I, H] and W_down [H, I] ~N(0, 0.02)."""
     dev = torch.device(device)
     g = torch.Generator(device=dev).manual_seed(seed)
     up = quantize_weight(_normal((intermediate, hidden), 0.02, g, dev))

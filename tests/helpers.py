@@ -9,7 +9,7 @@ import torch
 
 import __graft_entry__ as entry
 
-MAX_ABS_TOL = 2e-2      # north-star tolerance on the layer output
+MAX_ABS_TOL = 2e-2      # tolerance on the layer output
 COSINE_TOL = 0.9995
 # An intermediate FP4 code or scale byte of the device may differ from the oracle's only
 # where a shift of the up-projection's pre-activation by at most this many accumulation-

@@ -1,4 +1,4 @@
-"""GPU parity of one routed-expert NVFP4 FFN (configs[0]): y = W_down relu(W_up x)^2 with
+"""GPU parity of one routed-expert NVFP4 FFN: y = W_down relu(W_up x)^2 with
 dynamic per-16-block activation quantisation, against the reference's host FP32
 dequantise-then-matmul path as restated by the oracle."""
 import numpy as np

@@ -175,7 +175,7 @@ def test_synthetic_weight_quantiser_matches_oracle(oracle, synthetic):
     assert np.array_equal(packed.numpy(), op)
     assert np.array_equal(scales.numpy(), os_)
     assert np.float32(ts.item()) == np.float32(ots)
-    # global scale = amax / (6*448)
+    # one expert: global scale = amax / (6*448)
     assert np.float32(ots) == np.float32(w.abs().max().item()) / np.float32(2688.0)
 
 
