@@ -45,8 +45,8 @@ SHARED_BYTES = 2 * (S * H // 2 + S * H // 16 + 4)
 
 
 def load_traffic_capture():
-    """DRAM traffic of one routed up-GEMM launch as ncu counted it on a reduced token
-    count (the file says which command produced it), or None."""
+    """DRAM traffic of one routed up-GEMM launch as ncu counted it (the file says at how many
+    rows and in which capture), or None."""
     path = os.path.join(ROOT, "profiles", "grouped_gemm_up_traffic.json")
     try:
         return json.load(open(path))
@@ -435,17 +435,19 @@ def main():
     stages = stage_profile(layer, x, out, max(3, args.steps // 2), flush_buf)
 
     up_flops = tokens * K * 2 * H * I  # one GEMM: 2 * M * N * K
-    # DRAM traffic of one routed up-GEMM launch: ncu's count on a reduced token count,
-    # scaled to this launch (the weights are read once whatever the row count is, the rest
-    # grows with the rows)
+    # DRAM traffic of one routed up-GEMM launch: ncu's count, for another number of rows than it was
+    # taken at scaled to this launch (the weights are read once whatever the row count is, the
+    # rest grows with the rows)
     capture = load_traffic_capture()
     up_traffic, traffic_note = None, "no capture file under profiles/"
     if capture is not None:
         counted = capture["dram_bytes_read"] + capture["dram_bytes_write"]
         up_traffic = E * UP_BYTES + (counted - E * UP_BYTES) * (tokens * K) / float(capture["rows"])
-        traffic_note = (f"modelled: ncu dram__bytes_read+write of this kernel at "
-                        f"{capture['rows']} rows ({counted / 1e6:.1f} MB), weight bytes "
-                        f"({E * UP_BYTES / 1e6:.1f} MB, read once) kept, the rest scaled by rows")
+        traffic_note = (f"ncu dram__bytes_read+write of this kernel at {capture['rows']} rows "
+                        f"({counted / 1e6:.1f} MB)")
+        if capture["rows"] != tokens * K:
+            traffic_note += (f", weight bytes ({E * UP_BYTES / 1e6:.1f} MB, read once) kept, the "
+                             "rest scaled by rows")
     up_tf = up_flops / (stages["routed_up_gemm"] * 1e-3) / 1e12
     ceilings = tensor_peaks(peaks)
     fp4_peak = ceilings["fp4_4x_burst_bf16"]

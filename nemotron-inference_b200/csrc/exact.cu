@@ -211,9 +211,10 @@ void launch_slices(const void* in, int rows, int K, float scale, int tile_rows, 
 // MMA of up to 256 columns multiplies digit i with several token digits and adds each product to
 // the level it belongs to; A is read once for all of them.  A CTA takes one tile, or a share of
 // its K range, and stores the levels put together as doubles.
-// Bound by shared memory (64 token rows: 60 KB written and 154 KB read per 64-byte stage, 1680 cycles
-// at 128 a cycle, against 1400 of MMA).  The checkpoint's shared_up (5376 x 4096), 1000 rows: 13,800 ->
-// 370 us with the two kernels around it; 40 rows: 381 -> 44 us.
+// Bound by the MMAs (the checkpoint's shared_up, 5376 x 4096, 1000 rows, under ncu: a stage takes 1740
+// cycles, 1420 of them on the tensor pipe, and its 672 tiles are 4.54 waves of 148 SMs; shared memory
+// is at 32 % of its read and 13 % of its write rate).  With the two kernels around it 13,800 -> 370 us;
+// 40 rows 381 -> 44 us.
 // ---------------------------------------------------------------------------
 constexpr int kExactStages = 3;
 constexpr int kExactThreads = 6 * 32;

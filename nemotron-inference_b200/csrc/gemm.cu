@@ -69,7 +69,10 @@ __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, i
 // What bounds a K block is shared memory: at 128 bytes a cycle the copies of a 128 x 208 tile of
 // one CTA write 49 KB (380 cycles) and its MMAs read 43 KB (330), for 416 cycles of MMA.  A pair
 // stages each weight tile once for 256 rows (half in each CTA): 35 KB written and 30 KB read per
-// CTA and K block.
+// CTA and K block.  What is left to wait for is the delivery from L2 to the SMs: 3.16 GB in 254 to
+// 258 us at 16384 tokens, 12 TB/s, at SM clocks of 1.97 and of 1.56 GHz alike (tensor pipe 60 % busy
+// at the latter); the down projection 3.33 GB in 284 us beside 0.5 GB of row stores.  At 4096 tokens
+// it is HBM: 446 MB in 86.5 us, 0.79 of the copy rate.
 //
 // Roles per CTA: warp 0 loads (the CTA's own 128 activation rows, its half of the weight tile, the
 // scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues the scale
