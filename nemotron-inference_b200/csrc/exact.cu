@@ -458,7 +458,9 @@ constexpr int kFinishThreads = 256;
 //
 // B, in units of 2^(ea + ew): K * 2^-52 for the digit products of level 7 and beyond (two pairs of
 // digits up to 128 at level 7, one at level 8: K * 2^-53 * 1.01); 2^-39 for every value of the two
-// rows that its digits do not hold exactly; and |r| * 2^-50 for the roundings of the doubles.
+// rows that its digits do not hold exactly; and |r| * 2^-50 for the roundings of the doubles (three
+// of 2^-53: a sum of fewer than five levels is below 2^53).  The parts of a split sum may cancel, so
+// there it is their magnitudes that count, for those three and for every addition of a part.
 template <int KIND>
 __global__ void __launch_bounds__(kFinishThreads)
 exact_finish_kernel(const double* __restrict__ partial, int splits, int rows, int N, int K,
@@ -488,7 +490,12 @@ exact_finish_kernel(const double* __restrict__ partial, int splits, int rows, in
       const int e = a.exponent + w.exponent;
       r *= two_to(e - (12 + 8 * (kLevels - 1)));
       const double left_out = K + 8192.0 * (a.inexact + w.inexact);
-      const double bound = left_out * two_to(e - 52) + fabs(r) * 0x1p-50;
+      double bound = left_out * two_to(e - 52) + fabs(r) * 0x1p-50;
+      if (splits > 1) {
+        double magnitude = 0.0;
+        for (int s = 0; s < splits; ++s) magnitude += fabs(partial[i + s * count]);
+        bound += magnitude * two_to(e - (12 + 8 * (kLevels - 1)) - 53) * (splits + 7);
+      }
       const float low = static_cast<float>(r - bound), high = static_cast<float>(r + bound);
       decided = low == high;
       result = static_cast<float>(r);
