@@ -406,7 +406,8 @@ NMOE_API nmoe_status nmoe_ffn_create(const nmoe_nvfp4_matrix* up, const nmoe_nvf
 NMOE_API void nmoe_ffn_destroy(nmoe_ffn* ffn);
 /* input [rows][hidden] device FP32/bf16 -> output [rows][hidden] device FP32.
  * gemm_variant: 0 = choose by size, otherwise the kernel (for tests): 1 or 4 the CTA-pair GEMM
- * of large batches, 2 (rows <= 32) or 3 the streaming kernel of small ones. */
+ * of large batches, 2 or 3 the streaming kernel of small ones.  (2 and 4 name kernels that are gone;
+ * what 2 refused, more than 32 rows, it still refuses.) */
 NMOE_API nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream, const void* input,
                                   nmoe_dtype input_dtype, int64_t rows, float* output,
                                   int32_t gemm_variant);

@@ -831,6 +831,7 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
   if (rows > ffn->max_rows) return NMOE_ERR_CAPACITY;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   try {
+    // (2 was a kernel for few rows; the streaming kernel behind it now has no such limit)
     if (gemm_variant == 2 && rows > 32) return NMOE_ERR_INVALID_ARGUMENT;
     const TileClass tile_class =
         gemm_variant == 1 || gemm_variant == 4 ? kClassPair
