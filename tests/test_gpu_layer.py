@@ -202,10 +202,12 @@ def test_layer_stack_matches_oracle_applied_layer_by_layer(package, synthetic, o
         layer.close()
 
 
-def test_stage_times_are_of_the_launches_a_pass_makes(package, synthetic):
+@pytest.mark.parametrize("latent", [False, True])
+def test_stage_times_are_of_the_launches_a_pass_makes(package, synthetic, latent):
     # all expert projections in one launch, whose time is the first stage's
-    cfg = synthetic.baseline_config(max_tokens=1024, experts=32)
-    data = synthetic.make_layer(cfg, seed=31, device="cuda")
+    cfg = synthetic.baseline_config(max_tokens=1024, experts=32, latent=1024 if latent else 0)
+    data = synthetic.make_layer(cfg, seed=31, device="cuda", latent_family="fp8",
+                                shared_up_family="fp8" if latent else "nvfp4")
     layer = package.ExpertLayerSlice.create(cfg, data.bindings)
     assert layer is not None, package.ExpertLayerSlice.create_error
     for tokens in (40, 500):
