@@ -55,7 +55,7 @@ def load_traffic_capture():
 
 
 def tensor_peaks(peaks):
-    """No FP4 figure is measured on this pool.  The dense-FP4 ceiling is stated three
+    """No FP4 rate has been measured.  The dense-FP4 ceiling is stated three
     ways: 4 x the measured burst bf16 rate (the kernels here run a fraction of a
     millisecond at full clock, the burst case), 4 x the sustained rate, and the nominal
     9 PFLOP/s; `frac` uses the first."""
@@ -475,8 +475,8 @@ def main():
                      "traffic_note": traffic_note,
                      "peak_note": f"4 x {peaks['source']} burst dense bf16 "
                                   f"({peaks['bf16_tflops']} TF/s): the kernel runs ~0.3 ms at "
-                                  "full clock with no power cap, the burst case; no FP4 figure "
-                                  "is measured on this pool, the sustained and nominal "
+                                  "full clock with no power cap, the burst case; no FP4 rate "
+                                  "has been measured, the sustained and nominal "
                                   "ceilings are beside it",
                      "frac_of_4x_sustained_bf16": up_tf / ceilings["fp4_4x_sustained_bf16"],
                      "frac_of_nominal_9000": up_tf / ceilings["fp4_nominal"],
