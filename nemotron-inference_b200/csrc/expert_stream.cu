@@ -551,7 +551,11 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
               v[i + 3] = four.w;
             }
             if (ph.mode == kGemmUp) {
-              report_range(g, quantise_chunk(g, v, n, tile.row0 + from, row_scale, true));
+              uint32_t lo, hi, sf;
+              report_range(g, quantise_chunk(v, row_scale, lo, hi, sf));
+              *reinterpret_cast<uint2*>(hidden_codes(g, tile.row0 + from, n / 16)) =
+                  make_uint2(lo, hi);
+              *hidden_scale(g, tile.row0 + from, n / 16) = static_cast<uint8_t>(sf);
             } else if (row_dest != 0) {
               store_chunk(g, v, n, row_dest, row_scale, row_wt);
             }

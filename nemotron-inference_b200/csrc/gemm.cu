@@ -66,13 +66,10 @@ __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, i
 // CTA-pair kernel: one 256 x kPairBN tile per cluster of two CTAs
 // (tcgen05.mma.cta_group::2, M = 256).
 //
-// What bounds a K block is shared memory: at 128 bytes a cycle the copies of a 128 x 208 tile of
-// one CTA write 49 KB (380 cycles) and its MMAs read 43 KB (330), for 416 cycles of MMA.  A pair
-// stages each weight tile once for 256 rows (half in each CTA): 35 KB written and 30 KB read per
-// CTA and K block.  What is left to wait for is the delivery from L2 to the SMs: 3.16 GB in 254 to
-// 258 us at 16384 tokens, 12 TB/s, at SM clocks of 1.97 and of 1.56 GHz alike (tensor pipe 60 % busy
-// at the latter); the down projection 3.33 GB in 284 us beside 0.5 GB of row stores.  At 4096 tokens
-// it is HBM: 446 MB in 86.5 us, 0.79 of the copy rate.
+// What bounds a K block is what an SM takes in.  A pair stages each weight tile once for 256 rows (half
+// in each CTA), 35 KB per CTA and K block, and with the epilogue left out a K block takes 660 cycles, 54
+// bytes each, hardly less with half of the MMAs (98304 rows, up: 193 us and 187).  The rows stored by
+// the epilogue come on top of that: 221 us for up, 289 for down.  At 4096 tokens it is HBM: 446 MB in 86 us, 0.8 of the copy rate.
 //
 // Roles per CTA: warp 0 loads (the CTA's own 128 activation rows, its half of the weight tile, the
 // scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues the scale
@@ -82,7 +79,7 @@ __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, i
 // the loads of the partner name the leader's barrier.
 //
 // Measured, benchmark layer, up / down projection, against 128 x 208 tiles of single CTAs: 16384
-// tokens 334 / 405 -> 258 / 300 us, 8192 tokens 192 / 223 -> 152 / 170.
+// tokens 334 / 405 -> 221 / 284 us, 8192 tokens 192 / 223 -> 134 / 163.
 // ---------------------------------------------------------------------------
 constexpr int kPairBN = 208;
 constexpr int kPairBRows = kPairBN / 2;        // weight rows staged per CTA
@@ -96,19 +93,13 @@ constexpr int kPairSfbBytes = kPairSfbGroups * 512;
 constexpr int kPairStageBytes = kPairABytes + kPairBBytes + kPairSfaBytes + kPairSfbBytes;
 constexpr int kPairSfCol = 2 * kPairBN;        // TMEM: two accumulators, then the scale buffers
 constexpr int kPairSfBufCols = 16 + 4 * kPairSfbGroups;
-// the row-storing epilogue's staging takes the place of a pipeline stage
-constexpr int pair_stages(int mode) { return mode == kGemmUp ? 6 : 5; }
-constexpr int kPairBarBytes = ((2 * pair_stages(kGemmUp) + 4) * 8 + 16 + 15) / 16 * 16;
-constexpr int pair_smem_bytes(int mode) {
-  return pair_stages(mode) * kPairStageBytes + kPairBarBytes +
-         (mode == kGemmUp ? 0 : kEpilogueWarps * kStageBytes) + 1024;
-}
+constexpr int kPairStages = 6;
+constexpr int kPairBarBytes = ((2 * kPairStages + 4) * 8 + 16 + 15) / 16 * 16;
+constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + kPairBarBytes + 1024;
 static_assert(kPairSfCol + kPairSfBufs * kPairSfBufCols <= 512, "TMEM budget");
 static_assert(kPairBRows % 8 == 0, "half a weight tile is whole 8-row swizzle groups");
 static_assert(kPairBBytes % 1024 == 0, "stage regions keep the 1024-byte swizzle alignment");
-static_assert(pair_smem_bytes(kGemmUp) <= kMaxSharedBytes &&
-                  pair_smem_bytes(kGemmDown) <= kMaxSharedBytes,
-              "shared memory budget");
+static_assert(kPairSmemBytes <= kMaxSharedBytes, "shared memory budget");
 
 template <int MODE>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -116,7 +107,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
                                              ~static_cast<uintptr_t>(1023u));
-  constexpr int kStages = pair_stages(MODE);
+  constexpr int kStages = kPairStages;
   uint8_t* sA = smem;
   uint8_t* sB = sA + kStages * kPairABytes;
   uint8_t* sSFA = sB + kStages * kPairBBytes;
@@ -302,9 +293,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
     const int group = (warp - 2) >> 2;      // which share of the tile's 16-column chunks
     const int r = quarter * 32 + lane;      // row inside this CTA's 128 rows == TMEM lane
     constexpr int kChunks = kPairBN / 16;
-    constexpr int kGroups = kEpilogueWarps / 4;
-    const int chunk_begin = kChunks * group / kGroups;
-    const int chunk_end = kChunks * (group + 1) / kGroups;
+    static_assert(kEpilogueWarps == 8, "two groups");
     const uint32_t leader_empty0 = cluster_address_of(&tmem_empty_bar[0], 0);
     int local = 0;
     for (int t = unit; t < total_tiles; t += units, ++local) {
@@ -332,12 +321,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         const uint32_t t_addr =
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kPairBN;
         const int n0 = nt * kPairBN;
+        // the two groups part where 64 columns, which are stored together, begin
+        const int middle = (n0 / 16 + kChunks / 2 + 2) / 4 * 4 - n0 / 16;
+        const int chunk_begin = group == 0 ? 0 : middle;
+        const int chunk_end = group == 0 ? middle : kChunks;
         if constexpr (MODE == kGemmUp) {
-          epilogue_quantise<1>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
+          epilogue_quantise<2>(args, t_addr, n0, chunk_begin, chunk_end, grow, row_valid, scale);
         } else {
-          epilogue_rows(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt,
-                        reinterpret_cast<uint8_t*>(full_bar) + kPairBarBytes +
-                            (warp - 2) * kStageBytes);
+          epilogue_rows_direct<2>(args, t_addr, n0, chunk_begin, chunk_end, dest, scale, wt);
         }
         tcgen05_fence_before();
       }
@@ -365,7 +356,7 @@ cudaError_t launch_pair(const GemmMaps& maps, const GemmArgs& args, int num_sms,
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(num_sms & ~1), 1, 1);
   config.blockDim = dim3(kPairThreads, 1, 1);
-  config.dynamicSmemBytes = pair_smem_bytes(MODE);
+  config.dynamicSmemBytes = kPairSmemBytes;
   config.stream = stream;
   cudaLaunchAttribute attribute;
   attribute.id = cudaLaunchAttributeClusterDimension;

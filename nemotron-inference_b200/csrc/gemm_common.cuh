@@ -26,9 +26,17 @@ __device__ __forceinline__ void load_chunks(uint32_t t_addr, int count, uint32_t
   for (int j = 0; j < BATCH; ++j) tmem_ld_fence(raw[j]);
 }
 
-// relu^2 and NVFP4 quantisation of 16 columns from `n` of row `grow`; returns the largest value.
-__device__ __forceinline__ float quantise_chunk(const GemmArgs& args, float (&v)[16], int n, int grow,
-                                                float scale, bool store) {
+// 32 bytes from a 32-byte boundary: a whole sector by one thread.
+__device__ __forceinline__ void store_sector(void* to, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(to), "r"(w[0]),
+               "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+
+// relu^2 and NVFP4 quantisation of 16 columns: eight bytes of codes and the block's E4M3 scale;
+// returns the largest value.
+__device__ __forceinline__ float quantise_chunk(const float (&v)[16], float scale, uint32_t& lo,
+                                                uint32_t& hi, uint32_t& sf) {
   const uint64_t scale2 = pack2(scale, scale);
   uint64_t squares[8];
   float amax = 0.0f;
@@ -41,13 +49,16 @@ __device__ __forceinline__ float quantise_chunk(const GemmArgs& args, float (&v)
     unpack2(squares[i], a, b);
     amax = fmaxf(fmaxf(a, b), amax);
   }
-  uint32_t lo, hi;
-  const uint32_t sf = quantize_block16_unit_scale(squares, amax, lo, hi);
-  if (!store) return 0.0f;
-  *reinterpret_cast<uint2*>(args.out_packed + static_cast<size_t>(grow) * (args.N / 2) + n / 2) =
-      make_uint2(lo, hi);
-  args.out_sf[swizzled_scale_offset(grow, n / 16, args.out_k_blocks * 4)] = static_cast<uint8_t>(sf);
+  sf = quantize_block16_unit_scale(squares, amax, lo, hi);
   return amax;
+}
+
+// Where the codes and the scale of block `block` (16 columns) of row `grow` go.
+__device__ __forceinline__ uint8_t* hidden_codes(const GemmArgs& args, int grow, int block) {
+  return args.out_packed + static_cast<size_t>(grow) * (args.N / 2) + block * 8;
+}
+__device__ __forceinline__ uint8_t* hidden_scale(const GemmArgs& args, int grow, int block) {
+  return args.out_sf + swizzled_scale_offset(grow, block, args.out_k_blocks * 4);
 }
 
 __device__ __forceinline__ void report_range(const GemmArgs& args, float largest) {
@@ -85,6 +96,16 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& args, float (&v)[16]
   }
   if (args.out_kind == kRowF32) {
     float4* d = reinterpret_cast<float4*>(dest + static_cast<size_t>(n) * 4);
+    if (args.out_aligned) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t w[8];
+#pragma unroll
+        for (int h = 0; h < 8; ++h) w[h] = __float_as_uint(v[8 * i + h]);
+        store_sector(d + 2 * i, w);
+      }
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
@@ -93,6 +114,10 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& args, float (&v)[16]
   }
   uint32_t w[8];
   pack_rows16(args.out_kind, v, w);
+  if (args.out_aligned) {
+    store_sector(reinterpret_cast<void*>(dest + static_cast<size_t>(n) * 2), w);
+    return;
+  }
   uint4* d = reinterpret_cast<uint4*>(dest + static_cast<size_t>(n) * 2);
   d[0] = make_uint4(w[0], w[1], w[2], w[3]);
   d[1] = make_uint4(w[4], w[5], w[6], w[7]);
@@ -101,23 +126,50 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& args, float (&v)[16]
 // Up projection: relu^2 and NVFP4 quantisation of columns [n0 + 16 * chunk_begin,
 // n0 + 16 * chunk_end) of the accumulator at `t_addr` (this warp's lane quarter); the thread owns
 // row `grow` of the hidden activations.
+//
+// Four blocks from a multiple of four are one sector of codes and one word of scales.  Stored block by
+// block (8 bytes and 1 byte, each a sector's transaction) they held up the loads of the tiles behind:
+// 98304 rows of 1856 took 250 us, 213 without the stores.
 template <int BATCH>
 __device__ __forceinline__ void epilogue_quantise(const GemmArgs& args, uint32_t t_addr, int n0,
                                                   int chunk_begin, int chunk_end, int grow,
                                                   bool row_valid, float scale) {
   float row_max = 0.0f;
   chunk_end = min(chunk_end, (args.N - n0) / 16);
-  for (int first = chunk_begin; first < chunk_end; first += BATCH) {
-    uint32_t raw[BATCH][16];
-    load_chunks<BATCH>(t_addr + first * 16, chunk_end - first, raw);
+  for (int c = chunk_begin; c < chunk_end;) {
+    const int block = n0 / 16 + c;
+    const int count = min(4 - (block & 3), chunk_end - c);
+    uint32_t codes[8], scales[4];
 #pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-      float v[16];
+    for (int first = 0; first < 4; first += BATCH) {
+      if (first >= count) break;
+      uint32_t raw[BATCH][16];
+      load_chunks<BATCH>(t_addr + (c + first) * 16, count - first, raw);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[j][i]);
-      row_max = fmaxf(row_max, quantise_chunk(args, v, n0 + (first + j) * 16, grow, scale,
-                                              row_valid && first + j < chunk_end));
+      for (int j = 0; j < BATCH; ++j) {
+        if (first + j >= count) break;
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[j][i]);
+        const int k = first + j;
+        const float largest = quantise_chunk(v, scale, codes[2 * k], codes[2 * k + 1], scales[k]);
+        if (row_valid) row_max = fmaxf(row_max, largest);
+      }
     }
+    if (row_valid && count == 4) {
+      store_sector(hidden_codes(args, grow, block), codes);
+      *reinterpret_cast<uint32_t*>(hidden_scale(args, grow, block)) =
+          scales[0] | (scales[1] << 8) | (scales[2] << 16) | (scales[3] << 24);
+    } else if (row_valid) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        if (j >= count) break;
+        *reinterpret_cast<uint2*>(hidden_codes(args, grow, block + j)) =
+            make_uint2(codes[2 * j], codes[2 * j + 1]);
+        *hidden_scale(args, grow, block + j) = static_cast<uint8_t>(scales[j]);
+      }
+    }
+    c += count;
   }
   report_range(args, row_max);
 }
@@ -138,8 +190,9 @@ __device__ __forceinline__ unsigned long long output_row_address(const GemmArgs&
   return reinterpret_cast<unsigned long long>(args.out_rows) + d * row_bytes;
 }
 
-// Row-storing epilogue without staging: every thread stores its own row, 16 columns (32 or 64
-// bytes, whole sectors) at a time.
+// Row-storing epilogue: every thread stores its own row, 16 columns (32 or 64 bytes, whole sectors) at
+// a time.  In the CTA-pair kernel, lines of 128 bytes put together in shared memory first took 300 us
+// for 98304 rows of 2688, this 289: the room it leaves is a sixth pipeline stage.
 template <int BATCH>
 __device__ __forceinline__ void epilogue_rows_direct(const GemmArgs& args, uint32_t t_addr, int n0,
                                                      int chunk_begin, int chunk_end,
@@ -157,68 +210,6 @@ __device__ __forceinline__ void epilogue_rows_direct(const GemmArgs& args, uint3
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[j][i]);
       store_chunk(args, v, n0 + (first + j) * 16, dest, scale, wt);
-    }
-  }
-}
-
-// Row-storing epilogue through shared memory: each thread owns one row of the tile, but a store
-// instruction should write few lines.  64 bytes of 32 rows are staged at a time (`stage`:
-// kStageBytes of this warp's own; a row's pitch of five 16-byte units keeps both directions free
-// of bank conflicts), then every four lanes write one row's 64 bytes.
-constexpr int kStagePitch = 80;
-constexpr int kStageBytes = 32 * kStagePitch;
-
-__device__ __forceinline__ void epilogue_rows(const GemmArgs& args, uint32_t t_addr, int n0,
-                                              int chunk_begin, int chunk_end,
-                                              unsigned long long dest, float scale, float wt,
-                                              uint8_t* stage) {
-  const int lane = threadIdx.x & 31;
-  uint8_t* own = stage + lane * kStagePitch;
-  const uint8_t* part = stage + (lane >> 2) * kStagePitch + (lane & 3) * 16;
-  const bool f32 = args.out_kind == kRowF32;
-  const float factor = args.row_weight != nullptr ? wt : 1.0f;
-  chunk_end = min(chunk_end, (args.N - n0) / 16);
-  const int step = f32 ? 1 : 2;
-  for (int ch = chunk_begin; ch < chunk_end; ch += step) {
-    const bool wide = !f32 && ch + 1 < chunk_end;
-    uint32_t raw[2][16];
-    load_chunks<2>(t_addr + ch * 16, wide ? 2 : 1, raw);
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      if (j == 1 && !wide) break;
-      float v[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        // (a factor of one leaves every value as it is)
-        v[i] = __fmul_rn(__fmul_rn(__uint_as_float(raw[j][i]), scale), factor);
-        if (args.relu2) {  // Relu2 (expert_layer.cpp:138-140): x > 0 ? x * x : 0
-          const float p = fmaxf(v[i], 0.0f);
-          v[i] = __fmul_rn(p, p);
-        }
-      }
-      if (f32) {
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          *reinterpret_cast<float4*>(own + i * 4) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        }
-      } else {
-        uint32_t w[8];
-        pack_rows16(args.out_kind, v, w);
-        *reinterpret_cast<uint4*>(own + j * 32) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(own + j * 32 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-      }
-    }
-    __syncwarp();
-    const bool mine = f32 || wide || (lane & 3) < 2;
-    const size_t at = static_cast<size_t>(n0 + ch * 16) * (f32 ? 4 : 2) + (lane & 3) * 16;
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const unsigned long long d = __shfl_sync(0xffffffffu, dest, it * 8 + (lane >> 2));
-      if (d != 0 && mine) {
-        *reinterpret_cast<uint4*>(d + at) =
-            *reinterpret_cast<const uint4*>(part + it * 8 * kStagePitch);
-      }
     }
   }
 }

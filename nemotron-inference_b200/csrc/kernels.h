@@ -112,6 +112,7 @@ struct GemmArgs {
   // kGemmDown outputs
   void* out_rows = nullptr;           // [dest][N] of out_kind elements
   int32_t out_kind = kRowF32;         // RowKind
+  int32_t out_aligned = 0;            // every row of out_rows starts on a 32-byte boundary
   const int32_t* dest_row = nullptr;  // per activation row; nullptr => row*dest_mul+dest_add
   int32_t dest_mul = 1;
   int32_t dest_add = 0;

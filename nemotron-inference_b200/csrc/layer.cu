@@ -400,6 +400,8 @@ struct RowOutput {
 void set_row_output(GemmArgs* g, const RowOutput& out) {
   g->out_rows = out.rows;
   g->out_kind = out.kind;
+  // (rows in peers' windows lie behind a 256-byte boundary, and N is a multiple of 64)
+  g->out_aligned = out.segments.bases != nullptr || reinterpret_cast<uintptr_t>(out.rows) % 32 == 0;
   g->dest_row = out.dest_row;
   g->dest_mul = out.dest_mul;
   g->dest_add = out.dest_add;
