@@ -69,7 +69,9 @@ __device__ __forceinline__ TileRows tile_rows_of(const GemmArgs& args, int rt, i
 // What bounds a K block is what an SM takes in.  A pair stages each weight tile once for 256 rows (half
 // in each CTA), 35 KB per CTA and K block, and with the epilogue left out a K block takes 660 cycles, 54
 // bytes each, hardly less with half of the MMAs (98304 rows, up: 193 us and 187).  The rows stored by
-// the epilogue come on top of that: 221 us for up, 289 for down.  At 4096 tokens it is HBM: 446 MB in 86 us, 0.8 of the copy rate.
+// the epilogue come on top of that: 221 us for up, 284 for down.  Experts' rows are therefore spread
+// evenly over a pair's CTAs (csrc/plan.cu): 128 and 64 rows cost as much as 128 and 128.  At 4096 tokens
+// it is HBM: 446 MB in 86 us, 0.8 of the copy rate.
 //
 // Roles per CTA: warp 0 loads (the CTA's own 128 activation rows, its half of the weight tile, the
 // scales of its rows and of the whole weight tile), warp 1 of cluster rank 0 issues the scale
@@ -100,6 +102,15 @@ static_assert(kPairSfCol + kPairSfBufs * kPairSfBufCols <= 512, "TMEM budget");
 static_assert(kPairBRows % 8 == 0, "half a weight tile is whole 8-row swizzle groups");
 static_assert(kPairBBytes % 1024 == 0, "stage regions keep the 1024-byte swizzle alignment");
 static_assert(kPairSmemBytes <= kMaxSharedBytes, "shared memory budget");
+
+// Activation rows are loaded 16 at a time.
+__device__ __forceinline__ int boxes_of(int rows) {
+  return (rows + kPairBoxRows - 1) / kPairBoxRows;
+}
+// Bytes that a CTA with `rows` activation rows loads of them per K block, with its slot's scales.
+__device__ __forceinline__ uint32_t row_bytes(int rows) {
+  return rows > 0 ? boxes_of(rows) * (kPairBoxRows * 128) + kPairSfaBytes : 0u;
+}
 
 template <int MODE>
 __global__ void __launch_bounds__(kPairThreads, 1)
@@ -136,7 +147,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       mbar_init(&tmem_empty_bar[a], 2 * kEpilogueWarps);
     }
     fence_barrier_init();
-    prefetch_tensormap(&maps.a);
+    for (int i = 0; i < kPairBoxes; ++i) prefetch_tensormap(&maps.a[i]);
     prefetch_tensormap(&maps.b_tail);
     prefetch_tensormap(&maps.b_full);
     prefetch_tensormap(&maps.sfa);
@@ -173,6 +184,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       const TileRows rows = tile_rows_of(args, rt, num_row_tiles, cta_rank);
       const int load_row0 = warp_uniform(rows.load_row0);
       const int expert = warp_uniform(rows.expert);
+      // Rows that do not exist are not loaded: the MMAs read what an earlier tile left in their place,
+      // in rows that are never stored.
+      const int own_rows = warp_uniform(rows.rows);
+      const int other_rows =
+          warp_uniform(tile_rows_of(args, rt, num_row_tiles, cta_rank ^ 1u).rows);
+      const int box = max(boxes_of(own_rows) - 1, 0);
+      const uint32_t tile_bytes = row_bytes(own_rows) + row_bytes(other_rows) +
+                                  2 * (kPairBBytes + kPairSfbBytes);
       // the scale maps' rows are 1024 bytes: two to a K block of activations, four to one of weights
       const int sfa_row = (load_row0 >> 7) * k_blocks * 2;
       const int sfb_row = (expert * args.n_tiles + nt) * k_blocks * 4;
@@ -185,8 +204,11 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
         }
         if (elect_one()) {
           const uint32_t bar = leader_full0 + stage * 8;
-          if (leader) mbar_arrive_expect_tx_at(full0 + stage * 8, 2 * kPairStageBytes);
-          tma_load_2d_pair_at(a0 + stage * kPairABytes, &maps.a, kb * 128, load_row0, bar);
+          if (leader) mbar_arrive_expect_tx_at(full0 + stage * 8, tile_bytes);
+          if (own_rows > 0) {
+            tma_load_2d_pair_at(a0 + stage * kPairABytes, &maps.a[box], kb * 128, load_row0, bar);
+            tma_load_2d_pair_at(sfa0 + stage * kPairSfaBytes, &maps.sfa, 0, sfa_row + kb * 2, bar);
+          }
           if (kb < args.kb_full) {
             // the map's rows are eight weight rows' 128 bytes of a K block
             tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_full, 0,
@@ -195,7 +217,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
             tma_load_2d_pair_at(b0 + stage * kPairBBytes, &maps.b_tail, 0, expert * args.N + b_row,
                                 bar);
           }
-          tma_load_2d_pair_at(sfa0 + stage * kPairSfaBytes, &maps.sfa, 0, sfa_row + kb * 2, bar);
           tma_load_2d_pair_at(sfb0 + stage * kPairSfbBytes, &maps.sfb, 0, sfb_row + kb * 4, bar);
         }
         if (++stage == kStages) {

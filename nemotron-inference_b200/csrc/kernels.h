@@ -137,11 +137,13 @@ struct GemmTileInfo {
   int b_rows;      // weight rows one CTA stages per K block (half a tile in a pair)
 };
 
-// Tensor maps of a CTA-pair GEMM launch.  `a`: activation rows, 128-byte swizzle; `b_full`: the full
-// weight K blocks, the K-block-major panels as rows of eight weight rows' 128 bytes, no swizzle;
-// `b_tail`: the partial last K block of the weights.
+// Tensor maps of a CTA-pair GEMM launch.  `a`: activation rows, 128-byte swizzle, boxes of 16, 32, ..
+// 128 rows; `b_full`: the full weight K blocks, the K-block-major panels as rows of eight weight rows'
+// 128 bytes, no swizzle; `b_tail`: the partial last K block of the weights.
+constexpr int kPairBoxRows = 16;
+constexpr int kPairBoxes = 128 / kPairBoxRows;
 struct GemmMaps {
-  CUtensorMap a;
+  CUtensorMap a[kPairBoxes];
   CUtensorMap b_tail;
   CUtensorMap b_full;
   CUtensorMap sfa, sfb;  // both operands' tiled block scales as rows of 1024 bytes
@@ -377,9 +379,9 @@ struct PermuteSource {
   int capacity = 0;
 };
 // Lays out every expert's row slots (128 rows each; `tile_multiple`: every expert gets a multiple of
-// this many, 2 when CTA pairs consume them), writes the tile list, copies each pair's quantised
-// activation row into its expert's slots and records where it went;
-// sorted_dest[row] = source_row * dest_stride + slot.
+// this many, 2 when CTA pairs consume them, and its rows are then spread over them evenly), writes the
+// tile list, copies each pair's quantised activation row into its expert's slots and records where it
+// went; sorted_dest[row] = source_row * dest_stride + slot.
 cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src, int pairs,
                               int experts /* size of the local expert stack */, int tile_multiple,
                               int max_row_tiles, int cols, int k_blocks, uint8_t* sorted_packed,

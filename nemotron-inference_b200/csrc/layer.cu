@@ -313,7 +313,8 @@ struct WeightStack {
 struct ActivationOperand {
   const uint8_t* packed = nullptr;
   const uint8_t* sf_tiled = nullptr;
-  CUtensorMap boxes[kStreamBoxes];  // 8, 16, 32, 64 and 128 rows
+  CUtensorMap boxes[kStreamBoxes];     // 8, 16, 32, 64 and 128 rows
+  CUtensorMap pair_boxes[kPairBoxes];  // 16, 32, .. 128 rows
   CUtensorMap sf_map;               // the tiled scales as rows of 1024 bytes
   void bind(const uint8_t* packed_rows, const uint8_t* sf, size_t rows, int k) {
     packed = packed_rows;
@@ -322,12 +323,16 @@ struct ActivationOperand {
     for (int i = 0; i < kStreamBoxes; ++i) {
       boxes[i] = make_packed_map(packed_rows, rows, static_cast<size_t>(k) / 2, 8 << i);
     }
+    for (int i = 0; i < kPairBoxes; ++i) {
+      pair_boxes[i] = make_packed_map(packed_rows, rows, static_cast<size_t>(k) / 2,
+                                      kPairBoxRows * (i + 1));
+    }
   }
 };
 
 GemmMaps gemm_maps(const WeightStack& weights, const ActivationOperand& a) {
   GemmMaps maps;
-  maps.a = a.boxes[kStreamBoxes - 1];
+  for (int i = 0; i < kPairBoxes; ++i) maps.a[i] = a.pair_boxes[i];
   maps.b_tail = weights.tail_map(kClassPair);
   maps.b_full = weights.full_pair;
   maps.sfa = a.sf_map;

@@ -19,6 +19,14 @@ namespace {
 
 constexpr int kMaxPlanExperts = 512;
 
+// Rows per tile of an expert with `count` rows in `tiles` tiles.  Two CTAs that share a weight tile wait
+// for the one with more rows to load, so a pair's tiles get equal shares (in steps of the GEMM's boxes;
+// 96 and 96 rows in the place of 128 and 64).  Single tiles are filled one after the other.
+__device__ __forceinline__ int rows_per_tile(int count, int tiles, int tile_multiple) {
+  if (tile_multiple == 1 || tiles <= 1) return 128;
+  return ((count + tiles - 1) / tiles + kPairBoxRows - 1) / kPairBoxRows * kPairBoxRows;
+}
+
 // By all THREADS threads of a block: tiles_of[e] = row tiles of expert e, first_tile[e] = tiles of
 // the experts before it; returns the number of all tiles.  Ends with a barrier.
 template <int THREADS>
@@ -71,7 +79,7 @@ __device__ __forceinline__ int scan_expert_tiles(const int32_t* counts, int expe
 // The tile list of the grouped GEMM, by all threads of one block.
 template <int THREADS>
 __device__ __forceinline__ void write_row_tiles(const PlanBuffers& plan, int experts,
-                                                int max_row_tiles, int total,
+                                                int tile_multiple, int max_row_tiles, int total,
                                                 const int* first_tile, const int* tiles_of,
                                                 int32_t* error) {
   if (threadIdx.x == 0) {
@@ -80,10 +88,11 @@ __device__ __forceinline__ void write_row_tiles(const PlanBuffers& plan, int exp
   }
   for (int e = threadIdx.x; e < experts; e += THREADS) {
     const int count = plan.expert_counts[e];
+    const int per_tile = rows_per_tile(count, tiles_of[e], tile_multiple);
     for (int i = 0; i < tiles_of[e] && first_tile[e] + i < max_row_tiles; ++i) {
       RowTile tile;
       tile.row0 = (first_tile[e] + i) * 128;
-      tile.rows = max(0, min(128, count - i * 128));
+      tile.rows = max(0, min(per_tile, count - i * per_tile));
       tile.expert = e;
       tile.reserved = 0;
       plan.row_tiles[first_tile[e] + i] = tile;
@@ -129,7 +138,7 @@ place_rows_kernel(PlanBuffers plan, PermuteSource src, int pairs, int share, int
   const int total = scan_expert_tiles<kPlaceThreads>(plan.expert_counts, experts, tile_multiple,
                                                      first_tile, tiles_of);
   if (blockIdx.x == 0) {
-    write_row_tiles<kPlaceThreads>(plan, experts, max_row_tiles, total, first_tile, tiles_of, error);
+    write_row_tiles<kPlaceThreads>(plan, experts, tile_multiple, max_row_tiles, total, first_tile, tiles_of, error);
   }
   for (int unit = first_unit; unit < units; unit += warps) {
     const int source_row = unit / share, part = unit - source_row * share;
@@ -153,9 +162,11 @@ place_rows_kernel(PlanBuffers plan, PermuteSource src, int pairs, int share, int
                                                      : atomicAdd(&plan.expert_cursor[expert], 1);
         // an expert's rows stay inside the tiles the plan gave it, whatever the histogram said,
         // and plan overflow was already reported
-        const int tile = first_tile[expert] + position / 128;
-        if (position >= 0 && position / 128 < tiles_of[expert] && tile < max_row_tiles) {
-          row = tile * 128 + position % 128;
+        const int per_tile =
+            rows_per_tile(plan.expert_counts[expert], tiles_of[expert], tile_multiple);
+        const int of_expert = position / per_tile, tile = first_tile[expert] + of_expert;
+        if (position >= 0 && of_expert < tiles_of[expert] && tile < max_row_tiles) {
+          row = tile * 128 + position - of_expert * per_tile;
           out.tensor_scale[row] = *reinterpret_cast<const float*>(
               reinterpret_cast<const uint8_t*>(src.tensor_scale) +
               static_cast<size_t>(source_row) * src.tensor_scale_stride);

@@ -33,6 +33,21 @@ def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
     assert rep.ok(), rep.summary()
 
 
+def test_pairs_share_rows_of_every_count(package, synthetic):
+    # experts without rows, with fewer than a box of them and with several pairs of tiles
+    cfg = synthetic.baseline_config(max_tokens=1501, experts=32, hidden=512, routed=256, shared=512)
+    data = synthetic.make_layer(cfg, seed=43, device="cuda", skewed=True)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (534, 1501):
+        x = synthetic.make_tokens(tokens, 512, seed=tokens, device="cuda")
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        assert layer.run(x, out), layer.last_error
+        rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+        assert rep.ok(), rep.summary()
+    layer.close()
+
+
 @pytest.mark.parametrize("rows", [3, 1185])
 @pytest.mark.parametrize("cols", [16, 1008, 2048, 2064, 4096, 4112, 5376, 6144, 6160])
 def test_quantiser_row_lengths(package, oracle, rows, cols):

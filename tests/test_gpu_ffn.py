@@ -67,3 +67,28 @@ def test_single_expert_ffn_small_shapes(package, oracle, synthetic, hidden, inte
         r = _run_case(package, oracle, synthetic, rows, hidden, inter, variant, seed=hidden)
         print(hidden, inter, rows, variant, r)
         _check(r)
+
+
+# 64 columns are stored together: weight tiles of 208 columns that start inside such a group and end in
+# one (832 = 4 tiles), last tiles of 16 to 192 columns, one row and the rows around a tile's edge
+@pytest.mark.parametrize("hidden,inter", [(832, 448), (448, 832), (1088, 192)])
+def test_ffn_where_tiles_end(package, oracle, synthetic, hidden, inter):
+    for rows, variant in [(1, 1), (129, 1), (255, 4), (16, 3), (17, 3), (129, 3)]:
+        _check(_run_case(package, oracle, synthetic, rows, hidden, inter, variant, seed=inter))
+
+
+@pytest.mark.parametrize("variant", [1, 3])
+def test_ffn_rows_on_a_16_byte_boundary(package, synthetic, variant):
+    # whole sectors are stored only to rows that start on one
+    up, down = synthetic.make_ffn_weights(448, 192, seed=5, device="cuda")
+    x = synthetic.make_tokens(70, 448, seed=6, device="cuda")
+    ffn = package.ExpertFfn(up, down, max_rows=128)
+    expected = ffn.run(x, variant)
+    room = torch.zeros(70 * 448 + 8, device="cuda")
+    lib, stream = package.load_library(), torch.cuda.current_stream().cuda_stream
+    assert lib.nmoe_ffn_run(ffn._handle, stream, x.data_ptr(), package._dtype_code(x), 70,
+                            room[4:].data_ptr(), variant) == 0
+    assert lib.nmoe_ffn_sync_status(ffn._handle, stream) == 0
+    assert torch.equal(room[4:-4].view(70, 448), expected)
+    assert not room[:4].any() and not room[-4:].any()
+    ffn.close()
