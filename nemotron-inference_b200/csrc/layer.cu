@@ -917,7 +917,8 @@ struct nmoe_layer {
   DeviceBuffer norm_weight, gate, bias, logit_offset;
   ExactOperand gate_exact;  // the router's FP64 logits of small batches
   bool has_gate_exact = false;
-  ExactScratch exact;
+  ExactScratch exact;              // of the linears on the caller's stream
+  ExactScratch fc1_exact, up_exact;  // of fc1_latent and shared_up, which may run beside them
   bool has_logit_offset = false;
   // two-pass router (tensor-core logits + FP64 re-evaluation of near-ties)
   bool fast_router = false;
@@ -1020,6 +1021,9 @@ struct nmoe_layer {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t quant_done = nullptr, shared_done = nullptr;
   int fork_max_tokens = 1 << 30;  // (NMOE_FORK_MAX_TOKENS)
+  // Latent layers: fc1_latent and its quantiser run on one more stream beside the router.
+  cudaStream_t latent_stream = nullptr;
+  cudaEvent_t latent_done = nullptr;
   bool window_fork_shared = false;    // nmoe_ep_window_fork_shared
   bool window_shared_pending = false;
   RowKind window_shared_kind = kRowF32;  // type of shared_out for the pending combine
@@ -1053,7 +1057,9 @@ struct nmoe_layer {
     window.close_peers();
     if (quant_done != nullptr) cudaEventDestroy(quant_done);
     if (shared_done != nullptr) cudaEventDestroy(shared_done);
+    if (latent_done != nullptr) cudaEventDestroy(latent_done);
     if (side_stream != nullptr) cudaStreamDestroy(side_stream);
+    if (latent_stream != nullptr) cudaStreamDestroy(latent_stream);
     for (cudaEvent_t e : stage_events)
       if (e != nullptr) cudaEventDestroy(e);
   }
@@ -1082,11 +1088,15 @@ void allocate_exact(nmoe_layer* L, size_t T) {
     L->gate_exact.slice(nullptr);
     linears.emplace_back(L->cfg.n_routed_experts, L->cfg.hidden_size);
   }
-  for (const DenseLinear* linear :
-       {&L->fc1, &L->fc2, &L->shared_up_dense, &L->shared_down_dense}) {
+  const int sms = device_sm_count();
+  for (const DenseLinear* linear : {&L->fc2, &L->shared_down_dense}) {
     if (linear->present && linear->exact) linears.emplace_back(linear->out, linear->in);
   }
-  L->exact.allocate(T, linears, device_sm_count());
+  L->exact.allocate(T, linears, sms);
+  if (L->fc1.present && L->fc1.exact) L->fc1_exact.allocate(T, {{L->fc1.out, L->fc1.in}}, sms);
+  if (L->shared_up_dense.present && L->shared_up_dense.exact) {
+    L->up_exact.allocate(T, {{L->shared_up_dense.out, L->shared_up_dense.in}}, sms);
+  }
 }
 
 // Everything whose size follows the token capacity.  Called at creation and by
@@ -1254,6 +1264,10 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
     NMOE_CUDA(cudaStreamCreateWithFlags(&L->side_stream, cudaStreamNonBlocking));
     NMOE_CUDA(cudaEventCreateWithFlags(&L->quant_done, cudaEventDisableTiming));
     NMOE_CUDA(cudaEventCreateWithFlags(&L->shared_done, cudaEventDisableTiming));
+    if (w.fc1_latent.family != NMOE_LINEAR_ABSENT) {
+      NMOE_CUDA(cudaStreamCreateWithFlags(&L->latent_stream, cudaStreamNonBlocking));
+      NMOE_CUDA(cudaEventCreateWithFlags(&L->latent_done, cudaEventDisableTiming));
+    }
   }
   L->local_experts = w.n_local_experts;
   L->first_local_expert = w.first_local_expert;
@@ -1334,12 +1348,12 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
 }
 
 // y = x W^T of a dense / scaled-FP8 linear, rounded once from the FP64 sum [, relu^2 of it].
-void run_linear(nmoe_layer* L, const DenseLinear& linear, const float* in_rows, int rows,
-                float* out_rows, bool relu2, LaunchStream stream) {
+void run_linear(nmoe_layer* L, const DenseLinear& linear, ExactScratch& scratch,
+                const float* in_rows, int rows, float* out_rows, bool relu2, LaunchStream stream) {
   if (linear.exact) {
     // (clamped first, scaled_fp8_linear.cu:27-33: a scale of zero means no round trip further down)
     const float fp8_scale = linear.fp8 ? clamp_scale_host(linear.input_scale) : 0.0f;
-    run_exact(linear.operand.w, L->exact, in_rows, fp8_scale, rows, nullptr, relu2, out_rows,
+    run_exact(linear.operand.w, scratch, in_rows, fp8_scale, rows, nullptr, relu2, out_rows,
               L->error.device.as<int32_t>(), L->num_sms, stream);
     return;
   }
@@ -1563,8 +1577,8 @@ TileClass shared_tile_class(const nmoe_layer* L, int tokens) {
 void shared_hidden_rows(nmoe_layer* L, LaunchStream stream, int tokens) {
   float* raw = L->shared_raw.as<float>();
   if (L->shared_up_dense.present) {
-    run_linear(L, L->shared_up_dense, L->normalized.as<float>(), tokens, raw, /*relu2=*/true,
-               stream);
+    run_linear(L, L->shared_up_dense, L->up_exact, L->normalized.as<float>(), tokens, raw,
+               /*relu2=*/true, stream);
     return;
   }
   Schedule shared;
@@ -1612,7 +1626,7 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
     // only the latent data flow (FP32 rows of `hidden` per token) reaches this
     NMOE_REQUIRE(dest_mul == 1 && dest_add == 0 && out_kind == kRowF32,
                  "a dense shared_down writes FP32 token rows");
-    run_linear(L, L->shared_down_dense, L->shared_raw.as<float>(), tokens,
+    run_linear(L, L->shared_down_dense, L->exact, L->shared_raw.as<float>(), tokens,
                static_cast<float*>(out_rows), false, stream);
     return;
   }
@@ -1621,10 +1635,10 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
                 L->error.device.as<int32_t>(), L->num_sms, stream);
 }
 
-// The shared expert as part of the routed experts' launch (csrc/expert_stream.cu); rows of a dense
-// shared_up are made here, before it.
-StreamFfn shared_stream_ffn(nmoe_layer* L, LaunchStream stream, int tokens, void* out_rows,
-                            int dest_mul, int dest_add, RowKind out_kind) {
+// The shared expert as part of the routed experts' launch (csrc/expert_stream.cu); the hidden rows of
+// a dense shared_up were made before it.
+StreamFfn shared_stream_ffn(nmoe_layer* L, int tokens, void* out_rows, int dest_mul, int dest_add,
+                            RowKind out_kind) {
   StreamFfn ffn;
   ffn.down = &L->shared_down;
   ffn.schedule.dense_rows = tokens;
@@ -1638,8 +1652,6 @@ StreamFfn shared_stream_ffn(nmoe_layer* L, LaunchStream stream, int tokens, void
   ffn.out.dest_add = dest_add;
   ffn.row_slots = (tokens + 127) / 128;
   if (L->shared_up_dense.present) {
-    shared_hidden_rows(L, stream, tokens);
-    quantise_shared_hidden(L, stream, tokens);
     ffn.hidden_tensor_scale = L->sh_ts.as<float>();
   } else {
     ffn.up = &L->shared_up;
@@ -1667,6 +1679,14 @@ PermuteSource local_source(nmoe_layer* L) {
   return source;
 }
 
+// A latent layer's three chains behind the norm -- gate and selection; fc1_latent and its quantiser;
+// shared_up and its quantiser -- meet only in front of the experts.  On streams of their own one fills
+// what another leaves idle: latency at a few tokens, SMs at a hundred, last waves at a thousand.  Whole
+// pass of the checkpoint's layer, one stream against three: 1 token 77.8 us and 80.4 (the branches of
+// the graph cost more than they hide), 2 tokens 101 and 91, 8 tokens 189 and 171, 64 tokens 399 and 373,
+// 256 tokens 578 and 534, 1000 tokens 1075 and 962.
+constexpr int kBesideMinTokens = 2;
+
 void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype in_dtype,
                     int tokens, void* output, nmoe_dtype out_dtype) {
   const nmoe_config& c = L->cfg;
@@ -1691,7 +1711,10 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   // with the two-pass router there was nothing to gain (256 tokens 162 us either way) and at 700
   // tokens 2 to 4 us to lose.
   const LaunchStream chain(stream, !fork && !L->stage_timing && !L->unfused && !two_pass);
-  route_tokens(L, chain, input, in_dtype, tokens, fork ? L->quant_done : nullptr,
+  const bool beside = L->latent_stream != nullptr && one_launch && L->latent_mode &&
+                      !L->stage_timing && tokens >= kBesideMinTokens &&
+                      tokens <= L->fork_max_tokens;
+  route_tokens(L, chain, input, in_dtype, tokens, fork || beside ? L->quant_done : nullptr,
                fork && two_pass);
   L->last_tokens = tokens;
   L->last_parts_kind = parts_kind;
@@ -1699,12 +1722,34 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   if (L->latent_mode) {
     // latent = fc1_latent(normalized) (:809-813); every routed expert's up_proj packs
     // the same latent row (:913 -> nvfp4_packing.cpp:90)
-    run_linear(L, L->fc1, L->normalized.as<float>(), tokens, L->latent_rows.as<float>(), false,
-               chain);
+    LaunchStream latent = chain, up = chain, placing = chain;
+    if (beside) {
+      latent = LaunchStream(L->latent_stream);
+      up = LaunchStream(L->side_stream);
+      NMOE_CUDA(cudaStreamWaitEvent(L->latent_stream, L->quant_done, 0));
+      if (L->shared_up_dense.present) {
+        NMOE_CUDA(cudaStreamWaitEvent(L->side_stream, L->quant_done, 0));
+      }
+    }
+    run_linear(L, L->fc1, L->fc1_exact, L->normalized.as<float>(), tokens,
+               L->latent_rows.as<float>(), false, latent);
     NMOE_CUDA(launch_norm_quant(L->latent_rows.as<float>(), false, tokens, Lr, nullptr, 0.0f,
                                 nullptr, L->lat_packed.as<uint8_t>(),
                                 L->lat_sf_row_major.as<uint8_t>(), nullptr, 0,
-                                L->lat_ts.as<float>(), L->num_sms, chain));
+                                L->lat_ts.as<float>(), L->num_sms, latent));
+    if (one_launch && L->shared_up_dense.present) {
+      shared_hidden_rows(L, up, tokens);
+      quantise_shared_hidden(L, up, tokens);
+    }
+    if (beside) {
+      NMOE_CUDA(cudaEventRecord(L->latent_done, L->latent_stream));
+      NMOE_CUDA(cudaStreamWaitEvent(stream, L->latent_done, 0));
+      if (L->shared_up_dense.present) {
+        NMOE_CUDA(cudaEventRecord(L->shared_done, L->side_stream));
+        NMOE_CUDA(cudaStreamWaitEvent(stream, L->shared_done, 0));
+      }
+      placing.chained = false;  // it has more than one predecessor
+    }
     PermuteSource source = local_source(L);
     source.packed = L->lat_packed.as<uint8_t>();
     source.packed_stride = static_cast<size_t>(Lr) / 2;
@@ -1713,8 +1758,8 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     source.tensor_scale = L->lat_ts.as<float>();
     if (one_launch) {
       const StreamFfn shared =
-          shared_stream_ffn(L, chain, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
-      routed_experts(L, chain, source, tokens * K, K, L->parts.as<void>(), kRowF32, RowSegments(),
+          shared_stream_ffn(L, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
+      routed_experts(L, placing, source, tokens * K, K, L->parts.as<void>(), kRowF32, RowSegments(),
                      &shared);
       for (int i = 7; i <= 9; ++i) L->mark(i, stream);
     } else {
@@ -1728,8 +1773,8 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     // residual (:1064-1069)
     NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
                                chain));
-    run_linear(L, L->fc2, L->routed_latent.as<float>(), tokens, L->projected.as<float>(), false,
-               chain);
+    run_linear(L, L->fc2, L->exact, L->routed_latent.as<float>(), tokens, L->projected.as<float>(),
+               false, chain);
     NMOE_CUDA(launch_mixer(input, in_dtype == NMOE_BF16, L->projected.as<float>(),
                            L->shared_rows.as<float>(), tokens, H, output, out_dtype == NMOE_BF16,
                            chain));
@@ -1742,8 +1787,12 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     NMOE_CUDA(cudaEventRecord(L->shared_done, L->side_stream));
   }
   if (one_launch) {
+    if (L->shared_up_dense.present) {
+      shared_hidden_rows(L, chain, tokens);
+      quantise_shared_hidden(L, chain, tokens);
+    }
     const StreamFfn shared =
-        shared_stream_ffn(L, chain, tokens, L->parts.as<void>(), K + 1, K, parts_kind);
+        shared_stream_ffn(L, tokens, L->parts.as<void>(), K + 1, K, parts_kind);
     routed_experts(L, chain, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind,
                    RowSegments(), &shared);
   } else {

@@ -60,6 +60,30 @@ def test_checkpoint_shape_latent_layer(package, synthetic):
     layer.close()
 
 
+def test_chains_beside_each_other_give_the_same_bits(package, synthetic, monkeypatch):
+    # from two tokens gate, fc1_latent and shared_up run on three streams; passes follow each other
+    # without a wait, recorded (up to 256 tokens) and launched one by one
+    cfg = synthetic.baseline_config(max_tokens=300, experts=64, hidden=512, routed=256, shared=768,
+                                    latent=256)
+    data = synthetic.make_layer(cfg, seed=61, device="cuda", norm_weight_uniform=True,
+                                latent_family="fp8", shared_up_family="fp8")
+    beside = package.ExpertLayerSlice.create(cfg, data.bindings)
+    monkeypatch.setenv("NMOE_NO_SHARED_FORK", "1")
+    alone = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert beside is not None and alone is not None, package.ExpertLayerSlice.create_error
+    for tokens in (1, 2, 5, 65, 256, 257):
+        x = synthetic.make_tokens(tokens, cfg.hidden_size, seed=tokens, device="cuda")
+        want, outs = _run(alone, x), [torch.zeros(x.shape, device="cuda") for _ in range(6)]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for out in outs:
+                beside.run_async(x, out)
+            assert beside.sync_status() == 0
+        assert all(torch.equal(out, want) for out in outs)
+    beside.close()
+    alone.close()
+
+
 def test_unfused_activation_path_and_trace_fields(package, synthetic, oracle):
     cfg = synthetic.baseline_config(max_tokens=256, experts=32, hidden=512, routed=256, shared=512)
     data = synthetic.make_layer(cfg, seed=21, device="cuda", norm_weight_uniform=True)
