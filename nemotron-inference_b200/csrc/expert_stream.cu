@@ -87,7 +87,19 @@ static_assert(stages_for(32) * kBBytes >= 128 * 128, "A over-read stays inside s
 
 struct TileList {
   int first[kStreamPhases + 1];  // first tile of each phase, then the end
+  // The first row tiles of the grouped phases, two to a lane: a launch's first tile is looked up without
+  // another trip to memory, while its ticket is fetched (64 tokens 132.5 -> 131.3 us, 7 tokens 53.5 -> 53.2).
+  RowTile kept[2];
+  int kept_count;
+  // By all lanes of a warp; `ticket` is on its way meanwhile.
   __device__ __forceinline__ void load(const StreamArgs& args) {
+    const int lane = threadIdx.x & 31;
+    kept_count = min(64, args.row_tile_room);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      kept[i] = RowTile{};
+      if (lane + 32 * i < kept_count) kept[i] = args.row_tiles[lane + 32 * i];
+    }
     int running = 0;
 #pragma unroll
     for (int p = 0; p < kStreamPhases; ++p) {
@@ -120,10 +132,12 @@ struct TileList {
     const int rt = index / g.n_tiles;
     tile.nt = index - rt * g.n_tiles;
     if (g.row_tiles != nullptr) {
-      const RowTile row_tile = g.row_tiles[rt];
-      tile.row0 = warp_uniform(row_tile.row0);
-      tile.rows = warp_uniform(row_tile.rows);
-      tile.expert = warp_uniform(row_tile.expert);
+      RowTile row_tile = rt < 32 ? kept[0] : kept[1];
+      const int from = rt < kept_count ? rt & 31 : 0;
+      if (rt >= kept_count) row_tile = g.row_tiles[rt];
+      tile.row0 = __shfl_sync(0xffffffffu, row_tile.row0, from);
+      tile.rows = __shfl_sync(0xffffffffu, row_tile.rows, from);
+      tile.expert = __shfl_sync(0xffffffffu, row_tile.expert, from);
     } else {
       tile.row0 = rt * 128;
       tile.rows = min(128, g.dense_rows - tile.row0);
@@ -286,7 +300,6 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   if (warp == 0) {
     // ------------------------------------------------------- tiles and weights
     TileList list;
-    list.load(args);
     int slot = 0;
     uint32_t slot_phase = 0;
     int stage = 0;
@@ -296,7 +309,9 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       return args.ticket != nullptr && lane == 0 ? atomicAdd(args.ticket, 1) : dealt;
     };
     bool ok = true;
-    int t = warp_uniform(take(unit));
+    const int first = take(unit);
+    list.load(args);
+    int t = warp_uniform(first);
     while (ok) {
       const Tile tile = list.locate(args, t);
       if (!mbar_wait_warp(reader.empty0 + slot * 8, slot_phase ^ 1u)) {

@@ -166,6 +166,8 @@ struct StreamPhase {
 struct StreamArgs {
   StreamPhase phase[kStreamPhases];
   int32_t phases = 0;
+  const RowTile* row_tiles = nullptr;  // those of the grouped phases (all have the same), and how many
+  int32_t row_tile_room = 0;           // may be read
   int32_t tile_rows = 128;  // most rows a row tile holds: 32, 64 or 128
   int32_t* error = nullptr;
   // all `ready` words of the phases, the ticket the tiles are taken with and the count of CTAs that

@@ -511,6 +511,10 @@ void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCo
       }
     }
   };
+  if (routed != nullptr) {
+    args.row_tiles = routed->schedule.row_tiles;
+    args.row_tile_room = routed->row_slots;
+  }
   int32_t* routed_ready = args.ready;
   int32_t* shared_ready = args.ready + (routed != nullptr ? routed->row_slots : 0);
   args.ready_count = (routed != nullptr ? routed->row_slots : 0) +
