@@ -388,7 +388,8 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       const GemmArgs& g = ph.gemm;
       const int k_blocks = g.k_blocks;
       const int box = box_of(tile.rows);
-      const uint8_t* sfa_src = g.sfa + static_cast<size_t>(tile.row0 >> 7) * k_blocks * kSfaBytes;
+      const int a_row0 = ph.used != nullptr ? 0 : tile.row0;
+      const uint8_t* sfa_src = g.sfa + static_cast<size_t>(a_row0 >> 7) * k_blocks * kSfaBytes;
       if (ph.wait_target > 0) {
         ok = wait_count(ph.ready + (tile.row0 >> 7), ph.wait_target);
         fence_proxy_async();
@@ -397,7 +398,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
         ok = mbar_wait_warp(empty0 + stage * 8, phase ^ 1u);
         if (ok && elect_one()) {
           const uint32_t bar = full0 + stage * 8;
-          tma_load_2d_at(a0 + stage * a_room, &ph.a[box], kb * 128, tile.row0, bar);
+          tma_load_2d_at(a0 + stage * a_room, &ph.a[box], kb * 128, a_row0, bar);
           bulk_load_at(sfa0 + stage * kSfaBytes, sfa_src + kb * kSfaBytes, kSfaBytes, bar);
         }
         if (++stage == stages) {
@@ -510,11 +511,13 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       if (tile.phase < 0) break;
       const StreamPhase& ph = args.phase[tile.phase];
       const GemmArgs& g = ph.gemm;
-      const bool row_valid = r < tile.rows;
       const int grow = tile.row0 + r;
+      const bool row_valid = r < tile.rows && (ph.used == nullptr || ph.used[grow] >= 0);
       float scale = g.w_tensor_scale[tile.expert];
-      if (g.a_tensor_scale != nullptr && row_valid) scale *= g.a_tensor_scale[grow];
-      unsigned long long dest = 0;
+      if (g.a_tensor_scale != nullptr && row_valid) {
+        scale *= g.a_tensor_scale[ph.used != nullptr ? r : grow];
+      }
+      unsigned long long dest = row_valid ? 1 : 0;  // (up: whether the row counts)
       float wt = 1.0f;
       if (ph.mode == kGemmDown && row_valid) {
         dest = output_row_address(g, grow);
@@ -554,7 +557,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
             const float row_wt = __shfl_sync(0xffffffffu, wt, from & 31);
             const unsigned long long row_dest = __shfl_sync(0xffffffffu, dest, from & 31);
             const int n = n0 + half * (kBN / 2) + chunk * 16;
-            if (from >= tile.rows || chunk * 16 >= columns) continue;
+            if (from >= tile.rows || chunk * 16 >= columns || row_dest == 0) continue;
             float v[16];
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
@@ -571,7 +574,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
               *reinterpret_cast<uint2*>(hidden_codes(g, tile.row0 + from, n / 16)) =
                   make_uint2(lo, hi);
               *hidden_scale(g, tile.row0 + from, n / 16) = static_cast<uint8_t>(sf);
-            } else if (row_dest != 0) {
+            } else {
               store_chunk(g, v, n, row_dest, row_scale, row_wt);
             }
           }

@@ -158,6 +158,9 @@ struct StreamPhase {
   CUtensorMap b_tail;  // the partial last K block of the weights
   GemmArgs gemm;
   int32_t mode = kGemmUp;  // GemmMode
+  // Grouped phases whose row tiles hold all tokens in token order (csrc/front.cu): activation rows and
+  // their scales are those of the tokens, and rows that `used` names negative are of no use.
+  const int32_t* used = nullptr;
   // per 128-row slot: finished up tiles are counted here, down tiles wait for `wait_target` of
   // them (0 = their rows were complete before the launch)
   int32_t* ready = nullptr;
@@ -391,6 +394,52 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               float* sorted_weight, int32_t* sorted_dest,
                               int32_t* pair_row /* nullable */, int dest_stride, int32_t* error,
                               int num_sms, LaunchStream stream);
+// --- front end of a handful of tokens (csrc/front.cu) ---------------------------
+constexpr int kFrontMaxRows = 8;
+constexpr int kFrontMaxCols = 4096;
+constexpr int kFrontMaxExperts = 256;
+struct FrontArgs {
+  const void* in = nullptr;  // [rows][cols]
+  bool in_bf16 = false;
+  int rows = 0, cols = 0;
+  // launch_norm_quant's
+  const float* norm_weight = nullptr;
+  float eps = 0.0f;
+  float* normalized = nullptr;
+  uint8_t* packed = nullptr;
+  uint8_t* sf_row_major = nullptr;
+  uint8_t* sf_tiled = nullptr;
+  int k_tiles = 0;
+  float* tensor_scale = nullptr;
+  float* inv_rms = nullptr;
+  // the gate [experts][cols] and launch_router_topk's
+  const void* gate = nullptr;
+  bool gate_bf16 = false;
+  const float* logit_offset = nullptr;
+  const float* bias = nullptr;
+  int experts = 0, top_k = 0, n_group = 1, topk_group = 1;
+  bool norm_topk_prob = false;
+  float routed_scaling = 0.0f;
+  float* logits = nullptr;
+  int32_t* top_index = nullptr;
+  float* top_weight = nullptr;
+  // A row tile per selected expert, in expert order, that holds all `rows` tokens in token order: row r
+  // of tile i is row 128 * i + r of `dest` (token * dest_stride + slot, -1 where token r did not select
+  // the expert) and `row_weight`; `pair_row` [rows][top_k] says where a pair went.
+  RowTile* row_tiles = nullptr;
+  int32_t* num_row_tiles = nullptr;
+  int32_t* dest = nullptr;
+  float* row_weight = nullptr;
+  int32_t* pair_row = nullptr;
+  int dest_stride = 0;
+  void* scratch = nullptr;  // front_scratch_bytes(), zero before the first launch
+  int32_t* error = nullptr;
+};
+constexpr size_t front_scratch_bytes() {
+  return (kFrontMaxRows + 1) * sizeof(int32_t) + 2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
+}
+cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream);
+
 // --- expert-parallel dispatch / return (csrc/ep.cu) ---------------------------
 int dispatch_record_bytes(int cols);
 cudaError_t launch_dispatch_plan(const int32_t* expert_counts, int experts, int experts_per_rank,

@@ -468,6 +468,7 @@ struct StreamFfn {
   const ActivationOperand* hidden = nullptr;
   const float* hidden_tensor_scale = nullptr;
   RowOutput out;
+  const int32_t* used = nullptr;  // StreamPhase::used of the up projection
   int row_slots = 0;  // most 128-row slots the schedule may use
 };
 
@@ -503,6 +504,7 @@ void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCo
       set_row_output(&g, ffn.out);
     }
     set_phase(phase, up ? kGemmUp : kGemmDown, weights, a, g);
+    if (up) phase->used = ffn.used;
     if (ffn.up != nullptr) {
       phase->ready = ready;
       if (!up) {
@@ -1007,6 +1009,7 @@ struct nmoe_layer {
 
   ActivationOperand y_op, sh_op, a_op, h_op;
   StreamCounts stream_counts;
+  DeviceBuffer front_scratch;  // of csrc/front.cu
   ErrorSlot error;
   int last_tokens = 0;
   std::string last_error;
@@ -1157,6 +1160,7 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   // (an expert may leave a partly filled slot, and an empty one when pairs consume them)
   L->max_row_tiles = static_cast<int>(2 * static_cast<size_t>(EL) + (pairs + 127) / 128);
   L->stream_counts.allocate(L->max_row_tiles + token_slots);
+  L->front_scratch.allocate(front_scratch_bytes(), true);
   const size_t slots = static_cast<size_t>(L->max_row_tiles);
   L->counts.allocate(E * sizeof(int32_t), true);
   L->cursor.allocate(E * sizeof(int32_t), true);
@@ -1503,11 +1507,13 @@ TileClass routed_tile_class(const nmoe_layer* L, int pairs) {
 }
 
 // Plan + permute + the grouped GEMMs over `pairs` (row, slot) pairs whose per-local-expert
-// histogram is already in `counts`.  `shared` (stream class only): the shared expert's tiles join
+// histogram is already in `counts`.  `token_order`: csrc/front.cu has laid out the tiles, nothing is left
+// to plan or permute.  `shared` (stream class only): the shared expert's tiles join
 // the same launch.
 void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& source, int pairs,
                     int dest_stride, void* out_rows, RowKind out_kind,
-                    RowSegments segments = RowSegments(), const StreamFfn* shared = nullptr) {
+                    RowSegments segments = RowSegments(), const StreamFfn* shared = nullptr,
+                    bool token_order = false) {
   const int Lr = L->latent;
   int32_t* error = L->error.device.as<int32_t>();
   const TileClass routed_class = routed_tile_class(L, pairs);
@@ -1521,13 +1527,15 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
     NMOE_CUDA(cudaMemsetAsync(plan.expert_cursor, 0, L->local_experts * sizeof(int32_t), stream));
   }
   L->mark(4, stream);
-  NMOE_CUDA(launch_place_rows(plan, source, pairs, L->local_experts,
-                              routed_class == kClassPair ? 2 : 1, L->max_row_tiles, Lr,
-                              k_blocks_of(Lr), L->a_packed.as<uint8_t>(), L->a_sf.as<uint8_t>(),
-                              L->a_ts.as<float>(), L->a_weight.as<float>(),
-                              L->a_dest.as<int32_t>(),
-                              L->ep_world == 1 ? L->pair_row.as<int32_t>() : nullptr, dest_stride,
-                              error, L->num_sms, stream));
+  if (!token_order) {
+    NMOE_CUDA(launch_place_rows(plan, source, pairs, L->local_experts,
+                                routed_class == kClassPair ? 2 : 1, L->max_row_tiles, Lr,
+                                k_blocks_of(Lr), L->a_packed.as<uint8_t>(), L->a_sf.as<uint8_t>(),
+                                L->a_ts.as<float>(), L->a_weight.as<float>(),
+                                L->a_dest.as<int32_t>(),
+                                L->ep_world == 1 ? L->pair_row.as<int32_t>() : nullptr, dest_stride,
+                                error, L->num_sms, stream));
+  }
   if (!L->stage_timing) stream.chained = true;
   L->mark(5, stream);
   // routed experts (:896-954)
@@ -1546,8 +1554,9 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
     StreamFfn ffn;
     ffn.up = &L->up;
     ffn.down = &L->down;
-    ffn.a = &L->a_op;
-    ffn.a_tensor_scale = L->a_ts.as<float>();
+    ffn.a = token_order ? &L->y_op : &L->a_op;
+    ffn.a_tensor_scale = (token_order ? L->y_ts : L->a_ts).as<float>();
+    if (token_order) ffn.used = L->a_dest.as<int32_t>();
     ffn.schedule = routed;
     ffn.hidden_packed = L->h_packed.as<uint8_t>();
     ffn.hidden_sf = L->h_sf.as<uint8_t>();
@@ -1683,6 +1692,55 @@ PermuteSource local_source(nmoe_layer* L) {
   return source;
 }
 
+// Everything in front of the experts in one launch (csrc/front.cu).
+void route_few(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype in_dtype,
+               int tokens) {
+  const nmoe_config& c = L->cfg;
+  FrontArgs args;
+  args.in = input;
+  args.in_bf16 = in_dtype == NMOE_BF16;
+  args.rows = tokens;
+  args.cols = c.hidden_size;
+  args.norm_weight = L->norm_weight.as<float>();
+  args.eps = c.rms_epsilon;
+  args.normalized = L->normalized.as<float>();
+  args.packed = L->y_packed.as<uint8_t>();
+  args.sf_row_major = L->y_sf_row_major.as<uint8_t>();
+  args.sf_tiled = L->y_sf_tiled.as<uint8_t>();
+  args.k_tiles = k_blocks_of(c.hidden_size) * 4;
+  args.tensor_scale = L->y_ts.as<float>();
+  args.inv_rms = L->inv_rms.as<float>();
+  args.gate = L->gate_exact.w.weight;
+  args.gate_bf16 = L->gate_exact.w.kind == kWeightBf16;
+  args.logit_offset = L->has_logit_offset ? L->logit_offset.as<float>() : nullptr;
+  args.bias = L->bias.as<float>();
+  args.experts = c.n_routed_experts;
+  args.top_k = c.top_k;
+  args.n_group = c.n_group;
+  args.topk_group = c.topk_group;
+  args.norm_topk_prob = c.norm_topk_prob != 0;
+  args.routed_scaling = c.routed_scaling_factor;
+  args.logits = L->logits.as<float>();
+  args.top_index = L->top_index.as<int32_t>();
+  args.top_weight = L->top_weight.as<float>();
+  args.row_tiles = L->row_tiles.as<RowTile>();
+  args.num_row_tiles = L->num_row_tiles.as<int32_t>();
+  args.dest = L->a_dest.as<int32_t>();
+  args.row_weight = L->a_weight.as<float>();
+  args.pair_row = L->pair_row.as<int32_t>();
+  args.dest_stride = c.top_k + 1;
+  args.scratch = L->front_scratch.as<void>();
+  args.error = L->error.device.as<int32_t>();
+  NMOE_CUDA(launch_front(args, stream));
+  L->last_normalized = true;
+}
+
+// Whether csrc/front.cu takes a batch.
+bool front_takes(const nmoe_layer* L, int tokens) {
+  return tokens <= kFrontMaxRows && L->cfg.hidden_size <= kFrontMaxCols &&
+         L->cfg.n_routed_experts <= kFrontMaxExperts && L->has_gate_exact;
+}
+
 // A latent layer's three chains behind the norm -- gate and selection; fc1_latent and its quantiser;
 // shared_up and its quantiser -- meet only in front of the experts.  On streams of their own one fills
 // what another leaves idle: latency at a few tokens, SMs at a hundred, last waves at a thousand.  Whole
@@ -1718,8 +1776,14 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   const bool beside = L->latent_stream != nullptr && one_launch && L->latent_mode &&
                       !L->stage_timing && tokens >= kBesideMinTokens &&
                       tokens <= L->fork_max_tokens;
-  route_tokens(L, chain, input, in_dtype, tokens, fork || beside ? L->quant_done : nullptr,
-               fork && two_pass);
+  const bool few = front_takes(L, tokens) && one_launch && !L->latent_mode && !dense_shared &&
+                   !two_pass && !L->stage_timing;
+  if (few) {
+    route_few(L, stream, input, in_dtype, tokens);
+  } else {
+    route_tokens(L, chain, input, in_dtype, tokens, fork || beside ? L->quant_done : nullptr,
+                 fork && two_pass);
+  }
   L->last_tokens = tokens;
   L->last_parts_kind = parts_kind;
   L->last_unfused = L->unfused;
@@ -1798,7 +1862,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
     const StreamFfn shared =
         shared_stream_ffn(L, tokens, L->parts.as<void>(), K + 1, K, parts_kind);
     routed_experts(L, chain, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind,
-                   RowSegments(), &shared);
+                   RowSegments(), &shared, few);
   } else {
     routed_experts(L, chain, local_source(L), tokens * K, K + 1, L->parts.as<void>(), parts_kind);
   }

@@ -48,6 +48,33 @@ def test_pairs_share_rows_of_every_count(package, synthetic):
     layer.close()
 
 
+# up to eight tokens, 4096 columns and 256 experts have one launch in front of the experts; the stages
+# are timed through the four launches it stands for
+@pytest.mark.parametrize("experts,hidden,top_k,groups", [(32, 448, 6, 1), (256, 1024, 32, 4),
+                                                         (96, 4096, 1, 1), (128, 4160, 8, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_front_end_of_a_few_tokens(package, synthetic, experts, hidden, top_k, groups, dtype):
+    cfg = synthetic.baseline_config(max_tokens=16, experts=experts, hidden=hidden, routed=64,
+                                    shared=128, top_k=top_k)
+    cfg.n_group, cfg.topk_group = groups, max(1, groups // 2)
+    data = synthetic.make_layer(cfg, seed=experts, device="cuda", norm_weight_uniform=True,
+                                skewed=experts == 32)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (1, 2, 4, 5, 8, 9):
+        x = synthetic.make_tokens(tokens, hidden, seed=tokens, device="cuda").to(dtype)
+        out, launches = (torch.empty(x.shape, device="cuda") for _ in range(2))
+        layer.enable_stage_timing(True)
+        assert layer.run(x, launches), layer.last_error
+        layer.enable_stage_timing(False)
+        for _ in range(2):
+            assert layer.run(x, out), layer.last_error
+            assert torch.equal(out, launches)
+        rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+        assert rep.ok(), rep.summary()
+    layer.close()
+
+
 @pytest.mark.parametrize("rows", [3, 1185])
 @pytest.mark.parametrize("cols", [16, 1008, 2048, 2064, 4096, 4112, 5376, 6144, 6160])
 def test_quantiser_row_lengths(package, oracle, rows, cols):
