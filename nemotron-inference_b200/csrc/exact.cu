@@ -22,6 +22,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "quant_row.cuh"
 
 namespace nmoe {
 namespace {
@@ -91,13 +92,14 @@ constexpr int kExactChunk = 64;  // bytes of K per pipeline stage (64-byte swizz
 // Where the 8 bytes of row `row`, slice `slice`, columns k .. k + 7 go.  A tile of `tile_rows` rows
 // keeps every 64-byte chunk of K as one contiguous piece, [slice][row][64], already in the shared-
 // memory image of the tensor core's 64-byte swizzle, so that a stage is one bulk copy.
+template <int SLICES>
 __device__ __forceinline__ size_t slice_offset(size_t row, int slice, int k, int K,
                                                int tile_rows) {
   const size_t tile = row / tile_rows;
   const int r = static_cast<int>(row - tile * tile_rows);
   const size_t chunk = tile * (K / kExactChunk) + k / kExactChunk;
   const int c = k & (kExactChunk - 1);
-  return (chunk * kSlices + slice) * (static_cast<size_t>(tile_rows) * kExactChunk) +
+  return (chunk * SLICES + slice) * (static_cast<size_t>(tile_rows) * kExactChunk) +
          r * kExactChunk + ((((c >> 4) ^ (r >> 1)) & 3) << 4) + (c & 15);
 }
 
@@ -170,7 +172,7 @@ slice_rows_kernel(const void* __restrict__ in, int K, float scale, int tile_rows
     }
 #pragma unroll
     for (int i = 0; i < kSlices; ++i) {
-      *reinterpret_cast<uint2*>(slices + slice_offset(row, i, k, K, tile_rows)) =
+      *reinterpret_cast<uint2*>(slices + slice_offset<kSlices>(row, i, k, K, tile_rows)) =
           make_uint2(words[i][0], words[i][1]);
     }
   }
@@ -216,9 +218,18 @@ void launch_slices(const void* in, int rows, int K, float scale, int tile_rows, 
 // is at 32 % of its read and 13 % of its write rate).  With the two kernels around it 13,800 -> 370 us;
 // 40 rows 381 -> 44 us.
 // ---------------------------------------------------------------------------
-constexpr int kExactStages = 3;
 constexpr int kExactThreads = 6 * 32;
-constexpr int kExactABytes = kSlices * kExactRows * kExactChunk;
+// A product of matrices of SLICES digits: five of rows in fixed point (above), or the three of E4M3
+// codes as whole numbers (below), whose nine products are all computed.
+template <int SLICES>
+struct ExactShape {
+  static constexpr int kLevels = SLICES == kSlices ? nmoe::kLevels : 2 * SLICES - 1;
+  static constexpr int kStages = SLICES == kSlices ? 3 : 5;
+  static constexpr int kABytes = SLICES * kExactRows * kExactChunk;
+  static constexpr int smem_bytes(int nt) {
+    return kStages * (kABytes + SLICES * nt * kExactChunk) + (2 * kStages + 1) * 8 + 16 + 1024;
+  }
+};
 
 __device__ __forceinline__ void tcgen05_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                                uint32_t idesc, uint32_t accumulate) {
@@ -238,12 +249,13 @@ __device__ __forceinline__ uint32_t make_idesc_i8(uint32_t n) {
 // The products of one 32-byte step of K: digit I of W times its token digits, from the given shared-
 // memory descriptors.  A level that digit I is the first to reach is an MMA of its own, so that it
 // can start the sum when `first`.
-template <int NT, int I>
+template <int SLICES, int NT, int I>
 __device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t a_desc, uint64_t b_desc,
                                             bool first) {
+  constexpr int kLevels = ExactShape<SLICES>::kLevels;
   constexpr int kMost = 256 / NT;                                      // token digits of one MMA
-  constexpr int kMeet = kSlices < kLevels - I ? kSlices : kLevels - I;  // ... within the levels
-  constexpr bool kStarts = I > 0 && I <= kLevels - kSlices;
+  constexpr int kMeet = SLICES < kLevels - I ? SLICES : kLevels - I;  // ... within the levels
+  constexpr bool kStarts = I > 0 && I <= kLevels - SLICES;
   constexpr int kTogether = kStarts ? kMeet - 1 : kMeet;
   const uint64_t a = advance_smem_desc(a_desc, I * kExactRows * kExactChunk);
 #pragma unroll
@@ -260,21 +272,24 @@ __device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t a_desc, uint
   }
 }
 
-template <int NT>
+// `values` (only without splits): FP32 results, the sums times `scale`, in the place of `partial`.
+template <int SLICES, int NT>
 __global__ void __launch_bounds__(kExactThreads, 1)
 exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict__ x_slices,
-                  int rows, int N, int K, int row_tiles, int splits,
-                  double* __restrict__ partial, int32_t* error) {
+                  int rows, int N, int K, int row_tiles, int splits, double* __restrict__ partial,
+                  float* __restrict__ values, double scale, int32_t* error) {
+  using Shape = ExactShape<SLICES>;
+  constexpr int kLevels = Shape::kLevels, kStages = Shape::kStages, kABytes = Shape::kABytes;
   constexpr int nt = NT;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) &
                                              ~static_cast<uintptr_t>(1023u));
-  constexpr int b_bytes = kSlices * nt * kExactChunk;
+  constexpr int b_bytes = SLICES * nt * kExactChunk;
   uint8_t* sA = smem;
-  uint8_t* sB = sA + kExactStages * kExactABytes;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sB + kExactStages * b_bytes);
-  uint64_t* empty_bar = full_bar + kExactStages;
-  uint64_t* done_bar = empty_bar + kExactStages;
+  uint8_t* sB = sA + kStages * kABytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sB + kStages * b_bytes);
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* done_bar = empty_bar + kStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
 
   const int warp = warp_uniform(static_cast<int>(threadIdx.x >> 5));
@@ -291,7 +306,7 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
   const int chunks = all_chunks * (split + 1) / splits - chunk0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kExactStages; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -312,7 +327,7 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
 
   if (warp == 0) {
     const int8_t* w_from =
-        w_slices + (static_cast<size_t>(n0 / kExactRows) * all_chunks + chunk0) * kExactABytes;
+        w_slices + (static_cast<size_t>(n0 / kExactRows) * all_chunks + chunk0) * kABytes;
     const int8_t* x_from =
         x_slices + (static_cast<size_t>(row_tile) * all_chunks + chunk0) * b_bytes;
     int stage = 0;
@@ -324,13 +339,13 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
       }
       if (elect_one()) {
         const uint32_t bar = full0 + stage * 8;
-        mbar_arrive_expect_tx_at(bar, kExactABytes + b_bytes);
-        bulk_load_at(a0 + stage * kExactABytes, w_from, kExactABytes, bar);
+        mbar_arrive_expect_tx_at(bar, kABytes + b_bytes);
+        bulk_load_at(a0 + stage * kABytes, w_from, kABytes, bar);
         bulk_load_at(b0 + stage * b_bytes, x_from, b_bytes, bar);
       }
-      w_from += kExactABytes;
+      w_from += kABytes;
       x_from += b_bytes;
-      if (++stage == kExactStages) {
+      if (++stage == kStages) {
         stage = 0;
         phase ^= 1u;
       }
@@ -351,19 +366,21 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
       if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < kExactChunk / 32; ++ks) {
-          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * kExactABytes + ks * 32);
+          const uint64_t a_desc = advance_smem_desc(a_desc0, stage * kABytes + ks * 32);
           const uint64_t b_desc = advance_smem_desc(b_desc0, stage * b_bytes + ks * 32);
           const bool first = ks == 0 && c == 0;
-          static_assert(kSlices == 5, "one call per digit");
-          issue_digit<NT, 0>(tmem_base, a_desc, b_desc, first);
-          issue_digit<NT, 1>(tmem_base, a_desc, b_desc, first);
-          issue_digit<NT, 2>(tmem_base, a_desc, b_desc, first);
-          issue_digit<NT, 3>(tmem_base, a_desc, b_desc, first);
-          issue_digit<NT, 4>(tmem_base, a_desc, b_desc, first);
+          static_assert(SLICES == 5 || SLICES == 3, "one call per digit");
+          issue_digit<SLICES, NT, 0>(tmem_base, a_desc, b_desc, first);
+          issue_digit<SLICES, NT, 1>(tmem_base, a_desc, b_desc, first);
+          issue_digit<SLICES, NT, 2>(tmem_base, a_desc, b_desc, first);
+          if constexpr (SLICES == 5) {
+            issue_digit<SLICES, NT, 3>(tmem_base, a_desc, b_desc, first);
+            issue_digit<SLICES, NT, 4>(tmem_base, a_desc, b_desc, first);
+          }
         }
         tcgen05_commit_at(empty0 + stage * 8);
       }
-      if (++stage == kExactStages) {
+      if (++stage == kStages) {
         stage = 0;
         phase ^= 1u;
       }
@@ -377,6 +394,7 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
       tcgen05_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
       double* out = partial + static_cast<size_t>(split) * rows * N;
+      const bool as_values = values != nullptr;
       for (int c = 0; c < nt && row0 + c < rows; c += 16) {
         double sum[16];
 #pragma unroll
@@ -392,7 +410,13 @@ exact_gemm_kernel(const int8_t* __restrict__ w_slices, const int8_t* __restrict_
         if (n < N) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            if (row0 + c + i < rows) out[static_cast<size_t>(row0 + c + i) * N + n] = sum[i];
+            if (row0 + c + i >= rows) break;
+            const size_t at = static_cast<size_t>(row0 + c + i) * N + n;
+            if (as_values) {
+              values[at] = static_cast<float>(sum[i] * scale);
+            } else {
+              out[at] = sum[i];
+            }
           }
         }
       }
@@ -542,6 +566,284 @@ exact_finish_kernel(const double* __restrict__ partial, int splits, int rows, in
     if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
     out[i] = result;
   }
+}
+
+// ---------------------------------------------------------------------------
+// E4M3 times E4M3 that only has to be quantised again
+//
+// The scaled-FP8 family rounds its activations to E4M3 as well, so both operands are codes times a
+// scale.  A code is a whole number of 2^-9 below 2^18, three digits, and the nine products of two give
+// the sum of the codes' products, S, as a whole number.  The reference multiplies FP32 values,
+// RN(code * scale), which is S times the scales to within 2^-23 of the sum of the magnitudes: too far to
+// say the FP32 result, but a relu^2 row that is quantised to FP4 next needs only the side of a rounding
+// boundary.  So every block is quantised twice, from both ends of what its values can be, by the steps
+// that are monotone in them; where the two disagree (one block in a thousand) the values in doubt are
+// summed in FP64 like those that exact_finish_kernel leaves open.  Codes and scales are therefore those
+// of the correctly rounded sums.
+// The checkpoint's shared_up, 1000 rows (ncu, us): digits of the rows 17 -> 12, product 323 -> 146 (bound
+// by what an SM takes in, 39 KB in the 720 cycles that a stage's MMAs take), rounding and quantising
+// 43 + 10 -> 36.  Whole pass with the linears beside it, 1000 rows 962 -> 795 us, 40 rows 356 -> 343.
+// ---------------------------------------------------------------------------
+constexpr int kCodeSlices = 3;
+constexpr int kCodeTile = 80;  // token rows: five levels of 80 columns in TMEM, N = 240 in one MMA
+
+__device__ __forceinline__ int code_integer(uint32_t code) {
+  const int e = (code >> 3) & 15, m = code & 7;
+  const int magnitude = e == 0 ? m : (8 + m) << (e - 1);
+  return code & 0x80u ? -magnitude : magnitude;
+}
+
+// One block per row: its codes, the codes as three digits, and an upper bound of their 2-norm (an infinity
+// where a code is no number).  WEIGHT: the row is E4M3 codes already.
+template <bool WEIGHT>
+__global__ void __launch_bounds__(kSliceThreads)
+code_rows_kernel(const void* __restrict__ in, int K, float scale, int tile_rows,
+                 int8_t* __restrict__ slices, uint8_t* __restrict__ codes_out,
+                 float* __restrict__ norm) {
+  __shared__ float warp_sum[kSliceThreads / 32];
+  const size_t row = blockIdx.x;
+  float squares = 0.0f;
+  for (int k = static_cast<int>(threadIdx.x) * 8; k < K; k += kSliceThreads * 8) {
+    uint32_t codes[8];
+    if constexpr (WEIGHT) {
+      const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(in) +
+                                                        row * K + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) codes[j] = ((j < 4 ? raw.x : raw.y) >> (8 * (j & 3))) & 0xffu;
+    } else {
+      const float4* from =
+          reinterpret_cast<const float4*>(reinterpret_cast<const float*>(in) + row * K + k);
+      const float4 a = from[0], b = from[1];
+      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) codes[j] = encode_e4m3(__fdiv_rn(v[j], scale)) & 0xffu;
+      *reinterpret_cast<uint2*>(codes_out + row * K + k) =
+          make_uint2(codes[0] | codes[1] << 8 | codes[2] << 16 | codes[3] << 24,
+                     codes[4] | codes[5] << 8 | codes[6] << 16 | codes[7] << 24);
+    }
+    uint32_t words[kCodeSlices][2] = {};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const bool number = (codes[j] & 0x7fu) != 0x7fu;
+      int m = number ? code_integer(codes[j]) : 0;
+      squares = number ? fmaf(static_cast<float>(m), static_cast<float>(m), squares) : INFINITY;
+#pragma unroll
+      for (int i = kCodeSlices - 1; i >= 0; --i) {
+        const int8_t d = static_cast<int8_t>(m & 0xff);
+        m = (m - d) >> 8;
+        words[i][j >> 2] |= static_cast<uint32_t>(static_cast<uint8_t>(d)) << (8 * (j & 3));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kCodeSlices; ++i) {
+      *reinterpret_cast<uint2*>(slices + slice_offset<kCodeSlices>(row, i, k, K, tile_rows)) =
+          make_uint2(words[i][0], words[i][1]);
+    }
+  }
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1) {
+    squares += __shfl_xor_sync(0xffffffffu, squares, stride);
+  }
+  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = squares;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float total = 0.0f;
+    for (int w = 0; w < kSliceThreads / 32; ++w) total += warp_sum[w];
+    // (K <= 16384 additions lose less than 2^-10 of the sum)
+    norm[row] = sqrtf(total) * 1.002f;
+  }
+}
+
+// FP64 sum of one value by a warp, from the codes of both rows.
+__device__ __forceinline__ float exact_value(const uint8_t* x, float fp8_scale, const uint8_t* w,
+                                             float weight_scale, int K) {
+  using Vector = WeightVector<kWeightFp8>;
+  double sum = 0.0;
+#pragma unroll 2
+  for (int q = threadIdx.x & 31; q * Vector::kCount < K; q += 32) {
+    float a[Vector::kCount], v[Vector::kCount];
+    Vector::unpack(reinterpret_cast<const uint4*>(x)[q], fp8_scale, a);
+    Vector::unpack(reinterpret_cast<const uint4*>(w)[q], weight_scale, v);
+#pragma unroll
+    for (int j = 0; j < Vector::kCount; ++j) {
+      sum = fma(static_cast<double>(a[j]), static_cast<double>(v[j]), sum);
+    }
+  }
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, stride);
+  }
+  return static_cast<float>(sum);
+}
+
+__device__ __forceinline__ float relu_squared(float r) { return r > 0.0f ? __fmul_rn(r, r) : 0.0f; }
+
+__device__ __forceinline__ float (&eight_of(float (&v)[16], int i))[8] {
+  return *reinterpret_cast<float(*)[8]>(&v[i]);
+}
+
+// Largest `v` of the block's threads (none is negative).
+__device__ __forceinline__ float block_max_of(float v, float* warp_values) {
+  const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) warp_values[threadIdx.x >> 5] = __uint_as_float(most);
+  __syncthreads();
+  float all = 0.0f;
+  for (int w = 0; w < static_cast<int>(blockDim.x) / 32; ++w) all = fmaxf(all, warp_values[w]);
+  return all;
+}
+
+// relu^2 and NVFP4 of a row (nvfp4_packing.cpp:119-153) from values known to within a bound; one block
+// per row, one thread per 16-element block.  `values`, or the doubles of a split product.
+__global__ void __launch_bounds__(1024)
+coded_quant_kernel(const float* __restrict__ values,
+                                   const double* __restrict__ partial, int splits, double scale,
+                                   int rows, int N, int K, const uint8_t* __restrict__ in,
+                                   float fp8_scale, const float* __restrict__ in_norm,
+                                   const uint8_t* __restrict__ weight, float weight_scale,
+                                   const float* __restrict__ weight_norm, int first_row,
+                                   uint8_t* __restrict__ packed, uint8_t* __restrict__ sf_tiled,
+                                   int k_tiles, float* __restrict__ tensor_scale) {
+  constexpr int kListed = 256;  // values summed per round
+  __shared__ float warp_values[32];
+  __shared__ int list[kListed];
+  __shared__ float sums[kListed];
+  __shared__ int listed;
+  const int row = blockIdx.x, n0 = static_cast<int>(threadIdx.x) * 16;
+  const bool active = n0 < N;
+  const size_t at = static_cast<size_t>(row) * N + n0;
+  const uint8_t* x = in + static_cast<size_t>(row) * K;
+  float low[16], high[16];
+  {
+    // 2^-23 of the magnitudes for the operands' roundings, 2^-24 each for those of the result and of
+    // `values`; the factors make up for the roundings of the bounds
+    const float unit = static_cast<float>(scale) * in_norm[row] * 1.2e-7f;
+    float known_as[16], norms[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) known_as[i] = norms[i] = 0.0f;
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 8) load8<false>(weight_norm, n0 + i, eight_of(norms, i));
+      if (values != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 8) load8<false>(values, at + i, eight_of(known_as, i));
+      } else {
+        double sums_of[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sums_of[i] = 0.0;
+        for (int p = 0; p < splits; ++p) {
+          const double2* from =
+              reinterpret_cast<const double2*>(partial + at + static_cast<size_t>(p) * rows * N);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const double2 two = from[i];
+            sums_of[2 * i] += two.x;
+            sums_of[2 * i + 1] += two.y;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) known_as[i] = static_cast<float>(sums_of[i] * scale);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float r = known_as[i];
+      const float bound =
+          active ? fmaf(fabsf(r), 1.2e-7f, fmaf(unit, norms[i], 1e-37f)) : 0.0f;
+      // (a bound that is no number, or none: the value is summed)
+      const bool known = bound < 1e30f;
+      low[i] = known ? relu_squared(__fsub_rd(r, bound)) : 0.0f;
+      high[i] = known ? relu_squared(__fadd_ru(r, bound)) : INFINITY;
+    }
+  }
+  // Sums the values that the threads name in `which`, a warp each.
+  auto settle = [&](uint32_t which) {
+    while (__syncthreads_or(which != 0u)) {
+      if (threadIdx.x == 0) listed = 0;
+      __syncthreads();
+      int first = kListed;
+      bool fits = false;
+      if (which != 0u) {
+        first = atomicAdd(&listed, __popc(which));
+        fits = first + __popc(which) <= kListed;
+        int at = first;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (((which >> i) & 1u) != 0u && at < kListed) list[at++] = fits ? n0 + i : -1;
+        }
+      }
+      __syncthreads();
+      const int count = min(listed, kListed);
+      for (int at = threadIdx.x >> 5; at < count; at += static_cast<int>(blockDim.x) / 32) {
+        const int n = list[at];
+        if (n < 0) continue;
+        const float sum = exact_value(x, fp8_scale, weight + static_cast<size_t>(n) * K,
+                                      weight_scale, K);
+        if ((threadIdx.x & 31) == 0) sums[at] = relu_squared(sum);
+      }
+      __syncthreads();
+      if (fits) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (((which >> i) & 1u) != 0u) low[i] = high[i] = sums[first++];
+        }
+        which = 0;
+      }
+    }
+  };
+  // those of this thread that are open and may be as large as `least`
+  auto open_from = [&](float least) {
+    uint32_t which = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) which |= (low[i] != high[i] && high[i] >= least ? 1u : 0u) << i;
+    return which;
+  };
+  auto largest = [&](const float (&v)[16]) {
+    float most = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) most = fmaxf(most, v[i]);
+    return most;
+  };
+  // the row's tensor scale is 1 unless its largest value is beyond 6 * 448
+  float ts = 1.0f;
+  if (block_max_of(largest(high), warp_values) > kFp4Max * kFp8Max) {
+    settle(open_from(block_max_of(largest(low), warp_values)));
+    const float amax = block_max_of(largest(low), warp_values);
+    if (amax > kFp4Max * kFp8Max) ts = clamp_scale(__fdiv_rn(amax, kFp4Max * kFp8Max));
+  }
+  const float scale_divisor = __fmul_rn(kFp4Max, ts), scale_reciprocal = __frcp_rn(scale_divisor);
+  uint32_t in_doubt = 0;
+  {
+    const float low_scale = block_scale(largest(low), scale_divisor, scale_reciprocal);
+    const float high_scale = block_scale(largest(high), scale_divisor, scale_reciprocal);
+    const float low_divisor = __fmul_rn(ts, low_scale), high_divisor = __fmul_rn(ts, high_scale);
+    const float low_reciprocal = __frcp_rn(low_divisor), high_reciprocal = __frcp_rn(high_divisor);
+#pragma unroll
+    for (int i = 0; i < 16; i += 8) {
+      const uint32_t differ =
+          quantize_half_block(eight_of(low, i), high_divisor, high_reciprocal) ^
+          quantize_half_block(eight_of(high, i), low_divisor, low_reciprocal);
+      if (differ != 0u) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          in_doubt |= (((differ >> (4 * j)) & 15u) != 0u ? 1u : 0u) << (i + j);
+        }
+      }
+    }
+    // what the scale follows from is settled with the values that hang on it
+    if (encode_e4m3(low_scale) != encode_e4m3(high_scale)) in_doubt |= 0x10000u;
+    if (in_doubt != 0u) in_doubt = (in_doubt & open_from(0.0f)) | open_from(largest(low));
+  }
+  settle(in_doubt);
+  if (!active) return;
+  const float bs = block_scale(largest(high), scale_divisor, scale_reciprocal);
+  const float divisor = __fmul_rn(ts, bs), reciprocal = __frcp_rn(divisor);
+  const size_t out_row = static_cast<size_t>(first_row) + row;
+  *reinterpret_cast<uint2*>(packed + out_row * (N / 2) + n0 / 2) =
+      make_uint2(quantize_half_block(eight_of(high, 0), divisor, reciprocal),
+                 quantize_half_block(eight_of(high, 8), divisor, reciprocal));
+  sf_tiled[swizzled_scale_offset(out_row, n0 / 16, k_tiles)] = static_cast<uint8_t>(encode_e4m3(bs));
+  if (threadIdx.x == 0) tensor_scale[out_row] = ts;
 }
 
 // ---------------------------------------------------------------------------
@@ -934,19 +1236,19 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
   const int row_tiles = (rows + nt - 1) / nt;
   const int splits = exact_splits(rows, w.N, w.K, num_sms);
   const int grid = (w.N + kExactRows - 1) / kExactRows * row_tiles * splits;
-  const int smem = kExactStages * (kExactABytes + kSlices * nt * kExactChunk) +
-                   (2 * kExactStages + 1) * 8 + 16 + 1024;
-  auto multiply = [&](auto kernel) {
+  auto multiply = [&](auto kernel, int smem) {
     const cudaError_t attribute = allow_shared_memory(kernel);
     if (attribute != cudaSuccess) return attribute;
     kernel<<<grid, kExactThreads, smem, stream>>>(w.slices, space.slices, rows, w.N, w.K, row_tiles,
-                                                  splits, space.partial, error);
+                                                  splits, space.partial, nullptr, 0.0, error);
     return cudaGetLastError();
   };
-  const cudaError_t err = nt == 16   ? multiply(exact_gemm_kernel<16>)
-                          : nt == 32 ? multiply(exact_gemm_kernel<32>)
-                          : nt == 48 ? multiply(exact_gemm_kernel<48>)
-                                     : multiply(exact_gemm_kernel<64>);
+  using Shape = ExactShape<kSlices>;
+  const cudaError_t err =
+      nt == 16   ? multiply(exact_gemm_kernel<kSlices, 16>, Shape::smem_bytes(16))
+      : nt == 32 ? multiply(exact_gemm_kernel<kSlices, 32>, Shape::smem_bytes(32))
+      : nt == 48 ? multiply(exact_gemm_kernel<kSlices, 48>, Shape::smem_bytes(48))
+                 : multiply(exact_gemm_kernel<kSlices, 64>, Shape::smem_bytes(64));
   if (err != cudaSuccess) return err;
   const dim3 blocks((w.N + kFinishThreads - 1) / kFinishThreads, rows, 1);
   auto run = [&](auto kernel) {
@@ -961,6 +1263,70 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
   } else {
     run(exact_finish_kernel<kWeightF32>);
   }
+  return cudaGetLastError();
+}
+
+// Whether a weight's codes times `scale` are FP32 values rounded to 24 bits, none of them subnormal or
+// infinite, and a row fits one block's threads.
+bool coded_supported(int N, int K, float weight_scale) {
+  return exact_supported(N, K) && N % 16 == 0 && N <= 16 * 1024 && weight_scale >= 0x1p-80f &&
+         weight_scale <= 0x1p60f;
+}
+
+int coded_weight_tile_rows() { return kExactRows; }
+size_t coded_slice_bytes(size_t rows, int K, int tile_rows) {
+  return (rows + tile_rows - 1) / tile_rows * tile_rows * K * kCodeSlices;
+}
+
+cudaError_t launch_code_weights(const void* weight, int N, int K, int8_t* slices, float* norm,
+                                cudaStream_t stream) {
+  code_rows_kernel<true><<<N, kSliceThreads, 0, stream>>>(weight, K, 1.0f, kExactRows, slices, nullptr,
+                                                          norm);
+  return cudaGetLastError();
+}
+
+// Token rows per tile: as many as there is TMEM for, fewer when there are fewer.
+static int coded_tile_rows(int rows) {
+  return rows > kCodeTile - 16 ? kCodeTile : (rows + 15) / 16 * 16;
+}
+
+cudaError_t launch_coded_linear(const CodedWeight& w, const float* in, int rows, float fp8_scale,
+                                const ExactWorkspace& space, int first_row, uint8_t* packed,
+                                uint8_t* sf_tiled, int k_tiles, float* tensor_scale, int32_t* error,
+                                int num_sms, cudaStream_t stream) {
+  if (rows <= 0 || !coded_supported(w.N, w.K, w.scale) || !(fp8_scale >= kMinScale) ||
+      fp8_scale > 0x1p60f) {
+    return cudaErrorInvalidValue;
+  }
+  const int nt = coded_tile_rows(rows);
+  float* norm = reinterpret_cast<float*>(space.info);
+  // (behind the three digits; the workspace has room for five)
+  uint8_t* codes = reinterpret_cast<uint8_t*>(space.slices) + coded_slice_bytes(rows, w.K, nt);
+  code_rows_kernel<false><<<rows, kSliceThreads, 0, stream>>>(in, w.K, fp8_scale, nt, space.slices,
+                                                              codes, norm);
+  const int row_tiles = (rows + nt - 1) / nt;
+  const int tiles = (w.N + kExactRows - 1) / kExactRows * row_tiles;
+  const int splits = std::max(1, std::min(num_sms / tiles, w.K / kExactChunk));
+  float* values = splits == 1 ? reinterpret_cast<float*>(space.partial) : nullptr;
+  const double scale = 0x1p-18 * static_cast<double>(fp8_scale) * static_cast<double>(w.scale);
+  auto multiply = [&](auto kernel) {
+    const cudaError_t attribute = allow_shared_memory(kernel);
+    if (attribute != cudaSuccess) return attribute;
+    kernel<<<tiles * splits, kExactThreads, ExactShape<kCodeSlices>::smem_bytes(nt), stream>>>(
+        w.slices, space.slices, rows, w.N, w.K, row_tiles, splits, space.partial, values, scale,
+        error);
+    return cudaGetLastError();
+  };
+  const cudaError_t err = nt == 16   ? multiply(exact_gemm_kernel<kCodeSlices, 16>)
+                          : nt == 32 ? multiply(exact_gemm_kernel<kCodeSlices, 32>)
+                          : nt == 48 ? multiply(exact_gemm_kernel<kCodeSlices, 48>)
+                          : nt == 64 ? multiply(exact_gemm_kernel<kCodeSlices, 64>)
+                                     : multiply(exact_gemm_kernel<kCodeSlices, kCodeTile>);
+  if (err != cudaSuccess) return err;
+  coded_quant_kernel<<<rows, (w.N / 16 + 31) / 32 * 32, 0, stream>>>(
+      values, space.partial, splits, scale, rows, w.N, w.K, codes, fp8_scale, norm,
+      reinterpret_cast<const uint8_t*>(w.weight), w.scale, w.norm, first_row, packed, sf_tiled,
+      k_tiles, tensor_scale);
   return cudaGetLastError();
 }
 

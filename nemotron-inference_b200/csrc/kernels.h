@@ -334,6 +334,27 @@ cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_s
                               const float* offset, bool relu2, float* out, int num_sms,
                               LaunchStream stream);
 
+// relu^2 and NVFP4 of a scaled-FP8 linear's rows (csrc/exact.cu): the codes, block scales and tensor
+// scales that launch_norm_quant gives for the rows that launch_exact_linear computes.
+struct CodedWeight {
+  int N = 0, K = 0;
+  const void* weight = nullptr;    // [N][K] E4M3 codes, times `scale`; 16-byte aligned
+  float scale = 1.0f;
+  const int8_t* slices = nullptr;  // coded_slice_bytes(N, K, coded_weight_tile_rows()) bytes, zero
+                                   // where no row is; nullptr: not available
+  const float* norm = nullptr;     // [N]
+};
+bool coded_supported(int N, int K, float weight_scale);
+int coded_weight_tile_rows();
+size_t coded_slice_bytes(size_t rows, int K, int tile_rows);
+cudaError_t launch_code_weights(const void* weight, int N, int K, int8_t* slices, float* norm,
+                                cudaStream_t stream);
+// `in` [rows][K] gives rows first_row .. of the outputs (sf_tiled: k_tiles per 128-row slot).
+cudaError_t launch_coded_linear(const CodedWeight& w, const float* in, int rows, float fp8_scale,
+                                const ExactWorkspace& space, int first_row, uint8_t* packed,
+                                uint8_t* sf_tiled, int k_tiles, float* tensor_scale, int32_t* error,
+                                int num_sms, cudaStream_t stream);
+
 // --- dense and scaled-FP8 linear families, latent-MoE data flow (csrc/dense.cu) -
 // The dense matmul itself is launch_router_logits: out[rows][experts] =
 // a[rows][hidden] x w[experts][hidden]^T, FP64 accumulation, FP32 result.

@@ -668,6 +668,25 @@ struct DenseLinear {
   float input_scale = 1.0f;
   DeviceBuffer weight;
   ExactOperand operand;
+  CodedWeight coded;  // FP8 weights whose rows are only quantised again
+  DeviceBuffer coded_slices, coded_norm;
+
+  void prepare_coded(cudaStream_t stream) {
+    if (!fp8 || !exact || !coded_supported(out, in, operand.w.scale) ||
+        clamp_scale_host(input_scale) > 0x1p60f) {
+      return;
+    }
+    coded_slices.allocate(coded_slice_bytes(out, in, coded_weight_tile_rows()), true);
+    coded_norm.allocate(static_cast<size_t>(out) * sizeof(float));
+    NMOE_CUDA(launch_code_weights(weight.as<void>(), out, in, coded_slices.as<int8_t>(),
+                                  coded_norm.as<float>(), stream));
+    coded.N = out;
+    coded.K = in;
+    coded.weight = weight.as<void>();
+    coded.scale = operand.w.scale;
+    coded.norm = coded_norm.as<float>();
+    coded.slices = coded_slices.as<int8_t>();
+  }
 
   void upload(const nmoe_linear& linear, size_t out_rows, size_t in_cols, const char* name,
               cudaStream_t stream) {
@@ -737,8 +756,8 @@ struct ExactScratch {
     // (rows come in tiles of up to 64)
     slices.allocate(slice_bytes(max_rows, static_cast<int>(most_k), 64));
     info.allocate(max_rows * sizeof(SliceRow));
-    // a split contraction has at most one tile of 128 x 64 sums per SM
-    partial.allocate(std::max(max_rows * most_n, static_cast<size_t>(num_sms) * 128 * 64) *
+    // a split contraction has at most one tile of 128 x 80 sums per SM
+    partial.allocate(std::max(max_rows * most_n, static_cast<size_t>(num_sms) * 128 * 80) *
                      sizeof(double));
   }
 };
@@ -1317,6 +1336,9 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   } else {
     L->shared_up.upload(&w.shared_up, 1, S, H, "shared up_proj", stream);
   }
+  if (w.shared_down_linear.family == NMOE_LINEAR_ABSENT && L->shared_up_dense.present) {
+    L->shared_up_dense.prepare_coded(stream);
+  }
   if (w.shared_down_linear.family != NMOE_LINEAR_ABSENT) {
     L->shared_down_dense.upload(w.shared_down_linear, H, S, "shared down_proj", stream);
   } else {
@@ -1606,8 +1628,25 @@ void shared_hidden_rows(nmoe_layer* L, LaunchStream stream, int tokens) {
 
 // ... and quantised for an NVFP4 down projection, through the host linear's own packing step
 // (:981-1005).
-void quantise_shared_hidden(nmoe_layer* L, LaunchStream stream, int tokens) {
+void quantised_shared_hidden(nmoe_layer* L, LaunchStream stream, int tokens) {
   const int S = L->cfg.shared_expert_intermediate_size;
+  const DenseLinear& up = L->shared_up_dense;
+  if (up.coded.slices != nullptr && !L->unfused &&
+      !exact_prefers_gemv(tokens, up.out, up.in, L->num_sms)) {
+    const float fp8_scale = clamp_scale_host(up.input_scale);
+    const int most = L->up_exact.max_rows;
+    for (int first = 0; first < tokens; first += most) {
+      const ExactWorkspace space{L->up_exact.slices.as<int8_t>(), L->up_exact.info.as<SliceRow>(),
+                                 L->up_exact.partial.as<double>()};
+      NMOE_CUDA(launch_coded_linear(
+          up.coded, L->normalized.as<float>() + static_cast<size_t>(first) * up.in,
+          std::min(tokens - first, most), fp8_scale, space, first, L->sh_packed.as<uint8_t>(),
+          L->sh_sf.as<uint8_t>(), k_blocks_of(S) * 4, L->sh_ts.as<float>(),
+          L->error.device.as<int32_t>(), L->num_sms, stream));
+    }
+    return;
+  }
+  shared_hidden_rows(L, stream, tokens);
   NMOE_CUDA(launch_norm_quant(L->shared_raw.as<float>(), false, tokens, S, nullptr, 0.0f, nullptr,
                               L->sh_packed.as<uint8_t>(), nullptr, L->sh_sf.as<uint8_t>(),
                               k_blocks_of(S), L->sh_ts.as<float>(), L->num_sms, stream));
@@ -1632,9 +1671,9 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
             L->y_ts.as<float>(), shared, buffers, out, stream, between);
     return;
   }
-  shared_hidden_rows(L, stream, tokens);
-  if (between != nullptr) cudaEventRecord(between, stream);
   if (L->shared_down_dense.present) {
+    shared_hidden_rows(L, stream, tokens);
+    if (between != nullptr) cudaEventRecord(between, stream);
     // dense / scaled-FP8 down projection (:1006-1045) straight from the FP32 rows;
     // only the latent data flow (FP32 rows of `hidden` per token) reaches this
     NMOE_REQUIRE(dest_mul == 1 && dest_add == 0 && out_kind == kRowF32,
@@ -1643,7 +1682,8 @@ void shared_expert(nmoe_layer* L, cudaStream_t stream, int tokens, void* out_row
                static_cast<float*>(out_rows), false, stream);
     return;
   }
-  quantise_shared_hidden(L, stream, tokens);
+  quantised_shared_hidden(L, stream, tokens);
+  if (between != nullptr) cudaEventRecord(between, stream);
   run_down_gemm(L->shared_down, shared_class, L->sh_op, L->sh_ts.as<float>(), shared, out,
                 L->error.device.as<int32_t>(), L->num_sms, stream);
 }
@@ -1806,8 +1846,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
                                 L->lat_sf_row_major.as<uint8_t>(), nullptr, 0,
                                 L->lat_ts.as<float>(), L->num_sms, latent));
     if (one_launch && L->shared_up_dense.present) {
-      shared_hidden_rows(L, up, tokens);
-      quantise_shared_hidden(L, up, tokens);
+      quantised_shared_hidden(L, up, tokens);
     }
     if (beside) {
       NMOE_CUDA(cudaEventRecord(L->latent_done, L->latent_stream));
@@ -1856,8 +1895,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   }
   if (one_launch) {
     if (L->shared_up_dense.present) {
-      shared_hidden_rows(L, chain, tokens);
-      quantise_shared_hidden(L, chain, tokens);
+      quantised_shared_hidden(L, chain, tokens);
     }
     const StreamFfn shared =
         shared_stream_ffn(L, tokens, L->parts.as<void>(), K + 1, K, parts_kind);

@@ -84,6 +84,43 @@ def test_chains_beside_each_other_give_the_same_bits(package, synthetic, monkeyp
     alone.close()
 
 
+# FP8 shared_up: the hidden rows' codes are decided from whole-number sums of the operands' codes, in the
+# unfused path they follow from the correctly rounded rows.  Tiles of 16 to 80 token rows, an unfinished
+# tile of weight rows, more rows than the workspace holds at once; values beyond 6 * 448, whose rows get a
+# tensor scale of their own; a row that holds a NaN.
+@pytest.mark.parametrize("weight_scale", [1.0, 90.0])
+def test_fp8_shared_up_codes_are_those_of_the_rounded_rows(package, synthetic, weight_scale):
+    cfg = synthetic.baseline_config(max_tokens=1100, experts=64, hidden=448, routed=64, shared=704,
+                                    latent=192)
+    data = synthetic.make_layer(cfg, seed=17, device="cuda", norm_weight_uniform=True,
+                                latent_family="fp8", shared_up_family="fp8")
+    data.bindings.shared_up_linear.weight_scale *= weight_scale
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+
+    def shared_codes(tokens):
+        shared = cfg.shared_expert_intermediate_size
+        codes = torch.empty((tokens, shared // 2), dtype=torch.uint8, device="cuda")
+        scales = torch.empty((tokens, shared // 16), dtype=torch.uint8, device="cuda")
+        assert package.load_library().nmoe_layer_export_hidden(
+            layer._handle, torch.cuda.current_stream().cuda_stream, None, None, codes.data_ptr(),
+            scales.data_ptr()) == 0
+        return codes, scales
+
+    for tokens in (5, 16, 17, 64, 65, 80, 81, 161, 1100):
+        x = synthetic.make_tokens(tokens, cfg.hidden_size, seed=tokens, device="cuda")
+        if tokens == 81:
+            x[40, 7] = float("nan")
+        fused, decided = _run(layer, x), shared_codes(tokens)
+        layer.set_unfused_activation(True)
+        unfused, rounded = _run(layer, x), shared_codes(tokens)
+        layer.set_unfused_activation(False)
+        for got, expected in zip(decided, rounded):
+            assert torch.equal(got, expected)
+        assert torch.equal(fused.nan_to_num(7.0), unfused.nan_to_num(7.0))
+    layer.close()
+
+
 def test_unfused_activation_path_and_trace_fields(package, synthetic, oracle):
     cfg = synthetic.baseline_config(max_tokens=256, experts=32, hidden=512, routed=256, shared=512)
     data = synthetic.make_layer(cfg, seed=21, device="cuda", norm_weight_uniform=True)
