@@ -18,11 +18,10 @@
 // form it came in (FP8, bf16 or FP32) and sums in FP64.
 #include <algorithm>
 
-#include <cuda_fp16.h>
-
 #include "common.cuh"
 #include "kernels.h"
 #include "quant_row.cuh"
+#include "weights.cuh"
 
 namespace nmoe {
 namespace {
@@ -44,13 +43,6 @@ __device__ __forceinline__ float weight_value(const void* w, size_t i, float sca
   } else {
     return reinterpret_cast<const float*>(w)[i];
   }
-}
-
-// The activation the linear multiplies with: the row itself, or for the scaled-FP8 family its
-// round trip through E4M3 (scaled_fp8_linear.cu:94-106).
-__device__ __forceinline__ float input_value(float v, float fp8_scale) {
-  if (fp8_scale == 0.0f) return v;
-  return __fmul_rn(decode_e4m3(encode_e4m3(__fdiv_rn(v, fp8_scale))), fp8_scale);
 }
 
 // Exponent e with |v| < 2^e for every v of magnitude up to `amax`.
@@ -436,46 +428,6 @@ __device__ __forceinline__ double two_to(int e) {
   return e < -1022 ? 0.0 : __hiloint2double((min(e, 1023) + 1023) << 20, 0);
 }
 
-template <int KIND>
-struct WeightVector;  // 16 bytes of W as FP32 values
-template <>
-struct WeightVector<kWeightFp8> {
-  static constexpr int kCount = 16;
-  static __device__ __forceinline__ void unpack(const uint4& raw, float scale, float (&v)[16]) {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const __half2_raw two = __nv_cvt_fp8x2_to_halfraw2(
-          static_cast<__nv_fp8x2_storage_t>(w[i >> 1] >> (16 * (i & 1))), __NV_E4M3);
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
-      v[2 * i] = __fmul_rn(f.x, scale);
-      v[2 * i + 1] = __fmul_rn(f.y, scale);
-    }
-  }
-};
-template <>
-struct WeightVector<kWeightBf16> {
-  static constexpr int kCount = 8;
-  static __device__ __forceinline__ void unpack(const uint4& raw, float, float (&v)[8]) {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[2 * i] = __uint_as_float(w[i] << 16);
-      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
-  }
-};
-template <>
-struct WeightVector<kWeightF32> {
-  static constexpr int kCount = 4;
-  static __device__ __forceinline__ void unpack(const uint4& raw, float, float (&v)[4]) {
-    v[0] = __uint_as_float(raw.x);
-    v[1] = __uint_as_float(raw.y);
-    v[2] = __uint_as_float(raw.z);
-    v[3] = __uint_as_float(raw.w);
-  }
-};
-
 constexpr int kFinishThreads = 256;
 
 // FP32 results from the doubles of exact_gemm_kernel: one thread per value.
@@ -678,10 +630,6 @@ __device__ __forceinline__ float exact_value(const uint8_t* x, float fp8_scale, 
 
 __device__ __forceinline__ float relu_squared(float r) { return r > 0.0f ? __fmul_rn(r, r) : 0.0f; }
 
-__device__ __forceinline__ float (&eight_of(float (&v)[16], int i))[8] {
-  return *reinterpret_cast<float(*)[8]>(&v[i]);
-}
-
 // Largest `v` of the block's threads (none is negative).
 __device__ __forceinline__ float block_max_of(float v, float* warp_values) {
   const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
@@ -854,6 +802,48 @@ constexpr int kGemvThreads = 256;
 // consecutive values meet no bank conflict.
 __host__ __device__ constexpr int gemv_slot(int k) { return k + (k >> 4); }
 
+// Weight rows n0 and n0 + 1 times ROWS token rows (`padded` doubles apart, in slots), by a warp: the sums
+// in all its lanes.  A token value read from shared memory serves both weight rows.
+template <int KIND, int ROWS>
+__device__ __forceinline__ void dot_two_rows(const double* xs, int padded, const void* weight,
+                                             float weight_scale, int n0, int N, int K,
+                                             double (&acc)[ROWS][2]) {
+  constexpr int V = WeightVector<KIND>::kCount;
+  const size_t row_bytes = static_cast<size_t>(K) * (16 / V);
+  const uint8_t* rows = reinterpret_cast<const uint8_t*>(weight);
+  const uint4* w0 = reinterpret_cast<const uint4*>(rows + n0 * row_bytes);
+  const uint4* w1 = reinterpret_cast<const uint4*>(rows + min(n0 + 1, N - 1) * row_bytes);
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0.0;
+#pragma unroll 4
+  for (int q = threadIdx.x & 31; q * V < K; q += 32) {
+    float v0[V], v1[V];
+    WeightVector<KIND>::unpack(w0[q], weight_scale, v0);
+    WeightVector<KIND>::unpack(w1[q], weight_scale, v1);
+    const double* x = xs + gemv_slot(q * V);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const double d0 = static_cast<double>(v0[j]), d1 = static_cast<double>(v1[j]);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const double a = x[r * padded + j];
+        acc[r][0] = fma(a, d0, acc[r][0]);
+        acc[r][1] = fma(a, d1, acc[r][1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int stride = 16; stride > 0; stride >>= 1) {
+        acc[r][h] += __shfl_xor_sync(0xffffffffu, acc[r][h], stride);
+      }
+    }
+  }
+}
+
 // One warp per weight row at a time; the ROWS token rows wait in shared memory as doubles, so that
 // they are widened once per block.  Bound by reading W at one row: shared_up of the checkpoint
 // layer (22 MB of FP8) 37 -> 15 us.
@@ -896,47 +886,18 @@ exact_gemv_kernel(const float* in, float fp8_scale, int N, int K,
     }
   }
   __syncthreads();
-  // two weight rows at a time: a token value read from shared memory serves both
   const int pairs = (N + 1) / 2;
   for (int p = blockIdx.x * kWarps + (threadIdx.x >> 5); p < pairs; p += gridDim.x * kWarps) {
-    const int n0 = 2 * p, n1 = min(n0 + 1, N - 1);
-    const size_t row_bytes = static_cast<size_t>(K) * (16 / V);
-    const uint4* w0 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
-                                                     n0 * row_bytes);
-    const uint4* w1 = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
-                                                     n1 * row_bytes);
+    const int n0 = 2 * p;
     double acc[ROWS][2];
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = 0.0;
-#pragma unroll 4
-    for (int q = lane; q * V < K; q += 32) {
-      float v0[V], v1[V];
-      WeightVector<KIND>::unpack(w0[q], weight_scale, v0);
-      WeightVector<KIND>::unpack(w1[q], weight_scale, v1);
-      const double* x = xs + gemv_slot(q * V);
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const double d0 = static_cast<double>(v0[j]), d1 = static_cast<double>(v1[j]);
-#pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-          const double a = x[r * padded + j];
-          acc[r][0] = fma(a, d0, acc[r][0]);
-          acc[r][1] = fma(a, d1, acc[r][1]);
-        }
-      }
-    }
+    dot_two_rows<KIND, ROWS>(xs, padded, weight, weight_scale, n0, N, K, acc);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        double v = acc[r][h];
-#pragma unroll
-        for (int stride = 16; stride > 0; stride >>= 1) {
-          v += __shfl_xor_sync(0xffffffffu, v, stride);
-        }
         const int n = n0 + h;
         if (lane == 0 && n < N) {
-          float result = static_cast<float>(v);
+          float result = static_cast<float>(acc[r][h]);
           if (offset != nullptr) result = __fadd_rn(result, offset[n]);
           if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
           out[static_cast<size_t>(r) * N + n] = result;
@@ -1009,6 +970,80 @@ exact_gemv_block_kernel(const float* in, float fp8_scale, int rows, int N, int K
     if (offset != nullptr) result = __fadd_rn(result, offset[n]);
     if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
     out[static_cast<size_t>(row0 + r) * N + n] = result;
+  }
+}
+
+// The end of a latent layer over one token in one launch: the routed sum in selection order
+// (expert_layer.cpp:951-953), fc2_latent (:1047-1053), mixer and residual (:1064-1069).  Every block adds
+// up the parts for itself, 32 outputs at a time, which keeps 4096 of them to one block an SM.
+constexpr int kTailOutputs = 32;
+template <int KIND>
+__global__ void __launch_bounds__(kGemvThreads)
+latent_tail_kernel(const LatentTail tail, int N, int K, const void* __restrict__ weight,
+                   float weight_scale) {
+  constexpr int V = WeightVector<KIND>::kCount;
+  constexpr int kBatch = 8;  // loads of a part in flight
+  extern __shared__ double xs[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int block_n = blockIdx.x * kTailOutputs;
+  const size_t row_bytes = static_cast<size_t>(K) * (16 / V);
+  release_successor();
+  {
+    // the weights need not wait for the experts
+    const size_t bytes = min(kTailOutputs, N - block_n) * row_bytes;
+    const uint8_t* first = reinterpret_cast<const uint8_t*>(weight) + block_n * row_bytes;
+    for (size_t b = threadIdx.x * 128; b < bytes; b += kGemvThreads * 128) prefetch_l2(first + b);
+  }
+  wait_for_predecessor();
+  for (int c = static_cast<int>(threadIdx.x) * 4; c < K; c += kGemvThreads * 4) {
+    const float* base = tail.parts + c;
+    float4 acc = *reinterpret_cast<const float4*>(base);
+    for (int k0 = 1; k0 < tail.top_k; k0 += kBatch) {
+      float4 p[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (k0 + k < tail.top_k) {
+          p[k] = *reinterpret_cast<const float4*>(base + static_cast<size_t>(k0 + k) * K);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        if (k0 + k < tail.top_k) {
+          acc.x = __fadd_rn(acc.x, p[k].x);
+          acc.y = __fadd_rn(acc.y, p[k].y);
+          acc.z = __fadd_rn(acc.z, p[k].z);
+          acc.w = __fadd_rn(acc.w, p[k].w);
+        }
+      }
+    }
+    double* to = xs + gemv_slot(c);  // (four from a multiple of four: no gap between)
+    to[0] = acc.x;
+    to[1] = acc.y;
+    to[2] = acc.z;
+    to[3] = acc.w;
+    if (blockIdx.x == 0) *reinterpret_cast<float4*>(tail.routed + c) = acc;
+  }
+  __syncthreads();
+  constexpr int kPerWarp = kTailOutputs / (kGemvThreads / 32);
+#pragma unroll 1
+  for (int p = 0; p < kPerWarp; p += 2) {
+    const int n0 = block_n + warp * kPerWarp + p;
+    if (n0 >= N) break;
+    double acc[1][2];
+    dot_two_rows<KIND, 1>(xs, 0, weight, weight_scale, n0, N, K, acc);
+    const int n = n0 + lane;
+    if (lane >= 2 || n >= N) continue;
+    const float projected = static_cast<float>(lane == 0 ? acc[0][0] : acc[0][1]);
+    tail.projected[n] = projected;
+    const float x = tail.in_bf16
+                        ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(tail.in)[n])
+                        : reinterpret_cast<const float*>(tail.in)[n];
+    const float mixed = __fadd_rn(x, __fadd_rn(projected, tail.shared[n]));
+    if (tail.out_bf16) {
+      reinterpret_cast<__nv_bfloat16*>(tail.out)[n] = __float2bfloat16_rn(mixed);
+    } else {
+      reinterpret_cast<float*>(tail.out)[n] = mixed;
+    }
   }
 }
 
@@ -1343,6 +1378,18 @@ bool exact_prefers_gemv(int rows, int N, int K, int num_sms) {
   if (rows <= 4) return true;
   return gemv_by_blocks(rows, N, num_sms) &&
          static_cast<long long>(rows) * N * K <= kMostFp64Products;
+}
+
+cudaError_t launch_latent_tail(const ExactWeight& w, const LatentTail& tail, LaunchStream stream) {
+  if (!exact_supported(w.N, w.K) || w.kind == kWeightFp8) return cudaErrorInvalidValue;
+  auto run = [&](auto kernel) {
+    const cudaError_t err = allow_shared_memory(kernel);
+    if (err != cudaSuccess) return err;
+    return launch_kernel(kernel, (w.N + kTailOutputs - 1) / kTailOutputs, kGemvThreads,
+                         gemv_slot(w.K) * sizeof(double), stream, tail, w.N, w.K, w.weight, w.scale);
+  };
+  return w.kind == kWeightBf16 ? run(latent_tail_kernel<kWeightBf16>)
+                               : run(latent_tail_kernel<kWeightF32>);
 }
 
 cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,

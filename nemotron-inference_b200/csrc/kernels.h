@@ -355,6 +355,21 @@ cudaError_t launch_coded_linear(const CodedWeight& w, const float* in, int rows,
                                 uint8_t* sf_tiled, int k_tiles, float* tensor_scale, int32_t* error,
                                 int num_sms, cudaStream_t stream);
 
+// The end of a latent layer over one token: `routed` [K] = the sum of parts [top_k][K], `projected` [N] =
+// routed x W^T (dense), out = in + (projected + shared).
+struct LatentTail {
+  const float* parts;
+  int top_k;
+  const float* shared;
+  const void* in;
+  bool in_bf16;
+  float* routed;
+  float* projected;
+  void* out;
+  bool out_bf16;
+};
+cudaError_t launch_latent_tail(const ExactWeight& w, const LatentTail& tail, LaunchStream stream);
+
 // --- dense and scaled-FP8 linear families, latent-MoE data flow (csrc/dense.cu) -
 // The dense matmul itself is launch_router_logits: out[rows][experts] =
 // a[rows][hidden] x w[experts][hidden]^T, FP64 accumulation, FP32 result.
@@ -418,7 +433,23 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
 // --- front end of a handful of tokens (csrc/front.cu) ---------------------------
 constexpr int kFrontMaxRows = 8;
 constexpr int kFrontMaxCols = 4096;
-constexpr int kFrontMaxExperts = 256;
+constexpr int kFrontMaxExperts = 512;
+// A linear of the one token's normalised row whose FP32 row is then quantised with its tensor scale.
+constexpr int kFrontLinears = 2;
+constexpr int kFrontLinearMaxN = 6144;
+struct FrontLinear {
+  int N = 0, kind = 0;
+  const void* weight = nullptr;
+  float scale = 1.0f, fp8_scale = 0.0f;
+  bool relu2 = false;
+  float* rounded = nullptr;  // [cols]
+  float* out = nullptr;      // [N]
+  uint8_t* packed = nullptr;
+  uint8_t* sf_row_major = nullptr;
+  uint8_t* sf_tiled = nullptr;
+  int k_tiles = 0;
+  float* tensor_scale = nullptr;
+};
 struct FrontArgs {
   const void* in = nullptr;  // [rows][cols]
   bool in_bf16 = false;
@@ -453,11 +484,14 @@ struct FrontArgs {
   float* row_weight = nullptr;
   int32_t* pair_row = nullptr;
   int dest_stride = 0;
+  FrontLinear linear[kFrontLinears];
+  int linears = 0;
   void* scratch = nullptr;  // front_scratch_bytes(), zero before the first launch
   int32_t* error = nullptr;
 };
 constexpr size_t front_scratch_bytes() {
-  return (kFrontMaxRows + 1) * sizeof(int32_t) + 2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
+  return (kFrontMaxRows + 2 + 2 * kFrontLinears) * sizeof(int32_t) +
+         2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
 }
 cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream);
 

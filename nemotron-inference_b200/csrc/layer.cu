@@ -972,7 +972,8 @@ struct nmoe_layer {
   int latent = 0;
   bool latent_mode = false;
   DenseLinear fc1, fc2, shared_up_dense, shared_down_dense;
-  DeviceBuffer latent_rows, lat_packed, lat_sf_row_major, lat_ts;  // fc1 output and its NVFP4 form
+  // fc1 output and its NVFP4 form
+  DeviceBuffer latent_rows, lat_packed, lat_sf_row_major, lat_sf_tiled, lat_ts;
   DeviceBuffer routed_latent, projected, shared_rows;               // [T][latent], [T][H], [T][H]
   DeviceBuffer fp8_tmp;                                             // activation round trip
   DeviceBuffer shared_raw;  // [T][S] FP32: shared_up output, activated in place
@@ -1026,9 +1027,9 @@ struct nmoe_layer {
     }
   } window;
 
-  ActivationOperand y_op, sh_op, a_op, h_op;
+  ActivationOperand y_op, lat_op, sh_op, a_op, h_op;
   StreamCounts stream_counts;
-  DeviceBuffer front_scratch;  // of csrc/front.cu
+  DeviceBuffer front_scratch, front_rounded;  // of csrc/front.cu
   ErrorSlot error;
   int last_tokens = 0;
   std::string last_error;
@@ -1149,9 +1150,10 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   L->sh_ts.allocate(token_slots * 128 * sizeof(float), true);
   if (L->latent_mode) {
     L->latent_rows.allocate(T * Lr * sizeof(float));
-    L->lat_packed.allocate(T * Lr / 2);
+    L->lat_packed.allocate(token_slots * 128 * Lr / 2, true);
+    L->lat_sf_tiled.allocate(tiled_sf_bytes(token_slots, Lr), true);
     L->lat_sf_row_major.allocate(T * (Lr / 16));
-    L->lat_ts.allocate(T * sizeof(float));
+    L->lat_ts.allocate(token_slots * 128 * sizeof(float), true);
     L->routed_latent.allocate(T * Lr * sizeof(float));
     L->projected.allocate(T * H * sizeof(float));
     L->shared_rows.allocate(T * H * sizeof(float));
@@ -1180,6 +1182,9 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   L->max_row_tiles = static_cast<int>(2 * static_cast<size_t>(EL) + (pairs + 127) / 128);
   L->stream_counts.allocate(L->max_row_tiles + token_slots);
   L->front_scratch.allocate(front_scratch_bytes(), true);
+  if (L->latent_mode) {
+    L->front_rounded.allocate(static_cast<size_t>(kFrontLinears) * H * sizeof(float));
+  }
   const size_t slots = static_cast<size_t>(L->max_row_tiles);
   L->counts.allocate(E * sizeof(int32_t), true);
   L->cursor.allocate(E * sizeof(int32_t), true);
@@ -1216,6 +1221,9 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
   }
 
   L->y_op.bind(L->y_packed.as<uint8_t>(), L->y_sf_tiled.as<uint8_t>(), token_slots * 128, H);
+  if (L->latent_mode) {
+    L->lat_op.bind(L->lat_packed.as<uint8_t>(), L->lat_sf_tiled.as<uint8_t>(), token_slots * 128, Lr);
+  }
   L->sh_op.bind(L->sh_packed.as<uint8_t>(), L->sh_sf.as<uint8_t>(), token_slots * 128, S);
   L->a_op.bind(L->a_packed.as<uint8_t>(), L->a_sf.as<uint8_t>(), slots * 128, Lr);
   L->h_op.bind(L->h_packed.as<uint8_t>(), L->h_sf.as<uint8_t>(), slots * 128, I);
@@ -1576,8 +1584,9 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
     StreamFfn ffn;
     ffn.up = &L->up;
     ffn.down = &L->down;
-    ffn.a = token_order ? &L->y_op : &L->a_op;
-    ffn.a_tensor_scale = (token_order ? L->y_ts : L->a_ts).as<float>();
+    ffn.a = !token_order ? &L->a_op : L->latent_mode ? &L->lat_op : &L->y_op;
+    ffn.a_tensor_scale =
+        (!token_order ? L->a_ts : L->latent_mode ? L->lat_ts : L->y_ts).as<float>();
     if (token_order) ffn.used = L->a_dest.as<int32_t>();
     ffn.schedule = routed;
     ffn.hidden_packed = L->h_packed.as<uint8_t>();
@@ -1732,6 +1741,28 @@ PermuteSource local_source(nmoe_layer* L) {
   return source;
 }
 
+// What follows the experts of a latent layer: routed sum in selection order (:951-953), fc2_latent
+// (:1047-1053), mixer and residual (:1064-1069).
+void latent_tail(nmoe_layer* L, LaunchStream stream, const void* input, nmoe_dtype in_dtype, int tokens,
+                 void* output, nmoe_dtype out_dtype) {
+  const int H = L->cfg.hidden_size, K = L->cfg.top_k, Lr = L->latent;
+  if (tokens == 1 && L->fc2.exact && !L->stage_timing) {
+    const LatentTail tail{L->parts.as<float>(),       K,
+                          L->shared_rows.as<float>(), input,
+                          in_dtype == NMOE_BF16,      L->routed_latent.as<float>(),
+                          L->projected.as<float>(),   output,
+                          out_dtype == NMOE_BF16};
+    NMOE_CUDA(launch_latent_tail(L->fc2.operand.w, tail, stream));
+    return;
+  }
+  NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
+                             stream));
+  run_linear(L, L->fc2, L->exact, L->routed_latent.as<float>(), tokens, L->projected.as<float>(), false,
+             stream);
+  NMOE_CUDA(launch_mixer(input, in_dtype == NMOE_BF16, L->projected.as<float>(),
+                         L->shared_rows.as<float>(), tokens, H, output, out_dtype == NMOE_BF16, stream));
+}
+
 // Everything in front of the experts in one launch (csrc/front.cu).
 void route_few(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype in_dtype,
                int tokens) {
@@ -1768,17 +1799,54 @@ void route_few(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype
   args.dest = L->a_dest.as<int32_t>();
   args.row_weight = L->a_weight.as<float>();
   args.pair_row = L->pair_row.as<int32_t>();
-  args.dest_stride = c.top_k + 1;
+  args.dest_stride = L->latent_mode ? c.top_k : c.top_k + 1;
+  if (L->latent_mode) {
+    auto add = [&](const DenseLinear& linear) -> FrontLinear& {
+      FrontLinear& to = args.linear[args.linears++];
+      to.N = linear.out;
+      to.kind = linear.operand.w.kind;
+      to.weight = linear.operand.w.weight;
+      to.scale = linear.operand.w.scale;
+      to.fp8_scale = linear.fp8 ? clamp_scale_host(linear.input_scale) : 0.0f;
+      to.rounded = L->front_rounded.as<float>() +
+                   static_cast<size_t>(args.linears - 1) * c.hidden_size;
+      return to;
+    };
+    FrontLinear& fc1 = add(L->fc1);
+    fc1.out = L->latent_rows.as<float>();
+    fc1.packed = L->lat_packed.as<uint8_t>();
+    fc1.sf_row_major = L->lat_sf_row_major.as<uint8_t>();
+    fc1.sf_tiled = L->lat_sf_tiled.as<uint8_t>();
+    fc1.k_tiles = k_blocks_of(L->latent) * 4;
+    fc1.tensor_scale = L->lat_ts.as<float>();
+    if (L->shared_up_dense.present) {
+      FrontLinear& up = add(L->shared_up_dense);
+      up.relu2 = true;
+      up.out = L->shared_raw.as<float>();
+      up.packed = L->sh_packed.as<uint8_t>();
+      up.sf_tiled = L->sh_sf.as<uint8_t>();
+      up.k_tiles = k_blocks_of(c.shared_expert_intermediate_size) * 4;
+      up.tensor_scale = L->sh_ts.as<float>();
+    }
+  }
   args.scratch = L->front_scratch.as<void>();
   args.error = L->error.device.as<int32_t>();
   NMOE_CUDA(launch_front(args, stream));
   L->last_normalized = true;
 }
 
-// Whether csrc/front.cu takes a batch.
+// Whether csrc/front.cu takes a batch (with what it cannot quantise left out).
 bool front_takes(const nmoe_layer* L, int tokens) {
-  return tokens <= kFrontMaxRows && L->cfg.hidden_size <= kFrontMaxCols &&
-         L->cfg.n_routed_experts <= kFrontMaxExperts && L->has_gate_exact;
+  if (tokens > kFrontMaxRows || L->cfg.hidden_size > kFrontMaxCols ||
+      L->cfg.n_routed_experts > kFrontMaxExperts || !L->has_gate_exact) {
+    return false;
+  }
+  if (!L->latent_mode) return !L->shared_up_dense.present && !L->shared_down_dense.present;
+  auto fits = [](const DenseLinear& linear) {
+    return linear.exact && linear.out <= kFrontLinearMaxN;
+  };
+  return tokens == 1 && fits(L->fc1) &&
+         (!L->shared_up_dense.present || fits(L->shared_up_dense));
 }
 
 // A latent layer's three chains behind the norm -- gate and selection; fc1_latent and its quantiser;
@@ -1813,11 +1881,10 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   // with the two-pass router there was nothing to gain (256 tokens 162 us either way) and at 700
   // tokens 2 to 4 us to lose.
   const LaunchStream chain(stream, !fork && !L->stage_timing && !L->unfused && !two_pass);
-  const bool beside = L->latent_stream != nullptr && one_launch && L->latent_mode &&
+  const bool few = front_takes(L, tokens) && one_launch && !two_pass && !L->stage_timing;
+  const bool beside = !few && L->latent_stream != nullptr && one_launch && L->latent_mode &&
                       !L->stage_timing && tokens >= kBesideMinTokens &&
                       tokens <= L->fork_max_tokens;
-  const bool few = front_takes(L, tokens) && one_launch && !L->latent_mode && !dense_shared &&
-                   !two_pass && !L->stage_timing;
   if (few) {
     route_few(L, stream, input, in_dtype, tokens);
   } else {
@@ -1827,6 +1894,14 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   L->last_tokens = tokens;
   L->last_parts_kind = parts_kind;
   L->last_unfused = L->unfused;
+  if (L->latent_mode && few) {
+    const StreamFfn shared =
+        shared_stream_ffn(L, tokens, L->shared_rows.as<void>(), 1, 0, kRowF32);
+    routed_experts(L, chain, local_source(L), tokens * K, K, L->parts.as<void>(), kRowF32,
+                   RowSegments(), &shared, true);
+    latent_tail(L, chain, input, in_dtype, tokens, output, out_dtype);
+    return;
+  }
   if (L->latent_mode) {
     // latent = fc1_latent(normalized) (:809-813); every routed expert's up_proj packs
     // the same latent row (:913 -> nvfp4_packing.cpp:90)
@@ -1876,15 +1951,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
                     L->stage_timing ? L->stage_events[8] : nullptr, kRowF32);
       L->mark(9, stream);
     }
-    // routed sum in selection order (:951-953), fc2_latent (:1047-1053), mixer and
-    // residual (:1064-1069)
-    NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
-                               chain));
-    run_linear(L, L->fc2, L->exact, L->routed_latent.as<float>(), tokens, L->projected.as<float>(),
-               false, chain);
-    NMOE_CUDA(launch_mixer(input, in_dtype == NMOE_BF16, L->projected.as<float>(),
-                           L->shared_rows.as<float>(), tokens, H, output, out_dtype == NMOE_BF16,
-                           chain));
+    latent_tail(L, chain, input, in_dtype, tokens, output, out_dtype);
     L->mark(10, stream);
     return;
   }

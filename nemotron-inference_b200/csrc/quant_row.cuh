@@ -8,6 +8,10 @@ namespace nmoe {
 
 constexpr int kWarpsPerBlock = 8;
 
+__device__ __forceinline__ float (&eight_of(float (&v)[16], int i))[8] {
+  return *reinterpret_cast<float(*)[8]>(&v[i]);
+}
+
 template <bool BF16>
 __device__ __forceinline__ void load8(const void* base, size_t index, float (&v)[8]) {
   if constexpr (BF16) {

@@ -100,10 +100,9 @@ constexpr int kMaxExperts = 512;
 
 // One block per token.  All threads evaluate sigmoids (the exponential in double is the
 // longest single step; one for each expert while blocks are few, else 128), one warp selects:
-// expert e lives in lane e % 32, slot e / 32, every lane keeps the best of its remaining slots,
-// and a round is one warp-wide maximum of order-preserving keys, one minimum over the indices that
-// hold it (ties go to the lower expert) and a rescan by the lane that owned it.  Bound by the
-// latency of that chain (between events): 1 token, 128 experts, top-6 14.9 -> 8.2 us; 512 experts, top-22 33 -> 12.2.
+// expert e lives in lane e % 32, every lane keeps the best of its own at hand, and a round is one
+// warp-wide maximum of order-preserving keys and one minimum over the indices that hold it (ties go
+// to the lower expert).  Bound by the latency of that chain (between events): 1 token, 128 experts, top-6 14.9 -> 8.2 us; 512 experts, top-22 33 -> 12.2.
 template <int PER_LANE>
 __global__ void __launch_bounds__(PER_LANE * 32 < 128 ? 128 : PER_LANE * 32)
 router_topk_kernel(const float* logits, const float* __restrict__ bias, int experts,
@@ -113,6 +112,7 @@ router_topk_kernel(const float* logits, const float* __restrict__ bias, int expe
                    int32_t* __restrict__ position) {
   __shared__ float score_smem[PER_LANE * 32];
   __shared__ float choice_smem[PER_LANE * 32];
+  __shared__ uint32_t list[kSelectList];
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x;
   release_successor();
@@ -127,8 +127,9 @@ router_topk_kernel(const float* logits, const float* __restrict__ bias, int expe
 
   int my_index;
   float my_score;
-  const float weight_sum = select_experts<PER_LANE>(score_smem, choice_smem, experts, top_k, n_group,
-                                                    topk_group, my_index, my_score);
+  const float weight_sum =
+      select_experts<(PER_LANE > 4)>(score_smem, choice_smem, list, experts, top_k, n_group, topk_group,
+                                     my_index, my_score);
   if (lane < top_k) {
     top_index[static_cast<size_t>(row) * top_k + lane] = my_index;
     top_weight[static_cast<size_t>(row) * top_k + lane] =

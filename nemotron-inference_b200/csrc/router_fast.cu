@@ -512,26 +512,6 @@ __device__ __forceinline__ double gate_scaled(uint32_t w) {
   return __hiloint2double((static_cast<int>(w) >> 3) & static_cast<int>(0x8fffe000u), 0);
 }
 
-// Sums eight values over the warp: after the call lane L holds the total of value
-// ((L >> 4) & 1) * 4 + ((L >> 3) & 1) * 2 + ((L >> 2) & 1).  Half of the values change hands in
-// each of the first three steps, nine shuffles instead of forty.
-__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
-#pragma unroll
-  for (int half = 4; half > 0; half >>= 1) {
-    const int stride = half * 4;
-    const bool upper = (lane & stride) != 0;
-#pragma unroll
-    for (int i = 0; i < half; ++i) {
-      const double send = upper ? v[i] : v[i + half];
-      const double keep = upper ? v[i + half] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, stride);
-    }
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-  return v[0];
-}
-
 // WARPS warps per token: one for large batches (four tokens a block, nothing exchanged), four
 // for small ones, where the chain of loads and FP64 sums of one token is what counts: they
 // share the contraction and repeat the short steps around it.  BATCH candidates are evaluated

@@ -75,6 +75,50 @@ def test_front_end_of_a_few_tokens(package, synthetic, experts, hidden, top_k, g
     layer.close()
 
 
+# one token of a latent layer: linears of every family join that launch, unfinished groups of eight outputs
+# and all; the routed sum, fc2_latent and the mixer are one launch behind the experts
+@pytest.mark.parametrize("experts,top_k,hidden,latent,shared,fc1,up", [
+    (64, 6, 448, 192, 704, "fp8", "fp8"), (160, 8, 4096, 64, 64, "bf16", "fp32"),
+    (512, 22, 1024, 320, 448, "fp32", "bf16"), (288, 32, 512, 64, 128, "fp8", "nvfp4")])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_one_token_of_a_latent_layer(package, synthetic, experts, top_k, hidden, latent, shared, fc1, up,
+                                     dtype):
+    cfg = synthetic.baseline_config(max_tokens=2, experts=experts, hidden=hidden, routed=64,
+                                    shared=shared, top_k=top_k, latent=latent)
+    data = synthetic.make_layer(cfg, seed=experts, device="cuda", norm_weight_uniform=True,
+                                latent_family=fc1, shared_up_family=up)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    x = synthetic.make_tokens(1, hidden, seed=9, device="cuda").to(dtype)
+    out, launches = (torch.empty(x.shape, device="cuda") for _ in range(2))
+    layer.enable_stage_timing(True)
+    assert layer.run(x, launches), layer.last_error
+    layer.enable_stage_timing(False)
+    for _ in range(2):
+        assert layer.run(x, out), layer.last_error
+        assert torch.equal(out, launches)
+    rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+    assert rep.ok(), rep.summary()
+    assert rep.latent_max_diff == 0.0
+    layer.close()
+
+
+# experts beyond 128 are narrowed down first, unless too many share the bound
+@pytest.mark.parametrize("experts,top_k,n_group", [(160, 1, 1), (256, 8, 8), (512, 22, 1), (512, 32, 4)])
+@pytest.mark.parametrize("levels", [1, 3, 100000])
+def test_selection_among_many_with_ties(package, oracle, experts, top_k, n_group, levels):
+    g = torch.Generator().manual_seed(experts + levels)
+    logits = torch.randint(-levels, levels, (9, experts), generator=g).float() / levels
+    bias = torch.randint(0, 2, (experts,), generator=g).float() * 0.25
+    index, weight = package.router_topk(logits.cuda(), bias.cuda(), top_k, n_group, max(1, n_group // 2),
+                                        True, 2.5)
+    want_index, want_weight = oracle.select_top_experts(logits.numpy(), bias.numpy(), top_k, n_group,
+                                                        max(1, n_group // 2), True, 2.5)
+    assert np.array_equal(index.cpu().numpy(), want_index)
+    # (the host's exponential is within an ulp)
+    assert np.allclose(weight.cpu().numpy(), want_weight, rtol=1e-6, atol=0)
+
+
 @pytest.mark.parametrize("rows", [3, 1185])
 @pytest.mark.parametrize("cols", [16, 1008, 2048, 2064, 4096, 4112, 5376, 6144, 6160])
 def test_quantiser_row_lengths(package, oracle, rows, cols):
