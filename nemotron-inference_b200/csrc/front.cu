@@ -16,7 +16,7 @@
 // (latent_tail_kernel, csrc/exact.cu) a pass of the checkpoint's layer is three launches instead of
 // twelve: 78.6 -> 57.9 us.  Two tokens are faster on three streams (88 us against 94 in this way).
 //
-// Blocks wait for others of the launch only where those have a lower index and wait for nothing, so that
+// Blocks wait only for blocks of a lower index, which are started before them, so that
 // they end whatever the GPU runs beside them; the wait is bounded all the same.
 #include <type_traits>
 

@@ -476,7 +476,7 @@ router_folded_logits_kernel(const __grid_constant__ CUtensorMap tmap_x,
 // pass 2: candidates -> FP64 logits -> exact selection
 // ---------------------------------------------------------------------------
 constexpr int kSelectWarps = 4;
-constexpr int kSelectPerLane = 8;  // experts <= 256
+constexpr int kSelectMaxPerLane = 8;  // experts <= 256
 
 __device__ __forceinline__ float sigmoid_exact(float v) {
   // Sigmoid of expert_layer.cpp:129-136 with exp evaluated in double
@@ -517,14 +517,16 @@ __device__ __forceinline__ double gate_scaled(uint32_t w) {
 // share the contraction and repeat the short steps around it.  BATCH candidates are evaluated
 // per pass over the row (at least top_k, so that one pass is the rule).
 // Measured, 128 experts, hidden 2688, bf16 in: 256 tokens 35 -> 17 us, 16384 tokens
-// 143 -> 119 us.
+// 143 -> 92 us.
+// Bound by instructions (60 % of the issue slots, half of them the integer ones of gate_scaled) and by the
+// warps there are to fill the rest: 72 registers, seven blocks to an SM, instead of 84 took 16384 tokens
+// from 106 to 92 us, 1003 from 21 to 16.5; the short steps with a lane per candidate and without rounds
+// that look through eight slots 119 to 106 before that.
 // Up to kSelectWholeBlockRows tokens the block form is the faster one (us, block against warp; 128
-// experts of 2688, top-6: 768 tokens 19.8 and 30.2, 1280 28.7 and 31.0, 1536 28.4 and 29.3, 2048 34.9
-// and 29.3; 256 experts, top-8: 1280 35.7 and 43.9, 1536 45.6 and 41.9; 128 experts of 4096: 1280
-// 31.0 and 36.6, 2048 38.5 and 35.6).
-constexpr int kSelectWholeBlockRows = 1280;
-template <bool IN_BF16, int WARPS, int BATCH>
-__global__ void __launch_bounds__(kSelectWarps * 32)
+// experts of 2688, top-6: 1400 tokens 22.7 and 27.2, 2048 24.1 and 27.4, 4096 38.6 and 35.7).
+constexpr int kSelectWholeBlockRows = 2048;
+template <bool IN_BF16, int WARPS, int BATCH, int kSelectPerLane>
+__global__ void __launch_bounds__(kSelectWarps * 32, BATCH <= 6 ? 7 : 5)
 router_select_exact_kernel(float* __restrict__ logits, int splits, const void* __restrict__ x,
                            const float* inv_rms,
                            const float* __restrict__ norm_weight,
@@ -580,25 +582,23 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
       key[j] = ordered_bits(choice[j]);
     }
   }
-  // the top_k-th largest pass-1 choice
+  // the top_k-th largest pass-1 choice (equal ones are taken together)
   uint32_t kth_key = 0u;
-  for (int r = 0; r < top_k; ++r) {
-    uint32_t local_key = 0u, local_index = 0xffffffffu;
+  for (int taken = 0; taken < top_k;) {
+    uint32_t most = key[0];
+#pragma unroll
+    for (int j = 1; j < kSelectPerLane; ++j) most = max(most, key[j]);
+    kth_key = __reduce_max_sync(0xffffffffu, most);
+    if (kth_key == 0u) break;  // (nothing is left)
+    int mine = 0;
 #pragma unroll
     for (int j = 0; j < kSelectPerLane; ++j) {
-      if (key[j] > local_key) {  // ascending j is ascending expert index: first maximum wins
-        local_key = key[j];
-        local_index = static_cast<uint32_t>(lane + 32 * j);
+      if (key[j] == kth_key) {
+        key[j] = 0u;
+        ++mine;
       }
     }
-    uint32_t best_index;
-    warp_arg_max(local_key, local_index, kth_key, best_index);
-    if ((best_index & 31u) == static_cast<uint32_t>(lane)) {
-#pragma unroll
-      for (int j = 0; j < kSelectPerLane; ++j) {
-        if (j == static_cast<int>(best_index >> 5)) key[j] = 0u;  // taken
-      }
-    }
+    taken += __reduce_add_sync(0xffffffffu, mine);
   }
   // candidates: everything that could still be in the exact top-k (a score that is no number
   // could be anywhere, so a row of them is re-evaluated as a whole and keeps them)
@@ -608,23 +608,16 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
     kth = __uint_as_float(b);
   }
   const float threshold = kth - tie_margin;
-  uint32_t mine = 0;
+  int total = 0;
 #pragma unroll
   for (int j = 0; j < kSelectPerLane; ++j) {
-    if (j < per_lane && !(choice[j] < threshold)) mine |= 1u << j;
-  }
-  const int my_count = __popc(mine);
-  int prefix = my_count;
-#pragma unroll
-  for (int stride = 1; stride < 32; stride <<= 1) {
-    const int other = __shfl_up_sync(0xffffffffu, prefix, stride);
-    if (lane >= stride) prefix += other;
-  }
-  const int total = __shfl_sync(0xffffffffu, prefix, 31);
-  int offset = prefix - my_count;
-#pragma unroll
-  for (int j = 0; j < kSelectPerLane; ++j) {
-    if ((mine >> j) & 1u) candidate_list[warp][offset++] = static_cast<int16_t>(lane + 32 * j);
+    const bool mine = j < per_lane && !(choice[j] < threshold);
+    const uint32_t lanes = __ballot_sync(0xffffffffu, mine);
+    if (mine) {
+      candidate_list[warp][total + __popc(lanes & ((1u << lane) - 1u))] =
+          static_cast<int16_t>(lane + 32 * j);
+    }
+    total += __popc(lanes);
   }
   __syncwarp();
 
@@ -635,7 +628,7 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
   const int chunks = hidden / 8;
   for (int base = 0; base < total; base += BATCH) {
     const int batch = min(BATCH, total - base);
-    const uint4* gate_row[BATCH];
+    uint32_t gate_row[BATCH];  // in chunks of eight values (fewer registers than addresses)
     double acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.0;
@@ -643,12 +636,14 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
     for (int i = 0; i < BATCH; ++i) {
       // (past the end of the list the last candidate once more, ignored below)
       const int e = candidate_list[warp][min(base + i, total - 1)];
-      gate_row[i] = reinterpret_cast<const uint4*>(gate + static_cast<size_t>(e) * hidden);
+      gate_row[i] = static_cast<uint32_t>(e) * static_cast<uint32_t>(chunks);
     }
     for (int ch = lane + 32 * part; ch < chunks; ch += 32 * WARPS) {
       uint4 g[BATCH];
 #pragma unroll
-      for (int i = 0; i < BATCH; ++i) g[i] = gate_row[i][ch];
+      for (int i = 0; i < BATCH; ++i) {
+        g[i] = reinterpret_cast<const uint4*>(gate)[gate_row[i] + ch];
+      }
       float xv[8];
       load_x8<IN_BF16>(x, static_cast<size_t>(row) * hidden + ch * 8, xv);
       const float4 w0 = *reinterpret_cast<const float4*>(norm_weight + ch * 8);
@@ -689,64 +684,86 @@ router_select_exact_kernel(float* __restrict__ logits, int splits, const void* _
   if (part != 0) return;
   __syncwarp();
 
-  // exact scores, compacted: lane L takes candidates L, L + 32, ... of the list, so the
-  // double-precision exponential runs once per lane instead of once per expert slot
-  float score[kSelectPerLane];
-  uint32_t cand_key[kSelectPerLane];
-  int cand_expert[kSelectPerLane];
-  const int rounds = (total + 31) / 32;
-#pragma unroll
-  for (int j = 0; j < kSelectPerLane; ++j) {
-    score[j] = 0.0f;
-    cand_key[j] = 0u;
-    cand_expert[j] = -1;
-    if (j < rounds) {
-      const int slot = lane + 32 * j;
-      if (slot < total) {
-        const int ex = candidate_list[warp][slot];
-        const float l = *reinterpret_cast<volatile float*>(row_logits + ex);
-        score[j] = sigmoid_exact(l);
-        cand_key[j] = ordered_bits(__fadd_rn(score[j], bias[ex]));
-        cand_expert[j] = ex;
+  // Exact scores, compacted: lane L takes candidate L of the list (L, L + 32, ... where there are more),
+  // so the double-precision exponential runs once per lane instead of once per expert slot.
+  int my_index = -1;  // lane r: the r-th selection
+  float my_score = 0.0f, weight_sum = 0.0f;
+  if (total <= 32) {
+    // a candidate's place is the number of those before it: nothing waits for a round before
+    const int ex = candidate_list[warp][min(lane, total - 1)];
+    const float score = sigmoid_exact(*reinterpret_cast<volatile float*>(row_logits + ex));
+    const uint32_t score_key = ordered_bits(__fadd_rn(score, bias[ex]));
+    int place = lane < total ? 0 : 32;
+    for (int c = 0; c < total; ++c) {
+      const uint32_t other = __shfl_sync(0xffffffffu, score_key, c);
+      const int other_ex = __shfl_sync(0xffffffffu, ex, c);
+      place += other > score_key || (other == score_key && other_ex < ex) ? 1 : 0;
+    }
+    for (int r = 0; r < top_k; ++r) {
+      const int owner = __ffs(__ballot_sync(0xffffffffu, place == r)) - 1;
+      const float s = __shfl_sync(0xffffffffu, score, owner);
+      const int index = __shfl_sync(0xffffffffu, ex, owner);
+      weight_sum = __fadd_rn(weight_sum, s);
+      if (lane == r) {
+        my_index = index;
+        my_score = s;
       }
     }
-  }
-  int my_index = -1;
-  float my_score = 0.0f;
-  for (int r = 0; r < top_k; ++r) {
-    uint32_t local_key = 0u, local_index = 0xffffffffu;
-    float local_score = 0.0f;
-    int local_slot = -1;
-#pragma unroll
+  } else {
+    float score[kSelectPerLane];
+    uint32_t cand_key[kSelectPerLane];
+    int cand_expert[kSelectPerLane];
+    const int rounds = (total + 31) / 32;
+  #pragma unroll
     for (int j = 0; j < kSelectPerLane; ++j) {
-      const uint32_t ex = static_cast<uint32_t>(cand_expert[j]);
-      if (cand_key[j] > local_key || (cand_key[j] == local_key && cand_key[j] != 0u &&
-                                      ex < local_index)) {
-        local_key = cand_key[j];
-        local_index = ex;
-        local_score = score[j];
-        local_slot = j;
+      score[j] = 0.0f;
+      cand_key[j] = 0u;
+      cand_expert[j] = -1;
+      if (j < rounds) {
+        const int slot = lane + 32 * j;
+        if (slot < total) {
+          const int ex = candidate_list[warp][slot];
+          const float l = *reinterpret_cast<volatile float*>(row_logits + ex);
+          score[j] = sigmoid_exact(l);
+          cand_key[j] = ordered_bits(__fadd_rn(score[j], bias[ex]));
+          cand_expert[j] = ex;
+        }
       }
     }
-    uint32_t best_key, best_index;
-    warp_arg_max(local_key, local_index, best_key, best_index);
-    const bool owner = local_key == best_key && local_index == best_index && local_slot >= 0;
-    const int owner_lane = __ffs(__ballot_sync(0xffffffffu, owner)) - 1;
-    const float s = __shfl_sync(0xffffffffu, local_score, owner_lane < 0 ? 0 : owner_lane);
-    if (owner) {
-#pragma unroll
+    for (int r = 0; r < top_k; ++r) {
+      uint32_t local_key = 0u, local_index = 0xffffffffu;
+      float local_score = 0.0f;
+      int local_slot = -1;
+  #pragma unroll
       for (int j = 0; j < kSelectPerLane; ++j) {
-        if (j == local_slot) cand_key[j] = 0u;  // taken
+        const uint32_t ex = static_cast<uint32_t>(cand_expert[j]);
+        if (cand_key[j] > local_key || (cand_key[j] == local_key && cand_key[j] != 0u &&
+                                        ex < local_index)) {
+          local_key = cand_key[j];
+          local_index = ex;
+          local_score = score[j];
+          local_slot = j;
+        }
+      }
+      uint32_t best_key, best_index;
+      warp_arg_max(local_key, local_index, best_key, best_index);
+      const bool owner = local_key == best_key && local_index == best_index && local_slot >= 0;
+      const int owner_lane = __ffs(__ballot_sync(0xffffffffu, owner)) - 1;
+      const float s = __shfl_sync(0xffffffffu, local_score, owner_lane < 0 ? 0 : owner_lane);
+      if (owner) {
+  #pragma unroll
+        for (int j = 0; j < kSelectPerLane; ++j) {
+          if (j == local_slot) cand_key[j] = 0u;  // taken
+        }
+      }
+      if (lane == r) {
+        my_index = static_cast<int>(best_index);
+        my_score = s;
       }
     }
-    if (lane == r) {
-      my_index = static_cast<int>(best_index);
-      my_score = s;
+    for (int r = 0; r < top_k; ++r) {
+      weight_sum = __fadd_rn(weight_sum, __shfl_sync(0xffffffffu, my_score, r));
     }
-  }
-  float weight_sum = 0.0f;
-  for (int r = 0; r < top_k; ++r) {
-    weight_sum = __fadd_rn(weight_sum, __shfl_sync(0xffffffffu, my_score, r));
   }
   if (lane < top_k) {
     float w = my_score;
@@ -831,7 +848,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
                                        int top_k, bool norm_topk_prob, float routed_scaling,
                                        float tie_margin, int32_t* top_index, float* top_weight,
                                        int32_t* expert_counts, int32_t* position, cudaStream_t stream) {
-  if (rows <= 0 || experts % 32 != 0 || experts > 32 * kSelectPerLane || top_k <= 0 ||
+  if (rows <= 0 || experts % 32 != 0 || experts > 32 * kSelectMaxPerLane || top_k <= 0 ||
       top_k > 32 || top_k > experts || hidden % 8 != 0 || splits < 1) {
     return cudaErrorInvalidValue;
   }
@@ -843,13 +860,22 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
         top_k, norm_topk_prob, routed_scaling, tie_margin, top_index, top_weight, expert_counts,
         position);
   };
+  auto run_lanes = [&](auto bf16, auto warps, auto batch) {
+    constexpr bool kBf16 = decltype(bf16)::value;
+    constexpr int kWarps = decltype(warps)::value, kBatch = decltype(batch)::value;
+    if (experts <= 128) {
+      run(router_select_exact_kernel<kBf16, kWarps, kBatch, 4>);
+    } else {
+      run(router_select_exact_kernel<kBf16, kWarps, kBatch, kSelectMaxPerLane>);
+    }
+  };
   auto run_batch = [&](auto bf16, auto warps) {
     if (top_k <= 4) {
-      run(router_select_exact_kernel<decltype(bf16)::value, decltype(warps)::value, 4>);
+      run_lanes(bf16, warps, std::integral_constant<int, 4>());
     } else if (top_k <= 6) {
-      run(router_select_exact_kernel<decltype(bf16)::value, decltype(warps)::value, 6>);
+      run_lanes(bf16, warps, std::integral_constant<int, 6>());
     } else {
-      run(router_select_exact_kernel<decltype(bf16)::value, decltype(warps)::value, 8>);
+      run_lanes(bf16, warps, std::integral_constant<int, 8>());
     }
   };
   using One = std::integral_constant<int, 1>;

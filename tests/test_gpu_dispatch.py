@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def small_layer(package, synthetic):
-    cfg = synthetic.baseline_config(max_tokens=2048, experts=32, hidden=512, routed=256, shared=512)
+    cfg = synthetic.baseline_config(max_tokens=2049, experts=32, hidden=512, routed=256, shared=512)
     data = synthetic.make_layer(cfg, seed=41, device="cuda", norm_weight_uniform=True)
     layer = package.ExpertLayerSlice.create(cfg, data.bindings)
     assert layer is not None and layer.valid(), package.ExpertLayerSlice.create_error
@@ -21,9 +21,9 @@ def small_layer(package, synthetic):
 
 # 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; CTA pairs from 100 rows per expert (534 tokens); the shared expert in
 # the routed experts' launch up to 640; a block per row in the quantiser up to 888, per token in the
-# exact selection up to 1280
+# exact selection up to 2048
 @pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 888, 889, 1184, 1185,
-                                    1280, 1281])
+                                    1280, 1281, 2048, 2049])
 def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
     layer, data = small_layer
     x = synthetic.make_tokens(tokens, 512, seed=300 + tokens, device="cuda")
