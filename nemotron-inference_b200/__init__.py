@@ -186,7 +186,8 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
 
 
 def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (the raw handle: a torch.cuda.Stream object around it takes as long as a launch)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _dtype_code(t: torch.Tensor) -> int:

@@ -613,6 +613,13 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       if (lane == 0) {
         *args.ticket = 0;
         *args.finished = 0;
+        if (args.error_host != nullptr) {
+          const int code = *static_cast<volatile int32_t*>(args.error);
+          if (code != kDevOk) {
+            *static_cast<volatile int32_t*>(args.error_host) = code;
+            __threadfence_system();
+          }
+        }
       }
     }
   }

@@ -183,6 +183,8 @@ struct StreamArgs {
   bool fetch_dense = false;
   int32_t* ticket = nullptr;
   int32_t* finished = nullptr;
+  // nullable, host memory: the last CTA stores there what it finds in `error`, unless that is nothing
+  int32_t* error_host = nullptr;
 };
 inline int stream_tile_rows(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
 cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, LaunchStream stream);

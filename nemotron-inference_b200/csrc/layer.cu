@@ -485,8 +485,9 @@ struct StreamCounts {
 // The shared expert comes first among the up projections and among the down projections: its down
 // tiles are the longest, and short ones end together.
 void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCounts& counts,
-                int32_t* error, int num_sms, LaunchStream stream) {
+                int32_t* error, int num_sms, LaunchStream stream, int32_t* error_host = nullptr) {
   StreamArgs args;
+  args.error_host = error_host;
   args.fetch_dense = stream.chained;
   args.error = error;
   args.finished = counts.words.as<int32_t>();
@@ -557,7 +558,8 @@ nmoe_status status_from_device(int code) {
 
 // Hands the error word to the host and clears it: one launch in the place of a copy and a memset,
 // whose start-up a synchronous call over few rows waits for (64 rows through one expert, measured on
-// the host: 60.6 us with them, 50.7 so).
+// the host: 60.6 us with them, 50.7 so, 40.7 where the last CTA of the FFN's launch leaves an
+// error with the host by itself).
 __global__ void publish_error_kernel(int32_t* device, volatile int32_t* host) {
   *host = atomicExch(device, 0);
   __threadfence_system();
@@ -565,7 +567,7 @@ __global__ void publish_error_kernel(int32_t* device, volatile int32_t* host) {
 
 struct ErrorSlot {
   DeviceBuffer device;
-  int32_t* host = nullptr;  // pinned, written by publish_error_kernel
+  int32_t* host = nullptr;  // pinned, written by publish_error_kernel or a launch's last CTA
   void create() {
     device.allocate(sizeof(int32_t), true);
     NMOE_CUDA(cudaMallocHost(&host, sizeof(int32_t)));
@@ -574,11 +576,18 @@ struct ErrorSlot {
   ~ErrorSlot() {
     if (host != nullptr) cudaFreeHost(host);
   }
-  nmoe_status sync(cudaStream_t stream) {
+  // `published`: what was launched last has left its word with the host, if there is one.
+  nmoe_status sync(cudaStream_t stream, bool published = false) {
+    if (published) {
+      NMOE_CUDA(cudaStreamSynchronize(stream));
+      if (*static_cast<volatile int32_t*>(host) == kDevOk) return NMOE_OK;
+    }
     publish_error_kernel<<<1, 1, 0, stream>>>(device.as<int32_t>(), host);
     NMOE_CUDA(cudaGetLastError());
     NMOE_CUDA(cudaStreamSynchronize(stream));
-    return status_from_device(*static_cast<volatile int32_t*>(host));
+    const int code = *static_cast<volatile int32_t*>(host);
+    *host = kDevOk;
+    return status_from_device(code);
   }
 };
 
@@ -799,6 +808,7 @@ struct nmoe_ffn {
   StreamCounts stream_counts;
   ErrorSlot error;
   int last_rows = 0;
+  bool status_published = false;  // the last launch leaves its error word with the host
   std::string last_error;
 };
 
@@ -892,13 +902,14 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
       both.out = out;
       both.row_slots = (static_cast<int>(rows) + 127) / 128;
       run_stream(nullptr, &both, ffn->stream_counts, error, ffn->num_sms,
-                 LaunchStream(stream, true));
+                 LaunchStream(stream, true), ffn->error.host);
     } else {
       run_expert_gemms(ffn->up, ffn->down, tile_class, ffn->a_op, ffn->a_ts.as<float>(), schedule,
                        ffn->h_packed.as<uint8_t>(), ffn->h_sf.as<uint8_t>(), ffn->h_op, out, error,
                        ffn->num_sms, stream);
     }
     ffn->last_rows = static_cast<int>(rows);
+    ffn->status_published = tile_class == kClassStream;
   } catch (const Failure& failure) {
     ffn->last_error = failure.message;
     return failure.status;
@@ -909,7 +920,7 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
 nmoe_status nmoe_ffn_sync_status(nmoe_ffn* ffn, void* stream_ptr) {
   if (ffn == nullptr) return NMOE_ERR_INVALID_ARGUMENT;
   try {
-    return ffn->error.sync(static_cast<cudaStream_t>(stream_ptr));
+    return ffn->error.sync(static_cast<cudaStream_t>(stream_ptr), ffn->status_published);
   } catch (const Failure& failure) {
     ffn->last_error = failure.message;
     return failure.status;

@@ -92,3 +92,23 @@ def test_ffn_rows_on_a_16_byte_boundary(package, synthetic, variant):
     assert torch.equal(room[4:-4].view(70, 448), expected)
     assert not room[:4].any() and not room[-4:].any()
     ffn.close()
+
+
+@pytest.mark.parametrize("variants", [(3, 3), (1, 3), (3, 1)])
+def test_ffn_status_is_that_of_the_runs_since_the_last_one(package, synthetic, variants):
+    # rows beyond 6 * 448 are reported once, whichever kernel found them and whichever ran after it
+    up, down = synthetic.make_ffn_weights(448, 192, seed=5, device="cuda")
+    ffn = package.ExpertFfn(up, down, max_rows=128)
+    up.tensor_scale *= 400.0
+    beyond = package.ExpertFfn(up, down, max_rows=128)
+    x = synthetic.make_tokens(40, 448, seed=6, device="cuda")
+    out = torch.empty(40, 448, device="cuda")
+    lib, stream = package.load_library(), package._stream()
+    for f, expected in ((beyond, 5), (ffn, package.NMOE_OK)):  # (5: NMOE_ERR_ACTIVATION_RANGE)
+        for _ in range(2):
+            for variant in variants:
+                assert lib.nmoe_ffn_run(f._handle, stream, x.data_ptr(), package._dtype_code(x), 40,
+                                        out.data_ptr(), variant) == 0
+            assert lib.nmoe_ffn_sync_status(f._handle, stream) == expected
+        assert lib.nmoe_ffn_sync_status(f._handle, stream) == package.NMOE_OK
+        f.close()
