@@ -17,6 +17,7 @@
 // One token row or a handful is bound by reading W instead: exact_gemv_kernel reads W in the
 // form it came in (FP8, bf16 or FP32) and sums in FP64.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -98,11 +99,13 @@ __device__ __forceinline__ size_t slice_offset(size_t row, int slice, int k, int
 constexpr int kSliceThreads = 256;
 
 // One block per row, the row in registers (STEPS times eight consecutive values per thread): its
-// largest magnitude, then the digits.  KIND < 0: FP32 activation rows.
+// largest magnitude, then the digits.  KIND < 0: FP32 activation rows, with `sums` each the sum of top_k
+// rows of `in`, which is written there.
 template <int KIND, int STEPS>
 __global__ void __launch_bounds__(kSliceThreads)
 slice_rows_kernel(const void* __restrict__ in, int K, float scale, int tile_rows,
-                  int8_t* __restrict__ slices, SliceRow* __restrict__ info) {
+                  int8_t* __restrict__ slices, SliceRow* __restrict__ info, int top_k,
+                  float* __restrict__ sums) {
   __shared__ float warp_max[kSliceThreads / 32];
   const size_t row = blockIdx.x;
   float v[STEPS][8];
@@ -115,10 +118,22 @@ slice_rows_kernel(const void* __restrict__ in, int K, float scale, int tile_rows
     for (int j = 0; j < 8; ++j) v[s][j] = 0.0f;
     if (k < K) {
       if constexpr (KIND < 0) {
-        const float4* from =
-            reinterpret_cast<const float4*>(reinterpret_cast<const float*>(in) + row * K + k);
-        const float4 a = from[0], b = from[1];
-        const float raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const float* first = reinterpret_cast<const float*>(in) + row * top_k * K + k;
+        float raw[8];
+        load8<false>(first, 0, raw);
+        if (sums != nullptr) {
+          // the row is a sum of parts in selection order (expert_layer.cpp:951-953)
+#pragma unroll 4
+          for (int p = 1; p < top_k; ++p) {
+            float part[8];
+            load8<false>(first, static_cast<size_t>(p) * K, part);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) raw[j] = __fadd_rn(raw[j], part[j]);
+          }
+          float4* to = reinterpret_cast<float4*>(sums + row * K + k);
+          to[0] = make_float4(raw[0], raw[1], raw[2], raw[3]);
+          to[1] = make_float4(raw[4], raw[5], raw[6], raw[7]);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[s][j] = input_value(raw[j], scale);
       } else {
@@ -184,9 +199,9 @@ slice_rows_kernel(const void* __restrict__ in, int K, float scale, int tile_rows
 
 template <int KIND>
 void launch_slices(const void* in, int rows, int K, float scale, int tile_rows, int8_t* slices,
-                   SliceRow* info, cudaStream_t stream) {
+                   SliceRow* info, cudaStream_t stream, int top_k = 1, float* sums = nullptr) {
   auto run = [&](auto kernel) {
-    kernel<<<rows, kSliceThreads, 0, stream>>>(in, K, scale, tile_rows, slices, info);
+    kernel<<<rows, kSliceThreads, 0, stream>>>(in, K, scale, tile_rows, slices, info, top_k, sums);
   };
   if (K <= 2 * kSliceThreads * 8) {
     run(slice_rows_kernel<KIND, 2>);
@@ -430,72 +445,97 @@ __device__ __forceinline__ double two_to(int e) {
 
 constexpr int kFinishThreads = 256;
 
-// FP32 results from the doubles of exact_gemm_kernel: one thread per value.
+// FP32 results from the doubles of exact_gemm_kernel, VALUES per thread.
 //
 // B, in units of 2^(ea + ew): K * 2^-52 for the digit products of level 7 and beyond (two pairs of
 // digits up to 128 at level 7, one at level 8: K * 2^-53 * 1.01); 2^-39 for every value of the two
 // rows that its digits do not hold exactly; and |r| * 2^-50 for the roundings of the doubles (three
 // of 2^-53: a sum of fewer than five levels is below 2^53).  The parts of a split sum may cancel, so
 // there it is their magnitudes that count, for those three and for every addition of a part.
-template <int KIND>
+template <int KIND, int VALUES>
 __global__ void __launch_bounds__(kFinishThreads)
 exact_finish_kernel(const double* __restrict__ partial, int splits, int rows, int N, int K,
                     const float* __restrict__ in, float fp8_scale,
                     const SliceRow* __restrict__ in_info, const void* __restrict__ weight,
                     float weight_scale, const SliceRow* __restrict__ weight_info,
-                    const float* __restrict__ offset, bool relu2, float* __restrict__ out) {
+                    const float* __restrict__ offset, bool relu2, float* __restrict__ out,
+                    const ExactMix mix) {
   constexpr int V = WeightVector<KIND>::kCount;
   __shared__ int open_count;
-  __shared__ int open_list[kFinishThreads];
+  __shared__ int open_list[kFinishThreads * VALUES];
   __shared__ double warp_sum[kFinishThreads / 32];
   if (threadIdx.x == 0) open_count = 0;
   __syncthreads();
   const int t = blockIdx.y;
-  const int n = blockIdx.x * kFinishThreads + threadIdx.x;
-  const size_t i = static_cast<size_t>(t) * N + n;
-  float result = 0.0f;
-  bool decided = true;
-  if (n < N) {
-    const size_t count = static_cast<size_t>(rows) * N;
-    double r = partial[i];
+  const int first_n = blockIdx.x * (kFinishThreads * VALUES) + threadIdx.x;
+  const size_t first = static_cast<size_t>(t) * N + first_n;
+  const size_t count = static_cast<size_t>(rows) * N;
+  const SliceRow a = in_info[t];
+  // (the loads of all values are on their way before the first of them is looked at)
+  double r[VALUES];
+  SliceRow w[VALUES];
+  float x[VALUES], shared[VALUES];
+#pragma unroll
+  for (int v = 0; v < VALUES; ++v) {
+    const size_t i = first + v * kFinishThreads;
+    r[v] = 0.0;
+    w[v] = SliceRow{0, 0};
+    x[v] = shared[v] = 0.0f;
+    if (first_n + v * kFinishThreads >= N) continue;
+    r[v] = partial[i];
+    w[v] = weight_info[first_n + v * kFinishThreads];
+    if (mix.out != nullptr) {
+      x[v] = mix.in_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(mix.in)[i])
+                         : reinterpret_cast<const float*>(mix.in)[i];
+      shared[v] = mix.shared[i];
+    }
+  }
+  float result[VALUES];
+#pragma unroll
+  for (int v = 0; v < VALUES; ++v) {
+    const size_t i = first + v * kFinishThreads;
+    const int n = first_n + v * kFinishThreads;
+    result[v] = 0.0f;
+    if (n >= N) continue;
+    double sum = r[v];
 #pragma unroll 4
-    for (int s = 1; s < splits; ++s) r += partial[i + s * count];
-    const SliceRow a = in_info[t], w = weight_info[n];
-    decided = a.exponent != kNoExponent && w.exponent != kNoExponent;
+    for (int s = 1; s < splits; ++s) sum += partial[i + s * count];
+    bool decided = a.exponent != kNoExponent && w[v].exponent != kNoExponent;
     if (decided) {
-      const int e = a.exponent + w.exponent;
-      r *= two_to(e - (12 + 8 * (kLevels - 1)));
-      const double left_out = K + 8192.0 * (a.inexact + w.inexact);
-      double bound = left_out * two_to(e - 52) + fabs(r) * 0x1p-50;
+      const int e = a.exponent + w[v].exponent;
+      sum *= two_to(e - (12 + 8 * (kLevels - 1)));
+      const double left_out = K + 8192.0 * (a.inexact + w[v].inexact);
+      double bound = left_out * two_to(e - 52) + fabs(sum) * 0x1p-50;
       if (splits > 1) {
         double magnitude = 0.0;
         for (int s = 0; s < splits; ++s) magnitude += fabs(partial[i + s * count]);
         bound += magnitude * two_to(e - (12 + 8 * (kLevels - 1)) - 53) * (splits + 7);
       }
-      const float low = static_cast<float>(r - bound), high = static_cast<float>(r + bound);
+      const float low = static_cast<float>(sum - bound), high = static_cast<float>(sum + bound);
       decided = low == high;
-      result = static_cast<float>(r);
+      result[v] = static_cast<float>(sum);
     }
+    if (!decided) open_list[atomicAdd(&open_count, 1)] = n;
   }
-  if (!decided) open_list[atomicAdd(&open_count, 1)] = n;
   __syncthreads();
   // the block forms the FP64 sum of one undecided value at a time, each thread a part of it
   for (int o = 0; o < open_count; ++o) {
-    const float* x = in + static_cast<size_t>(t) * K;
-    const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
-                                                    static_cast<size_t>(open_list[o]) * K * (16 / V));
+    const float* row = in + static_cast<size_t>(t) * K;
+    const uint4* weights =
+        reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(weight) +
+                                       static_cast<size_t>(open_list[o]) * K * (16 / V));
     double sum = 0.0;
     for (int q = threadIdx.x; q * V < K; q += kFinishThreads) {
-      float v[V];
-      WeightVector<KIND>::unpack(w[q], weight_scale, v);
+      float values[V];
+      WeightVector<KIND>::unpack(weights[q], weight_scale, values);
 #pragma unroll
       for (int j = 0; j < V; j += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(x + q * V + j);
-        const float av[4] = {a.x, a.y, a.z, a.w};
+        const float4 four = *reinterpret_cast<const float4*>(row + q * V + j);
+        const float av[4] = {four.x, four.y, four.z, four.w};
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
           sum = fma(static_cast<double>(input_value(av[h], fp8_scale)),
-                    static_cast<double>(v[j + h]), sum);
+                    static_cast<double>(values[j + h]), sum);
         }
       }
     }
@@ -505,18 +545,33 @@ exact_finish_kernel(const double* __restrict__ partial, int splits, int rows, in
     }
     if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
     __syncthreads();
-    if (n == open_list[o]) {
+#pragma unroll
+    for (int v = 0; v < VALUES; ++v) {
+      if (first_n + v * kFinishThreads != open_list[o]) continue;
       double total = 0.0;
 #pragma unroll
       for (int w8 = 0; w8 < kFinishThreads / 32; ++w8) total += warp_sum[w8];
-      result = static_cast<float>(total);
+      result[v] = static_cast<float>(total);
     }
     __syncthreads();
   }
-  if (n < N) {
-    if (offset != nullptr) result = __fadd_rn(result, offset[n]);
-    if (relu2) result = result > 0.0f ? __fmul_rn(result, result) : 0.0f;
-    out[i] = result;
+#pragma unroll
+  for (int v = 0; v < VALUES; ++v) {
+    const int n = first_n + v * kFinishThreads;
+    if (n >= N) continue;
+    const size_t i = first + v * kFinishThreads;
+    float y = result[v];
+    if (offset != nullptr) y = __fadd_rn(y, offset[n]);
+    if (relu2) y = y > 0.0f ? __fmul_rn(y, y) : 0.0f;
+    out[i] = y;
+    if (mix.out != nullptr) {
+      const float mixed = __fadd_rn(x[v], __fadd_rn(y, shared[v]));
+      if (mix.out_bf16) {
+        reinterpret_cast<__nv_bfloat16*>(mix.out)[i] = __float2bfloat16_rn(mixed);
+      } else {
+        reinterpret_cast<float*>(mix.out)[i] = mixed;
+      }
+    }
   }
 }
 
@@ -1264,10 +1319,17 @@ int exact_splits(int rows, int N, int K, int num_sms) {
 
 cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows, float fp8_scale,
                                 const float* offset, bool relu2, const ExactWorkspace& space,
-                                float* out, int32_t* error, int num_sms, cudaStream_t stream) {
+                                float* out, int32_t* error, int num_sms, cudaStream_t stream,
+                                const ExactSum& sum, const ExactMix& mix) {
   if (rows <= 0 || !exact_supported(w.N, w.K)) return cudaErrorInvalidValue;
   const int nt = exact_tile_rows(rows);
-  launch_slices<-1>(in, rows, w.K, fp8_scale, nt, space.slices, space.info, stream);
+  if (sum.parts != nullptr) {
+    launch_slices<-1>(sum.parts, rows, w.K, fp8_scale, nt, space.slices, space.info, stream, sum.top_k,
+                      sum.sums);
+    in = sum.sums;
+  } else {
+    launch_slices<-1>(in, rows, w.K, fp8_scale, nt, space.slices, space.info, stream);
+  }
   const int row_tiles = (rows + nt - 1) / nt;
   const int splits = exact_splits(rows, w.N, w.K, num_sms);
   const int grid = (w.N + kExactRows - 1) / kExactRows * row_tiles * splits;
@@ -1285,18 +1347,27 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
       : nt == 48 ? multiply(exact_gemm_kernel<kSlices, 48>, Shape::smem_bytes(48))
                  : multiply(exact_gemm_kernel<kSlices, 64>, Shape::smem_bytes(64));
   if (err != cudaSuccess) return err;
-  const dim3 blocks((w.N + kFinishThreads - 1) / kFinishThreads, rows, 1);
-  auto run = [&](auto kernel) {
-    kernel<<<blocks, kFinishThreads, 0, stream>>>(space.partial, splits, rows, w.N, w.K, in,
-                                                  fp8_scale, space.info, w.weight, w.scale, w.info,
-                                                  offset, relu2, out);
+  auto run = [&](auto kernel, int values) {
+    const int columns = kFinishThreads * values;
+    kernel<<<dim3((w.N + columns - 1) / columns, rows), kFinishThreads, 0, stream>>>(
+        space.partial, splits, rows, w.N, w.K, in, fp8_scale, space.info, w.weight, w.scale, w.info,
+        offset, relu2, out, mix);
+  };
+  // four values a thread where that leaves none of a block's threads without one
+  auto run_kind = [&](auto kind) {
+    constexpr int kKind = decltype(kind)::value;
+    if (w.N >= 4 * kFinishThreads) {
+      run(exact_finish_kernel<kKind, 4>, 4);
+    } else {
+      run(exact_finish_kernel<kKind, 1>, 1);
+    }
   };
   if (w.kind == kWeightFp8) {
-    run(exact_finish_kernel<kWeightFp8>);
+    run_kind(std::integral_constant<int, kWeightFp8>());
   } else if (w.kind == kWeightBf16) {
-    run(exact_finish_kernel<kWeightBf16>);
+    run_kind(std::integral_constant<int, kWeightBf16>());
   } else {
-    run(exact_finish_kernel<kWeightF32>);
+    run_kind(std::integral_constant<int, kWeightF32>());
   }
   return cudaGetLastError();
 }

@@ -325,11 +325,27 @@ struct ExactWorkspace {
   SliceRow* info;   // [rows]
   double* partial;  // exact_splits() * rows * N
 };
+// What a linear may take in and hand on itself, in the place of kernels before and behind it: rows that
+// are sums of `top_k` parts each ([rows][top_k][K]; written to `sums` [rows][K], which stands for `in`),
+// and out = in + (y + shared), all [rows][N].
+struct ExactSum {
+  const float* parts = nullptr;
+  int top_k = 1;
+  float* sums = nullptr;
+};
+struct ExactMix {
+  const void* in = nullptr;
+  bool in_bf16 = false;
+  const float* shared = nullptr;
+  void* out = nullptr;
+  bool out_bf16 = false;
+};
 // `fp8_scale` != 0: every value of `in` takes the round trip of the scaled-FP8 family first.
 // `offset` (nullable [N]) is added to the rounded sum, `relu2` then squares what is positive.
 cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows, float fp8_scale,
                                 const float* offset, bool relu2, const ExactWorkspace& space,
-                                float* out, int32_t* error, int num_sms, cudaStream_t stream);
+                                float* out, int32_t* error, int num_sms, cudaStream_t stream,
+                                const ExactSum& sum = ExactSum(), const ExactMix& mix = ExactMix());
 bool exact_prefers_gemv(int rows, int N, int K, int num_sms);
 // The same for a handful of rows: reads W once per four rows, no slices.
 cudaError_t launch_exact_gemv(const ExactWeight& w, const float* in, float fp8_scale, int rows,

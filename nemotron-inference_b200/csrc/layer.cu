@@ -1766,6 +1766,18 @@ void latent_tail(nmoe_layer* L, LaunchStream stream, const void* input, nmoe_dty
     NMOE_CUDA(launch_latent_tail(L->fc2.operand.w, tail, stream));
     return;
   }
+  if (L->fc2.exact && tokens <= L->exact.max_rows &&
+      !exact_prefers_gemv(tokens, L->fc2.out, L->fc2.in, L->num_sms)) {
+    const ExactWorkspace space{L->exact.slices.as<int8_t>(), L->exact.info.as<SliceRow>(),
+                               L->exact.partial.as<double>()};
+    const ExactSum sum{L->parts.as<float>(), K, L->routed_latent.as<float>()};
+    const ExactMix mix{input, in_dtype == NMOE_BF16, L->shared_rows.as<float>(), output,
+                       out_dtype == NMOE_BF16};
+    NMOE_CUDA(launch_exact_linear(L->fc2.operand.w, nullptr, tokens, 0.0f, nullptr, false, space,
+                                  L->projected.as<float>(), L->error.device.as<int32_t>(), L->num_sms,
+                                  stream, sum, mix));
+    return;
+  }
   NMOE_CUDA(launch_sum_parts(L->parts.as<float>(), tokens, Lr, K, L->routed_latent.as<float>(),
                              stream));
   run_linear(L, L->fc2, L->exact, L->routed_latent.as<float>(), tokens, L->projected.as<float>(), false,
