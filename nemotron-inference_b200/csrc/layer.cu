@@ -1529,9 +1529,10 @@ void run_ffn(nmoe_layer* L, bool unfused, const WeightStack& up, const WeightSta
 }
 
 // Up to this many tokens the shared expert's tiles join the routed experts' launch; with more its
-// GEMMs are long enough to be worth running beside the router (512 tokens 199 against 203 us,
-// 1003 tokens 231 against 229, 2048 tokens 281 against 274).
-constexpr int kSharedInLaunchTokens = 640;
+// GEMMs are long enough to be worth running beside the router (joined against beside: 700 tokens 178.4
+// us and 187.8, 1003 195.5 and 202.8, 1200 210 and 225, 1400 217 and 215.5, 1800 234 and 231; popular and
+// unpopular experts, 1200 tokens 190 and 204, 1800 246 and 241).
+constexpr int kSharedInLaunchTokens = 1280;
 
 // Routed rows per expert (on average) up to which csrc/expert_stream.cu takes them: with more, most
 // experts have a second row tile and their weights would be read twice.  Where the two meet depends

@@ -33,6 +33,21 @@ def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
     assert rep.ok(), rep.summary()
 
 
+def test_shared_expert_on_both_sides_of_its_line(package, synthetic):
+    # in the routed experts' launch up to 1280 tokens, beside the router from there
+    cfg = synthetic.baseline_config(max_tokens=1281, experts=128, hidden=256, routed=64, shared=192)
+    data = synthetic.make_layer(cfg, seed=45, device="cuda", norm_weight_uniform=True)
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    for tokens in (1280, 1281):
+        x = synthetic.make_tokens(tokens, 256, seed=tokens, device="cuda")
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        assert layer.run(x, out), layer.last_error
+        rep = helpers.compare_layer_with_oracle(layer, data, x, out)
+        assert rep.ok(), rep.summary()
+    layer.close()
+
+
 def test_pairs_share_rows_of_every_count(package, synthetic):
     # experts without rows, with fewer than a box of them and with several pairs of tiles
     cfg = synthetic.baseline_config(max_tokens=1501, experts=32, hidden=512, routed=256, shared=512)
