@@ -1076,14 +1076,17 @@ struct nmoe_layer {
     int in_dtype, out_dtype;
     RowKind parts_kind;
     bool normalized;
-    cudaGraphExec_t exec;
+    cudaGraphExec_t exec;  // null while the run is not worth recording yet
     uint64_t last_use;
+    int eager_runs = 0;
   };
   std::vector<RecordedRun> recorded;
   int graph_max_tokens = 256;
   uint64_t run_counter = 0;
   void drop_recorded() {
-    for (RecordedRun& r : recorded) cudaGraphExecDestroy(r.exec);
+    for (RecordedRun& r : recorded) {
+      if (r.exec != nullptr) cudaGraphExecDestroy(r.exec);
+    }
     recorded.clear();
   }
 
@@ -2012,6 +2015,13 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   L->mark(10, stream);
 }
 
+// A latent layer's graph has three branches, and recording it costs a new pair of buffers 420 us more
+// than launching the pass (40 tokens: 784 us and 366 from an idle device; 2 tokens 415 and 115), while
+// a replay saves 9 to 12 us over the launches (40 tokens 342 and 354 us a pass, 2 tokens 90 and 100).
+// So it is recorded when the launches have cost as much as that.  One token is one branch and,
+// like every layer without a latent form, is recorded at once.
+constexpr int kEagerRunsOfBranches = 32;
+
 // nmoe_layer_run: small batches replay a recorded CUDA graph of the same run.
 void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input,
                            nmoe_dtype in_dtype, int tokens, void* output, nmoe_dtype out_dtype) {
@@ -2026,10 +2036,14 @@ void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input
     return;
   }
   ++L->run_counter;
+  const bool branches = L->latent_stream != nullptr && tokens >= kBesideMinTokens;
+  nmoe_layer::RecordedRun* known = nullptr;
   for (nmoe_layer::RecordedRun& r : L->recorded) {
     if (r.input == input && r.output == output && r.tokens == tokens &&
         r.in_dtype == in_dtype && r.out_dtype == out_dtype) {
       r.last_use = L->run_counter;
+      known = &r;
+      if (r.exec == nullptr) break;
       NMOE_CUDA(cudaGraphLaunch(r.exec, stream));
       L->last_tokens = tokens;
       L->last_parts_kind = r.parts_kind;
@@ -2037,6 +2051,24 @@ void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input
       L->last_unfused = false;
       return;
     }
+  }
+  if (known == nullptr) {
+    if (L->recorded.size() >= 16) {  // forget the run that was used longest ago
+      size_t oldest = 0;
+      for (size_t i = 1; i < L->recorded.size(); ++i) {
+        if (L->recorded[i].last_use < L->recorded[oldest].last_use) oldest = i;
+      }
+      if (L->recorded[oldest].exec != nullptr) cudaGraphExecDestroy(L->recorded[oldest].exec);
+      L->recorded.erase(L->recorded.begin() + static_cast<long>(oldest));
+    }
+    L->recorded.push_back(nmoe_layer::RecordedRun{input, output, tokens, in_dtype, out_dtype,
+                                                  RowKind(), false, nullptr, L->run_counter});
+    known = &L->recorded.back();
+  }
+  if (branches && known->eager_runs < kEagerRunsOfBranches) {
+    ++known->eager_runs;
+    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
+    return;
   }
   // record: the launches below go into a graph instead of onto the stream
   if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -2064,17 +2096,9 @@ void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input
     layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
     return;
   }
-  if (L->recorded.size() >= 16) {  // forget the run that was used longest ago
-    size_t oldest = 0;
-    for (size_t i = 1; i < L->recorded.size(); ++i) {
-      if (L->recorded[i].last_use < L->recorded[oldest].last_use) oldest = i;
-    }
-    cudaGraphExecDestroy(L->recorded[oldest].exec);
-    L->recorded.erase(L->recorded.begin() + static_cast<long>(oldest));
-  }
-  L->recorded.push_back(nmoe_layer::RecordedRun{input, output, tokens, in_dtype, out_dtype,
-                                                L->last_parts_kind, L->last_normalized, exec,
-                                                L->run_counter});
+  known->parts_kind = L->last_parts_kind;
+  known->normalized = L->last_normalized;
+  known->exec = exec;
   NMOE_CUDA(cudaGraphLaunch(exec, stream));
 }
 
