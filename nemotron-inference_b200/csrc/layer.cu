@@ -748,11 +748,13 @@ struct DenseLinear {
   }
 };
 
-// Workspace of the correctly rounded linears: sliced activation rows (up to `max_rows` at a time;
-// longer batches go through in turn) and the partial sums.
+// Workspace of the linears that run one after the other on a stream.  Of the correctly rounded ones:
+// sliced activation rows (up to `max_rows` at a time; longer batches go through in turn) and the partial
+// sums.  Of scaled-FP8 ones with contractions too long for that: the rows after their round trip.
 struct ExactScratch {
   int max_rows = 0;
   DeviceBuffer slices, info, partial;
+  DeviceBuffer round_trip;  // [tokens][in] FP32
   // `shapes`: (N, K) of every linear that will run
   void allocate(size_t tokens, const std::vector<std::pair<int, int>>& shapes, int num_sms) {
     max_rows = static_cast<int>(std::min<size_t>(tokens, 1024));
@@ -768,6 +770,10 @@ struct ExactScratch {
     // a split contraction has at most one tile of 128 x 80 sums per SM
     partial.allocate(std::max(max_rows * most_n, static_cast<size_t>(num_sms) * 128 * 80) *
                      sizeof(double));
+  }
+  void allocate_round_trip(size_t tokens, const DenseLinear& linear) {
+    if (!linear.fp8 || linear.exact) return;
+    round_trip.allocate(tokens * static_cast<size_t>(linear.in) * sizeof(float));
   }
 };
 
@@ -986,7 +992,6 @@ struct nmoe_layer {
   // fc1 output and its NVFP4 form
   DeviceBuffer latent_rows, lat_packed, lat_sf_row_major, lat_sf_tiled, lat_ts;
   DeviceBuffer routed_latent, projected, shared_rows;               // [T][latent], [T][H], [T][H]
-  DeviceBuffer fp8_tmp;                                             // activation round trip
   DeviceBuffer shared_raw;  // [T][S] FP32: shared_up output, activated in place
   DeviceBuffer sh_ts;       // per-row tensor scale of the quantised shared intermediate
 
@@ -1172,14 +1177,13 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
     L->projected.allocate(T * H * sizeof(float));
     L->shared_rows.allocate(T * H * sizeof(float));
   }
-  if ((L->fc1.fp8 && !L->fc1.exact) || (L->shared_up_dense.fp8 && !L->shared_up_dense.exact) ||
-      (L->shared_down_dense.fp8 && !L->shared_down_dense.exact)) {
-    L->fp8_tmp.allocate(T * static_cast<size_t>(std::max(H, S)) * sizeof(float));
-  }
   if (L->shared_up_dense.present || L->shared_down_dense.present || L->unfused) {
     L->shared_raw.allocate(T * S * sizeof(float));
   }
   allocate_exact(L, T);
+  L->fc1_exact.allocate_round_trip(T, L->fc1);
+  L->up_exact.allocate_round_trip(T, L->shared_up_dense);
+  L->exact.allocate_round_trip(T, L->shared_down_dense);
   if (L->ep_world == 1) {
     L->parts.allocate(T * (K + 1) * static_cast<size_t>(std::max(H, Lr)) * sizeof(float));
   }
@@ -1412,8 +1416,8 @@ void run_linear(nmoe_layer* L, const DenseLinear& linear, ExactScratch& scratch,
   const float* source = in_rows;
   if (linear.fp8) {
     NMOE_CUDA(launch_fp8_round_trip(in_rows, static_cast<size_t>(rows) * linear.in,
-                                    linear.input_scale, L->fp8_tmp.as<float>(), stream));
-    source = L->fp8_tmp.as<float>();
+                                    linear.input_scale, scratch.round_trip.as<float>(), stream));
+    source = scratch.round_trip.as<float>();
   }
   NMOE_CUDA(launch_router_logits(source, linear.weight.as<float>(), nullptr, rows, linear.out,
                                  linear.in, out_rows, L->num_sms, stream));

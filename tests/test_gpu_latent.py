@@ -86,6 +86,30 @@ def test_chains_beside_each_other_give_the_same_bits(package, synthetic, monkeyp
     alone.close()
 
 
+def test_long_fp8_contractions_beside_each_other(package, synthetic, monkeypatch):
+    # rows too long for the correctly rounded linears: fc1_latent and shared_up each multiply with the round
+    # trip of their own input scale, on two streams at once
+    cfg = synthetic.baseline_config(max_tokens=65, experts=32, hidden=16448, routed=64, shared=64,
+                                    latent=64, top_k=2)
+    data = synthetic.make_layer(cfg, seed=62, device="cuda", norm_weight_uniform=True,
+                                latent_family="fp8", shared_up_family="fp8")
+    data.bindings.fc1_latent.input_scale = 1.0
+    data.bindings.shared_up_linear.input_scale = 1.0 / 64.0
+    beside = package.ExpertLayerSlice.create(cfg, data.bindings)
+    monkeypatch.setenv("NMOE_NO_SHARED_FORK", "1")
+    alone = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert beside is not None and alone is not None, package.ExpertLayerSlice.create_error
+    for tokens in (2, 65):
+        x = synthetic.make_tokens(tokens, cfg.hidden_size, seed=tokens, device="cuda")
+        want = _run(alone, x)
+        for _ in range(20):
+            assert torch.equal(_run(beside, x), want)
+        rep = helpers.compare_layer_with_oracle(beside, data, x, want)
+        assert rep.ok(), rep.summary()
+    beside.close()
+    alone.close()
+
+
 # FP8 shared_up: the hidden rows' codes are decided from whole-number sums of the operands' codes, in the
 # unfused path they follow from the correctly rounded rows.  Tiles of 16 to 80 token rows, an unfinished
 # tile of weight rows, more rows than the workspace holds at once; values beyond 6 * 448, whose rows get a
