@@ -9,6 +9,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "front_words.h"
+
 namespace nmoe {
 
 // Where a kernel is launched.  `chained`: what precedes it on the stream is a kernel of this library,
@@ -449,11 +451,9 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               int32_t* pair_row /* nullable */, int dest_stride, int32_t* error,
                               int num_sms, LaunchStream stream);
 // --- front end of a handful of tokens (csrc/front.cu) ---------------------------
-constexpr int kFrontMaxRows = 8;
 constexpr int kFrontMaxCols = 4096;
 constexpr int kFrontMaxExperts = 512;
 // A linear of the one token's normalised row whose FP32 row is then quantised with its tensor scale.
-constexpr int kFrontLinears = 2;
 constexpr int kFrontLinearMaxN = 6144;
 struct FrontLinear {
   int N = 0, kind = 0;
@@ -508,8 +508,7 @@ struct FrontArgs {
   int32_t* error = nullptr;
 };
 constexpr size_t front_scratch_bytes() {
-  return (kFrontMaxRows + 2 + 2 * kFrontLinears) * sizeof(int32_t) +
-         2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
+  return sizeof(FrontWords) + 2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
 }
 cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream);
 
