@@ -71,13 +71,14 @@ struct NormShared {
 // By all kWarpsPerBlock * 32 threads.  Thread c owns the 8-element chunks c, c + 256, ...: it loads them
 // at once, and hands the values over through shared memory for the sum of squares, in which thread t
 // adds up columns t, t + 256, ... in order.  `inv_rms_known()` runs once inv_rms_out[row] is written
-// (by thread 0).
+// (by thread 0); it may hand that on to blocks that are running, so the pointer is not __restrict__: the
+// store must not move behind what the callback does.
 template <bool BF16, int CHUNKS, typename Known>
 __device__ __forceinline__ void norm_quant_by_block(
     const void* in, int row, int cols, const float* __restrict__ norm_weight, float eps,
     float* __restrict__ normalized, uint8_t* __restrict__ packed, uint8_t* __restrict__ sf_row_major,
     uint8_t* __restrict__ sf_tiled, int k_tiles, float* __restrict__ tensor_scale,
-    float* __restrict__ inv_rms_out, bool word_scales, NormShared<CHUNKS>& shared,
+    float* inv_rms_out, bool word_scales, NormShared<CHUNKS>& shared,
     Known&& inv_rms_known) {
   constexpr int kThreads = kWarpsPerBlock * 32;
   auto& row_values = shared.row_values;
