@@ -614,6 +614,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
         *args.ticket = 0;
         *args.finished = 0;
         if (args.error_host != nullptr) {
+          __threadfence();  // the count of the other CTAs comes before their error
           const int code = *static_cast<volatile int32_t*>(args.error);
           if (code != kDevOk) {
             *static_cast<volatile int32_t*>(args.error_host) = code;

@@ -576,7 +576,7 @@ struct ErrorSlot {
   ~ErrorSlot() {
     if (host != nullptr) cudaFreeHost(host);
   }
-  // `published`: what was launched last has left its word with the host, if there is one.
+  // `published`: what ran last has left its word with the host, if there is one.
   nmoe_status sync(cudaStream_t stream, bool published = false) {
     if (published) {
       NMOE_CUDA(cudaStreamSynchronize(stream));
@@ -815,8 +815,19 @@ struct nmoe_ffn {
   ErrorSlot error;
   int last_rows = 0;
   bool status_published = false;  // the last launch leaves its error word with the host
+  bool pair_captured = false;     // a launch that does not is in a graph and may run at any time
   std::string last_error;
 };
+
+// Whether what is launched on `stream` goes into a graph.
+static bool is_captured(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) {
+    return status != cudaStreamCaptureStatusNone;
+  }
+  cudaGetLastError();  // (the legacy stream, beside a capture on another one)
+  return false;
+}
 
 extern "C" {
 
@@ -913,6 +924,7 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
       run_expert_gemms(ffn->up, ffn->down, tile_class, ffn->a_op, ffn->a_ts.as<float>(), schedule,
                        ffn->h_packed.as<uint8_t>(), ffn->h_sf.as<uint8_t>(), ffn->h_op, out, error,
                        ffn->num_sms, stream);
+      ffn->pair_captured = ffn->pair_captured || is_captured(stream);
     }
     ffn->last_rows = static_cast<int>(rows);
     ffn->status_published = tile_class == kClassStream;
@@ -926,7 +938,9 @@ nmoe_status nmoe_ffn_run(nmoe_ffn* ffn, void* stream_ptr, const void* input,
 nmoe_status nmoe_ffn_sync_status(nmoe_ffn* ffn, void* stream_ptr) {
   if (ffn == nullptr) return NMOE_ERR_INVALID_ARGUMENT;
   try {
-    return ffn->error.sync(static_cast<cudaStream_t>(stream_ptr), ffn->status_published);
+    // (the host knows what it launched last, not which graph it replayed since)
+    return ffn->error.sync(static_cast<cudaStream_t>(stream_ptr),
+                           ffn->status_published && !ffn->pair_captured);
   } catch (const Failure& failure) {
     ffn->last_error = failure.message;
     return failure.status;

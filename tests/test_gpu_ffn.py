@@ -112,3 +112,38 @@ def test_ffn_status_is_that_of_the_runs_since_the_last_one(package, synthetic, v
             assert lib.nmoe_ffn_sync_status(f._handle, stream) == expected
         assert lib.nmoe_ffn_sync_status(f._handle, stream) == package.NMOE_OK
         f.close()
+
+
+@pytest.mark.parametrize("captured", [1, 3])
+def test_ffn_status_is_that_of_a_replayed_run(package, synthetic, captured):
+    # what ran last is a graph of the caller's, not the run that was launched last
+    up, down = synthetic.make_ffn_weights(448, 192, seed=5, device="cuda")
+    up.tensor_scale *= 400.0
+    ffn = package.ExpertFfn(up, down, max_rows=128)
+    ordinary = synthetic.make_tokens(40, 448, seed=6, device="cuda") * 0.01
+    x = ordinary.clone()
+    out = torch.empty(40, 448, device="cuda")
+    lib, stream = package.load_library(), torch.cuda.Stream()
+
+    def launch(rows, variant):
+        return lib.nmoe_ffn_run(ffn._handle, stream.cuda_stream, rows.data_ptr(),
+                                package._dtype_code(rows), 40, out.data_ptr(), variant)
+
+    def status():
+        return lib.nmoe_ffn_sync_status(ffn._handle, stream.cuda_stream)
+
+    torch.cuda.synchronize()
+    assert launch(x, captured) == 0 and status() == 0  # (its kernels are loaded)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        assert launch(x, captured) == 0
+    x.mul_(100.0)  # beyond 6 * 448 from here on
+    torch.cuda.synchronize()
+    for variant in (3, 1, 3):
+        assert launch(ordinary, variant) == 0
+        with torch.cuda.stream(stream):
+            graph.replay()
+        assert status() == 5  # NMOE_ERR_ACTIVATION_RANGE
+        assert launch(ordinary, variant) == 0
+        assert status() == 0
+    ffn.close()
