@@ -1141,18 +1141,23 @@ bool gate_needs_slices(const nmoe_layer* L, size_t T) {
          !exact_prefers_gemv(most_rows, L->cfg.n_routed_experts, L->cfg.hidden_size, L->num_sms);
 }
 
-// Slices of the gate and the workspace of the exact linears, for calls of up to `T` rows.
+// Slices of the gate and the workspace of the exact linears on the caller's stream, for calls of up to `T`
+// rows.
 void allocate_exact(nmoe_layer* L, size_t T) {
   std::vector<std::pair<int, int>> linears;
   if (gate_needs_slices(L, T)) {
     L->gate_exact.slice(nullptr);
     linears.emplace_back(L->cfg.n_routed_experts, L->cfg.hidden_size);
   }
-  const int sms = device_sm_count();
   for (const DenseLinear* linear : {&L->fc2, &L->shared_down_dense}) {
     if (linear->present && linear->exact) linears.emplace_back(linear->out, linear->in);
   }
-  L->exact.allocate(T, linears, sms);
+  L->exact.allocate(T, linears, device_sm_count());
+}
+
+// ... and of those that may run beside it.
+void allocate_exact_beside(nmoe_layer* L, size_t T) {
+  const int sms = device_sm_count();
   if (L->fc1.present && L->fc1.exact) L->fc1_exact.allocate(T, {{L->fc1.out, L->fc1.in}}, sms);
   if (L->shared_up_dense.present && L->shared_up_dense.exact) {
     L->up_exact.allocate(T, {{L->shared_up_dense.out, L->shared_up_dense.in}}, sms);
@@ -1195,6 +1200,7 @@ void allocate_scratch(nmoe_layer* L, size_t T) {
     L->shared_raw.allocate(T * S * sizeof(float));
   }
   allocate_exact(L, T);
+  allocate_exact_beside(L, T);
   L->fc1_exact.allocate_round_trip(T, L->fc1);
   L->up_exact.allocate_round_trip(T, L->shared_up_dense);
   L->exact.allocate_round_trip(T, L->shared_down_dense);
@@ -2198,6 +2204,11 @@ nmoe_status nmoe_layer_reserve_sms(nmoe_layer* layer, int32_t reserved_sms) {
   } catch (const Failure& failure) {
     layer->num_sms = before;
     layer->last_error = failure.message;
+    try {  // the workspace it had, or none (every run is then refused): no run finds a freed buffer
+      allocate_exact(layer, tokens);
+    } catch (const Failure&) {
+      layer->cfg.max_tokens = 0;
+    }
     return failure.status;
   }
   return NMOE_OK;

@@ -74,6 +74,31 @@ def test_a_layer_keeps_its_scratch_when_it_cannot_grow(package, synthetic):
     layer.close()
 
 
+def test_a_layer_keeps_its_workspace_when_fewer_sms_need_a_larger_one(package, synthetic):
+    # with 18 SMs left the gate goes through the integer kernel, whose digits of 1024 rows of 11008 are
+    # 56 MB; fc2_latent uses the same workspace
+    cfg = synthetic.baseline_config(max_tokens=1024, experts=32, hidden=11008, routed=64, shared=64,
+                                    latent=64, top_k=2)
+    data = synthetic.make_layer(cfg, seed=20, device="cuda")
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    x = synthetic.make_tokens(200, 11008, seed=21, device="cuda")
+    out, again = (torch.empty((200, 11008), dtype=torch.float32, device="cuda") for _ in range(2))
+    assert layer.run(x, out), layer.last_error
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    with pytest.raises(package.NmoeError):
+        layer.reserve_sms(130)
+    del held
+    torch.cuda.empty_cache()
+    for reserved in (0, 130):
+        layer.reserve_sms(reserved)
+        assert layer.run(x, again), layer.last_error
+        assert torch.equal(again, out)
+    layer.close()
+
+
 def test_unfused_rows_follow_the_scratch(package, synthetic):
     # enabled, disabled, grown, enabled: the FP32 rows have to be the larger scratch's
     cfg = synthetic.baseline_config(max_tokens=16, experts=32, hidden=512, routed=256, shared=256)
