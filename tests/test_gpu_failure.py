@@ -75,7 +75,7 @@ def test_a_layer_keeps_its_scratch_when_it_cannot_grow(package, synthetic):
 
 
 def test_a_layer_keeps_its_workspace_when_fewer_sms_need_a_larger_one(package, synthetic):
-    # with 18 SMs left the gate goes through the integer kernel, whose digits of 1024 rows of 11008 are
+    # with 4 SMs left the gate goes through the integer kernel, whose digits of 1024 rows of 11008 are
     # 56 MB; fc2_latent uses the same workspace
     cfg = synthetic.baseline_config(max_tokens=1024, experts=32, hidden=11008, routed=64, shared=64,
                                     latent=64, top_k=2)
@@ -89,10 +89,10 @@ def test_a_layer_keeps_its_workspace_when_fewer_sms_need_a_larger_one(package, s
     torch.cuda.empty_cache()
     held = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
     with pytest.raises(package.NmoeError):
-        layer.reserve_sms(130)
+        layer.reserve_sms(144)
     del held
     torch.cuda.empty_cache()
-    for reserved in (0, 130):
+    for reserved in (0, 144):
         layer.reserve_sms(reserved)
         assert layer.run(x, again), layer.last_error
         assert torch.equal(again, out)
