@@ -665,8 +665,8 @@ struct ExactOperand {
   }
 };
 
-// A dense or scaled-FP8 linear resident in HBM in the format it came in, with its fixed-point
-// slices; the values that count are FP32 [out][in], what the reference's UploadedLinearOp /
+// A dense or scaled-FP8 linear resident in HBM in the format it came in, with its fixed-point slices
+// (those of one with codes as soon as the unfused path is on, which alone reads them); the values that count are FP32 [out][in], what the reference's UploadedLinearOp /
 // ScaledFp8LinearOp multiply with (linear_op.cpp:274-303, scaled_fp8_linear.cu:121-139).
 // Contractions too long for the slices keep the FP32 matrix itself.
 struct DenseLinear {
@@ -679,6 +679,10 @@ struct DenseLinear {
   ExactOperand operand;
   CodedWeight coded;  // FP8 weights whose rows are only quantised again
   DeviceBuffer coded_slices, coded_norm;
+
+  void slice(cudaStream_t stream) {
+    if (present && exact) operand.slice(stream);
+  }
 
   void prepare_coded(cudaStream_t stream) {
     if (!fp8 || !exact || !coded_supported(out, in, operand.w.scale) ||
@@ -743,7 +747,6 @@ struct DenseLinear {
     } else {
       throw Failure{NMOE_ERR_INVALID_ARGUMENT, n + ": unknown linear family"};
     }
-    if (exact) operand.slice(stream);
     present = true;
   }
 };
@@ -1160,6 +1163,7 @@ void allocate_exact_beside(nmoe_layer* L, size_t T) {
   const int sms = device_sm_count();
   if (L->fc1.present && L->fc1.exact) L->fc1_exact.allocate(T, {{L->fc1.out, L->fc1.in}}, sms);
   if (L->shared_up_dense.present && L->shared_up_dense.exact) {
+    if (L->shared_up_dense.coded.slices == nullptr || L->unfused) L->shared_up_dense.slice(nullptr);
     L->up_exact.allocate(T, {{L->shared_up_dense.out, L->shared_up_dense.in}}, sms);
   }
 }
@@ -1376,6 +1380,8 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   if (L->latent_mode) {
     L->fc1.upload(w.fc1_latent, Lr, H, "fc1_latent", stream);
     L->fc2.upload(w.fc2_latent, H, Lr, "fc2_latent", stream);
+    L->fc1.slice(stream);
+    L->fc2.slice(stream);
   }
   if (w.shared_up_linear.family != NMOE_LINEAR_ABSENT) {
     L->shared_up_dense.upload(w.shared_up_linear, S, H, "shared up_proj", stream);
@@ -1387,6 +1393,7 @@ void layer_create_impl(nmoe_layer* L, const nmoe_config& c, const nmoe_weights& 
   }
   if (w.shared_down_linear.family != NMOE_LINEAR_ABSENT) {
     L->shared_down_dense.upload(w.shared_down_linear, H, S, "shared down_proj", stream);
+    L->shared_down_dense.slice(stream);
   } else {
     L->shared_down.upload(&w.shared_down, 1, H, S, "shared down_proj", stream);
   }

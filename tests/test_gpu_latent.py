@@ -147,6 +147,21 @@ def test_fp8_shared_up_codes_are_those_of_the_rounded_rows(package, synthetic, w
     layer.close()
 
 
+def test_digits_that_only_the_unfused_path_reads_come_with_it(package, synthetic):
+    cfg = synthetic.baseline_config(max_tokens=16, experts=32, hidden=4096, routed=64, shared=4096,
+                                    latent=64)
+    data = synthetic.make_layer(cfg, seed=18, device="cuda", latent_family="fp8", shared_up_family="fp8")
+    layer = package.ExpertLayerSlice.create(cfg, data.bindings)
+    assert layer is not None, package.ExpertLayerSlice.create_error
+    x = synthetic.make_tokens(16, 4096, seed=19, device="cuda")
+    fused = _run(layer, x)
+    free = torch.cuda.mem_get_info()[0]
+    layer.set_unfused_activation(True)
+    assert free - torch.cuda.mem_get_info()[0] >= 5 * 4096 * 4096
+    assert torch.equal(_run(layer, x), fused)
+    layer.close()
+
+
 def test_unfused_activation_path_and_trace_fields(package, synthetic, oracle):
     cfg = synthetic.baseline_config(max_tokens=256, experts=32, hidden=512, routed=256, shared=512)
     data = synthetic.make_layer(cfg, seed=21, device="cuda", norm_weight_uniform=True)
