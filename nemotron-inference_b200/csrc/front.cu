@@ -326,8 +326,7 @@ __device__ __forceinline__ void linear_outputs(const FrontArgs& args, const Scra
     for (int i = 0; i < kLinearOutputs; ++i) raw[i][0] = weight_row(i)[0];
   }
   // The weights of a block that starts when this one is through: HBM is idle until the row is known.
-  constexpr int kAhead = 444;
-  const int ahead = n0 + kAhead * kLinearOutputs;
+  const int ahead = n0 + args.resident_blocks * kLinearOutputs;
   if (ahead < linear.N) {
     const size_t bytes = min(kLinearOutputs, linear.N - ahead) * row_bytes;
     const uint8_t* from = weight + ahead * row_bytes;
@@ -406,7 +405,7 @@ __host__ __device__ constexpr int linear_blocks(int N) {
 }
 
 template <int ROWS, int PER_LANE, bool LINEARS>
-__global__ void __launch_bounds__(kThreads, LINEARS ? 3 : ROWS == 1 ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, LINEARS ? kFrontLinearBlocksPerSm : ROWS == 1 ? 4 : 2)
 front_kernel(const __grid_constant__ FrontArgs args) {
   // columns that a block quantises: the rows', or those of a linear's outputs
   constexpr int kQuantChunks = LINEARS ? kFrontLinearMaxN / (kThreads * 8) : kChunks;

@@ -455,6 +455,7 @@ constexpr int kFrontMaxCols = 4096;
 constexpr int kFrontMaxExperts = 512;
 // A linear of the one token's normalised row whose FP32 row is then quantised with its tensor scale.
 constexpr int kFrontLinearMaxN = 6144;
+constexpr int kFrontLinearBlocksPerSm = 3;  // of a launch with linears
 struct FrontLinear {
   int N = 0, kind = 0;
   const void* weight = nullptr;
@@ -504,6 +505,7 @@ struct FrontArgs {
   int dest_stride = 0;
   FrontLinear linear[kFrontLinears];
   int linears = 0;
+  int resident_blocks = 0;  // of a launch with linears, on all SMs together
   void* scratch = nullptr;  // front_scratch_bytes(), zero before the first launch
   int32_t* error = nullptr;
 };

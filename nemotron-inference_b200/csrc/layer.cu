@@ -1887,6 +1887,7 @@ void route_few(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype
       up.tensor_scale = L->sh_ts.as<float>();
     }
   }
+  args.resident_blocks = kFrontLinearBlocksPerSm * L->num_sms;
   args.scratch = L->front_scratch.as<void>();
   args.error = L->error.device.as<int32_t>();
   NMOE_CUDA(launch_front(args, stream));
