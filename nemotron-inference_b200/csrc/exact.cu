@@ -220,10 +220,11 @@ void launch_slices(const void* in, int rows, int K, float scale, int tile_rows, 
 // MMA of up to 256 columns multiplies digit i with several token digits and adds each product to
 // the level it belongs to; A is read once for all of them.  A CTA takes one tile, or a share of
 // its K range, and stores the levels put together as doubles.
-// Bound by the MMAs (the checkpoint's shared_up, 5376 x 4096, 1000 rows, under ncu: a stage takes 1740
-// cycles, 1420 of them on the tensor pipe, and its 672 tiles are 4.54 waves of 148 SMs; shared memory
-// is at 32 % of its read and 13 % of its write rate).  With the two kernels around it 13,800 -> 370 us;
-// 40 rows 381 -> 44 us.
+// Bound by the MMAs (five digits of a weight of the checkpoint's shared_up's shape, 5376 x 4096, 1000 rows,
+// under ncu: a stage takes 1740 cycles, 1420 of them on the tensor pipe, and its 672 tiles are 4.54 waves of
+// 148 SMs; shared memory is at 32 % of its read and 13 % of its write rate).  With the two kernels around
+// it 13,800 -> 370 us; 40 rows 381 -> 44 us.  (shared_up itself takes three digits where its rows are only
+// quantised again, further down.)
 // ---------------------------------------------------------------------------
 constexpr int kExactThreads = 6 * 32;
 // A product of matrices of SLICES digits: five of rows in fixed point (above), or the three of E4M3

@@ -19,9 +19,9 @@ def small_layer(package, synthetic):
     layer.close()
 
 
-# 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; CTA pairs from 100 rows per expert (534 tokens); the shared expert in
-# the routed experts' launch up to 640; a block per row in the quantiser up to 888, per token in the
-# exact selection up to 2048
+# 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; CTA pairs from 100
+# rows per expert (534 tokens), and with them the shared expert beside the router; a block per row in the
+# quantiser up to 888, per token in the exact selection up to 2048
 @pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 888, 889, 1184, 1185,
                                     1280, 1281, 2048, 2049])
 def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
@@ -63,10 +63,11 @@ def test_pairs_share_rows_of_every_count(package, synthetic):
     layer.close()
 
 
-# up to eight tokens, 4096 columns and 256 experts have one launch in front of the experts; the stages
+# up to eight tokens, 4096 columns and 512 experts have one launch in front of the experts; the stages
 # are timed through the four launches it stands for
 @pytest.mark.parametrize("experts,hidden,top_k,groups", [(32, 448, 6, 1), (256, 1024, 32, 4),
-                                                         (96, 4096, 1, 1), (128, 4160, 8, 8)])
+                                                         (96, 4096, 1, 1), (128, 4160, 8, 8),
+                                                         (288, 448, 8, 1), (512, 512, 22, 1)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_front_end_of_a_few_tokens(package, synthetic, experts, hidden, top_k, groups, dtype):
     cfg = synthetic.baseline_config(max_tokens=16, experts=experts, hidden=hidden, routed=64,
@@ -78,13 +79,14 @@ def test_front_end_of_a_few_tokens(package, synthetic, experts, hidden, top_k, g
     assert layer is not None, package.ExpertLayerSlice.create_error
     for tokens in (1, 2, 4, 5, 8, 9):
         x = synthetic.make_tokens(tokens, hidden, seed=tokens, device="cuda").to(dtype)
-        out, launches = (torch.empty(x.shape, device="cuda") for _ in range(2))
-        layer.enable_stage_timing(True)
-        assert layer.run(x, launches), layer.last_error
-        layer.enable_stage_timing(False)
-        for _ in range(2):
-            assert layer.run(x, out), layer.last_error
-            assert torch.equal(out, launches)
+        for out_dtype in (torch.bfloat16, torch.float32):
+            out, launches = (torch.empty(x.shape, dtype=out_dtype, device="cuda") for _ in range(2))
+            layer.enable_stage_timing(True)
+            assert layer.run(x, launches), layer.last_error
+            layer.enable_stage_timing(False)
+            for _ in range(2):
+                assert layer.run(x, out), layer.last_error
+                assert torch.equal(out, launches)
         rep = helpers.compare_layer_with_oracle(layer, data, x, out)
         assert rep.ok(), rep.summary()
     layer.close()
