@@ -54,8 +54,9 @@ class DeviceBuffer {
   ~DeviceBuffer() { reset(); }
   void allocate(size_t bytes, bool zero = false) {
     reset();
-    bytes_ = bytes == 0 ? 16 : bytes;
-    NMOE_CUDA(cudaMalloc(&ptr_, bytes_));
+    if (bytes == 0) bytes = 16;
+    NMOE_CUDA(cudaMalloc(&ptr_, bytes));
+    bytes_ = bytes;
     if (zero) NMOE_CUDA(cudaMemset(ptr_, 0, bytes_));
   }
   void reset() {
@@ -756,23 +757,30 @@ struct DenseLinear {
 // sums.  Of scaled-FP8 ones with contractions too long for that: the rows after their round trip.
 struct ExactScratch {
   int max_rows = 0;
+  size_t most_n = 0, most_k = 0;  // of the exact linears it has room for
   DeviceBuffer slices, info, partial;
   DeviceBuffer round_trip;  // [tokens][in] FP32
   // `shapes`: (N, K) of every linear that will run
   void allocate(size_t tokens, const std::vector<std::pair<int, int>>& shapes, int num_sms) {
     max_rows = static_cast<int>(std::min<size_t>(tokens, 1024));
-    size_t most_k = 0, most_n = 0;
+    most_n = most_k = 0;
+    size_t n = 0, k = 0;
     for (const auto& shape : shapes) {
-      most_n = std::max<size_t>(most_n, shape.first);
-      most_k = std::max<size_t>(most_k, shape.second);
+      n = std::max<size_t>(n, shape.first);
+      k = std::max<size_t>(k, shape.second);
     }
     if (shapes.empty()) return;
     // (rows come in tiles of up to 64)
-    slices.allocate(slice_bytes(max_rows, static_cast<int>(most_k), 64));
+    slices.allocate(slice_bytes(max_rows, static_cast<int>(k), 64));
     info.allocate(max_rows * sizeof(SliceRow));
     // a split contraction has at most one tile of 128 x 80 sums per SM
-    partial.allocate(std::max(max_rows * most_n, static_cast<size_t>(num_sms) * 128 * 80) *
+    partial.allocate(std::max(max_rows * n, static_cast<size_t>(num_sms) * 128 * 80) *
                      sizeof(double));
+    most_n = n;
+    most_k = k;
+  }
+  bool holds(const ExactWeight& w) const {
+    return static_cast<size_t>(w.N) <= most_n && static_cast<size_t>(w.K) <= most_k;
   }
   void allocate_round_trip(size_t tokens, const DenseLinear& linear) {
     if (!linear.fp8 || linear.exact) return;
@@ -787,7 +795,8 @@ void run_exact(const ExactWeight& w, ExactScratch& scratch, const float* in, flo
     NMOE_CUDA(launch_exact_gemv(w, in, fp8_scale, rows, offset, relu2, out, num_sms, stream));
     return;
   }
-  NMOE_REQUIRE(w.slices != nullptr, "an exact linear without its slices");
+  NMOE_REQUIRE(w.slices != nullptr && scratch.holds(w),
+               "an exact linear without its slices or its workspace");
   for (int first = 0; first < rows; first += scratch.max_rows) {
     const int count = std::min(rows - first, scratch.max_rows);
     const float* from = in + static_cast<size_t>(first) * w.K;
@@ -2204,7 +2213,10 @@ nmoe_status nmoe_layer_reserve_sms(nmoe_layer* layer, int32_t reserved_sms) {
   const int before = layer->num_sms;
   layer->num_sms = all - reserved_sms;
   const size_t tokens = static_cast<size_t>(layer->cfg.max_tokens);
-  if (layer->gate_exact.w.slices != nullptr || !gate_needs_slices(layer, tokens)) return NMOE_OK;
+  const ExactWeight& gate = layer->gate_exact.w;
+  if ((gate.slices != nullptr && layer->exact.holds(gate)) || !gate_needs_slices(layer, tokens)) {
+    return NMOE_OK;
+  }
   try {  // with this few SMs the gate goes through the integer kernel
     NMOE_CUDA(cudaDeviceSynchronize());
     allocate_exact(layer, tokens);

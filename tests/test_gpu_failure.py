@@ -96,6 +96,12 @@ def test_a_layer_keeps_its_workspace_when_fewer_sms_need_a_larger_one(package, s
         layer.reserve_sms(reserved)
         assert layer.run(x, again), layer.last_error
         assert torch.equal(again, out)
+    # scratch made for all SMs has no room for the gate, although its digits are there
+    layer.reserve_sms(0)
+    layer.reserve_tokens(1025)
+    layer.reserve_sms(144)
+    assert layer.run(x, again), layer.last_error
+    assert torch.equal(again, out)
     layer.close()
 
 
