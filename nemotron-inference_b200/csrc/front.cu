@@ -10,6 +10,7 @@
 //
 // Whole pass of the benchmark layer, four launches against this: 1 token 36.6 us and 31.6, 4 tokens 46.5
 // and 42.2, 7 tokens 57.3 and 54.7, 8 tokens 58.2 and 57.1 (the experts read their weights for the rest).
+// It pays for one token, and for more while all blocks of the gate are resident at once (front_pays).
 //
 // One token of a latent layer has its linears here too, eight outputs to a block: they were two FP64 gemvs
 // and two quantisers on the same chain.  With what follows the experts in one launch as well
@@ -405,7 +406,9 @@ __host__ __device__ constexpr int linear_blocks(int N) {
 }
 
 template <int ROWS, int PER_LANE, bool LINEARS>
-__global__ void __launch_bounds__(kThreads, LINEARS ? kFrontLinearBlocksPerSm : ROWS == 1 ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, LINEARS     ? kFrontLinearBlocksPerSm
+                                            : ROWS == 1 ? 4
+                                                        : kFrontBlocksPerSm)
 front_kernel(const __grid_constant__ FrontArgs args) {
   // columns that a block quantises: the rows', or those of a linear's outputs
   constexpr int kQuantChunks = LINEARS ? kFrontLinearMaxN / (kThreads * 8) : kChunks;
@@ -484,8 +487,22 @@ front_kernel(const __grid_constant__ FrontArgs args) {
 
 }  // namespace
 
+// One token: four launches against one, 128 experts of 2688 27.4 us and 26.8, 256 of 4096 33.0 and 29.3, 512
+// of 4096 43.5 and 39.6 (small experts, whole pass).  Several: a block of the gate is 124 registers a thread
+// and two fit an SM; with more of them than that a second wave computes what the first has long been waited
+// for.  128 experts, 4 tokens (128 blocks) 33.2 and 31.4, 8 tokens (256) 37.2 and 36.4; 256 of 2048, 4 tokens
+// (256) 33.1 and 33.4, 8 tokens (512) 37.2 and 41.6; 160 of 2048, 8 tokens (320) 35.1 and 36.9; 384 of 2048, 2
+// tokens (384) 31.0 and 33.9, 8 tokens (768) 39.3 and 46.4; 512 of 4096, 8 tokens 98.9 and 108.6.
+bool front_pays(int rows, int experts, int num_sms) {
+  if (rows == 1) return experts <= kFrontMaxExperts;
+  if (rows > kFrontMaxRows || experts > kFrontMaxExpertsOfRows) return false;
+  const int blocks = (rows + kFrontRowsPerBlock - 1) / kFrontRowsPerBlock * experts;
+  return blocks <= kFrontBlocksPerSm * num_sms;
+}
+
 cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream) {
-  if (args.rows < 1 || args.rows > kFrontMaxRows || args.cols > kFrontMaxCols || args.cols % 16 != 0 ||
+  if ((args.rows > 1 && args.experts > kFrontMaxExpertsOfRows) ||
+      args.rows < 1 || args.rows > kFrontMaxRows || args.cols > kFrontMaxCols || args.cols % 16 != 0 ||
       args.experts < 1 || args.experts > kFrontMaxExperts || args.top_k > 32 ||
       args.linears > kFrontLinears || (args.linears > 0 && args.rows != 1)) {
     return cudaErrorInvalidValue;
@@ -504,7 +521,11 @@ cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream) {
     constexpr int kPerLane = decltype(per_lane)::value;
     constexpr bool kLinears = decltype(linears)::value;
     if constexpr (!kLinears) {
-      if (args.rows > 1) return run(front_kernel<4, kPerLane, false>, 4);
+      if constexpr (kPerLane * 32 <= kFrontMaxExpertsOfRows) {
+        if (args.rows > 1) {
+          return run(front_kernel<kFrontRowsPerBlock, kPerLane, false>, kFrontRowsPerBlock);
+        }
+      }
     }
     run(front_kernel<1, kPerLane, kLinears>, 1);
   };

@@ -452,7 +452,10 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               int num_sms, LaunchStream stream);
 // --- front end of a handful of tokens (csrc/front.cu) ---------------------------
 constexpr int kFrontMaxCols = 4096;
-constexpr int kFrontMaxExperts = 512;
+constexpr int kFrontMaxExperts = 512;     // of one token
+constexpr int kFrontMaxExpertsOfRows = 256;  // of several
+constexpr int kFrontRowsPerBlock = 4;        // of several, for which a block forms an expert's logits
+constexpr int kFrontBlocksPerSm = 2;         // of a launch over several
 // A linear of the one token's normalised row whose FP32 row is then quantised with its tensor scale.
 constexpr int kFrontLinearMaxN = 6144;
 constexpr int kFrontLinearBlocksPerSm = 3;  // of a launch with linears
@@ -513,6 +516,8 @@ constexpr size_t front_scratch_bytes() {
   return sizeof(FrontWords) + 2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
 }
 cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream);
+// Whether one launch is the faster front end of `rows` tokens.
+bool front_pays(int rows, int experts, int num_sms);
 
 // --- expert-parallel dispatch / return (csrc/ep.cu) ---------------------------
 int dispatch_record_bytes(int cols);

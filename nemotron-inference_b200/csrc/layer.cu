@@ -1905,8 +1905,8 @@ void route_few(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype
 
 // Whether csrc/front.cu takes a batch (with what it cannot quantise left out).
 bool front_takes(const nmoe_layer* L, int tokens) {
-  if (tokens > kFrontMaxRows || L->cfg.hidden_size > kFrontMaxCols ||
-      L->cfg.n_routed_experts > kFrontMaxExperts || !L->has_gate_exact) {
+  if (!front_pays(tokens, L->cfg.n_routed_experts, L->num_sms) ||
+      L->cfg.hidden_size > kFrontMaxCols || !L->has_gate_exact) {
     return false;
   }
   if (!L->latent_mode) return !L->shared_up_dense.present && !L->shared_down_dense.present;

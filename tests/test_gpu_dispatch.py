@@ -63,8 +63,8 @@ def test_pairs_share_rows_of_every_count(package, synthetic):
     layer.close()
 
 
-# up to eight tokens, 4096 columns and 512 experts have one launch in front of the experts; the stages
-# are timed through the four launches it stands for
+# up to eight tokens, 4096 columns and two blocks of the gate per SM (one token: 512 experts; four: 256; eight:
+# 148) have one launch in front of the experts; the stages are timed through the four launches it stands for
 @pytest.mark.parametrize("experts,hidden,top_k,groups", [(32, 448, 6, 1), (256, 1024, 32, 4),
                                                          (96, 4096, 1, 1), (128, 4160, 8, 8),
                                                          (288, 448, 8, 1), (512, 512, 22, 1)])
