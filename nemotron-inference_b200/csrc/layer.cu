@@ -1923,10 +1923,35 @@ bool front_takes(const nmoe_layer* L, int tokens) {
 // pass of the checkpoint's layer, one stream against three: 1 token 77.8 us and 80.4 (the branches of
 // the graph cost more than they hide), 2 tokens 101 and 91, 8 tokens 189 and 171, 64 tokens 399 and 373,
 // 256 tokens 578 and 534, 1000 tokens 1075 and 962.
+//
+// Up to four tokens the linears are gemvs chained one to the other, and it depends on their size.  Long ones
+// gain (fc1_latent and shared_up of 4096 x 4096 together with 1024 x 4096, 21 million products, bf16, 3 tokens
+// 101 and 79, 4 tokens 95 and 84).  Short ones gain in a graph, where a branch costs least (1.3 million, FP32, 2
+// tokens 33.2 and 29.0; 5.2 million in FP8 45.7 and 41.2), and lose a little as launches (38.1 and 39.8; 53.8 and
+// 50.6, but 3 tokens 69.9 and 73.5).  Between, where a gemv by itself reads its weights with the whole GPU,
+// the branches cost more than they hide (5.2 million, bf16, 2 tokens 40.3 and 42.2, FP32 42.2 and 46.9).  From
+// five tokens on every shape gains in a graph (these 8 to 12 %), and none loses more than 2 % as launches.
 constexpr int kBesideMinTokens = 2;
+constexpr int kBesideAnyTokens = 5;
+constexpr size_t kBesideLongProducts = 16000000;
+constexpr size_t kBesideShortBytes = 6000000;
+bool linears_beside(const nmoe_layer* L, int tokens, bool in_graph) {
+  if (L->latent_stream == nullptr || tokens < kBesideMinTokens || tokens > L->fork_max_tokens) {
+    return false;
+  }
+  if (tokens >= kBesideAnyTokens) return true;
+  size_t products = 0, bytes = 0;
+  for (const DenseLinear* linear : {&L->fc1, &L->shared_up_dense}) {
+    if (!linear->present) continue;
+    products += static_cast<size_t>(linear->out) * linear->in;
+    bytes += linear->weight.bytes();
+  }
+  return products >= kBesideLongProducts || (in_graph && bytes <= kBesideShortBytes);
+}
 
+// `in_graph`: the launches are being recorded, by this library or by the caller.
 void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype in_dtype,
-                    int tokens, void* output, nmoe_dtype out_dtype) {
+                    int tokens, void* output, nmoe_dtype out_dtype, bool in_graph) {
   const nmoe_config& c = L->cfg;
   const int H = c.hidden_size, K = c.top_k, Lr = L->latent;
   const bool dense_shared = L->shared_up_dense.present || L->shared_down_dense.present;
@@ -1950,9 +1975,8 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   // tokens 2 to 4 us to lose.
   const LaunchStream chain(stream, !fork && !L->stage_timing && !L->unfused && !two_pass);
   const bool few = front_takes(L, tokens) && one_launch && !two_pass && !L->stage_timing;
-  const bool beside = !few && L->latent_stream != nullptr && one_launch && L->latent_mode &&
-                      !L->stage_timing && tokens >= kBesideMinTokens &&
-                      tokens <= L->fork_max_tokens;
+  const bool beside = !few && one_launch && L->latent_mode && !L->stage_timing &&
+                      linears_beside(L, tokens, in_graph);
   if (few) {
     route_few(L, stream, input, in_dtype, tokens);
   } else {
@@ -2059,8 +2083,8 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
 // A latent layer's graph has three branches, and recording it costs a new pair of buffers 420 us more
 // than launching the pass (40 tokens: 784 us and 366 from an idle device; 2 tokens 415 and 115), while
 // a replay saves 9 to 12 us over the launches (40 tokens 342 and 354 us a pass, 2 tokens 90 and 100).
-// So it is recorded when the launches have cost as much as that.  One token is one branch and,
-// like every layer without a latent form, is recorded at once.
+// So it is recorded when the launches have cost as much as that.  Where the linears stay on one stream, as
+// for one token, and in every layer without a latent form, a run is recorded at once.
 constexpr int kEagerRunsOfBranches = 32;
 
 // nmoe_layer_run: small batches replay a recorded CUDA graph of the same run.
@@ -2073,11 +2097,12 @@ void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input
                         can_query && capturing == cudaStreamCaptureStatusNone &&
                         stream != nullptr && stream != cudaStreamLegacy;
   if (!eligible) {
-    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
+    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype,
+                   can_query && capturing != cudaStreamCaptureStatusNone);
     return;
   }
   ++L->run_counter;
-  const bool branches = L->latent_stream != nullptr && tokens >= kBesideMinTokens;
+  const bool branches = linears_beside(L, tokens, true);
   nmoe_layer::RecordedRun* known = nullptr;
   for (nmoe_layer::RecordedRun& r : L->recorded) {
     if (r.input == input && r.output == output && r.tokens == tokens &&
@@ -2108,19 +2133,19 @@ void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input
   }
   if (branches && known->eager_runs < kEagerRunsOfBranches) {
     ++known->eager_runs;
-    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
+    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype, false);
     return;
   }
   // record: the launches below go into a graph instead of onto the stream
   if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     cudaGetLastError();      // this stream cannot be captured (e.g. the legacy default stream)
     L->graph_max_tokens = 0;  // stay eager from now on
-    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
+    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype, false);
     return;
   }
   cudaGraph_t graph = nullptr;
   try {
-    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
+    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype, true);
   } catch (...) {
     cudaStreamEndCapture(stream, &graph);
     if (graph != nullptr) cudaGraphDestroy(graph);
@@ -2134,7 +2159,7 @@ void run_recorded_or_eager(nmoe_layer* L, cudaStream_t stream, const void* input
   if (made != cudaSuccess) {
     cudaGetLastError();
     L->graph_max_tokens = 0;
-    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype);
+    layer_run_impl(L, stream, input, in_dtype, tokens, output, out_dtype, false);
     return;
   }
   known->parts_kind = L->last_parts_kind;

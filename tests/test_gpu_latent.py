@@ -61,7 +61,7 @@ def test_checkpoint_shape_latent_layer(package, synthetic):
 
 
 def test_chains_beside_each_other_give_the_same_bits(package, synthetic, monkeypatch):
-    # from two tokens gate, fc1_latent and shared_up run on three streams; passes follow each other
+    # gate, fc1_latent and shared_up run on three streams (two tokens: when recorded); passes follow each other
     # without a wait, launched one by one and (up to 256 tokens, from the 33rd of the same buffers) recorded
     cfg = synthetic.baseline_config(max_tokens=300, experts=64, hidden=512, routed=256, shared=768,
                                     latent=256)
