@@ -236,8 +236,8 @@ NMOE_API nmoe_status nmoe_layer_wait_flag(nmoe_layer* layer, void* stream, const
  * shared up GEMM, shared down GEMM, combine.  Every kernel runs alone then (no
  * recorded graph, no overlap).  Batches bound by reading the weights run several
  * expert projections as one launch: its time is that of the routed up GEMM, and
- * the stages it covers besides (routed down, and up to 640 tokens both shared
- * ones) show the gap between two events. */
+ * the stages it covers besides (routed down, and where the shared expert's tiles
+ * are few beside the SMs both shared ones) show the gap between two events. */
 #define NMOE_STAGE_COUNT 10
 NMOE_API nmoe_status nmoe_layer_enable_stage_timing(nmoe_layer* layer, int32_t enable);
 NMOE_API nmoe_status nmoe_layer_stage_times(nmoe_layer* layer, float* milliseconds,

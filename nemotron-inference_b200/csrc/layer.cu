@@ -1571,11 +1571,23 @@ void run_ffn(nmoe_layer* L, bool unfused, const WeightStack& up, const WeightSta
                 L->num_sms, stream);
 }
 
-// Up to this many tokens the shared expert's tiles join the routed experts' launch; with more its
-// GEMMs are long enough to be worth running beside the router (joined against beside: 700 tokens 178.4
-// us and 187.8, 1003 195.5 and 202.8, 1200 210 and 225, 1400 217 and 215.5, 1800 234 and 231; popular and
-// unpopular experts, 1200 tokens 190 and 204, 1800 246 and 241).
-constexpr int kSharedInLaunchTokens = 1280;
+// Whether the shared expert's tiles join the routed experts' launch; when they are many its GEMMs are long
+// enough to be worth running beside the router.  What counts is the K blocks its 128 x 128 tiles take of each
+// SM.  Whole pass, joined against beside (blocks per SM in brackets): benchmark layer 700 tokens 178.4 us and
+// 187.8, 1003 [34] 199.8 and 206.9, 1280 [43] 215.5 and 224.7, 1500 [51] 217.2 and 216.7, 1800 234 and 231,
+// popular and unpopular experts 246 and 241; shared expert of 1856 1500 tokens [27] 220 and 232, 2000 [36] 239
+// and 244, of 7424 800 [59] 202.8 and 204.4, 1280 [84] 232 and 226; 64 experts of 1024, hidden 4096, shared 8192
+// 450 tokens [55] 121 and 131, 1003 [110] 148 and 148, 1280 [138] 171 and 161; 256 experts of 768, hidden 2048,
+// shared 768 2000 tokens [9] 195 and 204.  With 74 SMs the line lies lower still (benchmark layer, 640 tokens
+// [43] 245 and 239).
+constexpr int kSharedInLaunchBlocksPerSm = 56;
+bool shared_joins(const nmoe_layer* L, int tokens) {
+  const int bn = stream_tile_info().bn;
+  const int H = L->cfg.hidden_size, S = L->cfg.shared_expert_intermediate_size;
+  long long blocks = static_cast<long long>((H + bn - 1) / bn) * k_blocks_of(S);
+  if (!L->shared_up_dense.present) blocks += static_cast<long long>((S + bn - 1) / bn) * k_blocks_of(H);
+  return (tokens + 127) / 128 * blocks <= static_cast<long long>(kSharedInLaunchBlocksPerSm) * L->num_sms;
+}
 
 // Routed rows per expert (on average) up to which csrc/expert_stream.cu takes them: with more, most
 // experts have a second row tile and their weights would be read twice.  Where the two meet depends
@@ -1966,7 +1978,7 @@ void layer_run_impl(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_
   // fork the shared expert onto a stream of its own.
   const bool one_launch = routed_tile_class(L, tokens * K) == kClassStream && !L->unfused &&
                           !L->shared_down_dense.present &&
-                          (L->latent_mode || tokens <= kSharedInLaunchTokens);
+                          (L->latent_mode || shared_joins(L, tokens));
   const bool fork = L->side_stream != nullptr && !L->stage_timing && !one_launch &&
                     tokens <= L->fork_max_tokens && !L->latent_mode && !dense_shared;
   const bool two_pass = L->fast_router && tokens >= L->fast_router_min_tokens;

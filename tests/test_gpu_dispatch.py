@@ -34,12 +34,14 @@ def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
 
 
 def test_shared_expert_on_both_sides_of_its_line(package, synthetic):
-    # in the routed experts' launch up to 1280 tokens, beside the router from there
-    cfg = synthetic.baseline_config(max_tokens=1281, experts=128, hidden=256, routed=64, shared=192)
+    # in the routed experts' launch up to 56 K blocks of its tiles per SM: 128 for every 128 tokens here, seven
+    # times that on 18 SMs
+    cfg = synthetic.baseline_config(max_tokens=897, experts=128, hidden=256, routed=64, shared=8192)
     data = synthetic.make_layer(cfg, seed=45, device="cuda", norm_weight_uniform=True)
     layer = package.ExpertLayerSlice.create(cfg, data.bindings)
     assert layer is not None, package.ExpertLayerSlice.create_error
-    for tokens in (1280, 1281):
+    layer.reserve_sms(torch.cuda.get_device_properties(0).multi_processor_count - 18)
+    for tokens in (896, 897):
         x = synthetic.make_tokens(tokens, 256, seed=tokens, device="cuda")
         out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
         assert layer.run(x, out), layer.last_error
