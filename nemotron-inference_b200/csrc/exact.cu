@@ -1354,10 +1354,14 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
         space.partial, splits, rows, w.N, w.K, in, fp8_scale, space.info, w.weight, w.scale, w.info,
         offset, relu2, out, mix);
   };
-  // four values a thread where that leaves none of a block's threads without one
+  // Four values a thread where four such blocks to an SM are left: then their loads count, before that a
+  // block's undecided values do, which it sums one after the other.  Whole latent pass, one value a thread
+  // against four: 4096 outputs, 40 rows 336 us and 341, 100 rows 389 and 393, 160 rows 416 and 416, 400 rows 552
+  // and 547, 1000 rows 824 and 792; 2048 outputs, 8 rows 53.9 and 62.2, 256 rows 113 and 115, 400 rows 154 and
+  // 153; 1024 outputs, 16 rows 47.5 and 55.8, 400 rows 94.3 and 96.0, 1000 rows 123.3 and 122.4.
   auto run_kind = [&](auto kind) {
     constexpr int kKind = decltype(kind)::value;
-    if (w.N >= 4 * kFinishThreads) {
+    if (static_cast<long long>(rows) * (w.N / (4 * kFinishThreads)) >= 4ll * num_sms) {
       run(exact_finish_kernel<kKind, 4>, 4);
     } else {
       run(exact_finish_kernel<kKind, 1>, 1);
