@@ -522,9 +522,17 @@ __device__ __forceinline__ double gate_scaled(uint32_t w) {
 // warps there are to fill the rest: 72 registers, seven blocks to an SM, instead of 84 took 16384 tokens
 // from 106 to 92 us, 1003 from 21 to 16.5; the short steps with a lane per candidate and without rounds
 // that look through eight slots 119 to 106 before that.
-// Up to kSelectWholeBlockRows tokens the block form is the faster one (us, block against warp; 128
-// experts of 2688, top-6: 1400 tokens 22.7 and 27.2, 2048 24.1 and 27.4, 4096 38.6 and 35.7).
-constexpr int kSelectWholeBlockRows = 2048;
+// Up to some number of tokens the block form is the faster one, the more the longer a token's sums and the
+// more its choices are.  us, block against warp, of the selection: 128 experts of 2688, top-6, 1280 tokens 22.6
+// and 28.7, 2048 24.6 and 26.6, 3072 34.6 and 34.6; of 4096 2048 tokens 28.5 and 34.6; of 1024 2048 tokens 20.6
+// and 22.9, 2560 24.6 and 23.3; 256 experts of 2688, top-8, 1536 tokens 32.5 and 36.6, 2048 34.6 and 34.6, 2560
+// 46.9 and 44.9; of 2048 2048 tokens 30.5 and 31.0.  Of a pass: 32 experts of 512 700 tokens 52.5 and 52.8, 1280
+// 59.8 and 58.2; 64 of 1024, top-4, 1024 tokens 53.8 and 55.8, 2048 74.6 and 71.7; 128 of 256 1024 tokens 50.3
+// and 51.3, 1280 54.7 and 52.6; 128 of 512 1280 tokens 60.5 and 60.9, 2048 66.1 and 64.5; 256 of 512 1280 tokens
+// 73.4 and 75.3, 1536 80.5 and 78.6.
+int select_whole_block_rows(int experts, int hidden) {
+  return std::min(2048, 600 + std::min(experts, 128) * hidden / 80);
+}
 template <bool IN_BF16, int WARPS, int BATCH, int kSelectPerLane>
 __global__ void __launch_bounds__(kSelectWarps * 32, BATCH <= 6 ? 7 : 5)
 router_select_exact_kernel(float* __restrict__ logits, int splits, const void* __restrict__ x,
@@ -852,7 +860,7 @@ cudaError_t launch_router_select_exact(float* logits, int splits, const void* x,
       top_k > 32 || top_k > experts || hidden % 8 != 0 || splits < 1) {
     return cudaErrorInvalidValue;
   }
-  const bool whole_block = rows <= kSelectWholeBlockRows;
+  const bool whole_block = rows <= select_whole_block_rows(experts, hidden);
   const int grid = whole_block ? rows : (rows + kSelectWarps - 1) / kSelectWarps;
   auto run = [&](auto kernel) {
     kernel<<<grid, kSelectWarps * 32, 0, stream>>>(

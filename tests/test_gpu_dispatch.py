@@ -21,9 +21,9 @@ def small_layer(package, synthetic):
 
 # 32 experts, top-6: few-row epilogue up to 16 rows a tile; two-pass router from 256; CTA pairs from 100
 # rows per expert (534 tokens), and with them the shared expert beside the router; a block per row in the
-# quantiser up to 888, per token in the exact selection up to 2048
-@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 888, 889, 1184, 1185,
-                                    1280, 1281, 2048, 2049])
+# quantiser up to 888, per token in the exact selection up to 804
+@pytest.mark.parametrize("tokens", [16, 17, 129, 255, 256, 394, 395, 533, 534, 640, 641, 804, 805, 888, 889,
+                                    1184, 1185, 1280, 1281, 2048, 2049])
 def test_layer_on_both_sides_of_each_line(small_layer, synthetic, tokens):
     layer, data = small_layer
     x = synthetic.make_tokens(tokens, 512, seed=300 + tokens, device="cuda")
