@@ -1354,14 +1354,17 @@ cudaError_t launch_exact_linear(const ExactWeight& w, const float* in, int rows,
         space.partial, splits, rows, w.N, w.K, in, fp8_scale, space.info, w.weight, w.scale, w.info,
         offset, relu2, out, mix);
   };
-  // Four values a thread where four such blocks to an SM are left: then their loads count, before that a
-  // block's undecided values do, which it sums one after the other.  Whole latent pass, one value a thread
+  // Four values a thread where enough such blocks are left to an SM (four, fewer with a short contraction):
+  // then their loads count, before that a block's undecided values do, which it sums one after the other, the
+  // more of them and the longer each the longer the contraction.  Whole latent pass, one value a thread
   // against four: 4096 outputs, 40 rows 336 us and 341, 100 rows 389 and 393, 160 rows 416 and 416, 400 rows 552
   // and 547, 1000 rows 824 and 792; 2048 outputs, 8 rows 53.9 and 62.2, 256 rows 113 and 115, 400 rows 154 and
-  // 153; 1024 outputs, 16 rows 47.5 and 55.8, 400 rows 94.3 and 96.0, 1000 rows 123.3 and 122.4.
+  // 153; 1024 outputs, 16 rows 47.5 and 55.8, 400 rows 94.3 and 96.0, 1000 rows 123.3 and 122.4.  Only fc2 that
+  // wide, K = 512, 2048 outputs: 100 rows 83.0 and 85.4, 256 rows 90.2 and 89.3.
   auto run_kind = [&](auto kind) {
     constexpr int kKind = decltype(kind)::value;
-    if (static_cast<long long>(rows) * (w.N / (4 * kFinishThreads)) >= 4ll * num_sms) {
+    const long long blocks = static_cast<long long>(rows) * (w.N / (4 * kFinishThreads));
+    if (blocks * 192 >= static_cast<long long>(num_sms) * std::min(w.K, 768)) {
       run(exact_finish_kernel<kKind, 4>, 4);
     } else {
       run(exact_finish_kernel<kKind, 1>, 1);

@@ -139,7 +139,8 @@ def test_longest_contraction_with_digits_of_one_sign(package, synthetic):
 
 @pytest.mark.parametrize("fc1,up", [("fp8", "bf16"), ("bf16", "fp32")])
 def test_roundings_four_to_a_thread_are_those_of_one(package, synthetic, fc1, up):
-    # four values a thread from four blocks of 1024 columns per SM; 1088 and 1152 columns end inside a block
+    # four values a thread from four blocks of 1024 columns per SM, from a third of one where the contraction
+    # is 64 long (fc2_latent); 1088 and 1152 columns end inside a block
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     cfg = synthetic.baseline_config(max_tokens=4 * sms, experts=32, hidden=1088, routed=64, shared=1152,
                                     latent=64, top_k=2)
@@ -150,10 +151,11 @@ def test_roundings_four_to_a_thread_are_those_of_one(package, synthetic, fc1, up
     x = synthetic.make_tokens(4 * sms, 1088, seed=92, device="cuda")
     for dtype in (torch.float32, torch.bfloat16):
         four = torch.empty(x.shape, dtype=dtype, device="cuda")
-        one = torch.empty_like(four[:-1])
         assert layer.run(x, four), layer.last_error
-        assert layer.run(x[:-1], one), layer.last_error
-        assert torch.equal(four[:-1], one)
+        for rows in (sms // 3, sms // 3 + 1, 4 * sms - 1):
+            one = torch.empty_like(four[:rows])
+            assert layer.run(x[:rows], one), layer.last_error
+            assert torch.equal(four[:rows], one)
     rep = helpers.compare_layer_with_oracle(layer, data, x[:-1], one, raw_run=False)
     assert rep.ok(), rep.summary()
     layer.close()
