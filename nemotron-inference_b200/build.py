@@ -8,7 +8,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnmoe_b200.so")
 SOURCES = ["gemm.cu", "expert_stream.cu", "quant.cu", "router.cu", "router_fast.cu", "plan.cu", "ep.cu", "layer.cu",
            "route_noalloc.cu", "dense.cu", "exact.cu", "front.cu"]
-HEADERS = ["common.cuh", "gemm_common.cuh", "kernels.h", "front_words.h", "quant_row.cuh", "topk.cuh", "weights.cuh",
+HEADERS = ["common.cuh", "gemm_common.cuh", "kernels.h", "quant_row.cuh", "topk.cuh", "weights.cuh",
            os.path.join("..", "..", "include", "nmoe.h")]
 NVCC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -153,6 +153,13 @@ __device__ __forceinline__ int load_acquire(const int32_t* p) {
   return v;
 }
 
+// What it held.  (With a fence behind it in the place of the acquire every short launch took 0.6 us more.)
+__device__ __forceinline__ int add_acquire(int32_t* p, int v) {
+  int before;
+  asm volatile("atom.acquire.gpu.global.add.s32 %0, [%1], %2;" : "=r"(before) : "l"(p), "r"(v) : "memory");
+  return before;
+}
+
 __device__ __forceinline__ void add_release(int32_t* p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -237,6 +244,11 @@ __device__ __forceinline__ void fetch_dense_weights(const StreamArgs& args, int 
   }
 }
 
+// TOKEN_ORDER: some phase's row tiles hold all tokens in token order (StreamPhase::used).  A kernel of its
+// own, since layers of many small experts have some fifty tiles an SM and looking it up in each of them
+// showed (384 experts of 512 at 400 tokens 166.5 us without and 168.4 with it, 256 of 768 at 64 tokens 99.8
+// and 101.1).
+template <bool TOKEN_ORDER>
 __global__ void __launch_bounds__(kThreads, 1)
 expert_stream_kernel(const __grid_constant__ StreamArgs args) {
   extern __shared__ uint8_t smem_raw[];
@@ -388,7 +400,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       const GemmArgs& g = ph.gemm;
       const int k_blocks = g.k_blocks;
       const int box = box_of(tile.rows);
-      const int a_row0 = ph.used != nullptr ? 0 : tile.row0;
+      const int a_row0 = TOKEN_ORDER && ph.used != nullptr ? 0 : tile.row0;
       const uint8_t* sfa_src = g.sfa + static_cast<size_t>(a_row0 >> 7) * k_blocks * kSfaBytes;
       if (ph.wait_target > 0) {
         ok = wait_count(ph.ready + (tile.row0 >> 7), ph.wait_target);
@@ -512,10 +524,11 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
       const StreamPhase& ph = args.phase[tile.phase];
       const GemmArgs& g = ph.gemm;
       const int grow = tile.row0 + r;
-      const bool row_valid = r < tile.rows && (ph.used == nullptr || ph.used[grow] >= 0);
+      const int32_t* used = TOKEN_ORDER ? ph.used : nullptr;
+      const bool row_valid = r < tile.rows && (used == nullptr || used[grow] >= 0);
       float scale = g.w_tensor_scale[tile.expert];
       if (g.a_tensor_scale != nullptr && row_valid) {
-        scale *= g.a_tensor_scale[ph.used != nullptr ? r : grow];
+        scale *= g.a_tensor_scale[used != nullptr ? r : grow];
       }
       unsigned long long dest = row_valid ? 1 : 0;  // (up: whether the row counts)
       float wt = 1.0f;
@@ -557,7 +570,8 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
             const float row_wt = __shfl_sync(0xffffffffu, wt, from & 31);
             const unsigned long long row_dest = __shfl_sync(0xffffffffu, dest, from & 31);
             const int n = n0 + half * (kBN / 2) + chunk * 16;
-            if (from >= tile.rows || chunk * 16 >= columns || row_dest == 0) continue;
+            if (from >= tile.rows || chunk * 16 >= columns) continue;
+            if ((TOKEN_ORDER || ph.mode == kGemmDown) && row_dest == 0) continue;
             float v[16];
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
@@ -601,18 +615,15 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   } else if (warp == 0 && args.ticket != nullptr) {
-    // the last CTA leaves the counts at zero for the next launch
+    // the last CTA leaves the counts at zero for the next launch, and the words of the front end before it
     int ticket = 0;
     if (lane == 0) {
       __threadfence();
-      ticket = atomicAdd(args.finished, 1);
+      ticket = add_acquire(args.finished, 1);
     }
     ticket = __shfl_sync(0xffffffffu, ticket, 0);
     if (ticket == units - 1) {
       if (lane == 0 && args.error_host != nullptr) {
-        // the count of the other CTAs comes before their error (a fence behind the stores below would
-        // wait for them, 0.6 us)
-        __threadfence();
         const int code = *static_cast<volatile int32_t*>(args.error);
         if (code != kDevOk) {
           *static_cast<volatile int32_t*>(args.error_host) = code;
@@ -620,6 +631,7 @@ expert_stream_kernel(const __grid_constant__ StreamArgs args) {
         }
       }
       for (int i = lane; i < args.ready_count; i += 32) args.ready[i] = 0;
+      if (TOKEN_ORDER && lane < args.front_word_count) args.front_words[lane] = 0;
       if (lane == 0) {
         *args.ticket = 0;
         *args.finished = 0;
@@ -637,19 +649,23 @@ cudaError_t launch_expert_stream(const StreamArgs& args, int num_sms, LaunchStre
       (args.tile_rows != 32 && args.tile_rows != 64 && args.tile_rows != 128)) {
     return cudaErrorInvalidValue;
   }
-  cudaError_t err = allow_shared_memory(expert_stream_kernel);
-  if (err != cudaSuccess) return err;
   // one persistent CTA per SM, fewer when the tiles are known to be fewer
   int grid = num_sms;
   int dense_tiles = 0;
-  bool grouped = false;
+  bool grouped = false, token_order = false;
   for (int p = 0; p < args.phases; ++p) {
     const GemmArgs& g = args.phase[p].gemm;
     grouped = grouped || g.row_tiles != nullptr;
+    token_order = token_order || args.phase[p].used != nullptr;
     dense_tiles += (g.dense_rows + 127) / 128 * g.n_tiles;
   }
   if (!grouped) grid = std::max(1, std::min(grid, dense_tiles));
-  return launch_kernel(expert_stream_kernel, grid, kThreads, smem_bytes(args.tile_rows), stream, args);
+  auto run = [&](auto kernel) {
+    const cudaError_t err = allow_shared_memory(kernel);
+    if (err != cudaSuccess) return err;
+    return launch_kernel(kernel, grid, kThreads, smem_bytes(args.tile_rows), stream, args);
+  };
+  return token_order ? run(expert_stream_kernel<true>) : run(expert_stream_kernel<false>);
 }
 
 }  // namespace nmoe

@@ -62,21 +62,15 @@ __device__ __forceinline__ void load_gate8(const FrontArgs& args, size_t i, floa
   }
 }
 
-struct Scratch : FrontWords {
+struct Scratch {
+  int32_t row_known[kFrontMaxRows];    // whether 1/rms is; cleared by the launch behind, as is the next
+  int32_t row_rounded[kFrontLinears];  // ... the one row as a linear multiplies with it
+  int32_t finished;                    // blocks whose logits are there; zero between launches, as is the next
+  int32_t linear_finished[kFrontLinears];
   float score[kFrontMaxRows][kFrontMaxExperts];
   float choice[kFrontMaxRows][kFrontMaxExperts];
 };
 static_assert(sizeof(Scratch) == front_scratch_bytes(), "scratch size");
-
-// By one thread of the group's last block, behind a barrier.
-__device__ __forceinline__ void group_through(const FrontArgs& args, Scratch* scratch) {
-  front_group_through(scratch, args.rows, args.linears, [](int32_t* word) {
-    __threadfence();  // what the group announced and waited for comes before the count
-    const int before = atomicAdd(word, 1);
-    __threadfence();
-    return before;
-  });
-}
 
 // The logits and scores of EXPERTS experts (`step` apart) for ROWS tokens from `row0` (the last one
 // repeated where there are fewer).
@@ -433,7 +427,6 @@ front_kernel(const __grid_constant__ FrontArgs args) {
           args.cols % 64 == 0, shared.norm, known);
     };
     if (args.in_bf16) run(std::true_type()); else run(std::false_type());
-    if (threadIdx.x == 0) group_through(args, scratch);
     return;
   }
   block -= args.rows;
@@ -444,7 +437,6 @@ front_kernel(const __grid_constant__ FrontArgs args) {
       if (threadIdx.x == 0) {
         __threadfence();  // what this block's threads stored, as of the barrier
         store_release_word(&scratch->row_rounded[block], 1);
-        group_through(args, scratch);
       }
       return;
     }
@@ -457,8 +449,6 @@ front_kernel(const __grid_constant__ FrontArgs args) {
   if (!LINEARS || block < gate_blocks) {
     expert_logits<ROWS, kExperts>(args, scratch, block % step, step, block / step * ROWS);
     if (!last_of(&scratch->finished, gate_blocks)) return;
-    // (by a thread that selects for the eighth token only, beside the loads of the scores)
-    if (threadIdx.x == kThreads - 1) group_through(args, scratch);
     select_and_plan<PER_LANE>(args, scratch, shared.select);
   } else {
     block -= gate_blocks;
@@ -477,7 +467,6 @@ front_kernel(const __grid_constant__ FrontArgs args) {
       linear_outputs<kWeightF32>(args, scratch, linear, which, n0, shared.warp_sum);
     }
     if (!last_of(&scratch->linear_finished[which], linear_blocks(linear.N))) return;
-    if (threadIdx.x == kThreads - 1) group_through(args, scratch);
     norm_quant_by_block<false, kQuantChunks>(
         linear.out, 0, linear.N, nullptr, 0.0f, nullptr, linear.packed, linear.sf_row_major,
         linear.sf_tiled, linear.k_tiles, linear.tensor_scale, nullptr, linear.N % 64 == 0, shared.norm,

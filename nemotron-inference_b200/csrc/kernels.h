@@ -9,8 +9,6 @@
 #include <cstddef>
 #include <cstdint>
 
-#include "front_words.h"
-
 namespace nmoe {
 
 // Where a kernel is launched.  `chained`: what precedes it on the stream is a kernel of this library,
@@ -185,6 +183,11 @@ struct StreamArgs {
   bool fetch_dense = false;
   int32_t* ticket = nullptr;
   int32_t* finished = nullptr;
+  // (with StreamPhase::used) words that the last CTA clears: those through which the blocks of the front end
+  // (csrc/front.cu) hand rows on.  That launch cannot clear them itself: a block that waits gives up after a
+  // while, and what it gave up on may be announced until the launch has ended.
+  int32_t* front_words = nullptr;
+  int32_t front_word_count = 0;
   // nullable, host memory: the last CTA stores there what it finds in `error`, unless that is nothing
   int32_t* error_host = nullptr;
 };
@@ -451,11 +454,13 @@ cudaError_t launch_place_rows(const PlanBuffers& plan, const PermuteSource& src,
                               int32_t* pair_row /* nullable */, int dest_stride, int32_t* error,
                               int num_sms, LaunchStream stream);
 // --- front end of a handful of tokens (csrc/front.cu) ---------------------------
+constexpr int kFrontMaxRows = 8;
 constexpr int kFrontMaxCols = 4096;
 constexpr int kFrontMaxExperts = 512;     // of one token
 constexpr int kFrontMaxExpertsOfRows = 256;  // of several
 constexpr int kFrontRowsPerBlock = 4;        // of several, for which a block forms an expert's logits
 constexpr int kFrontBlocksPerSm = 2;         // of a launch over several
+constexpr int kFrontLinears = 2;
 // A linear of the one token's normalised row whose FP32 row is then quantised with its tensor scale.
 constexpr int kFrontLinearMaxN = 6144;
 constexpr int kFrontLinearBlocksPerSm = 3;  // of a launch with linears
@@ -509,11 +514,14 @@ struct FrontArgs {
   FrontLinear linear[kFrontLinears];
   int linears = 0;
   int resident_blocks = 0;  // of a launch with linears, on all SMs together
-  void* scratch = nullptr;  // front_scratch_bytes(), zero before the first launch
+  // front_scratch_bytes(), zero before the first launch; its first kFrontWords words have to be zero again
+  // before every other, which is left to the kernel behind (StreamArgs::front_words)
+  void* scratch = nullptr;
   int32_t* error = nullptr;
 };
+constexpr int kFrontWords = kFrontMaxRows + kFrontLinears;
 constexpr size_t front_scratch_bytes() {
-  return sizeof(FrontWords) + 2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
+  return (kFrontWords + 1 + kFrontLinears) * sizeof(int32_t) + 2 * kFrontMaxRows * kFrontMaxExperts * sizeof(float);
 }
 cudaError_t launch_front(const FrontArgs& args, cudaStream_t stream);
 // Whether one launch is the faster front end of `rows` tokens.

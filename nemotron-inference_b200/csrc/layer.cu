@@ -470,6 +470,7 @@ struct StreamFfn {
   const float* hidden_tensor_scale = nullptr;
   RowOutput out;
   const int32_t* used = nullptr;  // StreamPhase::used of the up projection
+  int32_t* front_words = nullptr;  // StreamArgs::front_words
   int row_slots = 0;  // most 128-row slots the schedule may use
 };
 
@@ -518,6 +519,8 @@ void run_stream(const StreamFfn* routed, const StreamFfn* shared, const StreamCo
   if (routed != nullptr) {
     args.row_tiles = routed->schedule.row_tiles;
     args.row_tile_room = routed->row_slots;
+    args.front_words = routed->front_words;
+    args.front_word_count = routed->front_words != nullptr ? kFrontWords : 0;
   }
   int32_t* routed_ready = args.ready;
   int32_t* shared_ready = args.ready + (routed != nullptr ? routed->row_slots : 0);
@@ -1072,6 +1075,7 @@ struct nmoe_layer {
   ActivationOperand y_op, lat_op, sh_op, a_op, h_op;
   StreamCounts stream_counts;
   DeviceBuffer front_scratch, front_rounded;  // of csrc/front.cu
+  bool front_words_set = false;  // a front end was launched, and nothing behind it that clears its words
   ErrorSlot error;
   int last_tokens = 0;
   std::string last_error;
@@ -1654,7 +1658,10 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
     ffn.a = !token_order ? &L->a_op : L->latent_mode ? &L->lat_op : &L->y_op;
     ffn.a_tensor_scale =
         (!token_order ? L->a_ts : L->latent_mode ? L->lat_ts : L->y_ts).as<float>();
-    if (token_order) ffn.used = L->a_dest.as<int32_t>();
+    if (token_order) {
+      ffn.used = L->a_dest.as<int32_t>();
+      ffn.front_words = L->front_scratch.as<int32_t>();
+    }
     ffn.schedule = routed;
     ffn.hidden_packed = L->h_packed.as<uint8_t>();
     ffn.hidden_sf = L->h_sf.as<uint8_t>();
@@ -1662,6 +1669,7 @@ void routed_experts(nmoe_layer* L, LaunchStream stream, const PermuteSource& sou
     ffn.out = out;
     ffn.row_slots = L->max_row_tiles;
     run_stream(&ffn, shared, L->stream_counts, error, L->num_sms, stream);
+    if (token_order) L->front_words_set = false;
     L->mark(6, stream);  // (one launch: its time is that of the up projections' stage)
     return;
   }
@@ -1911,6 +1919,10 @@ void route_few(nmoe_layer* L, cudaStream_t stream, const void* input, nmoe_dtype
   args.resident_blocks = kFrontLinearBlocksPerSm * L->num_sms;
   args.scratch = L->front_scratch.as<void>();
   args.error = L->error.device.as<int32_t>();
+  if (L->front_words_set) {  // (the launch that clears them was not made)
+    NMOE_CUDA(cudaMemsetAsync(args.scratch, 0, front_scratch_bytes(), stream));
+  }
+  L->front_words_set = true;
   NMOE_CUDA(launch_front(args, stream));
   L->last_normalized = true;
 }
