@@ -147,13 +147,12 @@ grouped_gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const GemmArgs a
       mbar_init(&tmem_empty_bar[a], 2 * kEpilogueWarps);
     }
     fence_barrier_init();
+    for (int i = 0; i < kPairBoxes; ++i) prefetch_tensormap(&maps.a[i]);
     prefetch_tensormap(&maps.b_tail);
     prefetch_tensormap(&maps.b_full);
     prefetch_tensormap(&maps.sfa);
     prefetch_tensormap(&maps.sfb);
   }
-  // (one to a thread: eight in turn were 0.3 us of a launch)
-  if (warp == 2 && lane < kPairBoxes) prefetch_tensormap(&maps.a[lane]);
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, 512);
     tmem_relinquish_pair();
