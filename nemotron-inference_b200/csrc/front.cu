@@ -203,7 +203,7 @@ __device__ __forceinline__ void select_and_plan(const FrontArgs& args, const Scr
   float weight = 0.0f;
   if (warp < args.rows) {
     float score;
-    const float sum = select_experts<(PER_LANE > 4)>(
+    const float sum = select_experts<PER_LANE>(
         shared.scores[warp], shared.choices[warp], shared.list[PER_LANE > 4 ? warp : 0], experts, top_k,
         args.n_group, args.topk_group, index, score);
     weight = selected_weight(score, sum, args.norm_topk_prob, args.routed_scaling);

@@ -101,8 +101,8 @@ constexpr int kMaxExperts = 512;
 // One block per token.  All threads evaluate sigmoids (the exponential in double is the
 // longest single step; one for each expert while blocks are few, else 128), one warp selects:
 // expert e lives in lane e % 32, and a round is one warp-wide maximum of order-preserving keys and one
-// minimum over the indices that hold it (ties go to the lower expert).  Up to 128 experts every lane keeps
-// the best of its four at hand; more are narrowed down to some forty first, two to a lane (csrc/topk.cuh).
+// minimum over the indices that hold it (ties go to the lower expert).  Every lane keeps the best of its
+// own at hand, or many experts are narrowed down to some forty first, two to a lane (csrc/topk.cuh).
 // Bound by the latency of that chain: 1 token, 128 experts, top-6 14.9 -> 8.2 us between events; 3000
 // tokens, 512 experts, top-22 27.4 us with sixteen choices a lane, 19.1 narrowed down.
 template <int PER_LANE>
@@ -130,7 +130,7 @@ router_topk_kernel(const float* logits, const float* __restrict__ bias, int expe
   int my_index;
   float my_score;
   const float weight_sum =
-      select_experts<(PER_LANE > 4)>(score_smem, choice_smem, list, experts, top_k, n_group, topk_group,
+      select_experts<PER_LANE>(score_smem, choice_smem, list, experts, top_k, n_group, topk_group,
                                      my_index, my_score);
   if (lane < top_k) {
     top_index[static_cast<size_t>(row) * top_k + lane] = my_index;

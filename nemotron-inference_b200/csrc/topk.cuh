@@ -132,10 +132,11 @@ __device__ __forceinline__ int select_among_many(uint32_t* keys, uint32_t* list,
   return my_index;
 }
 
-// The same for up to 128 experts: each lane holds four, the best of which it keeps at hand.
+// The same for up to 32 * PER_LANE experts: each lane holds its own, the best of which it keeps at hand.
+template <int PER_LANE>
 __device__ __forceinline__ int select_among_few(const float* choice_smem, int experts, int top_k,
                                                 int n_group, uint32_t selected_groups) {
-  constexpr int kPerLane = 4;
+  constexpr int kPerLane = PER_LANE;
   const int lane = threadIdx.x & 31;
   const int group_size = experts / n_group;
   uint32_t key[kPerLane];
@@ -181,18 +182,28 @@ __device__ __forceinline__ int select_among_few(const float* choice_smem, int ex
 
 // By all lanes of a warp, from a token's scores and choices (score + bias) in shared memory: lane r ends
 // up with the r-th selected expert and its score; returns the sum of the selected scores in selection
-// order.  MANY: more than 128 experts; the choices are overwritten then.
-template <bool MANY>
+// order.  PER_LANE: 4, 8 or 16, for up to 32 times as many experts; the choices may be overwritten.
+//
+// Narrowing down pays from some ten rounds on, while the lanes' maxima still leave few: the bound of 24 of 32
+// lanes leaves more than the list holds for one token in a thousand of 512 experts, that of 27 for one in ten, and
+// a launch waits for the slowest (9 tokens, top-27 49.6 us looked through and 62.2, top-32 53.7 and 67.8).
+// Whole pass, looked through against narrowed down: 256 experts, 16 tokens, top-4 32.4 us and 33.1, top-8 35.7 and
+// 36.8, top-12 39.3 and 39.5, top-16 42.6 and 41.8, top-32 51.4 and 57.6; 160 experts, 9 tokens, top-4 27.5 and
+// 28.9, top-12 33.8 and 33.8, top-22 39.2 and 37.3, top-32 41.3 and 45.4.  Sixteen to a lane are narrowed down
+// whatever top_k up to that (512 experts, top-22 13 us in a launch's last block looked through, 5.8 narrowed down).
+constexpr int kSelectFewTopK = 10;
+constexpr int kSelectMostNarrowed = 23;
+template <int PER_LANE>
 __device__ __forceinline__ float select_experts(const float* score_smem, float* choice_smem,
                                                 uint32_t* list, int experts, int top_k, int n_group,
                                                 int topk_group, int& my_index, float& my_score) {
   const uint32_t groups = select_groups(choice_smem, experts, n_group, topk_group);
   __syncwarp();
-  if constexpr (MANY) {
+  if (PER_LANE <= 4 || (PER_LANE <= 8 && top_k <= kSelectFewTopK) || top_k > kSelectMostNarrowed) {
+    my_index = select_among_few<PER_LANE>(choice_smem, experts, top_k, n_group, groups);
+  } else {
     my_index = select_among_many(reinterpret_cast<uint32_t*>(choice_smem), list, experts, top_k,
                                  n_group, groups);
-  } else {
-    my_index = select_among_few(choice_smem, experts, top_k, n_group, groups);
   }
   // weight = score (no bias) normalised over the selection in selection order
   // (:349-365)

@@ -122,8 +122,11 @@ def test_one_token_of_a_latent_layer(package, synthetic, experts, top_k, hidden,
     layer.close()
 
 
-# experts beyond 128 are narrowed down first, unless too many share the bound
-@pytest.mark.parametrize("experts,top_k,n_group", [(160, 1, 1), (256, 8, 8), (512, 22, 1), (512, 32, 4)])
+# many experts are narrowed down first (from 11 to 23 selected ones, or beyond 256), unless too many share the
+# bound
+@pytest.mark.parametrize("experts,top_k,n_group", [(160, 1, 1), (256, 8, 8), (512, 22, 1), (512, 32, 4),
+                                                   (160, 10, 1), (160, 11, 1), (256, 16, 8), (384, 1, 1),
+                                                   (512, 23, 1), (512, 24, 1)])
 @pytest.mark.parametrize("levels", [1, 3, 100000])
 def test_selection_among_many_with_ties(package, oracle, experts, top_k, n_group, levels):
     g = torch.Generator().manual_seed(experts + levels)
