@@ -205,7 +205,7 @@ __device__ __forceinline__ void select_and_plan(const FrontArgs& args, const Scr
     float score;
     const float sum = select_experts<PER_LANE>(
         shared.scores[warp], shared.choices[warp], shared.list[PER_LANE > 4 ? warp : 0], experts, top_k,
-        args.n_group, args.topk_group, index, score);
+        args.n_group, args.topk_group, select_narrows(PER_LANE, top_k), index, score);
     weight = selected_weight(score, sum, args.norm_topk_prob, args.routed_scaling);
     if (lane < top_k) shared.slot_of[index][warp] = static_cast<int16_t>(lane);
   }

@@ -105,7 +105,9 @@ constexpr int kMaxExperts = 512;
 // own at hand, or many experts are narrowed down to some forty first, two to a lane (csrc/topk.cuh).
 // Bound by the latency of that chain: 1 token, 128 experts, top-6 14.9 -> 8.2 us between events; 3000
 // tokens, 512 experts, top-22 27.4 us with sixteen choices a lane, 19.1 narrowed down.
-template <int PER_LANE>
+// NARROWED: select_narrows(); a kernel that held both ways took the registers of the wider one (1003 tokens, 384
+// experts, top-8 205.7 us a pass and 214.5).
+template <int PER_LANE, bool NARROWED>
 __global__ void __launch_bounds__(PER_LANE * 32 < 128 ? 128 : PER_LANE * 32)
 router_topk_kernel(const float* logits, const float* __restrict__ bias, int experts,
                    int top_k, int n_group, int topk_group, bool norm_topk_prob,
@@ -131,7 +133,7 @@ router_topk_kernel(const float* logits, const float* __restrict__ bias, int expe
   float my_score;
   const float weight_sum =
       select_experts<PER_LANE>(score_smem, choice_smem, list, experts, top_k, n_group, topk_group,
-                                     my_index, my_score);
+                               NARROWED, my_index, my_score);
   if (lane < top_k) {
     top_index[static_cast<size_t>(row) * top_k + lane] = my_index;
     top_weight[static_cast<size_t>(row) * top_k + lane] =
@@ -188,12 +190,14 @@ cudaError_t launch_router_topk(const float* logits, const float* bias, int rows,
                                               norm_topk_prob, routed_scaling, top_index, top_weight,
                                               expert_counts, position);
   };
+  constexpr int kMostPerLane = kMaxExperts / 32;
   if (experts <= 128) {
-    run(router_topk_kernel<4>, 4 * 32);
+    run(router_topk_kernel<4, false>, 4 * 32);
   } else if (experts <= 256) {
-    run(router_topk_kernel<8>, 8 * 32);
+    run(select_narrows(8, top_k) ? router_topk_kernel<8, true> : router_topk_kernel<8, false>, 8 * 32);
   } else {
-    run(router_topk_kernel<kMaxExperts / 32>, kMaxExperts);
+    run(select_narrows(kMostPerLane, top_k) ? router_topk_kernel<kMostPerLane, true>
+                                            : router_topk_kernel<kMostPerLane, false>, kMaxExperts);
   }
   return cudaGetLastError();
 }

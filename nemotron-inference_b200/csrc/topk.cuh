@@ -193,17 +193,22 @@ __device__ __forceinline__ int select_among_few(const float* choice_smem, int ex
 // whatever top_k up to that (512 experts, top-22 13 us in a launch's last block looked through, 5.8 narrowed down).
 constexpr int kSelectFewTopK = 10;
 constexpr int kSelectMostNarrowed = 23;
+__host__ __device__ constexpr bool select_narrows(int per_lane, int top_k) {
+  return per_lane > 4 && (per_lane > 8 || top_k > kSelectFewTopK) && top_k <= kSelectMostNarrowed;
+}
+// (`narrowed`: select_narrows() of the two, a constant where a kernel is to hold only one of the ways)
 template <int PER_LANE>
 __device__ __forceinline__ float select_experts(const float* score_smem, float* choice_smem,
                                                 uint32_t* list, int experts, int top_k, int n_group,
-                                                int topk_group, int& my_index, float& my_score) {
+                                                int topk_group, bool narrowed, int& my_index,
+                                                float& my_score) {
   const uint32_t groups = select_groups(choice_smem, experts, n_group, topk_group);
   __syncwarp();
-  if (PER_LANE <= 4 || (PER_LANE <= 8 && top_k <= kSelectFewTopK) || top_k > kSelectMostNarrowed) {
-    my_index = select_among_few<PER_LANE>(choice_smem, experts, top_k, n_group, groups);
-  } else {
+  if (PER_LANE > 4 && narrowed) {
     my_index = select_among_many(reinterpret_cast<uint32_t*>(choice_smem), list, experts, top_k,
                                  n_group, groups);
+  } else {
+    my_index = select_among_few<PER_LANE>(choice_smem, experts, top_k, n_group, groups);
   }
   // weight = score (no bias) normalised over the selection in selection order
   // (:349-365)
